@@ -3,6 +3,7 @@
 There is no fallback: if the shared library is missing or a call fails, an exception is raised.
 """
 import ctypes
+import importlib.util
 import os
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_uint8, c_void_p
 
@@ -32,6 +33,7 @@ PROTOTYPES = {
     "lmk_last_error": (c_char_p, []),
     "lmk_device_status": (c_int, [POINTER(c_int), c_int]),
     "lmk_debug_set_max_ctas": (None, [c_int]),
+    "lmk_mask_is_regular": (c_int, [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p]),
     "lmk_attn_tcgen05_supported": (c_int, [c_int] * 7),
     "lmk_attn_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                              c_int, c_int, c_int, c_int, c_int, POINTER(c_int64), POINTER(c_int64), POINTER(c_int64),
@@ -91,6 +93,9 @@ PROTOTYPES = {
 }
 
 _lib = None
+_host = None
+_host_hooks = []
+HOST_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_lmk_host.so")
 c_void_p = c_void_p          # re-exported for callers that pass raw stream handles
 
 
@@ -107,6 +112,35 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+def host():
+    """The native host layer (csrc/host_torch.cpp): the public entry points' checks, allocations, autograd nodes and
+    kernel calls.  Its functions call the library that `lib()` loads."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: run `python -m landmark_attention_b200.build` "
+                               "(there is no fallback path)")
+        spec = importlib.util.spec_from_file_location("_lmk_host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.init(LIB_PATH)
+        _host = module
+        for fn in _host_hooks:
+            fn()
+    return _host
+
+
+def on_host_load(fn):
+    """Run fn once the host layer is loaded.  Tries to load it now, so that a tracing compiler finds the operators
+    registered; a package that has not been built yet stays importable and raises at the first call."""
+    _host_hooks.append(fn)
+    try:
+        host()
+    except (RuntimeError, AttributeError, OSError, ImportError):
+        pass
 
 
 def device_status(clear: bool = True) -> int:

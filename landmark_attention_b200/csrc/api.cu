@@ -79,6 +79,18 @@ int pick_path(int path, const AttnParams& p, int dtype, bool backward) {
   return LMK_PATH_GENERAL;
 }
 
+// *irregular = 1 (a word of mapped host memory) if any flag differs from "last token of every block"
+__global__ void __launch_bounds__(256) mask_is_regular_kernel(const uint8_t* __restrict__ m, int64_t n, int row, int block,
+                                                              int* irregular) {
+  bool bad = false;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    bad |= m[i] != (uint8_t)((i % row) % block == block - 1);
+  if (__syncthreads_or(bad) && threadIdx.x == 0) {
+    *irregular = 1;
+    __threadfence_system();
+  }
+}
+
 }  // namespace
 }  // namespace lmk
 
@@ -195,6 +207,16 @@ extern "C" int lmk_attn_bwd_static(const void* q, const void* k, const void* v, 
   if (rc != LMK_OK) return rc;
   return lmk_attn_bwd(q, k, v, o, dO, L, M, dQ, dK, dV, scratch, sizeof(float) * (size_t)LMK_STATIC_SCRATCH_FLOATS, B,
                       H, Lq, Lk, D, q_strides, k_strides, v_strides, block, sm_scale, dtype, path, stream);
+}
+
+extern "C" int lmk_mask_is_regular(const uint8_t* mask, int64_t n, int row, int block, int* irregular, void* stream) {
+  LMK_CHECK_ARG(mask && irregular, "mask_is_regular: null pointer");
+  LMK_CHECK_ARG(n >= 0 && row >= 1 && block >= 1, "mask_is_regular: bad sizes");
+  if (n == 0) return LMK_OK;
+  const int64_t ctas = (n + 255) / 256;
+  mask_is_regular_kernel<<<(unsigned)(ctas < 296 ? ctas : 296), 256, 0, (cudaStream_t)stream>>>(mask, n, row, block, irregular);
+  LMK_CUDA(cudaGetLastError());
+  return LMK_OK;
 }
 
 // ------------------------------------------------------------------------------------------------ arbitrary landmarks

@@ -1,0 +1,591 @@
+// Host layer between PyTorch and libb200lmk.so: argument checks, output allocation, autograd nodes and kernel calls of
+// the public entry points in native code.
+//
+// Why it exists: the kernels of a short call take 5 - 50 us, and the same steps written in Python (ctypes conversions,
+// Python autograd functions, torch.library wrappers) took 75 - 160 us of host time per call, so every small and
+// medium call was host-bound (a 77-token prompt: 83 us a call in Python, 48 us here with the same kernels; the GPT layer's
+// training step 416 -> 328 us).  Here a call is one Python -> C++ transition, and the backward pass runs in the autograd
+// engine without the interpreter lock.
+//
+// The C ABI of include/b200lmk.h stays the only way into the kernels: its functions are looked up in the library that
+// the Python side has loaded (init()), so an override of the library's location holds here as well.
+#include <dlfcn.h>
+
+#include <mutex>
+#include <optional>
+#include <string>
+#include <tuple>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/library.h>
+#include <Python.h>
+
+#include "../../include/b200lmk.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+// ------------------------------------------------------------------------------------------------ library functions
+#define LMK_FUNCS(X)                                                                                             \
+  X(lmk_last_error) X(lmk_attn_fwd) X(lmk_attn_bwd_workspace) X(lmk_attn_bwd) X(lmk_attn_mask_fwd)               \
+  X(lmk_attn_mask_bwd_workspace) X(lmk_attn_mask_bwd) X(lmk_grouped_softmax_fwd) X(lmk_grouped_softmax_bwd)      \
+  X(lmk_grouped_softmax_causal_fwd) X(lmk_grouped_softmax_causal_bwd) X(lmk_rotary_apply) X(lmk_mask_is_regular)
+struct Lib {
+#define X(name) decltype(&::name) name = nullptr;
+  LMK_FUNCS(X)
+#undef X
+} lib;
+
+// ------------------------------------------------------------------------------------------------ errors
+// AssertionError from any thread, with or without the interpreter lock (the backward pass runs without it)
+[[noreturn]] void raise_assertion(const std::string& msg) {
+  pybind11::gil_scoped_acquire gil;
+  PyErr_SetString(PyExc_AssertionError, msg.c_str());
+  python_error e;
+  e.persist();
+  throw e;
+}
+#define LMK_ASSERT(cond, msg) do { if (!(cond)) raise_assertion(msg); } while (0)
+
+// status codes -> the exception classes the reference raises for the same mistake
+void check(int rc, const char* what) {
+  if (rc == LMK_OK) return;
+  const std::string msg = lib.lmk_last_error();
+  if (rc == LMK_ERR_INVALID) raise_assertion(std::string(what) + ": " + msg);
+  if (rc == LMK_ERR_UNSUPPORTED) C10_THROW_ERROR(NotImplementedError, std::string(what) + ": " + msg);
+  TORCH_CHECK(false, what, " failed (", rc, "): ", msg);
+}
+
+void require_cuda(const Tensor& t) {
+  LMK_ASSERT(t.is_cuda(), "landmark_attention_b200 runs on CUDA tensors only (no CPU path)");
+}
+
+int dtype_code(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return LMK_F32;
+    case at::kHalf: return LMK_F16;
+    case at::kBFloat16: return LMK_BF16;
+    default: raise_assertion(std::string("unsupported dtype ") + c10::toString(t.scalar_type()));
+  }
+}
+
+struct S3 {
+  int64_t v[3];
+  explicit S3(const Tensor& t) { auto st = t.strides(); v[0] = st[0]; v[1] = st[1]; v[2] = st[2]; }
+};
+
+Tensor last_dim_dense(const Tensor& t) { return t.stride(3) == 1 ? t : t.contiguous(); }
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+Tensor empty_like_dtype(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().requires_grad(false)); }
+Tensor empty_f32(at::IntArrayRef sizes, const Tensor& like) {
+  return at::empty(sizes, like.options().requires_grad(false).dtype(at::kFloat));
+}
+bool needs_grad(std::initializer_list<std::reference_wrapper<const Tensor>> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor& t : ts) if (t.requires_grad()) return true;
+  return false;
+}
+
+// ------------------------------------------------------------------------------------------------ fused attention
+// statistics [2, B*H, Lq]: the outer softmax's sum and maximum
+Tensor attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, int64_t block, int64_t path, Tensor* stats) {
+  const auto B = q.size(0), H = q.size(1), Lq = q.size(2), D = q.size(3), Lk = k.size(2);
+  Tensor o = empty_like_dtype({B, H, Lq, D}, q);
+  *stats = empty_f32({2, B * H, Lq}, q);
+  float* l = stats->data_ptr<float>();
+  check(lib.lmk_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), l, l + B * H * Lq, B, H, Lq, Lk, D,
+                         S3(q).v, S3(k).v, S3(v).v, block, (float)scale, dtype_code(q), path, stream_of(q)),
+        "lmk_attn_fwd");
+  return o;
+}
+
+struct FusedLandmark : public torch::autograd::Function<FusedLandmark> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale,
+                        int64_t block, int64_t path) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    Tensor stats, o = attn_fwd(q, k, v, scale, block, path, &stats);
+    ctx->save_for_backward({q, k, v, o, stats});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["block"] = block;
+    ctx->saved_data["path"] = path;
+    return o;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    auto saved = ctx->get_saved_variables();
+    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &o = saved[3], &stats = saved[4];
+    const int64_t block = ctx->saved_data["block"].toInt(), path = ctx->saved_data["path"].toInt();
+    const double scale = ctx->saved_data["scale"].toDouble();
+    const auto B = q.size(0), H = q.size(1), Lq = q.size(2), D = q.size(3), Lk = k.size(2);
+    LMK_ASSERT(Lq % block == 0 && Lk % block == 0, "Backward supported only for full blocks");
+    c10::cuda::OptionalCUDAGuard guard(q.device());
+    Tensor dO = grads[0].contiguous();
+    if (dO.scalar_type() != q.scalar_type()) dO = dO.to(q.scalar_type());
+    Tensor dq = empty_like_dtype({B, H, Lq, D}, q), dk = empty_like_dtype({B, H, Lk, D}, q), dv = empty_like_dtype({B, H, Lk, D}, q);
+    const int code = dtype_code(q);
+    const size_t need = std::max<size_t>(lib.lmk_attn_bwd_workspace(B, H, Lq, Lk, D, block, code, path), 256);
+    Tensor ws = at::empty({(int64_t)need}, q.options().requires_grad(false).dtype(at::kByte));
+    const float* l = stats.data_ptr<float>();
+    check(lib.lmk_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dO.data_ptr(), l, l + B * H * Lq,
+                           dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), need, B, H, Lq, Lk, D, S3(q).v,
+                           S3(k).v, S3(v).v, block, (float)scale, code, path, stream_of(q)),
+          "lmk_attn_bwd");
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// The checks of FusedLandmarkAttention.forward (flash_landmark_attention.py:319-324), then the kernels.
+Tensor fused_attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, int64_t n_prefix, double scale, int64_t block,
+                       int64_t path) {
+  require_cuda(q_); require_cuda(k_); require_cuda(v_);
+  LMK_ASSERT(q_.dim() == 4 && k_.dim() == 4 && v_.dim() == 4, "expected q, k, v of shape [B, H, L, D]");
+  const auto d = q_.size(3);
+  for (const Tensor* t : {&k_, &v_})
+    LMK_ASSERT(t->size(0) == q_.size(0) && t->size(1) == q_.size(1) && t->size(2) == k_.size(2) && t->size(3) == d,
+               "k and v must be [B, H, Lk, D] with q's batch, heads and head dim");
+  LMK_ASSERT(d <= 128, "FlashAttention only support head dimensions up to 128");
+  LMK_ASSERT(q_.scalar_type() == k_.scalar_type() && q_.scalar_type() == v_.scalar_type(), "All tensors must have the same type");
+  LMK_ASSERT(k_.size(2) - q_.size(2) == n_prefix * block, "key history must be whole blocks");
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = last_dim_dense(q_), k = last_dim_dense(k_), v = last_dim_dense(v_);
+  if (!needs_grad({q, k, v})) {
+    Tensor stats;
+    return attn_fwd(q, k, v, scale, block, path, &stats);
+  }
+  return FusedLandmark::apply(q, k, v, scale, block, path);
+}
+
+// ------------------------------------------------------------------------------------------------ landmark mask check
+// One kernel compares every flag with the regular pattern and writes a word of mapped host memory; the host waits for
+// that kernel alone (an event), so what the caller enqueues between the constructor and failed() overlaps with it.
+class RegularCheck {
+ public:
+  RegularCheck(const Tensor& is_mem, int64_t block) {
+    Tensor m = is_mem.contiguous();
+    if (!m.is_cuda()) {
+      const Tensor want = at::arange(m.size(-1), m.options().dtype(at::kLong)).remainder(block).eq(block - 1);
+      host_failed_ = !m.eq(want).all().item<bool>();
+      return;
+    }
+    if (m.element_size() != 1) m = m.eq(1).to(at::kByte).add_(m.ne(0).logical_and_(m.ne(1)), 2);     // 2: neither
+    slot_ = &local_slot(m.get_device());
+    *slot_->word = 0;
+    check(lib.lmk_mask_is_regular((const uint8_t*)m.data_ptr(), m.numel(), m.size(-1), block, slot_->word, stream_of(m)),
+          "lmk_mask_is_regular");
+    C10_CUDA_CHECK(cudaEventRecord(slot_->event, (cudaStream_t)stream_of(m)));
+  }
+  bool failed() const {
+    if (slot_ == nullptr) return host_failed_;
+    C10_CUDA_CHECK(cudaEventSynchronize(slot_->event));
+    return *reinterpret_cast<volatile int*>(slot_->word) != 0;
+  }
+
+ private:
+  struct Slot { int* word = nullptr; cudaEvent_t event = nullptr; };
+  // one word and one event per thread and device, for the life of the program (16 bytes of pinned memory each)
+  static Slot& local_slot(int dev) {
+    constexpr int kMax = 64;
+    static thread_local Slot slots[kMax];
+    TORCH_CHECK(dev >= 0 && dev < kMax, "device index out of range");
+    Slot& s = slots[dev];
+    if (s.word == nullptr) {
+      C10_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&s.word), 16, cudaHostAllocMapped | cudaHostAllocPortable));
+      C10_CUDA_CHECK(cudaEventCreateWithFlags(&s.event, cudaEventDisableTiming));
+    }
+    return s;
+  }
+  Slot* slot_ = nullptr;
+  bool host_failed_ = false;
+};
+
+// ------------------------------------------------------------------------------------------------ masked attention
+Tensor flags_u8(const Tensor& is_mem) {
+  const Tensor m = is_mem.scalar_type() == at::kByte || is_mem.scalar_type() == at::kBool ? is_mem : is_mem.to(at::kByte);
+  return m.stride(-1) == 1 ? m : m.contiguous();
+}
+
+std::tuple<Tensor, Tensor, Tensor> masked_fwd_cuda(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& is_mem,
+                                                   double scale, int64_t G) {
+  require_cuda(q_); require_cuda(k_); require_cuda(v_); require_cuda(is_mem);
+  const auto B = q_.size(0), H = q_.size(1), Lq = q_.size(2), D = q_.size(3), Lk = k_.size(2);
+  for (const Tensor* t : {&k_, &v_})
+    LMK_ASSERT(t->dim() == 4 && t->size(0) == B && t->size(1) == H && t->size(2) == Lk && t->size(3) == D, "k and v must be [B, H, Lk, D]");
+  LMK_ASSERT(q_.scalar_type() == k_.scalar_type() && q_.scalar_type() == v_.scalar_type(), "All tensors must have the same type");
+  LMK_ASSERT(is_mem.dim() == 2 && is_mem.size(0) == B && is_mem.size(1) == Lk, "is_mem must hold one flag per (batch row, key)");
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = last_dim_dense(q_), k = last_dim_dense(k_), v = last_dim_dense(v_), m = flags_u8(is_mem);
+  Tensor o = empty_like_dtype({B, H, Lq, D}, q), R = empty_f32({B * H, Lq}, q), A = empty_f32({B * H, G, Lq}, q);
+  check(lib.lmk_attn_mask_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), (const uint8_t*)m.data_ptr(), m.stride(0), o.data_ptr(),
+                              R.data_ptr<float>(), A.data_ptr<float>(), B, H, Lq, Lk, D, S3(q).v, S3(k).v, S3(v).v, G,
+                              (float)scale, dtype_code(q), stream_of(q)),
+        "lmk_attn_mask_fwd");
+  return {o, R, A};
+}
+
+std::tuple<Tensor, Tensor, Tensor> masked_bwd_cuda(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& is_mem,
+                                                   const Tensor& o_, const Tensor& do_, const Tensor& R, const Tensor& A,
+                                                   double scale, int64_t G) {
+  const auto B = q_.size(0), H = q_.size(1), Lq = q_.size(2), D = q_.size(3), Lk = k_.size(2);
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = last_dim_dense(q_), k = last_dim_dense(k_), v = last_dim_dense(v_), m = flags_u8(is_mem), o = o_.contiguous();
+  Tensor dO = do_.contiguous();
+  if (dO.scalar_type() != q.scalar_type()) dO = dO.to(q.scalar_type());
+  Tensor dq = empty_like_dtype({B, H, Lq, D}, q), dk = empty_like_dtype({B, H, Lk, D}, q), dv = empty_like_dtype({B, H, Lk, D}, q);
+  const size_t need = std::max<size_t>(lib.lmk_attn_mask_bwd_workspace(B, H, Lq, G), 256);
+  Tensor ws = at::empty({(int64_t)need}, q.options().requires_grad(false).dtype(at::kByte));
+  check(lib.lmk_attn_mask_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), (const uint8_t*)m.data_ptr(), m.stride(0), o.data_ptr(),
+                              dO.data_ptr(), R.data_ptr<float>(), A.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                              ws.data_ptr(), need, B, H, Lq, Lk, D, S3(q).v, S3(k).v, S3(v).v, G, (float)scale,
+                              dtype_code(q), stream_of(q)),
+        "lmk_attn_mask_bwd");
+  return {dq, dk, dv};
+}
+
+using MaskedFwdSig = std::tuple<Tensor, Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, const Tensor&, double, int64_t);
+using MaskedBwdSig = std::tuple<Tensor, Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&,
+                                                        const Tensor&, const Tensor&, const Tensor&, double, int64_t);
+const c10::TypedOperatorHandle<MaskedFwdSig>& masked_fwd_op() {
+  static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("lmk::masked_attention_fwd", "").typed<MaskedFwdSig>();
+  return op;
+}
+const c10::TypedOperatorHandle<MaskedBwdSig>& masked_bwd_op() {
+  static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("lmk::masked_attention_bwd", "").typed<MaskedBwdSig>();
+  return op;
+}
+
+struct MaskedLandmark : public torch::autograd::Function<MaskedLandmark> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& is_mem,
+                               double scale, int64_t G) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    auto [o, R, A] = masked_fwd_op().call(q, k, v, is_mem, scale, G);
+    ctx->save_for_backward({q, k, v, is_mem, o, R, A});
+    ctx->mark_non_differentiable({R, A});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["groups"] = G;
+    return {o, R, A};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    auto s = ctx->get_saved_variables();
+    auto [dq, dk, dv] = masked_bwd_op().call(s[0], s[1], s[2], s[3], s[4], grads[0], s[5], s[6],
+                                             ctx->saved_data["scale"].toDouble(), ctx->saved_data["groups"].toInt());
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+std::tuple<Tensor, Tensor, Tensor> masked_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& is_mem,
+                                                       double scale, int64_t G) {
+  if (!needs_grad({q, k, v})) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return masked_fwd_op().call(q, k, v, is_mem, scale, G);
+  }
+  auto r = MaskedLandmark::apply(q, k, v, is_mem, scale, G);
+  return {r[0], r[1], r[2]};
+}
+
+// ------------------------------------------------------------------------------------------------ rotary
+std::tuple<Tensor, Tensor> rotary_launch(const Tensor& q_, const Tensor& k_, const Tensor& cos, const Tensor& sin, int64_t pos0,
+                                         int64_t mode, bool inverse) {
+  for (const Tensor* t : {&q_, &k_, &cos, &sin}) require_cuda(*t);
+  const auto B = q_.size(0), H = q_.size(1), T = q_.size(2), D = q_.size(3);
+  LMK_ASSERT(q_.sizes() == k_.sizes() && q_.scalar_type() == k_.scalar_type() && q_.scalar_type() == cos.scalar_type() &&
+             q_.scalar_type() == sin.scalar_type(), "rotary: q, k and the tables must agree in shape and type");
+  LMK_ASSERT(cos.is_contiguous() && sin.is_contiguous() && cos.size(1) == D, "rotary: tables must be dense [n_pos, D]");
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = last_dim_dense(q_), k = last_dim_dense(k_);
+  Tensor qo = empty_like_dtype({B, H, T, D}, q), ko = empty_like_dtype({B, H, T, D}, q);
+  check(lib.lmk_rotary_apply(q.data_ptr(), k.data_ptr(), S3(q).v, S3(k).v, cos.data_ptr(), sin.data_ptr(), cos.size(0), pos0,
+                             mode, inverse, qo.data_ptr(), ko.data_ptr(), B, H, T, D, dtype_code(q), stream_of(q)),
+        "lmk_rotary_apply");
+  return {qo, ko};
+}
+
+struct RotaryPair : public torch::autograd::Function<RotaryPair> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin,
+                               int64_t pos0, int64_t mode) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    ctx->save_for_backward({cos, sin});
+    ctx->saved_data["pos0"] = pos0;
+    ctx->saved_data["mode"] = mode;
+    auto [qo, ko] = rotary_launch(q, k, cos, sin, pos0, mode, false);
+    return {qo, ko};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    if (!g[0].defined()) g[0] = at::zeros_like(g[1]);
+    if (!g[1].defined()) g[1] = at::zeros_like(g[0]);
+    auto [dq, dk] = rotary_launch(g[0], g[1], s[0], s[1], ctx->saved_data["pos0"].toInt(), ctx->saved_data["mode"].toInt(), true);
+    return {dq, dk, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+std::tuple<Tensor, Tensor> rotary_apply(const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin, int64_t pos0,
+                                        int64_t mode) {
+  if (!needs_grad({q, k})) return rotary_launch(q, k, cos, sin, pos0, mode, false);
+  auto r = RotaryPair::apply(q, k, cos, sin, pos0, mode);
+  return {r[0], r[1]};
+}
+
+// ------------------------------------------------------------------------------------------------ grouped softmax
+// byte mask with element strides of the [B, H, Lq, Lk] scores (0 where broadcast)
+struct Mask {
+  Tensor keep;
+  const uint8_t* ptr = nullptr;
+  int64_t st[4] = {0, 0, 0, 0};
+  Mask(const Tensor& m, at::IntArrayRef shape) {
+    if (!m.defined()) return;
+    keep = m.scalar_type() == at::kBool ? m : m.ne(0);          // the kernels read bit 0 of every byte
+    ptr = reinterpret_cast<const uint8_t*>(keep.data_ptr());
+    const int64_t off = 4 - keep.dim();
+    LMK_ASSERT(off >= 0, "mask has more than four dimensions");
+    for (int64_t i = 0; i < keep.dim(); ++i) {
+      const int64_t n = keep.size(i), want = shape[off + i];
+      LMK_ASSERT(n == want || n == 1, "mask does not broadcast to the scores");
+      st[off + i] = n == 1 ? 0 : keep.stride(i);
+    }
+  }
+  const int64_t* strides() const { return ptr ? st : nullptr; }
+};
+
+struct GroupedSoftmax : public torch::autograd::Function<GroupedSoftmax> {
+  static std::tuple<Tensor, Tensor> run(const Tensor& x, const Tensor& is_mem, const Tensor& last, const Tensor& hidden, bool guards,
+                                        int64_t max_groups, int64_t max_mem_cnt) {
+    const auto B = x.size(0), H = x.size(1), Lq = x.size(2), Lk = x.size(3);
+    Tensor probs = empty_f32({B, H, Lq, Lk}, x), gp;
+    if (max_mem_cnt) gp = empty_f32({B, H, Lq, max_mem_cnt}, x);
+    Mask m(is_mem, x.sizes()), l(last, x.sizes()), h(hidden, x.sizes());
+    check(lib.lmk_grouped_softmax_fwd(x.data_ptr(), S3(x).v, m.ptr, m.strides(), l.ptr, l.strides(), h.ptr, h.strides(),
+                                      probs.data_ptr<float>(), max_mem_cnt ? gp.data_ptr<float>() : nullptr, max_mem_cnt, B, H,
+                                      Lq, Lk, dtype_code(x), guards, max_groups, stream_of(x)),
+          "lmk_grouped_softmax_fwd");
+    return {probs, gp};
+  }
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& is_mem, const Tensor& last,
+                               const std::optional<Tensor>& hidden, bool guards, int64_t max_groups, int64_t max_mem_cnt) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    auto [probs, gp] = run(x, is_mem, last, hidden.value_or(Tensor()), guards, max_groups, max_mem_cnt);
+    if (hidden) ctx->save_for_backward({x, is_mem, last, *hidden});
+    else ctx->save_for_backward({x, is_mem, last});
+    ctx->saved_data["guards"] = guards;
+    ctx->saved_data["groups"] = max_groups;
+    if (!gp.defined()) return {probs};
+    ctx->mark_non_differentiable({gp});
+    return {probs, gp};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    const Tensor& x = s[0];
+    const auto B = x.size(0), H = x.size(1), Lq = x.size(2), Lk = x.size(3);
+    c10::cuda::OptionalCUDAGuard guard(x.device());
+    Tensor gprobs = g[0].to(at::kFloat).contiguous(), gx = empty_f32({B, H, Lq, Lk}, x);
+    Mask m(s[1], x.sizes()), l(s[2], x.sizes()), h(s.size() > 3 ? s[3] : Tensor(), x.sizes());
+    check(lib.lmk_grouped_softmax_bwd(x.data_ptr(), S3(x).v, m.ptr, m.strides(), l.ptr, l.strides(), h.ptr, h.strides(),
+                                      gprobs.data_ptr<float>(), gx.data_ptr<float>(), B, H, Lq, Lk, dtype_code(x),
+                                      ctx->saved_data["guards"].toBool(), ctx->saved_data["groups"].toInt(), stream_of(x)),
+          "lmk_grouped_softmax_bwd");
+    return {gx.to(x.scalar_type()), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+std::tuple<Tensor, Tensor> grouped_softmax(const Tensor& x_, const Tensor& is_mem, const Tensor& last, const Tensor& hidden,
+                                           bool guards, int64_t max_groups, int64_t max_mem_cnt) {
+  require_cuda(x_); require_cuda(is_mem); require_cuda(last);
+  if (hidden.defined()) require_cuda(hidden);
+  TORCH_CHECK_VALUE(x_.dim() == 4, "expected scores of shape [B, H, Lq, Lk]");
+  c10::cuda::OptionalCUDAGuard guard(x_.device());
+  const Tensor x = last_dim_dense(x_);
+  if (!needs_grad({x})) return GroupedSoftmax::run(x, is_mem, last, hidden, guards, max_groups, max_mem_cnt);
+  auto r = GroupedSoftmax::apply(x, is_mem, last, hidden.defined() ? std::optional<Tensor>(hidden) : std::nullopt, guards,
+                                 max_groups, max_mem_cnt);
+  return {r[0], r.size() > 1 ? r[1] : Tensor()};
+}
+
+struct GroupedSoftmaxCausal : public torch::autograd::Function<GroupedSoftmaxCausal> {
+  static Tensor run(const Tensor& x, const Tensor& flags, int64_t max_groups) {
+    const auto B = x.size(0), H = x.size(1), Lq = x.size(2), Lk = x.size(3);
+    Tensor probs = empty_f32({B, H, Lq, Lk}, x);
+    check(lib.lmk_grouped_softmax_causal_fwd(x.data_ptr(), S3(x).v, (const uint8_t*)flags.data_ptr(), flags.stride(0),
+                                             probs.data_ptr<float>(), B, H, Lq, Lk, dtype_code(x), max_groups, stream_of(x)),
+          "lmk_grouped_softmax_causal_fwd");
+    return probs;
+  }
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& flags, int64_t max_groups) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    ctx->save_for_backward({x, flags});
+    ctx->saved_data["groups"] = max_groups;
+    return run(x, flags, max_groups);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &flags = s[1];
+    const auto B = x.size(0), H = x.size(1), Lq = x.size(2), Lk = x.size(3);
+    c10::cuda::OptionalCUDAGuard guard(x.device());
+    Tensor gprobs = g[0].to(at::kFloat).contiguous(), gx = empty_f32({B, H, Lq, Lk}, x);
+    check(lib.lmk_grouped_softmax_causal_bwd(x.data_ptr(), S3(x).v, (const uint8_t*)flags.data_ptr(), flags.stride(0),
+                                             gprobs.data_ptr<float>(), gx.data_ptr<float>(), B, H, Lq, Lk, dtype_code(x),
+                                             ctx->saved_data["groups"].toInt(), stream_of(x)),
+          "lmk_grouped_softmax_causal_bwd");
+    return {gx.to(x.scalar_type()), Tensor(), Tensor()};
+  }
+};
+
+Tensor grouped_softmax_causal(const Tensor& x_, const Tensor& is_mem_row, int64_t max_groups) {
+  require_cuda(x_); require_cuda(is_mem_row);
+  c10::cuda::OptionalCUDAGuard guard(x_.device());
+  const Tensor x = last_dim_dense(x_);
+  Tensor flags = is_mem_row.scalar_type() == at::kBool ? is_mem_row : is_mem_row.ne(0);
+  if (flags.stride(-1) != 1) flags = flags.contiguous();
+  if (!needs_grad({x})) return GroupedSoftmaxCausal::run(x, flags, max_groups);
+  return GroupedSoftmaxCausal::apply(x, flags, max_groups);
+}
+
+// ------------------------------------------------------------------------------------------------ Python entry points
+const Tensor& tensor_arg(PyObject* o, const char* name) {
+  if (!THPVariable_Check(o)) {
+    PyErr_Format(PyExc_TypeError, "%s must be a tensor", name);
+    throw python_error();
+  }
+  return THPVariable_Unpack(o);
+}
+Tensor opt_tensor_arg(PyObject* o, const char* name) { return o == Py_None ? Tensor() : tensor_arg(o, name); }
+int64_t int_arg(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+double float_arg(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+void need_args(Py_ssize_t n, Py_ssize_t want) {
+  if (n != want) {
+    PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
+    throw python_error();
+  }
+}
+PyObject* wrap_opt(const Tensor& t) {
+  if (!t.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(t);
+}
+template <typename... Ts> PyObject* wrap_tuple(const Ts&... ts) {
+  PyObject* out = PyTuple_New(sizeof...(ts));
+  if (!out) throw python_error();
+  Py_ssize_t i = 0;
+  (PyTuple_SET_ITEM(out, i++, wrap_opt(ts)), ...);
+  return out;
+}
+
+PyObject* py_init(PyObject*, PyObject* arg) {
+  HANDLE_TH_ERRORS
+  const char* path = PyUnicode_AsUTF8(arg);
+  if (!path) throw python_error();
+  void* h = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+  TORCH_CHECK(h != nullptr, "cannot load ", path, ": ", dlerror());
+#define X(name)                                                             \
+  lib.name = reinterpret_cast<decltype(lib.name)>(dlsym(h, #name));         \
+  TORCH_CHECK(lib.name != nullptr, path, " does not export " #name);
+  LMK_FUNCS(X)
+#undef X
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// fused_attention(q, k, v, is_mem | None, scale, block, path)
+PyObject* py_fused_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 7);
+  const Tensor &q = tensor_arg(a[0], "q"), &k = tensor_arg(a[1], "k"), &v = tensor_arg(a[2], "v");
+  const double scale = float_arg(a[4]);
+  const int64_t block = int_arg(a[5]), path = int_arg(a[6]);
+  std::optional<RegularCheck> mask;
+  if (a[3] != Py_None) mask.emplace(tensor_arg(a[3], "is_mem"), block);
+  const int64_t history = k.size(-2) - q.size(-2);
+  LMK_ASSERT(history % block == 0, "key history must be whole blocks");
+  Tensor o = fused_attention(q, k, v, history / block, scale, block, path);
+  if (mask) LMK_ASSERT(!mask->failed(), "is_mem must mark the last token of every block");
+  return THPVariable_Wrap(std::move(o));
+  END_HANDLE_TH_ERRORS
+}
+
+// check_regular(is_mem, block): the reference's assertion on the landmark mask (flash_landmark_attention.py:393-394)
+PyObject* py_check_regular(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 2);
+  const Tensor& m = tensor_arg(a[0], "is_mem");
+  c10::cuda::OptionalCUDAGuard guard;
+  if (m.is_cuda()) guard.set_device(m.device());
+  LMK_ASSERT(!RegularCheck(m, int_arg(a[1])).failed(), "is_mem must mark the last token of every block");
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// masked_attention(q, k, v, is_mem, scale, max_groups) -> (o, R, A)
+PyObject* py_masked_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 6);
+  auto [o, R, A] = masked_fwd_autograd(tensor_arg(a[0], "q"), tensor_arg(a[1], "k"), tensor_arg(a[2], "v"),
+                                       tensor_arg(a[3], "is_mem"), float_arg(a[4]), int_arg(a[5]));
+  return wrap_tuple(o, R, A);
+  END_HANDLE_TH_ERRORS
+}
+
+// rotary_apply(q, k, cos, sin, pos0, mode)
+PyObject* py_rotary_apply(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 6);
+  auto [q, k] = rotary_apply(tensor_arg(a[0], "q"), tensor_arg(a[1], "k"), tensor_arg(a[2], "cos"), tensor_arg(a[3], "sin"),
+                             int_arg(a[4]), int_arg(a[5]));
+  return wrap_tuple(q, k);
+  END_HANDLE_TH_ERRORS
+}
+
+// grouped_softmax(x, is_mem, last, hidden | None, guards, max_groups, max_mem_cnt) -> (probs, group_prob | None)
+PyObject* py_grouped_softmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 7);
+  auto [p, gp] = grouped_softmax(tensor_arg(a[0], "x"), tensor_arg(a[1], "is_mem"), tensor_arg(a[2], "last"),
+                                 opt_tensor_arg(a[3], "hidden"), int_arg(a[4]) != 0, int_arg(a[5]), int_arg(a[6]));
+  return wrap_tuple(p, gp);
+  END_HANDLE_TH_ERRORS
+}
+
+// grouped_softmax_causal(x, is_mem_row, max_groups)
+PyObject* py_grouped_softmax_causal(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 3);
+  return THPVariable_Wrap(grouped_softmax_causal(tensor_arg(a[0], "x"), tensor_arg(a[1], "is_mem_row"), int_arg(a[2])));
+  END_HANDLE_TH_ERRORS
+}
+
+#define FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
+                         FAST("fused_attention", py_fused_attention),
+                         FAST("check_regular", py_check_regular),
+                         FAST("masked_attention", py_masked_attention),
+                         FAST("rotary_apply", py_rotary_apply),
+                         FAST("grouped_softmax", py_grouped_softmax),
+                         FAST("grouped_softmax_causal", py_grouped_softmax_causal),
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_lmk_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+TORCH_LIBRARY(lmk, m) {
+  m.def("masked_attention_fwd(Tensor q, Tensor k, Tensor v, Tensor is_mem, float sm_scale, int max_groups) -> (Tensor, Tensor, Tensor)");
+  m.def("masked_attention_bwd(Tensor q, Tensor k, Tensor v, Tensor is_mem, Tensor o, Tensor do, Tensor R, Tensor A, "
+        "float sm_scale, int max_groups) -> (Tensor, Tensor, Tensor)");
+}
+TORCH_LIBRARY_IMPL(lmk, CUDA, m) {
+  m.impl("masked_attention_fwd", masked_fwd_cuda);
+  m.impl("masked_attention_bwd", masked_bwd_cuda);
+}
+TORCH_LIBRARY_IMPL(lmk, Autograd, m) { m.impl("masked_attention_fwd", masked_fwd_autograd); }
+
+PyMODINIT_FUNC PyInit__lmk_host(void) { return PyModule_Create(&module); }

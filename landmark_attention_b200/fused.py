@@ -9,55 +9,15 @@ import torch
 from . import _lib as L
 
 
-class FusedLandmarkAttention(torch.autograd.Function):
-    """Mirrors FusedLandmarkAttention (flash_landmark_attention.py:308-389): forward keeps q, k, v, o and the
-    softmax statistics L, M; backward recomputes the probabilities."""
+class FusedLandmarkAttention:
+    """The differentiable call behind `fused_landmark_attention` (FusedLandmarkAttention, flash_landmark_attention.py:308-389):
+    forward keeps q, k, v, o and the softmax statistics L, M; backward recomputes the probabilities.  The autograd node
+    itself is native (csrc/host_torch.cpp)."""
 
     @staticmethod
-    def forward(ctx, q, k, v, n_prefix_q, sm_scale, block_size, path=L.PATH_AUTO):
-        L.require_cuda(q, k, v)
-        batch, nheads, seqlen_q, d = q.shape
-        seqlen_k = k.shape[2]
-        assert k.shape == (batch, nheads, seqlen_k, d)
-        assert v.shape == (batch, nheads, seqlen_k, d)
-        assert d <= 128, 'FlashAttention only support head dimensions up to 128'
-        assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
-        assert seqlen_k - seqlen_q == n_prefix_q * block_size
-        q, k, v = [t if t.stride(3) == 1 else t.contiguous() for t in (q, k, v)]
-        o = torch.empty((batch, nheads, seqlen_q, d), device=q.device, dtype=q.dtype)
-        lse_l = torch.empty((batch * nheads, seqlen_q), device=q.device, dtype=torch.float32)
-        lse_m = torch.empty((batch * nheads, seqlen_q), device=q.device, dtype=torch.float32)
-        rc = L.lib().lmk_attn_fwd(L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(o), L.ptr(lse_l), L.ptr(lse_m),
-                                  batch, nheads, seqlen_q, seqlen_k, d, L.strides3(q), L.strides3(k), L.strides3(v),
-                                  block_size, float(sm_scale), L.dtype_code(q), path, L.stream_ptr(q.device))
-        L.check(rc, "lmk_attn_fwd")
-        ctx.save_for_backward(q, k, v, o, lse_l, lse_m)
-        ctx.sm_scale, ctx.block, ctx.path = sm_scale, block_size, path
-        return o
-
-    @staticmethod
-    def backward(ctx, do):
-        q, k, v, o, lse_l, lse_m = ctx.saved_tensors
-        block = ctx.block
-        assert q.shape[2] % block == 0, "Backward supported only for full blocks"
-        assert k.shape[2] % block == 0, "Backward supported only for full blocks"
-        batch, nheads, seqlen_q, d = q.shape
-        seqlen_k = k.shape[2]
-        do = do.contiguous()
-        if do.dtype != q.dtype:
-            do = do.to(q.dtype)
-        dq = torch.empty((batch, nheads, seqlen_q, d), device=q.device, dtype=q.dtype)
-        dk = torch.empty((batch, nheads, seqlen_k, d), device=q.device, dtype=q.dtype)
-        dv = torch.empty((batch, nheads, seqlen_k, d), device=q.device, dtype=q.dtype)
-        code = L.dtype_code(q)
-        need = L.lib().lmk_attn_bwd_workspace(batch, nheads, seqlen_q, seqlen_k, d, block, code, ctx.path)
-        ws = torch.empty(max(int(need), 256), device=q.device, dtype=torch.uint8)
-        rc = L.lib().lmk_attn_bwd(L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(o), L.ptr(do), L.ptr(lse_l), L.ptr(lse_m),
-                                  L.ptr(dq), L.ptr(dk), L.ptr(dv), L.ptr(ws), ws.numel(),
-                                  batch, nheads, seqlen_q, seqlen_k, d, L.strides3(q), L.strides3(k), L.strides3(v),
-                                  block, float(ctx.sm_scale), code, ctx.path, L.stream_ptr(q.device))
-        L.check(rc, "lmk_attn_bwd")
-        return dq, dk, dv, None, None, None, None
+    def apply(q, k, v, n_prefix_q, sm_scale, block_size, path=L.PATH_AUTO):
+        assert k.shape[-2] - q.shape[-2] == n_prefix_q * block_size
+        return L.host().fused_attention(q, k, v, None, sm_scale, block_size, path)
 
 
 def fused_landmark_attention(q, k, v, is_mem=None, sm_scale=None, block_size=64, path=L.PATH_AUTO):
@@ -67,12 +27,8 @@ def fused_landmark_attention(q, k, v, is_mem=None, sm_scale=None, block_size=64,
     `is_mem` may be None (fast path: no mask is read and the host is not synchronised); when given it must be the
     regular pattern over the keys, as the reference asserts (flash_landmark_attention.py:393-394).
     """
-    if is_mem is not None:
-        expected_is_mem = torch.arange(0, is_mem.shape[-1], device=is_mem.device) % block_size == (block_size - 1)
-        assert (is_mem == expected_is_mem).all()
     n_history_kv = k.shape[-2] - q.shape[-2]
     assert n_history_kv % block_size == 0
-    n_history_blocks = n_history_kv // block_size
     if sm_scale is None:
         sm_scale = 1.0 / math.sqrt(q.size(-1))
     D = q.shape[-1]
@@ -82,12 +38,14 @@ def fused_landmark_attention(q, k, v, is_mem=None, sm_scale=None, block_size=64,
         # so causality hides the extra keys and the extra query rows are dropped again
         extra = -q.shape[2] % 128
         if _tensor_core_route(q.shape[0], q.shape[1], q.shape[2] + extra, k.shape[2] + extra, block_size, q.dtype):
+            _check_mask(is_mem, block_size)
             qp, kp, vp = [torch.nn.functional.pad(t, (0, 0, 0, extra)) for t in (q, k, v)]
             return fused_landmark_attention(qp, kp, vp, None, sm_scale, block_size, path)[:, :, :q.shape[2]]
     if (path == L.PATH_AUTO and D < 128 and D % 8 == 0 and q.is_cuda and q.dtype in (torch.bfloat16, torch.float16)
             and _tensor_core_route(q.shape[0], q.shape[1], q.shape[2], k.shape[2], block_size, q.dtype)):
         # head dims below 128: zero columns change neither q k^T nor the real columns of p v, and the tensor-core
         # kernels at twice the work beat the general kernels by an order of magnitude
+        _check_mask(is_mem, block_size)
         pad = (0, 128 - D)
         qp, kp, vp = [torch.nn.functional.pad(t, pad) for t in (q, k, v)]
         return fused_landmark_attention(qp, kp, vp, None, sm_scale, block_size, path)[..., :D]
@@ -98,9 +56,15 @@ def fused_landmark_attention(q, k, v, is_mem=None, sm_scale=None, block_size=64,
         Lk = k.shape[2]
         groups = max(Lk // block_size, 1)          # landmarks in front of any query
         if groups <= 64 and sm_scale > 0 and masked_attention_supported(q, k, groups):
+            _check_mask(is_mem, block_size)
             return landmark_attention_masked(q, k, v, _regular_flags(q.shape[0], Lk, block_size, q.device), sm_scale,
                                              groups)
-    return FusedLandmarkAttention.apply(q, k, v, n_history_blocks, sm_scale, block_size, path)
+    return L.host().fused_attention(q, k, v, is_mem, sm_scale, block_size, path)
+
+
+def _check_mask(is_mem, block_size):
+    if is_mem is not None:
+        L.host().check_regular(is_mem, block_size)
 
 
 def _tensor_core_route(B, H, Lq, Lk, block_size, dtype):

@@ -11,101 +11,7 @@ import torch
 from . import _lib as L
 
 
-def _as_u8(mask):
-    if mask is None:
-        return None
-    if mask.dtype == torch.bool:
-        return mask.view(torch.uint8) if mask.is_contiguous() or mask.dim() == 0 else mask.to(torch.uint8)
-    return (mask != 0).to(torch.uint8)        # the kernels read bit 0 of every byte
-
-
-def _prep(x, is_mem, last, hidden):
-    if x.dim() != 4:
-        raise ValueError("expected scores of shape [B, H, Lq, Lk]")
-    if x.stride(3) != 1:
-        x = x.contiguous()
-    shape = x.shape
-    masks = []
-    for m in (is_mem, last, hidden):
-        if m is None:
-            masks.append((None, None))
-            continue
-        while m.dim() < 4:
-            m = m.unsqueeze(0)
-        m8 = _as_u8(m)
-        m8, st = L.strides4_broadcast(m8, shape)
-        masks.append((m8, st))
-    return x, masks
-
-
-class _GroupedSoftmax(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, is_mem, last, hidden, guards, max_groups, max_mem_cnt):
-        L.require_cuda(x, is_mem, last, hidden)
-        x, masks = _prep(x, is_mem, last, hidden)
-        B, H, Lq, Lk = x.shape
-        probs = torch.empty((B, H, Lq, Lk), device=x.device, dtype=torch.float32)
-        gp = torch.empty((B, H, Lq, max_mem_cnt), device=x.device, dtype=torch.float32) if max_mem_cnt else None
-        (m8, ms), (l8, ls), (h8, hs) = masks
-        rc = L.lib().lmk_grouped_softmax_fwd(L.ptr(x), L.strides3(x), L.ptr(m8), ms, L.ptr(l8), ls, L.ptr(h8), hs,
-                                             L.ptr(probs), L.ptr(gp), max_mem_cnt or 0, B, H, Lq, Lk,
-                                             L.dtype_code(x), int(guards), max_groups, L.stream_ptr(x.device))
-        L.check(rc, "lmk_grouped_softmax_fwd")
-        ctx.save_for_backward(x, is_mem, last, hidden if hidden is not None else torch.empty(0))
-        ctx.has_hidden = hidden is not None
-        ctx.guards, ctx.max_groups = guards, max_groups
-        if gp is not None:
-            ctx.mark_non_differentiable(gp)
-            return probs, gp
-        return probs, None
-
-    @staticmethod
-    def backward(ctx, gprobs, _ggp):
-        x, is_mem, last, hidden = ctx.saved_tensors
-        hidden = hidden if ctx.has_hidden else None
-        x, masks = _prep(x, is_mem, last, hidden)
-        B, H, Lq, Lk = x.shape
-        gprobs = gprobs.to(torch.float32).contiguous()
-        gx = torch.empty((B, H, Lq, Lk), device=x.device, dtype=torch.float32)
-        (m8, ms), (l8, ls), (h8, hs) = masks
-        rc = L.lib().lmk_grouped_softmax_bwd(L.ptr(x), L.strides3(x), L.ptr(m8), ms, L.ptr(l8), ls, L.ptr(h8), hs,
-                                             L.ptr(gprobs), L.ptr(gx), B, H, Lq, Lk, L.dtype_code(x),
-                                             int(ctx.guards), ctx.max_groups, L.stream_ptr(x.device))
-        L.check(rc, "lmk_grouped_softmax_bwd")
-        return gx.to(x.dtype), None, None, None, None, None, None
-
-
 _CAUSAL_MAX_KEYS = 4096      # rows the mask-free kernel takes (include/b200lmk.h, lmk_grouped_softmax_causal_fwd)
-
-
-class _GroupedSoftmaxCausal(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, is_mem_row, max_groups):
-        L.require_cuda(x, is_mem_row)
-        if x.stride(3) != 1:
-            x = x.contiguous()
-        B, H, Lq, Lk = x.shape
-        flags = _as_u8(is_mem_row)
-        flags = flags if flags.stride(-1) == 1 else flags.contiguous()
-        probs = torch.empty((B, H, Lq, Lk), device=x.device, dtype=torch.float32)
-        rc = L.lib().lmk_grouped_softmax_causal_fwd(L.ptr(x), L.strides3(x), L.ptr(flags), flags.stride(0), L.ptr(probs),
-                                                    B, H, Lq, Lk, L.dtype_code(x), max_groups, L.stream_ptr(x.device))
-        L.check(rc, "lmk_grouped_softmax_causal_fwd")
-        ctx.save_for_backward(x, flags)
-        ctx.max_groups = max_groups
-        return probs
-
-    @staticmethod
-    def backward(ctx, gprobs):
-        x, flags = ctx.saved_tensors
-        B, H, Lq, Lk = x.shape
-        gprobs = gprobs.to(torch.float32).contiguous()
-        gx = torch.empty((B, H, Lq, Lk), device=x.device, dtype=torch.float32)
-        rc = L.lib().lmk_grouped_softmax_causal_bwd(L.ptr(x), L.strides3(x), L.ptr(flags), flags.stride(0), L.ptr(gprobs),
-                                                    L.ptr(gx), B, H, Lq, Lk, L.dtype_code(x), ctx.max_groups,
-                                                    L.stream_ptr(x.device))
-        L.check(rc, "lmk_grouped_softmax_causal_bwd")
-        return gx.to(x.dtype), None, None
 
 
 def landmark_grouped_softmax_causal(x, is_mem_row, max_mem_cnt=None):
@@ -119,10 +25,10 @@ def landmark_grouped_softmax_causal(x, is_mem_row, max_mem_cnt=None):
         max_mem_cnt = min(2048, Lk + 1)
     max_groups = min(2048, max(int(max_mem_cnt), 2))
     if Lk <= _CAUSAL_MAX_KEYS and (Lk + 255) // 256 * 1280 * 4 + 64 * max_groups <= 96 * 1024:
-        return _GroupedSoftmaxCausal.apply(x, is_mem_row, max_groups)
+        return L.host().grouped_softmax_causal(x, is_mem_row, max_groups)
     hidden = torch.ones(Lq, Lk, dtype=torch.bool, device=x.device).triu(Lk - Lq + 1)
     mask, is_mem, last = prepare_landmark_masks(is_mem_row, hidden)
-    probs, _ = _GroupedSoftmax.apply(x.masked_fill(mask, float("-inf")), is_mem, last, mask, True, max_groups, 0)
+    probs, _ = L.host().grouped_softmax(x.masked_fill(mask, float("-inf")), is_mem, last, mask, True, max_groups, 0)
     return probs
 
 
@@ -139,7 +45,7 @@ def landmark_grouped_softmax(x, dim, is_mem, last_section_mask, max_groups=None)
     _check_dim(x, dim)
     if max_groups is None:
         max_groups = min(256, x.shape[-1] + 1)
-    probs, _ = _GroupedSoftmax.apply(x, is_mem, last_section_mask, None, False, max_groups, 0)
+    probs, _ = L.host().grouped_softmax(x, is_mem, last_section_mask, None, False, max_groups, 0)
     return probs
 
 
@@ -154,8 +60,8 @@ def landmark_grouped_softmax_lm(x, dim, is_mem, attn_mask, last_section_mask, re
     _check_dim(x, dim)
     max_groups = min(2048, max(int(max_mem_cnt), 2))
     drop = p_group_dropout is not None and p_group_dropout > 0
-    probs, gp = _GroupedSoftmax.apply(x, is_mem, last_section_mask, attn_mask, True, max_groups,
-                                      int(max_mem_cnt) if (return_group_prob or drop) else 0)
+    probs, gp = L.host().grouped_softmax(x, is_mem, last_section_mask, attn_mask, True, max_groups,
+                                         int(max_mem_cnt) if (return_group_prob or drop) else 0)
     if drop:
         p = float(p_group_dropout)
         B, H, Lq, Lk = probs.shape
