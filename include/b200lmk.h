@@ -378,6 +378,21 @@ int lmk_selected_attend(const void* q, const void* k_cache, const lmk_cache_desc
                         int n_pos, int rotary, const void* o_local, const float* R_local, int64_t local_rows, void* out,
                         int B, int H, int T, int D, float sm_scale, int dtype, void* stream);
 
+/* Token generation behind a block cache in one launch (llama/llama_mem.py:318-430, 447-474 for inputs that stay inside the
+ * unfinished block): rotate-half rotary of q and k_new at positions len .. len+T-1, landmark scores and the top_k selection per
+ * (head, token), attention over the selected blocks (keys rotated at their slot positions), the unfinished block's cached
+ * rows and the new tokens, and -- with append != 0 -- k_new / v_new stored un-rotated at rows len .. len+T-1 of the cache.
+ *   q, k_new, v_new [B,H,T,128] with element strides {batch, head, row}; caches likewise, len rows of which the first
+ *   len / block * block are whole blocks; 16-bit types; len % block + T <= block; the landmark is each block's last row.
+ *   out [B,H,T,128] dense.
+ */
+int lmk_decode_supported(int D, int block, int top_k, int len, int T, int dtype);
+int lmk_decode_attend(const void* q, const void* k_new, const void* v_new, const int64_t q_strides[3],
+                      const int64_t k_strides[3], const int64_t v_strides[3], void* k_cache, void* v_cache,
+                      const int64_t k_cache_strides[3], const int64_t v_cache_strides[3], int len, int append, int block,
+                      int top_k, const void* cos_table, const void* sin_table, int n_pos, void* out, int B, int H, int T,
+                      int D, float sm_scale, int dtype, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

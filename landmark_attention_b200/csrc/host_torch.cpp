@@ -11,6 +11,7 @@
 // the Python side has loaded (init()), so an override of the library's location holds here as well.
 #include <dlfcn.h>
 
+#include <cmath>
 #include <mutex>
 #include <optional>
 #include <string>
@@ -37,7 +38,8 @@ using torch::autograd::variable_list;
 #define LMK_FUNCS(X)                                                                                             \
   X(lmk_last_error) X(lmk_attn_fwd) X(lmk_attn_bwd_workspace) X(lmk_attn_bwd) X(lmk_attn_mask_fwd)               \
   X(lmk_attn_mask_bwd_workspace) X(lmk_attn_mask_bwd) X(lmk_grouped_softmax_fwd) X(lmk_grouped_softmax_bwd)      \
-  X(lmk_grouped_softmax_causal_fwd) X(lmk_grouped_softmax_causal_bwd) X(lmk_rotary_apply) X(lmk_mask_is_regular)
+  X(lmk_grouped_softmax_causal_fwd) X(lmk_grouped_softmax_causal_bwd) X(lmk_rotary_apply) X(lmk_mask_is_regular)        \
+  X(lmk_decode_supported) X(lmk_decode_attend)
 struct Lib {
 #define X(name) decltype(&::name) name = nullptr;
   LMK_FUNCS(X)
@@ -445,6 +447,43 @@ Tensor grouped_softmax_causal(const Tensor& x_, const Tensor& is_mem_row, int64_
   return GroupedSoftmaxCausal::apply(x, flags, max_groups);
 }
 
+// ------------------------------------------------------------------------------------------------ retrieval
+// rows of 16-byte vectors: dense features, strides that are multiples of 8 elements, aligned base
+Tensor vector_rows(const Tensor& t) {
+  const bool ok = t.stride(3) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && t.stride(2) % 8 == 0 &&
+                  (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  return ok ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+
+// One layer of token generation behind `len` cached tokens (lmk_decode_attend); undefined where the kernel does not take it.
+Tensor decode_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& kc, const Tensor& vc, int64_t len,
+                     bool append, int64_t block, int64_t top_k, const Tensor& cos, const Tensor& sin) {
+  const auto st = q_.scalar_type();
+  if (!q_.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || q_.dim() != 4 || kc.dim() != 4) return Tensor();
+  const auto B = q_.size(0), H = q_.size(1), T = q_.size(2), D = q_.size(3);
+  for (const Tensor* t : {&k_, &v_, &kc, &vc, &cos, &sin})
+    if (!t->is_cuda() || t->scalar_type() != st) return Tensor();
+  auto cache_ok = [&](const Tensor& t) {
+    return t.stride(3) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && t.stride(2) % 8 == 0 && t.size(0) == B &&
+           t.size(1) == H && t.size(3) == D && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  };
+  auto table_ok = [&](const Tensor& t) {
+    return t.is_contiguous() && t.dim() == 2 && t.size(1) == D && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  };
+  if (!cache_ok(kc) || !cache_ok(vc) || k_.sizes() != q_.sizes() || v_.sizes() != q_.sizes() || !table_ok(cos) ||
+      !table_ok(sin) || B * H > 65535 || kc.size(2) < len + (append ? T : 0) || vc.size(2) < len + (append ? T : 0) ||
+      !lib.lmk_decode_supported(D, block, top_k, len, T, dtype_code(q_)))
+    return Tensor();
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = vector_rows(q_), k = vector_rows(k_), v = vector_rows(v_);
+  Tensor out = empty_like_dtype({B, H, T, D}, q);
+  check(lib.lmk_decode_attend(q.data_ptr(), k.data_ptr(), v.data_ptr(), S3(q).v, S3(k).v, S3(v).v, kc.data_ptr(), vc.data_ptr(),
+                              S3(kc).v, S3(vc).v, len, append, block, top_k, cos.data_ptr(), sin.data_ptr(), cos.size(0),
+                              out.data_ptr(), B, H, T, D, 1.0 / std::sqrt((double)D), dtype_code(q), stream_of(q)),
+        "lmk_decode_attend");
+  return out;
+}
+
 // ------------------------------------------------------------------------------------------------ Python entry points
 const Tensor& tensor_arg(PyObject* o, const char* name) {
   if (!THPVariable_Check(o)) {
@@ -564,6 +603,16 @@ PyObject* py_grouped_softmax_causal(PyObject*, PyObject* const* a, Py_ssize_t n)
   END_HANDLE_TH_ERRORS
 }
 
+// decode_attend(q, k_new, v_new, k_cache, v_cache, len, append, block, top_k, cos, sin) -> out | None
+PyObject* py_decode_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 11);
+  return wrap_opt(decode_attend(tensor_arg(a[0], "q"), tensor_arg(a[1], "k_new"), tensor_arg(a[2], "v_new"),
+                                tensor_arg(a[3], "k_cache"), tensor_arg(a[4], "v_cache"), int_arg(a[5]), int_arg(a[6]) != 0,
+                                int_arg(a[7]), int_arg(a[8]), tensor_arg(a[9], "cos"), tensor_arg(a[10], "sin")));
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST("fused_attention", py_fused_attention),
@@ -572,6 +621,7 @@ PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST("rotary_apply", py_rotary_apply),
                          FAST("grouped_softmax", py_grouped_softmax),
                          FAST("grouped_softmax_causal", py_grouped_softmax_causal),
+                         FAST("decode_attend", py_decode_attend),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_lmk_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

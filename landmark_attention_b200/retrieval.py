@@ -274,7 +274,8 @@ def llama_retrieval_attention(q, k_new, v_new, past_k=None, past_v=None, mem_fre
       "max_over_tokens" = one selection per head from the softmax of the scores maximised over the chunk's tokens, the
       selected blocks prepended to the keys and the whole thing run through fused landmark attention (the reference's
       route with offload_cache_to_cpu, :369-377, 400-406, 445).
-    Three implementations of the default mode, same results within the 16-bit tolerances:
+    Tokens that stay inside the unfinished block (generation) run as one kernel (lmk_decode_attend) where tables are given.
+    Otherwise three implementations of the default mode, same results within the 16-bit tolerances:
       fused (default where it applies: 16-bit, D=128, no partial block in the cache): local keys through the
         tensor-core operator for arbitrary landmark positions, selected blocks read in place by one kernel that also
         merges the two parts -- no logits, probabilities or gathered copies in memory;
@@ -282,6 +283,11 @@ def llama_retrieval_attention(q, k_new, v_new, past_k=None, past_v=None, mem_fre
       materialize=True (what the reference does, :386-398): gathered [B,H,T,top_k*block,D] copies and matmuls.
     Returns (attn_output [B,H,T,D], new (past_k, past_v)).
     """
+    if (fused is None and materialize is None and not return_debug and aggregate is None and position_ids is None
+            and chunk_is_mem is None and cos is not None):
+        out = _decode(q, k_new, v_new, past_k, past_v, mem_freq + 1, cache_top_k, cos, sin, cache)
+        if out is not None:
+            return out
     if cache is not None:
         past_k, past_v = cache.views()
     if materialize is None:
@@ -398,6 +404,33 @@ def llama_retrieval_attention(q, k_new, v_new, past_k=None, past_v=None, mem_fre
     if return_debug:
         return out, new_cache(), dict(scores=scores, sel=sel, sel_k=sel_k, sel_v=sel_v, probs=probs)
     return out, new_cache()
+
+
+_DECODE_MAX_WHOLE_BLOCK_TOKENS = 16
+
+
+def _decode(q, k_new, v_new, past_k, past_v, block, cache_top_k, cos, sin, cache):
+    """llama_retrieval_attention for tokens that stay inside the unfinished block, as one launch (lmk_decode_attend); None
+    where that kernel does not apply.  Behind a cache of whole blocks it takes up to 16 tokens: more are cheaper as a chunk,
+    whose scores and local attention run on the tensor cores."""
+    C = past_k.shape[2] if cache is None else cache.length
+    T = q.shape[2]
+    inc = C % block
+    if T + inc > block or C < block or (inc == 0 and T > _DECODE_MAX_WHOLE_BLOCK_TOKENS):
+        return None
+    if cache is None:
+        kb, vb = past_k, past_v
+    else:
+        kb, vb = cache.k, cache.v
+        if C + T > kb.shape[2]:
+            raise ValueError(f"cache capacity {kb.shape[2]} exceeded ({C} + {T})")
+    out = L.host().decode_attend(q, k_new, v_new, kb, vb, C, cache is not None, block, min(cache_top_k, C // block), cos, sin)
+    if out is None:
+        return None
+    if cache is None:
+        return out, (torch.cat((past_k, k_new), dim=2), torch.cat((past_v, v_new), dim=2))
+    cache.length = C + T
+    return out, cache.views()
 
 
 class OffloadedLandmarkCache:
