@@ -393,6 +393,34 @@ int lmk_decode_attend(const void* q, const void* k_new, const void* v_new, const
                       int top_k, const void* cos_table, const void* sin_table, int n_pos, void* out, int B, int H, int T,
                       int D, float sm_scale, int dtype, void* stream);
 
+/* Block selection of lm_benchmark's cache (mem_cache.py:51-83) for at most 128 blocks, 16-bit types, D = 128, top_k <= 8: scores
+ * against landmark_keys (desc, the last "row" of a block), softmax over the blocks rounded to the data type, and per
+ * (head, token) the top_k picks in ascending logical age.  probs (fp32 [B,H,T,n_blocks]) and idx (int32 [B,H,T,top_k]) are
+ * each optional.  q dense [B,H,T,D].
+ */
+int lmk_block_select_supported(int D, int n_blocks, int top_k, int dtype);
+int lmk_block_select(const void* q, const void* landmark_keys, const lmk_cache_desc* desc, const void* cos_table,
+                     const void* sin_table, int n_pos, int rotary, float* probs, int32_t* idx, int B, int H, int T, int D,
+                     float sm_scale, int dtype, void* stream);
+
+/* The retrieved prefix of lm_benchmark's cache (mem_cache.py:85-109): logits att [B,H,T,P] of every query against the keys of
+ * its picks (rotated at their slot positions) followed by the tail rows (rotated at tail_pos, tail_pos + 1, ...), and the
+ * matching values v_out [B,H,T,P,D]; P = top_k * block + tail_len, both dense.  idx: pick i of token t of head h of batch row b
+ * at b * idx_strides[0] + h * idx_strides[1] + t * idx_strides[2] + i (a stride of 0 broadcasts); q dense.
+ */
+int lmk_prefix_gather_supported(int D, int block, int top_k, int T, int tail_len, int dtype);
+int lmk_prefix_gather(const void* q, const void* k_cache, const void* v_cache, const lmk_cache_desc* kdesc,
+                      const lmk_cache_desc* vdesc, const int32_t* idx, const int64_t idx_strides[3], const void* cos_table,
+                      const void* sin_table, int n_pos, int rotary, const void* tail_k, const void* tail_v,
+                      const int64_t tail_strides[3], int tail_len, int tail_pos, void* att, void* v_out, int B, int H, int T,
+                      int D, float sm_scale, int dtype, void* stream);
+
+/* y[b,h,t,:] += sum_{j < P} probs[b,h,t,j] v[b,h,t,j,:] (landmark.py:236-243): probabilities fp32 with row stride probs_ld, used
+ * rounded to the data type; v rows dense, v_strides {batch, head, token} in elements; y dense [B,H,T,D], updated in place.
+ */
+int lmk_prefix_pv(const float* probs, int64_t probs_ld, const void* v, const int64_t v_strides[3], void* y, int B, int H, int T,
+                  int P, int D, int dtype, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -92,6 +92,15 @@ PROTOTYPES = {
     "lmk_decode_attend": (c_int, [c_void_p] * 3 + [POINTER(c_int64)] * 3 + [c_void_p] * 2 + [POINTER(c_int64)] * 2 +
                           [c_int] * 4 + [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int,
                            c_void_p]),
+    "lmk_block_select_supported": (c_int, [c_int] * 4),
+    "lmk_block_select": (c_int, [c_void_p, c_void_p, POINTER(CacheDesc), c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
+                                 c_int, c_int, c_int, c_int, c_float, c_int, c_void_p]),
+    "lmk_prefix_gather_supported": (c_int, [c_int] * 6),
+    "lmk_prefix_gather": (c_int, [c_void_p, c_void_p, c_void_p, POINTER(CacheDesc), POINTER(CacheDesc), c_void_p,
+                                  POINTER(c_int64), c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, POINTER(c_int64),
+                                  c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p]),
+    "lmk_prefix_pv": (c_int, [c_void_p, c_int64, c_void_p, POINTER(c_int64), c_void_p, c_int, c_int, c_int, c_int, c_int,
+                              c_int, c_void_p]),
     "lmk_selected_pv": (c_int, [c_void_p, c_int64, c_int64, c_void_p, POINTER(CacheDesc), c_void_p, c_void_p, c_int,
                                 c_int, c_int, c_int, c_int, c_void_p]),
 }

@@ -39,7 +39,9 @@ using torch::autograd::variable_list;
   X(lmk_last_error) X(lmk_attn_fwd) X(lmk_attn_bwd_workspace) X(lmk_attn_bwd) X(lmk_attn_mask_fwd)               \
   X(lmk_attn_mask_bwd_workspace) X(lmk_attn_mask_bwd) X(lmk_grouped_softmax_fwd) X(lmk_grouped_softmax_bwd)      \
   X(lmk_grouped_softmax_causal_fwd) X(lmk_grouped_softmax_causal_bwd) X(lmk_rotary_apply) X(lmk_mask_is_regular)        \
-  X(lmk_decode_supported) X(lmk_decode_attend)
+  X(lmk_decode_supported) X(lmk_decode_attend) X(lmk_block_select) X(lmk_block_select_supported)                  \
+  X(lmk_prefix_gather) X(lmk_prefix_gather_supported) X(lmk_prefix_pv) X(lmk_landmark_scores)                     \
+  X(lmk_landmark_scores_workspace) X(lmk_topk_sorted)
 struct Lib {
 #define X(name) decltype(&::name) name = nullptr;
   LMK_FUNCS(X)
@@ -484,6 +486,104 @@ Tensor decode_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const
   return out;
 }
 
+lmk_cache_desc block_desc(const Tensor& t, bool block_before_head, int64_t n, int64_t ring_start, int64_t block, int64_t top_k) {
+  lmk_cache_desc d{};
+  d.stride_b = t.stride(0);
+  d.stride_h = t.stride(block_before_head ? 3 : 1);
+  d.stride_block = t.stride(block_before_head ? 1 : 2);
+  d.stride_row = t.stride(block_before_head ? 2 : 3);
+  d.n_blocks = n;
+  d.ring_start = ring_start;
+  d.block = block;
+  d.top_k = top_k;
+  return d;
+}
+
+// MemLMCacheStorage.retrieve_for_query with blocks in the cache (mem_cache.py:51-109): (att_prefix [B,H,T,P], values
+// [B,H,T,P,D]); undefined where the kernels do not take the problem.  kc, vc: the block buffers in either layout; lm: dense
+// landmark keys [B,H,capacity,D]; tail_k, tail_v [B,H,>=inc,D].  mode: 0 per token and head, 1 maximum over the
+// tokens, 2 over the heads.
+std::tuple<Tensor, Tensor> cache_retrieve(const Tensor& q_, const Tensor& kc, const Tensor& vc, const Tensor& lm, bool block_first,
+                                          int64_t n, int64_t ring_start, int64_t block, int64_t top_k, const Tensor& cos,
+                                          const Tensor& sin, int64_t mode, const Tensor& tail_k, const Tensor& tail_v, int64_t inc,
+                                          int64_t tail_pos) {
+  const auto st = q_.scalar_type();
+  const auto B = q_.size(0), H = q_.size(1), T = q_.size(2), D = q_.size(3);
+  if (!q_.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || B * H > 65535) return {};
+  for (const Tensor* t : {&kc, &vc, &lm, &cos, &sin, &tail_k, &tail_v})
+    if (!t->is_cuda() || t->scalar_type() != st || t->stride(-1) != 1 || (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15)) return {};
+  const int code = dtype_code(q_);
+  if (tail_k.strides() != tail_v.strides() || !lib.lmk_prefix_gather_supported(D, block, top_k, T, inc, code)) return {};
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = q_.contiguous();
+  void* stream = stream_of(q);
+  const float scale = 1.0 / std::sqrt((double)D);
+  const lmk_cache_desc kd = block_desc(kc, block_first, n, ring_start, block, top_k), vd = block_desc(vc, block_first, n, ring_start, block, top_k);
+  lmk_cache_desc ld{};
+  ld.stride_b = lm.stride(0);
+  ld.stride_h = lm.stride(1);
+  ld.stride_block = lm.stride(2);
+  ld.n_blocks = n;
+  ld.ring_start = ring_start;
+  ld.block = block;
+  ld.top_k = top_k;
+  const auto i32 = q.options().requires_grad(false).dtype(at::kInt);
+  const bool small = lib.lmk_block_select_supported(D, n, top_k, code);
+  Tensor idx, probs;
+  if (mode == 0 && small) idx = at::empty({B, H, T, top_k}, i32);
+  else probs = empty_f32({B, H, T, n}, q);
+  if (small) {
+    check(lib.lmk_block_select(q.data_ptr(), lm.data_ptr(), &ld, cos.data_ptr(), sin.data_ptr(), cos.size(0), LMK_ROTARY_INTERLEAVED,
+                               probs.defined() ? probs.data_ptr<float>() : nullptr, idx.defined() ? idx.data_ptr<int>() : nullptr,
+                               B, H, T, D, scale, code, stream),
+          "lmk_block_select");
+  } else {
+    const size_t need = lib.lmk_landmark_scores_workspace(B, H, T, D, n, code);
+    Tensor ws = need ? at::empty({(int64_t)need}, i32.dtype(at::kByte)) : Tensor();
+    check(lib.lmk_landmark_scores(q.data_ptr(), lm.data_ptr(), &ld, cos.data_ptr(), sin.data_ptr(), cos.size(0), LMK_ROTARY_INTERLEAVED,
+                                  probs.data_ptr<float>(), B, H, T, D, scale, 1, code, need ? ws.data_ptr() : nullptr, need, stream),
+          "lmk_landmark_scores");
+  }
+  int64_t is[3] = {H * T * top_k, T * top_k, top_k};
+  if (!idx.defined()) {
+    const float* s = probs.data_ptr<float>();
+    if (mode == 0) {
+      idx = at::empty({B, H, T, top_k}, i32);
+      check(lib.lmk_topk_sorted(s, idx.data_ptr<int>(), B * H * T, 1, n, 0, 1, 0, n, top_k, ring_start, stream), "lmk_topk_sorted");
+    } else if (mode == 1) {
+      idx = at::empty({B, H, 1, top_k}, i32);
+      check(lib.lmk_topk_sorted(s, idx.data_ptr<int>(), B * H, 1, T * n, 0, T, n, n, top_k, ring_start, stream), "lmk_topk_sorted");
+      is[0] = H * top_k, is[1] = top_k, is[2] = 0;
+    } else {
+      idx = at::empty({B, 1, T, top_k}, i32);
+      check(lib.lmk_topk_sorted(s, idx.data_ptr<int>(), B, T, H * T * n, n, H, T * n, n, top_k, ring_start, stream), "lmk_topk_sorted");
+      is[0] = T * top_k, is[1] = 0, is[2] = top_k;
+    }
+  }
+  const int64_t P = top_k * block + inc;
+  Tensor att = empty_like_dtype({B, H, T, P}, q), v = empty_like_dtype({B, H, T, P, D}, q);
+  check(lib.lmk_prefix_gather(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), &kd, &vd, idx.data_ptr<int>(), is, cos.data_ptr(), sin.data_ptr(),
+                              cos.size(0), LMK_ROTARY_INTERLEAVED, tail_k.data_ptr(), tail_v.data_ptr(), S3(tail_k).v, inc, tail_pos,
+                              att.data_ptr(), v.data_ptr(), B, H, T, D, scale, code, stream),
+        "lmk_prefix_gather");
+  return {att, v};
+}
+
+// y += probs[..., :P] @ v per token (lmk_prefix_pv); false where the kernel does not take the tensors
+bool prefix_pv(const Tensor& probs, const Tensor& v, const Tensor& y) {
+  const auto st = v.scalar_type();
+  const auto B = y.size(0), H = y.size(1), T = y.size(2), D = y.size(3), P = v.size(3);
+  if (!v.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || y.scalar_type() != st || D != 128 || P > 8192 || B * H > 65535 ||
+      P == 0 || !probs.is_contiguous() || !y.is_contiguous() || v.stride(4) != 1 || v.stride(3) != D || v.stride(0) % 8 ||
+      v.stride(1) % 8 || v.stride(2) % 8 || (reinterpret_cast<uintptr_t>(v.data_ptr()) & 15))
+    return false;
+  c10::cuda::OptionalCUDAGuard guard(v.device());
+  check(lib.lmk_prefix_pv(probs.data_ptr<float>(), probs.size(3), v.data_ptr(), S3(v).v, y.data_ptr(), B, H, T, P, D, dtype_code(v),
+                          stream_of(v)),
+        "lmk_prefix_pv");
+  return true;
+}
+
 // ------------------------------------------------------------------------------------------------ Python entry points
 const Tensor& tensor_arg(PyObject* o, const char* name) {
   if (!THPVariable_Check(o)) {
@@ -613,6 +713,27 @@ PyObject* py_decode_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// cache_retrieve(q, k, v, landmark keys, block_first, n, ring_start, block, top_k, cos, sin, mode, tail_k, tail_v, inc, tail_pos)
+// -> (att_prefix, values) | (None, None)
+PyObject* py_cache_retrieve(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 16);
+  auto [att, v] = cache_retrieve(tensor_arg(a[0], "q"), tensor_arg(a[1], "k_cache"), tensor_arg(a[2], "v_cache"),
+                                 tensor_arg(a[3], "landmark_keys"), int_arg(a[4]) != 0, int_arg(a[5]), int_arg(a[6]), int_arg(a[7]),
+                                 int_arg(a[8]), tensor_arg(a[9], "cos"), tensor_arg(a[10], "sin"), int_arg(a[11]),
+                                 tensor_arg(a[12], "tail_k"), tensor_arg(a[13], "tail_v"), int_arg(a[14]), int_arg(a[15]));
+  return wrap_tuple(att, v);
+  END_HANDLE_TH_ERRORS
+}
+
+// prefix_pv(probs, v, y) -> bool
+PyObject* py_prefix_pv(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 3);
+  return PyBool_FromLong(prefix_pv(tensor_arg(a[0], "probs"), tensor_arg(a[1], "v"), tensor_arg(a[2], "y")));
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST("fused_attention", py_fused_attention),
@@ -622,6 +743,8 @@ PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST("grouped_softmax", py_grouped_softmax),
                          FAST("grouped_softmax_causal", py_grouped_softmax_causal),
                          FAST("decode_attend", py_decode_attend),
+                         FAST("cache_retrieve", py_cache_retrieve),
+                         FAST("prefix_pv", py_prefix_pv),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_lmk_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

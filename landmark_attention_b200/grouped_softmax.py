@@ -123,6 +123,11 @@ def lm_landmark_attention(q, k, v, is_mem_row, sm_scale=None, max_groups=None, a
     # mask block + masked_fill + grouped softmax in one kernel, from the raw scores and the row flags
     probs = landmark_grouped_softmax_causal(att, is_mem_row, max_groups if max_groups is not None
                                             else min(2048, T + n_pre + 1))
+    if n_pre and not probs.requires_grad and cache_values['v'].dim() == v.dim() + 1 and not cache_values['v'].requires_grad:
+        # the retrieved values are read once, by one kernel, from the fp32 probabilities
+        y = torch.matmul(probs[..., n_pre:].to(v.dtype), v)
+        if L.host().prefix_pv(probs, cache_values['v'], y):
+            return y
     probs = probs.to(v.dtype)
     y = torch.matmul(probs[..., n_pre:], v)
     if n_pre:

@@ -111,6 +111,9 @@ class MemLMCacheStorage(nn.Module):
         scale = 1.0 / math.sqrt(hs)
         cos, sin = self._rotary(max(start_index + T, (top_k + 2) * blk) + 1, hs, q.dtype, q.device)
         inc = self.last_incomplete_len
+        fast = self._retrieve_native(q, cos, sin, inc, start_index)
+        if fast is not None:
+            return fast
         tail_pos = torch.arange(start_index - inc, start_index, device=q.device)
         tail_k = _rotate_interleaved(self.last_incomplete_k[:B, :, :inc], cos, sin, tail_pos)
         att_incomplete = (q @ tail_k.transpose(-2, -1)) * scale
@@ -135,25 +138,50 @@ class MemLMCacheStorage(nn.Module):
         is_mem_prefix = torch.cat((is_mem.view(B, -1), last_mem), dim=-1)
         return att_prefix, {'v': v_prefix, 'is_mem': is_mem_prefix}
 
+    _MODES = {"per_token_and_head": 0, "max_over_tokens": 1, "max_over_heads": 2}
+
+    def _retrieve_native(self, q, cos, sin, inc, start_index):
+        """retrieve_for_query in two or three launches (selection, then logits and values of the picks and the tail written in
+        place); None where those kernels do not apply."""
+        B, nh, T, hs = q.shape
+        blk, cap = self.block, self.capacity
+        mode = self._MODES.get(self.config.cache_selection_method)
+        if self.cache_size == 0 or self.config.cache_topk == 0 or mode is None or hs != 128 or torch.is_grad_enabled() and q.requires_grad:
+            return None
+        n = min(self.cache_size, cap)
+        top_k = min(self.config.cache_topk, n)
+        ring_start = self.cache_iter % n if self.cache_size >= cap else 0
+        att, v = L.host().cache_retrieve(q, self.cache_mem_k, self.cache_mem_v, self.cache_lm_k, self.layout == "reference", n,
+                                         ring_start, blk, top_k, cos, sin, mode, self.last_incomplete_k, self.last_incomplete_v,
+                                         inc, start_index - inc)
+        if att is None:
+            return None
+        is_mem = torch.zeros((B, top_k * blk + inc), dtype=torch.bool, device=q.device)
+        is_mem[:, blk - 1:top_k * blk:blk] = True
+        if inc:
+            is_mem[:, top_k * blk:] = self.last_incomplete_ismem[:B, :inc]
+        return att, {'v': v, 'is_mem': is_mem}
+
     def store_in_cache(self, keys, values_dict):
         """mem_cache.py:111-158: append whole blocks to the ring buffer, keep the unfinished tail aside."""
         B = keys.shape[0]
         blk, cap = self.block, self.capacity
         inc0 = self.last_incomplete_len
-        k = torch.cat((self.last_incomplete_k[:B, :, :inc0], keys), dim=-2)
-        v = torch.cat((self.last_incomplete_v[:B, :, :inc0], values_dict['v']), dim=-2)
-        is_mem = torch.cat((self.last_incomplete_ismem[:B, :inc0], values_dict['is_mem']), dim=-1)
+        k, v, is_mem = keys, values_dict['v'], values_dict['is_mem']
+        if inc0:
+            k = torch.cat((self.last_incomplete_k[:B, :, :inc0], k), dim=-2)
+            v = torch.cat((self.last_incomplete_v[:B, :, :inc0], v), dim=-2)
+            is_mem = torch.cat((self.last_incomplete_ismem[:B, :inc0], is_mem), dim=-1)
         _, nh, T, hs = k.shape
         inc = T % blk
         full = T - inc
-        self.last_incomplete_k[:B, :, :inc].copy_(k[:, :, full:])
-        self.last_incomplete_v[:B, :, :inc].copy_(v[:, :, full:])
-        self.last_incomplete_ismem[:B, :inc].copy_(is_mem[:, full:])
+        if inc:
+            self.last_incomplete_k[:B, :, :inc].copy_(k[:, :, full:])
+            self.last_incomplete_v[:B, :, :inc].copy_(v[:, :, full:])
+            self.last_incomplete_ismem[:B, :inc].copy_(is_mem[:, full:])
         self.last_incomplete_len = inc
-        im = is_mem[:, :full].view(B, -1, blk)
-        assert im[..., -1].all()
-        assert not im[..., :-1].any()
-        added = im.shape[1]
+        L.host().check_regular(is_mem[:, :full], blk)      # every block ends in its only landmark, or AssertionError
+        added = full // blk
         dropped = max(0, added - cap)           # more blocks than the ring holds: only the newest `cap` are kept
         self.cache_iter = (self.cache_iter + dropped) % cap
         self.cache_size += dropped
