@@ -55,14 +55,14 @@ void fill(AttnParams& p, const void* q, const void* k, const void* v, int B, int
   }
 }
 
-// 1 = general, 2 = tcgen05, <0 = error.  LMK_PATH_AUTO takes the tcgen05 kernels only when the shape AND the operands
-// (alignment, strides) qualify, and the general kernels otherwise; an explicit LMK_PATH_TCGEN05 request that cannot be
-// met is an error.
+// 1 = general, 2 = tcgen05, <0 = error.  LMK_PATH_AUTO takes the tcgen05 kernels when the problem (16-bit type, block 64) AND
+// the operands (alignment, strides) qualify, and the general kernels otherwise; an explicit LMK_PATH_TCGEN05 request asks
+// for whole tiles of head dim 128 and is an error where that cannot be met.
 int pick_path(int path, const AttnParams& p, int dtype, bool backward) {
   // the tcgen05 kernels take maxima on raw dot products, which needs a positive softmax scale
-  const bool shape_ok = attn_sm100_supported(p.B, p.H, p.Lq, p.Lk, p.D, p.block, dtype) && p.scale > 0.f;
-  const bool fast = shape_ok && attn_sm100_operands_ok(p, backward);
+  const bool fast = attn_sm100_takes(p.B, p.H, p.Lq, p.Lk, p.D, p.block, dtype) && p.scale > 0.f && attn_sm100_operands_ok(p, backward);
   if (path == LMK_PATH_TCGEN05) {
+    const bool shape_ok = attn_sm100_supported(p.B, p.H, p.Lq, p.Lk, p.D, p.block, dtype) && p.scale > 0.f;
     if (!shape_ok)
       return fail(LMK_ERR_UNSUPPORTED,
                   "tcgen05 path needs bf16/fp16, D=128, block=64, Lq a multiple of 128 and a positive scale (got "
@@ -149,13 +149,13 @@ extern "C" int lmk_attn_bwd(const void* q, const void* k, const void* v, const v
   int rc = check_common(q, k, v, B, H, Lq, Lk, D, q_strides, k_strides, v_strides, block, dtype, path);
   if (rc != LMK_OK) return rc;
   LMK_CHECK_ARG(o && dO && L && M && dQ && dK && dV, "attn_bwd: null tensor pointer");
-  LMK_CHECK_ARG(Lq % block == 0 && Lk % block == 0, "Backward supported only for full blocks (Lq=%d Lk=%d block=%d)",
-                Lq, Lk, block);
   AttnParams p{};
   fill(p, q, k, v, B, H, Lq, Lk, D, q_strides, k_strides, v_strides, block, sm_scale);
   p.o = const_cast<void*>(o); p.dO = dO;
   int which = pick_path(path, p, dtype, true);
   if (which < 0) return which;
+  LMK_CHECK_ARG(which == LMK_PATH_TCGEN05 || (Lq % block == 0 && Lk % block == 0),
+                "Backward supported only for full blocks (Lq=%d Lk=%d block=%d)", Lq, Lk, block);
   const size_t need = lmk_attn_bwd_workspace(B, H, Lq, Lk, D, block, dtype, which);
   if (need > 0 && (workspace == nullptr || workspace_bytes < need))
     return fail(LMK_ERR_WORKSPACE, "attn_bwd: workspace of %zu bytes required, %zu given", need, workspace_bytes);

@@ -1,23 +1,21 @@
 // Fused landmark attention for sm_100a: TMA-fed tcgen05 MMAs with TMEM accumulators.
 //
-// Shape contract: bf16 / fp16, head dim 128, landmark block 64, Lq a multiple of 128, Lk a multiple of 64.
+// Shape contract: bf16 / fp16, head dim up to 128 (a multiple of 8), landmark block 64, any Lq, Lk - Lq a multiple of 64.
+// Rows past the end of a sequence and features past the head dim are zeros that TMA fills in: no padded copies exist
+// (the copies took 86 of 146 us at Lq = 1999, H = 32, D = 128 and 104 of 237 us at D = 64), and what is computed for them
+// is dropped at the stores.  Head dims up to 64 run instances with half the products.
 //
-// Forward, one CTA per (128 query rows, batch*head); rows 0-63 belong to landmark block `own0`, rows 64-127 to
-// `own0 + 1`.  Warps 0-3 run the softmax (thread = query row = TMEM lane), warp 4 issues TMA loads, warp 5 issues
-// the MMAs and owns the TMEM allocation.
+// Forward, one or two tiles of 128 query rows per CTA; rows 0-63 of a tile belong to landmark block `own0`, rows 64-127 to
+// `own0 + 1`.
 //   1. Pre-pass: S_lm = Q . K_lm^T against the landmark keys only (every 64th key, fetched with a strided 5-D TMA box)
 //      gives each row the maximum landmark score of its earlier blocks.  Together with the row maximum of the
 //      own (diagonal) block, which is processed first, this is the FINAL maximum of the outer softmax, so the O
 //      accumulator in TMEM is never rescaled.
 //   2. Main loop over key blocks n = own0+1 ... 0:  S = Q . K_n^T (N = 64);  the softmax threads read S from TMEM,
 //      form the block's weights  p_j = softmax_inside_block(s)_j * exp(l_n - m)  (own block: exp(s_j - m), causal),
-//      write them as bf16 into shared memory (128-byte swizzled, K-major), and O += P . V_n runs with V as an
-//      MN-major operand straight from its row-major TMA tile.
+//      write them in 16 bits over the TMEM columns their S came from, and O += P . V_n takes P from there as the A operand
+//      and V as an MN-major operand straight from its row-major TMA tile.
 //   3. Epilogue: O / l -> global, plus the statistics L = l, M = m the backward pass needs.
-// When Lq is a multiple of 256 the paired kernel (sm100_fwd2_kernel) runs instead: two query tiles per CTA share every
-// K/V tile, each with its own softmax warpgroup; P goes back into the TMEM columns its S came from and P . V takes it
-// from there as the A operand (no shared-memory round trip); the exponentials are packed fp32 pairs, a quarter of them
-// evaluated on the FMA pipe.
 // Reference semantics: llama/ltriton/flash_landmark_attention.py:6-122.
 //
 // Backward is recompute-based and atomic-free (bit-reproducible), in two launches:
@@ -48,29 +46,11 @@ namespace {
 
 using namespace ptx;
 
-constexpr int kD = 128;
 constexpr int kBlk = 64;
 constexpr int kQTile = 128;
-constexpr int kFwdStages = 2;
-constexpr int kFwdThreads = 192;
 constexpr uint32_t kTileBytes = 16384;   // one [128 x 64] or two [64 x 64] 16-bit tiles
 constexpr uint32_t kHalfTile = 8192;
 constexpr float kLog2e = 1.4426950408889634f;
-
-// error sites reported through g_lmk_status
-enum { kErrFwdProducer = 101, kErrFwdMma = 102, kErrFwdSoftmax = 103, kErrFwdEpilogue = 104 };
-
-struct FwdSmem {
-  // tile storage is addressed manually from the 1024-byte aligned base; this struct holds the barriers only
-  uint64_t q_full;
-  uint64_t full[kFwdStages];
-  uint64_t empty[kFwdStages];
-  uint64_t p_ready[kFwdStages];
-  uint64_t s_full[2];
-  uint64_t s_free[2];
-  uint64_t o_full;
-  uint32_t tmem_base;
-};
 
 template <bool kBf16>
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -137,241 +117,8 @@ __device__ __forceinline__ float row_sum(const float (&v)[64]) {
   return (a + b) + (c + d);
 }
 
-template <bool kBf16>
-__global__ void __launch_bounds__(kFwdThreads, 2)
-sm100_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_klm,
-                 void* __restrict__ o_ptr, float* __restrict__ L_ptr, float* __restrict__ M_ptr, int H, int Lq, int Lk,
-                 int lm_box, float scale_log2) {
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  const uint32_t q_tile = base;                                        // 32 KB: two [128 x 64] sub-tiles
-  auto k_slot = [&](int s) { return base + 32768u + (uint32_t)s * 32768u; };   // 16 KB: K block, later P
-  auto v_slot = [&](int s) { return base + 32768u + (uint32_t)s * 32768u + 16384u; };
-  FwdSmem* sm = reinterpret_cast<FwdSmem*>(smem_raw + (base - raw) + 32768u + kFwdStages * 32768u);
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_tiles = Lq / kQTile;
-  // grid = (batch*head, tile): consecutive CTAs are different heads of the same tile, heaviest tiles first, so the
-  // hardware's in-order block dispatch is a longest-job-first schedule over the whole launch
-  const int t = n_tiles - 1 - (int)blockIdx.y;
-  const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
-  const int prefix_blocks = (Lk - Lq) / kBlk;
-  const int own0 = prefix_blocks + 2 * t;               // block of rows 0-63; rows 64-127 own own0+1
-  const int n_last = own0 + 1;
-  const int n_lm_tiles = (n_last + 63) / 64;            // landmarks 0 .. n_last-1
-  const int total = n_lm_tiles + n_last + 1;
-
-  if (tid == 0) {
-    mbar_init(smem_u32(&sm->q_full), 1);
-    for (int s = 0; s < kFwdStages; ++s) {
-      mbar_init(smem_u32(&sm->full[s]), 1);
-      mbar_init(smem_u32(&sm->empty[s]), 1);
-      mbar_init(smem_u32(&sm->p_ready[s]), 128);
-    }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(smem_u32(&sm->s_full[s]), 1);
-      mbar_init(smem_u32(&sm->s_free[s]), 128);
-    }
-    mbar_init(smem_u32(&sm->o_full), 1);
-    mbar_init_fence();
-  }
-  if (warp == 5) tmem_alloc(smem_u32(&sm->tmem_base), 256);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = sm->tmem_base;
-  const uint32_t tmem_s0 = tmem, tmem_o = tmem + 128;
-
-  if (warp == 4) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      prefetch_tensormap(&tm_q);
-      prefetch_tensormap(&tm_k);
-      prefetch_tensormap(&tm_v);
-      prefetch_tensormap(&tm_klm);
-      const uint32_t qb = smem_u32(&sm->q_full);
-      mbar_arrive_expect_tx(qb, 2 * kTileBytes);
-      tma_load_4d(q_tile, &tm_q, qb, 0, t * kQTile, h, b);
-      tma_load_4d(q_tile + kTileBytes, &tm_q, qb, 64, t * kQTile, h, b);
-      for (int i = 0; i < total; ++i) {
-        const int s = i % kFwdStages;
-        const uint32_t ph = (i / kFwdStages) & 1;
-        mbar_wait(smem_u32(&sm->empty[s]), ph ^ 1, &g_lmk_status, kErrFwdProducer);
-        const uint32_t fb = smem_u32(&sm->full[s]);
-        if (i < n_lm_tiles) {
-          // the landmark box holds lm_box <= 64 keys; rows beyond it keep stale data and are never used
-          mbar_arrive_expect_tx(fb, (uint32_t)lm_box * 256u);
-          tma_load_5d(k_slot(s), &tm_klm, fb, 0, kBlk - 1, i * 64, h, b);
-          tma_load_5d(k_slot(s) + kHalfTile, &tm_klm, fb, 64, kBlk - 1, i * 64, h, b);
-        } else {
-          const int n = n_last - (i - n_lm_tiles);
-          mbar_arrive_expect_tx(fb, 2 * kTileBytes);
-          tma_load_4d(k_slot(s), &tm_k, fb, 0, n * kBlk, h, b);
-          tma_load_4d(k_slot(s) + kHalfTile, &tm_k, fb, 64, n * kBlk, h, b);
-          tma_load_4d(v_slot(s), &tm_v, fb, 0, n * kBlk, h, b);
-          tma_load_4d(v_slot(s) + kHalfTile, &tm_v, fb, 64, n * kBlk, h, b);
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 5) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 64, 0, 0);    // S = Q K^T
-      constexpr uint32_t idesc_o = instr_desc_f16(fmt, 128, 128, 0, 1);   // O += P V   (V is MN-major)
-      mbar_wait(smem_u32(&sm->q_full), 0, &g_lmk_status, kErrFwdMma);
-      // Q and K: two 64-column sub-tiles; a K-step of 16 elements is 32 bytes inside the swizzle atom
-      const uint64_t dq = smem_desc_sw128(q_tile, 16, 1024);
-      const uint64_t dk0 = smem_desc_sw128(k_slot(0), 16, 1024);
-      const uint64_t dv0 = smem_desc_sw128(v_slot(0), kHalfTile, 1024);
-      auto issue_s = [&](int j) {
-        const int s = j % kFwdStages, sb = j & 1;
-        mbar_wait(smem_u32(&sm->full[s]), (j / kFwdStages) & 1, &g_lmk_status, kErrFwdMma);
-        if (j >= 2) mbar_wait(smem_u32(&sm->s_free[sb]), ((j / 2) & 1) ^ 1, &g_lmk_status, kErrFwdMma);
-        tc_fence_after();
-        const uint64_t dk = desc_advance(dk0, (uint32_t)s * 32768u);
-#pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk)
-          mma_f16_ss(tmem_s0 + sb * 64, desc_advance(dq, kmajor_step(kk, kTileBytes)),
-                     desc_advance(dk, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
-        mma_commit(smem_u32(&sm->s_full[sb]));
-      };
-      issue_s(0);
-      bool o_started = false;
-      for (int i = 0; i < total; ++i) {
-        if (i + 1 < total) issue_s(i + 1);
-        const int s = i % kFwdStages;
-        mbar_wait(smem_u32(&sm->p_ready[s]), (i / kFwdStages) & 1, &g_lmk_status, kErrFwdMma);
-        tc_fence_after();
-        if (i >= n_lm_tiles) {
-          // P: [128 x 64] K-major tile in the K slot.  V: two [64 keys x 64 features] sub-tiles, MN-major:
-          // 8-key groups 1024 B apart (SBO), the second 64-feature half 8192 B further (LBO); 16 keys = 2048 B.
-          const uint64_t dp = desc_advance(dk0, (uint32_t)s * 32768u);
-          const uint64_t dv = desc_advance(dv0, (uint32_t)s * 32768u);
-#pragma unroll
-          for (int kk = 0; kk < kBlk / 16; ++kk)
-            mma_f16_ss(tmem_o, desc_advance(dp, kk * 32), desc_advance(dv, kk * 2048), idesc_o,
-                       (o_started || kk > 0) ? 1u : 0u);
-          o_started = true;
-        }
-        mma_commit(smem_u32(&sm->empty[s]));
-      }
-      mma_commit(smem_u32(&sm->o_full));
-    }
-    __syncwarp();
-  } else {
-    // ------------------------------------------------------------------ softmax threads (row = tid)
-    const int row = tid;
-    const int half = row >> 6;
-    const int own = own0 + half;
-    const int vis = min(row & 63, kBlk - 2);
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    float m2 = -INFINITY;   // maximum of the outer softmax, log2 domain
-    float l = 0.f;
-    for (int i = 0; i < total; ++i) {
-      const int sb = i & 1, s = i % kFwdStages;
-      mbar_wait(smem_u32(&sm->s_full[sb]), (i / 2) & 1, &g_lmk_status, kErrFwdSoftmax);
-      tc_fence_after();
-      uint32_t ra[32], rb[32];
-      tmem_ld_32x32b_x32(tmem_s0 + sb * 64 + lane_base, ra);
-      tmem_ld_32x32b_x32(tmem_s0 + sb * 64 + 32 + lane_base, rb);
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(smem_u32(&sm->s_free[sb]));
-      float sv[64];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        sv[j] = __uint_as_float(ra[j]) * scale_log2;
-        sv[32 + j] = __uint_as_float(rb[j]) * scale_log2;
-      }
-      if (i < n_lm_tiles) {
-        // landmark scores of blocks i*64 .. i*64+63; only blocks before the row's own block count
-        const int first = i * 64;
-#pragma unroll
-        for (int j = 0; j < 64; ++j)
-          if (first + j < own) m2 = fmaxf(m2, sv[j]);
-      } else {
-        const int n = n_last - (i - n_lm_tiles);
-        uint32_t w[32];
-        if (n > own) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) w[j] = 0u;
-        } else if (n == own) {
-          float mx = -INFINITY;
-#pragma unroll
-          for (int j = 0; j < 64; ++j)
-            if (j <= vis) mx = fmaxf(mx, sv[j]);
-          m2 = fmaxf(m2, mx);
-          float sum = 0.f;
-#pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            sv[j] = (j <= vis) ? ex2(sv[j] - m2) : 0.f;
-            sum += sv[j];
-          }
-          l += sum;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) w[j] = pack2<kBf16>(sv[2 * j], sv[2 * j + 1]);
-        } else {
-          const float lm = sv[63];
-          float mx = -INFINITY;
-#pragma unroll
-          for (int j = 0; j < 63; ++j) mx = fmaxf(mx, sv[j]);
-          float den = 0.f;
-#pragma unroll
-          for (int j = 0; j < 63; ++j) {
-            sv[j] = ex2(sv[j] - mx);
-            den += sv[j];
-          }
-          const float el = ex2(lm - m2);
-          l += el;
-          const float wgt = el / den;
-          sv[63] = 0.f;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) w[j] = pack2<kBf16>(sv[2 * j] * wgt, sv[2 * j + 1] * wgt);
-        }
-        store_row_sw128(k_slot(s), row, w);
-        fence_proxy_async_smem();
-      }
-      mbar_arrive(smem_u32(&sm->p_ready[s]));
-    }
-    // ------------------------------------------------------------------ epilogue
-    mbar_wait(smem_u32(&sm->o_full), 0, &g_lmk_status, kErrFwdEpilogue);
-    tc_fence_after();
-    const float inv = 1.f / l;
-    const int grow = t * kQTile + row;
-    uint4* orow = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(o_ptr) + ((int64_t)bh * Lq + grow) * kD);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(tmem_o + c * 32 + lane_base, r);
-      tmem_ld_wait();
-#pragma unroll
-      for (int v4 = 0; v4 < 4; ++v4) {
-        uint4 pk;
-        pk.x = pack2<kBf16>(__uint_as_float(r[8 * v4 + 0]) * inv, __uint_as_float(r[8 * v4 + 1]) * inv);
-        pk.y = pack2<kBf16>(__uint_as_float(r[8 * v4 + 2]) * inv, __uint_as_float(r[8 * v4 + 3]) * inv);
-        pk.z = pack2<kBf16>(__uint_as_float(r[8 * v4 + 4]) * inv, __uint_as_float(r[8 * v4 + 5]) * inv);
-        pk.w = pack2<kBf16>(__uint_as_float(r[8 * v4 + 6]) * inv, __uint_as_float(r[8 * v4 + 7]) * inv);
-        orow[c * 4 + v4] = pk;
-      }
-    }
-    L_ptr[(int64_t)bh * Lq + grow] = l;
-    M_ptr[(int64_t)bh * Lq + grow] = m2 * (1.f / kLog2e);
-    tc_fence_before();
-  }
-  __syncthreads();
-  if (warp == 5) {
-    tc_fence_after();
-    tmem_dealloc(tmem, 256);
-  }
-}
-
-
 // ---------------------------------------------------------------------------------------------- forward, two tiles
-// Same algorithm with TWO adjacent 128-row query tiles per CTA (one CTA per SM): softmax warpgroup 0 owns tile A
+// Up to TWO adjacent 128-row query tiles per CTA (one CTA per SM): softmax warpgroup 0 owns tile A
 // (rows 256u .. 256u+127), warpgroup 1 owns tile B (the next 128 rows).  Both tiles consume the same K/V stream, so
 // every K/V block is fetched from L2 once per 256 query rows, and the two softmax pipelines overlap with each
 // other and with the MMAs.  Tile A skips the two newest key blocks (they lie after its own blocks).
@@ -394,12 +141,12 @@ struct Fwd2Smem {
   uint32_t tmem_base;
 };
 
-template <bool kBf16>
+template <bool kBf16, int kD>
 __global__ void __launch_bounds__(kFwd2Threads, 1)
 sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_klm,
                   void* __restrict__ o_ptr, float* __restrict__ L_ptr, float* __restrict__ M_ptr, int H, int Lq, int Lk,
-                  int lm_box, float scale_log2) {
+                  int D, int lm_box, int per_cta, float scale_log2) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -409,16 +156,16 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   Fwd2Smem* sm = reinterpret_cast<Fwd2Smem*>(smem_raw + (base - raw) + 65536u + kFwd2Stages * 32768u);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_pairs = Lq / (2 * kQTile);
-  const int u = n_pairs - 1 - (int)blockIdx.y;          // heaviest pairs first, across all heads
+  const int t_a = ((int)gridDim.y - 1 - (int)blockIdx.y) * per_cta;      // heaviest tiles first, across all heads
+  const bool has_b = per_cta == 2 && (t_a + 1) * kQTile < Lq;            // the second tile has at least one row
   const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
   const int prefix_blocks = (Lk - Lq) / kBlk;
-  const int own0_a = prefix_blocks + 4 * u;             // tile A: blocks own0_a, own0_a+1; tile B: +2, +3
-  const int n_last = own0_a + 3;                        // newest block of the pair
+  const int own0_a = prefix_blocks + 2 * t_a;           // tile A: blocks own0_a, own0_a+1; tile B: +2, +3
+  const int n_last = min(own0_a + (has_b ? 3 : 1), (Lk - 1) / kBlk);     // newest block that any row of the CTA sees
   const int n_lm_tiles = (n_last + 63) / 64;            // landmarks 0 .. n_last-1
   const int total = n_lm_tiles + n_last + 1;
-  // tile A takes part in item i unless it is one of the first two main items
-  auto active = [&](int w, int i) { return w == 1 || i < n_lm_tiles || i >= n_lm_tiles + 2; };
+  // tile A takes part in every item but the main items of tile B's own blocks
+  auto active = [&](int w, int i) { return w == 1 ? has_b : (i < n_lm_tiles || n_last - (i - n_lm_tiles) <= own0_a + 1); };
 
   if (tid == 0) {
     mbar_init(smem_u32(&sm->q_full), 1);
@@ -453,26 +200,25 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       prefetch_tensormap(&tm_v);
       prefetch_tensormap(&tm_klm);
       const uint32_t qb = smem_u32(&sm->q_full);
-      mbar_arrive_expect_tx(qb, 4 * kTileBytes);
-      for (int w = 0; w < 2; ++w) {
-        tma_load_4d(q_tile(w), &tm_q, qb, 0, (2 * u + w) * kQTile, h, b);
-        tma_load_4d(q_tile(w) + kTileBytes, &tm_q, qb, 64, (2 * u + w) * kQTile, h, b);
-      }
+      mbar_arrive_expect_tx(qb, (has_b ? 2 : 1) * (kD / 64) * kTileBytes);
+      for (int w = 0; w < (has_b ? 2 : 1); ++w)
+        for (int c = 0; c < kD / 64; ++c)
+          tma_load_4d(q_tile(w) + c * kTileBytes, &tm_q, qb, 64 * c, (t_a + w) * kQTile, h, b);
       for (int i = 0; i < total; ++i) {
         const int s = i % kFwd2Stages;
         mbar_wait(smem_u32(&sm->empty[s]), ((i / kFwd2Stages) & 1) ^ 1, &g_lmk_status, kErrFwd2Producer);
         const uint32_t fb = smem_u32(&sm->full[s]);
         if (i < n_lm_tiles) {
-          mbar_arrive_expect_tx(fb, (uint32_t)lm_box * 256u);
-          tma_load_5d(k_slot(s), &tm_klm, fb, 0, kBlk - 1, i * 64, h, b);
-          tma_load_5d(k_slot(s) + kHalfTile, &tm_klm, fb, 64, kBlk - 1, i * 64, h, b);
+          mbar_arrive_expect_tx(fb, (uint32_t)(lm_box * kD * 2));
+          for (int c = 0; c < kD / 64; ++c)
+            tma_load_5d(k_slot(s) + c * kHalfTile, &tm_klm, fb, 64 * c, kBlk - 1, i * 64, h, b);
         } else {
           const int n = n_last - (i - n_lm_tiles);
-          mbar_arrive_expect_tx(fb, 2 * kTileBytes);
-          tma_load_4d(k_slot(s), &tm_k, fb, 0, n * kBlk, h, b);
-          tma_load_4d(k_slot(s) + kHalfTile, &tm_k, fb, 64, n * kBlk, h, b);
-          tma_load_4d(v_slot(s), &tm_v, fb, 0, n * kBlk, h, b);
-          tma_load_4d(v_slot(s) + kHalfTile, &tm_v, fb, 64, n * kBlk, h, b);
+          mbar_arrive_expect_tx(fb, 2 * (kD / 64) * kHalfTile);
+          for (int c = 0; c < kD / 64; ++c) {
+            tma_load_4d(k_slot(s) + c * kHalfTile, &tm_k, fb, 64 * c, n * kBlk, h, b);
+            tma_load_4d(v_slot(s) + c * kHalfTile, &tm_v, fb, 64 * c, n * kBlk, h, b);
+          }
         }
       }
     }
@@ -514,7 +260,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     // ------------------------------------------------------------------ MMA issuer 2: O += P V
     if (lane == 0) {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_o = instr_desc_f16(fmt, 128, 128, 0, 1);
+      constexpr uint32_t idesc_o = instr_desc_f16(fmt, 128, kD, 0, 1);
       const uint64_t dv0 = smem_desc_sw128(v_slot(0), kHalfTile, 1024);
       int kp[2] = {0, 0};
       bool o_started[2] = {false, false};
@@ -639,25 +385,30 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mbar_wait(smem_u32(&sm->o_full), 0, &g_lmk_status, kErrFwd2Epilogue);
     tc_fence_after();
     const float inv = 1.f / l;
-    const int grow = (2 * u + w) * kQTile + row;
-    uint4* orow = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(o_ptr) + ((int64_t)bh * Lq + grow) * kD);
+    const int grow = (t_a + w) * kQTile + row;
+    const bool stored = grow < Lq && (w == 0 || has_b);
+    uint4* orow = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(o_ptr) + ((int64_t)bh * Lq + grow) * D);
+    if (w == 0 || has_b) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(tmem_o(w) + c * 32 + lane_base, r);
-      tmem_ld_wait();
+      for (int c = 0; c < kD / 32; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tmem_o(w) + c * 32 + lane_base, r);
+        tmem_ld_wait();
 #pragma unroll
-      for (int v4 = 0; v4 < 4; ++v4) {
-        uint4 pk;
-        pk.x = pack2<kBf16>(__uint_as_float(r[8 * v4 + 0]) * inv, __uint_as_float(r[8 * v4 + 1]) * inv);
-        pk.y = pack2<kBf16>(__uint_as_float(r[8 * v4 + 2]) * inv, __uint_as_float(r[8 * v4 + 3]) * inv);
-        pk.z = pack2<kBf16>(__uint_as_float(r[8 * v4 + 4]) * inv, __uint_as_float(r[8 * v4 + 5]) * inv);
-        pk.w = pack2<kBf16>(__uint_as_float(r[8 * v4 + 6]) * inv, __uint_as_float(r[8 * v4 + 7]) * inv);
-        orow[c * 4 + v4] = pk;
+        for (int v4 = 0; v4 < 4; ++v4) {
+          uint4 pk;
+          pk.x = pack2<kBf16>(__uint_as_float(r[8 * v4 + 0]) * inv, __uint_as_float(r[8 * v4 + 1]) * inv);
+          pk.y = pack2<kBf16>(__uint_as_float(r[8 * v4 + 2]) * inv, __uint_as_float(r[8 * v4 + 3]) * inv);
+          pk.z = pack2<kBf16>(__uint_as_float(r[8 * v4 + 4]) * inv, __uint_as_float(r[8 * v4 + 5]) * inv);
+          pk.w = pack2<kBf16>(__uint_as_float(r[8 * v4 + 6]) * inv, __uint_as_float(r[8 * v4 + 7]) * inv);
+          if (stored && c * 32 + v4 * 8 < D) orow[c * 4 + v4] = pk;
+        }
       }
     }
-    L_ptr[(int64_t)bh * Lq + grow] = l;
-    M_ptr[(int64_t)bh * Lq + grow] = m2 * (1.f / kLog2e);
+    if (stored) {
+      L_ptr[(int64_t)bh * Lq + grow] = l;
+      M_ptr[(int64_t)bh * Lq + grow] = m2 * (1.f / kLog2e);
+    }
     tc_fence_before();
   }
   __syncthreads();
@@ -881,7 +632,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                      const float* __restrict__ L_ptr, const float* __restrict__ M_ptr,
                      const float* __restrict__ delta_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                     int H, int BH, int Lq, int Lk, float scale, float scale_log2) {
+                     int H, int BH, int Lq, int Lk, int D, float scale, float scale_log2) {
+  constexpr int kD = 128;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -896,8 +648,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int prefix_blocks = (Lk - Lq) / kBlk;
-  const int n_tiles = Lq / kQTile;
-  const int n_blocks = Lk / kBlk;
+  const int n_tiles = (Lq + kQTile - 1) / kQTile;
+  const int n_blocks = (Lk + kBlk - 1) / kBlk;
   const int n_pairs = (n_blocks + 1) / 2;
   const int n_units = n_pairs * BH;
   auto unit_of = [&](int r) {
@@ -1063,15 +815,17 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int n = 2 * pair + g;
       const int tq0 = unit_tq0(pair), n_items = n_tiles - tq0;
       // the row statistics of the next item are fetched one item ahead, so their latency is never exposed
-      const int64_t grow0 = (int64_t)bh * Lq + tq0 * kQTile + row;
+      // (rows past the end of the sequence have zero Q and dO tiles: whatever finite weights they get contribute nothing)
+      const int64_t grow0 = (int64_t)bh * Lq + min(tq0 * kQTile + row, Lq - 1);
       if (u == 0) grid_dep_wait();     // delta comes from the dQ kernel, which may still be running (see the launch)
       float nM = M_ptr[grow0], nL = L_ptr[grow0], nDelta = delta_ptr[grow0];
       for (int i = 0; i < n_items; ++i, ++it) {
         const int tq = tq0 + i;
         const int own = prefix_blocks + 2 * tq + half;
-        const float M2L = fmaf(nM, kLog2e, __log2f(nL)), delta = nDelta;
+        const bool row_valid = tq * kQTile + row < Lq;
+        const float M2L = row_valid ? fmaf(nM, kLog2e, __log2f(nL)) : 0.f, delta = row_valid ? nDelta : 0.f;
         if (i + 1 < n_items) {
-          const int64_t grow = (int64_t)bh * Lq + (tq + 1) * kQTile + row;
+          const int64_t grow = (int64_t)bh * Lq + min((tq + 1) * kQTile + row, Lq - 1);
           nM = M_ptr[grow];
           nL = L_ptr[grow];
           nDelta = delta_ptr[grow];
@@ -1119,15 +873,17 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(smem_u32(&sm->acc_empty[g]));     // the next unit may start accumulating into this block's columns
-      if (n < n_blocks) {
-        uint16_t* dvp = reinterpret_cast<uint16_t*>(dv_ptr) + ((int64_t)bh * Lk + (int64_t)n * kBlk) * kD + row;
-        uint16_t* dkp = reinterpret_cast<uint16_t*>(dk_ptr) + ((int64_t)bh * Lk + (int64_t)n * kBlk) * kD + row;
+      if (n < n_blocks && row < D) {
+        const int keys = min(kBlk, Lk - n * kBlk);
+        uint16_t* dvp = reinterpret_cast<uint16_t*>(dv_ptr) + ((int64_t)bh * Lk + (int64_t)n * kBlk) * D + row;
+        uint16_t* dkp = reinterpret_cast<uint16_t*>(dk_ptr) + ((int64_t)bh * Lk + (int64_t)n * kBlk) * D + row;
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            dvp[(int64_t)(c * 32 + j) * kD] = (uint16_t)(pack2<kBf16>(__uint_as_float(rv[c][j]), 0.f) & 0xffffu);
-            dkp[(int64_t)(c * 32 + j) * kD] = (uint16_t)(pack2<kBf16>(__uint_as_float(rk[c][j]), 0.f) & 0xffffu);
+            if (c * 32 + j >= keys) continue;
+            dvp[(int64_t)(c * 32 + j) * D] = (uint16_t)(pack2<kBf16>(__uint_as_float(rv[c][j]), 0.f) & 0xffffu);
+            dkp[(int64_t)(c * 32 + j) * D] = (uint16_t)(pack2<kBf16>(__uint_as_float(rk[c][j]), 0.f) & 0xffffu);
           }
       }
     }
@@ -1167,13 +923,13 @@ struct DqSmem {
 // CTAs in a snake.  The K/V stream, the S/dP products and the softmax of the next unit start while dQ of the current
 // unit is drained by one warpgroup (the two warpgroups alternate); only the unit's first accumulating MMA waits for
 // the drain.  All barrier phases derive from counters that run across units.
-template <bool kBf16>
+template <bool kBf16, int kD>
 __global__ void __launch_bounds__(kDqThreads, 1)
 sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_o, const float* __restrict__ L_ptr,
                     const float* __restrict__ M_ptr, float* __restrict__ delta_ptr, void* __restrict__ dq_ptr, int H,
-                    int BH, int Lq, int Lk, float scale, float scale_log2) {
+                    int BH, int Lq, int Lk, int D, float scale, float scale_log2) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -1184,7 +940,8 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   DqSmem* sm = reinterpret_cast<DqSmem*>(smem_raw + (base - raw) + 65536u + kDqStages * 32768u + 32768u);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_tiles = Lq / kQTile;
+  const int n_tiles = (Lq + kQTile - 1) / kQTile;
+  const int n_blocks = (Lk + kBlk - 1) / kBlk;
   const int prefix_blocks = (Lk - Lq) / kBlk;
   const int n_units = n_tiles * BH;
   auto unit_of = [&](int r) {
@@ -1193,7 +950,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   };
   // unit w -> query tile (heaviest = last tile first) and number of key blocks it sees
   auto unit_tile = [&](int w) { return n_tiles - 1 - w / BH; };
-  auto unit_items = [&](int t) { return prefix_blocks + 2 * t + 2; };
+  auto unit_items = [&](int t) { return min(prefix_blocks + 2 * t + 2, n_blocks); };
 
   if (tid == 0) {
     mbar_init(smem_u32(&sm->qdo_full), 1);
@@ -1243,23 +1000,22 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int total = unit_items(t), n_last = total - 1;
         const uint32_t qb = smem_u32(&sm->qdo_full);
         mbar_wait(smem_u32(&sm->delta_read), (u & 1) ^ 1, &g_lmk_status, kErrDqProducer);
-        mbar_arrive_expect_tx(qb, 6 * kTileBytes);
-        tma_load_4d(o_tile, &tm_o, qb, 0, t * kQTile, h, b);
-        tma_load_4d(o_tile + kTileBytes, &tm_o, qb, 64, t * kQTile, h, b);
-        tma_load_4d(q_tile, &tm_q, qb, 0, t * kQTile, h, b);
-        tma_load_4d(q_tile + kTileBytes, &tm_q, qb, 64, t * kQTile, h, b);
-        tma_load_4d(do_tile, &tm_do, qb, 0, t * kQTile, h, b);
-        tma_load_4d(do_tile + kTileBytes, &tm_do, qb, 64, t * kQTile, h, b);
+        mbar_arrive_expect_tx(qb, 3 * (kD / 64) * kTileBytes);
+        for (int c = 0; c < kD / 64; ++c) {
+          tma_load_4d(o_tile + c * kTileBytes, &tm_o, qb, 64 * c, t * kQTile, h, b);
+          tma_load_4d(q_tile + c * kTileBytes, &tm_q, qb, 64 * c, t * kQTile, h, b);
+          tma_load_4d(do_tile + c * kTileBytes, &tm_do, qb, 64 * c, t * kQTile, h, b);
+        }
         for (int i = 0; i < total; ++i, ++it) {
           const int s = it % kDqStages;
           mbar_wait(smem_u32(&sm->empty[s]), ((it / kDqStages) & 1) ^ 1, &g_lmk_status, kErrDqProducer);
           const uint32_t fb = smem_u32(&sm->full[s]);
           const int n = n_last - i;
-          mbar_arrive_expect_tx(fb, 2 * kTileBytes);
-          tma_load_4d(k_slot(s), &tm_k, fb, 0, n * kBlk, h, b);
-          tma_load_4d(k_slot(s) + kHalfTile, &tm_k, fb, 64, n * kBlk, h, b);
-          tma_load_4d(v_slot(s), &tm_v, fb, 0, n * kBlk, h, b);
-          tma_load_4d(v_slot(s) + kHalfTile, &tm_v, fb, 64, n * kBlk, h, b);
+          mbar_arrive_expect_tx(fb, 2 * (kD / 64) * kHalfTile);
+          for (int c = 0; c < kD / 64; ++c) {
+            tma_load_4d(k_slot(s) + c * kHalfTile, &tm_k, fb, 64 * c, n * kBlk, h, b);
+            tma_load_4d(v_slot(s) + c * kHalfTile, &tm_v, fb, 64 * c, n * kBlk, h, b);
+          }
         }
       }
     }
@@ -1296,7 +1052,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   } else if (warp == kBwdGroups * 4 + 2) {
     if (lane == 0) {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_q = instr_desc_f16(fmt, 128, 128, 0, 1);   // dQ += dS K  (K is MN-major)
+      constexpr uint32_t idesc_q = instr_desc_f16(fmt, 128, kD, 0, 1);   // dQ += dS K  (K is MN-major)
       const uint64_t dv0 = smem_desc_sw128(v_slot(0), 16, 1024);
       const uint64_t dk0t = smem_desc_sw128(k_slot(0), kHalfTile, 1024);
       int it = 0, u = 0;
@@ -1329,17 +1085,18 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // prologue of the NEXT unit: the last dQ product queues behind the next unit's first S / dP products, so an
     // immediate drain would just wait for it.  (The next unit's first dQ product needs its first dS, far later.)
     int64_t drain_row = -1;
+    bool drain_valid = false;                      // rows past the end of the sequence are computed and dropped
     auto drain = [&]() {
       mbar_wait(smem_u32(&sm->acc_full[g]), drains & 1, &g_lmk_status, kErrDqEpilogue);
       ++drains;
       tc_fence_after();
-      uint4* orow = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dq_ptr) + drain_row * kD);
+      uint4* orow = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dq_ptr) + drain_row * D);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < kD / 32; ++c) {
         uint32_t r[32];
         tmem_ld_32x32b_x32(tmem_dq + c * 32 + lane_base, r);
         tmem_ld_wait();
-        if (c == 3) {
+        if (c == kD / 32 - 1) {
           tc_fence_before();
           mbar_arrive(smem_u32(&sm->acc_empty));     // the next unit may start accumulating
         }
@@ -1350,7 +1107,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           pk.y = pack2<kBf16>(__uint_as_float(r[8 * v4 + 2]), __uint_as_float(r[8 * v4 + 3]));
           pk.z = pack2<kBf16>(__uint_as_float(r[8 * v4 + 4]), __uint_as_float(r[8 * v4 + 5]));
           pk.w = pack2<kBf16>(__uint_as_float(r[8 * v4 + 6]), __uint_as_float(r[8 * v4 + 7]));
-          orow[c * 4 + v4] = pk;
+          if (drain_valid && c * 32 + v4 * 8 < D) orow[c * 4 + v4] = pk;
         }
       }
       drain_row = -1;
@@ -1360,7 +1117,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     {
       const int w0 = unit_of(0);
       if (w0 < n_units) {
-        const int64_t g0 = (int64_t)(w0 % BH) * Lq + unit_tile(w0) * kQTile + row;
+        const int64_t g0 = (int64_t)(w0 % BH) * Lq + min(unit_tile(w0) * kQTile + row, Lq - 1);
         nM = M_ptr[g0];
         nL = L_ptr[g0];
       }
@@ -1370,11 +1127,12 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const int own = prefix_blocks + 2 * t + half;
       const int total = unit_items(t), n_last = total - 1;
       const int64_t grow = (int64_t)bh * Lq + t * kQTile + row;
+      const bool row_valid = t * kQTile + row < Lq;
       const float M2L = fmaf(nM, kLog2e, __log2f(nL));
       {
         const int wn = unit_of(u + 1);
         if (wn < n_units) {
-          const int64_t gn = (int64_t)(wn % BH) * Lq + unit_tile(wn) * kQTile + row;
+          const int64_t gn = (int64_t)(wn % BH) * Lq + min(unit_tile(wn) * kQTile + row, Lq - 1);
           nM = M_ptr[gn];
           nL = L_ptr[gn];
         }
@@ -1383,9 +1141,9 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // also publishes it for the dK/dV kernel, which runs after this one
       mbar_wait(smem_u32(&sm->qdo_full), u & 1, &g_lmk_status, kErrDqSoftmax);
       float delta = 0.f;
-      uint32_t opw[2][32];      // this thread's row of the operand its warpgroup moves to TMEM (0: Q, 1: dO)
+      uint32_t opw[kD / 64][32];      // this thread's row of the operand its warpgroup moves to TMEM (0: Q, 1: dO)
 #pragma unroll
-      for (int sub = 0; sub < 2; ++sub)
+      for (int sub = 0; sub < kD / 64; ++sub)
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const uint32_t off = (uint32_t)sub * kTileBytes + (uint32_t)row * 128u + (uint32_t)((c ^ (row & 7)) << 4);
@@ -1423,12 +1181,12 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       {
         const uint32_t dst = (g == 0 ? tmem_q : tmem_do) + lane_base;
         tmem_st_32x32b_x32(dst, opw[0]);
-        tmem_st_32x32b_x32(dst + 32, opw[1]);
+        if constexpr (kD == 128) tmem_st_32x32b_x32(dst + 32, opw[1]);
         tmem_st_wait();
       }
       tc_fence_before();
       mbar_arrive(smem_u32(&sm->ops_ready));
-      if (g == 0) delta_ptr[grow] = delta;
+      if (g == 0 && row_valid) delta_ptr[grow] = delta;
       if (drain_row >= 0) drain();
       for (int i = (it0 + g) & 1; i < total; i += kBwdGroups) {
         const int it = it0 + i;
@@ -1445,7 +1203,10 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         mbar_arrive(smem_u32(&sm->ds_ready[s]));
       }
       it0 += total;
-      if (g == ((it0 - 1) & 1)) drain_row = grow;
+      if (g == ((it0 - 1) & 1)) {
+        drain_row = grow;
+        drain_valid = row_valid;
+      }
     }
     if (drain_row >= 0) drain();
     tc_fence_before();
@@ -1487,11 +1248,11 @@ EncodeTiledFn get_encode() {
 // is small, shared by all threads and replaced round-robin.
 struct MapKey {
   const void* ptr;
-  int kind, dtype, B, H, L, box;
+  int kind, dtype, B, H, L, box, D;
   int64_t st[3];
   bool operator==(const MapKey& o) const {
     return ptr == o.ptr && kind == o.kind && dtype == o.dtype && B == o.B && H == o.H && L == o.L && box == o.box &&
-           st[0] == o.st[0] && st[1] == o.st[1] && st[2] == o.st[2];
+           D == o.D && st[0] == o.st[0] && st[1] == o.st[1] && st[2] == o.st[2];
   }
 };
 constexpr int kMapCacheSize = 64;
@@ -1526,13 +1287,14 @@ int cached_map(CUtensorMap* m, const MapKey& key, EncodeFn encode) {
   return LMK_OK;
 }
 
-// [B, H, L, 128] tensor with element strides {b, h, row}; box = 64 features x `box_rows` rows, 128-byte swizzle
-int make_map_4d(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int L, const int64_t st[3], int box_rows) {
-  const MapKey key{ptr, 4, dtype, B, H, L, box_rows, {st[0], st[1], st[2]}};
+// [B, H, L, D] tensor with element strides {b, h, row}; box = 64 features x `box_rows` rows, 128-byte swizzle; what lies
+// outside the tensor (rows past L, features past D) reads as zeros
+int make_map_4d(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int L, int D, const int64_t st[3], int box_rows) {
+  const MapKey key{ptr, 4, dtype, B, H, L, box_rows, D, {st[0], st[1], st[2]}};
   return cached_map(m, key, [&](CUtensorMap* out) {
     EncodeTiledFn enc = get_encode();
     if (!enc) return fail(LMK_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[4] = {(cuuint64_t)kD, (cuuint64_t)L, (cuuint64_t)H, (cuuint64_t)B};
+    cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)L, (cuuint64_t)H, (cuuint64_t)B};
     cuuint64_t strides[3] = {(cuuint64_t)st[2] * 2, (cuuint64_t)st[1] * 2, (cuuint64_t)st[0] * 2};
     cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
@@ -1544,14 +1306,17 @@ int make_map_4d(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int L,
   });
 }
 
-// landmark keys: k viewed as [B, H, L/64, 64, 128]; box = 64 features x 1 row-in-block x 64 blocks
-int make_map_landmarks(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int L, const int64_t st[3],
+// landmark keys: k viewed as [B, H, L/64, 64, D]; box = 64 features x 1 row-in-block x 64 blocks
+int make_map_landmarks(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int L, int D, const int64_t st[3],
                        int lm_box) {
-  const MapKey key{ptr, 5, dtype, B, H, L, lm_box, {st[0], st[1], st[2]}};
+  const MapKey key{ptr, 5, dtype, B, H, L, lm_box, D, {st[0], st[1], st[2]}};
   return cached_map(m, key, [&](CUtensorMap* out) {
     EncodeTiledFn enc = get_encode();
     if (!enc) return fail(LMK_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[5] = {(cuuint64_t)kD, (cuuint64_t)kBlk, (cuuint64_t)(L / kBlk), (cuuint64_t)H, (cuuint64_t)B};
+    // whole blocks only (the rows of a partial last block have no landmark among them); a sequence shorter than one block
+    // has no landmark row at all, and its map no row 63
+    cuuint64_t dims[5] = {(cuuint64_t)D, (cuuint64_t)(L < kBlk ? L : kBlk), (cuuint64_t)(L < kBlk ? 1 : L / kBlk), (cuuint64_t)H,
+                          (cuuint64_t)B};
     cuuint64_t strides[4] = {(cuuint64_t)st[2] * 2, (cuuint64_t)st[2] * 2 * kBlk, (cuuint64_t)st[1] * 2,
                              (cuuint64_t)st[0] * 2};
     cuuint32_t box[5] = {64, 1, (cuuint32_t)lm_box, 1, 1};
@@ -1572,7 +1337,6 @@ struct DeviceFacts {
   int n_sm = 0;
 };
 constexpr size_t kSmemFwd2 = 1024 + 65536 + kFwd2Stages * 32768 + sizeof(Fwd2Smem);
-constexpr size_t kSmemFwd = 1024 + 32768 + kFwdStages * 32768 + sizeof(FwdSmem);
 constexpr size_t kSmemDkv = 1024 + 65536 + kDkvStages * 65536 + 32768 + sizeof(DkvSmem);
 constexpr size_t kSmemDq = 1024 + 65536 + kDqStages * 32768 + 32768 + sizeof(DqSmem);
 
@@ -1587,12 +1351,14 @@ int device_facts(const DeviceFacts** out) {
   if (!f.ready) {
     LMK_CUDA(cudaDeviceGetAttribute(&f.n_sm, cudaDevAttrMultiProcessorCount, dev));
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<true>, attr, (int)kSmemFwd2));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<false>, attr, (int)kSmemFwd2));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd_kernel<true>, attr, (int)kSmemFwd));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd_kernel<false>, attr, (int)kSmemFwd));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<true>, attr, (int)kSmemDq));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<false>, attr, (int)kSmemDq));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<true, 128>, attr, (int)kSmemFwd2));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<false, 128>, attr, (int)kSmemFwd2));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<true, 64>, attr, (int)kSmemFwd2));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<false, 64>, attr, (int)kSmemFwd2));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<true, 128>, attr, (int)kSmemDq));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<false, 128>, attr, (int)kSmemDq));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<true, 64>, attr, (int)kSmemDq));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<false, 64>, attr, (int)kSmemDq));
     LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<true>, attr, (int)kSmemDkv));
     LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<false>, attr, (int)kSmemDkv));
     f.ready = true;
@@ -1607,20 +1373,28 @@ std::atomic<int> g_max_ctas{0};
 
 // A tensor the TMA unit can address: 16-byte aligned base, positive strides that are multiples of 16 bytes
 // (an expanded view has stride 0), rows at least one head apart.
-bool tma_ok(const void* p, const int64_t st[3]) {
+bool tma_ok(const void* p, const int64_t st[3], int D = 128) {
   return ((uintptr_t)p % 16 == 0) && st[0] > 0 && st[1] > 0 && st[0] % 8 == 0 && st[1] % 8 == 0 && st[2] % 8 == 0 &&
-         st[2] >= kD;
+         st[2] >= D;
 }
 
 }  // namespace
 
+// whole tiles of full head dim: what an explicit request for this path asks for
 bool attn_sm100_supported(int B, int H, int Lq, int Lk, int D, int block, int dtype) {
-  return (dtype == LMK_BF16 || dtype == LMK_F16) && D == kD && block == kBlk && Lq >= kQTile && Lq % kQTile == 0 &&
+  return (dtype == LMK_BF16 || dtype == LMK_F16) && D == 128 && block == kBlk && Lq >= kQTile && Lq % kQTile == 0 &&
          Lk % kBlk == 0 && Lk >= Lq && B >= 1 && H >= 1;
 }
 
+// everything the kernels take: any length (rows past the end read as zeros and are dropped), head dims below 128 (features
+// past the end read as zeros; at most 64 of them run with half the products)
+bool attn_sm100_takes(int B, int H, int Lq, int Lk, int D, int block, int dtype) {
+  return (dtype == LMK_BF16 || dtype == LMK_F16) && D >= 8 && D <= 128 && D % 8 == 0 && block == kBlk && Lq >= 1 &&
+         Lk >= Lq && (Lk - Lq) % kBlk == 0 && B >= 1 && H >= 1;
+}
+
 bool attn_sm100_operands_ok(const AttnParams& p, bool backward) {
-  if (!tma_ok(p.q, p.qs) || !tma_ok(p.k, p.ks) || !tma_ok(p.v, p.vs)) return false;
+  if (!tma_ok(p.q, p.qs, p.D) || !tma_ok(p.k, p.ks, p.D) || !tma_ok(p.v, p.vs, p.D)) return false;
   if (backward && ((uintptr_t)p.dO % 16 != 0 || (uintptr_t)p.o % 16 != 0)) return false;
   return true;
 }
@@ -1629,71 +1403,66 @@ void attn_sm100_set_max_ctas(int n) { g_max_ctas.store(n > 0 ? n : 0); }
 
 int tensor_map_4d(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int L, const int64_t st[3], int box_rows) {
   bind_context();
-  return make_map_4d(m, ptr, dtype, B, H, L, st, box_rows);
+  return make_map_4d(m, ptr, dtype, B, H, L, 128, st, box_rows);
 }
 bool tensor_map_operand_ok(const void* p, const int64_t st[3]) { return tma_ok(p, st); }
 
 int attn_sm100_fwd(const AttnParams& p, int dtype, cudaStream_t st) {
-  if (!tma_ok(p.q, p.qs) || !tma_ok(p.k, p.ks) || !tma_ok(p.v, p.vs))
+  if (!attn_sm100_operands_ok(p, false))
     return fail(LMK_ERR_UNSUPPORTED, "tcgen05 path needs 16-byte aligned q/k/v with strides that are multiples of 8");
   bind_context();
   CUtensorMap tq, tk, tv, tl;
   int rc;
-  if ((rc = make_map_4d(&tq, p.q, dtype, p.B, p.H, p.Lq, p.qs, kQTile)) != LMK_OK) return rc;
-  if ((rc = make_map_4d(&tk, p.k, dtype, p.B, p.H, p.Lk, p.ks, kBlk)) != LMK_OK) return rc;
-  if ((rc = make_map_4d(&tv, p.v, dtype, p.B, p.H, p.Lk, p.vs, kBlk)) != LMK_OK) return rc;
-  const int lm_box = (p.Lk / kBlk) < 64 ? (p.Lk / kBlk) : 64;
-  if ((rc = make_map_landmarks(&tl, p.k, dtype, p.B, p.H, p.Lk, p.ks, lm_box)) != LMK_OK) return rc;
+  if ((rc = make_map_4d(&tq, p.q, dtype, p.B, p.H, p.Lq, p.D, p.qs, kQTile)) != LMK_OK) return rc;
+  if ((rc = make_map_4d(&tk, p.k, dtype, p.B, p.H, p.Lk, p.D, p.ks, kBlk)) != LMK_OK) return rc;
+  if ((rc = make_map_4d(&tv, p.v, dtype, p.B, p.H, p.Lk, p.D, p.vs, kBlk)) != LMK_OK) return rc;
+  const int whole_blocks = p.Lk / kBlk;
+  const int lm_box = whole_blocks < 1 ? 1 : (whole_blocks < 64 ? whole_blocks : 64);
+  if ((rc = make_map_landmarks(&tl, p.k, dtype, p.B, p.H, p.Lk, p.D, p.ks, lm_box)) != LMK_OK) return rc;
   const float scale_log2 = p.scale * kLog2e;
   const DeviceFacts* facts = nullptr;
   if ((rc = device_facts(&facts)) != LMK_OK) return rc;
-  if (p.Lq % (2 * kQTile) == 0) {
-    dim3 grid(p.B * p.H, p.Lq / (2 * kQTile));
-    if (dtype == LMK_BF16)
-      sm100_fwd2_kernel<true><<<grid, kFwd2Threads, kSmemFwd2, st>>>(tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk,
-                                                                     lm_box, scale_log2);
-    else
-      sm100_fwd2_kernel<false><<<grid, kFwd2Threads, kSmemFwd2, st>>>(tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk,
-                                                                      lm_box, scale_log2);
+  // Two query tiles a CTA share one K/V stream (a pair costs 1.2 - 1.3 times a single tile); one tile a CTA while that still
+  // leaves every CTA an SM of its own.
+  const int n_tiles = (p.Lq + kQTile - 1) / kQTile;
+  const int per_cta = (int64_t)n_tiles * p.B * p.H <= facts->n_sm ? 1 : 2;
+  const dim3 grid(p.B * p.H, (n_tiles + per_cta - 1) / per_cta);
+#define LMK_FWD_LAUNCH(BF, DIM)                                                                                          \
+  sm100_fwd2_kernel<BF, DIM><<<grid, kFwd2Threads, kSmemFwd2, st>>>(tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk, p.D, \
+                                                                    lm_box, per_cta, scale_log2)
+  if (dtype == LMK_BF16) {
+    if (p.D <= 64) LMK_FWD_LAUNCH(true, 64); else LMK_FWD_LAUNCH(true, 128);
   } else {
-    dim3 grid(p.B * p.H, p.Lq / kQTile);
-    if (dtype == LMK_BF16)
-      sm100_fwd_kernel<true><<<grid, kFwdThreads, kSmemFwd, st>>>(tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk,
-                                                                  lm_box, scale_log2);
-    else
-      sm100_fwd_kernel<false><<<grid, kFwdThreads, kSmemFwd, st>>>(tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk,
-                                                                   lm_box, scale_log2);
+    if (p.D <= 64) LMK_FWD_LAUNCH(false, 64); else LMK_FWD_LAUNCH(false, 128);
   }
+#undef LMK_FWD_LAUNCH
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }
 
 int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
-  if (!tma_ok(p.q, p.qs) || !tma_ok(p.k, p.ks) || !tma_ok(p.v, p.vs) || (uintptr_t)p.dO % 16 != 0 ||
-      (uintptr_t)p.o % 16 != 0)
+  if (!attn_sm100_operands_ok(p, true))
     return fail(LMK_ERR_UNSUPPORTED, "tcgen05 path needs 16-byte aligned tensors with strides that are multiples of 8");
-  if (p.Lk % kBlk != 0 || p.Lq % kQTile != 0)
-    return fail(LMK_ERR_INVALID, "Backward supported only for full blocks");
   bind_context();
   CUtensorMap tq, tk, tv, tdo;
   int rc;
-  const int64_t dense[3] = {(int64_t)p.H * p.Lq * kD, (int64_t)p.Lq * kD, (int64_t)kD};
-  if ((rc = make_map_4d(&tq, p.q, dtype, p.B, p.H, p.Lq, p.qs, kQTile)) != LMK_OK) return rc;
-  if ((rc = make_map_4d(&tk, p.k, dtype, p.B, p.H, p.Lk, p.ks, kBlk)) != LMK_OK) return rc;
-  if ((rc = make_map_4d(&tv, p.v, dtype, p.B, p.H, p.Lk, p.vs, kBlk)) != LMK_OK) return rc;
-  if ((rc = make_map_4d(&tdo, p.dO, dtype, p.B, p.H, p.Lq, dense, kQTile)) != LMK_OK) return rc;
+  const int64_t dense[3] = {(int64_t)p.H * p.Lq * p.D, (int64_t)p.Lq * p.D, (int64_t)p.D};
+  if ((rc = make_map_4d(&tq, p.q, dtype, p.B, p.H, p.Lq, p.D, p.qs, kQTile)) != LMK_OK) return rc;
+  if ((rc = make_map_4d(&tk, p.k, dtype, p.B, p.H, p.Lk, p.D, p.ks, kBlk)) != LMK_OK) return rc;
+  if ((rc = make_map_4d(&tv, p.v, dtype, p.B, p.H, p.Lk, p.D, p.vs, kBlk)) != LMK_OK) return rc;
+  if ((rc = make_map_4d(&tdo, p.dO, dtype, p.B, p.H, p.Lq, p.D, dense, kQTile)) != LMK_OK) return rc;
   float* delta = reinterpret_cast<float*>(p.workspace);
   const float scale_log2 = p.scale * kLog2e;
   const size_t smem_dkv = kSmemDkv, smem_dq = kSmemDq;
   CUtensorMap to;
-  if ((rc = make_map_4d(&to, p.o, dtype, p.B, p.H, p.Lq, dense, kQTile)) != LMK_OK) return rc;
+  if ((rc = make_map_4d(&to, p.o, dtype, p.B, p.H, p.Lq, p.D, dense, kQTile)) != LMK_OK) return rc;
   const DeviceFacts* facts = nullptr;
   if ((rc = device_facts(&facts)) != LMK_OK) return rc;
   int n_sm = facts->n_sm;
   const int cap = g_max_ctas.load();
   if (cap >= 1 && cap < n_sm) n_sm = cap;
-  const int dkv_units = ((p.Lk / kBlk + 1) / 2) * p.B * p.H;
-  const int dq_units = (p.Lq / kQTile) * p.B * p.H;
+  const int dkv_units = ((p.Lk + 2 * kBlk - 1) / (2 * kBlk)) * p.B * p.H;
+  const int dq_units = ((p.Lq + kQTile - 1) / kQTile) * p.B * p.H;
   dim3 grid_dkv(dkv_units < n_sm ? dkv_units : n_sm), grid_dq(dq_units < n_sm ? dq_units : n_sm);
   // Both launches can carry the programmatic-stream-serialization attribute.  The dQ kernel waits for the kernel before it
   // right after its set-up (only the set-up overlaps).  The dK/dV kernel reads q, k, v, dO, L, M, which were complete
@@ -1717,15 +1486,18 @@ int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
   const float* Mc = p.M;
   const float* deltac = delta;
   const int BH = p.B * p.H;
-#define LMK_BWD_LAUNCH(BF)                                                                                          \
-  do {                                                                                                              \
-    LMK_CUDA(cudaLaunchKernelEx(&cfg_dq, sm100_bwd_dq_kernel<BF>, tq, tk, tv, tdo, to, Lc, Mc, delta, p.dq, p.H, BH, \
-                                p.Lq, p.Lk, p.scale, scale_log2));                                                  \
-    LMK_CUDA(cudaLaunchKernelEx(&cfg_dkv, sm100_bwd_dkv_kernel<BF>, tq, tk, tv, tdo, Lc, Mc, deltac, p.dk, p.dv,    \
-                                p.H, BH, p.Lq, p.Lk, p.scale, scale_log2));                                         \
+#define LMK_BWD_LAUNCH(BF, DIM)                                                                                          \
+  do {                                                                                                                   \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg_dq, sm100_bwd_dq_kernel<BF, DIM>, tq, tk, tv, tdo, to, Lc, Mc, delta, p.dq, p.H,    \
+                                BH, p.Lq, p.Lk, p.D, p.scale, scale_log2));                                              \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg_dkv, sm100_bwd_dkv_kernel<BF>, tq, tk, tv, tdo, Lc, Mc, deltac, p.dk, p.dv,         \
+                                p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2));                                         \
   } while (0)
-  if (dtype == LMK_BF16) LMK_BWD_LAUNCH(true);
-  else LMK_BWD_LAUNCH(false);
+  if (dtype == LMK_BF16) {
+    if (p.D <= 64) LMK_BWD_LAUNCH(true, 64); else LMK_BWD_LAUNCH(true, 128);
+  } else {
+    if (p.D <= 64) LMK_BWD_LAUNCH(false, 64); else LMK_BWD_LAUNCH(false, 128);
+  }
 #undef LMK_BWD_LAUNCH
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;

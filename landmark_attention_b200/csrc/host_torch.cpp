@@ -128,7 +128,6 @@ struct FusedLandmark : public torch::autograd::Function<FusedLandmark> {
     const int64_t block = ctx->saved_data["block"].toInt(), path = ctx->saved_data["path"].toInt();
     const double scale = ctx->saved_data["scale"].toDouble();
     const auto B = q.size(0), H = q.size(1), Lq = q.size(2), D = q.size(3), Lk = k.size(2);
-    LMK_ASSERT(Lq % block == 0 && Lk % block == 0, "Backward supported only for full blocks");
     c10::cuda::OptionalCUDAGuard guard(q.device());
     Tensor dO = grads[0].contiguous();
     if (dO.scalar_type() != q.scalar_type()) dO = dO.to(q.scalar_type());
@@ -636,12 +635,12 @@ PyObject* py_init(PyObject*, PyObject* arg) {
   END_HANDLE_TH_ERRORS
 }
 
-// fused_attention(q, k, v, is_mem | None, scale, block, path)
+// fused_attention(q, k, v, is_mem | None, scale | None, block, path)
 PyObject* py_fused_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 7);
   const Tensor &q = tensor_arg(a[0], "q"), &k = tensor_arg(a[1], "k"), &v = tensor_arg(a[2], "v");
-  const double scale = float_arg(a[4]);
+  const double scale = a[4] == Py_None ? 1.0 / std::sqrt((double)q.size(-1)) : float_arg(a[4]);
   const int64_t block = int_arg(a[5]), path = int_arg(a[6]);
   std::optional<RegularCheck> mask;
   if (a[3] != Py_None) mask.emplace(tensor_arg(a[3], "is_mem"), block);

@@ -27,52 +27,34 @@ def fused_landmark_attention(q, k, v, is_mem=None, sm_scale=None, block_size=64,
     `is_mem` may be None (fast path: no mask is read and the host is not synchronised); when given it must be the
     regular pattern over the keys, as the reference asserts (flash_landmark_attention.py:393-394).
     """
-    n_history_kv = k.shape[-2] - q.shape[-2]
-    assert n_history_kv % block_size == 0
-    if sm_scale is None:
-        sm_scale = 1.0 / math.sqrt(q.size(-1))
-    D = q.shape[-1]
-    if (path == L.PATH_AUTO and q.is_cuda and q.dtype in (torch.bfloat16, torch.float16) and D <= 128 and D % 8 == 0
-            and q.shape[2] % 128 != 0 and n_history_kv % 64 == 0):
-        # lengths that are not whole 128-row tiles: rows of zeros appended to q, k and v come after every real query,
-        # so causality hides the extra keys and the extra query rows are dropped again
-        extra = -q.shape[2] % 128
-        if _tensor_core_route(q.shape[0], q.shape[1], q.shape[2] + extra, k.shape[2] + extra, block_size, q.dtype):
-            _check_mask(is_mem, block_size)
-            qp, kp, vp = [torch.nn.functional.pad(t, (0, 0, 0, extra)) for t in (q, k, v)]
-            return fused_landmark_attention(qp, kp, vp, None, sm_scale, block_size, path)[:, :, :q.shape[2]]
-    if (path == L.PATH_AUTO and D < 128 and D % 8 == 0 and q.is_cuda and q.dtype in (torch.bfloat16, torch.float16)
-            and _tensor_core_route(q.shape[0], q.shape[1], q.shape[2], k.shape[2], block_size, q.dtype)):
-        # head dims below 128: zero columns change neither q k^T nor the real columns of p v, and the tensor-core
-        # kernels at twice the work beat the general kernels by an order of magnitude
-        _check_mask(is_mem, block_size)
-        pad = (0, 128 - D)
-        qp, kp, vp = [torch.nn.functional.pad(t, pad) for t in (q, k, v)]
-        return fused_landmark_attention(qp, kp, vp, None, sm_scale, block_size, path)[..., :D]
-    if path == L.PATH_AUTO and block_size != 64:
-        # the tensor-core kernels of lmk_attn_fwd are built for blocks of 64; other block sizes run on the
-        # arbitrary-landmark tensor-core kernels with the regular pattern as flags, where those take the shape
-        from .masked import landmark_attention_masked, masked_attention_supported
-        Lk = k.shape[2]
-        groups = max(Lk // block_size, 1)          # landmarks in front of any query
-        if groups <= 64 and sm_scale > 0 and masked_attention_supported(q, k, groups):
-            _check_mask(is_mem, block_size)
-            return landmark_attention_masked(q, k, v, _regular_flags(q.shape[0], Lk, block_size, q.device), sm_scale,
-                                             groups)
+    if block_size != 64 and path == L.PATH_AUTO and q.is_cuda and q.dtype in (torch.bfloat16, torch.float16):
+        out = _other_block_size(q, k, v, is_mem, sm_scale, block_size)
+        if out is not None:
+            return out
     return L.host().fused_attention(q, k, v, is_mem, sm_scale, block_size, path)
 
 
-def _check_mask(is_mem, block_size):
+def _other_block_size(q, k, v, is_mem, sm_scale, block_size):
+    """The tensor-core kernels behind the host call are built for blocks of 64; other block sizes run on the arbitrary-landmark
+    tensor-core kernels with the regular pattern as flags, where those take the shape (None: they do not)."""
+    from .masked import landmark_attention_masked
+    B, Lq, Lk, D = q.shape[0], q.shape[2], k.shape[2], q.shape[3]
+    if D > 128 or D % 8 != 0 or (Lk - Lq) % block_size != 0 or (Lk - Lq) % 64 != 0 or Lk < Lq:
+        return None
+    if sm_scale is None:
+        sm_scale = 1.0 / math.sqrt(D)
+    # rows of zeros appended to q, k and v come after every real query, so causality hides the extra keys and the extra
+    # query rows are dropped again; zero columns change neither q k^T nor the real columns of p v
+    rows, cols = -Lq % 128, 128 - D
+    groups = max((Lk + rows) // block_size, 1)          # landmarks in front of any query
+    if groups > 64 or sm_scale <= 0 or Lk + rows > 32768:
+        return None
     if is_mem is not None:
         L.host().check_regular(is_mem, block_size)
-
-
-def _tensor_core_route(B, H, Lq, Lk, block_size, dtype):
-    """Whether a head-dim-128 problem of this shape runs on one of the two tensor-core kernel families."""
-    if block_size == 64:
-        return bool(L.lib().lmk_attn_tcgen05_supported(B, H, Lq, Lk, 128, 64, L._DTYPES[dtype]))
-    return (Lk // max(block_size, 1) <= 64 and Lq >= 128 and Lq % 128 == 0 and Lk % 64 == 0 and Lk >= Lq
-            and (Lk - Lq) % 64 == 0 and Lk <= 32768)
+    if rows or cols:
+        q, k, v = [torch.nn.functional.pad(t, (0, cols, 0, rows)) for t in (q, k, v)]
+    out = landmark_attention_masked(q, k, v, _regular_flags(B, Lk + rows, block_size, q.device), sm_scale, groups)
+    return out[:, :, :Lq, :D] if rows or cols else out
 
 
 _FLAGS = {}
