@@ -626,14 +626,15 @@ struct DkvSmem {
 // the item written before have read it), which settles them half an item apart.
 // CTA c takes units w = round * grid + c with the direction alternating per round (snake), heaviest pairs first.
 // Loads, S/dP products and the softmax of the next unit start while the accumulators of the current one are drained.
-template <bool kBf16>
+template <bool kBf16, bool kWhole>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                      const float* __restrict__ L_ptr, const float* __restrict__ M_ptr,
                      const float* __restrict__ delta_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                     int H, int BH, int Lq, int Lk, int D, float scale, float scale_log2) {
+                     int H, int BH, int Lq, int Lk, int D_any, float scale, float scale_log2) {
   constexpr int kD = 128;
+  const int D = kWhole ? kD : D_any;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -816,16 +817,16 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int tq0 = unit_tq0(pair), n_items = n_tiles - tq0;
       // the row statistics of the next item are fetched one item ahead, so their latency is never exposed
       // (rows past the end of the sequence have zero Q and dO tiles: whatever finite weights they get contribute nothing)
-      const int64_t grow0 = (int64_t)bh * Lq + min(tq0 * kQTile + row, Lq - 1);
+      const int64_t grow0 = (int64_t)bh * Lq + (kWhole ? tq0 * kQTile + row : min(tq0 * kQTile + row, Lq - 1));
       if (u == 0) grid_dep_wait();     // delta comes from the dQ kernel, which may still be running (see the launch)
       float nM = M_ptr[grow0], nL = L_ptr[grow0], nDelta = delta_ptr[grow0];
       for (int i = 0; i < n_items; ++i, ++it) {
         const int tq = tq0 + i;
         const int own = prefix_blocks + 2 * tq + half;
-        const bool row_valid = tq * kQTile + row < Lq;
+        const bool row_valid = kWhole || tq * kQTile + row < Lq;
         const float M2L = row_valid ? fmaf(nM, kLog2e, __log2f(nL)) : 0.f, delta = row_valid ? nDelta : 0.f;
         if (i + 1 < n_items) {
-          const int64_t grow = (int64_t)bh * Lq + min((tq + 1) * kQTile + row, Lq - 1);
+          const int64_t grow = (int64_t)bh * Lq + (kWhole ? (tq + 1) * kQTile + row : min((tq + 1) * kQTile + row, Lq - 1));
           nM = M_ptr[grow];
           nL = L_ptr[grow];
           nDelta = delta_ptr[grow];
@@ -873,7 +874,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(smem_u32(&sm->acc_empty[g]));     // the next unit may start accumulating into this block's columns
-      if (n < n_blocks && row < D) {
+      if (n < n_blocks && (kWhole || row < D)) {
         const int keys = min(kBlk, Lk - n * kBlk);
         uint16_t* dvp = reinterpret_cast<uint16_t*>(dv_ptr) + ((int64_t)bh * Lk + (int64_t)n * kBlk) * D + row;
         uint16_t* dkp = reinterpret_cast<uint16_t*>(dk_ptr) + ((int64_t)bh * Lk + (int64_t)n * kBlk) * D + row;
@@ -881,7 +882,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if (c * 32 + j >= keys) continue;
+            if (!kWhole && c * 32 + j >= keys) continue;
             dvp[(int64_t)(c * 32 + j) * D] = (uint16_t)(pack2<kBf16>(__uint_as_float(rv[c][j]), 0.f) & 0xffffu);
             dkp[(int64_t)(c * 32 + j) * D] = (uint16_t)(pack2<kBf16>(__uint_as_float(rk[c][j]), 0.f) & 0xffffu);
           }
@@ -923,13 +924,14 @@ struct DqSmem {
 // CTAs in a snake.  The K/V stream, the S/dP products and the softmax of the next unit start while dQ of the current
 // unit is drained by one warpgroup (the two warpgroups alternate); only the unit's first accumulating MMA waits for
 // the drain.  All barrier phases derive from counters that run across units.
-template <bool kBf16, int kD>
+template <bool kBf16, int kD, bool kWhole>
 __global__ void __launch_bounds__(kDqThreads, 1)
 sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_o, const float* __restrict__ L_ptr,
                     const float* __restrict__ M_ptr, float* __restrict__ delta_ptr, void* __restrict__ dq_ptr, int H,
-                    int BH, int Lq, int Lk, int D, float scale, float scale_log2) {
+                    int BH, int Lq, int Lk, int D_any, float scale, float scale_log2) {
+  const int D = kWhole ? kD : D_any;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -950,7 +952,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   };
   // unit w -> query tile (heaviest = last tile first) and number of key blocks it sees
   auto unit_tile = [&](int w) { return n_tiles - 1 - w / BH; };
-  auto unit_items = [&](int t) { return min(prefix_blocks + 2 * t + 2, n_blocks); };
+  auto unit_items = [&](int t) { return kWhole ? prefix_blocks + 2 * t + 2 : min(prefix_blocks + 2 * t + 2, n_blocks); };
 
   if (tid == 0) {
     mbar_init(smem_u32(&sm->qdo_full), 1);
@@ -1107,7 +1109,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           pk.y = pack2<kBf16>(__uint_as_float(r[8 * v4 + 2]), __uint_as_float(r[8 * v4 + 3]));
           pk.z = pack2<kBf16>(__uint_as_float(r[8 * v4 + 4]), __uint_as_float(r[8 * v4 + 5]));
           pk.w = pack2<kBf16>(__uint_as_float(r[8 * v4 + 6]), __uint_as_float(r[8 * v4 + 7]));
-          if (drain_valid && c * 32 + v4 * 8 < D) orow[c * 4 + v4] = pk;
+          if (kWhole || (drain_valid && c * 32 + v4 * 8 < D)) orow[c * 4 + v4] = pk;
         }
       }
       drain_row = -1;
@@ -1117,7 +1119,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     {
       const int w0 = unit_of(0);
       if (w0 < n_units) {
-        const int64_t g0 = (int64_t)(w0 % BH) * Lq + min(unit_tile(w0) * kQTile + row, Lq - 1);
+        const int64_t g0 = (int64_t)(w0 % BH) * Lq + (kWhole ? unit_tile(w0) * kQTile + row : min(unit_tile(w0) * kQTile + row, Lq - 1));
         nM = M_ptr[g0];
         nL = L_ptr[g0];
       }
@@ -1127,12 +1129,12 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const int own = prefix_blocks + 2 * t + half;
       const int total = unit_items(t), n_last = total - 1;
       const int64_t grow = (int64_t)bh * Lq + t * kQTile + row;
-      const bool row_valid = t * kQTile + row < Lq;
+      const bool row_valid = kWhole || t * kQTile + row < Lq;
       const float M2L = fmaf(nM, kLog2e, __log2f(nL));
       {
         const int wn = unit_of(u + 1);
         if (wn < n_units) {
-          const int64_t gn = (int64_t)(wn % BH) * Lq + min(unit_tile(wn) * kQTile + row, Lq - 1);
+          const int64_t gn = (int64_t)(wn % BH) * Lq + (kWhole ? unit_tile(wn) * kQTile + row : min(unit_tile(wn) * kQTile + row, Lq - 1));
           nM = M_ptr[gn];
           nL = L_ptr[gn];
         }
@@ -1355,12 +1357,12 @@ int device_facts(const DeviceFacts** out) {
     LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<false, 128>, attr, (int)kSmemFwd2));
     LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<true, 64>, attr, (int)kSmemFwd2));
     LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<false, 64>, attr, (int)kSmemFwd2));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<true, 128>, attr, (int)kSmemDq));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<false, 128>, attr, (int)kSmemDq));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<true, 64>, attr, (int)kSmemDq));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<false, 64>, attr, (int)kSmemDq));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<true>, attr, (int)kSmemDkv));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<false>, attr, (int)kSmemDkv));
+#define LMK_BWD_ATTR(BF, DIM, WHOLE)                                                                \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, WHOLE>, attr, (int)kSmemDq));        \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, WHOLE>, attr, (int)kSmemDkv));
+    LMK_BWD_ATTR(true, 128, true) LMK_BWD_ATTR(true, 128, false) LMK_BWD_ATTR(true, 64, true) LMK_BWD_ATTR(true, 64, false)
+    LMK_BWD_ATTR(false, 128, true) LMK_BWD_ATTR(false, 128, false) LMK_BWD_ATTR(false, 64, true) LMK_BWD_ATTR(false, 64, false)
+#undef LMK_BWD_ATTR
     f.ready = true;
   }
   *out = &f;
@@ -1486,18 +1488,28 @@ int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
   const float* Mc = p.M;
   const float* deltac = delta;
   const int BH = p.B * p.H;
-#define LMK_BWD_LAUNCH(BF, DIM)                                                                                          \
-  do {                                                                                                                   \
-    LMK_CUDA(cudaLaunchKernelEx(&cfg_dq, sm100_bwd_dq_kernel<BF, DIM>, tq, tk, tv, tdo, to, Lc, Mc, delta, p.dq, p.H,    \
-                                BH, p.Lq, p.Lk, p.D, p.scale, scale_log2));                                              \
-    LMK_CUDA(cudaLaunchKernelEx(&cfg_dkv, sm100_bwd_dkv_kernel<BF>, tq, tk, tv, tdo, Lc, Mc, deltac, p.dk, p.dv,         \
-                                p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2));                                         \
+#define LMK_BWD_LAUNCH(BF, DIM, DQ_WHOLE, DKV_WHOLE)                                                                       \
+  do {                                                                                                                     \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg_dq, sm100_bwd_dq_kernel<BF, DIM, DQ_WHOLE>, tq, tk, tv, tdo, to, Lc, Mc, delta, p.dq, \
+                                p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2));                                           \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg_dkv, sm100_bwd_dkv_kernel<BF, DKV_WHOLE>, tq, tk, tv, tdo, Lc, Mc, deltac, p.dk,      \
+                                p.dv, p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2));                                     \
   } while (0)
-  if (dtype == LMK_BF16) {
-    if (p.D <= 64) LMK_BWD_LAUNCH(true, 64); else LMK_BWD_LAUNCH(true, 128);
-  } else {
-    if (p.D <= 64) LMK_BWD_LAUNCH(false, 64); else LMK_BWD_LAUNCH(false, 128);
-  }
+#define LMK_BWD_DTYPE(BF)                                                      \
+  do {                                                                         \
+    if (p.D <= 64) {                                                           \
+      if (whole && p.D == 64) LMK_BWD_LAUNCH(BF, 64, true, false);             \
+      else LMK_BWD_LAUNCH(BF, 64, false, false);                               \
+    } else {                                                                   \
+      if (whole && p.D == 128) LMK_BWD_LAUNCH(BF, 128, true, true);            \
+      else LMK_BWD_LAUNCH(BF, 128, false, false);                              \
+    }                                                                          \
+  } while (0)
+  // instances without bounds where every tile is whole (the checks and run-time strides cost 8 us of 147 at L = 2048)
+  const bool whole = p.Lq % kQTile == 0 && p.Lk % kBlk == 0;
+  if (dtype == LMK_BF16) LMK_BWD_DTYPE(true);
+  else LMK_BWD_DTYPE(false);
+#undef LMK_BWD_DTYPE
 #undef LMK_BWD_LAUNCH
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
