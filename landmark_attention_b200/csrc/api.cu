@@ -55,7 +55,9 @@ void fill(AttnParams& p, const void* q, const void* k, const void* v, int B, int
   }
 }
 
-// 1 = general, 2 = tcgen05, <0 = error.  LMK_PATH_AUTO takes the tcgen05 kernels when the problem (16-bit type, block 64) AND
+constexpr int kPathSmallBlocks = 3;
+
+// 1 = general, 2 = tcgen05, 3 = tcgen05 with blocks below 64, <0 = error.  LMK_PATH_AUTO takes the tcgen05 kernels when the problem (16-bit type, block 64) AND
 // the operands (alignment, strides) qualify, and the general kernels otherwise; an explicit LMK_PATH_TCGEN05 request asks
 // for whole tiles of head dim 128 and is an error where that cannot be met.
 int pick_path(int path, const AttnParams& p, int dtype, bool backward) {
@@ -74,6 +76,9 @@ int pick_path(int path, const AttnParams& p, int dtype, bool backward) {
     return LMK_PATH_TCGEN05;
   }
   if (path == LMK_PATH_AUTO && fast) return LMK_PATH_TCGEN05;
+  if (path == LMK_PATH_AUTO && p.scale > 0.f && attn_sm100_small_blocks(p.B, p.H, p.Lq, p.Lk, p.D, p.block, dtype) &&
+      attn_sm100_operands_ok(p, backward))
+    return kPathSmallBlocks;
   const int block = p.block;
   if (block > 128) return fail(LMK_ERR_UNSUPPORTED, "general path supports block sizes up to 128 (got %d)", block);
   return LMK_PATH_GENERAL;
@@ -128,6 +133,7 @@ extern "C" int lmk_attn_fwd(const void* q, const void* k, const void* v, void* o
   int which = pick_path(path, p, dtype, false);
   if (which < 0) return which;
   if (which == LMK_PATH_TCGEN05) return attn_sm100_fwd(p, dtype, (cudaStream_t)stream);
+  if (which == kPathSmallBlocks) return attn_sm100_small_blocks_fwd(p, dtype, (cudaStream_t)stream);
   return attn_general_fwd(p, dtype, (cudaStream_t)stream);
 }
 
@@ -154,9 +160,9 @@ extern "C" int lmk_attn_bwd(const void* q, const void* k, const void* v, const v
   p.o = const_cast<void*>(o); p.dO = dO;
   int which = pick_path(path, p, dtype, true);
   if (which < 0) return which;
-  LMK_CHECK_ARG(which == LMK_PATH_TCGEN05 || (Lq % block == 0 && Lk % block == 0),
+  LMK_CHECK_ARG(which != LMK_PATH_GENERAL || (Lq % block == 0 && Lk % block == 0),
                 "Backward supported only for full blocks (Lq=%d Lk=%d block=%d)", Lq, Lk, block);
-  const size_t need = lmk_attn_bwd_workspace(B, H, Lq, Lk, D, block, dtype, which);
+  const size_t need = lmk_attn_bwd_workspace(B, H, Lq, Lk, D, block, dtype, which == kPathSmallBlocks ? LMK_PATH_TCGEN05 : which);
   if (need > 0 && (workspace == nullptr || workspace_bytes < need))
     return fail(LMK_ERR_WORKSPACE, "attn_bwd: workspace of %zu bytes required, %zu given", need, workspace_bytes);
   LMK_CHECK_ARG(((uintptr_t)workspace & 255) == 0, "attn_bwd: workspace must be 256-byte aligned");
@@ -164,6 +170,7 @@ extern "C" int lmk_attn_bwd(const void* q, const void* k, const void* v, const v
   p.dq = dQ; p.dk = dK; p.dv = dV;
   p.workspace = workspace; p.workspace_bytes = workspace_bytes;
   if (which == LMK_PATH_TCGEN05) return attn_sm100_bwd(p, dtype, (cudaStream_t)stream);
+  if (which == kPathSmallBlocks) return attn_sm100_small_blocks_bwd(p, dtype, (cudaStream_t)stream);
   p.delta = reinterpret_cast<float*>(workspace);
   return attn_general_bwd(p, dtype, (cudaStream_t)stream);
 }

@@ -161,7 +161,9 @@ __global__ void __launch_bounds__(kMfThreads, 2)
 sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const uint8_t* __restrict__ is_mem, int64_t is_mem_stride,
                       void* __restrict__ o_ptr, float* __restrict__ R_ptr, float* __restrict__ A_ptr, int H, int Lq,
-                      int Lk, int G, float scale_log2, int* status) {
+                      int Lk, int G, float scale_log2, int only_marked, int* status) {
+  // behind the single-pass kernel: only the tiles that it left (see attn_sm100.cu)
+  if (only_marked && R_ptr[(int64_t)blockIdx.x * Lq + (Lq / kQT - 1 - (int)blockIdx.y) * kQT] != -INFINITY) return;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -461,7 +463,9 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
                          const void* __restrict__ do_ptr, const float* __restrict__ R_ptr,
                          const float* __restrict__ A_ptr, float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
                          void* __restrict__ dq_ptr, int H, int Lq, int Lk, int G, float scale, float scale_log2,
-                         int* status) {
+                         const int* __restrict__ plan, int plan_stride, int* status) {
+  if (plan != nullptr && plan[(int64_t)(blockIdx.x / H) * plan_stride + 1] == 0) return;      // the single-pass kernels' rows
+
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -752,7 +756,9 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                           const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const float* __restrict__ R_ptr,
                           const float* __restrict__ A_ptr, const float* __restrict__ delta_ptr,
                           const float* __restrict__ nD_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                          int H, int Lq, int Lk, int G, float scale, float scale_log2, int* status) {
+                          int H, int Lq, int Lk, int G, float scale, float scale_log2, const int* __restrict__ plan, int plan_stride, int* status) {
+  if (plan != nullptr && plan[(int64_t)(blockIdx.x / H) * plan_stride + 1] == 0) return;      // the single-pass kernels' rows
+
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -1099,20 +1105,24 @@ int attn_mask_sm100_fwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
   int* status = device_status_word();
   if (!status) return fail(LMK_ERR_CUDA, "cannot resolve the device status word");
   const float scale_log2 = p.scale * kLog2e;
+  // Groups of up to 64 keys run on the single-pass kernels (51-key groups at B16 H8 T512: 51 -> 21 us); what these leave, and
+  // lengths that cannot consist of such groups, on the two-pass kernels here.
+  const int only_marked = attn_sm100_flags(p.Lk, G) && p.scale > 0.f;
+  if (only_marked && (rc = attn_sm100_flags_fwd(p, is_mem, is_mem_stride, G, R, dtype, st)) != LMK_OK) return rc;
   dim3 grid(p.B * p.H, p.Lq / kQT);
   const size_t smem = mf_smem_bytes(G, p.Lk / kKT);
   if (dtype == LMK_BF16)
     sm100_mask_fwd_kernel<true><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.Lq,
-                                                                 p.Lk, G, scale_log2, status);
+                                                                 p.Lk, G, scale_log2, only_marked, status);
   else
     sm100_mask_fwd_kernel<false><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.Lq,
-                                                                  p.Lk, G, scale_log2, status);
+                                                                  p.Lk, G, scale_log2, only_marked, status);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }
 
 size_t attn_mask_sm100_bwd_workspace(int B, int H, int Lq, int G) {
-  return sizeof(float) * ((size_t)B * H * Lq + (size_t)B * H * G * Lq);      // delta, nD
+  return sizeof(float) * ((size_t)B * H * Lq + (size_t)B * H * G * Lq) + attn_sm100_plan_bytes(B);      // delta, nD, plan
 }
 
 int attn_mask_sm100_bwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_mem_stride, const float* R,
@@ -1136,14 +1146,21 @@ int attn_mask_sm100_bwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
   const float scale_log2 = p.scale * kLog2e;
   dim3 grid_q(p.B * p.H, p.Lq / kQT), grid_k(p.B * p.H, p.Lk / kKT);
   const size_t smem_q = mq_smem_bytes(G);
+  const int* plan = nullptr;
+  const int plan_stride = attn_sm100_plan_stride();
+  if (attn_sm100_flags(p.Lk, G) && p.scale > 0.f) {
+    int* records = reinterpret_cast<int*>(nD + (size_t)p.B * p.H * G * p.Lq);
+    if ((rc = attn_sm100_flags_bwd(p, is_mem, is_mem_stride, G, R, records, dtype, st)) != LMK_OK) return rc;
+    plan = records;
+  }
 #define LMK_MASK_BWD(BF)                                                                                                \
   do {                                                                                                                  \
     sm100_mask_bwd_dq_kernel<BF><<<grid_q, kMqThreads, smem_q, st>>>(tq, tk, tv, tdo, is_mem, is_mem_stride, p.o, p.dO,  \
                                                                      R, A, delta, nD, p.dq, p.H, p.Lq, p.Lk, G,         \
-                                                                     p.scale, scale_log2, status);                      \
+                                                                     p.scale, scale_log2, plan, plan_stride, status);   \
     sm100_mask_bwd_dkv_kernel<BF><<<grid_k, kMkThreads, kMkSmemBytes, st>>>(tq, tk, tv, tdo, is_mem, is_mem_stride, R,  \
                                                                            A, delta, nD, p.dk, p.dv, p.H, p.Lq, p.Lk,   \
-                                                                           G, p.scale, scale_log2, status);             \
+                                                                           G, p.scale, scale_log2, plan, plan_stride, status); \
   } while (0)
   if (dtype == LMK_BF16) LMK_MASK_BWD(true);
   else LMK_MASK_BWD(false);

@@ -32,6 +32,16 @@ void attn_sm100_set_max_ctas(int n);
 int attn_sm100_fwd(const AttnParams& p, int dtype, cudaStream_t st);
 int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st);
 size_t attn_sm100_bwd_workspace(int B, int H, int Lq, int Lk, int D);
+// regular blocks below 64 keys, and landmarks anywhere in groups of up to 64 keys (see attn_sm100.cu)
+bool attn_sm100_small_blocks(int B, int H, int Lq, int Lk, int D, int block, int dtype);
+int attn_sm100_small_blocks_fwd(const AttnParams& p, int dtype, cudaStream_t st);
+int attn_sm100_small_blocks_bwd(const AttnParams& p, int dtype, cudaStream_t st);
+bool attn_sm100_flags(int Lk, int G);
+int attn_sm100_flags_fwd(const AttnParams& p, const uint8_t* flags, int64_t stride, int G, float* R, int dtype, cudaStream_t st);
+int attn_sm100_flags_bwd(const AttnParams& p, const uint8_t* flags, int64_t stride, int G, const float* R, int* plan, int dtype,
+                         cudaStream_t st);
+size_t attn_sm100_plan_bytes(int B);
+int attn_sm100_plan_stride();
 int device_status(int* out, int clear);
 int* device_status_word();
 

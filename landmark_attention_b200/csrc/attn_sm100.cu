@@ -117,6 +117,129 @@ __device__ __forceinline__ float row_sum(const float (&v)[64]) {
   return (a + b) + (c + d);
 }
 
+// ---------------------------------------------------------------------------------------------- other landmark patterns
+// Instances with kIrr take landmark groups of any length up to 64 keys: a regular pattern with blocks below 64, or landmarks
+// anywhere, given as one flag per (batch row, key).  The key tiles are then the GROUPS: tile n is the 64 keys that end with
+// the group's landmark (TMA has no alignment rule for rows; rows in front of the sequence read as zeros), so the landmark
+// is in column 63 as in the block-64 pattern and the first c0 columns, which belong to the group before, are hidden.  Each key
+// belongs to one tile, softmax inside a group never leaves a tile, and the kernels stay single-pass: 51-key groups use 80 % of
+// the columns and still take half the time of two passes over aligned tiles.  The keys behind the last landmark form the
+// last tile, which ends at a position of its own.
+// Rows whose groups do not fit (longer than 64 keys, or so short that tiles would be mostly empty) are left to the two-pass
+// kernels of attn_mask_sm100.cu: the forward kernel marks them in R, the backward ones find them in the plan.
+constexpr int kIrrMaxTiles = 65;                    // 64 landmarks and the open group
+constexpr int kIrrMaxKeys = 64 * kIrrMaxTiles;
+constexpr int kIrrMinMeanGroup = 16;
+
+struct IrrArgs {
+  const uint8_t* flags = nullptr;      // [B, Lk] or null: the regular pattern with `block`
+  int64_t stride = 0;
+  int block = 0, G = 0;
+  const int* plan = nullptr;           // backward, flags only: see irr_plan_kernel
+  float* R = nullptr;                  // flags only: log2 of the row's normaliser instead of L and M
+};
+
+// landmark positions and per-key landmark counts of one batch row, in shared memory
+struct IrrSmem {
+  uint64_t kmask[kIrrMaxTiles + 1];    // bit j of word w: key 64 w + j is a landmark
+  int gbase[kIrrMaxTiles + 1];         // landmarks before word w
+  int ends[kIrrMaxTiles + 1];          // position of column 63 of tile n
+  int n_lm;
+  int fallback;
+};
+__device__ __forceinline__ int irr_group(const IrrSmem& t, int pos) {          // landmarks strictly before pos
+  return t.gbase[pos >> 6] + __popcll(t.kmask[pos >> 6] & ((1ull << (pos & 63)) - 1ull));
+}
+// All threads of the CTA; contains __syncthreads().
+__device__ __forceinline__ void irr_build(IrrSmem& t, const uint8_t* __restrict__ flags, int Lk, int G) {
+  const int words = (Lk + 63) / 64, warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int w = warp; w < words; w += warps) {
+    const int k0 = w * 64 + lane;
+    const unsigned lo = __ballot_sync(0xffffffffu, k0 < Lk && flags[k0] != 0);
+    const unsigned hi = __ballot_sync(0xffffffffu, k0 + 32 < Lk && flags[k0 + 32] != 0);
+    if (lane == 0) t.kmask[w] = (uint64_t)lo | ((uint64_t)hi << 32);
+  }
+  if (threadIdx.x == 0) t.fallback = 0;
+  __syncthreads();
+  if (warp == 0) {                     // exclusive prefix sums of the words' counts, three words a lane
+    int c[3], sum = 0;
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const int w = lane * 3 + e;
+      c[e] = w < words ? __popcll(t.kmask[w]) : 0;
+      sum += c[e];
+    }
+    int inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    int run = inc - sum;
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const int w = lane * 3 + e;
+      if (w < words) t.gbase[w] = run;
+      run += c[e];
+    }
+    if (lane == 31) t.n_lm = run;
+  }
+  __syncthreads();
+  const int n_lm = t.n_lm;
+  const bool too_many = irr_group(t, Lk - 1) > min(G, kIrrMaxTiles - 1) || kIrrMinMeanGroup * (n_lm + 1) > Lk + 256;
+  if (threadIdx.x < words && !too_many) {
+    uint64_t m = t.kmask[threadIdx.x];
+    int n = t.gbase[threadIdx.x];
+    while (m) {
+      const int j = __ffsll((long long)m) - 1;
+      t.ends[n++] = threadIdx.x * 64 + j;
+      m &= m - 1;
+    }
+  }
+  if (threadIdx.x == 0) {
+    if (!too_many) t.ends[n_lm] = Lk;
+    else t.fallback = 1;
+  }
+  __syncthreads();
+  if (!too_many && threadIdx.x <= n_lm && t.ends[threadIdx.x] - (threadIdx.x ? t.ends[threadIdx.x - 1] : -1) > 64)
+    if (threadIdx.x < n_lm || n_lm == 0 || t.ends[n_lm - 1] + 1 < Lk) t.fallback = 1;       // (an empty open group is no group)
+  __syncthreads();
+}
+
+// The same table in global memory for the backward kernels, one record per batch row: [0] landmarks, [1] fallback, [2 ...]
+// ends, then one byte per key with its group.
+constexpr int kIrrPlanHead = 2 + kIrrMaxTiles + 1;
+constexpr int kIrrPlanInts = kIrrPlanHead + (kIrrMaxKeys + 3) / 4;
+__device__ __forceinline__ bool irr_plan_fallback(const int* plan, int b) { return __ldg(plan + (int64_t)b * kIrrPlanInts + 1) != 0; }
+__device__ __forceinline__ int irr_plan_end(const int* plan, int b, int n) { return __ldg(plan + (int64_t)b * kIrrPlanInts + 2 + n); }
+__device__ __forceinline__ int irr_plan_group(const int* plan, int b, int pos) {
+  return __ldg(reinterpret_cast<const uint8_t*>(plan + (int64_t)b * kIrrPlanInts + kIrrPlanHead) + pos);
+}
+__global__ void __launch_bounds__(256) irr_plan_kernel(const uint8_t* __restrict__ flags, int64_t stride, int Lk, int G, int* plan) {
+  __shared__ IrrSmem t;
+  const int b = blockIdx.x;
+  irr_build(t, flags + (int64_t)b * stride, Lk, G);
+  int* p = plan + (int64_t)b * kIrrPlanInts;
+  if (threadIdx.x == 0) {
+    p[0] = t.n_lm;
+    p[1] = t.fallback;
+  }
+  if (t.fallback) return;
+  for (int n = threadIdx.x; n <= t.n_lm; n += blockDim.x) p[2 + n] = t.ends[n];
+  uint8_t* own = reinterpret_cast<uint8_t*>(p + kIrrPlanHead);
+  for (int k = threadIdx.x; k < Lk; k += blockDim.x) own[k] = (uint8_t)irr_group(t, k);
+}
+
+// hides the columns of the group before: uniform tests, selects only in the chunks that need them
+__device__ __forceinline__ void irr_hide(float (&sv)[64], int c0) {
+#pragma unroll
+  for (int ch = 0; ch < 8; ++ch)
+    if (c0 > 8 * ch) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sv[8 * ch + e] = 8 * ch + e < c0 ? -INFINITY : sv[8 * ch + e];
+    }
+}
+
 // ---------------------------------------------------------------------------------------------- forward, two tiles
 // Up to TWO adjacent 128-row query tiles per CTA (one CTA per SM): softmax warpgroup 0 owns tile A
 // (rows 256u .. 256u+127), warpgroup 1 owns tile B (the next 128 rows).  Both tiles consume the same K/V stream, so
@@ -136,17 +259,18 @@ struct Fwd2Smem {
   uint64_t empty[kFwd2Stages];
   uint64_t s_full[2][2];    // [tile][S buffer]
   uint64_t s_free[2][2];
-  uint64_t p_ready[2];
+  uint64_t p_ready[2][2];   // [tile][buffer]: a warp whose rows have little to do can be one item ahead of the others
   uint64_t o_full;
   uint32_t tmem_base;
 };
 
-template <bool kBf16, int kD>
+template <bool kBf16, int kD, bool kIrr>
 __global__ void __launch_bounds__(kFwd2Threads, 1)
 sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_klm,
                   void* __restrict__ o_ptr, float* __restrict__ L_ptr, float* __restrict__ M_ptr, int H, int Lq, int Lk,
-                  int D, int lm_box, int per_cta, float scale_log2) {
+                  int D, int lm_box, int per_cta, float scale_log2, const void* __restrict__ k_ptr, int64_t ks_b, int64_t ks_h,
+                  int64_t ks_row, IrrArgs irr) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -160,12 +284,28 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const bool has_b = per_cta == 2 && (t_a + 1) * kQTile < Lq;            // the second tile has at least one row
   const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
   const int prefix_blocks = (Lk - Lq) / kBlk;
+  const int pos_a = Lk - Lq + t_a * kQTile;             // key position of tile A's first row
+  IrrSmem* tab = reinterpret_cast<IrrSmem*>(sm + 1);
+  if constexpr (kIrr) {
+    if (irr.flags != nullptr) {
+      irr_build(*tab, irr.flags + (int64_t)b * irr.stride, Lk, irr.G);
+      if (tab->fallback) {                              // uniform; the two-pass kernel takes the tiles marked here
+        if (tid < 2 && (tid == 0 || has_b)) irr.R[(int64_t)bh * Lq + (t_a + tid) * kQTile] = -INFINITY;
+        return;
+      }
+    }
+  }
+  auto group_of = [&](int pos) { return irr.flags != nullptr ? irr_group(*tab, pos) : pos / irr.block; };
+  auto end_of = [&](int n) { return irr.flags != nullptr ? (n < 0 ? -1 : tab->ends[n]) : (n + 1) * irr.block - 1; };
   const int own0_a = prefix_blocks + 2 * t_a;           // tile A: blocks own0_a, own0_a+1; tile B: +2, +3
-  const int n_last = min(own0_a + (has_b ? 3 : 1), (Lk - 1) / kBlk);     // newest block that any row of the CTA sees
+  // newest tile that any row of tile A / of the CTA sees
+  const int last_a = kIrr ? group_of(min(pos_a + kQTile, Lk) - 1) : own0_a + 1;
+  const int n_last = kIrr ? group_of(min(pos_a + (has_b ? 2 : 1) * kQTile, Lk) - 1)
+                          : min(own0_a + (has_b ? 3 : 1), (Lk - 1) / kBlk);
   const int n_lm_tiles = (n_last + 63) / 64;            // landmarks 0 .. n_last-1
   const int total = n_lm_tiles + n_last + 1;
   // tile A takes part in every item but the main items of tile B's own blocks
-  auto active = [&](int w, int i) { return w == 1 ? has_b : (i < n_lm_tiles || n_last - (i - n_lm_tiles) <= own0_a + 1); };
+  auto active = [&](int w, int i) { return w == 1 ? has_b : (i < n_lm_tiles || n_last - (i - n_lm_tiles) <= last_a); };
 
   if (tid == 0) {
     mbar_init(smem_u32(&sm->q_full), 1);
@@ -177,8 +317,8 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       for (int s = 0; s < 2; ++s) {
         mbar_init(smem_u32(&sm->s_full[w][s]), 1);
         mbar_init(smem_u32(&sm->s_free[w][s]), 1);
+        mbar_init(smem_u32(&sm->p_ready[w][s]), 128);
       }
-      mbar_init(smem_u32(&sm->p_ready[w]), 128);
     }
     mbar_init(smem_u32(&sm->o_full), 1);
     mbar_init_fence();
@@ -208,16 +348,18 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         const int s = i % kFwd2Stages;
         mbar_wait(smem_u32(&sm->empty[s]), ((i / kFwd2Stages) & 1) ^ 1, &g_lmk_status, kErrFwd2Producer);
         const uint32_t fb = smem_u32(&sm->full[s]);
+        if (kIrr && i < n_lm_tiles) continue;           // the softmax warps gather the landmark keys themselves
         if (i < n_lm_tiles) {
           mbar_arrive_expect_tx(fb, (uint32_t)(lm_box * kD * 2));
           for (int c = 0; c < kD / 64; ++c)
             tma_load_5d(k_slot(s) + c * kHalfTile, &tm_klm, fb, 64 * c, kBlk - 1, i * 64, h, b);
         } else {
           const int n = n_last - (i - n_lm_tiles);
+          const int r0 = kIrr ? end_of(n) - 63 : n * kBlk;
           mbar_arrive_expect_tx(fb, 2 * (kD / 64) * kHalfTile);
           for (int c = 0; c < kD / 64; ++c) {
-            tma_load_4d(k_slot(s) + c * kHalfTile, &tm_k, fb, 64 * c, n * kBlk, h, b);
-            tma_load_4d(v_slot(s) + c * kHalfTile, &tm_v, fb, 64 * c, n * kBlk, h, b);
+            tma_load_4d(k_slot(s) + c * kHalfTile, &tm_k, fb, 64 * c, r0, h, b);
+            tma_load_4d(v_slot(s) + c * kHalfTile, &tm_v, fb, 64 * c, r0, h, b);
           }
         }
       }
@@ -271,7 +413,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         for (int w = 0; w < 2; ++w) {
           if (!active(w, i)) continue;
           const int k = kp[w]++;
-          mbar_wait(smem_u32(&sm->p_ready[w]), k & 1, &g_lmk_status, kErrFwd2Mma);
+          mbar_wait(smem_u32(&sm->p_ready[w][k & 1]), (k >> 1) & 1, &g_lmk_status, kErrFwd2Mma);
           tc_fence_after();
           if (i >= n_lm_tiles) {
             // A = P straight from TMEM: the softmax threads wrote it over the first 32 columns of the S buffer it was
@@ -297,16 +439,31 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int w = warp >> 2;                       // 0: tile A, 1: tile B
     const int row = tid & 127;
     const int half = row >> 6;
-    const int own = own0_a + 2 * w + half;
-    const int vis = min(row & 63, kBlk - 2);
+    const int pos = min(pos_a + w * kQTile + row, Lk - 1);
+    const int own = kIrr ? group_of(pos) : own0_a + 2 * w + half;
+    const int vis = min(kIrr ? 63 - (end_of(own) - pos) : row & 63, kBlk - 2);
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     float m2 = -INFINITY, l = 0.f;
     int k = 0;
+    if (kIrr && n_lm_tiles > 0) {                  // landmark keys of tiles 0 .. n_last-1 -> rows of the first stage
+      const uint16_t* kb = reinterpret_cast<const uint16_t*>(k_ptr) + b * ks_b + h * ks_h;
+      for (int e = tid; e < n_last * (kD / 8); e += 256) {
+        const int n = e / (kD / 8), c = e - n * (kD / 8);
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (c * 8 < D) x = *reinterpret_cast<const uint4*>(kb + (int64_t)end_of(n) * ks_row + c * 8);
+        const uint32_t addr = k_slot(0) + (uint32_t)(c >> 3) * kHalfTile + (uint32_t)n * 128u + (uint32_t)(((c & 7) ^ (n & 7)) << 4);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
+      }
+      fence_proxy_async_smem();
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (tid == 0) mbar_arrive(smem_u32(&sm->full[0]));
+    }
     for (int i = 0; i < total; ++i) {
       if (!active(w, i)) continue;
       const int sb = k & 1;
       mbar_wait(smem_u32(&sm->s_full[w][sb]), (k / 2) & 1, &g_lmk_status, kErrFwd2Softmax);
       tc_fence_after();
+      if (kIrr) __syncwarp();
       float sv[64];
       {
         uint32_t ra[32], rb[32];
@@ -326,10 +483,34 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       } else {
         const int n = n_last - (i - n_lm_tiles);
         write_p = true;
-        if (n > own) {
+        // With kIrr the rows of a warp can stand differently to tile n; every branch is taken by whole warps all the same
+        // (votes), because the TMEM accesses behind it have to be executed by all lanes together.
+        bool later = n > own, mixed = false;
+        if constexpr (kIrr) {
+          const int c0 = 64 - (end_of(n) - end_of(n - 1));
+          irr_hide(sv, c0);
+          later = __all_sync(0xffffffffu, n > own);
+          mixed = !later && (c0 == 63 || !__all_sync(0xffffffffu, n < own));      // (c0 == 63: a landmark without keys)
+        }
+        if (later) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) wgt[j] = 0u;
-        } else if (n == own) {
+        } else if (kIrr && mixed) {
+          const bool earlier = n < own;
+          const int last = earlier ? kBlk - 2 : (n == own ? vis : -1);
+          const float mx = row_max_upto(sv, last) * scale_log2;
+          if (n == own) m2 = fmaxf(m2, mx);
+          const float el = earlier ? ex2(fmaf(sv[63], scale_log2, -m2)) : 0.f;
+          float shift = earlier ? mx : m2;
+          shift = shift == -INFINITY ? 0.f : shift;                               // nothing visible
+#pragma unroll
+          for (int j = 0; j < 64; ++j) sv[j] = (j <= last) ? ex2(fmaf(sv[j], scale_log2, -shift)) : 0.f;
+          const float sum = row_sum<64>(sv);
+          const float wg = earlier ? (sum > 0.f ? __fdividef(el, sum) : 0.f) : 1.f;
+          l += earlier ? el : sum;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) wgt[j] = pack2<kBf16>(sv[2 * j] * wg, sv[2 * j + 1] * wg);
+        } else if (!kIrr && n == own) {
           m2 = fmaxf(m2, row_max_upto(sv, vis) * scale_log2);
 #pragma unroll
           for (int j = 0; j < 64; ++j) sv[j] = (j <= vis) ? ex2(fmaf(sv[j], scale_log2, -m2)) : 0.f;
@@ -378,13 +559,13 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         tmem_st_wait();
       }
       tc_fence_before();
-      mbar_arrive(smem_u32(&sm->p_ready[w]));
+      mbar_arrive(smem_u32(&sm->p_ready[w][sb]));
       ++k;
     }
     // ------------------------------------------------------------------ epilogue
     mbar_wait(smem_u32(&sm->o_full), 0, &g_lmk_status, kErrFwd2Epilogue);
     tc_fence_after();
-    const float inv = 1.f / l;
+    const float inv = kIrr && l == 0.f ? 0.f : 1.f / l;
     const int grow = (t_a + w) * kQTile + row;
     const bool stored = grow < Lq && (w == 0 || has_b);
     uint4* orow = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(o_ptr) + ((int64_t)bh * Lq + grow) * D);
@@ -406,8 +587,12 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
     }
     if (stored) {
-      L_ptr[(int64_t)bh * Lq + grow] = l;
-      M_ptr[(int64_t)bh * Lq + grow] = m2 * (1.f / kLog2e);
+      if (kIrr && irr.R != nullptr) {
+        irr.R[(int64_t)bh * Lq + grow] = l > 0.f ? m2 + __log2f(l) : INFINITY;
+      } else {
+        L_ptr[(int64_t)bh * Lq + grow] = l;
+        M_ptr[(int64_t)bh * Lq + grow] = m2 * (1.f / kLog2e);
+      }
     }
     tc_fence_before();
   }
@@ -446,12 +631,14 @@ __device__ __forceinline__ uint32_t pack2p(uint64_t v) {
   return pack2<kBf16>(lo, hi);
 }
 
+// With kIrr the rows of a warp can be of different kinds (groups end anywhere).  The TMEM accesses have to be executed by all lanes
+// of a warp together, so nothing branches on `kind` there: mixed warps take one masked pass with per-row limits and shifts.
 // M2L = (row max + log(row sum)) * log2(e): exp2(s * c - M2L) is the outer-softmax probability.
 // S and dP are each read from TMEM once and held as packed pairs; dP's buffer is released (free_bar) as soon as it is
 // in registers, before the reductions, so the next dP product can start early.
-template <bool kBf16, bool kNeedP, typename WaitFn, typename AfterSFn = NoHook, typename BeforeDpFn = NoHook,
+template <bool kBf16, bool kNeedP, bool kIrr, typename WaitFn, typename AfterSFn = NoHook, typename BeforeDpFn = NoHook,
           typename BetweenFn = NoHook>
-__device__ __forceinline__ void bwd_item(uint32_t ts, uint32_t tdp, uint32_t free_bar, int kind, int vis, float c,
+__device__ __forceinline__ void bwd_item(int c0, uint32_t ts, uint32_t tdp, uint32_t free_bar, int kind, int vis, float c,
                                          float scale, float M2L, float delta, uint32_t p_dst, uint32_t ds_dst, int row,
                                          WaitFn wait_dst, AfterSFn after_s = AfterSFn(),
                                          BeforeDpFn before_dp = BeforeDpFn(),
@@ -459,12 +646,26 @@ __device__ __forceinline__ void bwd_item(uint32_t ts, uint32_t tdp, uint32_t fre
   uint64_t sp[32];      // the row as packed pairs: S, then P
   uint64_t dp[32];      // dP, then dS
   float nmx = 0.f, lm2 = 0.f;
+  if (kIrr) __syncwarp();
   {
     uint32_t ra[32], rb[32];
     tmem_ld_32x32b_x32(ts, ra);
     tmem_ld_32x32b_x32(ts + 32, rb);
     tmem_ld_wait();
-    if (kind == 2) {
+    if constexpr (kIrr) {             // the first c0 columns belong to the group before (uniform tests, see irr_hide)
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) {
+        if (c0 > 8 * ch) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) ra[8 * ch + e] = 8 * ch + e < c0 ? 0xff800000u : ra[8 * ch + e];
+        }
+        if (c0 > 32 + 8 * ch) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) rb[8 * ch + e] = 32 + 8 * ch + e < c0 ? 0xff800000u : rb[8 * ch + e];
+        }
+      }
+    }
+    if (kIrr || kind == 2) {
       float sv[64];
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
@@ -473,6 +674,7 @@ __device__ __forceinline__ void bwd_item(uint32_t ts, uint32_t tdp, uint32_t fre
       }
       nmx = -row_max<63>(sv) * c;
       lm2 = sv[63] * c;
+      if (kIrr && c0 == 63) nmx = 0.f;      // no key but the landmark
     }
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -484,10 +686,26 @@ __device__ __forceinline__ void bwd_item(uint32_t ts, uint32_t tdp, uint32_t fre
   float sub = delta, lm_ds = 0.f, pscale = 1.f;
   const uint64_t c2 = pk2(c, c);
   uint64_t s0 = 0ull, s1 = 0ull, s2 = 0ull, s3 = 0ull;
-  if (kind == 0) {
+  // all rows of the warp are of kind 2 and the group has keys (votes: the branches below are taken by whole warps)
+  const bool fast = kIrr && c0 != 63 && __all_sync(0xffffffffu, kind == 2);
+  if (kIrr && !fast) {
+    const int last = kind == 2 ? kBlk - 2 : (kind == 1 ? vis : -1);
+    const float shift = kind == 2 ? nmx : -M2L;
+    const uint64_t m2 = pk2(shift, shift);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      float a, b;
+      upk2(fma2(sp[j], c2, m2), a, b);
+      sp[j] = pk2(2 * j <= last ? ex2(a) : 0.f, 2 * j + 1 <= last ? ex2(b) : 0.f);
+      if (j % 4 == 0) s0 = add2(s0, sp[j]);
+      if (j % 4 == 1) s1 = add2(s1, sp[j]);
+      if (j % 4 == 2) s2 = add2(s2, sp[j]);
+      if (j % 4 == 3) s3 = add2(s3, sp[j]);
+    }
+  } else if (!kIrr && kind == 0) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) sp[j] = 0ull;
-  } else if (kind == 1) {
+  } else if (!kIrr && kind == 1) {
     const uint64_t m2 = pk2(-M2L, -M2L);
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
@@ -518,7 +736,8 @@ __device__ __forceinline__ void bwd_item(uint32_t ts, uint32_t tdp, uint32_t fre
     }
   }
   before_dp();    // a caller with separate S / dP buffers waits for dP only now, after the exponentials
-  if (kind == 0) {
+  if (kIrr) __syncwarp();
+  if (!kIrr && kind == 0) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) dp[j] = 0ull;
   } else {
@@ -534,7 +753,7 @@ __device__ __forceinline__ void bwd_item(uint32_t ts, uint32_t tdp, uint32_t fre
   }
   tc_fence_before();
   mbar_arrive(free_bar);
-  if (kind == 2) {
+  if (kIrr || kind == 2) {
     uint64_t n0 = 0ull, n1 = 0ull, n2a = 0ull, n3 = 0ull;
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
@@ -546,10 +765,11 @@ __device__ __forceinline__ void bwd_item(uint32_t ts, uint32_t tdp, uint32_t fre
     float dl, dh, ql, qh;
     upk2(add2(add2(s0, s1), add2(s2, s3)), dl, dh);
     upk2(add2(add2(n0, n1), add2(n2a, n3)), ql, qh);
-    const float rden = __fdividef(1.f, dl + dh);
+    const bool grouped = !kIrr || kind == 2;       // the rest is selects
+    const float rden = kIrr && (c0 == 63 || !grouped) ? 0.f : __fdividef(1.f, dl + dh);
     const float nd = (ql + qh) * rden;
     const float g = ex2(lm2 - M2L);
-    const float w = g * rden;
+    const float w = grouped ? g * rden : 1.f;
     if (kNeedP) {
       const uint64_t w2 = pk2(w, w);
 #pragma unroll
@@ -557,7 +777,7 @@ __device__ __forceinline__ void bwd_item(uint32_t ts, uint32_t tdp, uint32_t fre
     } else {
       pscale = w;       // P itself is not stored: its row factor is folded into the dS coefficients below
     }
-    sub = nd;
+    sub = grouped ? nd : delta;
     lm_ds = g * (nd - delta) * scale;
   }
   // dS = P * (dP - sub) * scale = P * fma(dP, scale, -sub * scale)
@@ -626,13 +846,14 @@ struct DkvSmem {
 // the item written before have read it), which settles them half an item apart.
 // CTA c takes units w = round * grid + c with the direction alternating per round (snake), heaviest pairs first.
 // Loads, S/dP products and the softmax of the next unit start while the accumulators of the current one are drained.
-template <bool kBf16, bool kWhole>
+template <bool kBf16, bool kWhole, bool kIrr>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                      const float* __restrict__ L_ptr, const float* __restrict__ M_ptr,
                      const float* __restrict__ delta_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                     int H, int BH, int Lq, int Lk, int D_any, float scale, float scale_log2) {
+                     int H, int BH, int Lq, int Lk, int D_any, float scale, float scale_log2, int max_tiles,
+                     IrrArgs irr) {
   constexpr int kD = 128;
   const int D = kWhole ? kD : D_any;
   extern __shared__ uint8_t smem_raw[];
@@ -651,13 +872,28 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int prefix_blocks = (Lk - Lq) / kBlk;
   const int n_tiles = (Lq + kQTile - 1) / kQTile;
   const int n_blocks = (Lk + kBlk - 1) / kBlk;
-  const int n_pairs = (n_blocks + 1) / 2;
+  const int n_pairs = ((kIrr ? max_tiles : n_blocks) + 1) / 2;
   const int n_units = n_pairs * BH;
   auto unit_of = [&](int r) {
     const int c = (r & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
     return r * (int)gridDim.x + c;
   };
-  auto unit_tq0 = [&](int pair) { return 2 * pair > prefix_blocks ? (2 * pair - prefix_blocks) / 2 : 0; };
+  // kIrr: tile table of the unit's batch row (flags), or the regular pattern
+  auto group_of = [&](int b, int pos) { return irr.flags != nullptr ? irr_plan_group(irr.plan, b, pos) : pos / irr.block; };
+  auto end_of = [&](int b, int n) {
+    return n < 0 ? -1 : (irr.flags != nullptr ? irr_plan_end(irr.plan, b, n) : (n + 1) * irr.block - 1);
+  };
+  auto tiles_of = [&](int b) { return kIrr ? group_of(b, Lk - 1) + 1 : n_blocks; };
+  auto skipped = [&](int w) {
+    if constexpr (!kIrr) return false;
+    const int b = (w % BH) / H;
+    return (irr.flags != nullptr && irr_plan_fallback(irr.plan, b)) || 2 * (w / BH) >= tiles_of(b);
+  };
+  auto unit_tq0 = [&](int w) {                       // first query tile that sees the pair
+    const int pair = w / BH;
+    if constexpr (kIrr) return max(end_of((w % BH) / H, 2 * pair - 1) + 1 - (Lk - Lq), 0) / kQTile;
+    return 2 * pair > prefix_blocks ? (2 * pair - prefix_blocks) / 2 : 0;
+  };
 
   if (tid == 0) {
     mbar_init(smem_u32(&sm->kv_full), 1);
@@ -699,14 +935,16 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       prefetch_tensormap(&tm_v);
       prefetch_tensormap(&tm_do);
       int it = 0, u = 0;
-      for (int w = unit_of(0); w < n_units; w = unit_of(++u)) {
+      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+        if (skipped(w)) continue;
         const int pair = w / BH, bh = w - pair * BH, b = bh / H, h = bh - b * H;
-        const int tq0 = unit_tq0(pair), n_items = n_tiles - tq0;
+        const int tq0 = unit_tq0(w), n_items = n_tiles - tq0;
         const uint32_t kvb = smem_u32(&sm->kv_full);
         mbar_wait(smem_u32(&sm->kv_empty), (u & 1) ^ 1, &g_lmk_status, kErrDkvProducer);
         mbar_arrive_expect_tx(kvb, 4 * kTileBytes);
         for (int g = 0; g < 2; ++g) {       // a block past the end of the sequence reads as zeros
-          const int r0 = (2 * pair + g) * kBlk;
+          const int n = 2 * pair + g;
+          const int r0 = kIrr ? (n < tiles_of(b) ? end_of(b, n) - 63 : Lk) : n * kBlk;
           tma_load_4d(k_pair + g * kHalfTile, &tm_k, kvb, 0, r0, h, b);
           tma_load_4d(k_pair + kTileBytes + g * kHalfTile, &tm_k, kvb, 64, r0, h, b);
           tma_load_4d(v_pair + g * kHalfTile, &tm_v, kvb, 0, r0, h, b);
@@ -723,6 +961,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           tma_load_4d(do_slot(s), &tm_do, fb, 0, r0, h, b);
           tma_load_4d(do_slot(s) + kTileBytes, &tm_do, fb, 64, r0, h, b);
         }
+        ++u;
       }
     }
     __syncwarp();
@@ -736,8 +975,9 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const uint64_t dk0 = smem_desc_sw128(k_pair, 16, 1024), dv0 = smem_desc_sw128(v_pair, 16, 1024);
       const uint64_t dq0 = smem_desc_sw128(q_slot(0), 16, 1024), ddo0 = smem_desc_sw128(do_slot(0), 16, 1024);
       int it = 0, u = 0;
-      for (int w = unit_of(0); w < n_units; w = unit_of(++u)) {
-        const int n_items = n_tiles - unit_tq0(w / BH);
+      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+        if (skipped(w)) continue;
+        const int n_items = n_tiles - unit_tq0(w);
         mbar_wait(smem_u32(&sm->kv_full), u & 1, &g_lmk_status, kErrDkvMma);
         for (int i = 0; i < n_items; ++i, ++it) {
           const int s = it % kDkvStages;
@@ -759,6 +999,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           mma_commit(smem_u32(&sm->dp_full));
         }
         mma_commit(smem_u32(&sm->kv_empty));      // K / V tiles may be replaced once these products are done
+        ++u;
       }
     }
     __syncwarp();
@@ -773,8 +1014,9 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const uint64_t ddo0t = smem_desc_sw128(do_slot(0), kTileBytes, 1024);
       const uint64_t dpt = smem_desc_sw128(p_tile, 16, 1024), ddst = smem_desc_sw128(ds_tile, 16, 1024);
       int it = 0, u = 0;
-      for (int w = unit_of(0); w < n_units; w = unit_of(++u)) {
-        const int n_items = n_tiles - unit_tq0(w / BH);
+      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+        if (skipped(w)) continue;
+        const int n_items = n_tiles - unit_tq0(w);
         for (int i = 0; i < n_items; ++i, ++it) {
           const int s = it % kDkvStages;
           const uint64_t ddot = desc_advance(ddo0t, (uint32_t)s * 65536u), dqt = desc_advance(dq0t, (uint32_t)s * 65536u);
@@ -801,6 +1043,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
         mma_commit(smem_u32(&sm->acc_full[0]));
         mma_commit(smem_u32(&sm->acc_full[1]));
+        ++u;
       }
     }
     __syncwarp();
@@ -808,33 +1051,41 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const int g = warp >> 2;                       // warpgroup g owns block g of every pair
     const int row = tid & 127;
     const int half = row >> 6;
-    const int vis = min(row & 63, kBlk - 2);
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     int it = 0, u = 0;
-    for (int w = unit_of(0); w < n_units; w = unit_of(++u)) {
-      const int pair = w / BH, bh = w - pair * BH;
+    for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+      if (skipped(w)) continue;
+      const int pair = w / BH, bh = w - pair * BH, b = bh / H;
       const int n = 2 * pair + g;
-      const int tq0 = unit_tq0(pair), n_items = n_tiles - tq0;
+      const int tq0 = unit_tq0(w), n_items = n_tiles - tq0;
+      const bool tile_exists = n < tiles_of(b);
+      const int end = kIrr && tile_exists ? end_of(b, n) : 0, c0 = kIrr && tile_exists ? 64 - (end - end_of(b, n - 1)) : 0;
+      auto stat_m = [&](int64_t i) { return kIrr && irr.R != nullptr ? irr.R[i] : M_ptr[i]; };
+      auto stat_l = [&](int64_t i) { return kIrr && irr.R != nullptr ? 1.f : L_ptr[i]; };
+      auto own_of = [&](int r) { return kIrr ? group_of(b, min(Lk - Lq + r, Lk - 1)) : 0; };
       // the row statistics of the next item are fetched one item ahead, so their latency is never exposed
       // (rows past the end of the sequence have zero Q and dO tiles: whatever finite weights they get contribute nothing)
       const int64_t grow0 = (int64_t)bh * Lq + (kWhole ? tq0 * kQTile + row : min(tq0 * kQTile + row, Lq - 1));
       if (u == 0) grid_dep_wait();     // delta comes from the dQ kernel, which may still be running (see the launch)
-      float nM = M_ptr[grow0], nL = L_ptr[grow0], nDelta = delta_ptr[grow0];
+      float nM = stat_m(grow0), nL = stat_l(grow0), nDelta = delta_ptr[grow0];
+      int nOwn = own_of(tq0 * kQTile + row);
       for (int i = 0; i < n_items; ++i, ++it) {
         const int tq = tq0 + i;
-        const int own = prefix_blocks + 2 * tq + half;
+        const int own = kIrr ? nOwn : prefix_blocks + 2 * tq + half;
+        const int vis = min(kIrr ? 63 - (end - (Lk - Lq + tq * kQTile + row)) : row & 63, kBlk - 2);      // used where n == own
         const bool row_valid = kWhole || tq * kQTile + row < Lq;
-        const float M2L = row_valid ? fmaf(nM, kLog2e, __log2f(nL)) : 0.f, delta = row_valid ? nDelta : 0.f;
+        const float M2L = !row_valid ? 0.f : (kIrr && irr.R != nullptr ? nM : fmaf(nM, kLog2e, __log2f(nL))), delta = row_valid ? nDelta : 0.f;
         if (i + 1 < n_items) {
           const int64_t grow = (int64_t)bh * Lq + (kWhole ? (tq + 1) * kQTile + row : min((tq + 1) * kQTile + row, Lq - 1));
-          nM = M_ptr[grow];
-          nL = L_ptr[grow];
+          nM = stat_m(grow);
+          nL = stat_l(grow);
           nDelta = delta_ptr[grow];
+          nOwn = own_of((tq + 1) * kQTile + row);
         }
         mbar_wait(smem_u32(&sm->s_full), it & 1, &g_lmk_status, kErrDkvSoftmax);
         tc_fence_after();
         const int kind = n > own ? 0 : (n == own ? 1 : 2);
-        bwd_item<kBf16, true>(tmem_s(g) + lane_base, tmem_dp(g) + lane_base, smem_u32(&sm->dp_free), kind, vis,
+        bwd_item<kBf16, true, kIrr>(c0, tmem_s(g) + lane_base, tmem_dp(g) + lane_base, smem_u32(&sm->dp_free), kind, vis,
                               scale_log2, scale, M2L, delta, p_tile, ds_tile, row, [&]() {
                                 // The single P/dS tile pair is written in the order a, b, a, b, ...: before writing,
                                 // the accumulating MMAs of the OTHER warpgroup's latest item must have read it.  Each
@@ -866,6 +1117,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // epilogue: each warpgroup drains its own block; thread = feature d, TMEM column = key j -> dV[key][d], dK[key][d]
       mbar_wait(smem_u32(&sm->acc_full[g]), u & 1, &g_lmk_status, kErrDkvEpilogue);
       tc_fence_after();
+      if (kIrr) __syncwarp();
       uint32_t rv[2][32], rk[2][32];
       tmem_ld_32x32b_x32(tmem_dv(g) + lane_base, rv[0]);
       tmem_ld_32x32b_x32(tmem_dv(g) + 32 + lane_base, rv[1]);
@@ -874,19 +1126,21 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(smem_u32(&sm->acc_empty[g]));     // the next unit may start accumulating into this block's columns
-      if (n < n_blocks && (kWhole || row < D)) {
-        const int keys = min(kBlk, Lk - n * kBlk);
-        uint16_t* dvp = reinterpret_cast<uint16_t*>(dv_ptr) + ((int64_t)bh * Lk + (int64_t)n * kBlk) * D + row;
-        uint16_t* dkp = reinterpret_cast<uint16_t*>(dk_ptr) + ((int64_t)bh * Lk + (int64_t)n * kBlk) * D + row;
+      if (tile_exists && (kWhole || row < D)) {
+        const int key0 = kIrr ? end - 63 : n * kBlk;        // key of column 0; columns c0 ... keys-1 are this tile's own
+        const int keys = min(kBlk, Lk - key0);
+        uint16_t* dvp = reinterpret_cast<uint16_t*>(dv_ptr) + ((int64_t)bh * Lk + key0) * D + row;
+        uint16_t* dkp = reinterpret_cast<uint16_t*>(dk_ptr) + ((int64_t)bh * Lk + key0) * D + row;
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if (!kWhole && c * 32 + j >= keys) continue;
+            if (!kWhole && (c * 32 + j >= keys || (kIrr && c * 32 + j < c0))) continue;
             dvp[(int64_t)(c * 32 + j) * D] = (uint16_t)(pack2<kBf16>(__uint_as_float(rv[c][j]), 0.f) & 0xffffu);
             dkp[(int64_t)(c * 32 + j) * D] = (uint16_t)(pack2<kBf16>(__uint_as_float(rk[c][j]), 0.f) & 0xffffu);
           }
       }
+      ++u;
     }
     tc_fence_before();
   }
@@ -924,13 +1178,13 @@ struct DqSmem {
 // CTAs in a snake.  The K/V stream, the S/dP products and the softmax of the next unit start while dQ of the current
 // unit is drained by one warpgroup (the two warpgroups alternate); only the unit's first accumulating MMA waits for
 // the drain.  All barrier phases derive from counters that run across units.
-template <bool kBf16, int kD, bool kWhole>
+template <bool kBf16, int kD, bool kWhole, bool kIrr>
 __global__ void __launch_bounds__(kDqThreads, 1)
 sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_o, const float* __restrict__ L_ptr,
                     const float* __restrict__ M_ptr, float* __restrict__ delta_ptr, void* __restrict__ dq_ptr, int H,
-                    int BH, int Lq, int Lk, int D_any, float scale, float scale_log2) {
+                    int BH, int Lq, int Lk, int D_any, float scale, float scale_log2, IrrArgs irr) {
   const int D = kWhole ? kD : D_any;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -952,7 +1206,17 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   };
   // unit w -> query tile (heaviest = last tile first) and number of key blocks it sees
   auto unit_tile = [&](int w) { return n_tiles - 1 - w / BH; };
-  auto unit_items = [&](int t) { return kWhole ? prefix_blocks + 2 * t + 2 : min(prefix_blocks + 2 * t + 2, n_blocks); };
+  // kIrr: tile table and group of every key of the unit's batch row (flags), or the regular pattern
+  auto skipped = [&](int w) { return kIrr && irr.flags != nullptr && irr_plan_fallback(irr.plan, (w % BH) / H); };
+  auto group_of = [&](int b, int pos) { return irr.flags != nullptr ? irr_plan_group(irr.plan, b, pos) : pos / irr.block; };
+  auto end_of = [&](int b, int n) { return irr.flags != nullptr ? irr_plan_end(irr.plan, b, n) : (n + 1) * irr.block - 1; };
+  auto regular_items = [&](int t) { return kWhole ? prefix_blocks + 2 * t + 2 : min(prefix_blocks + 2 * t + 2, n_blocks); };
+
+  auto unit_items = [&](int w) {
+    const int t = unit_tile(w);
+    if constexpr (kIrr) return group_of((w % BH) / H, min(Lk - Lq + (t + 1) * kQTile, Lk) - 1) + 1;
+    return regular_items(t);
+  };
 
   if (tid == 0) {
     mbar_init(smem_u32(&sm->qdo_full), 1);
@@ -997,9 +1261,10 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       prefetch_tensormap(&tm_do);
       prefetch_tensormap(&tm_o);
       int it = 0, u = 0;
-      for (int w = unit_of(0); w < n_units; w = unit_of(++u)) {
+      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+        if (skipped(w)) continue;
         const int t = unit_tile(w), bh = w % BH, b = bh / H, h = bh - b * H;
-        const int total = unit_items(t), n_last = total - 1;
+        const int total = unit_items(w), n_last = total - 1;
         const uint32_t qb = smem_u32(&sm->qdo_full);
         mbar_wait(smem_u32(&sm->delta_read), (u & 1) ^ 1, &g_lmk_status, kErrDqProducer);
         mbar_arrive_expect_tx(qb, 3 * (kD / 64) * kTileBytes);
@@ -1008,17 +1273,20 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           tma_load_4d(q_tile + c * kTileBytes, &tm_q, qb, 64 * c, t * kQTile, h, b);
           tma_load_4d(do_tile + c * kTileBytes, &tm_do, qb, 64 * c, t * kQTile, h, b);
         }
+        int next_end = kIrr ? end_of(b, n_last) : 0;     // read one tile ahead: the table may be in global memory
         for (int i = 0; i < total; ++i, ++it) {
           const int s = it % kDqStages;
+          const int n = n_last - i, r0 = kIrr ? next_end - 63 : n * kBlk;
+          if (kIrr && n > 0) next_end = end_of(b, n - 1);
           mbar_wait(smem_u32(&sm->empty[s]), ((it / kDqStages) & 1) ^ 1, &g_lmk_status, kErrDqProducer);
           const uint32_t fb = smem_u32(&sm->full[s]);
-          const int n = n_last - i;
           mbar_arrive_expect_tx(fb, 2 * (kD / 64) * kHalfTile);
           for (int c = 0; c < kD / 64; ++c) {
-            tma_load_4d(k_slot(s) + c * kHalfTile, &tm_k, fb, 64 * c, n * kBlk, h, b);
-            tma_load_4d(v_slot(s) + c * kHalfTile, &tm_v, fb, 64 * c, n * kBlk, h, b);
+            tma_load_4d(k_slot(s) + c * kHalfTile, &tm_k, fb, 64 * c, r0, h, b);
+            tma_load_4d(v_slot(s) + c * kHalfTile, &tm_v, fb, 64 * c, r0, h, b);
           }
         }
+        ++u;
       }
     }
     __syncwarp();
@@ -1032,8 +1300,9 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const uint64_t db0 = smem_desc_sw128(is_s ? k_slot(0) : v_slot(0), 16, 1024);
       const uint32_t t_out = is_s ? tmem_s : tmem_dp, t_a = is_s ? tmem_q : tmem_do;
       int it = 0, u = 0;
-      for (int w = unit_of(0); w < n_units; w = unit_of(++u)) {
-        const int total = unit_items(unit_tile(w));
+      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+        if (skipped(w)) continue;
+        const int total = unit_items(w);
         mbar_wait(smem_u32(&sm->ops_ready), u & 1, &g_lmk_status, kErrDqMma);
         for (int i = 0; i < total; ++i, ++it) {
           const int s = it % kDqStages, sb = it % kSdpBufs;
@@ -1048,6 +1317,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           mma_commit(smem_u32(&sm->sdp_full[sb]));
         }
         mma_commit(smem_u32(&sm->ops_free));        // the next unit's Q / dO rows may be written
+        ++u;
       }
     }
     __syncwarp();
@@ -1058,8 +1328,9 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const uint64_t dv0 = smem_desc_sw128(v_slot(0), 16, 1024);
       const uint64_t dk0t = smem_desc_sw128(k_slot(0), kHalfTile, 1024);
       int it = 0, u = 0;
-      for (int w = unit_of(0); w < n_units; w = unit_of(++u)) {
-        const int total = unit_items(unit_tile(w));
+      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+        if (skipped(w)) continue;
+        const int total = unit_items(w);
         for (int i = 0; i < total; ++i, ++it) {
           const int s = it % kDqStages;
           mbar_wait(smem_u32(&sm->ds_ready[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
@@ -1073,6 +1344,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           mma_commit(smem_u32(&sm->empty[s]));
         }
         mma_commit(smem_u32(&sm->acc_full[(it - 1) & 1]));     // drained by the warpgroup that took the last item
+        ++u;
       }
     }
     __syncwarp();
@@ -1080,7 +1352,6 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int g = warp >> 2;                       // warpgroup: items with (running item count) % 2 == g
     const int row = tid & 127;
     const int half = row >> 6;
-    const int vis = min(row & 63, kBlk - 2);
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     int it0 = 0, u = 0, drains = 0;
     // dQ of a unit is drained by the warpgroup that took its last item, but only after that warpgroup has done the
@@ -1092,6 +1363,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       mbar_wait(smem_u32(&sm->acc_full[g]), drains & 1, &g_lmk_status, kErrDqEpilogue);
       ++drains;
       tc_fence_after();
+      if (kIrr) __syncwarp();
       uint4* orow = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(dq_ptr) + drain_row * D);
 #pragma unroll
       for (int c = 0; c < kD / 32; ++c) {
@@ -1120,25 +1392,31 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const int w0 = unit_of(0);
       if (w0 < n_units) {
         const int64_t g0 = (int64_t)(w0 % BH) * Lq + (kWhole ? unit_tile(w0) * kQTile + row : min(unit_tile(w0) * kQTile + row, Lq - 1));
-        nM = M_ptr[g0];
-        nL = L_ptr[g0];
+        nM = kIrr && irr.R != nullptr ? irr.R[g0] : M_ptr[g0];
+        nL = kIrr && irr.R != nullptr ? 1.f : L_ptr[g0];
       }
     }
-    for (int w = unit_of(0); w < n_units; w = unit_of(++u)) {
-      const int t = unit_tile(w), bh = w % BH;
-      const int own = prefix_blocks + 2 * t + half;
-      const int total = unit_items(t), n_last = total - 1;
+    for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+      const int t = unit_tile(w), bh = w % BH, b = bh / H;
+      const int total = unit_items(w), n_last = total - 1;
       const int64_t grow = (int64_t)bh * Lq + t * kQTile + row;
       const bool row_valid = kWhole || t * kQTile + row < Lq;
-      const float M2L = fmaf(nM, kLog2e, __log2f(nL));
+      const float M2L = kIrr && irr.R != nullptr ? nM : fmaf(nM, kLog2e, __log2f(nL));
       {
-        const int wn = unit_of(u + 1);
+        const int wn = unit_of(r + 1);
         if (wn < n_units) {
           const int64_t gn = (int64_t)(wn % BH) * Lq + (kWhole ? unit_tile(wn) * kQTile + row : min(unit_tile(wn) * kQTile + row, Lq - 1));
-          nM = M_ptr[gn];
-          nL = L_ptr[gn];
+          nM = kIrr && irr.R != nullptr ? irr.R[gn] : M_ptr[gn];
+          nL = kIrr && irr.R != nullptr ? 1.f : L_ptr[gn];
         }
       }
+      if (skipped(w)) continue;                     // after the prefetch, which belongs to the next unit
+      const int pos = min(Lk - Lq + t * kQTile + row, Lk - 1);
+      const int own = kIrr ? group_of(b, pos) : prefix_blocks + 2 * t + half;
+      const int vis = min(kIrr ? 63 - (end_of(b, own) - pos) : row & 63, kBlk - 2);
+      // kIrr: first visible column of this warpgroup's items, read one item ahead (hidden columns of tile n)
+      auto first_col = [&](int n) { return n < 0 ? 0 : 64 - (end_of(b, n) - (n > 0 ? end_of(b, n - 1) : -1)); };
+      int c0 = kIrr ? first_col(n_last - ((it0 + g) & 1)) : 0;
       // delta = rowsum(O * dO), straight from the swizzled tiles (one row per thread, 16-byte chunks); warpgroup 0
       // also publishes it for the dK/dV kernel, which runs after this one
       mbar_wait(smem_u32(&sm->qdo_full), u & 1, &g_lmk_status, kErrDqSoftmax);
@@ -1180,6 +1458,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // row -> TMEM lane, 32-bit word j (two features) -> column j: the layout of a K-major A operand
       mbar_wait(smem_u32(&sm->ops_free), (u & 1) ^ 1, &g_lmk_status, kErrDqSoftmax);
       tc_fence_after();
+      if (kIrr) __syncwarp();
       {
         const uint32_t dst = (g == 0 ? tmem_q : tmem_do) + lane_base;
         tmem_st_32x32b_x32(dst, opw[0]);
@@ -1197,8 +1476,10 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         mbar_wait(smem_u32(&sm->sdp_full[sb]), (it / kSdpBufs) & 1, &g_lmk_status, kErrDqSoftmax);
         tc_fence_after();
         const int kind = n > own ? 0 : (n == own ? 1 : 2);
+        const int c_now = c0;
+        if (kIrr) c0 = first_col(n - kBwdGroups);
         // dS replaces the V tile of this stage, which dP = dO V^T has finished reading
-        bwd_item<kBf16, false>(tmem_s + sb * 64 + lane_base, tmem_dp + sb * 64 + lane_base,
+        bwd_item<kBf16, false, kIrr>(c_now, tmem_s + sb * 64 + lane_base, tmem_dp + sb * 64 + lane_base,
                                smem_u32(&sm->sdp_free[sb]), kind, vis, scale_log2, scale, M2L, delta, 0u,
                                v_slot(s), row, []() {});
         fence_proxy_async_smem();
@@ -1209,6 +1490,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         drain_row = grow;
         drain_valid = row_valid;
       }
+      ++u;
     }
     if (drain_row >= 0) drain();
     tc_fence_before();
@@ -1339,6 +1621,8 @@ struct DeviceFacts {
   int n_sm = 0;
 };
 constexpr size_t kSmemFwd2 = 1024 + 65536 + kFwd2Stages * 32768 + sizeof(Fwd2Smem);
+constexpr size_t kSmemFwd2Irr = kSmemFwd2 + sizeof(IrrSmem);
+static_assert(kSmemFwd2Irr <= 232448, "shared memory of one SM");
 constexpr size_t kSmemDkv = 1024 + 65536 + kDkvStages * 65536 + 32768 + sizeof(DkvSmem);
 constexpr size_t kSmemDq = 1024 + 65536 + kDqStages * 32768 + 32768 + sizeof(DqSmem);
 
@@ -1353,16 +1637,20 @@ int device_facts(const DeviceFacts** out) {
   if (!f.ready) {
     LMK_CUDA(cudaDeviceGetAttribute(&f.n_sm, cudaDevAttrMultiProcessorCount, dev));
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<true, 128>, attr, (int)kSmemFwd2));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<false, 128>, attr, (int)kSmemFwd2));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<true, 64>, attr, (int)kSmemFwd2));
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<false, 64>, attr, (int)kSmemFwd2));
-#define LMK_BWD_ATTR(BF, DIM, WHOLE)                                                                \
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, WHOLE>, attr, (int)kSmemDq));        \
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, WHOLE>, attr, (int)kSmemDkv));
-    LMK_BWD_ATTR(true, 128, true) LMK_BWD_ATTR(true, 128, false) LMK_BWD_ATTR(true, 64, true) LMK_BWD_ATTR(true, 64, false)
-    LMK_BWD_ATTR(false, 128, true) LMK_BWD_ATTR(false, 128, false) LMK_BWD_ATTR(false, 64, true) LMK_BWD_ATTR(false, 64, false)
-#undef LMK_BWD_ATTR
+#define LMK_ATTRS(BF, DIM)                                                                                   \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, false>, attr, (int)kSmemFwd2));                 \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, true>, attr, (int)kSmemFwd2Irr));               \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, true, false>, attr, (int)kSmemDq));           \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, false, false>, attr, (int)kSmemDq));          \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, false, true>, attr, (int)kSmemDq));
+#define LMK_ATTRS_DKV(BF)                                                                                    \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, true, false>, attr, (int)kSmemDkv));              \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, false, false>, attr, (int)kSmemDkv));             \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, false, true>, attr, (int)kSmemDkv));
+    LMK_ATTRS(true, 128) LMK_ATTRS(true, 64) LMK_ATTRS(false, 128) LMK_ATTRS(false, 64)
+    LMK_ATTRS_DKV(true) LMK_ATTRS_DKV(false)
+#undef LMK_ATTRS
+#undef LMK_ATTRS_DKV
     f.ready = true;
   }
   *out = &f;
@@ -1409,7 +1697,7 @@ int tensor_map_4d(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int 
 }
 bool tensor_map_operand_ok(const void* p, const int64_t st[3]) { return tma_ok(p, st); }
 
-int attn_sm100_fwd(const AttnParams& p, int dtype, cudaStream_t st) {
+static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaStream_t st) {
   if (!attn_sm100_operands_ok(p, false))
     return fail(LMK_ERR_UNSUPPORTED, "tcgen05 path needs 16-byte aligned q/k/v with strides that are multiples of 8");
   bind_context();
@@ -1420,7 +1708,8 @@ int attn_sm100_fwd(const AttnParams& p, int dtype, cudaStream_t st) {
   if ((rc = make_map_4d(&tv, p.v, dtype, p.B, p.H, p.Lk, p.D, p.vs, kBlk)) != LMK_OK) return rc;
   const int whole_blocks = p.Lk / kBlk;
   const int lm_box = whole_blocks < 1 ? 1 : (whole_blocks < 64 ? whole_blocks : 64);
-  if ((rc = make_map_landmarks(&tl, p.k, dtype, p.B, p.H, p.Lk, p.D, p.ks, lm_box)) != LMK_OK) return rc;
+  if (irr != nullptr) tl = tk;      // not read
+  else if ((rc = make_map_landmarks(&tl, p.k, dtype, p.B, p.H, p.Lk, p.D, p.ks, lm_box)) != LMK_OK) return rc;
   const float scale_log2 = p.scale * kLog2e;
   const DeviceFacts* facts = nullptr;
   if ((rc = device_facts(&facts)) != LMK_OK) return rc;
@@ -1429,20 +1718,50 @@ int attn_sm100_fwd(const AttnParams& p, int dtype, cudaStream_t st) {
   const int n_tiles = (p.Lq + kQTile - 1) / kQTile;
   const int per_cta = (int64_t)n_tiles * p.B * p.H <= facts->n_sm ? 1 : 2;
   const dim3 grid(p.B * p.H, (n_tiles + per_cta - 1) / per_cta);
-#define LMK_FWD_LAUNCH(BF, DIM)                                                                                          \
-  sm100_fwd2_kernel<BF, DIM><<<grid, kFwd2Threads, kSmemFwd2, st>>>(tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk, p.D, \
-                                                                    lm_box, per_cta, scale_log2)
-  if (dtype == LMK_BF16) {
-    if (p.D <= 64) LMK_FWD_LAUNCH(true, 64); else LMK_FWD_LAUNCH(true, 128);
-  } else {
-    if (p.D <= 64) LMK_FWD_LAUNCH(false, 64); else LMK_FWD_LAUNCH(false, 128);
-  }
+#define LMK_FWD_LAUNCH(BF, DIM, IRR)                                                                                     \
+  sm100_fwd2_kernel<BF, DIM, IRR><<<grid, kFwd2Threads, IRR ? kSmemFwd2Irr : kSmemFwd2, st>>>(                           \
+      tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk, p.D, lm_box, per_cta, scale_log2, p.k, p.ks[0], p.ks[1], p.ks[2], args)
+#define LMK_FWD_DTYPE(BF)                                                                     \
+  do {                                                                                        \
+    if (irr != nullptr) {                                                                     \
+      if (p.D <= 64) LMK_FWD_LAUNCH(BF, 64, true); else LMK_FWD_LAUNCH(BF, 128, true);        \
+    } else {                                                                                  \
+      if (p.D <= 64) LMK_FWD_LAUNCH(BF, 64, false); else LMK_FWD_LAUNCH(BF, 128, false);      \
+    }                                                                                         \
+  } while (0)
+  const IrrArgs args = irr != nullptr ? *irr : IrrArgs{};
+  if (dtype == LMK_BF16) LMK_FWD_DTYPE(true);
+  else LMK_FWD_DTYPE(false);
+#undef LMK_FWD_DTYPE
 #undef LMK_FWD_LAUNCH
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }
 
-int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
+int attn_sm100_fwd(const AttnParams& p, int dtype, cudaStream_t st) { return launch_fwd(p, dtype, nullptr, st); }
+
+// blocks below 64 in a regular pattern
+bool attn_sm100_small_blocks(int B, int H, int Lq, int Lk, int D, int block, int dtype) {
+  return (dtype == LMK_BF16 || dtype == LMK_F16) && D >= 8 && D <= 128 && D % 8 == 0 && block >= 2 && block < kBlk && Lq >= 1 &&
+         Lk >= Lq && (Lk - 1) / block < kIrrMaxTiles && B >= 1 && H >= 1;
+}
+int attn_sm100_small_blocks_fwd(const AttnParams& p, int dtype, cudaStream_t st) {
+  IrrArgs a;
+  a.block = p.block;
+  return launch_fwd(p, dtype, &a, st);
+}
+// landmarks anywhere: p.o and R; rows of the batch left to the two-pass kernels are marked in R
+bool attn_sm100_flags(int Lk, int G) { return Lk <= kIrrMaxKeys && Lk <= kBlk * (G + 1); }
+int attn_sm100_flags_fwd(const AttnParams& p, const uint8_t* flags, int64_t stride, int G, float* R, int dtype, cudaStream_t st) {
+  IrrArgs a;
+  a.flags = flags;
+  a.stride = stride;
+  a.G = G;
+  a.R = R;
+  return launch_fwd(p, dtype, &a, st);
+}
+
+static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaStream_t st) {
   if (!attn_sm100_operands_ok(p, true))
     return fail(LMK_ERR_UNSUPPORTED, "tcgen05 path needs 16-byte aligned tensors with strides that are multiples of 8");
   bind_context();
@@ -1463,7 +1782,10 @@ int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
   int n_sm = facts->n_sm;
   const int cap = g_max_ctas.load();
   if (cap >= 1 && cap < n_sm) n_sm = cap;
-  const int dkv_units = ((p.Lk + 2 * kBlk - 1) / (2 * kBlk)) * p.B * p.H;
+  // key tiles of a batch row: whole blocks, or at most that many groups
+  const int max_tiles = irr == nullptr ? (p.Lk + kBlk - 1) / kBlk
+                        : (irr->flags != nullptr ? (irr->G < kIrrMaxTiles - 1 ? irr->G : kIrrMaxTiles - 1) + 1 : (p.Lk - 1) / irr->block + 1);
+  const int dkv_units = ((max_tiles + 1) / 2) * p.B * p.H;
   const int dq_units = ((p.Lq + kQTile - 1) / kQTile) * p.B * p.H;
   dim3 grid_dkv(dkv_units < n_sm ? dkv_units : n_sm), grid_dq(dq_units < n_sm ? dq_units : n_sm);
   // Both launches can carry the programmatic-stream-serialization attribute.  The dQ kernel waits for the kernel before it
@@ -1488,23 +1810,27 @@ int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
   const float* Mc = p.M;
   const float* deltac = delta;
   const int BH = p.B * p.H;
-#define LMK_BWD_LAUNCH(BF, DIM, DQ_WHOLE, DKV_WHOLE)                                                                       \
+#define LMK_BWD_LAUNCH(BF, DIM, DQ_WHOLE, DKV_WHOLE, IRR)                                                                  \
   do {                                                                                                                     \
-    LMK_CUDA(cudaLaunchKernelEx(&cfg_dq, sm100_bwd_dq_kernel<BF, DIM, DQ_WHOLE>, tq, tk, tv, tdo, to, Lc, Mc, delta, p.dq, \
-                                p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2));                                           \
-    LMK_CUDA(cudaLaunchKernelEx(&cfg_dkv, sm100_bwd_dkv_kernel<BF, DKV_WHOLE>, tq, tk, tv, tdo, Lc, Mc, deltac, p.dk,      \
-                                p.dv, p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2));                                     \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg_dq, sm100_bwd_dq_kernel<BF, DIM, DQ_WHOLE, IRR>, tq, tk, tv, tdo, to, Lc, Mc, delta,  \
+                                p.dq, p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2, args));                               \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg_dkv, sm100_bwd_dkv_kernel<BF, DKV_WHOLE, IRR>, tq, tk, tv, tdo, Lc, Mc, deltac, p.dk, \
+                                p.dv, p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2, max_tiles, args));                    \
   } while (0)
 #define LMK_BWD_DTYPE(BF)                                                      \
   do {                                                                         \
-    if (p.D <= 64) {                                                           \
-      if (whole && p.D == 64) LMK_BWD_LAUNCH(BF, 64, true, false);             \
-      else LMK_BWD_LAUNCH(BF, 64, false, false);                               \
+    if (irr != nullptr) {                                                      \
+      if (p.D <= 64) LMK_BWD_LAUNCH(BF, 64, false, false, true);               \
+      else LMK_BWD_LAUNCH(BF, 128, false, false, true);                        \
+    } else if (p.D <= 64) {                                                    \
+      if (whole && p.D == 64) LMK_BWD_LAUNCH(BF, 64, true, false, false);      \
+      else LMK_BWD_LAUNCH(BF, 64, false, false, false);                        \
     } else {                                                                   \
-      if (whole && p.D == 128) LMK_BWD_LAUNCH(BF, 128, true, true);            \
-      else LMK_BWD_LAUNCH(BF, 128, false, false);                              \
+      if (whole && p.D == 128) LMK_BWD_LAUNCH(BF, 128, true, true, false);     \
+      else LMK_BWD_LAUNCH(BF, 128, false, false, false);                       \
     }                                                                          \
   } while (0)
+  const IrrArgs args = irr != nullptr ? *irr : IrrArgs{};
   // instances without bounds where every tile is whole (the checks and run-time strides cost 8 us of 147 at L = 2048)
   const bool whole = p.Lq % kQTile == 0 && p.Lk % kBlk == 0;
   if (dtype == LMK_BF16) LMK_BWD_DTYPE(true);
@@ -1514,6 +1840,29 @@ int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }
+
+int attn_sm100_bwd(const AttnParams& p, int dtype, cudaStream_t st) { return launch_bwd(p, dtype, nullptr, st); }
+int attn_sm100_small_blocks_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
+  IrrArgs a;
+  a.block = p.block;
+  return launch_bwd(p, dtype, &a, st);
+}
+size_t attn_sm100_plan_bytes(int B) { return sizeof(int) * (size_t)B * kIrrPlanInts; }
+// p.workspace: delta; plan: attn_sm100_plan_bytes(B), written here.  Word 1 of a batch row's record (attn_sm100_plan_stride ints
+// apart) tells the two-pass kernels whether the row is theirs.
+int attn_sm100_flags_bwd(const AttnParams& p, const uint8_t* flags, int64_t stride, int G, const float* R, int* plan, int dtype,
+                         cudaStream_t st) {
+  irr_plan_kernel<<<p.B, 256, 0, st>>>(flags, stride, p.Lk, G, plan);
+  LMK_CUDA(cudaGetLastError());
+  IrrArgs a;
+  a.flags = flags;
+  a.stride = stride;
+  a.G = G;
+  a.R = const_cast<float*>(R);
+  a.plan = plan;
+  return launch_bwd(p, dtype, &a, st);
+}
+int attn_sm100_plan_stride() { return kIrrPlanInts; }
 
 size_t attn_sm100_bwd_workspace(int B, int H, int Lq, int, int) { return sizeof(float) * (size_t)B * H * Lq; }
 

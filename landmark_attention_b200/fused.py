@@ -27,15 +27,15 @@ def fused_landmark_attention(q, k, v, is_mem=None, sm_scale=None, block_size=64,
     `is_mem` may be None (fast path: no mask is read and the host is not synchronised); when given it must be the
     regular pattern over the keys, as the reference asserts (flash_landmark_attention.py:393-394).
     """
-    if block_size != 64 and path == L.PATH_AUTO and q.is_cuda and q.dtype in (torch.bfloat16, torch.float16):
-        out = _other_block_size(q, k, v, is_mem, sm_scale, block_size)
+    if block_size > 64 and path == L.PATH_AUTO and q.is_cuda and q.dtype in (torch.bfloat16, torch.float16):
+        out = _large_blocks(q, k, v, is_mem, sm_scale, block_size)
         if out is not None:
             return out
     return L.host().fused_attention(q, k, v, is_mem, sm_scale, block_size, path)
 
 
-def _other_block_size(q, k, v, is_mem, sm_scale, block_size):
-    """The tensor-core kernels behind the host call are built for blocks of 64; other block sizes run on the arbitrary-landmark
+def _large_blocks(q, k, v, is_mem, sm_scale, block_size):
+    """The tensor-core kernels behind the host call take blocks of up to 64 keys; larger ones run on the arbitrary-landmark
     tensor-core kernels with the regular pattern as flags, where those take the shape (None: they do not)."""
     from .masked import landmark_attention_masked
     B, Lq, Lk, D = q.shape[0], q.shape[2], k.shape[2], q.shape[3]
