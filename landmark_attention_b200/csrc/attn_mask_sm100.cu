@@ -157,13 +157,11 @@ __host__ __device__ constexpr size_t mf_smem_bytes(int G, int n_kt) {
 }
 
 template <bool kBf16>
-__global__ void __launch_bounds__(kMfThreads, 2)
-sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                      const __grid_constant__ CUtensorMap tm_v, const uint8_t* __restrict__ is_mem, int64_t is_mem_stride,
+__device__ __forceinline__ void mask_fwd_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k,
+                      const CUtensorMap& tm_v, const uint8_t* __restrict__ is_mem, int64_t is_mem_stride,
                       void* __restrict__ o_ptr, float* __restrict__ R_ptr, float* __restrict__ A_ptr, int H, int Lq,
-                      int Lk, int G, float scale_log2, int only_marked, int* status) {
-  // behind the single-pass kernel: only the tiles that it left (see attn_sm100.cu)
-  if (only_marked && R_ptr[(int64_t)blockIdx.x * Lq + (Lq / kQT - 1 - (int)blockIdx.y) * kQT] != -INFINITY) return;
+                      int Lk, int G, float scale_log2, int* status,
+    int t, int bh, uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -179,8 +177,7 @@ sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = Lq / kQT;
-  const int t = n_tiles - 1 - (int)blockIdx.y;          // heaviest tiles first
-  const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
+  const int b = bh / H, h = bh - b * H;
   const int pos0 = (Lk - Lq) + t * kQT;                 // key position of row 0 (a multiple of 64)
   const int n_kt = pos0 / kKT + 2;                      // key tiles 0 .. diagonal
   const int total = 2 * n_kt;
@@ -199,11 +196,7 @@ sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     mbar_init(smem_u32(&sm->o_full), 1);
     mbar_init_fence();
   }
-  if (warp == 5) tmem_alloc(smem_u32(&sm->tmem_base), 256);
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = sm->tmem_base;
   const uint32_t tmem_s0 = tmem, tmem_o = tmem + 128;
 
   if (warp == 4) {
@@ -409,7 +402,39 @@ sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     tc_fence_before();
   }
   __syncthreads();
-  if (warp == 5) {
+  if (tid == 0)
+    for (uint64_t* bar = reinterpret_cast<uint64_t*>(sm); bar < reinterpret_cast<uint64_t*>(&sm->tmem_base); ++bar)
+      mbar_inval(smem_u32(bar));
+  __syncthreads();
+}
+
+template <bool kBf16>
+__global__ void __launch_bounds__(kMfThreads, 2)
+sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                      const __grid_constant__ CUtensorMap tm_v, const uint8_t* __restrict__ is_mem, int64_t is_mem_stride,
+                      void* __restrict__ o_ptr, float* __restrict__ R_ptr, float* __restrict__ A_ptr, int H, int BH, int Lq,
+                      int Lk, int G, float scale_log2, int only_marked, int* status) {
+  __shared__ uint32_t tmem_slot;
+  const int n_tiles = Lq / kQT;
+  const uint32_t warp = threadIdx.x >> 5;
+  bool held = false;
+  uint32_t tmem = 0;
+  // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left.
+  for (int w = blockIdx.x; w < n_tiles * BH; w += gridDim.x) {
+    const int t = n_tiles - 1 - w / BH;      // heaviest tiles first
+    const int bh = w % BH;
+    if (only_marked && R_ptr[(int64_t)bh * Lq + t * kQT] != -INFINITY) continue;
+    if (!held) {
+      if (warp == 5) tmem_alloc(smem_u32(&tmem_slot), 256);
+      tc_fence_before();
+      __syncthreads();
+      tc_fence_after();
+      tmem = tmem_slot;
+      held = true;
+    }
+    mask_fwd_tile<kBf16>(tm_q, tm_k, tm_v, is_mem, is_mem_stride, o_ptr, R_ptr, A_ptr, H, Lq, Lk, G, scale_log2, status, t, bh, tmem);
+  }
+  if (held && warp == 5) {
     tc_fence_after();
     tmem_dealloc(tmem, 256);
   }
@@ -456,16 +481,14 @@ __device__ __forceinline__ float dot8(const uint4& a, const uint4& b, float acc)
 }
 
 template <bool kBf16>
-__global__ void __launch_bounds__(kMqThreads, 1)
-sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                         const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+__device__ __forceinline__ void mask_bwd_dq_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k,
+                         const CUtensorMap& tm_v, const CUtensorMap& tm_do,
                          const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const void* __restrict__ o_ptr,
                          const void* __restrict__ do_ptr, const float* __restrict__ R_ptr,
                          const float* __restrict__ A_ptr, float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
                          void* __restrict__ dq_ptr, int H, int Lq, int Lk, int G, float scale, float scale_log2,
-                         const int* __restrict__ plan, int plan_stride, int* status) {
-  if (plan != nullptr && plan[(int64_t)(blockIdx.x / H) * plan_stride + 1] == 0) return;      // the single-pass kernels' rows
-
+                         const int* __restrict__ plan, int plan_stride, int* status,
+    int t, int bh, uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -481,8 +504,7 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = Lq / kQT;
-  const int t = n_tiles - 1 - (int)blockIdx.y;
-  const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
+  const int b = bh / H, h = bh - b * H;
   const int pos0 = (Lk - Lq) + t * kQT;
   const int n_kt = pos0 / kKT + 2;
   const int total = 2 * n_kt;
@@ -501,11 +523,7 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     mbar_init(smem_u32(&sm->acc_full), 1);
     mbar_init_fence();
   }
-  if (warp == 5) tmem_alloc(smem_u32(&sm->tmem_base), 512);
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = sm->tmem_base;
   const uint32_t tmem_s = tmem, tmem_dp = tmem + 128, tmem_dq = tmem + 256;
 
   if (warp == 4) {
@@ -721,7 +739,42 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     tc_fence_before();
   }
   __syncthreads();
-  if (warp == 5) {
+  if (tid == 0)
+    for (uint64_t* bar = reinterpret_cast<uint64_t*>(sm); bar < reinterpret_cast<uint64_t*>(&sm->tmem_base); ++bar)
+      mbar_inval(smem_u32(bar));
+  __syncthreads();
+}
+
+template <bool kBf16>
+__global__ void __launch_bounds__(kMqThreads, 1)
+sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                         const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                         const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const void* __restrict__ o_ptr,
+                         const void* __restrict__ do_ptr, const float* __restrict__ R_ptr,
+                         const float* __restrict__ A_ptr, float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
+                         void* __restrict__ dq_ptr, int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2,
+                         const int* __restrict__ plan, int plan_stride, int* status) {
+  __shared__ uint32_t tmem_slot;
+  const int n_tiles = Lq / kQT;
+  const uint32_t warp = threadIdx.x >> 5;
+  bool held = false;
+  uint32_t tmem = 0;
+  // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left.
+  for (int w = blockIdx.x; w < n_tiles * BH; w += gridDim.x) {
+    const int t = n_tiles - 1 - w / BH;
+    const int bh = w % BH;
+    if (plan != nullptr && plan[(int64_t)(bh / H) * plan_stride + 1] == 0) continue;
+    if (!held) {
+      if (warp == 5) tmem_alloc(smem_u32(&tmem_slot), 512);
+      tc_fence_before();
+      __syncthreads();
+      tc_fence_after();
+      tmem = tmem_slot;
+      held = true;
+    }
+    mask_bwd_dq_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, o_ptr, do_ptr, R_ptr, A_ptr, delta_ptr, nD_ptr, dq_ptr, H, Lq, Lk, G, scale, scale_log2, plan, plan_stride, status, t, bh, tmem);
+  }
+  if (held && warp == 5) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
@@ -750,15 +803,13 @@ struct MkSmem {
 constexpr size_t kMkSmemBytes = 1024 + 32768 + kMkStages * 65536 + 32768 + sizeof(MkSmem);
 
 template <bool kBf16>
-__global__ void __launch_bounds__(kMkThreads, 1)
-sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                          const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+__device__ __forceinline__ void mask_bwd_dkv_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k,
+                          const CUtensorMap& tm_v, const CUtensorMap& tm_do,
                           const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const float* __restrict__ R_ptr,
                           const float* __restrict__ A_ptr, const float* __restrict__ delta_ptr,
                           const float* __restrict__ nD_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                          int H, int Lq, int Lk, int G, float scale, float scale_log2, const int* __restrict__ plan, int plan_stride, int* status) {
-  if (plan != nullptr && plan[(int64_t)(blockIdx.x / H) * plan_stride + 1] == 0) return;      // the single-pass kernels' rows
-
+                          int H, int Lq, int Lk, int G, float scale, float scale_log2, int* status,
+    int kt, int bh, uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -771,8 +822,7 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = Lq / kQT;
-  const int kt = blockIdx.y;                            // early key tiles are seen by the most query tiles
-  const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
+  const int b = bh / H, h = bh - b * H;
   const int prefix = Lk - Lq;
   const int k0 = kt * kKT;
   const int t_first = k0 > prefix ? (k0 - prefix) / kQT : 0;
@@ -793,11 +843,7 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     mbar_init(smem_u32(&sm->acc_full), 1);
     mbar_init_fence();
   }
-  if (warp == 5) tmem_alloc(smem_u32(&sm->tmem_base), 512);
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = sm->tmem_base;
   const uint32_t tmem_s = tmem, tmem_dp = tmem + 128, tmem_dv = tmem + 256, tmem_dk = tmem + 320;
 
   if (warp == 4) {
@@ -1050,7 +1096,41 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     tc_fence_before();
   }
   __syncthreads();
-  if (warp == 5) {
+  if (tid == 0)
+    for (uint64_t* bar = reinterpret_cast<uint64_t*>(sm); bar < reinterpret_cast<uint64_t*>(&sm->tmem_base); ++bar)
+      mbar_inval(smem_u32(bar));
+  __syncthreads();
+}
+
+template <bool kBf16>
+__global__ void __launch_bounds__(kMkThreads, 1)
+sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                          const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                          const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const float* __restrict__ R_ptr,
+                          const float* __restrict__ A_ptr, const float* __restrict__ delta_ptr,
+                          const float* __restrict__ nD_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
+                          int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2, const int* __restrict__ plan, int plan_stride, int* status) {
+  __shared__ uint32_t tmem_slot;
+  const int n_tiles = Lk / kKT;
+  const uint32_t warp = threadIdx.x >> 5;
+  bool held = false;
+  uint32_t tmem = 0;
+  // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left.
+  for (int w = blockIdx.x; w < n_tiles * BH; w += gridDim.x) {
+    const int kt = w / BH;      // early key tiles are seen by the most query tiles
+    const int bh = w % BH;
+    if (plan != nullptr && plan[(int64_t)(bh / H) * plan_stride + 1] == 0) continue;
+    if (!held) {
+      if (warp == 5) tmem_alloc(smem_u32(&tmem_slot), 512);
+      tc_fence_before();
+      __syncthreads();
+      tc_fence_after();
+      tmem = tmem_slot;
+      held = true;
+    }
+    mask_bwd_dkv_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, R_ptr, A_ptr, delta_ptr, nD_ptr, dk_ptr, dv_ptr, H, Lq, Lk, G, scale, scale_log2, status, kt, bh, tmem);
+  }
+  if (held && warp == 5) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
@@ -1109,13 +1189,14 @@ int attn_mask_sm100_fwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
   // lengths that cannot consist of such groups, on the two-pass kernels here.
   const int only_marked = attn_sm100_flags(p.Lk, G) && p.scale > 0.f;
   if (only_marked && (rc = attn_sm100_flags_fwd(p, is_mem, is_mem_stride, G, R, dtype, st)) != LMK_OK) return rc;
-  dim3 grid(p.B * p.H, p.Lq / kQT);
+  const int tiles = p.B * p.H * (p.Lq / kQT);
+  const int grid = only_marked ? (tiles < 296 ? tiles : 296) : tiles;
   const size_t smem = mf_smem_bytes(G, p.Lk / kKT);
   if (dtype == LMK_BF16)
-    sm100_mask_fwd_kernel<true><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.Lq,
+    sm100_mask_fwd_kernel<true><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.B * p.H, p.Lq,
                                                                  p.Lk, G, scale_log2, only_marked, status);
   else
-    sm100_mask_fwd_kernel<false><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.Lq,
+    sm100_mask_fwd_kernel<false><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.B * p.H, p.Lq,
                                                                   p.Lk, G, scale_log2, only_marked, status);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
@@ -1144,7 +1225,7 @@ int attn_mask_sm100_bwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
   float* delta = reinterpret_cast<float*>(p.workspace);
   float* nD = delta + (size_t)p.B * p.H * p.Lq;
   const float scale_log2 = p.scale * kLog2e;
-  dim3 grid_q(p.B * p.H, p.Lq / kQT), grid_k(p.B * p.H, p.Lk / kKT);
+  int grid_q = p.B * p.H * (p.Lq / kQT), grid_k = p.B * p.H * (p.Lk / kKT);
   const size_t smem_q = mq_smem_bytes(G);
   const int* plan = nullptr;
   const int plan_stride = attn_sm100_plan_stride();
@@ -1152,14 +1233,16 @@ int attn_mask_sm100_bwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
     int* records = reinterpret_cast<int*>(nD + (size_t)p.B * p.H * G * p.Lq);
     if ((rc = attn_sm100_flags_bwd(p, is_mem, is_mem_stride, G, R, records, dtype, st)) != LMK_OK) return rc;
     plan = records;
+    grid_q = grid_q < 148 ? grid_q : 148;
+    grid_k = grid_k < 148 ? grid_k : 148;
   }
 #define LMK_MASK_BWD(BF)                                                                                                \
   do {                                                                                                                  \
     sm100_mask_bwd_dq_kernel<BF><<<grid_q, kMqThreads, smem_q, st>>>(tq, tk, tv, tdo, is_mem, is_mem_stride, p.o, p.dO,  \
-                                                                     R, A, delta, nD, p.dq, p.H, p.Lq, p.Lk, G,         \
+                                                                     R, A, delta, nD, p.dq, p.H, p.B * p.H, p.Lq, p.Lk, G, \
                                                                      p.scale, scale_log2, plan, plan_stride, status);   \
     sm100_mask_bwd_dkv_kernel<BF><<<grid_k, kMkThreads, kMkSmemBytes, st>>>(tq, tk, tv, tdo, is_mem, is_mem_stride, R,  \
-                                                                           A, delta, nD, p.dk, p.dv, p.H, p.Lq, p.Lk,   \
+                                                                           A, delta, nD, p.dk, p.dv, p.H, p.B * p.H, p.Lq, p.Lk, \
                                                                            G, p.scale, scale_log2, plan, plan_stride, status); \
   } while (0)
   if (dtype == LMK_BF16) LMK_MASK_BWD(true);

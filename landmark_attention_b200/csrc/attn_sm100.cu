@@ -245,18 +245,19 @@ __device__ __forceinline__ void irr_hide(float (&sv)[64], int c0) {
 // (rows 256u .. 256u+127), warpgroup 1 owns tile B (the next 128 rows).  Both tiles consume the same K/V stream, so
 // every K/V block is fetched from L2 once per 256 query rows, and the two softmax pipelines overlap with each
 // other and with the MMAs.  Tile A skips the two newest key blocks (they lie after its own blocks).
-constexpr int kFwd2Stages = 5;
-constexpr int kFwd2Threads = 352;
+// With one tile a CTA uses half of the registers, TMEM and shared memory, so that two CTAs share an SM and each other's start and end.
+template <int kTiles> constexpr int kFwdStages = kTiles == 2 ? 5 : 2;
+template <int kTiles> constexpr int kFwdThreads = (4 * kTiles + 3) * 32;
 enum { kErrFwd2Producer = 111, kErrFwd2Mma = 112, kErrFwd2Softmax = 113, kErrFwd2Epilogue = 114 };
 
 // one in this many pairs of exponentials uses ex2_poly2 (measured at L = 8192: 2 -> 544 us, 4 -> 523, 8 -> 515, 64 -> 508;
 // no difference at L = 2048: the special-function pipe is not what the forward kernel waits for)
 constexpr int kFwdPolyEvery = 64;
 
-struct Fwd2Smem {
+template <int kStages> struct Fwd2Smem {
   uint64_t q_full;
-  uint64_t full[kFwd2Stages];
-  uint64_t empty[kFwd2Stages];
+  uint64_t full[kStages];
+  uint64_t empty[kStages];
   uint64_t s_full[2][2];    // [tile][S buffer]
   uint64_t s_free[2][2];
   uint64_t p_ready[2][2];   // [tile][buffer]: a warp whose rows have little to do can be one item ahead of the others
@@ -264,24 +265,25 @@ struct Fwd2Smem {
   uint32_t tmem_base;
 };
 
-template <bool kBf16, int kD, bool kIrr>
-__global__ void __launch_bounds__(kFwd2Threads, 1)
+template <bool kBf16, int kD, bool kIrr, int kTiles>
+__global__ void __launch_bounds__(kFwdThreads<kTiles>, 3 - kTiles)
 sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_klm,
                   void* __restrict__ o_ptr, float* __restrict__ L_ptr, float* __restrict__ M_ptr, int H, int Lq, int Lk,
-                  int D, int lm_box, int per_cta, float scale_log2, const void* __restrict__ k_ptr, int64_t ks_b, int64_t ks_h,
+                  int D, int lm_box, float scale_log2, const void* __restrict__ k_ptr, int64_t ks_b, int64_t ks_h,
                   int64_t ks_row, IrrArgs irr) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   auto q_tile = [&](int w) { return base + (uint32_t)w * 32768u; };
-  auto k_slot = [&](int s) { return base + 65536u + (uint32_t)s * 32768u; };
-  auto v_slot = [&](int s) { return base + 65536u + (uint32_t)s * 32768u + 16384u; };
-  Fwd2Smem* sm = reinterpret_cast<Fwd2Smem*>(smem_raw + (base - raw) + 65536u + kFwd2Stages * 32768u);
+  constexpr int kStages = kFwdStages<kTiles>, kSw = 4 * kTiles;        // softmax warps; the three roles follow them
+  auto k_slot = [&](int s) { return base + kTiles * 32768u + (uint32_t)s * 32768u; };
+  auto v_slot = [&](int s) { return base + kTiles * 32768u + (uint32_t)s * 32768u + 16384u; };
+  Fwd2Smem<kStages>* sm = reinterpret_cast<Fwd2Smem<kStages>*>(smem_raw + (base - raw) + (kTiles + kStages) * 32768u);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int t_a = ((int)gridDim.y - 1 - (int)blockIdx.y) * per_cta;      // heaviest tiles first, across all heads
-  const bool has_b = per_cta == 2 && (t_a + 1) * kQTile < Lq;            // the second tile has at least one row
+  const int t_a = ((int)gridDim.y - 1 - (int)blockIdx.y) * kTiles;      // heaviest tiles first, across all heads
+  const bool has_b = kTiles == 2 && (t_a + 1) * kQTile < Lq;            // the second tile has at least one row
   const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
   const int prefix_blocks = (Lk - Lq) / kBlk;
   const int pos_a = Lk - Lq + t_a * kQTile;             // key position of tile A's first row
@@ -309,7 +311,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
   if (tid == 0) {
     mbar_init(smem_u32(&sm->q_full), 1);
-    for (int s = 0; s < kFwd2Stages; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       mbar_init(smem_u32(&sm->full[s]), 1);
       mbar_init(smem_u32(&sm->empty[s]), 1);
     }
@@ -323,16 +325,16 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mbar_init(smem_u32(&sm->o_full), 1);
     mbar_init_fence();
   }
-  if (warp == 9) tmem_alloc(smem_u32(&sm->tmem_base), 512);
+  if (warp == kSw + 1) tmem_alloc(smem_u32(&sm->tmem_base), kTiles * 256);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   auto tmem_s = [&](int w, int sb) { return tmem + (uint32_t)(w * 128 + sb * 64); };
-  auto tmem_o = [&](int w) { return tmem + 256u + (uint32_t)w * 128u; };
+  auto tmem_o = [&](int w) { return tmem + kTiles * 128u + (uint32_t)w * 128u; };
   grid_dep_launch();      // a dependent kernel (the backward pass) may do its set-up while this grid drains
 
-  if (warp == 8) {
+  if (warp == kSw) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       prefetch_tensormap(&tm_q);
@@ -345,8 +347,8 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         for (int c = 0; c < kD / 64; ++c)
           tma_load_4d(q_tile(w) + c * kTileBytes, &tm_q, qb, 64 * c, (t_a + w) * kQTile, h, b);
       for (int i = 0; i < total; ++i) {
-        const int s = i % kFwd2Stages;
-        mbar_wait(smem_u32(&sm->empty[s]), ((i / kFwd2Stages) & 1) ^ 1, &g_lmk_status, kErrFwd2Producer);
+        const int s = i % kStages;
+        mbar_wait(smem_u32(&sm->empty[s]), ((i / kStages) & 1) ^ 1, &g_lmk_status, kErrFwd2Producer);
         const uint32_t fb = smem_u32(&sm->full[s]);
         if (kIrr && i < n_lm_tiles) continue;           // the softmax warps gather the landmark keys themselves
         if (i < n_lm_tiles) {
@@ -365,7 +367,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
     }
     __syncwarp();
-  } else if (warp == 9) {
+  } else if (warp == kSw + 1) {
     // ------------------------------------------------------------------ MMA issuer 1: S = Q K^T
     // Two issuer threads keep the scalar bookkeeping between tcgen05.mma instructions short, and the S MMAs of the
     // next key block never queue behind a wait for the softmax of the current one.
@@ -382,7 +384,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         mbar_wait(smem_u32(&sm->full[s]), ph, &g_lmk_status, kErrFwd2Mma);
         const uint64_t dk = desc_advance(dk0, (uint32_t)s * 32768u);
 #pragma unroll
-        for (int w = 0; w < 2; ++w) {
+        for (int w = 0; w < kTiles; ++w) {
           if (!active(w, j)) continue;
           const int k = ks[w]++, sb = k & 1;
           if (k >= 2) mbar_wait(smem_u32(&sm->s_free[w][sb]), ((k >> 1) & 1) ^ 1, &g_lmk_status, kErrFwd2Mma);
@@ -394,11 +396,11 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                        desc_advance(dk, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
           mma_commit(smem_u32(&sm->s_full[w][sb]));
         }
-        if (++s == kFwd2Stages) { s = 0; ph ^= 1; }
+        if (++s == kStages) { s = 0; ph ^= 1; }
       }
     }
     __syncwarp();
-  } else if (warp == 10) {
+  } else if (warp == kSw + 2) {
     // ------------------------------------------------------------------ MMA issuer 2: O += P V
     if (lane == 0) {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
@@ -410,7 +412,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       for (int i = 0; i < total; ++i) {
         const uint64_t dv = desc_advance(dv0, (uint32_t)s * 32768u);
 #pragma unroll
-        for (int w = 0; w < 2; ++w) {
+        for (int w = 0; w < kTiles; ++w) {
           if (!active(w, i)) continue;
           const int k = kp[w]++;
           mbar_wait(smem_u32(&sm->p_ready[w][k & 1]), (k >> 1) & 1, &g_lmk_status, kErrFwd2Mma);
@@ -429,7 +431,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
         // the stage is free once both P V products are done; each of them waited for its S product to be read
         mma_commit(smem_u32(&sm->empty[s]));
-        if (++s == kFwd2Stages) s = 0;
+        if (++s == kStages) s = 0;
       }
       mma_commit(smem_u32(&sm->o_full));
     }
@@ -447,7 +449,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     int k = 0;
     if (kIrr && n_lm_tiles > 0) {                  // landmark keys of tiles 0 .. n_last-1 -> rows of the first stage
       const uint16_t* kb = reinterpret_cast<const uint16_t*>(k_ptr) + b * ks_b + h * ks_h;
-      for (int e = tid; e < n_last * (kD / 8); e += 256) {
+      for (int e = tid; e < n_last * (kD / 8); e += kSw * 32) {
         const int n = e / (kD / 8), c = e - n * (kD / 8);
         uint4 x = make_uint4(0u, 0u, 0u, 0u);
         if (c * 8 < D) x = *reinterpret_cast<const uint4*>(kb + (int64_t)end_of(n) * ks_row + c * 8);
@@ -455,7 +457,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
       }
       fence_proxy_async_smem();
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(kSw * 32) : "memory");
       if (tid == 0) mbar_arrive(smem_u32(&sm->full[0]));
     }
     for (int i = 0; i < total; ++i) {
@@ -597,9 +599,9 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     tc_fence_before();
   }
   __syncthreads();
-  if (warp == 9) {
+  if (warp == kSw + 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 512);
+    tmem_dealloc(tmem, kTiles * 256);
   }
 }
 
@@ -846,7 +848,7 @@ struct DkvSmem {
 // the item written before have read it), which settles them half an item apart.
 // CTA c takes units w = round * grid + c with the direction alternating per round (snake), heaviest pairs first.
 // Loads, S/dP products and the softmax of the next unit start while the accumulators of the current one are drained.
-template <bool kBf16, bool kWhole, bool kIrr>
+template <bool kBf16, bool kWhole, bool kIrr>      // kWhole: whole tiles and D = 128
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -1126,18 +1128,28 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(smem_u32(&sm->acc_empty[g]));     // the next unit may start accumulating into this block's columns
-      if (tile_exists && (kWhole || row < D)) {
+      if (tile_exists) {
         const int key0 = kIrr ? end - 63 : n * kBlk;        // key of column 0; columns c0 ... keys-1 are this tile's own
         const int keys = min(kBlk, Lk - key0);
-        uint16_t* dvp = reinterpret_cast<uint16_t*>(dv_ptr) + ((int64_t)bh * Lk + key0) * D + row;
-        uint16_t* dkp = reinterpret_cast<uint16_t*>(dk_ptr) + ((int64_t)bh * Lk + key0) * D + row;
+        // A lane holds one feature of all keys.  Neighbouring lanes swap halves, so that a lane stores two features of every
+        // second key in one word (half as many stores as 16-bit ones, and the same 64 bytes a row and warp).
+        const bool odd = lane & 1;
+        const int f = row & ~1;
+        uint32_t* dvp = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dv_ptr) + ((int64_t)bh * Lk + key0 + (odd ? 1 : 0)) * D + f);
+        uint32_t* dkp = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dk_ptr) + ((int64_t)bh * Lk + key0 + (odd ? 1 : 0)) * D + f);
+        const bool stores = kWhole || f < D;
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (!kWhole && (c * 32 + j >= keys || (kIrr && c * 32 + j < c0))) continue;
-            dvp[(int64_t)(c * 32 + j) * D] = (uint16_t)(pack2<kBf16>(__uint_as_float(rv[c][j]), 0.f) & 0xffffu);
-            dkp[(int64_t)(c * 32 + j) * D] = (uint16_t)(pack2<kBf16>(__uint_as_float(rk[c][j]), 0.f) & 0xffffu);
+          for (int j = 0; j < 32; j += 2) {
+            const uint32_t v = pack2<kBf16>(__uint_as_float(rv[c][j]), __uint_as_float(rv[c][j + 1]));
+            const uint32_t k = pack2<kBf16>(__uint_as_float(rk[c][j]), __uint_as_float(rk[c][j + 1]));
+            const uint32_t vo = __shfl_xor_sync(0xffffffffu, v, 1), ko = __shfl_xor_sync(0xffffffffu, k, 1);
+            const int col = c * 32 + j + (odd ? 1 : 0);
+            if (stores && (kWhole || (col < keys && (!kIrr || col >= c0)))) {
+              dvp[(c * 32 + j) * (D / 2)] = odd ? __byte_perm(vo, v, 0x7632) : __byte_perm(v, vo, 0x5410);
+              dkp[(c * 32 + j) * (D / 2)] = odd ? __byte_perm(ko, k, 0x7632) : __byte_perm(k, ko, 0x5410);
+            }
           }
       }
       ++u;
@@ -1620,9 +1632,10 @@ struct DeviceFacts {
   bool ready = false;
   int n_sm = 0;
 };
-constexpr size_t kSmemFwd2 = 1024 + 65536 + kFwd2Stages * 32768 + sizeof(Fwd2Smem);
-constexpr size_t kSmemFwd2Irr = kSmemFwd2 + sizeof(IrrSmem);
-static_assert(kSmemFwd2Irr <= 232448, "shared memory of one SM");
+template <int kTiles> constexpr size_t fwd_smem(bool irr) {
+  return 1024 + (kTiles + kFwdStages<kTiles>) * 32768 + sizeof(Fwd2Smem<kFwdStages<kTiles>>) + (irr ? sizeof(IrrSmem) : 0);
+}
+static_assert(fwd_smem<2>(true) <= 232448 && fwd_smem<1>(true) <= 232448 / 2 - 1024, "shared memory of one SM");
 constexpr size_t kSmemDkv = 1024 + 65536 + kDkvStages * 65536 + 32768 + sizeof(DkvSmem);
 constexpr size_t kSmemDq = 1024 + 65536 + kDqStages * 32768 + 32768 + sizeof(DqSmem);
 
@@ -1638,8 +1651,10 @@ int device_facts(const DeviceFacts** out) {
     LMK_CUDA(cudaDeviceGetAttribute(&f.n_sm, cudaDevAttrMultiProcessorCount, dev));
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
 #define LMK_ATTRS(BF, DIM)                                                                                   \
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, false>, attr, (int)kSmemFwd2));                 \
-    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, true>, attr, (int)kSmemFwd2Irr));               \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, false, 1>, attr, (int)fwd_smem<1>(false)));     \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, true, 1>, attr, (int)fwd_smem<1>(true)));       \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, false, 2>, attr, (int)fwd_smem<2>(false)));     \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, true, 2>, attr, (int)fwd_smem<2>(true)));       \
     LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, true, false>, attr, (int)kSmemDq));           \
     LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, false, false>, attr, (int)kSmemDq));          \
     LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, false, true>, attr, (int)kSmemDq));
@@ -1697,6 +1712,15 @@ int tensor_map_4d(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int 
 }
 bool tensor_map_operand_ok(const void* p, const int64_t st[3]) { return tma_ok(p, st); }
 
+// Two query tiles a CTA share one K/V stream; one tile a CTA puts two CTAs on an SM, whose starts and ends overlap and which the
+// hardware deals out in smaller pieces.  Measured (us, one / two): 32 heads of L = 512 14.4 / 16.5, 1024 24.7 / 25.0, 1536 35.0 /
+// 33.1, 2048 50.0 / 47.5, 4096 164 / 148; 8 heads of 2048 (less than two CTAs an SM) 36.9 / 39.0; 51-key groups, 128 heads of
+// 512 37.0 / 41.1, 32-key blocks at 2000 105 / 109.  A single tile of a long history wants the deeper pipeline of the second form.
+static int fwd_tiles_per_cta(int n_tiles, int BH, int n_sm, bool irr) {
+  if (n_tiles == 1) return 2;
+  return n_tiles <= (irr ? 16 : 8) || (int64_t)n_tiles * BH <= 2 * n_sm ? 1 : 2;
+}
+
 static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaStream_t st) {
   if (!attn_sm100_operands_ok(p, false))
     return fail(LMK_ERR_UNSUPPORTED, "tcgen05 path needs 16-byte aligned q/k/v with strides that are multiples of 8");
@@ -1713,26 +1737,29 @@ static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   const float scale_log2 = p.scale * kLog2e;
   const DeviceFacts* facts = nullptr;
   if ((rc = device_facts(&facts)) != LMK_OK) return rc;
-  // Two query tiles a CTA share one K/V stream (a pair costs 1.2 - 1.3 times a single tile); one tile a CTA while that still
-  // leaves every CTA an SM of its own.
   const int n_tiles = (p.Lq + kQTile - 1) / kQTile;
-  const int per_cta = (int64_t)n_tiles * p.B * p.H <= facts->n_sm ? 1 : 2;
+  const int per_cta = fwd_tiles_per_cta(n_tiles, p.B * p.H, facts->n_sm, irr != nullptr);
   const dim3 grid(p.B * p.H, (n_tiles + per_cta - 1) / per_cta);
-#define LMK_FWD_LAUNCH(BF, DIM, IRR)                                                                                     \
-  sm100_fwd2_kernel<BF, DIM, IRR><<<grid, kFwd2Threads, IRR ? kSmemFwd2Irr : kSmemFwd2, st>>>(                           \
-      tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk, p.D, lm_box, per_cta, scale_log2, p.k, p.ks[0], p.ks[1], p.ks[2], args)
+#define LMK_FWD_LAUNCH(BF, DIM, IRR, TILES)                                                                              \
+  sm100_fwd2_kernel<BF, DIM, IRR, TILES><<<grid, kFwdThreads<TILES>, fwd_smem<TILES>(IRR), st>>>(                        \
+      tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk, p.D, lm_box, scale_log2, p.k, p.ks[0], p.ks[1], p.ks[2], args)
+#define LMK_FWD_TILES(BF, DIM, IRR)                                                           \
+  do {                                                                                        \
+    if (per_cta == 1) LMK_FWD_LAUNCH(BF, DIM, IRR, 1); else LMK_FWD_LAUNCH(BF, DIM, IRR, 2);  \
+  } while (0)
 #define LMK_FWD_DTYPE(BF)                                                                     \
   do {                                                                                        \
     if (irr != nullptr) {                                                                     \
-      if (p.D <= 64) LMK_FWD_LAUNCH(BF, 64, true); else LMK_FWD_LAUNCH(BF, 128, true);        \
+      if (p.D <= 64) LMK_FWD_TILES(BF, 64, true); else LMK_FWD_TILES(BF, 128, true);          \
     } else {                                                                                  \
-      if (p.D <= 64) LMK_FWD_LAUNCH(BF, 64, false); else LMK_FWD_LAUNCH(BF, 128, false);      \
+      if (p.D <= 64) LMK_FWD_TILES(BF, 64, false); else LMK_FWD_TILES(BF, 128, false);        \
     }                                                                                         \
   } while (0)
   const IrrArgs args = irr != nullptr ? *irr : IrrArgs{};
   if (dtype == LMK_BF16) LMK_FWD_DTYPE(true);
   else LMK_FWD_DTYPE(false);
 #undef LMK_FWD_DTYPE
+#undef LMK_FWD_TILES
 #undef LMK_FWD_LAUNCH
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
