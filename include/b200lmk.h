@@ -109,6 +109,15 @@ int lmk_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
                  const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
                  int block, float sm_scale, int dtype, int path, void* stream);
 
+/* lmk_attn_bwd with element strides {batch, head, row} of dO instead of a dense one (contiguous features). */
+int lmk_attn_bwd_strided(const void* q, const void* k, const void* v, const void* o, const void* dO,
+                 const float* L, const float* M, void* dQ, void* dK, void* dV,
+                 void* workspace, size_t workspace_bytes,
+                 int B, int H, int Lq, int Lk, int D,
+                 const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
+                 const int64_t do_strides[3],
+                 int block, float sm_scale, int dtype, int path, void* stream);
+
 /*
  * Backward pass for callers that cannot allocate device memory.  (No counterpart in the reference.)
  *
@@ -169,6 +178,15 @@ int lmk_attn_mask_bwd(const void* q, const void* k, const void* v, const uint8_t
                       void* dQ, void* dK, void* dV, void* workspace, size_t workspace_bytes,
                       int B, int H, int Lq, int Lk, int D,
                       const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
+                      int max_groups, float sm_scale, int dtype, void* stream);
+
+/* lmk_attn_mask_bwd with element strides {batch, head, row} of dO instead of a dense one (contiguous features). */
+int lmk_attn_mask_bwd_strided(const void* q, const void* k, const void* v, const uint8_t* is_mem, int64_t is_mem_stride,
+                      const void* o, const void* dO, const float* R, const float* A,
+                      void* dQ, void* dK, void* dV, void* workspace, size_t workspace_bytes,
+                      int B, int H, int Lq, int Lk, int D,
+                      const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
+                      const int64_t do_strides[3],
                       int max_groups, float sm_scale, int dtype, void* stream);
 
 /*

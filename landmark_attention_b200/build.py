@@ -18,7 +18,7 @@ OBJ_DIR = os.path.join(HERE, "_obj")
 LIB_PATH = os.path.join(LIB_DIR, "libb200lmk.so")
 HOST_SOURCE = os.path.join(CSRC, "host_torch.cpp")
 HOST_PATH = os.path.join(LIB_DIR, "_lmk_host.so")
-SOURCES = ["api.cu", "attn_general.cu", "attn_sm100.cu", "attn_mask_sm100.cu", "grouped_softmax.cu", "retrieval.cu",
+SOURCES = ["api.cu", "attn_general.cu", "attn_f32.cu", "attn_sm100.cu", "attn_mask_sm100.cu", "grouped_softmax.cu", "retrieval.cu",
            "scores_sm100.cu", "cache_store.cu", "decode.cu",
            "block_cache.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -152,12 +152,23 @@ extern "C" int lmk_attn_bwd(const void* q, const void* k, const void* v, const v
                             size_t workspace_bytes, int B, int H, int Lq, int Lk, int D,
                             const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
                             int block, float sm_scale, int dtype, int path, void* stream) {
+  const int64_t dense[3] = {(int64_t)H * Lq * D, (int64_t)Lq * D, D};
+  return lmk_attn_bwd_strided(q, k, v, o, dO, L, M, dQ, dK, dV, workspace, workspace_bytes, B, H, Lq, Lk, D, q_strides, k_strides,
+                              v_strides, dense, block, sm_scale, dtype, path, stream);
+}
+
+extern "C" int lmk_attn_bwd_strided(const void* q, const void* k, const void* v, const void* o, const void* dO,
+                                    const float* L, const float* M, void* dQ, void* dK, void* dV, void* workspace,
+                                    size_t workspace_bytes, int B, int H, int Lq, int Lk, int D,
+                                    const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
+                                    const int64_t do_strides[3], int block, float sm_scale, int dtype, int path, void* stream) {
   int rc = check_common(q, k, v, B, H, Lq, Lk, D, q_strides, k_strides, v_strides, block, dtype, path);
   if (rc != LMK_OK) return rc;
-  LMK_CHECK_ARG(o && dO && L && M && dQ && dK && dV, "attn_bwd: null tensor pointer");
+  LMK_CHECK_ARG(o && dO && L && M && dQ && dK && dV && do_strides, "attn_bwd: null pointer");
   AttnParams p{};
   fill(p, q, k, v, B, H, Lq, Lk, D, q_strides, k_strides, v_strides, block, sm_scale);
   p.o = const_cast<void*>(o); p.dO = dO;
+  for (int i = 0; i < 3; ++i) p.dos[i] = do_strides[i];
   int which = pick_path(path, p, dtype, true);
   if (which < 0) return which;
   LMK_CHECK_ARG(which != LMK_PATH_GENERAL || (Lq % block == 0 && Lk % block == 0),
@@ -273,9 +284,19 @@ extern "C" int lmk_attn_mask_bwd(const void* q, const void* k, const void* v, co
                                  void* dQ, void* dK, void* dV, void* workspace, size_t workspace_bytes, int B, int H,
                                  int Lq, int Lk, int D, const int64_t q_strides[3], const int64_t k_strides[3],
                                  const int64_t v_strides[3], int max_groups, float sm_scale, int dtype, void* stream) {
+  const int64_t dense[3] = {(int64_t)H * Lq * D, (int64_t)Lq * D, D};
+  return lmk_attn_mask_bwd_strided(q, k, v, is_mem, is_mem_stride, o, dO, R, A, dQ, dK, dV, workspace, workspace_bytes, B, H, Lq, Lk,
+                                   D, q_strides, k_strides, v_strides, dense, max_groups, sm_scale, dtype, stream);
+}
+
+extern "C" int lmk_attn_mask_bwd_strided(const void* q, const void* k, const void* v, const uint8_t* is_mem,
+                                 int64_t is_mem_stride, const void* o, const void* dO, const float* R, const float* A,
+                                 void* dQ, void* dK, void* dV, void* workspace, size_t workspace_bytes, int B, int H,
+                                 int Lq, int Lk, int D, const int64_t q_strides[3], const int64_t k_strides[3],
+                                 const int64_t v_strides[3], const int64_t do_strides[3], int max_groups, float sm_scale, int dtype, void* stream) {
   int rc = check_mask_common(q, k, v, is_mem, B, H, Lq, Lk, D, q_strides, k_strides, v_strides, max_groups, dtype);
   if (rc != LMK_OK) return rc;
-  LMK_CHECK_ARG(o && dO && R && A && dQ && dK && dV, "attn_mask_bwd: null tensor pointer");
+  LMK_CHECK_ARG(o && dO && R && A && dQ && dK && dV && do_strides, "attn_mask_bwd: null pointer");
   const size_t need = attn_mask_sm100_bwd_workspace(B, H, Lq, max_groups);
   if (workspace == nullptr || workspace_bytes < need)
     return fail(LMK_ERR_WORKSPACE, "attn_mask_bwd: workspace of %zu bytes required, %zu given", need, workspace_bytes);
@@ -283,6 +304,7 @@ extern "C" int lmk_attn_mask_bwd(const void* q, const void* k, const void* v, co
   AttnParams p{};
   fill(p, q, k, v, B, H, Lq, Lk, D, q_strides, k_strides, v_strides, 0, sm_scale);
   p.o = const_cast<void*>(o); p.dO = dO;
+  for (int i = 0; i < 3; ++i) p.dos[i] = do_strides[i];
   p.dq = dQ; p.dk = dK; p.dv = dV;
   p.workspace = workspace; p.workspace_bytes = workspace_bytes;
   return attn_mask_sm100_bwd(p, is_mem, is_mem_stride, R, A, max_groups, dtype, (cudaStream_t)stream);

@@ -2,8 +2,7 @@
 //
 // These kernels cover every dtype (fp32 / fp16 / bf16), any head dim <= 128 that is a multiple of 32, any
 // landmark block size in [2, 128], a key prefix (Lk > Lq) and, in the forward pass, a ragged last block.
-// They are the path for fp32 inputs (where bf16 tensor-core products would miss the 1e-4 tolerance) and
-// for shapes the tcgen05 kernels do not take.
+// They are the path for shapes that neither the tcgen05 kernels nor the tiled fp32 kernels (attn_f32.cu: blocks of 64) take.
 //
 // Math (same quantities as the reference Triton kernels, llama/ltriton/flash_landmark_attention.py):
 //   query row at key position p, own block b = p / block.
@@ -211,10 +210,10 @@ __global__ void __launch_bounds__(kFwdWarps * 32) general_bwd_dq_kernel(AttnPara
   const T* kp = reinterpret_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const T* vp = reinterpret_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
   const T* op = reinterpret_cast<const T*>(p.o) + ((int64_t)bh * p.Lq) * D;
-  const T* dop = reinterpret_cast<const T*>(p.dO) + ((int64_t)bh * p.Lq) * D;
+  const T* dop = reinterpret_cast<const T*>(p.dO) + b * p.dos[0] + h * p.dos[1];
 
   load_rows_f32(Qs, D, qp, p.qs[2], q0, kFwdRows, p.Lq, D, tid, blockDim.x);
-  load_rows_f32(dOs, D, dop, (int64_t)D, q0, kFwdRows, p.Lq, D, tid, blockDim.x);
+  load_rows_f32(dOs, D, dop, p.dos[2], q0, kFwdRows, p.Lq, D, tid, blockDim.x);
   __syncthreads();
 
   int own[kRowsPerWarp], vis[kRowsPerWarp];
@@ -359,7 +358,7 @@ __global__ void __launch_bounds__(kDkvWarps * 32) general_bwd_dkv_kernel(AttnPar
   const T* qp = reinterpret_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const T* kp = reinterpret_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const T* vp = reinterpret_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
-  const T* dop = reinterpret_cast<const T*>(p.dO) + ((int64_t)bh * p.Lq) * D;
+  const T* dop = reinterpret_cast<const T*>(p.dO) + b * p.dos[0] + h * p.dos[1];
 
   load_rows_f32(Ks, DP, kp, p.ks[2], key0, blk, p.Lk, D, tid, blockDim.x);
   load_rows_f32(Vs, DP, vp, p.vs[2], key0, blk, p.Lk, D, tid, blockDim.x);
@@ -376,7 +375,7 @@ __global__ void __launch_bounds__(kDkvWarps * 32) general_bwd_dkv_kernel(AttnPar
   for (int t0 = (r_start / kDkvRows) * kDkvRows; t0 < p.Lq; t0 += kDkvRows) {
     __syncthreads();
     load_rows_f32(Qs, D, qp, p.qs[2], t0, kDkvRows, p.Lq, D, tid, blockDim.x);
-    load_rows_f32(dOs, D, dop, (int64_t)D, t0, kDkvRows, p.Lq, D, tid, blockDim.x);
+    load_rows_f32(dOs, D, dop, p.dos[2], t0, kDkvRows, p.Lq, D, tid, blockDim.x);
     __syncthreads();
     // phase 1: two rows per warp
 #pragma unroll
@@ -527,6 +526,8 @@ int launch_bwd(const AttnParams& p, cudaStream_t st) {
 }  // namespace
 
 int attn_general_fwd(const AttnParams& p, int dtype, cudaStream_t st) {
+  if (dtype == LMK_F32)
+    if (const int rc = attn_f32_fwd(p, st)) return rc < 0 ? rc : LMK_OK;
   switch (dtype) {
     case LMK_F32: return launch_fwd<float>(p, st);
     case LMK_F16: return launch_fwd<__half>(p, st);
@@ -535,6 +536,8 @@ int attn_general_fwd(const AttnParams& p, int dtype, cudaStream_t st) {
 }
 
 int attn_general_bwd(const AttnParams& p, int dtype, cudaStream_t st) {
+  if (dtype == LMK_F32)
+    if (const int rc = attn_f32_bwd(p, st)) return rc < 0 ? rc : LMK_OK;
   switch (dtype) {
     case LMK_F32: return launch_bwd<float>(p, st);
     case LMK_F16: return launch_bwd<__half>(p, st);

@@ -484,7 +484,7 @@ template <bool kBf16>
 __device__ __forceinline__ void mask_bwd_dq_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k,
                          const CUtensorMap& tm_v, const CUtensorMap& tm_do,
                          const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const void* __restrict__ o_ptr,
-                         const void* __restrict__ do_ptr, const float* __restrict__ R_ptr,
+                         const void* __restrict__ do_ptr, int64_t do_b, int64_t do_h, int64_t do_row, const float* __restrict__ R_ptr,
                          const float* __restrict__ A_ptr, float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
                          void* __restrict__ dq_ptr, int H, int Lq, int Lk, int G, float scale, float scale_log2,
                          const int* __restrict__ plan, int plan_stride, int* status,
@@ -613,7 +613,7 @@ __device__ __forceinline__ void mask_bwd_dq_tile(const CUtensorMap& tm_q, const 
     float delta = 0.f;
     {
       const uint4* orow = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(o_ptr) + grow * kD);
-      const uint4* grw = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(do_ptr) + grow * kD);
+      const uint4* grw = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(do_ptr) + b * do_b + h * do_h + (int64_t)(t * kQT + row) * do_row);
 #pragma unroll 4
       for (int c = 0; c < kD / 8; ++c) delta = dot8<kBf16>(orow[c], grw[c], delta);
     }
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(kMqThreads, 1)
 sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                          const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const void* __restrict__ o_ptr,
-                         const void* __restrict__ do_ptr, const float* __restrict__ R_ptr,
+                         const void* __restrict__ do_ptr, int64_t do_b, int64_t do_h, int64_t do_row, const float* __restrict__ R_ptr,
                          const float* __restrict__ A_ptr, float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
                          void* __restrict__ dq_ptr, int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2,
                          const int* __restrict__ plan, int plan_stride, int* status) {
@@ -772,7 +772,7 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       tmem = tmem_slot;
       held = true;
     }
-    mask_bwd_dq_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, o_ptr, do_ptr, R_ptr, A_ptr, delta_ptr, nD_ptr, dq_ptr, H, Lq, Lk, G, scale, scale_log2, plan, plan_stride, status, t, bh, tmem);
+    mask_bwd_dq_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, o_ptr, do_ptr, do_b, do_h, do_row, R_ptr, A_ptr, delta_ptr, nD_ptr, dq_ptr, H, Lq, Lk, G, scale, scale_log2, plan, plan_stride, status, t, bh, tmem);
   }
   if (held && warp == 5) {
     tc_fence_after();
@@ -1209,16 +1209,15 @@ size_t attn_mask_sm100_bwd_workspace(int B, int H, int Lq, int G) {
 int attn_mask_sm100_bwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_mem_stride, const float* R,
                         const float* A, int G, int dtype, cudaStream_t st) {
   if (!tensor_map_operand_ok(p.q, p.qs) || !tensor_map_operand_ok(p.k, p.ks) || !tensor_map_operand_ok(p.v, p.vs) ||
-      (uintptr_t)p.dO % 16 != 0 || (uintptr_t)p.o % 16 != 0)
+      !tensor_map_operand_ok(p.dO, p.dos) || (uintptr_t)p.o % 16 != 0)
     return fail(LMK_ERR_UNSUPPORTED, "masked attention needs 16-byte aligned tensors with strides that are multiples of 8");
   if (G < 1 || G > kMaxGroups) return fail(LMK_ERR_UNSUPPORTED, "max_groups must be in 1..%d (got %d)", kMaxGroups, G);
   CUtensorMap tq, tk, tv, tdo;
   int rc;
-  const int64_t dense[3] = {(int64_t)p.H * p.Lq * kD, (int64_t)p.Lq * kD, (int64_t)kD};
   if ((rc = tensor_map_4d(&tq, p.q, dtype, p.B, p.H, p.Lq, p.qs, kQT)) != LMK_OK) return rc;
   if ((rc = tensor_map_4d(&tk, p.k, dtype, p.B, p.H, p.Lk, p.ks, kKT)) != LMK_OK) return rc;
   if ((rc = tensor_map_4d(&tv, p.v, dtype, p.B, p.H, p.Lk, p.vs, kKT)) != LMK_OK) return rc;
-  if ((rc = tensor_map_4d(&tdo, p.dO, dtype, p.B, p.H, p.Lq, dense, kQT)) != LMK_OK) return rc;
+  if ((rc = tensor_map_4d(&tdo, p.dO, dtype, p.B, p.H, p.Lq, p.dos, kQT)) != LMK_OK) return rc;
   if ((rc = mask_kernel_attributes()) != LMK_OK) return rc;
   int* status = device_status_word();
   if (!status) return fail(LMK_ERR_CUDA, "cannot resolve the device status word");
@@ -1239,6 +1238,7 @@ int attn_mask_sm100_bwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
 #define LMK_MASK_BWD(BF)                                                                                                \
   do {                                                                                                                  \
     sm100_mask_bwd_dq_kernel<BF><<<grid_q, kMqThreads, smem_q, st>>>(tq, tk, tv, tdo, is_mem, is_mem_stride, p.o, p.dO,  \
+                                                                     p.dos[0], p.dos[1], p.dos[2],                      \
                                                                      R, A, delta, nD, p.dq, p.H, p.B * p.H, p.Lq, p.Lk, G, \
                                                                      p.scale, scale_log2, plan, plan_stride, status);   \
     sm100_mask_bwd_dkv_kernel<BF><<<grid_k, kMkThreads, kMkSmemBytes, st>>>(tq, tk, tv, tdo, is_mem, is_mem_stride, R,  \

@@ -17,9 +17,13 @@ struct AttnParams {
   void* workspace; size_t workspace_bytes;
   int B, H, Lq, Lk, D, block;
   int64_t qs[3], ks[3], vs[3];   // element strides {batch, head, row}
+  int64_t dos[3];                // of dO (backward)
   float scale;
 };
 
+// fp32 with blocks of 64 (attn_f32.cu): 1 = launched, 0 = not taken, < 0 = error
+int attn_f32_fwd(const AttnParams& p, cudaStream_t st);
+int attn_f32_bwd(const AttnParams& p, cudaStream_t st);
 int attn_general_fwd(const AttnParams& p, int dtype, cudaStream_t st);
 int attn_general_bwd(const AttnParams& p, int dtype, cudaStream_t st);
 size_t attn_general_bwd_workspace(int B, int H, int Lq);

@@ -1700,7 +1700,7 @@ bool attn_sm100_takes(int B, int H, int Lq, int Lk, int D, int block, int dtype)
 
 bool attn_sm100_operands_ok(const AttnParams& p, bool backward) {
   if (!tma_ok(p.q, p.qs, p.D) || !tma_ok(p.k, p.ks, p.D) || !tma_ok(p.v, p.vs, p.D)) return false;
-  if (backward && ((uintptr_t)p.dO % 16 != 0 || (uintptr_t)p.o % 16 != 0)) return false;
+  if (backward && (!tma_ok(p.dO, p.dos, p.D) || (uintptr_t)p.o % 16 != 0)) return false;
   return true;
 }
 
@@ -1798,7 +1798,7 @@ static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   if ((rc = make_map_4d(&tq, p.q, dtype, p.B, p.H, p.Lq, p.D, p.qs, kQTile)) != LMK_OK) return rc;
   if ((rc = make_map_4d(&tk, p.k, dtype, p.B, p.H, p.Lk, p.D, p.ks, kBlk)) != LMK_OK) return rc;
   if ((rc = make_map_4d(&tv, p.v, dtype, p.B, p.H, p.Lk, p.D, p.vs, kBlk)) != LMK_OK) return rc;
-  if ((rc = make_map_4d(&tdo, p.dO, dtype, p.B, p.H, p.Lq, p.D, dense, kQTile)) != LMK_OK) return rc;
+  if ((rc = make_map_4d(&tdo, p.dO, dtype, p.B, p.H, p.Lq, p.D, p.dos, kQTile)) != LMK_OK) return rc;
   float* delta = reinterpret_cast<float*>(p.workspace);
   const float scale_log2 = p.scale * kLog2e;
   const size_t smem_dkv = kSmemDkv, smem_dq = kSmemDq;

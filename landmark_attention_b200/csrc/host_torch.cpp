@@ -36,8 +36,8 @@ using torch::autograd::variable_list;
 
 // ------------------------------------------------------------------------------------------------ library functions
 #define LMK_FUNCS(X)                                                                                             \
-  X(lmk_last_error) X(lmk_attn_fwd) X(lmk_attn_bwd_workspace) X(lmk_attn_bwd) X(lmk_attn_mask_fwd)               \
-  X(lmk_attn_mask_bwd_workspace) X(lmk_attn_mask_bwd) X(lmk_grouped_softmax_fwd) X(lmk_grouped_softmax_bwd)      \
+  X(lmk_last_error) X(lmk_attn_fwd) X(lmk_attn_bwd_workspace) X(lmk_attn_bwd_strided) X(lmk_attn_mask_fwd)               \
+  X(lmk_attn_mask_bwd_workspace) X(lmk_attn_mask_bwd_strided) X(lmk_grouped_softmax_fwd) X(lmk_grouped_softmax_bwd)      \
   X(lmk_grouped_softmax_causal_fwd) X(lmk_grouped_softmax_causal_bwd) X(lmk_rotary_apply) X(lmk_mask_is_regular)        \
   X(lmk_decode_supported) X(lmk_decode_attend) X(lmk_block_select) X(lmk_block_select_supported)                  \
   X(lmk_prefix_gather) X(lmk_prefix_gather_supported) X(lmk_prefix_pv) X(lmk_landmark_scores)                     \
@@ -92,6 +92,15 @@ Tensor empty_like_dtype(at::IntArrayRef sizes, const Tensor& like) { return at::
 Tensor empty_f32(at::IntArrayRef sizes, const Tensor& like) {
   return at::empty(sizes, like.options().requires_grad(false).dtype(at::kFloat));
 }
+// dO as the kernels read it: q's type, dense features, rows of 16-byte vectors (a view of the output projection's gradient
+// comes as [B, L, H, D] and is read in place)
+Tensor grad_rows(const Tensor& g, const Tensor& q) {
+  const Tensor t = g.scalar_type() == q.scalar_type() ? g : g.to(q.scalar_type());
+  const int64_t vec = 16 / t.element_size(), D = t.size(3);
+  const bool ok = t.stride(3) == 1 && t.stride(0) > 0 && t.stride(1) > 0 && t.stride(0) % vec == 0 && t.stride(1) % vec == 0 &&
+                  t.stride(2) % vec == 0 && t.stride(2) >= D && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  return ok ? t : t.clone(at::MemoryFormat::Contiguous);
+}
 bool needs_grad(std::initializer_list<std::reference_wrapper<const Tensor>> ts) {
   if (!at::GradMode::is_enabled()) return false;
   for (const Tensor& t : ts) if (t.requires_grad()) return true;
@@ -129,16 +138,15 @@ struct FusedLandmark : public torch::autograd::Function<FusedLandmark> {
     const double scale = ctx->saved_data["scale"].toDouble();
     const auto B = q.size(0), H = q.size(1), Lq = q.size(2), D = q.size(3), Lk = k.size(2);
     c10::cuda::OptionalCUDAGuard guard(q.device());
-    Tensor dO = grads[0].contiguous();
-    if (dO.scalar_type() != q.scalar_type()) dO = dO.to(q.scalar_type());
+    const Tensor dO = grad_rows(grads[0], q);
     Tensor dq = empty_like_dtype({B, H, Lq, D}, q), dk = empty_like_dtype({B, H, Lk, D}, q), dv = empty_like_dtype({B, H, Lk, D}, q);
     const int code = dtype_code(q);
     const size_t need = std::max<size_t>(lib.lmk_attn_bwd_workspace(B, H, Lq, Lk, D, block, code, path), 256);
     Tensor ws = at::empty({(int64_t)need}, q.options().requires_grad(false).dtype(at::kByte));
     const float* l = stats.data_ptr<float>();
-    check(lib.lmk_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dO.data_ptr(), l, l + B * H * Lq,
+    check(lib.lmk_attn_bwd_strided(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dO.data_ptr(), l, l + B * H * Lq,
                            dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), need, B, H, Lq, Lk, D, S3(q).v,
-                           S3(k).v, S3(v).v, block, (float)scale, code, path, stream_of(q)),
+                           S3(k).v, S3(v).v, S3(dO).v, block, (float)scale, code, path, stream_of(q)),
           "lmk_attn_bwd");
     return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
   }
@@ -238,14 +246,13 @@ std::tuple<Tensor, Tensor, Tensor> masked_bwd_cuda(const Tensor& q_, const Tenso
   const auto B = q_.size(0), H = q_.size(1), Lq = q_.size(2), D = q_.size(3), Lk = k_.size(2);
   c10::cuda::OptionalCUDAGuard guard(q_.device());
   const Tensor q = last_dim_dense(q_), k = last_dim_dense(k_), v = last_dim_dense(v_), m = flags_u8(is_mem), o = o_.contiguous();
-  Tensor dO = do_.contiguous();
-  if (dO.scalar_type() != q.scalar_type()) dO = dO.to(q.scalar_type());
+  const Tensor dO = grad_rows(do_, q);
   Tensor dq = empty_like_dtype({B, H, Lq, D}, q), dk = empty_like_dtype({B, H, Lk, D}, q), dv = empty_like_dtype({B, H, Lk, D}, q);
   const size_t need = std::max<size_t>(lib.lmk_attn_mask_bwd_workspace(B, H, Lq, G), 256);
   Tensor ws = at::empty({(int64_t)need}, q.options().requires_grad(false).dtype(at::kByte));
-  check(lib.lmk_attn_mask_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), (const uint8_t*)m.data_ptr(), m.stride(0), o.data_ptr(),
+  check(lib.lmk_attn_mask_bwd_strided(q.data_ptr(), k.data_ptr(), v.data_ptr(), (const uint8_t*)m.data_ptr(), m.stride(0), o.data_ptr(),
                               dO.data_ptr(), R.data_ptr<float>(), A.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                              ws.data_ptr(), need, B, H, Lq, Lk, D, S3(q).v, S3(k).v, S3(v).v, G, (float)scale,
+                              ws.data_ptr(), need, B, H, Lq, Lk, D, S3(q).v, S3(k).v, S3(v).v, S3(dO).v, G, (float)scale,
                               dtype_code(q), stream_of(q)),
         "lmk_attn_mask_bwd");
   return {dq, dk, dv};
@@ -270,11 +277,13 @@ struct MaskedLandmark : public torch::autograd::Function<MaskedLandmark> {
     auto [o, R, A] = masked_fwd_op().call(q, k, v, is_mem, scale, G);
     ctx->save_for_backward({q, k, v, is_mem, o, R, A});
     ctx->mark_non_differentiable({R, A});
+    ctx->set_materialize_grads(false);             // no zero gradients for the statistics
     ctx->saved_data["scale"] = scale;
     ctx->saved_data["groups"] = G;
     return {o, R, A};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     auto s = ctx->get_saved_variables();
     auto [dq, dk, dv] = masked_bwd_op().call(s[0], s[1], s[2], s[3], s[4], grads[0], s[5], s[6],
                                              ctx->saved_data["scale"].toDouble(), ctx->saved_data["groups"].toInt());
