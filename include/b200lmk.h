@@ -396,6 +396,26 @@ int lmk_selected_attend(const void* q, const void* k_cache, const lmk_cache_desc
                         int n_pos, int rotary, const void* o_local, const float* R_local, int64_t local_rows, void* out,
                         int B, int H, int T, int D, float sm_scale, int dtype, void* stream);
 
+/* lmk_attn_fwd for callers that merge its output with other keys: R [B*H, Lq] = log2 of the row's normaliser (the form that
+ * lmk_selected_attend takes) instead of L and M.  16-bit types and blocks of up to 64 keys (the tensor-core kernels).
+ */
+int lmk_attn_fwd_lse(const void* q, const void* k, const void* v, void* o, float* R, int B, int H, int Lq, int Lk, int D,
+                     const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3], int block,
+                     float sm_scale, int dtype, void* stream);
+
+/* lmk_gather_kv into a wider tensor: out_head_stride elements between the rows of consecutive (batch, head) pairs. */
+int lmk_gather_kv_to(const void* k_cache, const void* v_cache, const lmk_cache_desc* kdesc, const lmk_cache_desc* vdesc,
+                     const int32_t* idx, const void* cos_table, const void* sin_table, int n_pos, int rotary, void* k_out,
+                     void* v_out, int64_t out_head_stride, int B, int H, int T, int D, int dtype, void* stream);
+
+/* lmk_chunk_prepare without padding: rotated q (dense) and k, and a copy of v if v_copy is given, k_rot and v_copy with
+ * kv_head_stride elements between heads and dense rows (a part of a wider tensor), and the append if cache_k is given.
+ */
+int lmk_chunk_rotate(const void* q, const void* k, const void* v, const int64_t q_strides[3], const int64_t k_strides[3],
+                     const int64_t v_strides[3], const void* cos_table, const void* sin_table, int n_pos, int64_t pos0,
+                     void* q_rot, void* k_rot, void* v_copy, int64_t kv_head_stride, void* cache_k, void* cache_v,
+                     const int64_t cache_strides[3], int64_t cache_pos, int B, int H, int T, int D, int dtype, void* stream);
+
 /* Token generation behind a block cache in one launch (llama/llama_mem.py:318-430, 447-474 for inputs that stay inside the
  * unfinished block): rotate-half rotary of q and k_new at positions len .. len+T-1, landmark scores and the top_k selection per
  * (head, token), attention over the selected blocks (keys rotated at their slot positions), the unfinished block's cached

@@ -94,6 +94,12 @@ PROTOTYPES = {
     "lmk_selected_attend": (c_int, [c_void_p, c_void_p, POINTER(CacheDesc), c_void_p, POINTER(CacheDesc), c_void_p,
                                     c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int64, c_void_p, c_int,
                                     c_int, c_int, c_int, c_float, c_int, c_void_p]),
+    "lmk_attn_fwd_lse": (c_int, [c_void_p] * 5 + [c_int] * 5 + [POINTER(c_int64)] * 3 + [c_int, c_float, c_int, c_void_p]),
+    "lmk_gather_kv_to": (c_int, [c_void_p, c_void_p, POINTER(CacheDesc), POINTER(CacheDesc), c_void_p, c_void_p,
+                                 c_void_p, c_int, c_int, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int,
+                                 c_void_p]),
+    "lmk_chunk_rotate": (c_int, [c_void_p] * 3 + [POINTER(c_int64)] * 3 + [c_void_p, c_void_p, c_int, c_int64] + [c_void_p] * 3 +
+                         [c_int64, c_void_p, c_void_p, POINTER(c_int64), c_int64] + [c_int] * 5 + [c_void_p]),
     "lmk_decode_supported": (c_int, [c_int] * 6),
     "lmk_decode_attend": (c_int, [c_void_p] * 3 + [POINTER(c_int64)] * 3 + [c_void_p] * 2 + [POINTER(c_int64)] * 2 +
                           [c_int] * 4 + [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int,

@@ -137,6 +137,21 @@ extern "C" int lmk_attn_fwd(const void* q, const void* k, const void* v, void* o
   return attn_general_fwd(p, dtype, (cudaStream_t)stream);
 }
 
+extern "C" int lmk_attn_fwd_lse(const void* q, const void* k, const void* v, void* o, float* R, int B, int H, int Lq, int Lk, int D,
+                                const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3], int block,
+                                float sm_scale, int dtype, void* stream) {
+  int rc = check_common(q, k, v, B, H, Lq, Lk, D, q_strides, k_strides, v_strides, block, dtype, LMK_PATH_AUTO);
+  if (rc != LMK_OK) return rc;
+  LMK_CHECK_ARG(o && R, "attn_fwd_lse: o or R is null");
+  AttnParams p{};
+  fill(p, q, k, v, B, H, Lq, Lk, D, q_strides, k_strides, v_strides, block, sm_scale);
+  p.o = o;
+  const int which = pick_path(LMK_PATH_AUTO, p, dtype, false);
+  if (which < 0) return which;
+  if (which == LMK_PATH_GENERAL) return fail(LMK_ERR_UNSUPPORTED, "attn_fwd_lse runs on the tensor-core kernels only");
+  return attn_sm100_fwd_lse(p, R, dtype, (cudaStream_t)stream);
+}
+
 extern "C" size_t lmk_attn_bwd_workspace(int B, int H, int Lq, int Lk, int D, int block, int dtype, int path) {
   if (B < 1 || H < 1 || Lq < 1 || Lk < 1) return 0;
   // with LMK_PATH_AUTO the kernel family also depends on the operands' alignment, which is not known here: both

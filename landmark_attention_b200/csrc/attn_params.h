@@ -40,6 +40,7 @@ size_t attn_sm100_bwd_workspace(int B, int H, int Lq, int Lk, int D);
 bool attn_sm100_small_blocks(int B, int H, int Lq, int Lk, int D, int block, int dtype);
 int attn_sm100_small_blocks_fwd(const AttnParams& p, int dtype, cudaStream_t st);
 int attn_sm100_small_blocks_bwd(const AttnParams& p, int dtype, cudaStream_t st);
+int attn_sm100_fwd_lse(const AttnParams& p, float* R, int dtype, cudaStream_t st);
 bool attn_sm100_flags(int Lk, int G);
 int attn_sm100_flags_fwd(const AttnParams& p, const uint8_t* flags, int64_t stride, int G, float* R, int dtype, cudaStream_t st);
 int attn_sm100_flags_bwd(const AttnParams& p, const uint8_t* flags, int64_t stride, int G, const float* R, int* plan, int dtype,

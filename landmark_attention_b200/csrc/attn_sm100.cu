@@ -136,7 +136,7 @@ struct IrrArgs {
   int64_t stride = 0;
   int block = 0, G = 0;
   const int* plan = nullptr;           // backward, flags only: see irr_plan_kernel
-  float* R = nullptr;                  // flags only: log2 of the row's normaliser instead of L and M
+  float* R = nullptr;                  // log2 of the row's normaliser instead of L and M (always with flags; forward otherwise)
 };
 
 // landmark positions and per-key landmark counts of one batch row, in shared memory
@@ -589,7 +589,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
     }
     if (stored) {
-      if (kIrr && irr.R != nullptr) {
+      if (irr.R != nullptr) {
         irr.R[(int64_t)bh * Lq + grow] = l > 0.f ? m2 + __log2f(l) : INFINITY;
       } else {
         L_ptr[(int64_t)bh * Lq + grow] = l;
@@ -1732,13 +1732,14 @@ static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   if ((rc = make_map_4d(&tv, p.v, dtype, p.B, p.H, p.Lk, p.D, p.vs, kBlk)) != LMK_OK) return rc;
   const int whole_blocks = p.Lk / kBlk;
   const int lm_box = whole_blocks < 1 ? 1 : (whole_blocks < 64 ? whole_blocks : 64);
-  if (irr != nullptr) tl = tk;      // not read
+  const bool other = irr != nullptr && (irr->flags != nullptr || irr->block != 0);      // not the block-64 pattern
+  if (other) tl = tk;               // not read
   else if ((rc = make_map_landmarks(&tl, p.k, dtype, p.B, p.H, p.Lk, p.D, p.ks, lm_box)) != LMK_OK) return rc;
   const float scale_log2 = p.scale * kLog2e;
   const DeviceFacts* facts = nullptr;
   if ((rc = device_facts(&facts)) != LMK_OK) return rc;
   const int n_tiles = (p.Lq + kQTile - 1) / kQTile;
-  const int per_cta = fwd_tiles_per_cta(n_tiles, p.B * p.H, facts->n_sm, irr != nullptr);
+  const int per_cta = fwd_tiles_per_cta(n_tiles, p.B * p.H, facts->n_sm, other);
   const dim3 grid(p.B * p.H, (n_tiles + per_cta - 1) / per_cta);
 #define LMK_FWD_LAUNCH(BF, DIM, IRR, TILES)                                                                              \
   sm100_fwd2_kernel<BF, DIM, IRR, TILES><<<grid, kFwdThreads<TILES>, fwd_smem<TILES>(IRR), st>>>(                        \
@@ -1749,7 +1750,7 @@ static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   } while (0)
 #define LMK_FWD_DTYPE(BF)                                                                     \
   do {                                                                                        \
-    if (irr != nullptr) {                                                                     \
+    if (other) {                                                                     \
       if (p.D <= 64) LMK_FWD_TILES(BF, 64, true); else LMK_FWD_TILES(BF, 128, true);          \
     } else {                                                                                  \
       if (p.D <= 64) LMK_FWD_TILES(BF, 64, false); else LMK_FWD_TILES(BF, 128, false);        \
@@ -1775,6 +1776,13 @@ bool attn_sm100_small_blocks(int B, int H, int Lq, int Lk, int D, int block, int
 int attn_sm100_small_blocks_fwd(const AttnParams& p, int dtype, cudaStream_t st) {
   IrrArgs a;
   a.block = p.block;
+  return launch_fwd(p, dtype, &a, st);
+}
+// forward only, R instead of p.L and p.M (blocks of 64 or below)
+int attn_sm100_fwd_lse(const AttnParams& p, float* R, int dtype, cudaStream_t st) {
+  IrrArgs a;
+  a.block = p.block == kBlk ? 0 : p.block;
+  a.R = R;
   return launch_fwd(p, dtype, &a, st);
 }
 // landmarks anywhere: p.o and R; rows of the batch left to the two-pass kernels are marked in R

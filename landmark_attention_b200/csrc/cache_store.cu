@@ -68,7 +68,8 @@ struct PrepParams {
   int64_t pos0;
   const uint8_t* chunk_flags;
   int block;
-  void *q_rot, *q_pad, *k_pad, *v_pad;
+  void *q_rot, *q_pad, *k_pad, *v_pad;  // q_pad, v_pad, flags_pad may be null
+  int64_t pad_head;                     // elements between the heads of k_pad, v_pad (and q_pad)
   uint8_t* flags_pad;
   void *cache_k, *cache_v;
   int64_t cs[3];                        // cache element strides {batch, head, row}
@@ -87,13 +88,13 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepParams p) {
   if (threadIdx.x >= rows_per_cta * lp || t >= p.t_pad) return;
   auto vec = [](const void* base, int64_t off) { return *reinterpret_cast<const uint4*>(static_cast<const T*>(base) + off); };
   auto put = [](void* base, int64_t off, const uint4& w) { *reinterpret_cast<uint4*>(static_cast<T*>(base) + off) = w; };
-  const int64_t pad_off = ((int64_t)bh * p.t_pad + t) * p.D + d0;
+  const int64_t pad_off = bh * p.pad_head + (int64_t)t * p.D + d0;
   if (t >= p.T) {                                  // padding rows of the tiles
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    put(p.q_pad, pad_off, z); put(p.q_pad, pad_off + half, z);
+    if (p.q_pad != nullptr) { put(p.q_pad, pad_off, z); put(p.q_pad, pad_off + half, z); }
     put(p.k_pad, pad_off, z); put(p.k_pad, pad_off + half, z);
-    put(p.v_pad, pad_off, z); put(p.v_pad, pad_off + half, z);
-    if (h == 0 && sub == 0) p.flags_pad[(int64_t)b * p.t_pad + t] = 0;
+    if (p.v_pad != nullptr) { put(p.v_pad, pad_off, z); put(p.v_pad, pad_off + half, z); }
+    if (p.flags_pad != nullptr && h == 0 && sub == 0) p.flags_pad[(int64_t)b * p.t_pad + t] = 0;
     return;
   }
   const int64_t pos = min(p.pos0 + t, (int64_t)p.n_pos - 1);
@@ -114,10 +115,10 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepParams p) {
   rotate_half_pair<T>(kl, kh, cl, ch, sl, sh);
   const int64_t rot_off = ((int64_t)bh * p.T + t) * p.D + d0;
   put(p.q_rot, rot_off, ql); put(p.q_rot, rot_off + half, qh);
-  put(p.q_pad, pad_off, ql); put(p.q_pad, pad_off + half, qh);
+  if (p.q_pad != nullptr) { put(p.q_pad, pad_off, ql); put(p.q_pad, pad_off + half, qh); }
   put(p.k_pad, pad_off, kl); put(p.k_pad, pad_off + half, kh);
-  put(p.v_pad, pad_off, vl); put(p.v_pad, pad_off + half, vh);
-  if (h == 0 && sub == 0)
+  if (p.v_pad != nullptr) { put(p.v_pad, pad_off, vl); put(p.v_pad, pad_off + half, vh); }
+  if (p.flags_pad != nullptr && h == 0 && sub == 0)
     p.flags_pad[(int64_t)b * p.t_pad + t] =
         p.chunk_flags != nullptr ? (p.chunk_flags[t] != 0) : ((p.pos0 + t) % p.block == p.block - 1);
 }
@@ -260,15 +261,16 @@ extern "C" int lmk_cache_store(const void* k_src, const void* v_src, const int64
   return LMK_OK;
 }
 
-extern "C" int lmk_chunk_prepare(const void* q, const void* k, const void* v, const int64_t q_strides[3],
+static int chunk_prepare(const void* q, const void* k, const void* v, const int64_t q_strides[3],
                                  const int64_t k_strides[3], const int64_t v_strides[3], const void* cos_table,
                                  const void* sin_table, int n_pos, int64_t pos0, const uint8_t* chunk_flags, int block,
-                                 void* q_rot, void* q_pad, void* k_pad, void* v_pad, uint8_t* flags_pad, void* cache_k,
+                                 void* q_rot, void* q_pad, void* k_pad, void* v_pad, int64_t pad_head,
+                         uint8_t* flags_pad, void* cache_k,
                                  void* cache_v, const int64_t cache_strides[3], int64_t cache_pos, int B, int H, int T,
                                  int t_pad, int D, int dtype, void* stream) {
   using namespace lmk;
-  LMK_CHECK_ARG(q && k && v && q_strides && k_strides && v_strides && cos_table && sin_table && q_rot && q_pad &&
-                    k_pad && v_pad && flags_pad, "chunk_prepare: null pointer");
+  LMK_CHECK_ARG(q && k && v && q_strides && k_strides && v_strides && cos_table && sin_table && q_rot && k_pad,
+                "chunk_prepare: null pointer");
   LMK_CHECK_ARG(dtype == LMK_F16 || dtype == LMK_BF16, "chunk_prepare: 16-bit types only (dtype %d)", dtype);
   LMK_CHECK_ARG(B >= 0 && H >= 1 && T >= 1 && t_pad >= T, "chunk_prepare: bad shape");
   LMK_CHECK_ARG(D >= 16 && D <= 2048 && D % 16 == 0 && 128 % (D / 16) == 0,
@@ -279,6 +281,7 @@ extern "C" int lmk_chunk_prepare(const void* q, const void* k, const void* v, co
   uintptr_t align = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)cos_table | (uintptr_t)sin_table |
                     (uintptr_t)q_rot | (uintptr_t)q_pad | (uintptr_t)k_pad | (uintptr_t)v_pad | (uintptr_t)cache_k |
                     (uintptr_t)cache_v;
+  LMK_CHECK_ARG(pad_head % 8 == 0, "chunk_prepare: output strides must be multiples of 8 elements");
   LMK_CHECK_ARG((align & 15) == 0, "chunk_prepare: pointers must be 16-byte aligned");
   for (int i = 0; i < 3; ++i) {
     LMK_CHECK_ARG(q_strides[i] % 8 == 0 && k_strides[i] % 8 == 0 && v_strides[i] % 8 == 0,
@@ -295,6 +298,7 @@ extern "C" int lmk_chunk_prepare(const void* q, const void* k, const void* v, co
   }
   p.cos_t = cos_table; p.sin_t = sin_table; p.n_pos = n_pos; p.pos0 = pos0;
   p.chunk_flags = chunk_flags; p.block = block;
+  p.pad_head = pad_head;
   p.q_rot = q_rot; p.q_pad = q_pad; p.k_pad = k_pad; p.v_pad = v_pad; p.flags_pad = flags_pad;
   p.cache_k = cache_k; p.cache_v = cache_v; p.cache_pos = cache_pos;
   p.H = H; p.T = T; p.t_pad = t_pad; p.D = D;
@@ -304,6 +308,27 @@ extern "C" int lmk_chunk_prepare(const void* q, const void* k, const void* v, co
   else chunk_prepare_kernel<__half><<<grid, 128, 0, (cudaStream_t)stream>>>(p);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
+}
+
+extern "C" int lmk_chunk_prepare(const void* q, const void* k, const void* v, const int64_t q_strides[3],
+                                 const int64_t k_strides[3], const int64_t v_strides[3], const void* cos_table,
+                                 const void* sin_table, int n_pos, int64_t pos0, const uint8_t* chunk_flags, int block,
+                                 void* q_rot, void* q_pad, void* k_pad, void* v_pad, uint8_t* flags_pad, void* cache_k,
+                                 void* cache_v, const int64_t cache_strides[3], int64_t cache_pos, int B, int H, int T,
+                                 int t_pad, int D, int dtype, void* stream) {
+  using namespace lmk;
+  LMK_CHECK_ARG(q_pad && v_pad && flags_pad, "chunk_prepare: null pointer");
+  return chunk_prepare(q, k, v, q_strides, k_strides, v_strides, cos_table, sin_table, n_pos, pos0, chunk_flags, block, q_rot, q_pad, k_pad, v_pad,
+                       (int64_t)t_pad * D, flags_pad, cache_k, cache_v, cache_strides, cache_pos, B, H, T, t_pad, D, dtype, stream);
+}
+
+extern "C" int lmk_chunk_rotate(const void* q, const void* k, const void* v, const int64_t q_strides[3], const int64_t k_strides[3],
+                                const int64_t v_strides[3], const void* cos_table, const void* sin_table, int n_pos, int64_t pos0,
+                                void* q_rot, void* k_rot, void* v_copy, int64_t kv_head_stride, void* cache_k, void* cache_v,
+                                const int64_t cache_strides[3], int64_t cache_pos, int B, int H, int T, int D, int dtype,
+                                void* stream) {
+  return chunk_prepare(q, k, v, q_strides, k_strides, v_strides, cos_table, sin_table, n_pos, pos0, nullptr, 1, q_rot, nullptr, k_rot,
+                       v_copy, kv_head_stride, nullptr, cache_k, cache_v, cache_strides, cache_pos, B, H, T, T, D, dtype, stream);
 }
 
 extern "C" int lmk_rotary_apply(const void* q, const void* k, const int64_t q_strides[3], const int64_t k_strides[3],

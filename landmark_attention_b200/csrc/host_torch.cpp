@@ -41,7 +41,8 @@ using torch::autograd::variable_list;
   X(lmk_grouped_softmax_causal_fwd) X(lmk_grouped_softmax_causal_bwd) X(lmk_rotary_apply) X(lmk_mask_is_regular)        \
   X(lmk_decode_supported) X(lmk_decode_attend) X(lmk_block_select) X(lmk_block_select_supported)                  \
   X(lmk_prefix_gather) X(lmk_prefix_gather_supported) X(lmk_prefix_pv) X(lmk_landmark_scores)                     \
-  X(lmk_landmark_scores_workspace) X(lmk_topk_sorted)
+  X(lmk_landmark_scores_workspace) X(lmk_topk_sorted) X(lmk_chunk_rotate) X(lmk_attn_fwd_lse)                     \
+  X(lmk_selected_attend) X(lmk_gather_kv_to)
 struct Lib {
 #define X(name) decltype(&::name) name = nullptr;
   LMK_FUNCS(X)
@@ -592,6 +593,168 @@ bool prefix_pv(const Tensor& probs, const Tensor& v, const Tensor& y) {
   return true;
 }
 
+// ---- a chunk of a prompt behind a block cache (llama/llama_mem.py:318-430, 447-474), 16-bit types, head dim 128
+struct Chunk {
+  Tensor q, k, v;                 // rows of 16-byte vectors
+  int64_t B = 0, H = 0, T = 0, D = 0;
+  int code = 0;
+  float scale = 0.f;
+  void* stream = nullptr;
+};
+bool table_ok(const Tensor& t, const Tensor& q) {
+  return t.is_cuda() && t.scalar_type() == q.scalar_type() && t.is_contiguous() && t.dim() == 2 && t.size(1) == q.size(3) &&
+         (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+bool rows_ok(const Tensor& t) {      // a cache [B, H, rows, D]
+  return t.dim() == 4 && t.stride(3) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && t.stride(2) % 8 == 0 &&
+         (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+bool chunk_of(Chunk* c, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& kc, const Tensor& vc, const Tensor& cos,
+              const Tensor& sin) {
+  const auto st = q.scalar_type();
+  if (!q.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || q.dim() != 4 || q.size(3) != 128 || k.sizes() != q.sizes() ||
+      v.sizes() != q.sizes() || k.scalar_type() != st || v.scalar_type() != st || !k.is_cuda() || !v.is_cuda() ||
+      kc.scalar_type() != st || vc.scalar_type() != st || !rows_ok(kc) || !rows_ok(vc) || kc.strides() != vc.strides() ||
+      kc.size(0) != q.size(0) || kc.size(1) != q.size(1) || kc.size(3) != q.size(3) || !table_ok(cos, q) || !table_ok(sin, q) ||
+      q.size(0) * q.size(1) > 65535)
+    return false;
+  c->B = q.size(0), c->H = q.size(1), c->T = q.size(2), c->D = q.size(3);
+  c->q = vector_rows(q), c->k = vector_rows(k), c->v = vector_rows(v);
+  c->code = dtype_code(q);
+  c->scale = 1.0 / std::sqrt((double)c->D);
+  c->stream = stream_of(q);
+  return true;
+}
+lmk_cache_desc rows_desc(const Tensor& cache, int64_t n, int64_t block, int64_t top_k) {
+  lmk_cache_desc d{};
+  d.stride_b = cache.stride(0);
+  d.stride_h = cache.stride(1);
+  d.stride_block = cache.stride(2) * block;
+  d.stride_row = cache.stride(2);
+  d.n_blocks = n;
+  d.block = block;
+  d.top_k = top_k;
+  d.pos_base = (n - top_k - 1) * block;
+  return d;
+}
+Tensor landmark_scores(const Chunk& c, const Tensor& q_rot, const Tensor& keys, const lmk_cache_desc& d, const Tensor& cos,
+                       const Tensor& sin, bool softmax) {
+  Tensor s = empty_f32({c.B, c.H, c.T, d.n_blocks}, q_rot);
+  if (softmax && lib.lmk_block_select_supported(c.D, d.n_blocks, d.top_k, c.code)) {
+    check(lib.lmk_block_select(q_rot.data_ptr(), keys.data_ptr(), &d, cos.data_ptr(), sin.data_ptr(), cos.size(0), LMK_ROTARY_HALF,
+                               s.data_ptr<float>(), nullptr, c.B, c.H, c.T, c.D, c.scale, c.code, c.stream), "lmk_block_select");
+    return s;
+  }
+  const size_t need = lib.lmk_landmark_scores_workspace(c.B, c.H, c.T, c.D, d.n_blocks, c.code);
+  Tensor ws = need ? at::empty({(int64_t)need}, q_rot.options().dtype(at::kByte)) : Tensor();
+  check(lib.lmk_landmark_scores(q_rot.data_ptr(), keys.data_ptr(), &d, cos.data_ptr(), sin.data_ptr(), cos.size(0), LMK_ROTARY_HALF,
+                                s.data_ptr<float>(), c.B, c.H, c.T, c.D, c.scale, softmax, c.code, need ? ws.data_ptr() : nullptr, need,
+                                c.stream), "lmk_landmark_scores");
+  return s;
+}
+
+// One selection per (head, token); `len` whole-block tokens in the caches; append: k, v stored behind them.
+Tensor chunk_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& kc, const Tensor& vc, int64_t len, bool append,
+                    int64_t block, int64_t top_k, const Tensor& cos, const Tensor& sin, int64_t rotary) {
+  if (block < 2 || block > 64 || len % block != 0 || len < block || (q_.size(2) - 1) / block > 64 || top_k < 1 || top_k > 32) return Tensor();
+  const int64_t n = len / block;
+  Chunk c;
+  if (n > 49152 || kc.size(2) < len + (append ? q_.size(2) : 0) || !kc.is_cuda() || !vc.is_cuda() || !chunk_of(&c, q_, k_, v_, kc, vc, cos, sin))
+    return Tensor();
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const lmk_cache_desc d = rows_desc(kc, n, block, top_k);
+  Tensor qr = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q), kr = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q);
+  check(lib.lmk_chunk_rotate(c.q.data_ptr(), c.k.data_ptr(), c.v.data_ptr(), S3(c.q).v, S3(c.k).v, S3(c.v).v, cos.data_ptr(),
+                             sin.data_ptr(), cos.size(0), len, qr.data_ptr(), kr.data_ptr(), nullptr, c.T * c.D,
+                             append ? kc.data_ptr() : nullptr, append ? vc.data_ptr() : nullptr, append ? S3(kc).v : nullptr, len, c.B,
+                             c.H, c.T, c.D, c.code, c.stream), "lmk_chunk_rotate");
+  const Tensor s = landmark_scores(c, qr, kc, d, cos, sin, false);
+  Tensor idx = at::empty({c.B, c.H, c.T, top_k}, c.q.options().requires_grad(false).dtype(at::kInt));
+  check(lib.lmk_topk_sorted(s.data_ptr<float>(), idx.data_ptr<int>(), c.B * c.H * c.T, 1, n, 0, 1, 0, n, top_k, 0, c.stream), "lmk_topk_sorted");
+  Tensor o = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q), R = empty_f32({c.B * c.H, c.T}, c.q);
+  check(lib.lmk_attn_fwd_lse(qr.data_ptr(), kr.data_ptr(), c.v.data_ptr(), o.data_ptr(), R.data_ptr<float>(), c.B, c.H, c.T, c.T, c.D,
+                             S3(qr).v, S3(kr).v, S3(c.v).v, block, c.scale, c.code, c.stream), "lmk_attn_fwd_lse");
+  Tensor out = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q);
+  check(lib.lmk_selected_attend(qr.data_ptr(), kc.data_ptr(), &d, vc.data_ptr(), &d, idx.data_ptr<int>(), cos.data_ptr(), sin.data_ptr(),
+                                cos.size(0), rotary, o.data_ptr(), R.data_ptr<float>(), c.T, out.data_ptr(), c.B, c.H, c.T, c.D, c.scale,
+                                c.code, c.stream), "lmk_selected_attend");
+  return out;
+}
+
+// A second stream for the part of a call that nothing else in it waits for, with the events of the fork and the join (one set per
+// thread and device, reused: a wait refers to the event's state when it is enqueued).
+struct Fork {
+  c10::cuda::CUDAStream side;
+  cudaEvent_t begin, end;
+};
+Fork fork_of(int dev) {
+  constexpr int kMax = 64;
+  static thread_local cudaEvent_t events[kMax][2] = {};
+  TORCH_CHECK(dev >= 0 && dev < kMax, "device index out of range");
+  for (auto& e : events[dev])
+    if (e == nullptr) C10_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return {c10::cuda::getStreamFromPool(false, dev), events[dev][0], events[dev][1]};
+}
+
+// One selection per head, the maximum over the chunk's tokens; the chunk then attends to [selected blocks | chunk].  The caches hold
+// n blocks, on the device (lm undefined: landmarks are read from kc; append: k, v stored behind the n blocks) or in pinned host memory
+// (lm: their landmark keys; append: the chunk's whole blocks stored, on a second stream, because the writes over the host link
+// do not depend on the attention and run against the direction of its reads).
+Tensor per_head_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& kc, const Tensor& vc, const Tensor& lm, int64_t n,
+                       bool append, int64_t block, int64_t top_k, const Tensor& cos, const Tensor& sin) {
+  const bool host = lm.defined();
+  Chunk c;
+  if (block < 1 || n < 1 || n > 49152 || top_k < 1 || top_k > 32 || kc.is_cuda() == host || vc.is_cuda() == host ||
+      kc.size(2) < n * block + (append ? q_.size(2) : 0) || !chunk_of(&c, q_, k_, v_, kc, vc, cos, sin))
+    return Tensor();
+  if (host && (!kc.is_pinned() || !vc.is_pinned() || kc.stride(2) != c.D || lm.scalar_type() != q_.scalar_type() || !rows_ok(lm) || lm.size(2) < n || (append && c.T % block != 0)))
+    return Tensor();
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const lmk_cache_desc d = rows_desc(kc, n, block, top_k);
+  lmk_cache_desc ld = d;
+  if (host) {
+    ld.stride_b = lm.stride(0);
+    ld.stride_h = lm.stride(1);
+    ld.stride_block = lm.stride(2);
+    ld.stride_row = 0;
+  }
+  std::optional<Fork> fork;
+  if (host && append) {
+    // by the copy engine: the same stores from a kernel fill the memory system's queues towards the host link and slow down
+    // everything that runs beside them (the rotary kernel 4 -> 35 us)
+    c.k = c.k.contiguous(), c.v = c.v.contiguous();
+    fork = fork_of(q_.get_device());
+    C10_CUDA_CHECK(cudaEventRecord(fork->begin, (cudaStream_t)c.stream));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(fork->side.stream(), fork->begin, 0));
+    const size_t width = (size_t)c.T * c.D * 2, pitch = (size_t)kc.stride(1) * 2, at = (size_t)n * block * c.D * 2;
+    const bool one = kc.stride(0) == c.H * kc.stride(1);      // one copy for all (batch, head) pairs
+    for (int64_t b = 0; b < (one ? 1 : c.B); ++b)
+      for (const auto& [dst, src] : {std::pair(&kc, &c.k), std::pair(&vc, &c.v)})
+        C10_CUDA_CHECK(cudaMemcpy2DAsync(static_cast<char*>(dst->data_ptr()) + b * dst->stride(0) * 2 + at, pitch,
+                                         static_cast<const char*>(src->data_ptr()) + b * src->stride(0) * 2, width, width,
+                                         one ? c.B * c.H : c.H, cudaMemcpyDeviceToHost, fork->side.stream()));
+    C10_CUDA_CHECK(cudaEventRecord(fork->end, fork->side.stream()));
+    lm.narrow(2, n, c.T / block).copy_(c.k.slice(2, block - 1, c.T, block));
+  }
+  const bool device_append = append && !host;
+  const int64_t P = top_k * block, W = P + c.T;
+  Tensor qr = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q), keys = empty_like_dtype({c.B, c.H, W, c.D}, c.q), vals = empty_like_dtype({c.B, c.H, W, c.D}, c.q);
+  auto behind = [&](const Tensor& t) { return static_cast<uint16_t*>(t.data_ptr()) + P * c.D; };
+  check(lib.lmk_chunk_rotate(c.q.data_ptr(), c.k.data_ptr(), c.v.data_ptr(), S3(c.q).v, S3(c.k).v, S3(c.v).v, cos.data_ptr(),
+                             sin.data_ptr(), cos.size(0), n * block, qr.data_ptr(), behind(keys), behind(vals), W * c.D,
+                             device_append ? kc.data_ptr() : nullptr, device_append ? vc.data_ptr() : nullptr,
+                             device_append ? S3(kc).v : nullptr, n * block, c.B, c.H, c.T, c.D, c.code, c.stream), "lmk_chunk_rotate");
+  const Tensor probs = landmark_scores(c, qr, host ? lm : kc, ld, cos, sin, true);
+  Tensor idx = at::empty({c.B, c.H, 1, top_k}, c.q.options().requires_grad(false).dtype(at::kInt));
+  check(lib.lmk_topk_sorted(probs.data_ptr<float>(), idx.data_ptr<int>(), c.B * c.H, 1, c.T * n, 0, c.T, n, n, top_k, 0, c.stream), "lmk_topk_sorted");
+  check(lib.lmk_gather_kv_to(kc.data_ptr(), vc.data_ptr(), &d, &d, idx.data_ptr<int>(), cos.data_ptr(), sin.data_ptr(), cos.size(0), LMK_ROTARY_HALF,
+                             keys.data_ptr(), vals.data_ptr(), W * c.D, c.B, c.H, 1, c.D, c.code, c.stream), "lmk_gather_kv");
+  Tensor stats;
+  Tensor out = attn_fwd(qr, keys, vals, c.scale, block, LMK_PATH_AUTO, &stats);
+  if (fork) C10_CUDA_CHECK(cudaStreamWaitEvent((cudaStream_t)c.stream, fork->end, 0));
+  return out;
+}
+
 // ------------------------------------------------------------------------------------------------ Python entry points
 const Tensor& tensor_arg(PyObject* o, const char* name) {
   if (!THPVariable_Check(o)) {
@@ -742,6 +905,26 @@ PyObject* py_prefix_pv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// chunk_attend(q, k_new, v_new, k_cache, v_cache, len, append, block, top_k, cos, sin, rotary) -> out | None
+PyObject* py_chunk_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 12);
+  return wrap_opt(chunk_attend(tensor_arg(a[0], "q"), tensor_arg(a[1], "k_new"), tensor_arg(a[2], "v_new"), tensor_arg(a[3], "k_cache"),
+                               tensor_arg(a[4], "v_cache"), int_arg(a[5]), int_arg(a[6]) != 0, int_arg(a[7]), int_arg(a[8]),
+                               tensor_arg(a[9], "cos"), tensor_arg(a[10], "sin"), int_arg(a[11])));
+  END_HANDLE_TH_ERRORS
+}
+
+// per_head_attend(q, k_new, v_new, k_cache, v_cache, landmark keys | None, n_blocks, append, block, top_k, cos, sin) -> out | None
+PyObject* py_per_head_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 12);
+  return wrap_opt(per_head_attend(tensor_arg(a[0], "q"), tensor_arg(a[1], "k_new"), tensor_arg(a[2], "v_new"), tensor_arg(a[3], "k_cache"),
+                                  tensor_arg(a[4], "v_cache"), opt_tensor_arg(a[5], "landmark keys"), int_arg(a[6]), int_arg(a[7]) != 0,
+                                  int_arg(a[8]), int_arg(a[9]), tensor_arg(a[10], "cos"), tensor_arg(a[11], "sin")));
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST("fused_attention", py_fused_attention),
@@ -751,6 +934,8 @@ PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST("grouped_softmax", py_grouped_softmax),
                          FAST("grouped_softmax_causal", py_grouped_softmax_causal),
                          FAST("decode_attend", py_decode_attend),
+                         FAST("chunk_attend", py_chunk_attend),
+                         FAST("per_head_attend", py_per_head_attend),
                          FAST("cache_retrieve", py_cache_retrieve),
                          FAST("prefix_pv", py_prefix_pv),
                          {nullptr, nullptr, 0, nullptr}};

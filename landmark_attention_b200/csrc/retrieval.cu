@@ -421,8 +421,8 @@ __global__ void __launch_bounds__(128) gather_kv_kernel(const T* __restrict__ kc
                                                         lmk_cache_desc kd, lmk_cache_desc vd,
                                                         const int32_t* __restrict__ idx, const T* __restrict__ cos_t,
                                                         const T* __restrict__ sin_t, int n_pos, int rotary,
-                                                        T* __restrict__ k_out, T* __restrict__ v_out, int H, int Tq,
-                                                        int D) {
+                                                        T* __restrict__ k_out, T* __restrict__ v_out, int64_t out_head,
+                                                        int H, int Tq, int D) {
   constexpr int VEC = 16 / sizeof(T);
   struct __align__(16) Vec { T v[VEC]; };
   const int i = blockIdx.x, t = blockIdx.y, bh = blockIdx.z;
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(128) gather_kv_kernel(const T* __restrict__ kc
   const bool recent = logical_age(sel, kd.ring_start, N) >= N - top_k;
   const int pos0 = kd.pos_base + (i + (recent ? 1 : 0)) * blk;
   const int vec_per_row = D / VEC;
-  const int64_t out_base = (((int64_t)bh * Tq + t) * top_k + i) * blk * D;
+  const int64_t out_base = (int64_t)bh * out_head + ((int64_t)t * top_k + i) * blk * D;
   const T* ksrc = kc + b * kd.stride_b + h * kd.stride_h + (int64_t)sel * kd.stride_block;
   const T* vsrc = vc ? vc + b * vd.stride_b + h * vd.stride_h + (int64_t)sel * vd.stride_block : nullptr;
   for (int e = threadIdx.x; e < blk * vec_per_row; e += blockDim.x) {
@@ -1037,6 +1037,15 @@ extern "C" int lmk_gather_kv(const void* k_cache, const void* v_cache, const lmk
                              const lmk_cache_desc* vdesc, const int32_t* idx, const void* cos_table,
                              const void* sin_table, int n_pos, int rotary, void* k_out, void* v_out, int B, int H,
                              int T, int D, int dtype, void* stream) {
+  const int64_t dense = kdesc != nullptr ? (int64_t)T * kdesc->top_k * kdesc->block * D : 0;
+  return lmk_gather_kv_to(k_cache, v_cache, kdesc, vdesc, idx, cos_table, sin_table, n_pos, rotary, k_out, v_out, dense, B, H, T, D,
+                          dtype, stream);
+}
+
+extern "C" int lmk_gather_kv_to(const void* k_cache, const void* v_cache, const lmk_cache_desc* kdesc,
+                             const lmk_cache_desc* vdesc, const int32_t* idx, const void* cos_table,
+                             const void* sin_table, int n_pos, int rotary, void* k_out, void* v_out, int64_t out_head_stride, int B, int H,
+                             int T, int D, int dtype, void* stream) {
   int rc = check_desc(kdesc, "gather_kv");
   if (rc != LMK_OK) return rc;
   if (v_out != nullptr) {
@@ -1064,6 +1073,7 @@ extern "C" int lmk_gather_kv(const void* k_cache, const void* v_cache, const lmk
   LMK_CHECK_ARG(((uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)k_out | (uintptr_t)v_out |
                  (uintptr_t)cos_table | (uintptr_t)sin_table) % 16 == 0,
                 "gather_kv: pointers must be 16-byte aligned");
+  LMK_CHECK_ARG(out_head_stride % vec == 0, "gather_kv: output stride must be a multiple of %d elements", vec);
   LMK_CHECK_ARG((int64_t)B * H <= 65535 && T <= 65535, "gather_kv: grid too large");
   dim3 grid(kdesc->top_k, T, B * H);
   cudaStream_t st = (cudaStream_t)stream;
@@ -1071,7 +1081,7 @@ extern "C" int lmk_gather_kv(const void* k_cache, const void* v_cache, const lmk
 #define LMK_GA_LAUNCH(TT)                                                                                      \
   gather_kv_kernel<TT><<<grid, 128, 0, st>>>((const TT*)k_cache, (const TT*)v_cache, *kdesc, vd, idx,          \
                                              (const TT*)cos_table, (const TT*)sin_table, n_pos, rotary,        \
-                                             (TT*)k_out, (TT*)v_out, H, T, D)
+                                             (TT*)k_out, (TT*)v_out, out_head_stride, H, T, D)
   if (dtype == LMK_F32) LMK_GA_LAUNCH(float);
   else if (dtype == LMK_F16) LMK_GA_LAUNCH(__half);
   else LMK_GA_LAUNCH(__nv_bfloat16);

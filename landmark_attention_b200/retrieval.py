@@ -283,9 +283,9 @@ def llama_retrieval_attention(q, k_new, v_new, past_k=None, past_v=None, mem_fre
       materialize=True (what the reference does, :386-398): gathered [B,H,T,top_k*block,D] copies and matmuls.
     Returns (attn_output [B,H,T,D], new (past_k, past_v)).
     """
-    if (fused is None and materialize is None and not return_debug and aggregate is None and position_ids is None
-            and chunk_is_mem is None and cos is not None):
-        out = _decode(q, k_new, v_new, past_k, past_v, mem_freq + 1, cache_top_k, cos, sin, cache)
+    if (fused is None and materialize is None and not return_debug and position_ids is None and chunk_is_mem is None
+            and cos is not None and aggregate in (None, "max_over_tokens")):
+        out = _native(q, k_new, v_new, past_k, past_v, mem_freq + 1, cache_top_k, cos, sin, cache, aggregate is not None)
         if out is not None:
             return out
     if cache is not None:
@@ -409,14 +409,16 @@ def llama_retrieval_attention(q, k_new, v_new, past_k=None, past_v=None, mem_fre
 _DECODE_MAX_WHOLE_BLOCK_TOKENS = 16
 
 
-def _decode(q, k_new, v_new, past_k, past_v, block, cache_top_k, cos, sin, cache):
-    """llama_retrieval_attention for tokens that stay inside the unfinished block, as one launch (lmk_decode_attend); None
-    where that kernel does not apply.  Behind a cache of whole blocks it takes up to 16 tokens: more are cheaper as a chunk,
-    whose scores and local attention run on the tensor cores."""
+def _native(q, k_new, v_new, past_k, past_v, block, cache_top_k, cos, sin, cache, per_head):
+    """llama_retrieval_attention at the default positions as one native call; None where its kernels do not apply.
+
+    Tokens that stay inside the unfinished block are one launch (lmk_decode_attend); behind a cache of whole blocks that
+    kernel takes up to 16 tokens, more are cheaper as a chunk, whose scores and local attention run on the tensor cores."""
     C = past_k.shape[2] if cache is None else cache.length
     T = q.shape[2]
-    inc = C % block
-    if T + inc > block or C < block or (inc == 0 and T > _DECODE_MAX_WHOLE_BLOCK_TOKENS):
+    inc, n = C % block, C // block
+    top_k = min(cache_top_k, n)
+    if top_k < 1:
         return None
     if cache is None:
         kb, vb = past_k, past_v
@@ -424,7 +426,17 @@ def _decode(q, k_new, v_new, past_k, past_v, block, cache_top_k, cos, sin, cache
         kb, vb = cache.k, cache.v
         if C + T > kb.shape[2]:
             raise ValueError(f"cache capacity {kb.shape[2]} exceeded ({C} + {T})")
-    out = L.host().decode_attend(q, k_new, v_new, kb, vb, C, cache is not None, block, min(cache_top_k, C // block), cos, sin)
+    append = cache is not None
+    if per_head:
+        out = None if inc else L.host().per_head_attend(q, k_new, v_new, kb, vb, None, n, append, block, top_k, cos, sin)
+    elif T + inc <= block and (inc or T <= _DECODE_MAX_WHOLE_BLOCK_TOKENS):
+        out = L.host().decode_attend(q, k_new, v_new, kb, vb, C, append, block, top_k, cos, sin)
+    elif inc:
+        return None
+    else:
+        sym = q.is_cuda and _halves_equal(cos, sin, check=not torch.cuda.is_current_stream_capturing())
+        out = L.host().chunk_attend(q, k_new, v_new, kb, vb, C, append, block, top_k, cos, sin,
+                                    L.ROTARY_HALF_SYM if sym else L.ROTARY_HALF)
     if out is None:
         return None
     if cache is None:
@@ -484,6 +496,18 @@ class OffloadedLandmarkCache:
         from .fused import fused_landmark_attention
         assert self.tail_len == 0, "offloaded attention needs whole blocks in the cache (as the fused route does)"
         B, H, T, D = q.shape
+        if cos is not None and not return_debug and self.n_blocks and cache_top_k >= 1:
+            n_new, whole = T // self.block, T % self.block == 0
+            if whole and self.n_blocks + n_new > self.capacity:
+                raise ValueError(f"cache capacity of {self.capacity} blocks exceeded")
+            out = L.host().per_head_attend(q, k_new, v_new, self.k_host, self.v_host, self.lm_keys, self.n_blocks, whole,
+                                           self.block, min(cache_top_k, self.n_blocks), cos, sin)
+            if out is not None:
+                if whole:
+                    self.n_blocks += n_new
+                else:
+                    self.append(k_new, v_new)
+                return out
         blk, n, C = self.block, self.n_blocks, self.n_blocks * self.block
         dev = q.device
         if cos is None:
