@@ -221,6 +221,14 @@ int lmk_grouped_softmax_bwd(const void* x, const int64_t x_strides[3],
                             const float* grad_probs, float* grad_x,
                             int B, int H, int Lq, int Lk, int dtype, int guards, int max_groups, void* stream);
 
+/* lmk_grouped_softmax_bwd with grad_x in the type of x (rounded once from the fp32 result). */
+int lmk_grouped_softmax_bwd_typed(const void* x, const int64_t x_strides[3],
+                                  const uint8_t* is_mem, const int64_t is_mem_strides[4],
+                                  const uint8_t* last_section, const int64_t last_strides[4],
+                                  const uint8_t* hidden, const int64_t hidden_strides[4],
+                                  const float* grad_probs, void* grad_x,
+                                  int B, int H, int Lq, int Lk, int dtype, int guards, int max_groups, void* stream);
+
 /*
  * The same softmax for the lm_benchmark call site without any [Lq,Lk] mask: the mask block of
  * lm_benchmark/models/landmark.py:210-224 (causal rule "query i sees keys 0 .. i + Lk - Lq", last section, the masked
@@ -236,6 +244,10 @@ int lmk_grouped_softmax_causal_fwd(const void* x, const int64_t x_strides[3], co
                                    int max_groups, void* stream);
 int lmk_grouped_softmax_causal_bwd(const void* x, const int64_t x_strides[3], const uint8_t* is_mem_row,
                                    int64_t is_mem_stride, const float* grad_probs, float* grad_x, int B, int H, int Lq,
+                                   int Lk, int dtype, int max_groups, void* stream);
+/* the same with grad_x in the type of x */
+int lmk_grouped_softmax_causal_bwd_typed(const void* x, const int64_t x_strides[3], const uint8_t* is_mem_row,
+                                   int64_t is_mem_stride, const float* grad_probs, void* grad_x, int B, int H, int Lq,
                                    int Lk, int dtype, int max_groups, void* stream);
 
 /* Rotary conventions for the retrieval kernels. */

@@ -9,6 +9,8 @@
 //
 // Reference semantics: llama/llama_mem.py:168-243 (guards = 0) and lm_benchmark/models/landmark.py:37-119
 // (guards = 1: an all -inf group yields 0 instead of NaN, :48,:54).
+#include <algorithm>
+
 #include "common.cuh"
 #include "attn_params.h"
 
@@ -26,7 +28,7 @@ struct GsParams {
   float* probs;
   float* group_prob; int max_mem_cnt;
   const float* gprobs;
-  float* gx;
+  void* gx; int gx_as_x;     // gx holds fp32, or x's type where gx_as_x is set
   int B, H, Lq, Lk, guards, max_groups;
   // causal mode of the rows kernel: the three masks are derived from one flag per (batch row, key) and the rule
   // "query i sees keys 0 .. i + Lk - Lq" (mask block of lm_benchmark/models/landmark.py:210-224); hidden scores count
@@ -217,7 +219,6 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_kernel(GsParams
     }
     total = warp_sum(total);
     // pass 4: gradients
-    float* out = p.gx + row * p.Lk;
     rd.restart();
     for (int j0 = 0; j0 < p.Lk; j0 += 32) {
       Elem e = rd.load(j0);
@@ -235,7 +236,8 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_kernel(GsParams
         float inner = (guards && den < 0.5f) ? 0.f : expf(e.x - mx) / den;
         dx = inner * gw[e.c] * binv * (gj - gc[e.c]);
       }
-      out[j0 + lane] = dx;
+      if (p.gx_as_x) reinterpret_cast<T*>(p.gx)[row * p.Lk + j0 + lane] = from_f32<T>(dx);
+      else reinterpret_cast<float*>(p.gx)[row * p.Lk + j0 + lane] = dx;
     }
   }
 }
@@ -444,32 +446,31 @@ __device__ __forceinline__ void fold_chunk(float head, float tail, int nlm, int 
   __syncwarp();
 }
 
-template <typename T, bool kBackward, bool kCausal>
-__global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsParams p, int n_chunks) {
-  extern __shared__ __align__(16) float gs_smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int G = p.max_groups;
-  const size_t per_warp = (size_t)n_chunks * (kFastChunk + 64) + 4 * (size_t)G;
-  float* xbuf = gs_smem + warp * per_warp;
-  Meta* meta = reinterpret_cast<Meta*>(xbuf + (size_t)n_chunks * kFastChunk) + lane;   // [chunk][lane]
-  float* gmax = xbuf + (size_t)n_chunks * (kFastChunk + 64);
-  float* gsum = gmax + G;
-  float* gw = gsum + G;     // exp(landmark score - bucket max) of the landmark closing each group
-  float* gc = gw + G;       // backward: sum over the group of inner prob * grad
-  const int64_t row = (int64_t)blockIdx.x * kGsWarps + warp;
-  const int64_t rows = (int64_t)p.B * p.H * p.Lq;
-  if (row >= rows) return;
-  uint32_t bh;                                      // B * H fits 32 bits
-  int i;
-  if (rows <= 0xffffffffLL) {
+// (batch, head, query) of a row; B * H fits 32 bits
+__device__ __forceinline__ void row_index(const GsParams& p, int64_t row, int& b, int& h, int& i) {
+  uint32_t bh;
+  if ((int64_t)p.B * p.H * p.Lq <= 0xffffffffLL) {
     bh = (uint32_t)row / (uint32_t)p.Lq;
     i = (int)((uint32_t)row - bh * (uint32_t)p.Lq);
   } else {
     bh = (uint32_t)(row / p.Lq);
     i = (int)(row - (int64_t)bh * p.Lq);
   }
-  const int b = (int)(bh / (uint32_t)p.H);
-  const int h = (int)(bh - (uint32_t)b * (uint32_t)p.H);
+  b = (int)(bh / (uint32_t)p.H);
+  h = (int)(bh - (uint32_t)b * (uint32_t)p.H);
+}
+
+template <typename T, bool kBackward, bool kCausal>
+__device__ __forceinline__ void grouped_softmax_chunked_row(const GsParams& p, int n_chunks, int64_t row, float* xbuf) {
+  const int lane = threadIdx.x & 31;
+  const int G = p.max_groups;
+  Meta* meta = reinterpret_cast<Meta*>(xbuf + (size_t)n_chunks * kFastChunk) + lane;   // [chunk][lane]
+  float* gmax = xbuf + (size_t)n_chunks * (kFastChunk + 64);
+  float* gsum = gmax + G;
+  float* gw = gsum + G;     // exp(landmark score - bucket max) of the landmark closing each group
+  float* gc = gw + G;       // backward: sum over the group of inner prob * grad
+  int b, h, i;
+  row_index(p, row, b, h, i);
   const bool guards = p.guards != 0;
 
   const T* xrow = reinterpret_cast<const T*>(p.x) + b * p.xs[0] + h * p.xs[1] + i * p.xs[2];
@@ -715,9 +716,18 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsP
     }
   } else {
     const float* gr = p.gprobs + row * p.Lk;
-    float* out = p.gx + row * p.Lk;
     const bool gvec = (reinterpret_cast<uintptr_t>(gr) & 15) == 0;
-    const bool ovec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    auto store_grad = [&](int j, int n_in, const float (&x)[8]) {
+      if (p.gx_as_x && sizeof(T) == 2) {
+        T* o = reinterpret_cast<T*>(p.gx) + row * p.Lk + j;
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          if (v < n_in) o[v] = from_f32<T>(x[v]);
+      } else {
+        float* o = reinterpret_cast<float*>(p.gx) + row * p.Lk;
+        store8f(o + j, (reinterpret_cast<uintptr_t>(o) & 15) == 0, n_in, x);
+      }
+    };
     // pass 3: c_g = sum_j inner_j * grad_j per group, total = sum_j P_j * grad_j over the row
     float total = 0.f;
     // the gradients of the next live chunk are requested before the current one is worked on
@@ -782,7 +792,7 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsP
       if (mt.dead()) {
 #pragma unroll
         for (int v = 0; v < 8; ++v) x[v] = 0.f;
-        store8f(out + j, ovec, n_in, x);
+        store_grad(j, n_in, x);
         continue;
       }
       row_get(xbuf + k * kFastChunk, lane, x);
@@ -804,11 +814,428 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsP
         }
         x[v] = dx;
       }
-      store8f(out + j, ovec, n_in, x);
+      store_grad(j, n_in, x);
     }
   }
 }
 #undef LMK_KEY_FLAG
+
+template <typename T, bool kBackward, bool kCausal>
+__global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsParams p, int n_chunks) {
+  extern __shared__ __align__(16) float gs_smem[];
+  const int warp = threadIdx.x >> 5;
+  const int64_t row = (int64_t)blockIdx.x * kGsWarps + warp;
+  if (row >= (int64_t)p.B * p.H * p.Lq) return;
+  grouped_softmax_chunked_row<T, kBackward, kCausal>(
+      p, n_chunks, row, gs_smem + warp * ((size_t)n_chunks * (kFastChunk + 64) + 4 * (size_t)p.max_groups));
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Rows of up to kLaneMaxLk keys with a landmark at most every Lk / 32 keys or so: lane l owns the 4 n4 contiguous keys
+// from l * 4 n4 on (n4 = ceil(Lk / 128)), which stay in registers through all passes, and at most one landmark falls
+// into a lane.  A group is then the tail of one lane, whole lanes behind it and the head of the lane that holds its
+// landmark: one segmented scan over the lanes per pass reduces every group of the row, and two shuffles hand each lane
+// the results of the (at most two) groups its keys lie in.  Nothing per group is kept in memory and no pass looks
+// anything up per key.  A row in which two landmarks share a lane is done by the chunked form above.
+//
+// The masks are packed to one bit per key, read as words at any alignment.  The row passes through shared memory once
+// on its way in and once on its way out (16 bytes a lane, consecutive lanes consecutive addresses on the global side;
+// an odd lane stride in 16-byte units keeps the lane's own accesses free of bank conflicts).  The gradients are
+// requested as soon as the scores have been read, up to the last key that is not merely hidden, and arrive under the
+// two passes that rebuild the exponentials.
+//
+// Bound by the memory traffic of scores, gradients and results.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int kLaneMaxLk = 2048;
+
+template <typename T>
+struct LaneRow {
+  float* buf;
+  int n4, magic, pad, lane;
+  __device__ __forceinline__ LaneRow(float* b, int n4_, int lane_)
+      : buf(b), n4(n4_), magic((65536 + n4_ - 1) / n4_), pad(~n4_ & 1), lane(lane_) {}
+  // place of the row's c-th piece of four keys (c < 512: the product is exact)
+  __device__ __forceinline__ int slot(int c) const { return c + ((c * magic) >> 16) * pad; }
+  __device__ __forceinline__ int own(int q) const { return lane * (n4 + pad) + q; }
+
+  // starts copying keys [0, n) of a row of E, `fill` from there to the end of the pieces
+  template <typename E>
+  __device__ __forceinline__ void stage(const E* src, int n, float fill) {
+    E* s = reinterpret_cast<E*>(buf);
+    const bool vec = (reinterpret_cast<uintptr_t>(src) & (4 * sizeof(E) - 1)) == 0;
+    const int whole = n >> 2, nv = vec ? whole : 0;
+    for (int c = lane; c < 32 * n4; c += 32) {
+      E* d = s + slot(c) * 4;
+      if (c < nv) {
+        const uint32_t a = (uint32_t)__cvta_generic_to_shared(d);
+        if constexpr (sizeof(E) == 4) cp_async16(a, src + c * 4);
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(src + c * 4) : "memory");
+      } else if (c >= whole) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (c * 4 + v >= n) d[v] = from_f32<E>(fill);
+      }
+    }
+    for (int e = nv * 4 + lane; e < n; e += 32) {
+      E* d = s + slot(e >> 2) * 4 + (e & 3);
+      if constexpr (sizeof(E) == 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src + e) : "memory");
+      else
+        *d = src[e];
+    }
+  }
+  template <typename E>
+  __device__ __forceinline__ void get(int q, float* x) const {
+    if constexpr (sizeof(E) == 4) {
+      const float4 a = reinterpret_cast<const float4*>(buf)[own(q)];
+      x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    } else {
+      const uint2 w = reinterpret_cast<const uint2*>(buf)[own(q)];
+      const E* e = reinterpret_cast<const E*>(&w);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) x[v] = to_f32(e[v]);
+    }
+  }
+  __device__ __forceinline__ void put(int q, const float* x) {
+    reinterpret_cast<float4*>(buf)[own(q)] = make_float4(x[0], x[1], x[2], x[3]);
+  }
+  // the row from shared memory to `out`
+  template <typename E>
+  __device__ __forceinline__ void write(E* out, int n) const {
+    const int nv = (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(E) - 1)) == 0 ? n >> 2 : 0;
+    for (int c = lane; c < nv; c += 32) {
+      const float4 a = reinterpret_cast<const float4*>(buf)[slot(c)];
+      if constexpr (sizeof(E) == 4) {
+        *reinterpret_cast<float4*>(out + c * 4) = a;
+      } else {
+        E t[4] = {from_f32<E>(a.x), from_f32<E>(a.y), from_f32<E>(a.z), from_f32<E>(a.w)};
+        *reinterpret_cast<uint2*>(out + c * 4) = *reinterpret_cast<const uint2*>(t);
+      }
+    }
+    for (int e = nv * 4 + lane; e < n; e += 32) out[e] = from_f32<E>(buf[slot(e >> 2) * 4 + (e & 3)]);
+  }
+};
+
+// bit v of the result = bit 0 of mask byte j0 + v; words that hold no byte of the row are not read
+template <int K>
+struct Bits {
+  uint32_t w[(K + 31) / 32];
+  __device__ __forceinline__ bool at(int v) const { return (w[v >> 5] >> (v & 31)) & 1u; }
+  // the lowest n of K bits
+  static __device__ __forceinline__ Bits low(int n) {
+    Bits r;
+#pragma unroll
+    for (int i = 0; i < (K + 31) / 32; ++i) {
+      const int m = n - 32 * i;
+      r.w[i] = m >= 32 ? ~0u : m <= 0 ? 0u : (1u << m) - 1u;
+    }
+    return r;
+  }
+  template <typename F>
+  static __device__ __forceinline__ Bits zip(F f) {
+    Bits r;
+#pragma unroll
+    for (int i = 0; i < (K + 31) / 32; ++i) r.w[i] = f(i);
+    return r;
+  }
+  __device__ __forceinline__ int count() const {
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < (K + 31) / 32; ++i) n += __popc(w[i]);
+    return n;
+  }
+  __device__ __forceinline__ int first() const {           // K where none is set
+    int r = K;
+#pragma unroll
+    for (int i = (K + 31) / 32 - 1; i >= 0; --i)
+      if (w[i]) r = 32 * i + __ffs(w[i]) - 1;
+    return r;
+  }
+  __device__ __forceinline__ int top() const {              // highest set bit, -1 where none is set
+    int r = -1;
+#pragma unroll
+    for (int i = 0; i < (K + 31) / 32; ++i)
+      if (w[i]) r = 32 * i + 31 - __clz(w[i]);
+    return r;
+  }
+};
+
+__device__ __noinline__ uint32_t mask_quad_slow(const uint8_t* p, int64_t cs, int j, int n) {
+  uint32_t b = 0;
+  for (int v = 0; v < 4 && j + v < n; ++v) b |= (p[(int64_t)(j + v) * cs] & 1u) << v;
+  return b;
+}
+
+template <int K>
+__device__ __forceinline__ Bits<K> load_bits(const uint8_t* p, int64_t cs, int j0, int n4, int n) {
+  Bits<K> r = Bits<K>::low(0);
+  if (p == nullptr || j0 >= n) return r;
+  auto pack = [](uint32_t w) -> uint32_t { return ((w & 0x01010101u) * 0x01020408u) >> 24; };   // bits 0, 8, 16, 24 -> 0 .. 3
+  if (cs == 1) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p + j0), end = reinterpret_cast<uintptr_t>(p + n);
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0 && (n4 & 3) == 0) {        // 16 bytes at a time
+#pragma unroll
+      for (int q = 0; q < K / 4; q += 4) {
+        if (q >= n4) break;
+        if (j0 + 4 * q + 16 <= n) {
+          const uint4 w = *reinterpret_cast<const uint4*>(a + 4 * q);
+          r.w[q >> 3] |= (pack(w.x) | (pack(w.y) << 4) | (pack(w.z) << 8) | (pack(w.w) << 12)) << (4 * (q & 7));
+        } else {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (j0 + 4 * (q + u) < n)
+              r.w[q >> 3] |= pack(*reinterpret_cast<const uint32_t*>(a + 4 * (q + u))) << (4 * ((q + u) & 7));
+        }
+      }
+    } else {
+      const uint32_t sh = (uint32_t)(a & 3) * 8;
+      const uint32_t* base = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+      uint32_t w0 = base[0];
+#pragma unroll
+      for (int q = 0; q < K / 4; ++q) {
+        if (q >= n4) break;
+        const uint32_t w1 = reinterpret_cast<uintptr_t>(base + q + 1) < end ? base[q + 1] : 0u;
+        r.w[q >> 3] |= pack(__funnelshift_r(w0, w1, sh)) << (4 * (q & 7));
+        w0 = w1;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < K / 4; ++q) {
+      if (q >= n4) break;
+      r.w[q >> 3] |= mask_quad_slow(p, cs, j0 + 4 * q, n) << (4 * (q & 7));
+    }
+  }
+  const Bits<K> in = Bits<K>::low(n - j0);
+#pragma unroll
+  for (int i = 0; i < (K + 31) / 32; ++i) r.w[i] &= in.w[i];
+  return r;
+}
+
+// Which lanes a lane's groups reach to.  Group a holds the lane's keys up to its landmark (all of them where it has
+// none), group b the keys behind it; a group is closed by the lane of its landmark (none for the row's last group).
+struct LaneGroups {
+  int lane, dist, src_a, src_b;
+  bool own, has_a, has_b;
+  __device__ __forceinline__ LaneGroups(int lane_, unsigned owners) : lane(lane_) {
+    own = (owners >> lane) & 1u;
+    const unsigned below = owners & ((2u << lane) - 1u);                  // landmark lanes up to this one
+    dist = lane - (below ? 31 - __clz(below) : 0);
+    const unsigned from = owners & ~((1u << lane) - 1u), behind = owners & ~((2u << lane) - 1u);
+    has_a = from != 0;
+    has_b = behind != 0;
+    src_a = has_a ? __ffs(from) - 1 : 31;
+    src_b = has_b ? __ffs(behind) - 1 : 31;
+  }
+  // a: the lane's share of group a, b: of group b (read where it owns a landmark).  Returns both groups' totals;
+  // `closed`: the total of the group that this lane's landmark closes.
+  template <bool kMax>
+  __device__ __forceinline__ void reduce(float a, float b, float& ta, float& tb, float& closed) const {
+    float v = own ? b : a;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float u = __shfl_up_sync(0xffffffffu, v, o);
+      if (o <= dist) v = kMax ? fmaxf(v, u) : v + u;
+    }
+    float prev = __shfl_up_sync(0xffffffffu, v, 1);
+    if (lane == 0) prev = kMax ? -INFINITY : 0.f;
+    closed = kMax ? fmaxf(prev, a) : prev + a;
+    const float open = __shfl_sync(0xffffffffu, v, 31);
+    ta = __shfl_sync(0xffffffffu, closed, src_a);
+    tb = __shfl_sync(0xffffffffu, closed, src_b);
+    if (!has_a) ta = open;
+    if (!has_b) tb = open;
+  }
+};
+
+template <typename T, bool kBackward, bool kCausal>
+__device__ __noinline__ void grouped_softmax_crowded_row(const GsParams& p, int n_chunks, int64_t row, float* buf) {
+  grouped_softmax_chunked_row<T, kBackward, kCausal>(p, n_chunks, row, buf);
+}
+
+template <typename T, bool kBackward, bool kCausal, int K>
+__global__ void __launch_bounds__(kGsWarps * 32, K == 16 ? 8 : K == 32 ? 5 : 3)
+    grouped_softmax_lanes_kernel(const __grid_constant__ GsParams p, int n_chunks, int n4, int per_warp) {
+  extern __shared__ __align__(16) float gs_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t row = (int64_t)blockIdx.x * kGsWarps + warp;
+  if (row >= (int64_t)p.B * p.H * p.Lq) return;
+  int b, h, i;
+  row_index(p, row, b, h, i);
+  const bool guards = p.guards != 0;
+  const int G = p.max_groups, Lk = p.Lk, j0 = lane * 4 * n4;
+  LaneRow<T> lr(gs_smem + (size_t)warp * per_warp, n4, lane);
+  const T* xrow = reinterpret_cast<const T*>(p.x) + b * p.xs[0] + h * p.xs[1] + i * p.xs[2];
+
+  using Mask = Bits<K>;
+  Mask mem, last, bk, off;          // landmark, last section, bucket, hidden only
+  int n_seen = Lk;                  // keys whose scores are read
+  if (kCausal) {
+    const uint8_t* flags = p.row_flags + b * p.row_flags_stride;
+    const int pi = i + Lk - p.Lq;                       // the last key this query sees
+    n_seen = pi + ((flags[pi] & 1u) ? 0 : 1);           // a landmark at pi itself counts as hidden
+    lr.template stage<T>(xrow, n_seen, -INFINITY);
+    const Mask f = load_bits<K>(flags, 1, j0, n4, Lk);
+    const Mask vis = Mask::low(pi + 1 - j0), front = Mask::low(pi - j0);
+    mem = Mask::zip([&](int w) { return f.w[w] & front.w[w]; });
+    const unsigned with = __ballot_sync(0xffffffffu, mem.count() != 0);
+    int p_last = __shfl_sync(0xffffffffu, j0 + mem.top(), with ? 31 - __clz(with) : 0);
+    if (!with) p_last = -1;
+    const Mask closed = Mask::low(p_last + 1 - j0);
+    last = Mask::zip([&](int w) { return vis.w[w] & ~f.w[w] & ~closed.w[w]; });
+    off = Mask::zip([&](int w) { return ~(vis.w[w] & (~f.w[w] | mem.w[w])); });
+    bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | off.w[w]; });
+  } else {
+    lr.template stage<T>(xrow, Lk, -INFINITY);
+    mem = load_bits<K>(p.is_mem + b * p.ms[0] + h * p.ms[1] + i * p.ms[2], p.ms[3], j0, n4, Lk);
+    last = load_bits<K>(p.last + b * p.ls[0] + h * p.ls[1] + i * p.ls[2], p.ls[3], j0, n4, Lk);
+    const Mask hid = load_bits<K>(p.hidden ? p.hidden + b * p.hs[0] + h * p.hs[1] + i * p.hs[2] : nullptr, p.hs[3], j0, n4, Lk);
+    const Mask in = Mask::low(Lk - j0);
+    bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | hid.w[w] | ~in.w[w]; });
+    off = Mask::zip([&](int w) { return (hid.w[w] | ~in.w[w]) & ~mem.w[w] & ~last.w[w]; });
+  }
+  const int nlm = mem.count();
+  cp_async_wait_all();
+  if (__any_sync(0xffffffffu, nlm > 1)) {
+    __syncwarp();
+    grouped_softmax_crowded_row<T, kBackward, kCausal>(p, n_chunks, row, lr.buf);
+    return;
+  }
+  __syncwarp();
+  const unsigned owners = __ballot_sync(0xffffffffu, nlm != 0);
+  const LaneGroups lg(lane, owners);
+  const int ca = __popc(owners & ((1u << lane) - 1u)), cb = ca + 1, n_groups = __popc(owners);
+  const int t = mem.first();                            // keys behind it lie in group b
+  if (lane == 0 && n_groups >= G && p.status != nullptr) atomicCAS(p.status, 0, kErrSoftmaxGroups);
+
+  // pass 1: group and bucket maxima
+  float x[K];
+  float head = -INFINITY, run = -INFINITY, bmax = -INFINITY;
+#pragma unroll
+  for (int q = 0; q < K / 4; ++q) {
+    if (q >= n4) break;
+    lr.template get<T>(q, x + 4 * q);
+#pragma unroll
+    for (int v = 4 * q; v < 4 * q + 4; ++v) {
+      if (mem.at(v)) { head = run; run = -INFINITY; }
+      run = fmaxf(run, bk.at(v) ? -INFINITY : x[v]);
+      bmax = fmaxf(bmax, bk.at(v) ? x[v] : -INFINITY);
+    }
+  }
+  __syncwarp();                                         // the buffer has been read
+  if (kBackward) {                                      // gradients up to the last key that is not merely hidden
+    Mask live = Mask::zip([&](int w) { return ~off.w[w]; });
+    const Mask mine = Mask::low(4 * n4);
+    live = Mask::zip([&](int w) { return live.w[w] & mine.w[w]; });
+    const int top = live.top();
+    const int n_live = __reduce_max_sync(0xffffffffu, top < 0 ? 0 : j0 + top + 1);
+    lr.template stage<float>(p.gprobs + row * Lk, min(n_live, Lk), 0.f);
+  }
+  bmax = warp_max(bmax);
+  if (guards && isinf(bmax)) bmax = 0.f;
+  float ma, mb, unused;
+  lg.reduce<true>(lg.own ? head : run, run, ma, mb, unused);
+  // stabilisers; +inf beyond the last slot makes every exponential of such a group 0
+  ma = ca >= G ? INFINITY : (guards && isinf(ma)) ? 0.f : ma;
+  mb = cb >= G ? INFINITY : (guards && isinf(mb)) ? 0.f : mb;
+
+  // pass 2: exponentials, group and bucket sums
+  float bsum = 0.f, elm = 0.f;
+  head = 0.f;
+  run = 0.f;
+#pragma unroll
+  for (int q = 0; q < K / 4; ++q) {
+    if (q >= n4) break;
+#pragma unroll
+    for (int v = 4 * q; v < 4 * q + 4; ++v) {
+      const float ex = exp_diff(x[v], bk.at(v) ? bmax : v > t ? mb : ma);      // keys beyond the row's end hold -inf
+      x[v] = ex;
+      if (bk.at(v)) bsum += ex;
+      else run += ex;
+      if (mem.at(v)) { elm = ex; head = run; run = 0.f; }
+    }
+  }
+  bsum = warp_sum(bsum);
+  const float binv = (guards && bsum < 0.5f) ? 0.f : 1.f / bsum;
+  float da, db, wa, wb;
+  lg.reduce<false>(lg.own ? head : run, run, da, db, unused);
+  // scale of a non-bucket key: its landmark's weight over its group's sum (0 only for a group without keys)
+  auto inv_den = [&](int c, float den) -> float { return (c >= G || (guards && den < 0.5f) || den == 0.f) ? 0.f : 1.f / den; };
+  const float ia = inv_den(ca, da), ib = inv_den(cb, db);
+  wa = __shfl_sync(0xffffffffu, elm, lg.src_a);
+  wb = __shfl_sync(0xffffffffu, elm, lg.src_b);
+  wa = lg.has_a && ca < G ? wa * binv : 0.f;
+  wb = lg.has_b && cb < G ? wb * binv : 0.f;
+  const float sa = ia * wa, sb = ib * wb;
+
+  if (!kBackward) {
+    const float none = guards ? 0.f : binv * 0.f;       // bucket keys outside the last section (NaN if binv is not finite)
+    float last_total = 0.f;
+#pragma unroll
+    for (int q = 0; q < K / 4; ++q) {
+      if (q >= n4) break;
+#pragma unroll
+      for (int v = 4 * q; v < 4 * q + 4; ++v) {
+        x[v] *= last.at(v) ? binv : bk.at(v) ? none : v > t ? sb : sa;
+        if (last.at(v)) last_total += x[v];
+      }
+      lr.put(q, x + 4 * q);
+    }
+    if (p.group_prob != nullptr) {
+      last_total = warp_sum(last_total);
+      float* gp = p.group_prob + row * p.max_mem_cnt;
+      for (int g = n_groups + lane; g < p.max_mem_cnt - 1; g += 32) gp[g] = 0.f;
+      if (lg.own && ca < p.max_mem_cnt - 1) gp[ca] = wa;
+      if (lane == 0) gp[p.max_mem_cnt - 1] = last_total;
+    }
+    __syncwarp();
+    lr.template write<float>(p.probs + row * Lk, Lk);
+  } else {
+    cp_async_wait_all();
+    __syncwarp();
+    // pass 3: c_g = sum_j inner_j * grad_j per group, total = sum_j P_j * grad_j over the row
+    float lsum = 0.f;
+    head = 0.f;
+    run = 0.f;
+#pragma unroll
+    for (int q = 0; q < K / 4; ++q) {
+      if (q >= n4) break;
+      float g[4];
+      lr.template get<float>(q, g);
+#pragma unroll
+      for (int v = 4 * q; v < 4 * q + 4; ++v) {
+        const float xg = x[v] * g[v - 4 * q];
+        if (last.at(v)) lsum += xg;
+        if (!bk.at(v)) run += xg;
+        if (mem.at(v)) { head = run; run = 0.f; }
+      }
+    }
+    float ga, gb, closed;
+    lg.reduce<false>(lg.own ? head : run, run, ga, gb, closed);
+    ga *= ia;
+    gb *= ib;
+    const float total = warp_sum((lg.own ? closed * ia * wa : 0.f) + lsum * binv);
+    // pass 4: bucket key P_j * ((g_j if last section) - total), a landmark also receives its group's c_g;
+    // group member P_j * (g_j - c_g)
+#pragma unroll
+    for (int q = 0; q < K / 4; ++q) {
+      if (q >= n4) break;
+      float g[4];
+      lr.template get<float>(q, g);
+#pragma unroll
+      for (int v = 4 * q; v < 4 * q + 4; ++v) {
+        const float s = off.at(v) ? 0.f : bk.at(v) ? binv : v > t ? sb : sa;
+        const float sub = mem.at(v) ? total - ga : bk.at(v) ? total : v > t ? gb : ga;
+        const float a = (bk.at(v) && !last.at(v)) ? 0.f : g[v - 4 * q];
+        x[v] = x[v] * s * (a - sub);
+      }
+      lr.put(q, x + 4 * q);                             // the lane's own pieces, read just before
+    }
+    __syncwarp();
+    if (p.gx_as_x) lr.template write<T>(reinterpret_cast<T*>(p.gx) + row * Lk, Lk);
+    else lr.template write<float>(reinterpret_cast<float*>(p.gx) + row * Lk, Lk);
+  }
+}
 
 static size_t fast_smem_bytes(int Lk, int max_groups) {
   const size_t n_chunks = (size_t)(Lk + kFastChunk - 1) / kFastChunk;
@@ -829,25 +1256,39 @@ int launch(const GsParams& p, int dtype, cudaStream_t st) {
                 p.max_groups, kFastMaxLk);
   const int n_chunks = (p.Lk + kFastChunk - 1) / kFastChunk;
   size_t smem = fast ? fast_smem_bytes(p.Lk, p.max_groups) : sizeof(float) * 4 * (size_t)p.max_groups * kGsWarps;
+  const int n4 = (p.Lk + 127) / 128;
+  const bool lanes = fast && p.Lk <= kLaneMaxLk;
+  // shared memory of a row: the larger of the lanes form and of the chunked one that a crowded row takes
+  int per_warp = 0;
+  if (lanes) {
+    per_warp = (int)(smem / sizeof(float) / kGsWarps);
+    per_warp = (std::max(per_warp, 32 * (n4 | 1) * 4) + 3) & ~3;
+    smem = sizeof(float) * (size_t)per_warp * kGsWarps;
+  }
+#define LMK_GS_RUN(kernel, ...)                                                                              \
+  do {                                                                                                       \
+    LMK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
+    kernel<<<grid, kGsWarps * 32, smem, st>>>(__VA_ARGS__);                                                  \
+  } while (0)
+#define LMK_GS_LANES(T, causal)                                                                              \
+  do {                                                                                                       \
+    if (n4 <= 4) LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 16>), p, n_chunks, n4, per_warp);        \
+    else if (n4 <= 8) LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 32>), p, n_chunks, n4, per_warp);   \
+    else LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 64>), p, n_chunks, n4, per_warp);                \
+  } while (0)
 #define LMK_GS_LAUNCH(T)                                                                                     \
   do {                                                                                                       \
-    if (fast && p.causal) {                                                                                  \
-      LMK_CUDA(cudaFuncSetAttribute(grouped_softmax_rows_kernel<T, kBackward, true>,                         \
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                \
-      grouped_softmax_rows_kernel<T, kBackward, true><<<grid, kGsWarps * 32, smem, st>>>(p, n_chunks);       \
-    } else if (fast) {                                                                                       \
-      LMK_CUDA(cudaFuncSetAttribute(grouped_softmax_rows_kernel<T, kBackward, false>,                        \
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                \
-      grouped_softmax_rows_kernel<T, kBackward, false><<<grid, kGsWarps * 32, smem, st>>>(p, n_chunks);      \
-    } else {                                                                                                 \
-      LMK_CUDA(cudaFuncSetAttribute(grouped_softmax_kernel<T, kBackward>,                                    \
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                \
-      grouped_softmax_kernel<T, kBackward><<<grid, kGsWarps * 32, smem, st>>>(p);                            \
-    }                                                                                                        \
+    if (lanes && p.causal) LMK_GS_LANES(T, true);                                                            \
+    else if (lanes) LMK_GS_LANES(T, false);                                                                  \
+    else if (fast && p.causal) LMK_GS_RUN((grouped_softmax_rows_kernel<T, kBackward, true>), p, n_chunks);   \
+    else if (fast) LMK_GS_RUN((grouped_softmax_rows_kernel<T, kBackward, false>), p, n_chunks);              \
+    else LMK_GS_RUN((grouped_softmax_kernel<T, kBackward>), p);                                              \
   } while (0)
   if (dtype == LMK_F32) LMK_GS_LAUNCH(float);
   else if (dtype == LMK_F16) LMK_GS_LAUNCH(__half);
   else LMK_GS_LAUNCH(__nv_bfloat16);
+#undef LMK_GS_LANES
+#undef LMK_GS_RUN
 #undef LMK_GS_LAUNCH
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
@@ -894,20 +1335,37 @@ extern "C" int lmk_grouped_softmax_fwd(const void* x, const int64_t x_strides[3]
   return lmk::launch<false>(p, dtype, (cudaStream_t)stream);
 }
 
+static int run_bwd(const void* x, const int64_t* xs, const uint8_t* is_mem, const int64_t* ms, const uint8_t* last,
+                   const int64_t* ls, const uint8_t* hidden, const int64_t* hs, const float* grad_probs, void* grad_x,
+                   int typed, int B, int H, int Lq, int Lk, int dtype, int guards, int max_groups, void* stream) {
+  lmk::GsParams p{};
+  int rc = lmk::fill(p, x, xs, is_mem, ms, last, ls, hidden, hs, B, H, Lq, Lk, dtype, guards, max_groups);
+  if (rc != LMK_OK) return rc;
+  LMK_CHECK_ARG(grad_probs && grad_x, "grouped_softmax_bwd: null gradient pointer");
+  p.gprobs = grad_probs;
+  p.gx = grad_x;
+  p.gx_as_x = typed && dtype != LMK_F32;
+  return lmk::launch<true>(p, dtype, (cudaStream_t)stream);
+}
+
 extern "C" int lmk_grouped_softmax_bwd(const void* x, const int64_t x_strides[3], const uint8_t* is_mem,
                                        const int64_t is_mem_strides[4], const uint8_t* last_section,
                                        const int64_t last_strides[4], const uint8_t* hidden,
                                        const int64_t hidden_strides[4], const float* grad_probs, float* grad_x,
                                        int B, int H, int Lq, int Lk, int dtype, int guards, int max_groups,
                                        void* stream) {
-  lmk::GsParams p{};
-  int rc = lmk::fill(p, x, x_strides, is_mem, is_mem_strides, last_section, last_strides, hidden, hidden_strides,
-                     B, H, Lq, Lk, dtype, guards, max_groups);
-  if (rc != LMK_OK) return rc;
-  LMK_CHECK_ARG(grad_probs && grad_x, "grouped_softmax_bwd: null gradient pointer");
-  p.gprobs = grad_probs;
-  p.gx = grad_x;
-  return lmk::launch<true>(p, dtype, (cudaStream_t)stream);
+  return run_bwd(x, x_strides, is_mem, is_mem_strides, last_section, last_strides, hidden, hidden_strides, grad_probs,
+                 grad_x, 0, B, H, Lq, Lk, dtype, guards, max_groups, stream);
+}
+
+extern "C" int lmk_grouped_softmax_bwd_typed(const void* x, const int64_t x_strides[3], const uint8_t* is_mem,
+                                             const int64_t is_mem_strides[4], const uint8_t* last_section,
+                                             const int64_t last_strides[4], const uint8_t* hidden,
+                                             const int64_t hidden_strides[4], const float* grad_probs, void* grad_x,
+                                             int B, int H, int Lq, int Lk, int dtype, int guards, int max_groups,
+                                             void* stream) {
+  return run_bwd(x, x_strides, is_mem, is_mem_strides, last_section, last_strides, hidden, hidden_strides, grad_probs,
+                 grad_x, 1, B, H, Lq, Lk, dtype, guards, max_groups, stream);
 }
 
 // Mask block + grouped softmax of the lm_benchmark call site (lm_benchmark/models/landmark.py:210-232) from one flag
@@ -936,14 +1394,29 @@ extern "C" int lmk_grouped_softmax_causal_fwd(const void* x, const int64_t x_str
   return lmk::launch<false>(p, dtype, (cudaStream_t)stream);
 }
 
-extern "C" int lmk_grouped_softmax_causal_bwd(const void* x, const int64_t x_strides[3], const uint8_t* is_mem_row,
-                                              int64_t is_mem_stride, const float* grad_probs, float* grad_x, int B,
-                                              int H, int Lq, int Lk, int dtype, int max_groups, void* stream) {
+static int run_causal_bwd(const void* x, const int64_t* xs, const uint8_t* is_mem_row, int64_t is_mem_stride,
+                          const float* grad_probs, void* grad_x, int typed, int B, int H, int Lq, int Lk, int dtype,
+                          int max_groups, void* stream) {
   lmk::GsParams p{};
-  int rc = fill_causal(p, x, x_strides, is_mem_row, is_mem_stride, B, H, Lq, Lk, dtype, max_groups);
+  int rc = fill_causal(p, x, xs, is_mem_row, is_mem_stride, B, H, Lq, Lk, dtype, max_groups);
   if (rc != LMK_OK) return rc;
   LMK_CHECK_ARG(grad_probs && grad_x, "grouped_softmax_causal_bwd: null gradient pointer");
   p.gprobs = grad_probs;
   p.gx = grad_x;
+  p.gx_as_x = typed && dtype != LMK_F32;
   return lmk::launch<true>(p, dtype, (cudaStream_t)stream);
+}
+
+extern "C" int lmk_grouped_softmax_causal_bwd(const void* x, const int64_t x_strides[3], const uint8_t* is_mem_row,
+                                              int64_t is_mem_stride, const float* grad_probs, float* grad_x, int B,
+                                              int H, int Lq, int Lk, int dtype, int max_groups, void* stream) {
+  return run_causal_bwd(x, x_strides, is_mem_row, is_mem_stride, grad_probs, grad_x, 0, B, H, Lq, Lk, dtype, max_groups,
+                        stream);
+}
+
+extern "C" int lmk_grouped_softmax_causal_bwd_typed(const void* x, const int64_t x_strides[3], const uint8_t* is_mem_row,
+                                                    int64_t is_mem_stride, const float* grad_probs, void* grad_x, int B,
+                                                    int H, int Lq, int Lk, int dtype, int max_groups, void* stream) {
+  return run_causal_bwd(x, x_strides, is_mem_row, is_mem_stride, grad_probs, grad_x, 1, B, H, Lq, Lk, dtype, max_groups,
+                        stream);
 }

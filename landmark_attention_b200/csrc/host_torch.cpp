@@ -37,8 +37,8 @@ using torch::autograd::variable_list;
 // ------------------------------------------------------------------------------------------------ library functions
 #define LMK_FUNCS(X)                                                                                             \
   X(lmk_last_error) X(lmk_attn_fwd) X(lmk_attn_bwd_workspace) X(lmk_attn_bwd_strided) X(lmk_attn_mask_fwd)               \
-  X(lmk_attn_mask_bwd_workspace) X(lmk_attn_mask_bwd_strided) X(lmk_grouped_softmax_fwd) X(lmk_grouped_softmax_bwd)      \
-  X(lmk_grouped_softmax_causal_fwd) X(lmk_grouped_softmax_causal_bwd) X(lmk_rotary_apply) X(lmk_mask_is_regular)        \
+  X(lmk_attn_mask_bwd_workspace) X(lmk_attn_mask_bwd_strided) X(lmk_grouped_softmax_fwd) X(lmk_grouped_softmax_bwd_typed)      \
+  X(lmk_grouped_softmax_causal_fwd) X(lmk_grouped_softmax_causal_bwd_typed) X(lmk_rotary_apply) X(lmk_mask_is_regular)        \
   X(lmk_decode_supported) X(lmk_decode_attend) X(lmk_block_select) X(lmk_block_select_supported)                  \
   X(lmk_prefix_gather) X(lmk_prefix_gather_supported) X(lmk_prefix_pv) X(lmk_landmark_scores)                     \
   X(lmk_landmark_scores_workspace) X(lmk_topk_sorted) X(lmk_chunk_rotate) X(lmk_attn_fwd_lse)                     \
@@ -396,13 +396,13 @@ struct GroupedSoftmax : public torch::autograd::Function<GroupedSoftmax> {
     const Tensor& x = s[0];
     const auto B = x.size(0), H = x.size(1), Lq = x.size(2), Lk = x.size(3);
     c10::cuda::OptionalCUDAGuard guard(x.device());
-    Tensor gprobs = g[0].to(at::kFloat).contiguous(), gx = empty_f32({B, H, Lq, Lk}, x);
+    Tensor gprobs = g[0].to(at::kFloat).contiguous(), gx = at::empty({B, H, Lq, Lk}, x.options());
     Mask m(s[1], x.sizes()), l(s[2], x.sizes()), h(s.size() > 3 ? s[3] : Tensor(), x.sizes());
-    check(lib.lmk_grouped_softmax_bwd(x.data_ptr(), S3(x).v, m.ptr, m.strides(), l.ptr, l.strides(), h.ptr, h.strides(),
-                                      gprobs.data_ptr<float>(), gx.data_ptr<float>(), B, H, Lq, Lk, dtype_code(x),
+    check(lib.lmk_grouped_softmax_bwd_typed(x.data_ptr(), S3(x).v, m.ptr, m.strides(), l.ptr, l.strides(), h.ptr, h.strides(),
+                                      gprobs.data_ptr<float>(), gx.data_ptr(), B, H, Lq, Lk, dtype_code(x),
                                       ctx->saved_data["guards"].toBool(), ctx->saved_data["groups"].toInt(), stream_of(x)),
           "lmk_grouped_softmax_bwd");
-    return {gx.to(x.scalar_type()), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    return {gx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -439,12 +439,12 @@ struct GroupedSoftmaxCausal : public torch::autograd::Function<GroupedSoftmaxCau
     const Tensor &x = s[0], &flags = s[1];
     const auto B = x.size(0), H = x.size(1), Lq = x.size(2), Lk = x.size(3);
     c10::cuda::OptionalCUDAGuard guard(x.device());
-    Tensor gprobs = g[0].to(at::kFloat).contiguous(), gx = empty_f32({B, H, Lq, Lk}, x);
-    check(lib.lmk_grouped_softmax_causal_bwd(x.data_ptr(), S3(x).v, (const uint8_t*)flags.data_ptr(), flags.stride(0),
-                                             gprobs.data_ptr<float>(), gx.data_ptr<float>(), B, H, Lq, Lk, dtype_code(x),
+    Tensor gprobs = g[0].to(at::kFloat).contiguous(), gx = at::empty({B, H, Lq, Lk}, x.options());
+    check(lib.lmk_grouped_softmax_causal_bwd_typed(x.data_ptr(), S3(x).v, (const uint8_t*)flags.data_ptr(), flags.stride(0),
+                                             gprobs.data_ptr<float>(), gx.data_ptr(), B, H, Lq, Lk, dtype_code(x),
                                              ctx->saved_data["groups"].toInt(), stream_of(x)),
           "lmk_grouped_softmax_causal_bwd");
-    return {gx.to(x.scalar_type()), Tensor(), Tensor()};
+    return {gx, Tensor(), Tensor()};
   }
 };
 
