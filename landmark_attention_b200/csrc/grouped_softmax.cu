@@ -831,96 +831,102 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsP
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Rows of up to kLaneMaxLk keys with a landmark at most every Lk / 32 keys or so: lane l owns the 4 n4 contiguous keys
-// from l * 4 n4 on (n4 = ceil(Lk / 128)), which stay in registers through all passes, and at most one landmark falls
-// into a lane.  A group is then the tail of one lane, whole lanes behind it and the head of the lane that holds its
+// Rows of up to about 2048 keys with a landmark at most every 1/32 of the row or so: lane l owns the 4 n4 contiguous keys
+// from l * 4 n4 on (n4 = ceil(keys / 128)), in shared memory through all passes, and at most one landmark falls into
+// a lane.  A group is then the tail of one lane, whole lanes behind it and the head of the lane that holds its
 // landmark: one segmented scan over the lanes per pass reduces every group of the row, and two shuffles hand each lane
 // the results of the (at most two) groups its keys lie in.  Nothing per group is kept in memory and no pass looks
 // anything up per key.  A row in which two landmarks share a lane is done by the chunked form above.
 //
-// The masks are packed to one bit per key, read as words at any alignment.  The row passes through shared memory once
-// on its way in and once on its way out (16 bytes a lane, consecutive lanes consecutive addresses on the global side;
-// an odd lane stride in 16-byte units keeps the lane's own accesses free of bank conflicts).  The gradients are
-// requested as soon as the scores have been read, up to the last key that is not merely hidden, and arrive under the
-// two passes that rebuild the exponentials.
+// Bound by the instructions per row (two thirds of the issue slots at 40 % of the copy bandwidth), so what can be shared is:
+// a warp takes the same query of several heads in turn, and masks that are broadcast over the heads are read, packed to a
+// bit per key and split into groups once.  The gradients arrive under the two passes that rebuild the exponentials.  The
+// passes are loops over four keys: with the keys in registers and the loops unrolled the kernel took as long (104 + 129 us),
+// its code no longer fitted the instruction caches.  A guarded row is worked on only up to its
+// last score above -inf, which halves a causal matrix.
 //
-// Bound by the memory traffic of scores, gradients and results.
+// Keys are counted from the 4-element boundary at or in front of the row's place in the dense results (`lead` keys earlier),
+// so rows of any length are copied, read and written four elements at a time except for the row's two ends.
+// B16 H8 512 x 512 fp32, landmarks every 51 keys: forward 138 -> 98 us, backward 216 -> 130 us.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int kLaneMaxLk = 2048;
+constexpr int kLaneMaxPieces = 16;             // n4 of the longest row
 
-template <typename T>
+// A row in shared memory as pieces of four keys, 16 bytes each (scores of 16 bits wait in the upper half of theirs).
 struct LaneRow {
   float* buf;
-  int n4, magic, pad, lane;
-  __device__ __forceinline__ LaneRow(float* b, int n4_, int lane_)
-      : buf(b), n4(n4_), magic((65536 + n4_ - 1) / n4_), pad(~n4_ & 1), lane(lane_) {}
-  // place of the row's c-th piece of four keys (c < 512: the product is exact)
-  __device__ __forceinline__ int slot(int c) const { return c + ((c * magic) >> 16) * pad; }
-  __device__ __forceinline__ int own(int q) const { return lane * (n4 + pad) + q; }
+  int lane;
+  // place of the row's c-th piece: one place left out after eight spreads the strides of two to eight pieces, with which
+  // the lanes read their own keys, over the banks
+  static __device__ __forceinline__ int slot(int c) { return c + (c >> 3); }
 
-  // starts copying keys [0, n) of a row of E, `fill` from there to the end of the pieces
+  // starts copying the row's keys (counted with its lead) [lead, n) into n4 pieces a lane, `fill` elsewhere.
+  // src: key 0, i.e. `lead` elements in front of the row
   template <typename E>
-  __device__ __forceinline__ void stage(const E* src, int n, float fill) {
-    E* s = reinterpret_cast<E*>(buf);
+  __device__ __forceinline__ void stage(const E* src, int lead, int n, int n4, float fill) {
     const bool vec = (reinterpret_cast<uintptr_t>(src) & (4 * sizeof(E) - 1)) == 0;
-    const int whole = n >> 2, nv = vec ? whole : 0;
+#pragma unroll 1
     for (int c = lane; c < 32 * n4; c += 32) {
-      E* d = s + slot(c) * 4;
-      if (c < nv) {
+      float* d = buf + slot(c) * 4 + (sizeof(E) == 4 ? 0 : 2);
+      if (vec && 4 * c >= lead && 4 * c + 4 <= n) {
         const uint32_t a = (uint32_t)__cvta_generic_to_shared(d);
-        if constexpr (sizeof(E) == 4) cp_async16(a, src + c * 4);
-        else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(src + c * 4) : "memory");
-      } else if (c >= whole) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (c * 4 + v >= n) d[v] = from_f32<E>(fill);
+        if constexpr (sizeof(E) == 4) cp_async16(a, src + 4 * c);
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(src + 4 * c) : "memory");
+      } else {
+        E* e = reinterpret_cast<E*>(d);
+#pragma unroll 1
+        for (int v = 0; v < 4; ++v) e[v] = (4 * c + v >= lead && 4 * c + v < n) ? src[4 * c + v] : from_f32<E>(fill);
       }
     }
-    for (int e = nv * 4 + lane; e < n; e += 32) {
-      E* d = s + slot(e >> 2) * 4 + (e & 3);
-      if constexpr (sizeof(E) == 4)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src + e) : "memory");
-      else
-        *d = src[e];
-    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
   template <typename E>
-  __device__ __forceinline__ void get(int q, float* x) const {
+  __device__ __forceinline__ void get(int slot_c, float* x) const {
     if constexpr (sizeof(E) == 4) {
-      const float4 a = reinterpret_cast<const float4*>(buf)[own(q)];
+      const float4 a = reinterpret_cast<const float4*>(buf)[slot_c];
       x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
     } else {
-      const uint2 w = reinterpret_cast<const uint2*>(buf)[own(q)];
+      const uint2 w = reinterpret_cast<const uint2*>(buf)[2 * slot_c + 1];
       const E* e = reinterpret_cast<const E*>(&w);
 #pragma unroll
       for (int v = 0; v < 4; ++v) x[v] = to_f32(e[v]);
     }
   }
-  __device__ __forceinline__ void put(int q, const float* x) {
-    reinterpret_cast<float4*>(buf)[own(q)] = make_float4(x[0], x[1], x[2], x[3]);
+  __device__ __forceinline__ void put(int slot_c, const float* x) {
+    reinterpret_cast<float4*>(buf)[slot_c] = make_float4(x[0], x[1], x[2], x[3]);
   }
-  // the row from shared memory to `out`
+  // keys [lead, n) to `out` (key 0): n4 pieces a lane from shared memory, zeros behind them
   template <typename E>
-  __device__ __forceinline__ void write(E* out, int n) const {
-    const int nv = (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(E) - 1)) == 0 ? n >> 2 : 0;
-    for (int c = lane; c < nv; c += 32) {
-      const float4 a = reinterpret_cast<const float4*>(buf)[slot(c)];
-      if constexpr (sizeof(E) == 4) {
-        *reinterpret_cast<float4*>(out + c * 4) = a;
+  __device__ __forceinline__ void write(E* out, int lead, int n, int n4) const {
+    const bool vec = (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(E) - 1)) == 0;
+#pragma unroll 1
+    for (int c = lane; 4 * c < n; c += 32) {
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < 32 * n4) a = reinterpret_cast<const float4*>(buf)[slot(c)];
+      if (vec && 4 * c >= lead && 4 * c + 4 <= n) {
+        if constexpr (sizeof(E) == 4) {
+          *reinterpret_cast<float4*>(out + 4 * c) = a;
+        } else {
+          const E t[4] = {from_f32<E>(a.x), from_f32<E>(a.y), from_f32<E>(a.z), from_f32<E>(a.w)};
+          *reinterpret_cast<uint2*>(out + 4 * c) = *reinterpret_cast<const uint2*>(t);
+        }
       } else {
-        E t[4] = {from_f32<E>(a.x), from_f32<E>(a.y), from_f32<E>(a.z), from_f32<E>(a.w)};
-        *reinterpret_cast<uint2*>(out + c * 4) = *reinterpret_cast<const uint2*>(t);
+        const float t[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (4 * c + v >= lead && 4 * c + v < n) out[4 * c + v] = from_f32<E>(t[v]);
       }
     }
-    for (int e = nv * 4 + lane; e < n; e += 32) out[e] = from_f32<E>(buf[slot(e >> 2) * 4 + (e & 3)]);
   }
 };
 
-// bit v of the result = bit 0 of mask byte j0 + v; words that hold no byte of the row are not read
+// one bit for each of a lane's keys
 template <int K>
 struct Bits {
   uint32_t w[(K + 31) / 32];
-  __device__ __forceinline__ bool at(int v) const { return (w[v >> 5] >> (v & 31)) & 1u; }
+  // bits of the keys of piece q in the lowest four places (others behind them)
+  __device__ __forceinline__ uint32_t piece(int q) const {
+    return (K <= 32 || q < 8 ? w[0] : w[K <= 32 ? 0 : 1]) >> (4 * (q & 7));
+  }
   // the lowest n of K bits
   static __device__ __forceinline__ Bits low(int n) {
     Bits r;
@@ -962,53 +968,40 @@ struct Bits {
 
 __device__ __noinline__ uint32_t mask_quad_slow(const uint8_t* p, int64_t cs, int j, int n) {
   uint32_t b = 0;
-  for (int v = 0; v < 4 && j + v < n; ++v) b |= (p[(int64_t)(j + v) * cs] & 1u) << v;
+  for (int v = 0; v < 4; ++v)
+    if (j + v >= 0 && j + v < n) b |= (p[(int64_t)(j + v) * cs] & 1u) << v;
   return b;
 }
 
+// bit v of the result = bit 0 of mask byte j0 + v (0 outside the n keys of the row); only words that hold a byte of the
+// row are read
 template <int K>
 __device__ __forceinline__ Bits<K> load_bits(const uint8_t* p, int64_t cs, int j0, int n4, int n) {
   Bits<K> r = Bits<K>::low(0);
-  if (p == nullptr || j0 >= n) return r;
-  auto pack = [](uint32_t w) -> uint32_t { return ((w & 0x01010101u) * 0x01020408u) >> 24; };   // bits 0, 8, 16, 24 -> 0 .. 3
   if (cs == 1) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p + j0), end = reinterpret_cast<uintptr_t>(p + n);
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0 && (n4 & 3) == 0) {        // 16 bytes at a time
-#pragma unroll
-      for (int q = 0; q < K / 4; q += 4) {
-        if (q >= n4) break;
-        if (j0 + 4 * q + 16 <= n) {
-          const uint4 w = *reinterpret_cast<const uint4*>(a + 4 * q);
-          r.w[q >> 3] |= (pack(w.x) | (pack(w.y) << 4) | (pack(w.z) << 8) | (pack(w.w) << 12)) << (4 * (q & 7));
-        } else {
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (j0 + 4 * (q + u) < n)
-              r.w[q >> 3] |= pack(*reinterpret_cast<const uint32_t*>(a + 4 * (q + u))) << (4 * ((q + u) & 7));
-        }
-      }
-    } else {
-      const uint32_t sh = (uint32_t)(a & 3) * 8;
-      const uint32_t* base = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
-      uint32_t w0 = base[0];
-#pragma unroll
-      for (int q = 0; q < K / 4; ++q) {
-        if (q >= n4) break;
-        const uint32_t w1 = reinterpret_cast<uintptr_t>(base + q + 1) < end ? base[q + 1] : 0u;
-        r.w[q >> 3] |= pack(__funnelshift_r(w0, w1, sh)) << (4 * (q & 7));
-        w0 = w1;
-      }
-    }
-  } else {
+    const int mis = (int)(reinterpret_cast<uintptr_t>(p) & 3), at = j0 + mis;
+    const int first = at >> 2, sh = (at & 3) * 8, words = (mis + n + 3) >> 2;
+    const uint32_t* base = reinterpret_cast<const uint32_t*>(p - mis) + first;
+    uint32_t w0 = (unsigned)first < (unsigned)words ? base[0] : 0u;
 #pragma unroll
     for (int q = 0; q < K / 4; ++q) {
       if (q >= n4) break;
-      r.w[q >> 3] |= mask_quad_slow(p, cs, j0 + 4 * q, n) << (4 * (q & 7));
+      const uint32_t w1 = (unsigned)(first + q + 1) < (unsigned)words ? base[q + 1] : 0u;
+      // bits 0, 8, 16, 24 -> 0 .. 3
+      r.w[q >> 3] |= (((__funnelshift_r(w0, w1, sh) & 0x01010101u) * 0x01020408u) >> 24) << (4 * (q & 7));
+      w0 = w1;
+    }
+  } else {
+#pragma unroll 1
+    for (int q = 0; q < n4; ++q) {
+      const uint32_t quad = mask_quad_slow(p, cs, j0 + 4 * q, n) << (4 * (q & 7));
+      if (K <= 32 || q < 8) r.w[0] |= quad;
+      else r.w[K <= 32 ? 0 : 1] |= quad;
     }
   }
-  const Bits<K> in = Bits<K>::low(n - j0);
+  const Bits<K> in = Bits<K>::low(n - j0), before = Bits<K>::low(-j0);
 #pragma unroll
-  for (int i = 0; i < (K + 31) / 32; ++i) r.w[i] &= in.w[i];
+  for (int i = 0; i < (K + 31) / 32; ++i) r.w[i] &= in.w[i] & ~before.w[i];
   return r;
 }
 
@@ -1027,7 +1020,7 @@ struct LaneGroups {
     src_a = has_a ? __ffs(from) - 1 : 31;
     src_b = has_b ? __ffs(behind) - 1 : 31;
   }
-  // a: the lane's share of group a, b: of group b (read where it owns a landmark).  Returns both groups' totals;
+  // a: the lane's share of group a, b: of group b (counted where it owns a landmark).  Returns both groups' totals;
   // `closed`: the total of the group that this lane's landmark closes.
   template <bool kMax>
   __device__ __forceinline__ void reduce(float a, float b, float& ta, float& tb, float& closed) const {
@@ -1054,186 +1047,241 @@ __device__ __noinline__ void grouped_softmax_crowded_row(const GsParams& p, int 
 }
 
 template <typename T, bool kBackward, bool kCausal, int K>
-__global__ void __launch_bounds__(kGsWarps * 32, K == 16 ? 8 : K == 32 ? 5 : 3)
-    grouped_softmax_lanes_kernel(const __grid_constant__ GsParams p, int n_chunks, int n4, int per_warp) {
+__global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
+    grouped_softmax_lanes_kernel(const __grid_constant__ GsParams p, int n_chunks, int per_head_group, int per_warp) {
   extern __shared__ __align__(16) float gs_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row = (int64_t)blockIdx.x * kGsWarps + warp;
-  if (row >= (int64_t)p.B * p.H * p.Lq) return;
-  int b, h, i;
-  row_index(p, row, b, h, i);
+  const int head_groups = (p.H + per_head_group - 1) / per_head_group;
+  const unsigned task = blockIdx.x * kGsWarps + warp;             // (batch row, group of heads, query)
+  const int bg = (int)(task / (unsigned)p.Lq), i = (int)(task - (unsigned)bg * p.Lq);
+  if (bg >= p.B * head_groups) return;
+  const int b = bg / head_groups, h0 = (bg - b * head_groups) * per_head_group, h1 = min(h0 + per_head_group, p.H);
   const bool guards = p.guards != 0;
-  const int G = p.max_groups, Lk = p.Lk, j0 = lane * 4 * n4;
-  LaneRow<T> lr(gs_smem + (size_t)warp * per_warp, n4, lane);
-  const T* xrow = reinterpret_cast<const T*>(p.x) + b * p.xs[0] + h * p.xs[1] + i * p.xs[2];
+  const int G = p.max_groups, Lk = p.Lk;
+  // scores, then exponentials (and the forward's results) in the first half of the warp's memory, gradients (and the
+  // backward's results) in the second
+  LaneRow xr{gs_smem + (size_t)warp * per_warp, lane};
+  LaneRow gr{xr.buf + (kBackward ? per_warp >> 1 : 0), lane};
+  const bool shared_masks = kCausal || ((p.ms[1] | p.ls[1] | p.hs[1]) == 0);
+  const int pi = i + Lk - p.Lq;                         // causal: the last key this query sees
+  int seen = Lk;                                        // keys whose scores are read
+  if (kCausal) seen = pi + ((p.row_flags[b * p.row_flags_stride + pi] & 1u) ? 0 : 1);   // a landmark at pi itself is hidden
+
+  auto row_of = [&](int h) { return ((int64_t)b * p.H + h) * p.Lq + i; };
+  auto lead_of = [&](int h) { return (int)((row_of(h) * Lk) & 3); };
 
   using Mask = Bits<K>;
-  Mask mem, last, bk, off;          // landmark, last section, bucket, hidden only
-  int n_seen = Lk;                  // keys whose scores are read
-  if (kCausal) {
-    const uint8_t* flags = p.row_flags + b * p.row_flags_stride;
-    const int pi = i + Lk - p.Lq;                       // the last key this query sees
-    n_seen = pi + ((flags[pi] & 1u) ? 0 : 1);           // a landmark at pi itself counts as hidden
-    lr.template stage<T>(xrow, n_seen, -INFINITY);
-    const Mask f = load_bits<K>(flags, 1, j0, n4, Lk);
-    const Mask vis = Mask::low(pi + 1 - j0), front = Mask::low(pi - j0);
-    mem = Mask::zip([&](int w) { return f.w[w] & front.w[w]; });
-    const unsigned with = __ballot_sync(0xffffffffu, mem.count() != 0);
-    int p_last = __shfl_sync(0xffffffffu, j0 + mem.top(), with ? 31 - __clz(with) : 0);
-    if (!with) p_last = -1;
-    const Mask closed = Mask::low(p_last + 1 - j0);
-    last = Mask::zip([&](int w) { return vis.w[w] & ~f.w[w] & ~closed.w[w]; });
-    off = Mask::zip([&](int w) { return ~(vis.w[w] & (~f.w[w] | mem.w[w])); });
-    bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | off.w[w]; });
-  } else {
-    lr.template stage<T>(xrow, Lk, -INFINITY);
-    mem = load_bits<K>(p.is_mem + b * p.ms[0] + h * p.ms[1] + i * p.ms[2], p.ms[3], j0, n4, Lk);
-    last = load_bits<K>(p.last + b * p.ls[0] + h * p.ls[1] + i * p.ls[2], p.ls[3], j0, n4, Lk);
-    const Mask hid = load_bits<K>(p.hidden ? p.hidden + b * p.hs[0] + h * p.hs[1] + i * p.hs[2] : nullptr, p.hs[3], j0, n4, Lk);
-    const Mask in = Mask::low(Lk - j0);
-    bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | hid.w[w] | ~in.w[w]; });
-    off = Mask::zip([&](int w) { return (hid.w[w] | ~in.w[w]) & ~mem.w[w] & ~last.w[w]; });
-  }
-  const int nlm = mem.count();
-  cp_async_wait_all();
-  if (__any_sync(0xffffffffu, nlm > 1)) {
+  // what follows from the masks, kept while they, the lead and the number of pieces stay the same
+  Mask last, bk, act, ga, gb;       // last section, bucket, all but merely hidden keys, members of the lane's two groups
+  unsigned owners = 0;              // lanes with a landmark
+  int n4 = 0, lead = -1, c0 = 0, lm_slot = 0;     // c0: the lane's first piece
+  bool crowded = false, lm_last = false;                // lm_last: the lane's landmark is in the last section too
+  unsigned later = 0;               // heads whose row has two landmarks in one lane
+  for (int h = h0; h < h1; ++h) {
+    const int64_t row = row_of(h);
+    const int lead_h = lead_of(h);
+    int n = lead_h + seen;          // keys that the row is worked on for
+    int n4_h = max((n + 127) >> 7, 1);
+    xr.stage<T>(reinterpret_cast<const T*>(p.x) + b * p.xs[0] + h * p.xs[1] + i * p.xs[2] - lead_h, lead_h, n, n4_h, -INFINITY);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
-    grouped_softmax_crowded_row<T, kBackward, kCausal>(p, n_chunks, row, lr.buf);
-    return;
-  }
-  __syncwarp();
-  const unsigned owners = __ballot_sync(0xffffffffu, nlm != 0);
-  const LaneGroups lg(lane, owners);
-  const int ca = __popc(owners & ((1u << lane) - 1u)), cb = ca + 1, n_groups = __popc(owners);
-  const int t = mem.first();                            // keys behind it lie in group b
-  if (lane == 0 && n_groups >= G && p.status != nullptr) atomicCAS(p.status, 0, kErrSoftmaxGroups);
-
-  // pass 1: group and bucket maxima
-  float x[K];
-  float head = -INFINITY, run = -INFINITY, bmax = -INFINITY;
-#pragma unroll
-  for (int q = 0; q < K / 4; ++q) {
-    if (q >= n4) break;
-    lr.template get<T>(q, x + 4 * q);
-#pragma unroll
-    for (int v = 4 * q; v < 4 * q + 4; ++v) {
-      if (mem.at(v)) { head = run; run = -INFINITY; }
-      run = fmaxf(run, bk.at(v) ? -INFINITY : x[v]);
-      bmax = fmaxf(bmax, bk.at(v) ? x[v] : -INFINITY);
-    }
-  }
-  __syncwarp();                                         // the buffer has been read
-  if (kBackward) {                                      // gradients up to the last key that is not merely hidden
-    Mask live = Mask::zip([&](int w) { return ~off.w[w]; });
-    const Mask mine = Mask::low(4 * n4);
-    live = Mask::zip([&](int w) { return live.w[w] & mine.w[w]; });
-    const int top = live.top();
-    const int n_live = __reduce_max_sync(0xffffffffu, top < 0 ? 0 : j0 + top + 1);
-    lr.template stage<float>(p.gprobs + row * Lk, min(n_live, Lk), 0.f);
-  }
-  bmax = warp_max(bmax);
-  if (guards && isinf(bmax)) bmax = 0.f;
-  float ma, mb, unused;
-  lg.reduce<true>(lg.own ? head : run, run, ma, mb, unused);
-  // stabilisers; +inf beyond the last slot makes every exponential of such a group 0
-  ma = ca >= G ? INFINITY : (guards && isinf(ma)) ? 0.f : ma;
-  mb = cb >= G ? INFINITY : (guards && isinf(mb)) ? 0.f : mb;
-
-  // pass 2: exponentials, group and bucket sums
-  float bsum = 0.f, elm = 0.f;
-  head = 0.f;
-  run = 0.f;
-#pragma unroll
-  for (int q = 0; q < K / 4; ++q) {
-    if (q >= n4) break;
-#pragma unroll
-    for (int v = 4 * q; v < 4 * q + 4; ++v) {
-      const float ex = exp_diff(x[v], bk.at(v) ? bmax : v > t ? mb : ma);      // keys beyond the row's end hold -inf
-      x[v] = ex;
-      if (bk.at(v)) bsum += ex;
-      else run += ex;
-      if (mem.at(v)) { elm = ex; head = run; run = 0.f; }
-    }
-  }
-  bsum = warp_sum(bsum);
-  const float binv = (guards && bsum < 0.5f) ? 0.f : 1.f / bsum;
-  float da, db, wa, wb;
-  lg.reduce<false>(lg.own ? head : run, run, da, db, unused);
-  // scale of a non-bucket key: its landmark's weight over its group's sum (0 only for a group without keys)
-  auto inv_den = [&](int c, float den) -> float { return (c >= G || (guards && den < 0.5f) || den == 0.f) ? 0.f : 1.f / den; };
-  const float ia = inv_den(ca, da), ib = inv_den(cb, db);
-  wa = __shfl_sync(0xffffffffu, elm, lg.src_a);
-  wb = __shfl_sync(0xffffffffu, elm, lg.src_b);
-  wa = lg.has_a && ca < G ? wa * binv : 0.f;
-  wb = lg.has_b && cb < G ? wb * binv : 0.f;
-  const float sa = ia * wa, sb = ib * wb;
-
-  if (!kBackward) {
-    const float none = guards ? 0.f : binv * 0.f;       // bucket keys outside the last section (NaN if binv is not finite)
-    float last_total = 0.f;
-#pragma unroll
-    for (int q = 0; q < K / 4; ++q) {
-      if (q >= n4) break;
-#pragma unroll
-      for (int v = 4 * q; v < 4 * q + 4; ++v) {
-        x[v] *= last.at(v) ? binv : bk.at(v) ? none : v > t ? sb : sa;
-        if (last.at(v)) last_total += x[v];
+    if (!kCausal && guards) {
+      // scores of -inf at the row's end weigh nothing, whatever their flags say, and neither does a landmark among them
+      int top = 0;
+#pragma unroll 1
+      for (int c = lane; c < 32 * n4_h; c += 32) {
+        float e[4];
+        xr.get<T>(xr.slot(c), e);
+        if (e[0] != -INFINITY || e[1] != -INFINITY || e[2] != -INFINITY || e[3] != -INFINITY) top = c + 1;
       }
-      lr.put(q, x + 4 * q);
+      n = min(4 * __reduce_max_sync(0xffffffffu, top), n);
+      n4_h = max((n + 127) >> 7, 1);
     }
-    if (p.group_prob != nullptr) {
-      last_total = warp_sum(last_total);
-      float* gp = p.group_prob + row * p.max_mem_cnt;
-      for (int g = n_groups + lane; g < p.max_mem_cnt - 1; g += 32) gp[g] = 0.f;
-      if (lg.own && ca < p.max_mem_cnt - 1) gp[ca] = wa;
-      if (lane == 0) gp[p.max_mem_cnt - 1] = last_total;
+    if (!shared_masks || n4_h != n4 || lead_h != lead) {
+      n4 = n4_h;
+      lead = lead_h;
+      c0 = lane * n4;
+      const int j0 = 4 * c0;
+      Mask mem;
+      const Mask in = Mask::low(lead + Lk - j0), before = Mask::low(lead - j0);
+      if (kCausal) {
+        const Mask f = load_bits<K>(p.row_flags + b * p.row_flags_stride, 1, j0 - lead, n4, Lk);
+        const Mask upto = Mask::low(lead + pi + 1 - j0), front = Mask::low(lead + pi - j0);
+        const Mask vis = Mask::zip([&](int w) { return upto.w[w] & ~before.w[w]; });
+        mem = Mask::zip([&](int w) { return f.w[w] & front.w[w]; });
+        const unsigned with = __ballot_sync(0xffffffffu, mem.count() != 0);
+        int p_last = __shfl_sync(0xffffffffu, j0 + mem.top(), with ? 31 - __clz(with) : 0);
+        if (!with) p_last = -1;
+        const Mask closed = Mask::low(p_last + 1 - j0);
+        last = Mask::zip([&](int w) { return vis.w[w] & ~f.w[w] & ~closed.w[w]; });
+        act = Mask::zip([&](int w) { return vis.w[w] & (~f.w[w] | mem.w[w]); });
+        bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | ~act.w[w]; });
+      } else {
+        mem = load_bits<K>(p.is_mem + b * p.ms[0] + h * p.ms[1] + i * p.ms[2], p.ms[3], j0 - lead, n4, Lk);
+        last = load_bits<K>(p.last + b * p.ls[0] + h * p.ls[1] + i * p.ls[2], p.ls[3], j0 - lead, n4, Lk);
+        Mask hid = Mask::low(0);
+        if (p.hidden != nullptr)
+          hid = load_bits<K>(p.hidden + b * p.hs[0] + h * p.hs[1] + i * p.hs[2], p.hs[3], j0 - lead, n4, Lk);
+        bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | hid.w[w] | ~in.w[w] | before.w[w]; });
+        act = Mask::zip([&](int w) { return ~bk.w[w] | mem.w[w] | last.w[w]; });
+      }
+      const int nlm = mem.count();
+      crowded = __any_sync(0xffffffffu, nlm > 1);
+      owners = __ballot_sync(0xffffffffu, nlm != 0);
+      const int t = mem.first();                        // the lane's landmark: group a in front of it, group b behind
+      const Mask upto = Mask::low(t);
+      ga = Mask::zip([&](int w) { return ~bk.w[w] & upto.w[w]; });
+      gb = Mask::zip([&](int w) { return ~bk.w[w] & ~upto.w[w]; });
+      lm_last = (mem.w[0] & last.w[0]) != 0 || (K > 32 && (mem.w[K > 32 ? 1 : 0] & last.w[K > 32 ? 1 : 0]) != 0);
+      lm_slot = xr.slot(min(c0 + (t >> 2), 32 * n4 - 1)) * 4 + (t & 3);
     }
-    __syncwarp();
-    lr.template write<float>(p.probs + row * Lk, Lk);
-  } else {
-    cp_async_wait_all();
-    __syncwarp();
-    // pass 3: c_g = sum_j inner_j * grad_j per group, total = sum_j P_j * grad_j over the row
-    float lsum = 0.f;
-    head = 0.f;
-    run = 0.f;
+    if (crowded) {
+      later |= 1u << (h - h0);
+      continue;
+    }
+    if (kBackward) gr.stage<float>(p.gprobs + row * Lk - lead, lead, n, n4, 0.f);
+    asm volatile("" : "+r"(owners));                     // recomputed for every head rather than kept in registers
+    const LaneGroups lg(lane, owners);
+    const int ca = __popc(owners & ((1u << lane) - 1u)), cb = ca + 1, n_groups = __popc(owners);
+    if (lane == 0 && n_groups >= G && p.status != nullptr) atomicCAS(p.status, 0, kErrSoftmaxGroups);
+
+    // pass 1: group and bucket maxima
+    float va = -INFINITY, vb = -INFINITY, bmax = -INFINITY;
+#pragma unroll 1
+    for (int q = 0; q < n4; ++q) {
+      const uint32_t fa = ga.piece(q), fb = gb.piece(q), fk = bk.piece(q);
+      float x[4];
+      xr.get<T>(xr.slot(c0 + q), x);
 #pragma unroll
-    for (int q = 0; q < K / 4; ++q) {
-      if (q >= n4) break;
-      float g[4];
-      lr.template get<float>(q, g);
-#pragma unroll
-      for (int v = 4 * q; v < 4 * q + 4; ++v) {
-        const float xg = x[v] * g[v - 4 * q];
-        if (last.at(v)) lsum += xg;
-        if (!bk.at(v)) run += xg;
-        if (mem.at(v)) { head = run; run = 0.f; }
+      for (int v = 0; v < 4; ++v) {
+        if ((fa >> v) & 1u) va = fmaxf(va, x[v]);
+        if ((fb >> v) & 1u) vb = fmaxf(vb, x[v]);
+        if ((fk >> v) & 1u) bmax = fmaxf(bmax, x[v]);
       }
     }
-    float ga, gb, closed;
-    lg.reduce<false>(lg.own ? head : run, run, ga, gb, closed);
-    ga *= ia;
-    gb *= ib;
-    const float total = warp_sum((lg.own ? closed * ia * wa : 0.f) + lsum * binv);
-    // pass 4: bucket key P_j * ((g_j if last section) - total), a landmark also receives its group's c_g;
-    // group member P_j * (g_j - c_g)
+    // the landmark's score
+    float elm = sizeof(T) == 4 ? xr.buf[lm_slot] : to_f32(reinterpret_cast<const T*>(xr.buf)[2 * lm_slot + 4 - (lm_slot & 3)]);
+    bmax = warp_max(bmax);
+    if (guards && isinf(bmax)) bmax = 0.f;
+    float ma, mb, closed;
+    lg.reduce<true>(va, vb, ma, mb, closed);
+    // stabilisers; +inf beyond the last slot makes every exponential of such a group 0
+    ma = ca >= G ? INFINITY : (guards && isinf(ma)) ? 0.f : ma;
+    mb = cb >= G ? INFINITY : (guards && isinf(mb)) ? 0.f : mb;
+
+    // pass 2: exponentials, group and bucket sums
+    float bsum = 0.f;
+    va = vb = 0.f;
+#pragma unroll 1
+    for (int q = 0; q < n4; ++q) {
+      const uint32_t fa = ga.piece(q), fb = gb.piece(q), fk = bk.piece(q);
+      const int at = xr.slot(c0 + q);
+      float x[4];
+      xr.get<T>(at, x);
 #pragma unroll
-    for (int q = 0; q < K / 4; ++q) {
-      if (q >= n4) break;
-      float g[4];
-      lr.template get<float>(q, g);
-#pragma unroll
-      for (int v = 4 * q; v < 4 * q + 4; ++v) {
-        const float s = off.at(v) ? 0.f : bk.at(v) ? binv : v > t ? sb : sa;
-        const float sub = mem.at(v) ? total - ga : bk.at(v) ? total : v > t ? gb : ga;
-        const float a = (bk.at(v) && !last.at(v)) ? 0.f : g[v - 4 * q];
-        x[v] = x[v] * s * (a - sub);
+      for (int v = 0; v < 4; ++v) {
+        const bool ib = (fb >> v) & 1u, ik = (fk >> v) & 1u;
+        x[v] = exp_diff(x[v], ik ? bmax : ib ? mb : ma);               // keys outside the row hold -inf
+        if ((fa >> v) & 1u) va += x[v];
+        if (ib) vb += x[v];
+        if (ik) bsum += x[v];
       }
-      lr.put(q, x + 4 * q);                             // the lane's own pieces, read just before
+      xr.put(at, x);
     }
+    elm = exp_diff(elm, bmax);
+    bsum = warp_sum(bsum);
+    const float binv = (guards && bsum < 0.5f) ? 0.f : 1.f / bsum;
+    float da, db;
+    lg.reduce<false>(va, vb, da, db, closed);
+    // scale of a non-bucket key: its landmark's weight over its group's sum (0 only for a group without keys)
+    auto inv_den = [&](int c, float den) -> float {
+      return (c >= G || (guards && den < 0.5f) || den == 0.f) ? 0.f : 1.f / den;
+    };
+    const float ia = inv_den(ca, da), ib = inv_den(cb, db);
+    float wa = __shfl_sync(0xffffffffu, elm, lg.src_a), wb = __shfl_sync(0xffffffffu, elm, lg.src_b);
+    wa = lg.has_a && ca < G ? wa * binv : 0.f;
+    wb = lg.has_b && cb < G ? wb * binv : 0.f;
+    const float sa = ia * wa, sb = ib * wb;
+
+    if (!kBackward) {
+      const float none = guards ? 0.f : binv * 0.f;     // bucket keys outside the last section (NaN if binv is not finite)
+      float last_total = 0.f;
+#pragma unroll 1
+      for (int q = 0; q < n4; ++q) {
+        const uint32_t fa = ga.piece(q), fb = gb.piece(q), fl = last.piece(q);
+        const int at = xr.slot(c0 + q);
+        float x[4];
+        xr.get<float>(at, x);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const bool il = (fl >> v) & 1u;
+          x[v] *= il ? binv : (fb >> v) & 1u ? sb : (fa >> v) & 1u ? sa : none;
+          if (il) last_total += x[v];
+        }
+        xr.put(at, x);
+      }
+      if (p.group_prob != nullptr) {
+        last_total = warp_sum(last_total);
+        float* gp = p.group_prob + row * p.max_mem_cnt;
+        for (int g = n_groups + lane; g < p.max_mem_cnt - 1; g += 32) gp[g] = 0.f;
+        if (lg.own && ca < p.max_mem_cnt - 1) gp[ca] = wa;
+        if (lane == 0) gp[p.max_mem_cnt - 1] = last_total;
+      }
+      __syncwarp();
+      xr.write<float>(p.probs + row * Lk - lead, lead, lead + Lk, n4);
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      // pass 3: c_g = sum_j inner_j * grad_j per group, total = sum_j P_j * grad_j over the row
+      float lsum = 0.f;
+      va = vb = 0.f;
+#pragma unroll 1
+      for (int q = 0; q < n4; ++q) {
+        const uint32_t fa = ga.piece(q), fb = gb.piece(q), fl = last.piece(q);
+        const int at = xr.slot(c0 + q);
+        float x[4], g[4];
+        xr.get<float>(at, x);
+        gr.get<float>(at, g);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          if ((fa >> v) & 1u) va = fmaf(x[v], g[v], va);
+          if ((fb >> v) & 1u) vb = fmaf(x[v], g[v], vb);
+          if ((fl >> v) & 1u) lsum = fmaf(x[v], g[v], lsum);
+        }
+      }
+      float c_a, c_b;
+      lg.reduce<false>(va, vb, c_a, c_b, closed);
+      c_a *= ia;
+      c_b *= ib;
+      const float total = warp_sum((lg.own ? closed * ia * wa : 0.f) + lsum * binv);
+      // pass 4: last section P_j * (g_j - total), group member P_j * (g_j - c_g); a landmark P_j * (c_g - total), plus g_j
+      // if it is in the last section too
+      const float lm_g = lm_last ? gr.buf[lm_slot] : 0.f;
+#pragma unroll 1
+      for (int q = 0; q < n4; ++q) {
+        const uint32_t fb = gb.piece(q), fl = last.piece(q), fx = act.piece(q);
+        const int at = xr.slot(c0 + q);
+        float x[4], g[4];
+        xr.get<float>(at, x);
+        gr.get<float>(at, g);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const bool ib = (fb >> v) & 1u, il = (fl >> v) & 1u;
+          const float s = il ? binv : ib ? sb : sa, sub = il ? total : ib ? c_b : c_a;
+          x[v] = (fx >> v) & 1u ? x[v] * s * (g[v] - sub) : 0.f;
+        }
+        gr.put(at, x);                                  // the lane's own pieces, read just before
+      }
+      if (lg.own) gr.buf[lm_slot] = elm * binv * (lm_g + c_a - total);
+      __syncwarp();
+      if (p.gx_as_x) gr.write<T>(reinterpret_cast<T*>(p.gx) + row * Lk - lead, lead, lead + Lk, n4);
+      else gr.write<float>(reinterpret_cast<float*>(p.gx) + row * Lk - lead, lead, lead + Lk, n4);
+    }
+    __syncwarp();                                       // the results have been read
+  }
+  for (; later; later &= later - 1) {
+    grouped_softmax_crowded_row<T, kBackward, kCausal>(p, n_chunks, row_of(h0 + __ffs(later) - 1), xr.buf);
     __syncwarp();
-    if (p.gx_as_x) lr.template write<T>(reinterpret_cast<T*>(p.gx) + row * Lk, Lk);
-    else lr.template write<float>(reinterpret_cast<float*>(p.gx) + row * Lk, Lk);
   }
 }
 
@@ -1256,13 +1304,21 @@ int launch(const GsParams& p, int dtype, cudaStream_t st) {
                 p.max_groups, kFastMaxLk);
   const int n_chunks = (p.Lk + kFastChunk - 1) / kFastChunk;
   size_t smem = fast ? fast_smem_bytes(p.Lk, p.max_groups) : sizeof(float) * 4 * (size_t)p.max_groups * kGsWarps;
-  const int n4 = (p.Lk + 127) / 128;
-  const bool lanes = fast && p.Lk <= kLaneMaxLk;
-  // shared memory of a row: the larger of the lanes form and of the chunked one that a crowded row takes
-  int per_warp = 0;
+  // pieces a lane of the longest row, counted with its lead (rows of a multiple of four keys have none)
+  const int n4 = (p.Lk + (p.Lk % 4 ? 3 : 0) + 127) / 128;
+  const bool lanes = fast && n4 <= kLaneMaxPieces && rows < (1LL << 31);
+  // Heads a warp takes in turn: as many as leave every SM three rounds of
+  // warps (causal rows differ in length), eight at most.
+  int per_group = 1, per_warp = 0;
   if (lanes) {
-    per_warp = (int)(smem / sizeof(float) / kGsWarps);
-    per_warp = (std::max(per_warp, 32 * (n4 | 1) * 4) + 3) & ~3;
+    const int64_t resident = 148 * kGsWarps * 8;
+    per_group = (int)std::min<int64_t>(std::max<int64_t>(rows / (3 * resident), 1), std::min(p.H, 8));
+    const int groups = (p.H + per_group - 1) / per_group;
+    per_group = (p.H + groups - 1) / groups;
+    grid = (unsigned)(((int64_t)p.B * groups * p.Lq + kGsWarps - 1) / kGsWarps);
+    // shared memory of a warp: two rows, or what the chunked form of a crowded row takes
+    per_warp = ((int)(smem / sizeof(float) / kGsWarps) + 7) & ~7;
+    per_warp = std::max(per_warp, (kBackward ? 2 : 1) * 144 * n4);
     smem = sizeof(float) * (size_t)per_warp * kGsWarps;
   }
 #define LMK_GS_RUN(kernel, ...)                                                                              \
@@ -1272,9 +1328,8 @@ int launch(const GsParams& p, int dtype, cudaStream_t st) {
   } while (0)
 #define LMK_GS_LANES(T, causal)                                                                              \
   do {                                                                                                       \
-    if (n4 <= 4) LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 16>), p, n_chunks, n4, per_warp);        \
-    else if (n4 <= 8) LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 32>), p, n_chunks, n4, per_warp);   \
-    else LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 64>), p, n_chunks, n4, per_warp);                \
+    if (n4 <= 8) LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 32>), p, n_chunks, per_group, per_warp);   \
+    else LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 64>), p, n_chunks, per_group, per_warp);                \
   } while (0)
 #define LMK_GS_LAUNCH(T)                                                                                     \
   do {                                                                                                       \
