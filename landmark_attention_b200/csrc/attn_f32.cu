@@ -26,6 +26,7 @@ using ptx::upk2;
 constexpr int kBK = 64;      // keys of a block
 constexpr int kRT = 32;      // query rows of a tile
 constexpr int kPS = 68;      // row stride of the probability tiles
+constexpr int kSplit = 2;    // groups of threads that take the key blocks (dK / dV: the row tiles) of a CTA in turn
 
 __device__ __forceinline__ void cp16(float* dst, const float* src, bool valid) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -35,10 +36,17 @@ __device__ __forceinline__ void cp16(float* dst, const float* src, bool valid) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// rows row0 .. row0+kRows-1 of a [.., D] tensor into a padded tile; rows past `limit` and features past D become zeros
+// Groups of kThreads threads of a CTA run at their own pace: barrier number 1 + group.
+template <int kThreads>
+__device__ __forceinline__ void group_sync(int group) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kThreads) : "memory");
+}
+
+// rows row0 .. row0+kRows-1 of a [.., D] tensor into a padded tile by kThreads threads (this one is `tid`); rows past `limit`
+// and features past D become zeros
 template <int kD, int kRows, int kThreads>
-__device__ __forceinline__ void load_tile(float* tile, const float* base, int64_t row_stride, int row0, int limit, int D) {
-  for (int e = threadIdx.x; e < kRows * (kD / 4); e += kThreads) {
+__device__ __forceinline__ void load_tile(float* tile, const float* base, int64_t row_stride, int row0, int limit, int D, int tid) {
+  for (int e = tid; e < kRows * (kD / 4); e += kThreads) {
     const int r = e / (kD / 4), c = (e - r * (kD / 4)) * 4;
     const bool ok = row0 + r < limit && c < D;
     cp16(tile + r * (kD + 4) + c, ok ? base + (int64_t)(row0 + r) * row_stride + c : base, ok);
@@ -124,26 +132,26 @@ __device__ __forceinline__ int last_key(int n, int own, int pos) {
   return n < own ? kBK - 2 : (n == own ? min(pos & 63, kBK - 2) : -1);
 }
 
-template <int kD> constexpr size_t fwd_smem_f32 = sizeof(float) * ((kRT + 2 * kBK) * (kD + 4) + kRT * kPS);
+template <int kD> constexpr size_t fwd_smem_f32 = sizeof(float) * (kRT * (kD + 4) + kSplit * (2 * kBK * (kD + 4) + kRT * kPS));
 
 template <int kD>
-__global__ void __launch_bounds__(128) f32_fwd_kernel(AttnParams p) {
+__global__ void __launch_bounds__(128 * kSplit) f32_fwd_kernel(AttnParams p) {
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;
-  float* Ks = Qs + kRT * (kD + 4);
+  const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, tx = tid & 15, ty = tid >> 4;
+  float* Ks = Qs + kRT * (kD + 4) + group * (2 * kBK * (kD + 4) + kRT * kPS);
   float* Vs = Ks + kBK * (kD + 4);
   float* Ps = Vs + kBK * (kD + 4);
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int bh = blockIdx.x, b = bh / p.H, h = bh - b * p.H;
   const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRT, prefix = p.Lk - p.Lq;      // longest rows first
   const float* q = static_cast<const float*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const float* k = static_cast<const float*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const float* v = static_cast<const float*>(p.v) + b * p.vs[0] + h * p.vs[1];
   const int n_last = (prefix + min(q0 + kRT, p.Lq) - 1) / kBK;
-  load_tile<kD, kRT, 128>(Qs, q, p.qs[2], q0, p.Lq, p.D);
-  load_tile<kD, kBK, 128>(Ks, k, p.ks[2], 0, p.Lk, p.D);
+  load_tile<kD, kRT, 128 * kSplit>(Qs, q, p.qs[2], q0, p.Lq, p.D, threadIdx.x);
+  load_tile<kD, kBK, 128>(Ks, k, p.ks[2], group * kBK, p.Lk, p.D, tid);
   cp_commit();
-  load_tile<kD, kBK, 128>(Vs, v, p.vs[2], 0, p.Lk, p.D);
+  load_tile<kD, kBK, 128>(Vs, v, p.vs[2], group * kBK, p.Lk, p.D, tid);
   cp_commit();
   int pos[4];
   float m[4], l[4];
@@ -156,13 +164,15 @@ __global__ void __launch_bounds__(128) f32_fwd_kernel(AttnParams p) {
 #pragma unroll
     for (int c = 0; c < kD / 32; ++c) acc[i][c] = 0ull;
   }
-  for (int n = 0; n <= n_last; ++n) {
+  cp_wait<1>();
+  __syncthreads();                             // every group's part of the rows
+  for (int n = group; n <= n_last; n += kSplit) {
     cp_wait<1>();
-    __syncthreads();
+    group_sync<128>(group);
     float s[4][4];
     dots<kD, 4>(Qs, 8, Ks, ty, tx, s);
-    __syncthreads();
-    if (n < n_last) load_tile<kD, kBK, 128>(Ks, k, p.ks[2], (n + 1) * kBK, p.Lk, p.D);
+    group_sync<128>(group);
+    if (n + kSplit <= n_last) load_tile<kD, kBK, 128>(Ks, k, p.ks[2], (n + kSplit) * kBK, p.Lk, p.D, tid);
     cp_commit();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -197,11 +207,41 @@ __global__ void __launch_bounds__(128) f32_fwd_kernel(AttnParams p) {
       for (int j = 0; j < 4; ++j) Ps[(ty + 8 * i) * kPS + tx + 16 * j] = s[i][j] * w;
     }
     cp_wait<1>();
-    __syncthreads();
+    group_sync<128>(group);
     weighted_rows<kD>(Ps, Vs, ty, tx, acc);
-    __syncthreads();
-    if (n < n_last) load_tile<kD, kBK, 128>(Vs, v, p.vs[2], (n + 1) * kBK, p.Lk, p.D);
+    group_sync<128>(group);
+    if (n + kSplit <= n_last) load_tile<kD, kBK, 128>(Vs, v, p.vs[2], (n + kSplit) * kBK, p.Lk, p.D, tid);
     cp_commit();
+  }
+  // the first group adds the others' sums in their order; each leaves its own in its key tile
+  cp_wait<0>();
+  if (group > 0) {
+    group_sync<128>(group);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int c = 0; c < kD / 32; ++c) reinterpret_cast<uint64_t*>(Ks)[(i * (kD / 32) + c) * 128 + tid] = acc[i][c];
+      Vs[i * 128 + tid] = m[i];
+      Vs[(4 + i) * 128 + tid] = l[i];
+    }
+  }
+  __syncthreads();
+  if (group > 0) return;
+#pragma unroll
+  for (int g = 1; g < kSplit; ++g) {
+    const float* Kg = Ks + g * (2 * kBK * (kD + 4) + kRT * kPS);
+    const float* Vg = Kg + kBK * (kD + 4);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float mg = Vg[i * 128 + tid], top = fmaxf(m[i], mg);
+      const float fa = m[i] == -INFINITY ? 0.f : expf(m[i] - top), fb = mg == -INFINITY ? 0.f : expf(mg - top);
+      const uint64_t fa2 = pk2(fa, fa), fb2 = pk2(fb, fb);
+#pragma unroll
+      for (int c = 0; c < kD / 32; ++c)
+        acc[i][c] = fma2(reinterpret_cast<const uint64_t*>(Kg)[(i * (kD / 32) + c) * 128 + tid], fb2, ptx::mul2(acc[i][c], fa2));
+      l[i] = l[i] * fa + Vg[(4 + i) * 128 + tid] * fb;
+      m[i] = top;
+    }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -224,17 +264,17 @@ __global__ void __launch_bounds__(128) f32_fwd_kernel(AttnParams p) {
   }
 }
 
-template <int kD> constexpr size_t dq_smem_f32 = sizeof(float) * ((2 * kRT + 2 * kBK) * (kD + 4) + kRT * kPS);
+template <int kD> constexpr size_t dq_smem_f32 = sizeof(float) * (2 * kRT * (kD + 4) + kSplit * (2 * kBK * (kD + 4) + kRT * kPS));
 
 template <int kD>
-__global__ void __launch_bounds__(128) f32_bwd_dq_kernel(AttnParams p) {
+__global__ void __launch_bounds__(128 * kSplit) f32_bwd_dq_kernel(AttnParams p) {
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;
   float* Gs = Qs + kRT * (kD + 4);            // dO
-  float* Ks = Gs + kRT * (kD + 4);
+  const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, tx = tid & 15, ty = tid >> 4;
+  float* Ks = Gs + kRT * (kD + 4) + group * (2 * kBK * (kD + 4) + kRT * kPS);
   float* Vs = Ks + kBK * (kD + 4);
   float* Ps = Vs + kBK * (kD + 4);            // dS
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int bh = blockIdx.x, b = bh / p.H, h = bh - b * p.H;
   const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRT, prefix = p.Lk - p.Lq;
   const float* q = static_cast<const float*>(p.q) + b * p.qs[0] + h * p.qs[1];
@@ -242,10 +282,10 @@ __global__ void __launch_bounds__(128) f32_bwd_dq_kernel(AttnParams p) {
   const float* v = static_cast<const float*>(p.v) + b * p.vs[0] + h * p.vs[1];
   const float* g = static_cast<const float*>(p.dO) + b * p.dos[0] + h * p.dos[1];
   const int n_last = (prefix + min(q0 + kRT, p.Lq) - 1) / kBK;
-  load_tile<kD, kRT, 128>(Qs, q, p.qs[2], q0, p.Lq, p.D);
-  load_tile<kD, kRT, 128>(Gs, g, p.dos[2], q0, p.Lq, p.D);
-  load_tile<kD, kBK, 128>(Ks, k, p.ks[2], 0, p.Lk, p.D);
-  load_tile<kD, kBK, 128>(Vs, v, p.vs[2], 0, p.Lk, p.D);
+  load_tile<kD, kRT, 128 * kSplit>(Qs, q, p.qs[2], q0, p.Lq, p.D, threadIdx.x);
+  load_tile<kD, kRT, 128 * kSplit>(Gs, g, p.dos[2], q0, p.Lq, p.D, threadIdx.x);
+  load_tile<kD, kBK, 128>(Ks, k, p.ks[2], group * kBK, p.Lk, p.D, tid);
+  load_tile<kD, kBK, 128>(Vs, v, p.vs[2], group * kBK, p.Lk, p.D, tid);
   cp_commit();
   int pos[4];
   float M[4], Linv[4], delta[4];
@@ -270,18 +310,18 @@ __global__ void __launch_bounds__(128) f32_bwd_dq_kernel(AttnParams p) {
       }
     }
     delta[i] = sum16(d);
-    if (ok && tx == 0) p.delta[gr] = delta[i];
+    if (ok && tx == 0 && group == 0) p.delta[gr] = delta[i];
 #pragma unroll
     for (int c = 0; c < kD / 32; ++c) acc[i][c] = 0ull;
   }
-  for (int n = 0; n <= n_last; ++n) {
-    if (n > 0) {
-      __syncthreads();
-      load_tile<kD, kBK, 128>(Ks, k, p.ks[2], n * kBK, p.Lk, p.D);
-      load_tile<kD, kBK, 128>(Vs, v, p.vs[2], n * kBK, p.Lk, p.D);
+  for (int n = group; n <= n_last; n += kSplit) {
+    if (n != group) {
+      group_sync<128>(group);
+      load_tile<kD, kBK, 128>(Ks, k, p.ks[2], n * kBK, p.Lk, p.D, tid);
+      load_tile<kD, kBK, 128>(Vs, v, p.vs[2], n * kBK, p.Lk, p.D, tid);
       cp_commit();
       cp_wait<0>();
-      __syncthreads();
+      group_sync<128>(group);
     }
     float s[4][4], dp[4][4];
     dots<kD, 4>(Qs, 8, Ks, ty, tx, s);
@@ -321,6 +361,23 @@ __global__ void __launch_bounds__(128) f32_bwd_dq_kernel(AttnParams p) {
     __syncwarp();                              // a row's weights are written and read by the same half-warp
     weighted_rows<kD>(Ps, Ks, ty, tx, acc);
   }
+  if (group > 0) {                             // the first group adds the others' sums in their order
+    group_sync<128>(group);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < kD / 32; ++c) reinterpret_cast<uint64_t*>(Ks)[(i * (kD / 32) + c) * 128 + tid] = acc[i][c];
+  }
+  __syncthreads();
+  if (group > 0) return;
+#pragma unroll
+  for (int g = 1; g < kSplit; ++g)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < kD / 32; ++c)
+        acc[i][c] = ptx::add2(acc[i][c], reinterpret_cast<const uint64_t*>(Ks + g * (2 * kBK * (kD + 4) + kRT * kPS))
+                                             [(i * (kD / 32) + c) * 128 + tid]);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int row = q0 + ty + 8 * i;
@@ -337,30 +394,33 @@ __global__ void __launch_bounds__(128) f32_bwd_dq_kernel(AttnParams p) {
   }
 }
 
-// keys, values | rows of q and dO | P and dS tiles of 32 rows x 64 keys; the partial sums of the second CTA reuse the front
-template <int kD> constexpr size_t dkv_smem_f32 = sizeof(float) * ((2 * kBK + 2 * kRT) * (kD + 4) + 2 * kRT * kPS);
+// keys, values | per group: rows of q and dO, P and dS tiles of 32 rows x 64 keys; partial sums reuse the front
+template <int kD> constexpr size_t dkv_smem_f32 =
+    sizeof(float) * (2 * kBK * (kD + 4) + kSplit * (2 * kRT * (kD + 4) + 2 * kRT * kPS));
 
 template <int kD>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) f32_bwd_dkv_kernel(AttnParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256 * kSplit) f32_bwd_dkv_kernel(AttnParams p) {
   extern __shared__ __align__(16) float sm[];
   float* Ks = sm;
   float* Vs = Ks + kBK * (kD + 4);
-  float* Qs = Vs + kBK * (kD + 4);
+  const int group = threadIdx.x >> 8, tid = threadIdx.x & 255, tx = tid & 15, ty = tid >> 4;              // ty 0 .. 15
+  float* Qs = Vs + kBK * (kD + 4) + group * (2 * kRT * (kD + 4) + 2 * kRT * kPS);
   float* Gs = Qs + kRT * (kD + 4);
   float* Ps = Gs + kRT * (kD + 4);
   float* Ds = Ps + kRT * kPS;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;              // ty 0 .. 15
   const int n = blockIdx.y, bh = blockIdx.x >> 1, b = bh / p.H, h = bh - b * p.H;      // early blocks are seen by the most rows
   const int prefix = p.Lk - p.Lq, key0 = n * kBK;
   const float* q = static_cast<const float*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const float* k = static_cast<const float*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const float* v = static_cast<const float*>(p.v) + b * p.vs[0] + h * p.vs[1];
   const float* g = static_cast<const float*>(p.dO) + b * p.dos[0] + h * p.dos[1];
-  load_tile<kD, kBK, 256>(Ks, k, p.ks[2], key0, p.Lk, p.D);
-  load_tile<kD, kBK, 256>(Vs, v, p.vs[2], key0, p.Lk, p.D);
+  load_tile<kD, kBK, 256 * kSplit>(Ks, k, p.ks[2], key0, p.Lk, p.D, threadIdx.x);
+  load_tile<kD, kBK, 256 * kSplit>(Vs, v, p.vs[2], key0, p.Lk, p.D, threadIdx.x);
   cp_commit();
+  cp_wait<0>();
+  __syncthreads();
   // thread: keys 4 ty .. 4 ty + 3, features 4 tx + 64 c
   uint64_t dv[4][kD / 32], dk[4][kD / 32];
 #pragma unroll
@@ -368,11 +428,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) f32_bwd_dkv_ker
 #pragma unroll
     for (int c = 0; c < kD / 32; ++c) dv[i][c] = dk[i][c] = 0ull;
   const int t_first = max(0, key0 - prefix) / kRT, n_tiles = (p.Lq + kRT - 1) / kRT;
-  for (int t = t_first + rank; t < n_tiles; t += 2) {
+  for (int t = t_first + rank + 2 * group; t < n_tiles; t += 2 * kSplit) {
     const int q0 = t * kRT;
-    __syncthreads();
-    load_tile<kD, kRT, 256>(Qs, q, p.qs[2], q0, p.Lq, p.D);
-    load_tile<kD, kRT, 256>(Gs, g, p.dos[2], q0, p.Lq, p.D);
+    group_sync<256>(group);
+    load_tile<kD, kRT, 256>(Qs, q, p.qs[2], q0, p.Lq, p.D, tid);
+    load_tile<kD, kRT, 256>(Gs, g, p.dos[2], q0, p.Lq, p.D, tid);
     cp_commit();
     float M[2], Linv[2], delta[2];
 #pragma unroll
@@ -385,7 +445,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) f32_bwd_dkv_ker
       delta[i] = ok ? p.delta[gr] : 0.f;
     }
     cp_wait<0>();
-    __syncthreads();
+    group_sync<256>(group);
     float s[2][4], dp[2][4];
     dots<kD, 2>(Qs, 16, Ks, ty, tx, s);
     dots<kD, 2>(Gs, 16, Vs, ty, tx, dp);
@@ -424,7 +484,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) f32_bwd_dkv_ker
         Ds[r + tx + 16 * j] = ds;
       }
     }
-    __syncthreads();
+    group_sync<256>(group);
 #pragma unroll 2
     for (int r = 0; r < kRT; ++r) {
       const float4 pw = *reinterpret_cast<const float4*>(Ps + r * kPS + 4 * ty), dw = *reinterpret_cast<const float4*>(Ds + r * kPS + 4 * ty);
@@ -443,7 +503,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) f32_bwd_dkv_ker
       }
     }
   }
-  cp_wait<0>();
+  // the first group adds the others' sums in their order
+#pragma unroll
+  for (int g1 = 1; g1 < kSplit; ++g1) {
+    __syncthreads();
+    uint64_t* part = reinterpret_cast<uint64_t*>(sm);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < kD / 32; ++c) {
+        const int at = (i * (kD / 32) + c) * 512 + tid;
+        if (group == g1) {
+          part[at] = dv[i][c];
+          part[at + 256] = dk[i][c];
+        }
+      }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < kD / 32; ++c) {
+        const int at = (i * (kD / 32) + c) * 512 + tid;
+        if (group == 0) {
+          dv[i][c] = ptx::add2(dv[i][c], part[at]);
+          dk[i][c] = ptx::add2(dk[i][c], part[at + 256]);
+        }
+      }
+  }
   // the first CTA finishes dV, the second dK: each leaves the other's part in its own shared memory
   __syncthreads();
   float* mine = sm;                              // [64][kD]
@@ -451,6 +537,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) f32_bwd_dkv_ker
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int c = 0; c < kD / 64; ++c) {
+      if (group) break;
       F4 x;
       x.a = rank == 0 ? dk[i][2 * c] : dv[i][2 * c];
       x.b = rank == 0 ? dk[i][2 * c + 1] : dv[i][2 * c + 1];
@@ -463,6 +550,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) f32_bwd_dkv_ker
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int c = 0; c < kD / 64; ++c) {
+      if (group) break;
       const int key = 4 * ty + i, d = 64 * c + 4 * tx;
       const float4 y = *reinterpret_cast<const float4*>(theirs + key * kD + d);
       float4 x;
@@ -484,7 +572,7 @@ bool f32_operands_ok(const AttnParams& p) {
 template <int kD>
 int fwd_launch(const AttnParams& p, cudaStream_t st) {
   LMK_CUDA(cudaFuncSetAttribute(f32_fwd_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem_f32<kD>));
-  f32_fwd_kernel<kD><<<dim3(p.B * p.H, (p.Lq + kRT - 1) / kRT), 128, fwd_smem_f32<kD>, st>>>(p);
+  f32_fwd_kernel<kD><<<dim3(p.B * p.H, (p.Lq + kRT - 1) / kRT), 128 * kSplit, fwd_smem_f32<kD>, st>>>(p);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }
@@ -492,9 +580,9 @@ template <int kD>
 int bwd_launch(const AttnParams& p, cudaStream_t st) {
   LMK_CUDA(cudaFuncSetAttribute(f32_bwd_dq_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq_smem_f32<kD>));
   LMK_CUDA(cudaFuncSetAttribute(f32_bwd_dkv_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dkv_smem_f32<kD>));
-  f32_bwd_dq_kernel<kD><<<dim3(p.B * p.H, (p.Lq + kRT - 1) / kRT), 128, dq_smem_f32<kD>, st>>>(p);
+  f32_bwd_dq_kernel<kD><<<dim3(p.B * p.H, (p.Lq + kRT - 1) / kRT), 128 * kSplit, dq_smem_f32<kD>, st>>>(p);
   LMK_CUDA(cudaGetLastError());
-  f32_bwd_dkv_kernel<kD><<<dim3(2 * p.B * p.H, (p.Lk + kBK - 1) / kBK), 256, dkv_smem_f32<kD>, st>>>(p);
+  f32_bwd_dkv_kernel<kD><<<dim3(2 * p.B * p.H, (p.Lk + kBK - 1) / kBK), 256 * kSplit, dkv_smem_f32<kD>, st>>>(p);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }

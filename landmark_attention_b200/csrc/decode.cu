@@ -5,13 +5,17 @@
 //
 // What bounds it: nothing but latency.  One token against 1024 blocks of 32 reads 11 MB (1.7 us at the HBM peak) and
 // needs 11 MFLOP, so the design is about how much of that is in flight at once and how few dependent steps there are:
-//   * a cluster of CL CTAs works on one (token, head): CL * 8 warps score the landmarks (8 lanes a row, 16 rows in
-//     flight a warp), every warp keeps its own k best, the CL * 8 * k candidates go to every CTA of the cluster through
-//     distributed shared memory and each CTA picks the same final k;
+//   * a cluster of CL CTAs works on one (token, head): CL * 16 warps score the landmarks (8 lanes a row, 16 rows in
+//     flight a warp, requested together with the query and the tables), every warp keeps its own k best and the CL * 16 * k
+//     candidates go to the CTAs that need them through distributed shared memory;
+//   * a candidate is one word, the 16-bit score made sortable above the inverted block number, so a maximum over a warp
+//     is one reduction instruction and ties go to the lower block;
 //   * selected blocks, tail and new tokens are cut into items of 16 key rows, one warp each (values requested before the
 //     logits are computed); an item leaves (max, sum, unnormalised value sum) and the landmark's logit in the first CTA's
-//     shared memory, which merges the <= 64 items.
-// Measured at B1 H32 cache 32768 (blocks of 32, tail 17, top 4): see the kernel below.
+//     shared memory, which merges the <= 64 items.  Up to 16 items are all done by the first CTA's warps: the others
+//     finish after the selection and there is one cluster barrier less.
+// B1 H32, 32768 cached tokens (blocks of 32, tail 17, top 4): 60 launches, 190 us -> one of 15.4 us (pairs of floats and
+// indices reduced by shuffles, eight warps a CTA, items over the cluster) -> 10.6 us.
 #include <cooperative_groups.h>
 #include <type_traits>
 #include "common.cuh"
@@ -22,7 +26,7 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int kDecD = 128, kDecHalf = 64;
-constexpr int kDecWarps = 8;
+constexpr int kDecWarps = 16;
 constexpr int kDecMaxItems = 64;
 constexpr int kDecMaxK = 32;
 constexpr float kL2e = 1.4426950408889634f;
@@ -102,26 +106,22 @@ __device__ __forceinline__ float dot_pair(const float (&q)[16], const V4& lo, co
   }
   return a + b;
 }
-struct Best { float v; int i; };
-// a better than b: larger value, then lower index; index INT_MAX marks "none"
-__device__ __forceinline__ bool better(float v, int i, float bv, int bi) {
-  return i != 0x7fffffff && (bi == 0x7fffffff || v > bv || (v == bv && i < bi));
+// Score (already rounded to the 16-bit type) and block as one word: larger score, then lower block; 0 is below all of them.
+template <typename T>
+__device__ __forceinline__ uint32_t cand_key(float score, int n) {
+  const T t = from_f32<T>(score);
+  uint32_t bits = *reinterpret_cast<const uint16_t*>(&t);
+  if (bits == 0x8000u) bits = 0u;                                        // -0 counts as +0
+  return ((bits ^ (bits & 0x8000u ? 0xffffu : 0x8000u)) << 16) | (0xffffu - (uint32_t)n);
 }
-__device__ __forceinline__ Best warp_best(Best b) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, b.v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, b.i, o);
-    if (better(ov, oi, b.v, b.i)) b = {ov, oi};
-  }
-  return b;
-}
+__device__ __forceinline__ int cand_block(uint32_t key) { return 0xffff - (int)(key & 0xffffu); }
 
-// dynamic shared memory, in floats: rotated query | items (m, s, landmark logit, coefficient, values) | picks | candidates |
-// landmark scores of this CTA's slice
-__host__ __device__ constexpr int dec_slice(int n, int cl) { return ((n + cl - 1) / cl + 31) & ~31; }
+// dynamic shared memory, in words: items (m, s, landmark logit, coefficient, values) | picks | candidates | this CTA's keys
+__host__ __device__ constexpr int dec_slice(int n, int cl) {             // landmarks of a CTA: four a step and warp
+  return ((n + cl - 1) / cl + 4 * kDecWarps - 1) / (4 * kDecWarps) * (4 * kDecWarps);
+}
 __host__ __device__ constexpr size_t dec_smem(int n, int k, int cl) {
-  return sizeof(float) * (64 + kDecMaxItems * (4 + kDecD) + kDecMaxK + 2 * (size_t)cl * kDecWarps * k + dec_slice(n, cl));
+  return sizeof(float) * (kDecMaxItems * (4 + kDecD) + kDecMaxK + (size_t)cl * kDecWarps * k + dec_slice(n, cl));
 }
 
 template <typename T, int CL>
@@ -133,16 +133,14 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDecWarps * 32) dec
   const int t = blockIdx.x / CL, bh = blockIdx.y, b = bh / p.H, h = bh - b * p.H;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int K = p.top_k, N = p.n_blocks, blk = p.block;
-  uint32_t* qrot = reinterpret_cast<uint32_t*>(dec_smem_buf);     // 128 16-bit values
-  float* it_m = dec_smem_buf + 64;
+  float* it_m = dec_smem_buf;
   float* it_s = it_m + kDecMaxItems;
   float* it_lm = it_s + kDecMaxItems;
   float* it_c = it_lm + kDecMaxItems;
   float* it_o = it_c + kDecMaxItems;                               // [item][128]
   int* sel = reinterpret_cast<int*>(it_o + kDecMaxItems * kDecD);
-  float* cand_v = reinterpret_cast<float*>(sel + kDecMaxK);        // [CL * 8 * K]
-  int* cand_i = reinterpret_cast<int*>(cand_v + CL * kDecWarps * K);
-  float* sc = reinterpret_cast<float*>(cand_i + CL * kDecWarps * K);
+  uint32_t* cand = reinterpret_cast<uint32_t*>(sel + kDecMaxK);    // [CL * 16 * K]
+  uint32_t* keys = cand + CL * kDecWarps * K;
 
   const T* cos_t = static_cast<const T*>(p.cos_t);
   const T* sin_t = static_cast<const T*>(p.sin_t);
@@ -150,18 +148,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDecWarps * 32) dec
   auto clamp_pos = [&](int x) { return (int64_t)max(0, min(x, p.n_pos - 1)) * kDecD; };
   const int pos_base = full - (K + 1) * blk;
 
-  // ---- the query, rotated at its position; the first warp of the last CTA also stores the new key and value
-  if (tid < 8) {
-    const T* q = static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1] + t * p.qs[2] + tid * 8;
-    const int64_t po = clamp_pos(p.len + t) + tid * 8;
-    V4 lo = ldv(q), hi = ldv(q + kDecHalf);
-    rotate<T>(lo, hi, ldv(cos_t + po), ldv(cos_t + po + kDecHalf), ldv(sin_t + po), ldv(sin_t + po + kDecHalf));
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      qrot[tid * 4 + u] = lo.w[u];
-      qrot[32 + tid * 4 + u] = hi.w[u];
-    }
-  }
+  const int nch = (blk + 15) / 16, n_sel = K * nch;
+  const int n_loc_rows = inc + t + 1 - ((p.len + t) % blk == blk - 1 ? 1 : 0);     // a landmark does not see its own key
+  const int n_items = n_sel + (n_loc_rows + 15) / 16;
+  const bool solo = n_items <= kDecWarps;                          // all items in the first CTA
+
+  // ---- the query, rotated at its position; a warp of the last CTA also stores the new key and value
   if (p.append && rank == CL - 1 && warp == 1) {
     const int c = (lane & 15) * 8;
     const bool key = lane < 16;
@@ -174,99 +166,141 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDecWarps * 32) dec
   const T* kc = static_cast<const T*>(p.k_cache) + b * p.kcs[0] + h * p.kcs[1];
   const T* vc = static_cast<const T*>(p.v_cache) + b * p.vcs[0] + h * p.vcs[1];
   const int sub = lane & 7, grp = lane >> 3, d0 = sub * 8;
-  __syncthreads();
-  float q[16];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const float2 x = Px2<T>::f(qrot[sub * 4 + u]), y = Px2<T>::f(qrot[32 + sub * 4 + u]);
-    q[2 * u] = x.x;
-    q[2 * u + 1] = x.y;
-    q[8 + 2 * u] = y.x;
-    q[8 + 2 * u + 1] = y.y;
-  }
 
   // ---- landmark scores of this CTA's slice: 8 lanes a row; every block but the newest K shares slot 0 and its tables
   const int per = dec_slice(N, CL), n0 = rank * per, n1 = min(N, n0 + per);
+  const int steps = per / (4 * kDecWarps);
+  constexpr int kFly = 4;                                         // steps whose rows are requested together
+  V4 lo[kFly], hi[kFly];
+  auto request = [&](int st0) {
+#pragma unroll
+    for (int u = 0; u < kFly; ++u) {
+      const int n = n0 + 4 * kDecWarps * (st0 + u) + 4 * warp + grp;
+      if (st0 + u < steps && n < n1) {
+        const T* row = kc + ((int64_t)n * blk + blk - 1) * p.kcs[2] + d0;
+        lo[u] = ldv(row);
+        hi[u] = ldv(row + kDecHalf);
+      } else {
+        lo[u] = hi[u] = {{0u, 0u, 0u, 0u}};
+      }
+    }
+  };
+  request(0);
   const int64_t po0 = clamp_pos(pos_base + blk - 1) + d0;
   const V4 cl0 = ldv(cos_t + po0), ch0 = ldv(cos_t + po0 + kDecHalf), sl0 = ldv(sin_t + po0), sh0 = ldv(sin_t + po0 + kDecHalf);
-  float* my_sc = sc + warp * (per / kDecWarps);                   // per is a multiple of 32: 4 rows a step and warp
-  const int steps = per / 32;
-#pragma unroll 4
-  for (int st = 0; st < steps; ++st) {
-    const int n = n0 + 32 * st + 4 * warp + grp;
-    float s = -INFINITY;
-    if (n < n1) {
-      const T* row = kc + ((int64_t)n * blk + blk - 1) * p.kcs[2] + d0;
-      V4 lo = ldv(row), hi = ldv(row + kDecHalf);
-      if (n < N - K) {
-        rotate<T>(lo, hi, cl0, ch0, sl0, sh0);
+  float q[16];
+  {
+    const T* qp = static_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1] + t * p.qs[2] + d0;
+    const int64_t po = clamp_pos(p.len + t) + d0;
+    V4 ql = ldv(qp), qh = ldv(qp + kDecHalf);
+    rotate<T>(ql, qh, ldv(cos_t + po), ldv(cos_t + po + kDecHalf), ldv(sin_t + po), ldv(sin_t + po + kDecHalf));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float2 x = Px2<T>::f(ql.w[u]), y = Px2<T>::f(qh.w[u]);
+      q[2 * u] = x.x;
+      q[2 * u + 1] = x.y;
+      q[8 + 2 * u] = y.x;
+      q[8 + 2 * u + 1] = y.y;
+    }
+  }
+  uint32_t* my_keys = keys + warp * 4 * steps;
+  for (int st0 = 0; st0 < steps; st0 += kFly) {
+    if (st0) request(st0);
+#pragma unroll
+    for (int u = 0; u < kFly; ++u) {
+      if (st0 + u >= steps) break;
+      const int n = n0 + 4 * kDecWarps * (st0 + u) + 4 * warp + grp;
+      if (n < N - K || n >= n1) {
+        rotate<T>(lo[u], hi[u], cl0, ch0, sl0, sh0);
       } else {
         const int64_t po = clamp_pos(pos_base + (n - (N - K) + 1) * blk + blk - 1) + d0;
-        rotate<T>(lo, hi, ldv(cos_t + po), ldv(cos_t + po + kDecHalf), ldv(sin_t + po), ldv(sin_t + po + kDecHalf));
+        rotate<T>(lo[u], hi[u], ldv(cos_t + po), ldv(cos_t + po + kDecHalf), ldv(sin_t + po), ldv(sin_t + po + kDecHalf));
       }
-      s = dot_pair<T>(q, lo, hi);
+      float s = dot_pair<T>(q, lo[u], hi[u]);
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      s += __shfl_xor_sync(0xffffffffu, s, 4);
+      // the reference's matmul output and the scaling are each rounded to the input type; NaN ranks lowest
+      s = to_f32(from_f32<T>(s)) * p.scale;
+      if (sub == 0) my_keys[4 * (st0 + u) + grp] = n < n1 ? cand_key<T>(s == s ? s : -INFINITY, n) : 0u;
     }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
-    // the reference's matmul output and the scaling are each rounded to the input type; NaN ranks lowest
-    s = n < n1 ? to_f32(from_f32<T>(to_f32(from_f32<T>(s)) * p.scale)) : -INFINITY;
-    if (sub == 0) my_sc[4 * st + grp] = s == s ? s : -INFINITY;
   }
   __syncwarp();
 
-  // ---- every warp's K best of its own rows, to every CTA of the cluster
+  // ---- every warp's K best of its own rows, to every CTA of the cluster that works on items
+  uint32_t won = 0;                                               // lane `it` keeps the it-th
+  if (4 * steps <= 32) {
+    uint32_t mine = lane < 4 * steps ? my_keys[lane] : 0u;
+    for (int it = 0; it < K; ++it) {
+      const uint32_t best = __reduce_max_sync(0xffffffffu, mine);
+      if (mine == best) mine = 0u;
+      if (lane == it) won = best;
+    }
+  } else {
+    for (int it = 0; it < K; ++it) {
+      uint32_t mine = 0u;
+      for (int j = lane; j < 4 * steps; j += 32) mine = max(mine, my_keys[j]);
+      const uint32_t best = __reduce_max_sync(0xffffffffu, mine);
+      if (mine == best && best) {
+        const int r = cand_block(best) - n0;
+        my_keys[4 * (r / (4 * kDecWarps)) + (r & 3)] = 0u;
+      }
+      if (lane == it) won = best;
+      __syncwarp();
+    }
+  }
   cluster.barrier_wait();
-  for (int it = 0; it < K; ++it) {
-    Best best = {-INFINITY, 0x7fffffff};
-    for (int j = lane; j < 4 * steps; j += 32) {
-      const int n = n0 + 32 * (j >> 2) + 4 * warp + (j & 3);
-      const float v = my_sc[j];
-      if (n < n1 && v == v && better(v, n, best.v, best.i)) best = {v, n};       // NaN: taken
-    }
-    best = warp_best(best);
-    if (best.i != 0x7fffffff && lane == 0) {
-      const int r = best.i - n0;
-      my_sc[4 * (r >> 5) + (r & 3)] = __int_as_float(0x7fc00000);
-    }
-    if (lane < CL) {
-      const int slot = (rank * kDecWarps + warp) * K + it;
-      cluster.map_shared_rank(cand_v, lane)[slot] = best.v;
-      cluster.map_shared_rank(cand_i, lane)[slot] = best.i;
-    }
-    __syncwarp();
+  if (lane < K) {
+#pragma unroll
+    for (int c = 0; c < CL; ++c)
+      if (c == 0 || !solo) cluster.map_shared_rank(cand, c)[(rank * kDecWarps + warp) * K + lane] = won;
   }
   cluster.sync();
+  if (solo && rank != 0) return;                                  // nothing reads this CTA's memory any more
 
-  // ---- the final K (value, then lower index), in ascending order of age
-  if (warp == 0) {
+  // ---- the final K, in ascending order of age: by every warp for itself from registers, by the first one if there are many
+  const int n_cand = CL * kDecWarps * K;
+  const bool few = n_cand <= 256;
+  if (few || warp == 0) {
     int mine = 0x7fffffff;
-    for (int it = 0; it < K; ++it) {
-      Best best = {-INFINITY, 0x7fffffff};
-      for (int j = lane; j < CL * kDecWarps * K; j += 32)
-        if (better(cand_v[j], cand_i[j], best.v, best.i)) best = {cand_v[j], cand_i[j]};
-      best = warp_best(best);
-      for (int j = lane; j < CL * kDecWarps * K; j += 32)
-        if (cand_i[j] == best.i) cand_i[j] = 0x7fffffff;
-      if (lane == it) mine = best.i;
-      __syncwarp();
+    if (few) {
+      uint32_t v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = lane + 32 * u < n_cand ? cand[lane + 32 * u] : 0u;
+      for (int it = 0; it < K; ++it) {
+        const uint32_t top = max(max(max(v[0], v[1]), max(v[2], v[3])), max(max(v[4], v[5]), max(v[6], v[7])));
+        const uint32_t best = __reduce_max_sync(0xffffffffu, top);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (v[u] == best) v[u] = 0u;
+        if (lane == it) mine = cand_block(best);
+      }
+    } else {
+      for (int it = 0; it < K; ++it) {
+        uint32_t top = 0u;
+        for (int j = lane; j < n_cand; j += 32) top = max(top, cand[j]);
+        const uint32_t best = __reduce_max_sync(0xffffffffu, top);
+        if (top == best)
+          for (int j = lane; j < n_cand; j += 32)
+            if (cand[j] == best) cand[j] = 0u;
+        if (lane == it) mine = cand_block(best);
+        __syncwarp();
+      }
     }
     int order = 0;
     for (int u = 0; u < K; ++u) order += __shfl_sync(0xffffffffu, mine, u) < mine ? 1 : 0;
-    if (lane < K) sel[order] = mine;
+    if (lane < K) sel[order] = mine;                              // all warps write the same
   }
-  __syncthreads();
+  if (few) __syncwarp();
+  else __syncthreads();
 
   // ---- items of 16 key rows: chunk c of selected block i, then chunks of the tail and the new tokens
-  const int nch = (blk + 15) / 16, n_sel = K * nch;
-  const int n_loc_rows = inc + t + 1 - ((p.len + t) % blk == blk - 1 ? 1 : 0);     // a landmark does not see its own key
-  const int n_items = n_sel + (n_loc_rows + 15) / 16;
   const float scale_log2 = p.scale * kL2e;
   float* m_out = cluster.map_shared_rank(it_m, 0);
   float* s_out = cluster.map_shared_rank(it_s, 0);
   float* lm_out = cluster.map_shared_rank(it_lm, 0);
   float* o_out = cluster.map_shared_rank(it_o, 0);
-  for (int item = rank * kDecWarps + warp; item < n_items; item += CL * kDecWarps) {
+  for (int item = rank * kDecWarps + warp; item < n_items; item += CL * kDecWarps) {                // solo: rank 0, one each
     const bool selected = item < n_sel;
     const int i = selected ? item / nch : 0, c = selected ? item - i * nch : item - n_sel;
     const int nrows = min(16, (selected ? blk : n_loc_rows) - 16 * c);             // >= 1
@@ -349,8 +383,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDecWarps * 32) dec
       s_out[item] = sum;
     }
   }
-  cluster.sync();
-  if (rank != 0) return;
+  if (solo) {
+    __syncthreads();
+  } else {
+    cluster.sync();
+    if (rank != 0) return;
+  }
 
   // ---- merge: softmax inside each block over its chunks, then the outer softmax over landmarks and local keys
   if (warp == 0) {
@@ -388,7 +426,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDecWarps * 32) dec
 template <typename T, int CL>
 int dec_launch(const DecParams& p, int BH, cudaStream_t st) {
   const size_t smem = dec_smem(p.n_blocks, p.top_k, CL);
-  LMK_CUDA(cudaFuncSetAttribute(decode_attend_kernel<T, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024)
+    LMK_CUDA(cudaFuncSetAttribute(decode_attend_kernel<T, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   decode_attend_kernel<T, CL><<<dim3(CL * p.T, BH), kDecWarps * 32, smem, st>>>(p);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;

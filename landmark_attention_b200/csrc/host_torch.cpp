@@ -466,10 +466,18 @@ Tensor vector_rows(const Tensor& t) {
   return ok ? t : t.clone(at::MemoryFormat::Contiguous);
 }
 
-// One layer of token generation behind `len` cached tokens (lmk_decode_attend); undefined where the kernel does not take it.
+// Behind a cache of whole blocks the generation kernel takes up to this many tokens: more are cheaper as a chunk, whose scores
+// and local attention run on the tensor cores.
+constexpr int64_t kDecodeMaxWholeBlockTokens = 16;
+
+// One layer of token generation behind `len` cached tokens (lmk_decode_attend): tokens that stay inside the unfinished
+// block; undefined where the kernel does not take them.
 Tensor decode_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& kc, const Tensor& vc, int64_t len,
                      bool append, int64_t block, int64_t top_k, const Tensor& cos, const Tensor& sin) {
   const auto st = q_.scalar_type();
+  if (block < 2 || top_k < 1 || len < block) return Tensor();
+  const int64_t tail = len % block;
+  top_k = std::min(top_k, len / block);
   if (!q_.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || q_.dim() != 4 || kc.dim() != 4) return Tensor();
   const auto B = q_.size(0), H = q_.size(1), T = q_.size(2), D = q_.size(3);
   for (const Tensor* t : {&k_, &v_, &kc, &vc, &cos, &sin})
@@ -482,7 +490,7 @@ Tensor decode_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const
     return t.is_contiguous() && t.dim() == 2 && t.size(1) == D && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
   };
   if (!cache_ok(kc) || !cache_ok(vc) || k_.sizes() != q_.sizes() || v_.sizes() != q_.sizes() || !table_ok(cos) ||
-      !table_ok(sin) || B * H > 65535 || kc.size(2) < len + (append ? T : 0) || vc.size(2) < len + (append ? T : 0) ||
+      !table_ok(sin) || B * H > 65535 || T + tail > block || (!tail && T > kDecodeMaxWholeBlockTokens) || kc.size(2) < len + (append ? T : 0) || vc.size(2) < len + (append ? T : 0) ||
       !lib.lmk_decode_supported(D, block, top_k, len, T, dtype_code(q_)))
     return Tensor();
   c10::cuda::OptionalCUDAGuard guard(q_.device());
@@ -874,13 +882,26 @@ PyObject* py_grouped_softmax_causal(PyObject*, PyObject* const* a, Py_ssize_t n)
   END_HANDLE_TH_ERRORS
 }
 
-// decode_attend(q, k_new, v_new, k_cache, v_cache, len, append, block, top_k, cos, sin) -> out | None
+// (out, (keys, values)) with the cache's tokens up to `len` where the call appended to it, else out; None if out is undefined
+PyObject* wrap_appended(const Tensor& out, bool append, const Tensor& kc, const Tensor& vc, int64_t len) {
+  if (!out.defined() || !append) return wrap_opt(out);
+  PyObject *o = THPVariable_Wrap(out), *k = THPVariable_Wrap(kc.narrow(2, 0, len)), *v = THPVariable_Wrap(vc.narrow(2, 0, len));
+  PyObject* kv = PyTuple_Pack(2, k, v);
+  PyObject* r = PyTuple_Pack(2, o, kv);
+  for (PyObject* x : {o, k, v, kv}) Py_DECREF(x);
+  return r;
+}
+
+// decode_attend(q, k_new, v_new, k_cache, v_cache, len, append, block, top_k, cos, sin) -> see wrap_appended
 PyObject* py_decode_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 11);
-  return wrap_opt(decode_attend(tensor_arg(a[0], "q"), tensor_arg(a[1], "k_new"), tensor_arg(a[2], "v_new"),
-                                tensor_arg(a[3], "k_cache"), tensor_arg(a[4], "v_cache"), int_arg(a[5]), int_arg(a[6]) != 0,
-                                int_arg(a[7]), int_arg(a[8]), tensor_arg(a[9], "cos"), tensor_arg(a[10], "sin")));
+  const Tensor &q = tensor_arg(a[0], "q"), &kc = tensor_arg(a[3], "k_cache"), &vc = tensor_arg(a[4], "v_cache");
+  const int64_t len = int_arg(a[5]);
+  const bool append = int_arg(a[6]) != 0;
+  return wrap_appended(decode_attend(q, tensor_arg(a[1], "k_new"), tensor_arg(a[2], "v_new"), kc, vc, len, append, int_arg(a[7]),
+                                     int_arg(a[8]), tensor_arg(a[9], "cos"), tensor_arg(a[10], "sin")),
+                       append, kc, vc, len + q.size(2));
   END_HANDLE_TH_ERRORS
 }
 
@@ -905,13 +926,16 @@ PyObject* py_prefix_pv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// chunk_attend(q, k_new, v_new, k_cache, v_cache, len, append, block, top_k, cos, sin, rotary) -> out | None
+// chunk_attend(q, k_new, v_new, k_cache, v_cache, len, append, block, top_k, cos, sin, rotary) -> see wrap_appended
 PyObject* py_chunk_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 12);
-  return wrap_opt(chunk_attend(tensor_arg(a[0], "q"), tensor_arg(a[1], "k_new"), tensor_arg(a[2], "v_new"), tensor_arg(a[3], "k_cache"),
-                               tensor_arg(a[4], "v_cache"), int_arg(a[5]), int_arg(a[6]) != 0, int_arg(a[7]), int_arg(a[8]),
-                               tensor_arg(a[9], "cos"), tensor_arg(a[10], "sin"), int_arg(a[11])));
+  const Tensor &q = tensor_arg(a[0], "q"), &kc = tensor_arg(a[3], "k_cache"), &vc = tensor_arg(a[4], "v_cache");
+  const int64_t len = int_arg(a[5]);
+  const bool append = int_arg(a[6]) != 0;
+  return wrap_appended(chunk_attend(q, tensor_arg(a[1], "k_new"), tensor_arg(a[2], "v_new"), kc, vc, len, append, int_arg(a[7]),
+                                    int_arg(a[8]), tensor_arg(a[9], "cos"), tensor_arg(a[10], "sin"), int_arg(a[11])),
+                       append, kc, vc, len + q.size(2));
   END_HANDLE_TH_ERRORS
 }
 

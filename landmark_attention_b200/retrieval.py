@@ -285,6 +285,12 @@ def llama_retrieval_attention(q, k_new, v_new, past_k=None, past_v=None, mem_fre
     """
     if (fused is None and materialize is None and not return_debug and position_ids is None and chunk_is_mem is None
             and cos is not None and aggregate in (None, "max_over_tokens")):
+        if cache is not None and aggregate is None:           # generation first: its host path is as long as its kernel
+            out = L.host().decode_attend(q, k_new, v_new, cache.k, cache.v, cache.length, True, mem_freq + 1, cache_top_k,
+                                         cos, sin)
+            if out is not None:
+                cache.length += q.shape[2]
+                return out
         out = _native(q, k_new, v_new, past_k, past_v, mem_freq + 1, cache_top_k, cos, sin, cache, aggregate is not None)
         if out is not None:
             return out
@@ -406,14 +412,11 @@ def llama_retrieval_attention(q, k_new, v_new, past_k=None, past_v=None, mem_fre
     return out, new_cache()
 
 
-_DECODE_MAX_WHOLE_BLOCK_TOKENS = 16
-
-
 def _native(q, k_new, v_new, past_k, past_v, block, cache_top_k, cos, sin, cache, per_head):
     """llama_retrieval_attention at the default positions as one native call; None where its kernels do not apply.
 
-    Tokens that stay inside the unfinished block are one launch (lmk_decode_attend); behind a cache of whole blocks that
-    kernel takes up to 16 tokens, more are cheaper as a chunk, whose scores and local attention run on the tensor cores."""
+    Tokens that stay inside the unfinished block are one launch (lmk_decode_attend), whole chunks behind whole blocks the
+    chunk kernels."""
     C = past_k.shape[2] if cache is None else cache.length
     T = q.shape[2]
     inc, n = C % block, C // block
@@ -429,11 +432,11 @@ def _native(q, k_new, v_new, past_k, past_v, block, cache_top_k, cos, sin, cache
     append = cache is not None
     if per_head:
         out = None if inc else L.host().per_head_attend(q, k_new, v_new, kb, vb, None, n, append, block, top_k, cos, sin)
-    elif T + inc <= block and (inc or T <= _DECODE_MAX_WHOLE_BLOCK_TOKENS):
-        out = L.host().decode_attend(q, k_new, v_new, kb, vb, C, append, block, top_k, cos, sin)
-    elif inc:
-        return None
+        if out is not None and append:
+            out = out, (kb[:, :, :C + T], vb[:, :, :C + T])
     else:
+        out = None if append else L.host().decode_attend(q, k_new, v_new, kb, vb, C, False, block, top_k, cos, sin)
+    if out is None and not per_head and inc == 0:
         sym = q.is_cuda and _halves_equal(cos, sin, check=not torch.cuda.is_current_stream_capturing())
         out = L.host().chunk_attend(q, k_new, v_new, kb, vb, C, append, block, top_k, cos, sin,
                                     L.ROTARY_HALF_SYM if sym else L.ROTARY_HALF)
@@ -442,7 +445,7 @@ def _native(q, k_new, v_new, past_k, past_v, block, cache_top_k, cos, sin, cache
     if cache is None:
         return out, (torch.cat((past_k, k_new), dim=2), torch.cat((past_v, v_new), dim=2))
     cache.length = C + T
-    return out, cache.views()
+    return out
 
 
 class OffloadedLandmarkCache:
