@@ -661,6 +661,21 @@ Tensor landmark_scores(const Chunk& c, const Tensor& q_rot, const Tensor& keys, 
   return s;
 }
 
+// A second stream for the part of a call that nothing else in it waits for, with the events of the fork and the join (one set per
+// thread and device, reused: a wait refers to the event's state when it is enqueued).
+struct Fork {
+  c10::cuda::CUDAStream side;
+  cudaEvent_t begin, end;
+};
+Fork fork_of(int dev) {
+  constexpr int kMax = 64;
+  static thread_local cudaEvent_t events[kMax][2] = {};
+  TORCH_CHECK(dev >= 0 && dev < kMax, "device index out of range");
+  for (auto& e : events[dev])
+    if (e == nullptr) C10_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return {c10::cuda::getStreamFromPool(false, dev), events[dev][0], events[dev][1]};
+}
+
 // One selection per (head, token); `len` whole-block tokens in the caches; append: k, v stored behind them.
 Tensor chunk_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& kc, const Tensor& vc, int64_t len, bool append,
                     int64_t block, int64_t top_k, const Tensor& cos, const Tensor& sin, int64_t rotary) {
@@ -676,32 +691,25 @@ Tensor chunk_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
                              sin.data_ptr(), cos.size(0), len, qr.data_ptr(), kr.data_ptr(), nullptr, c.T * c.D,
                              append ? kc.data_ptr() : nullptr, append ? vc.data_ptr() : nullptr, append ? S3(kc).v : nullptr, len, c.B,
                              c.H, c.T, c.D, c.code, c.stream), "lmk_chunk_rotate");
+  // The chunk's local attention runs beside the scores and the selection: it has 96 CTAs at 32 heads of 258
+  // tokens (the whole call 158 -> 147 us), and neither needs the other's results.
+  Tensor o = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q), R = empty_f32({c.B * c.H, c.T}, c.q);
+  const Fork fork = fork_of(q_.get_device());
+  C10_CUDA_CHECK(cudaEventRecord(fork.begin, (cudaStream_t)c.stream));
   const Tensor s = landmark_scores(c, qr, kc, d, cos, sin, false);
   Tensor idx = at::empty({c.B, c.H, c.T, top_k}, c.q.options().requires_grad(false).dtype(at::kInt));
   check(lib.lmk_topk_sorted(s.data_ptr<float>(), idx.data_ptr<int>(), c.B * c.H * c.T, 1, n, 0, 1, 0, n, top_k, 0, c.stream), "lmk_topk_sorted");
-  Tensor o = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q), R = empty_f32({c.B * c.H, c.T}, c.q);
-  check(lib.lmk_attn_fwd_lse(qr.data_ptr(), kr.data_ptr(), c.v.data_ptr(), o.data_ptr(), R.data_ptr<float>(), c.B, c.H, c.T, c.T, c.D,
-                             S3(qr).v, S3(kr).v, S3(c.v).v, block, c.scale, c.code, c.stream), "lmk_attn_fwd_lse");
+  C10_CUDA_CHECK(cudaStreamWaitEvent(fork.side.stream(), fork.begin, 0));
+  const int local = lib.lmk_attn_fwd_lse(qr.data_ptr(), kr.data_ptr(), c.v.data_ptr(), o.data_ptr(), R.data_ptr<float>(), c.B, c.H, c.T,
+                                         c.T, c.D, S3(qr).v, S3(kr).v, S3(c.v).v, block, c.scale, c.code, fork.side.stream());
+  C10_CUDA_CHECK(cudaEventRecord(fork.end, fork.side.stream()));
+  C10_CUDA_CHECK(cudaStreamWaitEvent((cudaStream_t)c.stream, fork.end, 0));
+  check(local, "lmk_attn_fwd_lse");
   Tensor out = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q);
   check(lib.lmk_selected_attend(qr.data_ptr(), kc.data_ptr(), &d, vc.data_ptr(), &d, idx.data_ptr<int>(), cos.data_ptr(), sin.data_ptr(),
                                 cos.size(0), rotary, o.data_ptr(), R.data_ptr<float>(), c.T, out.data_ptr(), c.B, c.H, c.T, c.D, c.scale,
                                 c.code, c.stream), "lmk_selected_attend");
   return out;
-}
-
-// A second stream for the part of a call that nothing else in it waits for, with the events of the fork and the join (one set per
-// thread and device, reused: a wait refers to the event's state when it is enqueued).
-struct Fork {
-  c10::cuda::CUDAStream side;
-  cudaEvent_t begin, end;
-};
-Fork fork_of(int dev) {
-  constexpr int kMax = 64;
-  static thread_local cudaEvent_t events[kMax][2] = {};
-  TORCH_CHECK(dev >= 0 && dev < kMax, "device index out of range");
-  for (auto& e : events[dev])
-    if (e == nullptr) C10_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  return {c10::cuda::getStreamFromPool(false, dev), events[dev][0], events[dev][1]};
 }
 
 // One selection per head, the maximum over the chunk's tokens; the chunk then attends to [selected blocks | chunk].  The caches hold
