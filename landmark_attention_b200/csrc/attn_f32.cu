@@ -8,7 +8,8 @@
 //   dQ        the same with S and dP; writes delta.
 //   dK, dV    a cluster of two CTAs per key block: each takes every second tile of rows, partial sums are added through
 //             distributed shared memory in a fixed order (bit-reproducible, no atomics).
-// Measured at config 1 (before: one warp per 4 rows, scalar key loads): see the launch functions.
+// Measured at B2 H8 L512 D64 (before: one warp per 4 rows, scalar key loads): forward 214 -> 32, dQ 281 -> 43.5, dK/dV 362 -> 56 us;
+// one group of threads a CTA took 46, 57 and 71.
 // Math and statistics as in attn_general.cu, which keeps the other block sizes and unaligned operands.
 #include <cooperative_groups.h>
 #include "common.cuh"
@@ -35,6 +36,14 @@ __device__ __forceinline__ void cp16(float* dst, const float* src, bool valid) {
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Place in the order of falling work of the c-th of `total` CTAs on `slots` SMs, two of which fit an SM.  Up to twice the slots
+// all are resident from the start, so the second of an SM has to be light where its first is heavy: the rest comes in the order
+// of rising work.  (B2 H8 L512: at most 9 blocks an SM instead of 12; forward 36 -> 32, dQ 50 -> 43.5 us.)  Longer grids are dealt out as SMs
+// become free, heaviest first.
+__device__ __forceinline__ int work_rank(int c, int total, int slots) {
+  return c >= slots && total <= 2 * slots ? total - 1 - (c - slots) : c;
+}
 
 // Groups of kThreads threads of a CTA run at their own pace: barrier number 1 + group.
 template <int kThreads>
@@ -135,15 +144,15 @@ __device__ __forceinline__ int last_key(int n, int own, int pos) {
 template <int kD> constexpr size_t fwd_smem_f32 = sizeof(float) * (kRT * (kD + 4) + kSplit * (2 * kBK * (kD + 4) + kRT * kPS));
 
 template <int kD>
-__global__ void __launch_bounds__(128 * kSplit) f32_fwd_kernel(AttnParams p) {
+__global__ void __launch_bounds__(128 * kSplit, kD == 64 ? 2 : 1) f32_fwd_kernel(AttnParams p, int n_sm) {
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;
   const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, tx = tid & 15, ty = tid >> 4;
   float* Ks = Qs + kRT * (kD + 4) + group * (2 * kBK * (kD + 4) + kRT * kPS);
   float* Vs = Ks + kBK * (kD + 4);
   float* Ps = Vs + kBK * (kD + 4);
-  const int bh = blockIdx.x, b = bh / p.H, h = bh - b * p.H;
-  const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRT, prefix = p.Lk - p.Lq;      // longest rows first
+  const int BH = p.B * p.H, work = work_rank(blockIdx.x, gridDim.x, n_sm), bh = work % BH, b = bh / p.H, h = bh - b * p.H;
+  const int q0 = ((int)gridDim.x / BH - 1 - work / BH) * kRT, prefix = p.Lk - p.Lq;
   const float* q = static_cast<const float*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const float* k = static_cast<const float*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const float* v = static_cast<const float*>(p.v) + b * p.vs[0] + h * p.vs[1];
@@ -267,7 +276,7 @@ __global__ void __launch_bounds__(128 * kSplit) f32_fwd_kernel(AttnParams p) {
 template <int kD> constexpr size_t dq_smem_f32 = sizeof(float) * (2 * kRT * (kD + 4) + kSplit * (2 * kBK * (kD + 4) + kRT * kPS));
 
 template <int kD>
-__global__ void __launch_bounds__(128 * kSplit) f32_bwd_dq_kernel(AttnParams p) {
+__global__ void __launch_bounds__(128 * kSplit, kD == 64 ? 2 : 1) f32_bwd_dq_kernel(AttnParams p, int n_sm) {
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;
   float* Gs = Qs + kRT * (kD + 4);            // dO
@@ -275,8 +284,8 @@ __global__ void __launch_bounds__(128 * kSplit) f32_bwd_dq_kernel(AttnParams p) 
   float* Ks = Gs + kRT * (kD + 4) + group * (2 * kBK * (kD + 4) + kRT * kPS);
   float* Vs = Ks + kBK * (kD + 4);
   float* Ps = Vs + kBK * (kD + 4);            // dS
-  const int bh = blockIdx.x, b = bh / p.H, h = bh - b * p.H;
-  const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRT, prefix = p.Lk - p.Lq;
+  const int BH = p.B * p.H, work = work_rank(blockIdx.x, gridDim.x, n_sm), bh = work % BH, b = bh / p.H, h = bh - b * p.H;
+  const int q0 = ((int)gridDim.x / BH - 1 - work / BH) * kRT, prefix = p.Lk - p.Lq;
   const float* q = static_cast<const float*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const float* k = static_cast<const float*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const float* v = static_cast<const float*>(p.v) + b * p.vs[0] + h * p.vs[1];
@@ -410,7 +419,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256 * kSplit) f32_bw
   float* Ds = Ps + kRT * kPS;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
-  const int n = blockIdx.y, bh = blockIdx.x >> 1, b = bh / p.H, h = bh - b * p.H;      // early blocks are seen by the most rows
+  const int BH = p.B * p.H, work = blockIdx.x >> 1;                        // one CTA an SM (registers): heaviest first
+  const int n = work / BH, bh = work % BH, b = bh / p.H, h = bh - b * p.H;      // early blocks are seen by the most rows
   const int prefix = p.Lk - p.Lq, key0 = n * kBK;
   const float* q = static_cast<const float*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const float* k = static_cast<const float*>(p.k) + b * p.ks[0] + h * p.ks[1];
@@ -569,20 +579,33 @@ bool f32_operands_ok(const AttnParams& p) {
   return p.block == kBK && p.D <= 128 && p.D % 8 == 0 && vec_ok(p.q, p.qs) && vec_ok(p.k, p.ks) && vec_ok(p.v, p.vs);
 }
 
+int sm_count(int* n) {
+  int dev = 0;
+  LMK_CUDA(cudaGetDevice(&dev));
+  LMK_CUDA(cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev));
+  return LMK_OK;
+}
+
 template <int kD>
 int fwd_launch(const AttnParams& p, cudaStream_t st) {
+  int n_sm, rc = sm_count(&n_sm);
+  if (rc != LMK_OK) return rc;
   LMK_CUDA(cudaFuncSetAttribute(f32_fwd_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem_f32<kD>));
-  f32_fwd_kernel<kD><<<dim3(p.B * p.H, (p.Lq + kRT - 1) / kRT), 128 * kSplit, fwd_smem_f32<kD>, st>>>(p);
+  const int grid = p.B * p.H * ((p.Lq + kRT - 1) / kRT);
+  f32_fwd_kernel<kD><<<grid, 128 * kSplit, fwd_smem_f32<kD>, st>>>(p, n_sm);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }
 template <int kD>
 int bwd_launch(const AttnParams& p, cudaStream_t st) {
+  int n_sm, rc = sm_count(&n_sm);
+  if (rc != LMK_OK) return rc;
   LMK_CUDA(cudaFuncSetAttribute(f32_bwd_dq_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq_smem_f32<kD>));
   LMK_CUDA(cudaFuncSetAttribute(f32_bwd_dkv_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dkv_smem_f32<kD>));
-  f32_bwd_dq_kernel<kD><<<dim3(p.B * p.H, (p.Lq + kRT - 1) / kRT), 128 * kSplit, dq_smem_f32<kD>, st>>>(p);
+  const int grid = p.B * p.H * ((p.Lq + kRT - 1) / kRT);
+  f32_bwd_dq_kernel<kD><<<grid, 128 * kSplit, dq_smem_f32<kD>, st>>>(p, n_sm);
   LMK_CUDA(cudaGetLastError());
-  f32_bwd_dkv_kernel<kD><<<dim3(2 * p.B * p.H, (p.Lk + kBK - 1) / kBK), 256 * kSplit, dkv_smem_f32<kD>, st>>>(p);
+  f32_bwd_dkv_kernel<kD><<<2 * p.B * p.H * ((p.Lk + kBK - 1) / kBK), 256 * kSplit, dkv_smem_f32<kD>, st>>>(p);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }
