@@ -419,7 +419,14 @@ sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const uint32_t warp = threadIdx.x >> 5;
   bool held = false;
   uint32_t tmem = 0;
-  // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left.
+  // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left:
+  // all of a CTA's marks at once, then one by one where there is any.
+  if (only_marked) {
+    bool any = false;
+    for (int w = blockIdx.x + (int)threadIdx.x * gridDim.x; w < n_tiles * BH; w += (int)blockDim.x * gridDim.x)
+      any |= R_ptr[(int64_t)(w % BH) * Lq + (n_tiles - 1 - w / BH) * kQT] == -INFINITY;
+    if (!__syncthreads_or(any)) return;
+  }
   for (int w = blockIdx.x; w < n_tiles * BH; w += gridDim.x) {
     const int t = n_tiles - 1 - w / BH;      // heaviest tiles first
     const int bh = w % BH;
@@ -760,6 +767,11 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   bool held = false;
   uint32_t tmem = 0;
   // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left.
+  if (plan != nullptr) {
+    bool any = false;
+    for (int b = threadIdx.x; b < BH / H; b += blockDim.x) any |= plan[(int64_t)b * plan_stride + 1] != 0;
+    if (!__syncthreads_or(any)) return;
+  }
   for (int w = blockIdx.x; w < n_tiles * BH; w += gridDim.x) {
     const int t = n_tiles - 1 - w / BH;
     const int bh = w % BH;
@@ -1116,6 +1128,11 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   bool held = false;
   uint32_t tmem = 0;
   // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left.
+  if (plan != nullptr) {
+    bool any = false;
+    for (int b = threadIdx.x; b < BH / H; b += blockDim.x) any |= plan[(int64_t)b * plan_stride + 1] != 0;
+    if (!__syncthreads_or(any)) return;
+  }
   for (int w = blockIdx.x; w < n_tiles * BH; w += gridDim.x) {
     const int kt = w / BH;      // early key tiles are seen by the most query tiles
     const int bh = w % BH;
@@ -1185,12 +1202,12 @@ int attn_mask_sm100_fwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
   int* status = device_status_word();
   if (!status) return fail(LMK_ERR_CUDA, "cannot resolve the device status word");
   const float scale_log2 = p.scale * kLog2e;
-  // Groups of up to 64 keys run on the single-pass kernels (51-key groups at B16 H8 T512: 51 -> 21 us); what these leave, and
+  // Groups of up to 64 keys run on the single-pass kernels (51-key groups at B16 H8 T512: 51 -> 41 us); what these leave, and
   // lengths that cannot consist of such groups, on the two-pass kernels here.
   const int only_marked = attn_sm100_flags(p.Lk, G) && p.scale > 0.f;
   if (only_marked && (rc = attn_sm100_flags_fwd(p, is_mem, is_mem_stride, G, R, dtype, st)) != LMK_OK) return rc;
   const int tiles = p.B * p.H * (p.Lq / kQT);
-  const int grid = only_marked ? (tiles < 296 ? tiles : 296) : tiles;
+  const int grid = only_marked && tiles > 148 ? 148 : tiles;
   const size_t smem = mf_smem_bytes(G, p.Lk / kKT);
   if (dtype == LMK_BF16)
     sm100_mask_fwd_kernel<true><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.B * p.H, p.Lq,
