@@ -332,7 +332,8 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const uint32_t tmem = sm->tmem_base;
   auto tmem_s = [&](int w, int sb) { return tmem + (uint32_t)(w * 128 + sb * 64); };
   auto tmem_o = [&](int w) { return tmem + kTiles * 128u + (uint32_t)w * 128u; };
-  grid_dep_launch();      // a dependent kernel (the backward pass) may do its set-up while this grid drains
+  if constexpr (!kIrr) grid_dep_wait();      // only the set-up may overlap the kernel in front (see the launch)
+  grid_dep_launch();      // a dependent kernel (the backward pass, the next call) may do its set-up while this grid drains
 
   if (warp == kSw) {
     // ------------------------------------------------------------------ TMA producer
@@ -1741,12 +1742,28 @@ static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   const int n_tiles = (p.Lq + kQTile - 1) / kQTile;
   const int per_cta = fwd_tiles_per_cta(n_tiles, p.B * p.H, facts->n_sm, other);
   const dim3 grid(p.B * p.H, (n_tiles + per_cta - 1) / per_cta);
+  // With the programmatic-stream-serialization attribute the set-up (barriers, TMEM, tensor maps) may run while the kernel in
+  // front drains: it is a quarter of a short prompt's time (L = 77: 8.2 -> 5.9 us a call).  Flags are read during the set-up, so
+  // launches that take them do without.
+  cudaLaunchAttribute pdl[1];
+  pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.stream = st;
+  cfg.attrs = pdl;
+  cfg.numAttrs = other ? 0u : 1u;
 #define LMK_FWD_LAUNCH(BF, DIM, IRR, TILES)                                                                              \
-  sm100_fwd2_kernel<BF, DIM, IRR, TILES><<<grid, kFwdThreads<TILES>, fwd_smem<TILES>(IRR), st>>>(                        \
-      tq, tk, tv, tl, p.o, p.L, p.M, p.H, p.Lq, p.Lk, p.D, lm_box, scale_log2, p.k, p.ks[0], p.ks[1], p.ks[2], args)
+  do {                                                                                                                   \
+    cfg.blockDim = dim3(kFwdThreads<TILES>);                                                                             \
+    cfg.dynamicSmemBytes = fwd_smem<TILES>(IRR);                                                                         \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg, sm100_fwd2_kernel<BF, DIM, IRR, TILES>, tq, tk, tv, tl, (void*)p.o, p.L, p.M, p.H, \
+                                p.Lq, p.Lk, p.D, lm_box, scale_log2, (const void*)p.k, p.ks[0], p.ks[1], p.ks[2], args)); \
+  } while (0)
 #define LMK_FWD_TILES(BF, DIM, IRR)                                                           \
   do {                                                                                        \
-    if (per_cta == 1) LMK_FWD_LAUNCH(BF, DIM, IRR, 1); else LMK_FWD_LAUNCH(BF, DIM, IRR, 2);  \
+    if (per_cta == 1) LMK_FWD_LAUNCH(BF, DIM, IRR, 1);                                        \
+    else LMK_FWD_LAUNCH(BF, DIM, IRR, 2);                                                     \
   } while (0)
 #define LMK_FWD_DTYPE(BF)                                                                     \
   do {                                                                                        \
@@ -1827,15 +1844,15 @@ static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   // right after its set-up (only the set-up overlaps).  The dK/dV kernel reads q, k, v, dO, L, M, which were complete
   // before the dQ kernel started, and `delta`, which the dQ kernel writes: its loads and S / dP products start on
   // every SM the dQ kernel has left, and only its softmax threads wait (griddepcontrol.wait) before they read delta.
-  // The attribute is only attached while the stream is being captured into a CUDA graph: there it becomes a programmatic
-  // edge that costs nothing per replay, whereas an eager launch that carries launch attributes takes a slower path
-  // through the driver (measured: ~50 us more host time per call, which makes a 0.2 ms step host-bound).
+  // Not for other landmark patterns outside of graphs: the dK/dV kernel's units start late there (plan, gathered landmarks), and
+  // its CTAs that wait on SMs which the dQ kernel has left cost more than they hide (B16 H8 T512, groups of 51: the layer
+  // 212 -> 215 us; blocks of 64 at B1 H32 L2048 206 -> 203, B4 H16 L1024 D64 120 -> 118.5).
   cudaLaunchAttribute pdl[1];
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = 1;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   LMK_CUDA(cudaStreamIsCapturing(st, &capturing));
-  const unsigned n_attrs = capturing == cudaStreamCaptureStatusActive ? 1u : 0u;
+  const unsigned n_attrs = irr == nullptr || capturing == cudaStreamCaptureStatusActive ? 1u : 0u;
   cudaLaunchConfig_t cfg_dq = {}, cfg_dkv = {};
   cfg_dq.gridDim = grid_dq;  cfg_dq.blockDim = dim3(kDqThreads);  cfg_dq.dynamicSmemBytes = smem_dq;  cfg_dq.stream = st;
   cfg_dq.attrs = pdl;  cfg_dq.numAttrs = n_attrs;
