@@ -421,6 +421,8 @@ sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint32_t tmem = 0;
   // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left:
   // all of a CTA's marks at once, then one by one where there is any.
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   if (only_marked) {
     bool any = false;
     for (int w = blockIdx.x + (int)threadIdx.x * gridDim.x; w < n_tiles * BH; w += (int)blockDim.x * gridDim.x)
@@ -767,6 +769,8 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   bool held = false;
   uint32_t tmem = 0;
   // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left.
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   if (plan != nullptr) {
     bool any = false;
     for (int b = threadIdx.x; b < BH / H; b += blockDim.x) any |= plan[(int64_t)b * plan_stride + 1] != 0;
@@ -1128,6 +1132,8 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   bool held = false;
   uint32_t tmem = 0;
   // One tile a CTA, or -- behind the single-pass kernel, which usually leaves nothing -- a small grid that looks for what it left.
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   if (plan != nullptr) {
     bool any = false;
     for (int b = threadIdx.x; b < BH / H; b += blockDim.x) any |= plan[(int64_t)b * plan_stride + 1] != 0;
@@ -1210,12 +1216,11 @@ int attn_mask_sm100_fwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
   const int grid = only_marked && tiles > 148 ? 148 : tiles;
   const size_t smem = mf_smem_bytes(G, p.Lk / kKT);
   if (dtype == LMK_BF16)
-    sm100_mask_fwd_kernel<true><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.B * p.H, p.Lq,
-                                                                 p.Lk, G, scale_log2, only_marked, status);
+    LMK_CUDA(launch_overlapped(sm100_mask_fwd_kernel<true>, dim3(grid), dim3(kMfThreads), smem, st, tq, tk, tv, is_mem, is_mem_stride,
+                               p.o, R, A, p.H, p.B * p.H, p.Lq, p.Lk, G, scale_log2, only_marked, status));
   else
-    sm100_mask_fwd_kernel<false><<<grid, kMfThreads, smem, st>>>(tq, tk, tv, is_mem, is_mem_stride, p.o, R, A, p.H, p.B * p.H, p.Lq,
-                                                                  p.Lk, G, scale_log2, only_marked, status);
-  LMK_CUDA(cudaGetLastError());
+    LMK_CUDA(launch_overlapped(sm100_mask_fwd_kernel<false>, dim3(grid), dim3(kMfThreads), smem, st, tq, tk, tv, is_mem, is_mem_stride,
+                               p.o, R, A, p.H, p.B * p.H, p.Lq, p.Lk, G, scale_log2, only_marked, status));
   return LMK_OK;
 }
 
@@ -1254,18 +1259,16 @@ int attn_mask_sm100_bwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
   }
 #define LMK_MASK_BWD(BF)                                                                                                \
   do {                                                                                                                  \
-    sm100_mask_bwd_dq_kernel<BF><<<grid_q, kMqThreads, smem_q, st>>>(tq, tk, tv, tdo, is_mem, is_mem_stride, p.o, p.dO,  \
-                                                                     p.dos[0], p.dos[1], p.dos[2],                      \
-                                                                     R, A, delta, nD, p.dq, p.H, p.B * p.H, p.Lq, p.Lk, G, \
-                                                                     p.scale, scale_log2, plan, plan_stride, status);   \
-    sm100_mask_bwd_dkv_kernel<BF><<<grid_k, kMkThreads, kMkSmemBytes, st>>>(tq, tk, tv, tdo, is_mem, is_mem_stride, R,  \
-                                                                           A, delta, nD, p.dk, p.dv, p.H, p.B * p.H, p.Lq, p.Lk, \
-                                                                           G, p.scale, scale_log2, plan, plan_stride, status); \
+    LMK_CUDA(launch_overlapped(sm100_mask_bwd_dq_kernel<BF>, dim3(grid_q), dim3(kMqThreads), smem_q, st, tq, tk, tv, tdo, is_mem, \
+                               is_mem_stride, p.o, p.dO, p.dos[0], p.dos[1], p.dos[2], R, A, delta, nD, p.dq, p.H,      \
+                               p.B * p.H, p.Lq, p.Lk, G, p.scale, scale_log2, plan, plan_stride, status));              \
+    LMK_CUDA(launch_overlapped(sm100_mask_bwd_dkv_kernel<BF>, dim3(grid_k), dim3(kMkThreads), kMkSmemBytes, st, tq, tk, tv, tdo, \
+                               is_mem, is_mem_stride, R, A, delta, nD, p.dk, p.dv, p.H, p.B * p.H, p.Lq, p.Lk, G, p.scale, \
+                               scale_log2, plan, plan_stride, status));                                                 \
   } while (0)
   if (dtype == LMK_BF16) LMK_MASK_BWD(true);
   else LMK_MASK_BWD(false);
 #undef LMK_MASK_BWD
-  LMK_CUDA(cudaGetLastError());
   return LMK_OK;
 }
 

@@ -216,6 +216,8 @@ __device__ __forceinline__ int irr_plan_group(const int* plan, int b, int pos) {
   return __ldg(reinterpret_cast<const uint8_t*>(plan + (int64_t)b * kIrrPlanInts + kIrrPlanHead) + pos);
 }
 __global__ void __launch_bounds__(256) irr_plan_kernel(const uint8_t* __restrict__ flags, int64_t stride, int Lk, int G, int* plan) {
+  grid_dep_wait();
+  grid_dep_launch();
   __shared__ IrrSmem t;
   const int b = blockIdx.x;
   irr_build(t, flags + (int64_t)b * stride, Lk, G);
@@ -289,6 +291,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int pos_a = Lk - Lq + t_a * kQTile;             // key position of tile A's first row
   IrrSmem* tab = reinterpret_cast<IrrSmem*>(sm + 1);
   if constexpr (kIrr) {
+    grid_dep_wait();                                    // flags may come from the kernel in front
     if (irr.flags != nullptr) {
       irr_build(*tab, irr.flags + (int64_t)b * irr.stride, Lk, irr.G);
       if (tab->fallback) {                              // uniform; the two-pass kernel takes the tiles marked here
@@ -332,7 +335,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const uint32_t tmem = sm->tmem_base;
   auto tmem_s = [&](int w, int sb) { return tmem + (uint32_t)(w * 128 + sb * 64); };
   auto tmem_o = [&](int w) { return tmem + kTiles * 128u + (uint32_t)w * 128u; };
-  if constexpr (!kIrr) grid_dep_wait();      // only the set-up may overlap the kernel in front (see the launch)
+  if constexpr (!kIrr) grid_dep_wait();      // only the set-up may overlap the kernel in front (see the launch; kIrr: above)
   grid_dep_launch();      // a dependent kernel (the backward pass, the next call) may do its set-up while this grid drains
 
   if (warp == kSw) {
@@ -1743,8 +1746,7 @@ static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   const int per_cta = fwd_tiles_per_cta(n_tiles, p.B * p.H, facts->n_sm, other);
   const dim3 grid(p.B * p.H, (n_tiles + per_cta - 1) / per_cta);
   // With the programmatic-stream-serialization attribute the set-up (barriers, TMEM, tensor maps) may run while the kernel in
-  // front drains: it is a quarter of a short prompt's time (L = 77: 8.2 -> 5.9 us a call).  Flags are read during the set-up, so
-  // launches that take them do without.
+  // front drains: it is a quarter of a short prompt's time (L = 77: 8.2 -> 5.9 us a call).
   cudaLaunchAttribute pdl[1];
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1752,7 +1754,7 @@ static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   cfg.gridDim = grid;
   cfg.stream = st;
   cfg.attrs = pdl;
-  cfg.numAttrs = other ? 0u : 1u;
+  cfg.numAttrs = 1;
 #define LMK_FWD_LAUNCH(BF, DIM, IRR, TILES)                                                                              \
   do {                                                                                                                   \
     cfg.blockDim = dim3(kFwdThreads<TILES>);                                                                             \
@@ -1904,8 +1906,7 @@ size_t attn_sm100_plan_bytes(int B) { return sizeof(int) * (size_t)B * kIrrPlanI
 // apart) tells the two-pass kernels whether the row is theirs.
 int attn_sm100_flags_bwd(const AttnParams& p, const uint8_t* flags, int64_t stride, int G, const float* R, int* plan, int dtype,
                          cudaStream_t st) {
-  irr_plan_kernel<<<p.B, 256, 0, st>>>(flags, stride, p.Lk, G, plan);
-  LMK_CUDA(cudaGetLastError());
+  LMK_CUDA(launch_overlapped(irr_plan_kernel, dim3(p.B), dim3(256), 0, st, flags, stride, p.Lk, G, plan));
   IrrArgs a;
   a.flags = flags;
   a.stride = stride;

@@ -50,4 +50,22 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 static inline int dtype_size(int dtype) { return dtype == LMK_F32 ? 4 : 2; }
 
+// Launch with the programmatic-stream-serialization attribute: the kernel's CTAs may start, and its launch be processed, while the
+// kernel in front of it in the stream drains.  Such a kernel executes griddepcontrol.wait (ptx::grid_dep_wait) before it
+// touches global memory.
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 }  // namespace lmk
