@@ -146,6 +146,8 @@ template <int kD> constexpr size_t fwd_smem_f32 = sizeof(float) * (kRT * (kD + 4
 template <int kD>
 __global__ void __launch_bounds__(128 * kSplit, kD == 64 ? 2 : 1) f32_fwd_kernel(AttnParams p, int n_sm) {
   extern __shared__ __align__(16) float sm[];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   float* Qs = sm;
   const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, tx = tid & 15, ty = tid >> 4;
   float* Ks = Qs + kRT * (kD + 4) + group * (2 * kBK * (kD + 4) + kRT * kPS);
@@ -278,6 +280,8 @@ template <int kD> constexpr size_t dq_smem_f32 = sizeof(float) * (2 * kRT * (kD 
 template <int kD>
 __global__ void __launch_bounds__(128 * kSplit, kD == 64 ? 2 : 1) f32_bwd_dq_kernel(AttnParams p, int n_sm) {
   extern __shared__ __align__(16) float sm[];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   float* Qs = sm;
   float* Gs = Qs + kRT * (kD + 4);            // dO
   const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, tx = tid & 15, ty = tid >> 4;
@@ -410,6 +414,8 @@ template <int kD> constexpr size_t dkv_smem_f32 =
 template <int kD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256 * kSplit) f32_bwd_dkv_kernel(AttnParams p) {
   extern __shared__ __align__(16) float sm[];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   float* Ks = sm;
   float* Vs = Ks + kBK * (kD + 4);
   const int group = threadIdx.x >> 8, tid = threadIdx.x & 255, tx = tid & 15, ty = tid >> 4;              // ty 0 .. 15
@@ -592,8 +598,7 @@ int fwd_launch(const AttnParams& p, cudaStream_t st) {
   if (rc != LMK_OK) return rc;
   LMK_CUDA(cudaFuncSetAttribute(f32_fwd_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem_f32<kD>));
   const int grid = p.B * p.H * ((p.Lq + kRT - 1) / kRT);
-  f32_fwd_kernel<kD><<<grid, 128 * kSplit, fwd_smem_f32<kD>, st>>>(p, n_sm);
-  LMK_CUDA(cudaGetLastError());
+  LMK_CUDA(launch_overlapped(f32_fwd_kernel<kD>, dim3(grid), dim3(128 * kSplit), fwd_smem_f32<kD>, st, p, n_sm));
   return LMK_OK;
 }
 template <int kD>
@@ -603,10 +608,8 @@ int bwd_launch(const AttnParams& p, cudaStream_t st) {
   LMK_CUDA(cudaFuncSetAttribute(f32_bwd_dq_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq_smem_f32<kD>));
   LMK_CUDA(cudaFuncSetAttribute(f32_bwd_dkv_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dkv_smem_f32<kD>));
   const int grid = p.B * p.H * ((p.Lq + kRT - 1) / kRT);
-  f32_bwd_dq_kernel<kD><<<grid, 128 * kSplit, dq_smem_f32<kD>, st>>>(p, n_sm);
-  LMK_CUDA(cudaGetLastError());
-  f32_bwd_dkv_kernel<kD><<<2 * p.B * p.H * ((p.Lk + kBK - 1) / kBK), 256 * kSplit, dkv_smem_f32<kD>, st>>>(p);
-  LMK_CUDA(cudaGetLastError());
+  LMK_CUDA(launch_overlapped(f32_bwd_dq_kernel<kD>, dim3(grid), dim3(128 * kSplit), dq_smem_f32<kD>, st, p, n_sm));
+  LMK_CUDA(launch_overlapped(f32_bwd_dkv_kernel<kD>, dim3(2 * p.B * p.H * ((p.Lk + kBK - 1) / kBK)), dim3(256 * kSplit), dkv_smem_f32<kD>, st, p));
   return LMK_OK;
 }
 

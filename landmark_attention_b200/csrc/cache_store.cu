@@ -81,6 +81,8 @@ struct PrepParams {
 // 16-bit types; D / 16 threads per row, each owning one vector of the low half and its partner of the high half.
 template <typename T>
 __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepParams p) {
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const int lp = p.D / 16;                         // threads per row
   const int rows_per_cta = 128 / lp;
   const int t = blockIdx.x * rows_per_cta + threadIdx.x / lp;
@@ -155,9 +157,10 @@ __global__ void __launch_bounds__(128) cache_store_kernel(const uint4* __restric
 // Rotary position embedding of a [B,H,T,D] tensor pair (queries and keys of one layer) in one launch, both rotary
 // flavours, forward or inverse (the inverse rotation is the gradient of the forward one).  16-bit types use packed
 // arithmetic with the three roundings of the tensor formulation x * cos + rotate(x) * sin.
-// Bound by HBM (four tensors read or written once): a thread takes the same vector of four heads of both tensors, eight loads in
-// flight, and the tables' values once (B16 H8 T512 D128: 14.5 us with one head a thread -> @@R@@ us for 67 MB).
-constexpr int kRotHeads = 4;
+// Bound by HBM (four tensors read or written once): a thread takes the same vector of two heads of both tensors, four loads in
+// flight, and the tables' values once (B16 H8 T512 D128, the whole layer: one head 199.4 us, two 198.1, four 206.6; loads issued one
+// after the other 210).
+constexpr int kRotHeads = 2;
 struct RotParams {
   const void* in[2];
   void* out[2];
@@ -321,9 +324,8 @@ static int chunk_prepare(const void* q, const void* k, const void* v, const int6
   p.H = H; p.T = T; p.t_pad = t_pad; p.D = D;
   const int rows_per_cta = 128 / (D / 16);
   dim3 grid((t_pad + rows_per_cta - 1) / rows_per_cta, B * H);
-  if (dtype == LMK_BF16) chunk_prepare_kernel<__nv_bfloat16><<<grid, 128, 0, (cudaStream_t)stream>>>(p);
-  else chunk_prepare_kernel<__half><<<grid, 128, 0, (cudaStream_t)stream>>>(p);
-  LMK_CUDA(cudaGetLastError());
+  LMK_CUDA(launch_overlapped(dtype == LMK_BF16 ? chunk_prepare_kernel<__nv_bfloat16> : chunk_prepare_kernel<__half>, grid, dim3(128), 0,
+                             (cudaStream_t)stream, p));
   return LMK_OK;
 }
 

@@ -19,6 +19,7 @@
 #include <cooperative_groups.h>
 #include <type_traits>
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace lmk {
 namespace {
@@ -130,6 +131,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDecWarps * 32) dec
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   cluster.barrier_arrive();                       // completed by barrier_wait() before the first remote write
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const int t = blockIdx.x / CL, bh = blockIdx.y, b = bh / p.H, h = bh - b * p.H;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int K = p.top_k, N = p.n_blocks, blk = p.block;
@@ -428,8 +431,7 @@ int dec_launch(const DecParams& p, int BH, cudaStream_t st) {
   const size_t smem = dec_smem(p.n_blocks, p.top_k, CL);
   if (smem > 48 * 1024)
     LMK_CUDA(cudaFuncSetAttribute(decode_attend_kernel<T, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  decode_attend_kernel<T, CL><<<dim3(CL * p.T, BH), kDecWarps * 32, smem, st>>>(p);
-  LMK_CUDA(cudaGetLastError());
+  LMK_CUDA(launch_overlapped(decode_attend_kernel<T, CL>, dim3(CL * p.T, BH), dim3(kDecWarps * 32), smem, st, p));
   return LMK_OK;
 }
 

@@ -12,6 +12,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 #include "attn_params.h"
 
 namespace lmk {
@@ -1051,6 +1052,8 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
     grouped_softmax_lanes_kernel(const __grid_constant__ GsParams p, int n_chunks, int per_head_group, int per_warp) {
   extern __shared__ __align__(16) float gs_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const int head_groups = (p.H + per_head_group - 1) / per_head_group;
   const unsigned task = blockIdx.x * kGsWarps + warp;             // (batch row, group of heads, query)
   const int bg = (int)(task / (unsigned)p.Lq), i = (int)(task - (unsigned)bg * p.Lq);
@@ -1326,10 +1329,15 @@ int launch(const GsParams& p, int dtype, cudaStream_t st) {
     LMK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
     kernel<<<grid, kGsWarps * 32, smem, st>>>(__VA_ARGS__);                                                  \
   } while (0)
+#define LMK_GS_OVERLAPPED(kernel, ...)                                                                       \
+  do {                                                                                                       \
+    LMK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
+    LMK_CUDA(launch_overlapped(kernel, dim3(grid), dim3(kGsWarps * 32), smem, st, __VA_ARGS__));             \
+  } while (0)
 #define LMK_GS_LANES(T, causal)                                                                              \
   do {                                                                                                       \
-    if (n4 <= 8) LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 32>), p, n_chunks, per_group, per_warp);   \
-    else LMK_GS_RUN((grouped_softmax_lanes_kernel<T, kBackward, causal, 64>), p, n_chunks, per_group, per_warp);                \
+    if (n4 <= 8) LMK_GS_OVERLAPPED((grouped_softmax_lanes_kernel<T, kBackward, causal, 32>), p, n_chunks, per_group, per_warp);   \
+    else LMK_GS_OVERLAPPED((grouped_softmax_lanes_kernel<T, kBackward, causal, 64>), p, n_chunks, per_group, per_warp);                \
   } while (0)
 #define LMK_GS_LAUNCH(T)                                                                                     \
   do {                                                                                                       \
@@ -1343,6 +1351,7 @@ int launch(const GsParams& p, int dtype, cudaStream_t st) {
   else if (dtype == LMK_F16) LMK_GS_LAUNCH(__half);
   else LMK_GS_LAUNCH(__nv_bfloat16);
 #undef LMK_GS_LANES
+#undef LMK_GS_OVERLAPPED
 #undef LMK_GS_RUN
 #undef LMK_GS_LAUNCH
   LMK_CUDA(cudaGetLastError());

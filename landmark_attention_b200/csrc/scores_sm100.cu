@@ -59,6 +59,8 @@ __global__ void __launch_bounds__(128) rotate_landmarks_kernel(const T* __restri
   constexpr int D = 128, HALF = 64;
   const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
   const int N = desc.n_blocks, blk = desc.block;
+  grid_dep_wait();
+  grid_dep_launch();
   const int n = blockIdx.x * kRotPerCta + (threadIdx.x >> 3), d0 = (threadIdx.x & 7) * 8;
   if (n >= N) return;
   const T* row = kc + b * desc.stride_b + h * desc.stride_h + (int64_t)n * desc.stride_block +
@@ -125,6 +127,8 @@ __global__ void __launch_bounds__(128) scores_gemm_kernel(const __grid_constant_
   if (warp == 0) tmem_alloc(smem_u32(&sm->tmem_base), 128);
   tc_fence_before();
   __syncthreads();
+  grid_dep_wait();                 // only the set-up overlaps the kernel in front
+  grid_dep_launch();
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   if (tid == 0) {
@@ -225,8 +229,8 @@ int run(const void* q, const void* k_cache, const lmk_cache_desc& desc, const vo
         int rotary, float* scores, int B, int H, int Tq, float scale, int dtype, void* workspace, cudaStream_t st) {
   const int N = desc.n_blocks;
   dim3 g1((N + kRotPerCta - 1) / kRotPerCta, B * H);
-  rotate_landmarks_kernel<T><<<g1, 128, 0, st>>>((const T*)k_cache, desc, (const T*)cos_t, (const T*)sin_t, n_pos,
-                                                 rotary, (T*)workspace, H);
+  LMK_CUDA(launch_overlapped(rotate_landmarks_kernel<T>, g1, dim3(128), 0, st, (const T*)k_cache, desc, (const T*)cos_t,
+                             (const T*)sin_t, n_pos, rotary, (T*)workspace, H));
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) (void)cudaSetDevice(dev);   // bind the context for the driver call
   CUtensorMap tq, tk;
@@ -238,8 +242,7 @@ int run(const void* q, const void* k_cache, const lmk_cache_desc& desc, const vo
   dim3 g2((N + 127) / 128, (Tq + 127) / 128, B * H);
   int* status = device_status_word();
   if (status == nullptr) return fail(LMK_ERR_CUDA, "device status word is not addressable");
-  scores_gemm_kernel<T><<<g2, 128, smem, st>>>(tq, tk, scores, Tq, N, scale, status);
-  LMK_CUDA(cudaGetLastError());
+  LMK_CUDA(launch_overlapped(scores_gemm_kernel<T>, g2, dim3(128), smem, st, tq, tk, scores, Tq, N, scale, status));
   return LMK_OK;
 }
 
