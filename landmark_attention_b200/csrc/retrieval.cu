@@ -5,6 +5,7 @@
 // "slot" positions: the newest top_k blocks occupy slots 1..top_k, every older block shares slot 0.
 #include <type_traits>
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 #include "scores_sm100.h"
 
 namespace lmk {
@@ -256,6 +257,8 @@ __global__ void __launch_bounds__(128, 8) topk_sorted_rows_kernel(const float* _
   extern __shared__ __align__(16) float tk_smem[];          // per warp: n floats (general selection) + candidates
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t row = (int64_t)blockIdx.x * 4 + warp;
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   if (row >= rows) return;
   float* vals = tk_smem + (size_t)warp * (n + 2 * kTopkRegCand);
   float* cand_v = vals + n;
@@ -740,6 +743,8 @@ __global__ void __launch_bounds__(128, 8) selected_attend_kernel(const T* __rest
   constexpr int VGROUPS = 32 / LPR > 0 ? 32 / LPR : 1;      // value rows a warp reads per step
   struct __align__(16) Vec { T v[VEC]; };
   extern __shared__ __align__(16) float att_smem[];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const int t = blockIdx.x, bh = blockIdx.y;
   const int b = bh / H, h = bh - b * H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1019,9 +1024,8 @@ extern "C" int lmk_topk_sorted(const float* scores, int32_t* idx_out, int64_t ou
   if (n <= 1024 && (n & 3) == 0 && k <= 32 &&
       (((uintptr_t)scores | (uintptr_t)(outer_stride * 4) | (uintptr_t)(inner_stride * 4)) & 15) == 0) {
     const size_t rsm = sizeof(float) * 4 * ((size_t)n + 2 * kTopkRegCand);
-    topk_sorted_rows_kernel<<<(unsigned)((rows + 3) / 4), 128, rsm, (cudaStream_t)stream>>>(
-        scores, idx_out, rows, inner_count, outer_stride, inner_stride, n, k, ring_start);
-    LMK_CUDA(cudaGetLastError());
+    LMK_CUDA(launch_overlapped(topk_sorted_rows_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), rsm, (cudaStream_t)stream, scores,
+                               idx_out, rows, inner_count, outer_stride, inner_stride, n, k, ring_start));
     return LMK_OK;
   }
   int wpc = n <= 2048 ? 4 : (n <= 8192 ? 2 : 1);
@@ -1213,10 +1217,9 @@ extern "C" int lmk_selected_attend(const void* q, const void* k_cache, const lmk
   dim3 grid(T, B * H);
   cudaStream_t st = (cudaStream_t)stream;
 #define LMK_SA_LAUNCH(TT, LPR)                                                                                        \
-  selected_attend_kernel<TT, LPR><<<grid, 128, smem, st>>>((const TT*)q, (const TT*)k_cache, *kdesc,                 \
-                                                           (const TT*)v_cache, *vdesc, idx, (const TT*)cos_table,    \
-                                                           (const TT*)sin_table, n_pos, rotary, (const TT*)o_local,  \
-                                                           R_local, local_rows, (TT*)out, H, T, sm_scale)
+  LMK_CUDA(launch_overlapped(selected_attend_kernel<TT, LPR>, grid, dim3(128), smem, st, (const TT*)q, (const TT*)k_cache, \
+                             *kdesc, (const TT*)v_cache, *vdesc, idx, (const TT*)cos_table, (const TT*)sin_table, n_pos, \
+                             rotary, (const TT*)o_local, R_local, local_rows, (TT*)out, H, T, sm_scale))
 #define LMK_SA_DISPATCH(TT)                     \
   switch (lpr) {                                \
     case 4: LMK_SA_LAUNCH(TT, 4); break;        \
