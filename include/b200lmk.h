@@ -471,6 +471,18 @@ int lmk_prefix_gather(const void* q, const void* k_cache, const void* v_cache, c
 int lmk_prefix_pv(const float* probs, int64_t probs_ld, const void* v, const int64_t v_strides[3], void* y, int B, int H, int T,
                   int P, int D, int dtype, void* stream);
 
+/*
+ * Attention rows behind a retrieved prefix (lm_benchmark/models/landmark.py:196-243 with a cache): scores of the chunk's own keys,
+ * grouped softmax over [prefix | chunk] (query i sees the prefix and the chunk's keys 0 .. i; prefix_logits [B,H,T,P] dense, is_mem_row
+ * [B, P + T] bytes), prefix_probs [B,H,T,P] fp32 dense and out = probabilities of the chunk times v, [B,H,T,D] dense, to which
+ * lmk_prefix_pv adds the prefix' part.  16-bit types, D = 128; lmk_cached_rows_supported tells whether T and P fit.
+ */
+int lmk_cached_rows_supported(int D, int T, int P, int dtype);
+int lmk_cached_rows(const void* q, const void* k, const void* v, const int64_t q_strides[3], const int64_t k_strides[3],
+                    const int64_t v_strides[3], const void* prefix_logits, const uint8_t* is_mem_row, int64_t is_mem_stride,
+                    float* prefix_probs, void* out, int B, int H, int T, int P, int D, int max_groups, float sm_scale, int dtype,
+                    void* stream);
+
 #ifdef __cplusplus
 }
 #endif

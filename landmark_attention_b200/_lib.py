@@ -75,6 +75,9 @@ PROTOTYPES = {
                                                c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "lmk_grouped_softmax_causal_bwd_typed": (c_int, [c_void_p, POINTER(c_int64), c_void_p, c_int64, c_void_p, c_void_p, c_int,
                                                      c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "lmk_cached_rows_supported": (c_int, [c_int] * 4),
+    "lmk_cached_rows": (c_int, [c_void_p] * 3 + [POINTER(c_int64)] * 3 + [c_void_p, c_void_p, c_int64, c_void_p, c_void_p] +
+                        [c_int] * 6 + [c_float, c_int, c_void_p]),
     "lmk_cache_store": (c_int, [c_void_p, c_void_p, POINTER(c_int64), c_void_p, c_void_p, POINTER(CacheDesc),
                                 POINTER(CacheDesc), c_void_p, POINTER(c_int64), c_int, c_int, c_int, c_int, c_int, c_int,
                                 c_int, c_void_p]),

@@ -12,6 +12,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "mma16.cuh"
 #include "sm100_ptx.cuh"
 #include "attn_params.h"
 
@@ -1042,6 +1043,90 @@ struct LaneGroups {
   }
 };
 
+// the masks of a causal row: f = landmark flags, pi = the last key the query sees, `before` = places in front of the row
+template <int K>
+__device__ __forceinline__ void causal_masks(const Bits<K>& f, const Bits<K>& before, int pi, int lead, int j0, Bits<K>& mem,
+                                             Bits<K>& last, Bits<K>& act, Bits<K>& bk) {
+  using Mask = Bits<K>;
+  const Mask upto = Mask::low(lead + pi + 1 - j0), front = Mask::low(lead + pi - j0);
+  const Mask vis = Mask::zip([&](int w) { return upto.w[w] & ~before.w[w]; });
+  mem = Mask::zip([&](int w) { return f.w[w] & front.w[w]; });
+  const unsigned with = __ballot_sync(0xffffffffu, mem.count() != 0);
+  int p_last = __shfl_sync(0xffffffffu, j0 + mem.top(), with ? 31 - __clz(with) : 0);
+  if (!with) p_last = -1;
+  const Mask closed = Mask::low(p_last + 1 - j0);
+  last = Mask::zip([&](int w) { return vis.w[w] & ~f.w[w] & ~closed.w[w]; });
+  act = Mask::zip([&](int w) { return vis.w[w] & (~f.w[w] | mem.w[w]); });
+  bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | ~act.w[w]; });
+}
+
+// Passes 1 and 2 of a row: maxima of the groups and of the bucket, then exponentials (they replace the scores in shared
+// memory), sums and landmark weights.  binv: 1 / the bucket's sum; for the lane's groups a and b: i = 1 / the group's sum, w = the
+// landmark's share of the bucket; elm: exponential of the lane's own landmark.
+struct LaneWeights { float binv, ia, ib, wa, wb, elm; };
+template <typename T, int K>
+__device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4, int lm_slot, const Bits<K>& ga, const Bits<K>& gb,
+                                                    const Bits<K>& bk, const LaneGroups& lg, int ca, int G, bool guards) {
+  const int cb = ca + 1;
+  // pass 1: group and bucket maxima
+  float va = -INFINITY, vb = -INFINITY, bmax = -INFINITY;
+#pragma unroll 1
+  for (int q = 0; q < n4; ++q) {
+    const uint32_t fa = ga.piece(q), fb = gb.piece(q), fk = bk.piece(q);
+    float x[4];
+    xr.get<T>(xr.slot(c0 + q), x);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      if ((fa >> v) & 1u) va = fmaxf(va, x[v]);
+      if ((fb >> v) & 1u) vb = fmaxf(vb, x[v]);
+      if ((fk >> v) & 1u) bmax = fmaxf(bmax, x[v]);
+    }
+  }
+  // the landmark's score
+  float elm = sizeof(T) == 4 ? xr.buf[lm_slot] : to_f32(reinterpret_cast<const T*>(xr.buf)[2 * lm_slot + 4 - (lm_slot & 3)]);
+  bmax = warp_max(bmax);
+  if (guards && isinf(bmax)) bmax = 0.f;
+  float ma, mb, closed;
+  lg.reduce<true>(va, vb, ma, mb, closed);
+  // stabilisers; +inf beyond the last slot makes every exponential of such a group 0
+  ma = ca >= G ? INFINITY : (guards && isinf(ma)) ? 0.f : ma;
+  mb = cb >= G ? INFINITY : (guards && isinf(mb)) ? 0.f : mb;
+
+  // pass 2: exponentials, group and bucket sums
+  float bsum = 0.f;
+  va = vb = 0.f;
+#pragma unroll 1
+  for (int q = 0; q < n4; ++q) {
+    const uint32_t fa = ga.piece(q), fb = gb.piece(q), fk = bk.piece(q);
+    const int at = xr.slot(c0 + q);
+    float x[4];
+    xr.get<T>(at, x);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const bool ib = (fb >> v) & 1u, ik = (fk >> v) & 1u;
+      x[v] = exp_diff(x[v], ik ? bmax : ib ? mb : ma);               // keys outside the row hold -inf
+      if ((fa >> v) & 1u) va += x[v];
+      if (ib) vb += x[v];
+      if (ik) bsum += x[v];
+    }
+    xr.put(at, x);
+  }
+  elm = exp_diff(elm, bmax);
+  bsum = warp_sum(bsum);
+  const float binv = (guards && bsum < 0.5f) ? 0.f : 1.f / bsum;
+  float da, db;
+  lg.reduce<false>(va, vb, da, db, closed);
+  // scale of a non-bucket key: its landmark's weight over its group's sum (0 only for a group without keys)
+  auto inv_den = [&](int c, float den) -> float {
+    return (c >= G || (guards && den < 0.5f) || den == 0.f) ? 0.f : 1.f / den;
+  };
+  const float ia = inv_den(ca, da), ib = inv_den(cb, db);
+  float wa = __shfl_sync(0xffffffffu, elm, lg.src_a), wb = __shfl_sync(0xffffffffu, elm, lg.src_b);
+  wa = lg.has_a && ca < G ? wa * binv : 0.f;
+  wb = lg.has_b && cb < G ? wb * binv : 0.f;
+  return {binv, ia, ib, wa, wb, elm};
+}
+
 template <typename T, bool kBackward, bool kCausal>
 __device__ __noinline__ void grouped_softmax_crowded_row(const GsParams& p, int n_chunks, int64_t row, float* buf) {
   grouped_softmax_chunked_row<T, kBackward, kCausal>(p, n_chunks, row, buf);
@@ -1108,17 +1193,8 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
       Mask mem;
       const Mask in = Mask::low(lead + Lk - j0), before = Mask::low(lead - j0);
       if (kCausal) {
-        const Mask f = load_bits<K>(p.row_flags + b * p.row_flags_stride, 1, j0 - lead, n4, Lk);
-        const Mask upto = Mask::low(lead + pi + 1 - j0), front = Mask::low(lead + pi - j0);
-        const Mask vis = Mask::zip([&](int w) { return upto.w[w] & ~before.w[w]; });
-        mem = Mask::zip([&](int w) { return f.w[w] & front.w[w]; });
-        const unsigned with = __ballot_sync(0xffffffffu, mem.count() != 0);
-        int p_last = __shfl_sync(0xffffffffu, j0 + mem.top(), with ? 31 - __clz(with) : 0);
-        if (!with) p_last = -1;
-        const Mask closed = Mask::low(p_last + 1 - j0);
-        last = Mask::zip([&](int w) { return vis.w[w] & ~f.w[w] & ~closed.w[w]; });
-        act = Mask::zip([&](int w) { return vis.w[w] & (~f.w[w] | mem.w[w]); });
-        bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | ~act.w[w]; });
+        causal_masks<K>(load_bits<K>(p.row_flags + b * p.row_flags_stride, 1, j0 - lead, n4, Lk), before, pi, lead, j0, mem, last,
+                        act, bk);
       } else {
         mem = load_bits<K>(p.is_mem + b * p.ms[0] + h * p.ms[1] + i * p.ms[2], p.ms[3], j0 - lead, n4, Lk);
         last = load_bits<K>(p.last + b * p.ls[0] + h * p.ls[1] + i * p.ls[2], p.ls[3], j0 - lead, n4, Lk);
@@ -1145,66 +1221,13 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
     if (kBackward) gr.stage<float>(p.gprobs + row * Lk - lead, lead, n, n4, 0.f);
     asm volatile("" : "+r"(owners));                     // recomputed for every head rather than kept in registers
     const LaneGroups lg(lane, owners);
-    const int ca = __popc(owners & ((1u << lane) - 1u)), cb = ca + 1, n_groups = __popc(owners);
+    const int ca = __popc(owners & ((1u << lane) - 1u)), n_groups = __popc(owners);
     if (lane == 0 && n_groups >= G && p.status != nullptr) atomicCAS(p.status, 0, kErrSoftmaxGroups);
 
-    // pass 1: group and bucket maxima
-    float va = -INFINITY, vb = -INFINITY, bmax = -INFINITY;
-#pragma unroll 1
-    for (int q = 0; q < n4; ++q) {
-      const uint32_t fa = ga.piece(q), fb = gb.piece(q), fk = bk.piece(q);
-      float x[4];
-      xr.get<T>(xr.slot(c0 + q), x);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        if ((fa >> v) & 1u) va = fmaxf(va, x[v]);
-        if ((fb >> v) & 1u) vb = fmaxf(vb, x[v]);
-        if ((fk >> v) & 1u) bmax = fmaxf(bmax, x[v]);
-      }
-    }
-    // the landmark's score
-    float elm = sizeof(T) == 4 ? xr.buf[lm_slot] : to_f32(reinterpret_cast<const T*>(xr.buf)[2 * lm_slot + 4 - (lm_slot & 3)]);
-    bmax = warp_max(bmax);
-    if (guards && isinf(bmax)) bmax = 0.f;
-    float ma, mb, closed;
-    lg.reduce<true>(va, vb, ma, mb, closed);
-    // stabilisers; +inf beyond the last slot makes every exponential of such a group 0
-    ma = ca >= G ? INFINITY : (guards && isinf(ma)) ? 0.f : ma;
-    mb = cb >= G ? INFINITY : (guards && isinf(mb)) ? 0.f : mb;
-
-    // pass 2: exponentials, group and bucket sums
-    float bsum = 0.f;
-    va = vb = 0.f;
-#pragma unroll 1
-    for (int q = 0; q < n4; ++q) {
-      const uint32_t fa = ga.piece(q), fb = gb.piece(q), fk = bk.piece(q);
-      const int at = xr.slot(c0 + q);
-      float x[4];
-      xr.get<T>(at, x);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const bool ib = (fb >> v) & 1u, ik = (fk >> v) & 1u;
-        x[v] = exp_diff(x[v], ik ? bmax : ib ? mb : ma);               // keys outside the row hold -inf
-        if ((fa >> v) & 1u) va += x[v];
-        if (ib) vb += x[v];
-        if (ik) bsum += x[v];
-      }
-      xr.put(at, x);
-    }
-    elm = exp_diff(elm, bmax);
-    bsum = warp_sum(bsum);
-    const float binv = (guards && bsum < 0.5f) ? 0.f : 1.f / bsum;
-    float da, db;
-    lg.reduce<false>(va, vb, da, db, closed);
-    // scale of a non-bucket key: its landmark's weight over its group's sum (0 only for a group without keys)
-    auto inv_den = [&](int c, float den) -> float {
-      return (c >= G || (guards && den < 0.5f) || den == 0.f) ? 0.f : 1.f / den;
-    };
-    const float ia = inv_den(ca, da), ib = inv_den(cb, db);
-    float wa = __shfl_sync(0xffffffffu, elm, lg.src_a), wb = __shfl_sync(0xffffffffu, elm, lg.src_b);
-    wa = lg.has_a && ca < G ? wa * binv : 0.f;
-    wb = lg.has_b && cb < G ? wb * binv : 0.f;
-    const float sa = ia * wa, sb = ib * wb;
+    const LaneWeights lw = lane_weights<T, K>(xr, c0, n4, lm_slot, ga, gb, bk, lg, ca, G, guards);
+    const float binv = lw.binv, ia = lw.ia, ib = lw.ib, wa = lw.wa, elm = lw.elm;
+    float va, vb, closed;
+    const float sa = ia * wa, sb = ib * lw.wb;
 
     if (!kBackward) {
       const float none = guards ? 0.f : binv * 0.f;     // bucket keys outside the last section (NaN if binv is not finite)
@@ -1286,6 +1309,234 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
     grouped_softmax_crowded_row<T, kBackward, kCausal>(p, n_chunks, row_of(h0 + __ffs(later) - 1), xr.buf);
     __syncwarp();
   }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Attention rows behind a retrieved prefix, up to the prefix' values: local scores, grouped softmax over [prefix | chunk] and
+// the local part of probabilities times values (the cache branch of CausalSelfAttention.forward,
+// lm_benchmark/models/landmark.py:196-243).  One CTA per 16 queries of a head, its rows in shared memory from the scores to the
+// probabilities; scores and local output as mma.sync tiles, rounded where the tensor formulation rounds (the product, the
+// scaling, the probabilities, the output).  Written out: the prefix' probabilities (fp32) and the local output.
+// Bound by latency: 5 MB of operands and 80 MB of prefix logits and probabilities at B16 H8 T255 P204; library products, scaling,
+// concatenation, softmax and casts as kernels of their own took 167 us, this one takes 116 us (32 rows a CTA, half as many warps an SM: 130).
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int kCrRows = 16, kCrTiles = kCrRows / 16, kCrThreads = 256, kCrVPitch = 136;
+constexpr size_t kCrMaxSmem = 224 * 1024;
+
+struct CrParams {
+  const void *q, *k, *v;
+  int64_t qs[3], ks[3], vs[3];
+  const void* prefix;                   // [B, H, T, P] dense logits
+  const uint8_t* flags; int64_t flags_stride;      // [B, P + T]
+  float* probs;                         // [B, H, T, P]
+  void* out;                            // [B, H, T, 128]
+  int H, T, P, G;
+  float scale;
+  int* status;
+};
+__host__ __device__ constexpr int cr_pieces(int W) { return (W + 10 + 127) / 128; }      // lead, and scores are computed for eight keys at a time
+__host__ __device__ constexpr int cr_prob_pitch(int T) { return ((T + 15) & ~15) + 8; }
+__host__ __device__ constexpr size_t cr_smem(int T, int P) {
+  return sizeof(float) * kCrRows * 144 * (size_t)cr_pieces(P + T) + 2 * (size_t)kCrRows * cr_prob_pitch(T) + 2 * 64 * kCrVPitch;
+}
+
+// A row in which two landmarks share a lane: group after group, the whole warp on each.  Probabilities replace the scores.
+template <int K>
+__device__ __noinline__ void crowded_smem_row(LaneRow xr, int c0, int n4, Bits<K> mem, Bits<K> last, Bits<K> bk, int G) {
+  const int lane = threadIdx.x & 31;
+  const int nlm = mem.count();
+  int inc = nlm;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  const int before = inc - nlm, n_groups = __shfl_sync(0xffffffffu, inc, 31);
+  // f(score slot, landmarks in front of the key, landmark, last section, bucket) for every key of the lane
+  auto each = [&](auto f) {
+    int c = before;
+#pragma unroll 1
+    for (int v = 0; v < 4 * n4; ++v) {
+      const uint32_t m = mem.piece(v >> 2) >> (v & 3), l = last.piece(v >> 2) >> (v & 3), b = bk.piece(v >> 2) >> (v & 3);
+      f(xr.slot(c0 + (v >> 2)) * 4 + (v & 3), c, m & 1u, l & 1u, b & 1u);
+      c += m & 1u;
+    }
+  };
+  float mx = -INFINITY, sum = 0.f;
+  each([&](int e, int, uint32_t, uint32_t, uint32_t b) { if (b) mx = fmaxf(mx, xr.buf[e]); });
+  mx = warp_max(mx);
+  if (isinf(mx)) mx = 0.f;
+  each([&](int e, int, uint32_t, uint32_t, uint32_t b) { if (b) sum += exp_diff(xr.buf[e], mx); });
+  sum = warp_sum(sum);
+  const float binv = sum < 0.5f ? 0.f : 1.f / sum;
+  for (int g = 0; g <= n_groups; ++g) {
+    float gm = -INFINITY, lm = 0.f, den = 0.f;
+    each([&](int e, int c, uint32_t m, uint32_t, uint32_t b) {
+      if (c != g) return;
+      if (!b) gm = fmaxf(gm, xr.buf[e]);
+      if (m) lm = exp_diff(xr.buf[e], mx);
+    });
+    gm = warp_max(gm);
+    lm = g < G ? warp_sum(lm) * binv : warp_sum(lm) * 0.f;
+    if (isinf(gm)) gm = 0.f;
+    each([&](int e, int c, uint32_t, uint32_t, uint32_t b) { if (c == g && !b) den += exp_diff(xr.buf[e], gm); });
+    den = warp_sum(den);
+    const float w = den < 0.5f ? 0.f : lm / den;
+    each([&](int e, int c, uint32_t, uint32_t, uint32_t b) { if (c == g && !b) xr.buf[e] = exp_diff(xr.buf[e], gm) * w; });
+  }
+  each([&](int e, int, uint32_t, uint32_t l, uint32_t b) { if (b) xr.buf[e] = l ? exp_diff(xr.buf[e], mx) * binv : 0.f; });
+}
+
+template <typename T, int K>
+__global__ void __launch_bounds__(kCrThreads, K == 32 ? 4 : 2) cached_rows_kernel(const __grid_constant__ CrParams p) {
+  extern __shared__ __align__(16) float gs_smem[];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int bh = blockIdx.y, b = bh / p.H, h = bh - b * p.H;
+  const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kCrRows;             // longest rows first
+  const int W = p.P + p.T, n4max = cr_pieces(W), row_floats = 144 * n4max, pitch = cr_prob_pitch(p.T);
+  const int lead = (4 - (p.P & 3)) & 3;                                       // the chunk's first key starts a piece
+  T* pb = reinterpret_cast<T*>(gs_smem + kCrRows * row_floats);               // [16][pitch] local probabilities
+  T* vt = pb + kCrRows * pitch;                                               // [64][kCrVPitch] values
+  const T* q = reinterpret_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
+  const T* k = reinterpret_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
+  const T* v = reinterpret_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
+  const int n_keys = min(q0 + kCrRows, p.T);                                  // keys that any of the rows sees
+
+  // ---- local scores
+  {
+    uint4 a[kCrTiles][4], a8[kCrTiles][4];
+#pragma unroll
+    for (int m = 0; m < kCrTiles; ++m)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        a[m][c] = *reinterpret_cast<const uint4*>(q + (int64_t)min(q0 + 16 * m + g, p.T - 1) * p.qs[2] + 32 * c + 8 * t4);
+        a8[m][c] = *reinterpret_cast<const uint4*>(q + (int64_t)min(q0 + 16 * m + 8 + g, p.T - 1) * p.qs[2] + 32 * c + 8 * t4);
+      }
+    for (int nb = warp; nb * 8 < n_keys; nb += kCrThreads / 32) {
+      const T* kr = k + (int64_t)min(nb * 8 + g, p.T - 1) * p.ks[2] + 8 * t4;
+      uint4 kv[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) kv[c] = *reinterpret_cast<const uint4*>(kr + 32 * c);
+#pragma unroll
+      for (int m = 0; m < kCrTiles; ++m) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mma_chunk<T>(acc, a[m][c], a8[m][c], kv[c]);
+        const int e = lead + p.P + nb * 8 + 2 * t4;                           // even: both keys in one piece
+        const int at = LaneRow::slot(e >> 2) * 4 + (e & 3);
+        float* s = gs_smem + (16 * m + g) * row_floats + at;
+        *reinterpret_cast<float2*>(s) = make_float2(rnd<T>(rnd<T>(acc[0]) * p.scale), rnd<T>(rnd<T>(acc[1]) * p.scale));
+        *reinterpret_cast<float2*>(s + 8 * row_floats) =
+            make_float2(rnd<T>(rnd<T>(acc[2]) * p.scale), rnd<T>(rnd<T>(acc[3]) * p.scale));
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- softmax: a warp's rows one after the other
+  for (int r = warp; r < kCrRows; r += kCrThreads / 32) {
+    LaneRow xr{gs_smem + r * row_floats, lane};
+    T* prow = pb + r * pitch;
+    const int i = q0 + r;
+    if (i >= p.T) {
+      for (int j = lane; j < pitch; j += 32) prow[j] = from_f32<T>(0.f);
+      continue;
+    }
+    const uint8_t* fl = p.flags + b * p.flags_stride;
+    const int pi = p.P + i, n = lead + pi + ((fl[pi] & 1u) ? 0 : 1), n4 = max((n + 127) >> 7, 1);
+    const T* pre = reinterpret_cast<const T*>(p.prefix) + ((int64_t)bh * p.T + i) * p.P;
+    if (lane < lead) xr.buf[lane] = -INFINITY;
+    for (int e = n + lane; e < 128 * n4; e += 32) xr.buf[LaneRow::slot(e >> 2) * 4 + (e & 3)] = -INFINITY;
+    for (int c = lane; c < p.P; c += 32) {
+      const int e = lead + c;
+      if (e < n) xr.buf[LaneRow::slot(e >> 2) * 4 + (e & 3)] = to_f32(pre[c]);
+    }
+    __syncwarp();
+    using Mask = Bits<K>;
+    const int c0 = lane * n4, j0 = 4 * c0;
+    Mask mem, last, act, bk;
+    causal_masks<K>(load_bits<K>(fl, 1, j0 - lead, n4, W), Mask::low(lead - j0), pi, lead, j0, mem, last, act, bk);
+    const int nlm = mem.count();
+    const unsigned owners = __ballot_sync(0xffffffffu, nlm != 0);
+    const int n_groups = __reduce_add_sync(0xffffffffu, nlm);
+    if (lane == 0 && n_groups >= p.G && p.status != nullptr) atomicCAS(p.status, 0, kErrSoftmaxGroups);
+    if (__any_sync(0xffffffffu, nlm > 1)) {
+      crowded_smem_row<K>(xr, c0, n4, mem, last, bk, p.G);
+    } else {
+      const LaneGroups lg(lane, owners);
+      const int t = mem.first();
+      const Mask upto = Mask::low(t);
+      const Mask ga = Mask::zip([&](int w) { return ~bk.w[w] & upto.w[w]; });
+      const Mask gb = Mask::zip([&](int w) { return ~bk.w[w] & ~upto.w[w]; });
+      const int lm_slot = xr.slot(min(c0 + (t >> 2), 32 * n4 - 1)) * 4 + (t & 3);
+      const LaneWeights lw =
+          lane_weights<float, K>(xr, c0, n4, lm_slot, ga, gb, bk, lg, __popc(owners & ((1u << lane) - 1u)), p.G, true);
+      const float sa = lw.ia * lw.wa, sb = lw.ib * lw.wb;
+#pragma unroll 1
+      for (int c = 0; c < n4; ++c) {
+        const uint32_t fa = ga.piece(c), fb = gb.piece(c), fl2 = last.piece(c);
+        const int at = xr.slot(c0 + c);
+        float x[4];
+        xr.get<float>(at, x);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          x[u] *= (fl2 >> u) & 1u ? lw.binv : (fb >> u) & 1u ? sb : (fa >> u) & 1u ? sa : 0.f;
+        xr.put(at, x);
+      }
+    }
+    __syncwarp();
+    float* pr = p.probs + ((int64_t)bh * p.T + i) * p.P;
+    for (int c = lane; c < p.P; c += 32) {
+      const int e = lead + c;
+      pr[c] = e < 128 * n4 ? xr.buf[LaneRow::slot(e >> 2) * 4 + (e & 3)] : 0.f;
+    }
+    for (int j = lane; j < pitch; j += 32) {
+      const int e = lead + p.P + j;
+      prow[j] = from_f32<T>(j < p.T && e < n ? xr.buf[LaneRow::slot(e >> 2) * 4 + (e & 3)] : 0.f);
+    }
+  }
+
+  // ---- local output: warp w has features 16 w .. 16 w + 15 of all rows
+  float acc[kCrTiles][2][4] = {};
+  for (int j0 = 0; j0 < n_keys; j0 += 64) {
+    __syncthreads();                                    // probabilities written; the tile before has been read
+    for (int e = tid; e < 64 * 16; e += kCrThreads) {
+      const int r = e >> 4, c = (e & 15) * 8;
+      uint4 x = make_uint4(0u, 0u, 0u, 0u);
+      if (j0 + r < n_keys) x = *reinterpret_cast<const uint4*>(v + (int64_t)(j0 + r) * p.vs[2] + c);
+      *reinterpret_cast<uint4*>(vt + r * kCrVPitch + c) = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < 64; kk += 16) {
+      if (j0 + kk >= n_keys) break;
+      uint32_t bf[4], af[kCrTiles][4];
+      // values of keys kk .. kk + 15, features 16 warp .. + 15: two 16 x 8 B fragments
+      ldmatrix_x4_trans(bf, vt + (kk + (lane & 15)) * kCrVPitch + 16 * warp + 8 * (lane >> 4));
+#pragma unroll
+      for (int m = 0; m < kCrTiles; ++m) ldmatrix_x4(af[m], pb + (16 * m + (lane & 15)) * pitch + j0 + kk + 8 * (lane >> 4));
+#pragma unroll
+      for (int m = 0; m < kCrTiles; ++m) {
+        mma16<T>(acc[m][0], af[m][0], af[m][1], af[m][2], af[m][3], bf[0], bf[1]);
+        mma16<T>(acc[m][1], af[m][0], af[m][1], af[m][2], af[m][3], bf[2], bf[3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < kCrTiles; ++m)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int i = q0 + 16 * m + 8 * half + g;
+      if (i >= p.T) continue;
+      T* o = reinterpret_cast<T*>(p.out) + ((int64_t)bh * p.T + i) * 128 + 16 * warp + 2 * t4;
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn) {
+        o[8 * nn] = from_f32<T>(acc[m][nn][2 * half]);
+        o[8 * nn + 1] = from_f32<T>(acc[m][nn][2 * half + 1]);
+      }
+    }
 }
 
 static size_t fast_smem_bytes(int Lk, int max_groups) {
@@ -1483,4 +1734,40 @@ extern "C" int lmk_grouped_softmax_causal_bwd_typed(const void* x, const int64_t
                                                     int H, int Lq, int Lk, int dtype, int max_groups, void* stream) {
   return run_causal_bwd(x, x_strides, is_mem_row, is_mem_stride, grad_probs, grad_x, 1, B, H, Lq, Lk, dtype, max_groups,
                         stream);
+}
+
+extern "C" int lmk_cached_rows_supported(int D, int T, int P, int dtype) {
+  return (dtype == LMK_BF16 || dtype == LMK_F16) && D == 128 && T >= 1 && P >= 1 && P + T <= 2000 &&
+         lmk::cr_smem(T, P) <= lmk::kCrMaxSmem ? 1 : 0;
+}
+
+extern "C" int lmk_cached_rows(const void* q, const void* k, const void* v, const int64_t q_strides[3], const int64_t k_strides[3],
+                               const int64_t v_strides[3], const void* prefix_logits, const uint8_t* is_mem_row, int64_t is_mem_stride,
+                               float* prefix_probs, void* out, int B, int H, int T, int P, int D, int max_groups, float sm_scale,
+                               int dtype, void* stream) {
+  using namespace lmk;
+  LMK_CHECK_ARG(q && k && v && q_strides && k_strides && v_strides && prefix_logits && is_mem_row && prefix_probs && out,
+                "cached_rows: null pointer");
+  LMK_CHECK_ARG(B >= 1 && H >= 1 && (int64_t)B * H <= 65535, "cached_rows: bad sizes");
+  LMK_CHECK_ARG(max_groups >= 1 && max_groups <= 2048, "cached_rows: max_groups %d outside [1, 2048]", max_groups);
+  if (!lmk_cached_rows_supported(D, T, P, dtype))
+    return fail(LMK_ERR_UNSUPPORTED, "cached_rows needs a 16-bit type, D=128 and 16 rows of P + T keys in shared memory "
+                "(got dtype=%d D=%d T=%d P=%d)", dtype, D, T, P);
+  LMK_CHECK_ARG((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0, "cached_rows: pointers must be 16-byte aligned");
+  CrParams p{};
+  for (int i = 0; i < 3; ++i) {
+    LMK_CHECK_ARG(q_strides[i] % 8 == 0 && k_strides[i] % 8 == 0 && v_strides[i] % 8 == 0,
+                  "cached_rows: strides must be multiples of 8 elements");
+    p.qs[i] = q_strides[i]; p.ks[i] = k_strides[i]; p.vs[i] = v_strides[i];
+  }
+  p.q = q; p.k = k; p.v = v; p.prefix = prefix_logits; p.flags = is_mem_row; p.flags_stride = is_mem_stride;
+  p.probs = prefix_probs; p.out = out; p.H = H; p.T = T; p.P = P; p.G = max_groups; p.scale = sm_scale;
+  p.status = device_status_word();
+  const size_t smem = cr_smem(T, P);
+  const bool wide = cr_pieces(P + T) > 8;
+  const auto kernel = dtype == LMK_BF16 ? (wide ? cached_rows_kernel<__nv_bfloat16, 64> : cached_rows_kernel<__nv_bfloat16, 32>)
+                                        : (wide ? cached_rows_kernel<__half, 64> : cached_rows_kernel<__half, 32>);
+  LMK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LMK_CUDA(launch_overlapped(kernel, dim3((T + kCrRows - 1) / kCrRows, B * H), dim3(kCrThreads), smem, (cudaStream_t)stream, p));
+  return LMK_OK;
 }

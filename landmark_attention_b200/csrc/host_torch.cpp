@@ -42,7 +42,7 @@ using torch::autograd::variable_list;
   X(lmk_decode_supported) X(lmk_decode_attend) X(lmk_block_select) X(lmk_block_select_supported)                  \
   X(lmk_prefix_gather) X(lmk_prefix_gather_supported) X(lmk_prefix_pv) X(lmk_landmark_scores)                     \
   X(lmk_landmark_scores_workspace) X(lmk_topk_sorted) X(lmk_chunk_rotate) X(lmk_attn_fwd_lse)                     \
-  X(lmk_selected_attend) X(lmk_gather_kv_to)
+  X(lmk_selected_attend) X(lmk_gather_kv_to) X(lmk_cached_rows) X(lmk_cached_rows_supported)
 struct Lib {
 #define X(name) decltype(&::name) name = nullptr;
   LMK_FUNCS(X)
@@ -661,6 +661,30 @@ Tensor landmark_scores(const Chunk& c, const Tensor& q_rot, const Tensor& keys, 
   return s;
 }
 
+// A chunk behind a retrieved prefix (lmk_cached_rows, lmk_prefix_pv); undefined where the kernels do not take it or a gradient is asked for.
+Tensor cached_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& prefix, const Tensor& values, const Tensor& flags,
+                     int64_t max_groups, double scale) {
+  const auto st = q_.scalar_type();
+  if (!q_.is_cuda() || q_.dim() != 4 || k_.sizes() != q_.sizes() || v_.sizes() != q_.sizes() || prefix.dim() != 4 || values.dim() != 5 ||
+      needs_grad({q_, k_, v_, prefix, values}))
+    return Tensor();
+  const auto B = q_.size(0), H = q_.size(1), T = q_.size(2), D = q_.size(3), P = prefix.size(3);
+  for (const Tensor* t : {&k_, &v_, &prefix, &values})
+    if (!t->is_cuda() || t->scalar_type() != st) return Tensor();
+  if ((st != at::kHalf && st != at::kBFloat16) || D != 128 || B * H > 65535 || values.size(3) != P || !prefix.is_contiguous() ||
+      prefix.size(0) != B || prefix.size(1) != H || prefix.size(2) != T || !flags.is_cuda() || flags.scalar_type() != at::kBool ||
+      flags.dim() != 2 || flags.size(0) != B || flags.size(1) != P + T || flags.stride(1) != 1 || max_groups < 1 || max_groups > 2048 ||
+      !lib.lmk_cached_rows_supported(D, T, P, dtype_code(q_)))
+    return Tensor();
+  c10::cuda::OptionalCUDAGuard guard(q_.device());
+  const Tensor q = vector_rows(q_), k = vector_rows(k_), v = vector_rows(v_);
+  Tensor probs = empty_f32({B, H, T, P}, q), y = empty_like_dtype({B, H, T, D}, q);
+  check(lib.lmk_cached_rows(q.data_ptr(), k.data_ptr(), v.data_ptr(), S3(q).v, S3(k).v, S3(v).v, prefix.data_ptr(),
+                            (const uint8_t*)flags.data_ptr(), flags.stride(0), probs.data_ptr<float>(), y.data_ptr(), B, H, T, P, D,
+                            max_groups, scale, dtype_code(q), stream_of(q)), "lmk_cached_rows");
+  return prefix_pv(probs, values, y) ? y : Tensor();
+}
+
 // A second stream for the part of a call that nothing else in it waits for, with the events of the fork and the join (one set per
 // thread and device, reused: a wait refers to the event's state when it is enqueued).
 struct Fork {
@@ -934,6 +958,15 @@ PyObject* py_prefix_pv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// cached_attend(q, k, v, att_prefix, values, is_mem_row, max_groups, scale) -> out | None
+PyObject* py_cached_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 8);
+  return wrap_opt(cached_attend(tensor_arg(a[0], "q"), tensor_arg(a[1], "k"), tensor_arg(a[2], "v"), tensor_arg(a[3], "att_prefix"),
+                                tensor_arg(a[4], "values"), tensor_arg(a[5], "is_mem"), int_arg(a[6]), float_arg(a[7])));
+  END_HANDLE_TH_ERRORS
+}
+
 // chunk_attend(q, k_new, v_new, k_cache, v_cache, len, append, block, top_k, cos, sin, rotary) -> see wrap_appended
 PyObject* py_chunk_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -966,6 +999,7 @@ PyMethodDef methods[] = {{"init", py_init, METH_O, nullptr},
                          FAST("grouped_softmax", py_grouped_softmax),
                          FAST("grouped_softmax_causal", py_grouped_softmax_causal),
                          FAST("decode_attend", py_decode_attend),
+                         FAST("cached_attend", py_cached_attend),
                          FAST("chunk_attend", py_chunk_attend),
                          FAST("per_head_attend", py_per_head_attend),
                          FAST("cache_retrieve", py_cache_retrieve),

@@ -104,7 +104,8 @@ def lm_landmark_attention(q, k, v, is_mem_row, sm_scale=None, max_groups=None, a
     With a cache (the evaluation branch, :182-209 and :236-243): `att_prefix` [B,H,T,P] and `cache_values`
     {'v': [B,H,T,P,D] or [B,H,P,D], 'is_mem': [B,P] (optional)} are what `MemLMCacheStorage.retrieve_for_query`
     returns; the prefix columns are visible to every query and go through the same grouped softmax in front of the
-    chunk's own keys.  This branch takes the unfused route."""
+    chunk's own keys.  Without gradients, in 16-bit types with head dim 128, one kernel goes from the scores to the chunk's output
+    and a second one adds the prefix' part; otherwise this branch takes the unfused route."""
     from .masked import DEFAULT_MAX_GROUPS, landmark_attention_masked, masked_attention_supported
     B, H, T, D = q.shape
     if sm_scale is None:
@@ -113,16 +114,21 @@ def lm_landmark_attention(q, k, v, is_mem_row, sm_scale=None, max_groups=None, a
     fused_groups = DEFAULT_MAX_GROUPS if max_groups is None else int(max_groups)
     if n_pre == 0 and masked_attention_supported(q, k, fused_groups):
         return landmark_attention_masked(q, k, v, is_mem_row, sm_scale, fused_groups)
-    att = torch.matmul(q, k.transpose(-2, -1)) * sm_scale
+    groups = int(max_groups) if max_groups is not None else min(2048, T + n_pre + 1)
     if n_pre:
-        att = torch.cat((att_prefix.to(att.dtype), att), dim=-1)
         pre_mem = cache_values.get('is_mem')
         if pre_mem is None:
             pre_mem = torch.zeros((B, n_pre), dtype=torch.bool, device=q.device)
         is_mem_row = torch.cat((pre_mem.to(torch.bool), is_mem_row.to(torch.bool)), dim=-1)
+        # without gradients one kernel goes from the scores to the chunk's output, a second one reads the retrieved values once
+        y = L.host().cached_attend(q, k, v, att_prefix, cache_values['v'], is_mem_row, min(2048, max(groups, 2)), float(sm_scale))
+        if y is not None:
+            return y
+    att = torch.matmul(q, k.transpose(-2, -1)) * sm_scale
+    if n_pre:
+        att = torch.cat((att_prefix.to(att.dtype), att), dim=-1)
     # mask block + masked_fill + grouped softmax in one kernel, from the raw scores and the row flags
-    probs = landmark_grouped_softmax_causal(att, is_mem_row, max_groups if max_groups is not None
-                                            else min(2048, T + n_pre + 1))
+    probs = landmark_grouped_softmax_causal(att, is_mem_row, groups)
     if n_pre and not probs.requires_grad and cache_values['v'].dim() == v.dim() + 1 and not cache_values['v'].requires_grad:
         # the retrieved values are read once, by one kernel, from the fp32 probabilities
         y = torch.matmul(probs[..., n_pre:].to(v.dtype), v)
