@@ -1170,9 +1170,15 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
     const int lead_h = lead_of(h);
     int n = lead_h + seen;          // keys that the row is worked on for
     int n4_h = max((n + 127) >> 7, 1);
-    xr.stage<T>(reinterpret_cast<const T*>(p.x) + b * p.xs[0] + h * p.xs[1] + i * p.xs[2] - lead_h, lead_h, n, n4_h, -INFINITY);
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncwarp();
+    // Where the row's extent does not depend on its scores the masks come first: a crowded row is then not even read here.
+    auto stage_scores = [&]() {
+      xr.stage<T>(reinterpret_cast<const T*>(p.x) + b * p.xs[0] + h * p.xs[1] + i * p.xs[2] - lead_h, lead_h, lead_h + seen,
+                  max((lead_h + seen + 127) >> 7, 1), -INFINITY);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+    };
+    const bool by_scores = !kCausal && guards;
+    if (by_scores) stage_scores();
     if (!kCausal && guards) {
       // scores of -inf at the row's end weigh nothing, whatever their flags say, and neither does a landmark among them
       int top = 0;
@@ -1218,6 +1224,7 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
       later |= 1u << (h - h0);
       continue;
     }
+    if (!by_scores) stage_scores();
     if (kBackward) gr.stage<float>(p.gprobs + row * Lk - lead, lead, n, n4, 0.f);
     asm volatile("" : "+r"(owners));                     // recomputed for every head rather than kept in registers
     const LaneGroups lg(lane, owners);
@@ -1560,7 +1567,11 @@ int launch(const GsParams& p, int dtype, cudaStream_t st) {
   size_t smem = fast ? fast_smem_bytes(p.Lk, p.max_groups) : sizeof(float) * 4 * (size_t)p.max_groups * kGsWarps;
   // pieces a lane of the longest row, counted with its lead (rows of a multiple of four keys have none)
   const int n4 = (p.Lk + (p.Lk % 4 ? 3 : 0) + 127) / 128;
-  const bool lanes = fast && n4 <= kLaneMaxPieces && rows < (1LL << 31);
+  // Rows with two landmarks in a lane are done by the chunked form in the end; with guards, where a lane's keys follow the row's
+  // extent, those are the rows beyond 32 groups' length.  max_groups tells when they would be the greater part (masked
+  // scores, forward and backward, B2 H32, groups of 32 in rows of 1030: 1247 us chunked, 540 with six rows of that kind).
+  const bool sparse = n4 <= 8 || !p.guards || p.max_groups <= 67;
+  const bool lanes = fast && n4 <= kLaneMaxPieces && sparse && rows < (1LL << 31);
   // Heads a warp takes in turn: as many as leave every SM three rounds of
   // warps (causal rows differ in length), eight at most.
   int per_group = 1, per_warp = 0;
