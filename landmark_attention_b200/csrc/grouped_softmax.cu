@@ -833,12 +833,11 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsP
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Rows of up to about 2048 keys with a landmark at most every 1/32 of the row or so: lane l owns the 4 n4 contiguous keys
-// from l * 4 n4 on (n4 = ceil(keys / 128)), in shared memory through all passes, and at most one landmark falls into
-// a lane.  A group is then the tail of one lane, whole lanes behind it and the head of the lane that holds its
+// Rows of up to about 2048 keys with at most two landmarks in 1/32 of the row: lane l owns the 4 n4 contiguous keys
+// from l * 4 n4 on (n4 = ceil(keys / 128)), in shared memory through all passes.  A group is then the tail of one lane, whole lanes behind it and the head of the lane that holds its
 // landmark: one segmented scan over the lanes per pass reduces every group of the row, and two shuffles hand each lane
-// the results of the (at most two) groups its keys lie in.  Nothing per group is kept in memory and no pass looks
-// anything up per key.  A row in which two landmarks share a lane is done by the chunked form above.
+// the results of the (at most two) groups its keys lie in; where lanes hold two landmarks, the keys between them are a third one.  Nothing per group is kept in memory and no pass looks
+// anything up per key.  A row with three landmarks in a lane is done by the chunked form above.
 //
 // Bound by the instructions per row (two thirds of the issue slots at 40 % of the copy bandwidth), so what can be shared is:
 // a warp takes the same query of several heads in turn, and masks that are broadcast over the heads are read, packed to a
@@ -849,7 +848,8 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsP
 //
 // Keys are counted from the 4-element boundary at or in front of the row's place in the dense results (`lead` keys earlier),
 // so rows of any length are copied, read and written four elements at a time except for the row's two ends.
-// B16 H8 512 x 512 fp32, landmarks every 51 keys: forward 138 -> 98 us, backward 216 -> 130 us.
+// B16 H8 512 x 512 fp32, landmarks every 51 keys: forward 138 -> 98 us, backward 216 -> 130 us.  Two landmarks in a lane have code of
+// their own (rows of 1064 keys, groups of 32, B2 H32, forward and backward: 994 -> 668 us; by the chunked form 1054).
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kLaneMaxPieces = 16;             // n4 of the longest row
 
@@ -1063,11 +1063,14 @@ __device__ __forceinline__ void causal_masks(const Bits<K>& f, const Bits<K>& be
 // Passes 1 and 2 of a row: maxima of the groups and of the bucket, then exponentials (they replace the scores in shared
 // memory), sums and landmark weights.  binv: 1 / the bucket's sum; for the lane's groups a and b: i = 1 / the group's sum, w = the
 // landmark's share of the bucket; elm: exponential of the lane's own landmark.
-struct LaneWeights { float binv, ia, ib, wa, wb, elm; };
-template <typename T, int K>
+// kTwo: some lanes hold two landmarks; the keys between them (gm) are a group of their own, closed by the second one (lm2_slot).
+struct LaneWeights { float binv, ia, ib, wa, wb, elm, im, wm, elm2; };
+template <typename T, int K, bool kTwo>
 __device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4, int lm_slot, const Bits<K>& ga, const Bits<K>& gb,
-                                                    const Bits<K>& bk, const LaneGroups& lg, int ca, int G, bool guards) {
-  const int cb = ca + 1;
+                                                    const Bits<K>& bk, const LaneGroups& lg, int ca, int G, bool guards,
+                                                    const Bits<K>& gm = Bits<K>(), int lm2_slot = 0, int nlm = 1) {
+  const int cb = kTwo ? ca + max(nlm, 1) : ca + 1;
+  float vm = -INFINITY;
   // pass 1: group and bucket maxima
   float va = -INFINITY, vb = -INFINITY, bmax = -INFINITY;
 #pragma unroll 1
@@ -1080,10 +1083,12 @@ __device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4,
       if ((fa >> v) & 1u) va = fmaxf(va, x[v]);
       if ((fb >> v) & 1u) vb = fmaxf(vb, x[v]);
       if ((fk >> v) & 1u) bmax = fmaxf(bmax, x[v]);
+      if (kTwo && ((gm.piece(q) >> v) & 1u)) vm = fmaxf(vm, x[v]);
     }
   }
-  // the landmark's score
-  float elm = sizeof(T) == 4 ? xr.buf[lm_slot] : to_f32(reinterpret_cast<const T*>(xr.buf)[2 * lm_slot + 4 - (lm_slot & 3)]);
+  // the landmarks' scores
+  auto score = [&](int at) { return sizeof(T) == 4 ? xr.buf[at] : to_f32(reinterpret_cast<const T*>(xr.buf)[2 * at + 4 - (at & 3)]); };
+  float elm = score(lm_slot), elm2 = kTwo ? score(lm2_slot) : 0.f;
   bmax = warp_max(bmax);
   if (guards && isinf(bmax)) bmax = 0.f;
   float ma, mb, closed;
@@ -1092,9 +1097,11 @@ __device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4,
   ma = ca >= G ? INFINITY : (guards && isinf(ma)) ? 0.f : ma;
   mb = cb >= G ? INFINITY : (guards && isinf(mb)) ? 0.f : mb;
 
+  const float mm = ca + 1 >= G ? INFINITY : (guards && isinf(vm)) ? 0.f : vm;
+
   // pass 2: exponentials, group and bucket sums
   float bsum = 0.f;
-  va = vb = 0.f;
+  va = vb = vm = 0.f;
 #pragma unroll 1
   for (int q = 0; q < n4; ++q) {
     const uint32_t fa = ga.piece(q), fb = gb.piece(q), fk = bk.piece(q);
@@ -1104,7 +1111,9 @@ __device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4,
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       const bool ib = (fb >> v) & 1u, ik = (fk >> v) & 1u;
-      x[v] = exp_diff(x[v], ik ? bmax : ib ? mb : ma);               // keys outside the row hold -inf
+      const bool im = kTwo && ((gm.piece(q) >> v) & 1u);
+      x[v] = exp_diff(x[v], ik ? bmax : ib ? mb : im ? mm : ma);       // keys outside the row hold -inf
+      if (im) vm += x[v];
       if ((fa >> v) & 1u) va += x[v];
       if (ib) vb += x[v];
       if (ik) bsum += x[v];
@@ -1112,6 +1121,7 @@ __device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4,
     xr.put(at, x);
   }
   elm = exp_diff(elm, bmax);
+  elm2 = exp_diff(elm2, bmax);
   bsum = warp_sum(bsum);
   const float binv = (guards && bsum < 0.5f) ? 0.f : 1.f / bsum;
   float da, db;
@@ -1124,7 +1134,8 @@ __device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4,
   float wa = __shfl_sync(0xffffffffu, elm, lg.src_a), wb = __shfl_sync(0xffffffffu, elm, lg.src_b);
   wa = lg.has_a && ca < G ? wa * binv : 0.f;
   wb = lg.has_b && cb < G ? wb * binv : 0.f;
-  return {binv, ia, ib, wa, wb, elm};
+  const float im = inv_den(ca + 1, vm), wm = ca + 1 < G ? elm2 * binv : 0.f;
+  return {binv, ia, ib, wa, wb, elm, im, wm, elm2};
 }
 
 template <typename T, bool kBackward, bool kCausal>
@@ -1160,11 +1171,11 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
 
   using Mask = Bits<K>;
   // what follows from the masks, kept while they, the lead and the number of pieces stay the same
-  Mask last, bk, act, ga, gb;       // last section, bucket, all but merely hidden keys, members of the lane's two groups
+  Mask last, bk, act, ga, gb, gm;   // last section, bucket, all but merely hidden keys, members of the lane's groups
   unsigned owners = 0;              // lanes with a landmark
-  int n4 = 0, lead = -1, c0 = 0, lm_slot = 0;     // c0: the lane's first piece
-  bool crowded = false, lm_last = false;                // lm_last: the lane's landmark is in the last section too
-  unsigned later = 0;               // heads whose row has two landmarks in one lane
+  int n4 = 0, lead = -1, c0 = 0, nlm = 0, lm_slot = 0, lm2_slot = 0;     // c0: the lane's first piece
+  bool crowded = false, two = false, lm_last = false, lm2_last = false;      // lm_last: the landmark is in the last section too
+  unsigned later = 0;               // heads whose row has three landmarks in one lane
   for (int h = h0; h < h1; ++h) {
     const int64_t row = row_of(h);
     const int lead_h = lead_of(h);
@@ -1210,15 +1221,20 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
         bk = Mask::zip([&](int w) { return mem.w[w] | last.w[w] | hid.w[w] | ~in.w[w] | before.w[w]; });
         act = Mask::zip([&](int w) { return ~bk.w[w] | mem.w[w] | last.w[w]; });
       }
-      const int nlm = mem.count();
-      crowded = __any_sync(0xffffffffu, nlm > 1);
+      nlm = mem.count();
+      crowded = __any_sync(0xffffffffu, nlm > 2);
+      two = __any_sync(0xffffffffu, nlm == 2);
       owners = __ballot_sync(0xffffffffu, nlm != 0);
-      const int t = mem.first();                        // the lane's landmark: group a in front of it, group b behind
-      const Mask upto = Mask::low(t);
+      // the lane's landmarks t <= t2: group a in front of the first, group b behind the last, a group of its own between them
+      const int t = mem.first(), t2 = nlm ? mem.top() : K;
+      const Mask upto = Mask::low(t), upto2 = Mask::low(t2);
       ga = Mask::zip([&](int w) { return ~bk.w[w] & upto.w[w]; });
-      gb = Mask::zip([&](int w) { return ~bk.w[w] & ~upto.w[w]; });
-      lm_last = (mem.w[0] & last.w[0]) != 0 || (K > 32 && (mem.w[K > 32 ? 1 : 0] & last.w[K > 32 ? 1 : 0]) != 0);
+      gb = Mask::zip([&](int w) { return ~bk.w[w] & ~upto2.w[w]; });
+      gm = Mask::zip([&](int w) { return ~bk.w[w] & ~upto.w[w] & upto2.w[w]; });
+      lm_last = nlm != 0 && ((last.piece(t >> 2) >> (t & 3)) & 1u);
+      lm2_last = nlm != 0 && ((last.piece(t2 >> 2) >> (t2 & 3)) & 1u);
       lm_slot = xr.slot(min(c0 + (t >> 2), 32 * n4 - 1)) * 4 + (t & 3);
+      lm2_slot = xr.slot(min(c0 + (t2 >> 2), 32 * n4 - 1)) * 4 + (t2 & 3);
     }
     if (crowded) {
       later |= 1u << (h - h0);
@@ -1226,15 +1242,27 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
     }
     if (!by_scores) stage_scores();
     if (kBackward) gr.stage<float>(p.gprobs + row * Lk - lead, lead, n, n4, 0.f);
+    auto finish = [&](auto two_in_a_lane) {
+    constexpr bool kTwo = decltype(two_in_a_lane)::value;
     asm volatile("" : "+r"(owners));                     // recomputed for every head rather than kept in registers
     const LaneGroups lg(lane, owners);
-    const int ca = __popc(owners & ((1u << lane) - 1u)), n_groups = __popc(owners);
+    int ca = __popc(owners & ((1u << lane) - 1u)), n_groups = __popc(owners);
+    if constexpr (kTwo) {                               // landmarks in front of the lane
+      int inc = nlm;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+      }
+      ca = inc - nlm;
+      n_groups = __shfl_sync(0xffffffffu, inc, 31);
+    }
     if (lane == 0 && n_groups >= G && p.status != nullptr) atomicCAS(p.status, 0, kErrSoftmaxGroups);
 
-    const LaneWeights lw = lane_weights<T, K>(xr, c0, n4, lm_slot, ga, gb, bk, lg, ca, G, guards);
+    const LaneWeights lw = lane_weights<T, K, kTwo>(xr, c0, n4, lm_slot, ga, gb, bk, lg, ca, G, guards, gm, lm2_slot, nlm);
     const float binv = lw.binv, ia = lw.ia, ib = lw.ib, wa = lw.wa, elm = lw.elm;
     float va, vb, closed;
-    const float sa = ia * wa, sb = ib * lw.wb;
+    const float sa = ia * wa, sb = ib * lw.wb, sm = lw.im * lw.wm;
 
     if (!kBackward) {
       const float none = guards ? 0.f : binv * 0.f;     // bucket keys outside the last section (NaN if binv is not finite)
@@ -1248,7 +1276,7 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
           const bool il = (fl >> v) & 1u;
-          x[v] *= il ? binv : (fb >> v) & 1u ? sb : (fa >> v) & 1u ? sa : none;
+          x[v] *= il ? binv : (fb >> v) & 1u ? sb : (kTwo && ((gm.piece(q) >> v) & 1u)) ? sm : (fa >> v) & 1u ? sa : none;
           if (il) last_total += x[v];
         }
         xr.put(at, x);
@@ -1258,6 +1286,7 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
         float* gp = p.group_prob + row * p.max_mem_cnt;
         for (int g = n_groups + lane; g < p.max_mem_cnt - 1; g += 32) gp[g] = 0.f;
         if (lg.own && ca < p.max_mem_cnt - 1) gp[ca] = wa;
+        if (kTwo && nlm == 2 && ca + 1 < p.max_mem_cnt - 1) gp[ca + 1] = lw.wm;
         if (lane == 0) gp[p.max_mem_cnt - 1] = last_total;
       }
       __syncwarp();
@@ -1266,7 +1295,7 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncwarp();
       // pass 3: c_g = sum_j inner_j * grad_j per group, total = sum_j P_j * grad_j over the row
-      float lsum = 0.f;
+      float lsum = 0.f, vm = 0.f;
       va = vb = 0.f;
 #pragma unroll 1
       for (int q = 0; q < n4; ++q) {
@@ -1280,16 +1309,19 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
           if ((fa >> v) & 1u) va = fmaf(x[v], g[v], va);
           if ((fb >> v) & 1u) vb = fmaf(x[v], g[v], vb);
           if ((fl >> v) & 1u) lsum = fmaf(x[v], g[v], lsum);
+          if (kTwo && ((gm.piece(q) >> v) & 1u)) vm = fmaf(x[v], g[v], vm);
         }
       }
       float c_a, c_b;
       lg.reduce<false>(va, vb, c_a, c_b, closed);
       c_a *= ia;
       c_b *= ib;
-      const float total = warp_sum((lg.own ? closed * ia * wa : 0.f) + lsum * binv);
+      const float c_m = kTwo ? vm * lw.im : 0.f;
+      const float total = warp_sum((lg.own ? closed * ia * wa : 0.f) + (kTwo && nlm == 2 ? c_m * lw.wm : 0.f) + lsum * binv);
       // pass 4: last section P_j * (g_j - total), group member P_j * (g_j - c_g); a landmark P_j * (c_g - total), plus g_j
       // if it is in the last section too
       const float lm_g = lm_last ? gr.buf[lm_slot] : 0.f;
+      const float lm2_g = kTwo && lm2_last ? gr.buf[lm2_slot] : 0.f;
 #pragma unroll 1
       for (int q = 0; q < n4; ++q) {
         const uint32_t fb = gb.piece(q), fl = last.piece(q), fx = act.piece(q);
@@ -1300,16 +1332,21 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
           const bool ib = (fb >> v) & 1u, il = (fl >> v) & 1u;
-          const float s = il ? binv : ib ? sb : sa, sub = il ? total : ib ? c_b : c_a;
+          const bool im = kTwo && ((gm.piece(q) >> v) & 1u);
+          const float s = il ? binv : ib ? sb : im ? sm : sa, sub = il ? total : ib ? c_b : im ? c_m : c_a;
           x[v] = (fx >> v) & 1u ? x[v] * s * (g[v] - sub) : 0.f;
         }
         gr.put(at, x);                                  // the lane's own pieces, read just before
       }
       if (lg.own) gr.buf[lm_slot] = elm * binv * (lm_g + c_a - total);
+      if (kTwo && nlm == 2) gr.buf[lm2_slot] = lw.elm2 * binv * (lm2_g + c_m - total);
       __syncwarp();
       if (p.gx_as_x) gr.write<T>(reinterpret_cast<T*>(p.gx) + row * Lk - lead, lead, lead + Lk, n4);
       else gr.write<float>(reinterpret_cast<float*>(p.gx) + row * Lk - lead, lead, lead + Lk, n4);
     }
+    };
+    if (two) finish(std::true_type{});
+    else finish(std::false_type{});
     __syncwarp();                                       // the results have been read
   }
   for (; later; later &= later - 1) {
@@ -1347,7 +1384,7 @@ __host__ __device__ constexpr size_t cr_smem(int T, int P) {
   return sizeof(float) * kCrRows * 144 * (size_t)cr_pieces(P + T) + 2 * (size_t)kCrRows * cr_prob_pitch(T) + 2 * 64 * kCrVPitch;
 }
 
-// A row in which two landmarks share a lane: group after group, the whole warp on each.  Probabilities replace the scores.
+// A row in which two landmarks share a lane (cached rows): group after group, the whole warp on each.  Probabilities replace the scores.
 template <int K>
 __device__ __noinline__ void crowded_smem_row(LaneRow xr, int c0, int n4, Bits<K> mem, Bits<K> last, Bits<K> bk, int G) {
   const int lane = threadIdx.x & 31;
@@ -1479,7 +1516,7 @@ __global__ void __launch_bounds__(kCrThreads, K == 32 ? 4 : 2) cached_rows_kerne
       const Mask gb = Mask::zip([&](int w) { return ~bk.w[w] & ~upto.w[w]; });
       const int lm_slot = xr.slot(min(c0 + (t >> 2), 32 * n4 - 1)) * 4 + (t & 3);
       const LaneWeights lw =
-          lane_weights<float, K>(xr, c0, n4, lm_slot, ga, gb, bk, lg, __popc(owners & ((1u << lane) - 1u)), p.G, true);
+          lane_weights<float, K, false>(xr, c0, n4, lm_slot, ga, gb, bk, lg, __popc(owners & ((1u << lane) - 1u)), p.G, true);
       const float sa = lw.ia * lw.wa, sb = lw.ib * lw.wb;
 #pragma unroll 1
       for (int c = 0; c < n4; ++c) {
@@ -1567,11 +1604,7 @@ int launch(const GsParams& p, int dtype, cudaStream_t st) {
   size_t smem = fast ? fast_smem_bytes(p.Lk, p.max_groups) : sizeof(float) * 4 * (size_t)p.max_groups * kGsWarps;
   // pieces a lane of the longest row, counted with its lead (rows of a multiple of four keys have none)
   const int n4 = (p.Lk + (p.Lk % 4 ? 3 : 0) + 127) / 128;
-  // Rows with two landmarks in a lane are done by the chunked form in the end; with guards, where a lane's keys follow the row's
-  // extent, those are the rows beyond 32 groups' length.  max_groups tells when they would be the greater part (masked
-  // scores, forward and backward, B2 H32, groups of 32 in rows of 1030: 1247 us chunked, 540 with six rows of that kind).
-  const bool sparse = n4 <= 8 || !p.guards || p.max_groups <= 67;
-  const bool lanes = fast && n4 <= kLaneMaxPieces && sparse && rows < (1LL << 31);
+  const bool lanes = fast && n4 <= kLaneMaxPieces && rows < (1LL << 31);
   // Heads a warp takes in turn: as many as leave every SM three rounds of
   // warps (causal rows differ in length), eight at most.
   int per_group = 1, per_warp = 0;

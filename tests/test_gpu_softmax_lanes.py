@@ -26,7 +26,8 @@ def test_sparse_landmarks(Lk, dtype, guards):
         is_mem[:, :, r, (k - 1 if r % 2 else 2 * k)::3 * k] = True
     is_mem[..., 0] = False
     if Lk > 8:
-        is_mem[:, :, Lq - 1, 4:7:2] = k > 7                        # two landmarks in one lane: the other form
+        is_mem[:, :, Lq - 1, 4:7:2] = k > 7                        # two landmarks in one lane: a group between them
+        is_mem[:, :, Lq - 2, 1:6:2] = k > 7                        # three: the other form
     last = torch.zeros_like(is_mem)
     last[..., Lk - max(1, Lk // 5):] = True
     last &= ~is_mem
@@ -53,6 +54,33 @@ def test_sparse_landmarks(Lk, dtype, guards):
     assert (got.detach().cpu() - exp.detach()).abs().max().item() < 2e-6
     (gx,) = torch.autograd.grad(got, [xd], gp.to(DEV))
     assert gx.dtype == dtype and (gx.float().cpu() - gx_exp).abs().max().item() < _grad_tol(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("Lk,block", [(1064, 32), (2048, 32), (1500, 51), (2047, 64), (700, 12)])
+@pytest.mark.parametrize("guards", [True, False])
+def test_regular_groups(Lk, block, dtype, guards):
+    import landmark_attention_b200 as P
+    g = torch.Generator().manual_seed(Lk + block)
+    B, H, Lq = 1, 4, 3
+    row = (torch.arange(Lk) % block == block - 1).view(1, Lk).expand(B, Lk)
+    mask, is_mem, last = P.prepare_landmark_masks(row, torch.ones(Lq, Lk, dtype=torch.bool).triu(Lk - Lq - 200))
+    x = (torch.randn(B, H, Lq, Lk, generator=g) * 3).to(dtype)
+    x = x.masked_fill(mask, float("-inf") if guards else torch.finfo(dtype).min)
+    gp = torch.randn(B, H, Lq, Lk, generator=g)
+    xo = x.float().requires_grad_(True)
+    exp = O.grouped_softmax(xo, is_mem, last, attn_mask=mask if guards else None, guards=guards)
+    (gx_exp,) = torch.autograd.grad(exp, [xo], gp)
+    xd, n = x.to(DEV).requires_grad_(True), Lk // block + 3
+    if guards:
+        got, group = P.landmark_grouped_softmax_lm(xd, -1, is_mem.to(DEV), mask.to(DEV), last.to(DEV), True, n)
+        _, group_exp = O.grouped_softmax(xo, is_mem, last, attn_mask=mask, guards=True, return_group_prob=True, max_mem_cnt=n)
+        assert (group.cpu() - group_exp.detach()).abs().max().item() < 2e-6
+    else:
+        got = P.landmark_grouped_softmax(xd, -1, is_mem.to(DEV), last.to(DEV))
+    assert (got.detach().cpu() - exp.detach()).abs().max().item() < 2e-6
+    (gx,) = torch.autograd.grad(got, [xd], gp.to(DEV))
+    assert (gx.float().cpu() - gx_exp).abs().max().item() < _grad_tol(dtype)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
