@@ -834,9 +834,10 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsP
 
 // ---------------------------------------------------------------------------------------------------------------
 // Rows of up to about 2048 keys with at most two landmarks in 1/32 of the row: lane l owns the 4 n4 contiguous keys
-// from l * 4 n4 on (n4 = ceil(keys / 128)), in shared memory through all passes.  A group is then the tail of one lane, whole lanes behind it and the head of the lane that holds its
-// landmark: one segmented scan over the lanes per pass reduces every group of the row, and two shuffles hand each lane
-// the results of the (at most two) groups its keys lie in; where lanes hold two landmarks, the keys between them are a third one.  Nothing per group is kept in memory and no pass looks
+// from l * 4 n4 on (n4 = ceil(keys / 128)), in shared memory through all passes.  A group is then the tail of one lane, whole
+// lanes behind it and the head of the lane that holds its landmark: one segmented scan over the lanes per pass reduces
+// every group of the row, and two shuffles hand each lane the results of the (at most two) groups its keys lie in; where lanes
+// hold two landmarks, the keys between them are a third one.  Nothing per group is kept in memory and no pass looks
 // anything up per key.  A row with three landmarks in a lane is done by the chunked form above.
 //
 // Bound by the instructions per row (two thirds of the issue slots at 40 % of the copy bandwidth), so what can be shared is:
