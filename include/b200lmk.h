@@ -67,7 +67,7 @@ void lmk_debug_set_max_ctas(int n);
 
 /* Compares n landmark flags (bytes; rows of `row` keys) with the regular pattern "last token of every block" and stores 1
  * to *irregular if any differs (the assertion of flash_landmark_attention.py:393-394 in one launch).  `irregular` is device-
- * accessible memory, e.g. mapped host memory, which the caller has set to 0.
+ * accessible memory, e.g. mapped host memory, which the caller has set to 0.  n = 0 is regular: nothing is read or launched.
  */
 int lmk_mask_is_regular(const uint8_t* mask, int64_t n, int row, int block, int* irregular, void* stream);
 

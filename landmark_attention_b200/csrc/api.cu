@@ -243,9 +243,10 @@ extern "C" int lmk_attn_bwd_static(const void* q, const void* k, const void* v, 
 }
 
 extern "C" int lmk_mask_is_regular(const uint8_t* mask, int64_t n, int row, int block, int* irregular, void* stream) {
+  LMK_CHECK_ARG(n >= 0 && block >= 1, "mask_is_regular: bad sizes");
+  if (n == 0) return LMK_OK;      // an empty mask has no irregular flag, and neither a row nor an address
   LMK_CHECK_ARG(mask && irregular, "mask_is_regular: null pointer");
-  LMK_CHECK_ARG(n >= 0 && row >= 1 && block >= 1, "mask_is_regular: bad sizes");
-  if (n == 0) return LMK_OK;
+  LMK_CHECK_ARG(row >= 1, "mask_is_regular: bad sizes");
   const int64_t ctas = (n + 255) / 256;
   mask_is_regular_kernel<<<(unsigned)(ctas < 296 ? ctas : 296), 256, 0, (cudaStream_t)stream>>>(mask, n, row, block, irregular);
   LMK_CUDA(cudaGetLastError());

@@ -180,7 +180,8 @@ class MemLMCacheStorage(nn.Module):
             self.last_incomplete_v[:B, :, :inc].copy_(v[:, :, full:])
             self.last_incomplete_ismem[:B, :inc].copy_(is_mem[:, full:])
         self.last_incomplete_len = inc
-        L.host().check_regular(is_mem[:, :full], blk)      # every block ends in its only landmark, or AssertionError
+        if full:
+            L.host().check_regular(is_mem[:, :full], blk)      # every block ends in its only landmark, or AssertionError
         added = full // blk
         dropped = max(0, added - cap)           # more blocks than the ring holds: only the newest `cap` are kept
         self.cache_iter = (self.cache_iter + dropped) % cap

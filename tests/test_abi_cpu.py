@@ -54,6 +54,15 @@ def test_attention_argument_checks_return_codes():
     assert lib.lmk_attn_bwd_workspace(1, 2, 64, 64, 64, 64, L.LMK_F32, L.PATH_GENERAL) == 2 * 64 * 4
 
 
+def test_an_empty_landmark_mask_is_regular():
+    # a chunk that completes no block: an empty slice has no address and rows of no flags
+    lib, one = P.lib(), ctypes.c_void_p(256)          # never dereferenced
+    assert lib.lmk_mask_is_regular(None, 0, 0, 8, one, None) == L.LMK_OK
+    assert lib.lmk_mask_is_regular(None, 0, 8, 0, one, None) == L.LMK_ERR_INVALID
+    assert lib.lmk_mask_is_regular(None, 8, 8, 8, one, None) == L.LMK_ERR_INVALID
+    assert lib.lmk_mask_is_regular(one, 8, 0, 8, one, None) == L.LMK_ERR_INVALID
+
+
 def test_retrieval_argument_checks():
     lib = P.lib()
     one = ctypes.c_void_p(256)

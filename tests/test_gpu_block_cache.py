@@ -48,3 +48,29 @@ def test_retrieval_and_prefix_attention_match_the_gathered_route(B, H, blk, cap,
         ye = P.lm_landmark_attention(q.clone().requires_grad_(True), k, v, im, att_prefix=exp, cache_values=ed)
     assert (y.float() - ye.float()).abs().max().item() < 3e-2
     assert ((y.float() - ye.float()).norm() / ye.float().norm()).item() < 5e-3
+
+
+@pytest.mark.parametrize("dtype,layout", [(torch.bfloat16, "reference"), (torch.float16, "head_major")])
+@pytest.mark.parametrize("chunks", [(3, 3, 1, 9, 20, 7), (1,) * 19, (8, 2, 3, 3, 5), (5,)])
+def test_chunks_below_a_block_are_stored_as_the_whole_is(chunks, dtype, layout):
+    B, H, blk, cap, n = 2, 3, 8, 4, sum(chunks)          # the longest wraps the ring
+    g = torch.Generator(device=DEV).manual_seed(n)
+    k, v = [torch.randn(B, H, n, 128, generator=g, device=DEV).to(dtype) for _ in range(2)]
+    im = (torch.arange(n, device=DEV) % blk == blk - 1).view(1, n).expand(B, n)
+    cfg = types.SimpleNamespace(batch_size=B, mem_cache_size=cap, mem_cache_freq=blk - 1, n_head=H, n_embd=H * 128,
+                                cache_topk=2, cache_selection_method="per_token_and_head")
+    one, many = [P.MemLMCacheStorage(cfg, None, dtype=dtype, device=DEV, layout=layout) for _ in range(2)]
+    for st in (one, many):
+        for buf in (st.cache_mem_k, st.cache_mem_v, st.cache_lm_k):
+            buf.zero_()
+    one.store_in_cache(k, {"v": v, "is_mem": im})
+    lo = 0
+    for c in chunks:
+        many.store_in_cache(k[:, :, lo:lo + c], {"v": v[:, :, lo:lo + c], "is_mem": im[:, lo:lo + c]})
+        lo += c
+    assert (many.last_incomplete_len, many.cache_iter, many.cache_size) == (one.last_incomplete_len, one.cache_iter, one.cache_size)
+    tail = n % blk
+    for a, b in ((many.cache_mem_k, one.cache_mem_k), (many.cache_mem_v, one.cache_mem_v), (many.cache_lm_k, one.cache_lm_k),
+                 (many.last_incomplete_k[:, :, :tail], k[:, :, n - tail:]), (many.last_incomplete_v[:, :, :tail], v[:, :, n - tail:]),
+                 (many.last_incomplete_ismem[:, :tail], im[:, n - tail:])):
+        assert torch.equal(a, b)
