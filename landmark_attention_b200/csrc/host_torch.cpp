@@ -471,12 +471,15 @@ Tensor vector_rows(const Tensor& t) {
 constexpr int64_t kDecodeMaxWholeBlockTokens = 16;
 
 // One layer of token generation behind `len` cached tokens (lmk_decode_attend): tokens that stay inside the unfinished
-// block; undefined where the kernel does not take them.
+// block; undefined where the kernel does not take them, and where a gradient is asked for behind an unfinished block: the tensor
+// formulation that runs there is differentiable through the unfinished block's keys and values and the new ones.  (Behind whole
+// blocks the other route has no gradient either.)
 Tensor decode_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& kc, const Tensor& vc, int64_t len,
                      bool append, int64_t block, int64_t top_k, const Tensor& cos, const Tensor& sin) {
   const auto st = q_.scalar_type();
   if (block < 2 || top_k < 1 || len < block) return Tensor();
   const int64_t tail = len % block;
+  if (tail && needs_grad({q_, k_, v_, kc, vc, cos, sin})) return Tensor();
   top_k = std::min(top_k, len / block);
   if (!q_.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || q_.dim() != 4 || kc.dim() != 4) return Tensor();
   const auto B = q_.size(0), H = q_.size(1), T = q_.size(2), D = q_.size(3);

@@ -281,6 +281,8 @@ def llama_retrieval_attention(q, k_new, v_new, past_k=None, past_v=None, mem_fre
         merges the two parts -- no logits, probabilities or gathered copies in memory;
       materialize=False: selected-block logits / value sums read in place, grouped softmax on a logits buffer;
       materialize=True (what the reference does, :386-398): gathered [B,H,T,top_k*block,D] copies and matmuls.
+    Gradients of q, k_new and v_new: whole with aggregate="max_over_tokens" and with materialize=True; behind an unfinished block the
+    default route passes on the part through the local keys and values, and behind whole blocks none.
     Returns (attn_output [B,H,T,D], new (past_k, past_v)).
     """
     if (fused is None and materialize is None and not return_debug and position_ids is None and chunk_is_mem is None

@@ -59,3 +59,36 @@ def test_per_head_selection_is_differentiable(T, blk, N, top_k, dtype):
     with torch.no_grad():
         out, _ = call(leaves(q, k, v), past_k=pk, past_v=pv)
         assert not out.requires_grad and close(out, exp)
+
+
+@DTYPES
+@pytest.mark.parametrize("T,blk,N,tail,top_k", [(1, 32, 9, 17, 4), (3, 64, 5, 50, 2)])
+def test_tokens_inside_an_unfinished_block_are_differentiable(T, blk, N, tail, top_k, dtype):
+    C = N * blk + tail
+    (pk, pv, q, k, v), do = problem(1, 2, T, C, dtype, C)
+    cos, sin = P.rotary_tables_half(C + T + 1, 128, dtype, DEV)
+    call = lambda a, **kw: P.llama_retrieval_attention(*a, mem_freq=blk - 1, cache_top_k=top_k, cos=cos, sin=sin, **kw)
+    a = leaves(q, k, v, pk, pv)
+    exp, _ = call(a[:3], past_k=a[3], past_v=a[4], materialize=False)
+    grads = torch.autograd.grad(exp, a, do)
+    # the values' gradients (new ones, and the cached ones of the unfinished block) against the oracle, with this call's selection
+    _, _, dbg = call((q, k, v), past_k=pk, past_v=pv, return_debug=True)
+    o = [t.float().cpu().requires_grad_(True) for t in (q, k, v, pk, pv)]
+    want = torch.autograd.grad(O.llama_retrieval_attention(*o, blk, top_k, sel=dbg["sel"].long().cpu()), o, do.float().cpu())
+    assert close(grads[2], want[2]) and close(grads[4][:, :, N * blk:], want[4][:, :, N * blk:])
+
+    for wanted in ((0, 1, 2, 3, 4), (1,), (4,)):                 # also a gradient of one input alone
+        a = [t.clone().requires_grad_(i in wanted) for i, t in enumerate((q, k, v, pk, pv))]
+        out, _ = call(a[:3], past_k=a[3], past_v=a[4])
+        assert out.requires_grad and torch.equal(out, exp)
+        for i, got in zip(wanted, torch.autograd.grad(out, [a[i] for i in wanted], do)):
+            assert torch.equal(got, grads[i])
+    cache = P.LandmarkKVCache(1, 2, C + T, 128, dtype, DEV)
+    cache.append(pk, pv)
+    a = leaves(q, k, v)
+    out, _ = call(a, cache=cache)
+    for got, want in zip(torch.autograd.grad(out, a, do), grads):
+        assert torch.equal(got, want)
+    with torch.no_grad():
+        out, _ = call(leaves(q, k, v), past_k=pk, past_v=pv)
+        assert not out.requires_grad and close(out, exp)
