@@ -16,6 +16,7 @@
 #include <optional>
 #include <string>
 #include <tuple>
+#include <vector>
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -175,8 +176,62 @@ Tensor fused_attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, int
 }
 
 // ------------------------------------------------------------------------------------------------ landmark mask check
-// One kernel compares every flag with the regular pattern and writes a word of mapped host memory; the host waits for
-// that kernel alone (an event), so what the caller enqueues between the constructor and failed() overlaps with it.
+// A word of mapped host memory that one kernel may write, and the event behind that kernel.  Words are handed from check to check
+// through a list of idle ones (16 bytes of pinned memory each, as many as there were checks at one time): a word is idle again once
+// its kernel has finished, whether or not anybody asked for the result.
+class FlagWord {
+ public:
+  explicit FlagWord(int dev) : idle_(idle_of(dev)) {
+    const std::lock_guard<std::mutex> lock(idle_.mutex);
+    if (idle_.words.empty()) {
+      C10_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&w_.word), 16, cudaHostAllocMapped | cudaHostAllocPortable));
+      C10_CUDA_CHECK(cudaEventCreateWithFlags(&w_.event, cudaEventDisableTiming));
+    } else {
+      w_ = idle_.words.back();
+      idle_.words.pop_back();
+    }
+    *w_.word = 0;
+  }
+  ~FlagWord() {
+    // a check that was given up (an exception between its launch and its result): the kernel may still be queued
+    if (queued_ && (!recorded_ || cudaEventSynchronize(w_.event) != cudaSuccess)) {
+      (void)cudaGetLastError();
+      return;                          // the kernel may still write it: no other check gets this word
+    }
+    const std::lock_guard<std::mutex> lock(idle_.mutex);
+    idle_.words.push_back(w_);
+  }
+  FlagWord(const FlagWord&) = delete;
+  FlagWord& operator=(const FlagWord&) = delete;
+
+  int* word() const { return w_.word; }
+  void launched(cudaStream_t stream) {             // behind the launch of the kernel that writes the word
+    queued_ = true;
+    C10_CUDA_CHECK(cudaEventRecord(w_.event, stream));
+    recorded_ = true;
+  }
+  int wait() {
+    if (queued_) C10_CUDA_CHECK(cudaEventSynchronize(w_.event));
+    queued_ = false;
+    return *static_cast<volatile int*>(w_.word);
+  }
+
+ private:
+  struct Word { int* word = nullptr; cudaEvent_t event = nullptr; };
+  struct Idle { std::mutex mutex; std::vector<Word> words; };
+  static Idle& idle_of(int dev) {
+    constexpr int kMax = 64;
+    static Idle* idle = new Idle[kMax];            // not destroyed: a thread may end after the program's statics
+    TORCH_CHECK(dev >= 0 && dev < kMax, "device index out of range");
+    return idle[dev];
+  }
+  Idle& idle_;
+  Word w_;
+  bool queued_ = false, recorded_ = false;
+};
+
+// One kernel compares every flag with the regular pattern and writes its word; the host waits for that kernel alone, so what
+// the caller enqueues between the constructor and failed() overlaps with it.
 class RegularCheck {
  public:
   RegularCheck(const Tensor& is_mem, int64_t block) {
@@ -186,34 +241,17 @@ class RegularCheck {
       host_failed_ = !m.eq(want).all().item<bool>();
       return;
     }
+    c10::cuda::OptionalCUDAGuard guard(m.device());
     if (m.element_size() != 1) m = m.eq(1).to(at::kByte).add_(m.ne(0).logical_and_(m.ne(1)), 2);     // 2: neither
-    slot_ = &local_slot(m.get_device());
-    *slot_->word = 0;
-    check(lib.lmk_mask_is_regular((const uint8_t*)m.data_ptr(), m.numel(), m.size(-1), block, slot_->word, stream_of(m)),
+    flag_.emplace(m.get_device());
+    check(lib.lmk_mask_is_regular((const uint8_t*)m.data_ptr(), m.numel(), m.size(-1), block, flag_->word(), stream_of(m)),
           "lmk_mask_is_regular");
-    C10_CUDA_CHECK(cudaEventRecord(slot_->event, (cudaStream_t)stream_of(m)));
+    flag_->launched((cudaStream_t)stream_of(m));
   }
-  bool failed() const {
-    if (slot_ == nullptr) return host_failed_;
-    C10_CUDA_CHECK(cudaEventSynchronize(slot_->event));
-    return *reinterpret_cast<volatile int*>(slot_->word) != 0;
-  }
+  bool failed() { return flag_ ? flag_->wait() != 0 : host_failed_; }
 
  private:
-  struct Slot { int* word = nullptr; cudaEvent_t event = nullptr; };
-  // one word and one event per thread and device, for the life of the program (16 bytes of pinned memory each)
-  static Slot& local_slot(int dev) {
-    constexpr int kMax = 64;
-    static thread_local Slot slots[kMax];
-    TORCH_CHECK(dev >= 0 && dev < kMax, "device index out of range");
-    Slot& s = slots[dev];
-    if (s.word == nullptr) {
-      C10_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&s.word), 16, cudaHostAllocMapped | cudaHostAllocPortable));
-      C10_CUDA_CHECK(cudaEventCreateWithFlags(&s.event, cudaEventDisableTiming));
-    }
-    return s;
-  }
-  Slot* slot_ = nullptr;
+  std::optional<FlagWord> flag_;
   bool host_failed_ = false;
 };
 
