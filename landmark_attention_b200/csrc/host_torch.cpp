@@ -558,7 +558,8 @@ lmk_cache_desc block_desc(const Tensor& t, bool block_before_head, int64_t n, in
 }
 
 // MemLMCacheStorage.retrieve_for_query with blocks in the cache (mem_cache.py:51-109): (att_prefix [B,H,T,P], values
-// [B,H,T,P,D]); undefined where the kernels do not take the problem.  kc, vc: the block buffers in either layout; lm: dense
+// [B,H,T,P,D]); undefined where the kernels do not take the problem or a gradient is asked for (of the queries, or of the unfinished
+// block, whose rows belong to the graph of the chunk that stored them).  kc, vc: the block buffers in either layout; lm: dense
 // landmark keys [B,H,capacity,D]; tail_k, tail_v [B,H,>=inc,D].  mode: 0 per token and head, 1 maximum over the
 // tokens, 2 over the heads.
 std::tuple<Tensor, Tensor> cache_retrieve(const Tensor& q_, const Tensor& kc, const Tensor& vc, const Tensor& lm, bool block_first,
@@ -568,6 +569,7 @@ std::tuple<Tensor, Tensor> cache_retrieve(const Tensor& q_, const Tensor& kc, co
   const auto st = q_.scalar_type();
   const auto B = q_.size(0), H = q_.size(1), T = q_.size(2), D = q_.size(3);
   if (!q_.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || B * H > 65535) return {};
+  if (needs_grad({q_}) || (inc && needs_grad({tail_k, tail_v}))) return {};
   for (const Tensor* t : {&kc, &vc, &lm, &cos, &sin, &tail_k, &tail_v})
     if (!t->is_cuda() || t->scalar_type() != st || t->stride(-1) != 1 || (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15)) return {};
   const int code = dtype_code(q_);

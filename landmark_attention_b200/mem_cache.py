@@ -146,7 +146,7 @@ class MemLMCacheStorage(nn.Module):
         B, nh, T, hs = q.shape
         blk, cap = self.block, self.capacity
         mode = self._MODES.get(self.config.cache_selection_method)
-        if self.cache_size == 0 or self.config.cache_topk == 0 or mode is None or hs != 128 or torch.is_grad_enabled() and q.requires_grad:
+        if self.cache_size == 0 or self.config.cache_topk == 0 or mode is None or hs != 128:
             return None
         n = min(self.cache_size, cap)
         top_k = min(self.config.cache_topk, n)

@@ -1,6 +1,8 @@
 """Gradients of the retrieval entry points: where the tensor formulation of a call is differentiable, a call that wants gradients takes
 that formulation, and gets its gradients; without gradients the native call runs."""
 
+import types
+
 import pytest
 import torch
 
@@ -92,3 +94,40 @@ def test_tokens_inside_an_unfinished_block_are_differentiable(T, blk, N, tail, t
     with torch.no_grad():
         out, _ = call(leaves(q, k, v), past_k=pk, past_v=pv)
         assert not out.requires_grad and close(out, exp)
+
+
+@DTYPES
+@pytest.mark.parametrize("wanted", [("q",), ("k",), ("v",), ("q", "k", "v")])
+def test_block_cache_retrieval_is_differentiable(wanted, dtype):
+    # the queries, and what an earlier chunk left in the unfinished block
+    B, H, blk, T, tail = 1, 2, 16, 5, 7
+    n = 4 * blk + tail
+    (k, v, q, _, _), _ = problem(B, H, T, n, dtype, len(wanted))
+    cfg = types.SimpleNamespace(batch_size=B, mem_cache_size=8, mem_cache_freq=blk - 1, n_head=H, n_embd=H * 128,
+                                cache_topk=2, cache_selection_method="per_token_and_head")
+    im = (torch.arange(n, device=DEV) % blk == blk - 1).view(1, n).expand(B, n)
+    x = {name: t.clone().requires_grad_(name in wanted) for name, t in (("q", q), ("k", k), ("v", v))}
+    st = P.MemLMCacheStorage(cfg, None, dtype=dtype, device=DEV)
+    st.store_in_cache(x["k"], {"v": x["v"], "is_mem": im})
+    att, d = st.retrieve_for_query(x["q"], None, None, 3 * blk + tail)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    da, dv = [torch.randn(t.shape, generator=g, device=DEV).to(dtype) for t in (att, d["v"])]
+    outs = [(att, da)] * att.requires_grad + [(d["v"], dv)] * d["v"].requires_grad
+    grads = dict(zip(wanted, torch.autograd.grad([o for o, _ in outs], [x[w] for w in wanted], [go for _, go in outs])))
+    # the tail's logits are q . rotated key / sqrt(D), its values are handed on once per token
+    pos = torch.arange(3 * blk, 3 * blk + tail)
+    qf, kt = [t.detach().float().cpu().requires_grad_(True) for t in (x["q"], x["k"][:, :, n - tail:])]
+    logits = qf @ O.rotary_interleaved(kt, pos.view(1, 1, tail).expand(B, H, tail).float()).transpose(2, 3) / 128 ** 0.5
+    want_q, want_k = torch.autograd.grad(logits, [qf, kt], da[..., 2 * blk:].float().cpu(), retain_graph=True)
+    if "k" in wanted:
+        assert close(grads["k"][:, :, n - tail:], want_k) and not grads["k"][:, :, :n - tail].any()
+    if "v" in wanted:
+        assert close(grads["v"][:, :, n - tail:], dv[:, :, :, 2 * blk:].float().sum(2)) and not grads["v"][:, :, :n - tail].any()
+    if wanted == ("q",):
+        # the gathered blocks' part comes on top of the tail's
+        zero = torch.cat((torch.zeros_like(da[..., :2 * blk]), da[..., 2 * blk:]), -1)
+        att, _ = st.retrieve_for_query(x["q"], None, None, 3 * blk + tail)
+        assert close(torch.autograd.grad(att, x["q"], zero)[0], want_q)
+    with torch.no_grad():
+        fast, fd = st.retrieve_for_query(x["q"], None, None, 3 * blk + tail)
+        assert not fast.requires_grad and close(fast, att.detach()) and torch.equal(fd["v"], d["v"].detach())
