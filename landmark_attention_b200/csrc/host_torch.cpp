@@ -103,9 +103,12 @@ Tensor grad_rows(const Tensor& g, const Tensor& q) {
                   t.stride(2) % vec == 0 && t.stride(2) >= D && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
   return ok ? t : t.clone(at::MemoryFormat::Contiguous);
 }
+// Whether a derivative through the call is asked for: backward, or forward (a tangent; the autograd nodes here refuse those, which
+// the raw kernel calls would drop).
 bool needs_grad(std::initializer_list<std::reference_wrapper<const Tensor>> ts) {
-  if (!at::GradMode::is_enabled()) return false;
-  for (const Tensor& t : ts) if (t.requires_grad()) return true;
+  const bool backward = at::GradMode::is_enabled(), forward = c10::AutogradState::get_tls_state().get_fw_grad_mode();
+  for (const Tensor& t : ts)
+    if ((backward && t.requires_grad()) || (forward && t._fw_grad(0).defined())) return true;
   return false;
 }
 
@@ -629,11 +632,11 @@ std::tuple<Tensor, Tensor> cache_retrieve(const Tensor& q_, const Tensor& kc, co
   return {att, v};
 }
 
-// y += probs[..., :P] @ v per token (lmk_prefix_pv); false where the kernel does not take the tensors
+// y += probs[..., :P] @ v per token (lmk_prefix_pv); false where the kernel does not take the tensors or a gradient of them is asked for
 bool prefix_pv(const Tensor& probs, const Tensor& v, const Tensor& y) {
   const auto st = v.scalar_type();
   const auto B = y.size(0), H = y.size(1), T = y.size(2), D = y.size(3), P = v.size(3);
-  if (!v.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || y.scalar_type() != st || D != 128 || P > 8192 || B * H > 65535 ||
+  if (needs_grad({probs, v}) || !v.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || y.scalar_type() != st || D != 128 || P > 8192 || B * H > 65535 ||
       P == 0 || !probs.is_contiguous() || !y.is_contiguous() || v.stride(4) != 1 || v.stride(3) != D || v.stride(0) % 8 ||
       v.stride(1) % 8 || v.stride(2) % 8 || (reinterpret_cast<uintptr_t>(v.data_ptr()) & 15))
     return false;
