@@ -746,6 +746,29 @@ Fork fork_of(int dev) {
   return {c10::cuda::getStreamFromPool(false, dev), events[dev][0], events[dev][1]};
 }
 
+// Makes `main` wait for what a call put on its side stream, also where the call ends in an exception: its tensors are given back to
+// main's allocator, and its destination may be written again by what main does next.
+class Join {
+ public:
+  Join(const Fork& fork, cudaStream_t main) : fork_(fork), main_(main) {}
+  ~Join() {
+    if (done_) return;
+    (void)cudaEventRecord(fork_.end, fork_.side.stream());
+    (void)cudaStreamWaitEvent(main_, fork_.end, 0);
+  }
+  Join(const Join&) = delete;
+  Join& operator=(const Join&) = delete;
+  void now() {                        // with `end` recorded behind the last thing that matters
+    C10_CUDA_CHECK(cudaStreamWaitEvent(main_, fork_.end, 0));
+    done_ = true;
+  }
+
+ private:
+  const Fork fork_;
+  const cudaStream_t main_;
+  bool done_ = false;
+};
+
 // One selection per (head, token); `len` whole-block tokens in the caches; append: k, v stored behind them.
 Tensor chunk_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& kc, const Tensor& vc, int64_t len, bool append,
                     int64_t block, int64_t top_k, const Tensor& cos, const Tensor& sin, int64_t rotary) {
@@ -807,11 +830,13 @@ Tensor per_head_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, con
     ld.stride_row = 0;
   }
   std::optional<Fork> fork;
+  std::optional<Join> join;
   if (host && append) {
     // by the copy engine: the same stores from a kernel fill the memory system's queues towards the host link and slow down
     // everything that runs beside them (the rotary kernel 4 -> 35 us)
     c.k = c.k.contiguous(), c.v = c.v.contiguous();
     fork = fork_of(q_.get_device());
+    join.emplace(*fork, (cudaStream_t)c.stream);
     C10_CUDA_CHECK(cudaEventRecord(fork->begin, (cudaStream_t)c.stream));
     C10_CUDA_CHECK(cudaStreamWaitEvent(fork->side.stream(), fork->begin, 0));
     const size_t width = (size_t)c.T * c.D * 2, pitch = (size_t)kc.stride(1) * 2, at = (size_t)n * block * c.D * 2;
@@ -839,7 +864,7 @@ Tensor per_head_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, con
                              keys.data_ptr(), vals.data_ptr(), W * c.D, c.B, c.H, 1, c.D, c.code, c.stream), "lmk_gather_kv");
   Tensor stats;
   Tensor out = attn_fwd(qr, keys, vals, c.scale, block, LMK_PATH_AUTO, &stats);
-  if (fork) C10_CUDA_CHECK(cudaStreamWaitEvent((cudaStream_t)c.stream, fork->end, 0));
+  if (join) join->now();
   return out;
 }
 

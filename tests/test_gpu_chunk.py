@@ -70,3 +70,25 @@ def test_ragged_chunk_against_the_host_cache_waits_in_the_tail():
     assert (off.n_blocks, off.tail_len) == (11, 36) and torch.equal(off.tail_k[:, :, :36], k[:, :, 64:])
     with pytest.raises(AssertionError):
         off.attend(q, k, v, 2, cos, sin)
+
+
+def test_a_chunk_refused_after_its_stores_began_leaves_nothing_in_flight():
+    # blocks of one key are refused by the attention, which comes behind the copies to the host cache: what the current stream does next
+    # must come behind them too
+    T, H = 2048, 32
+    k, v = [torch.randn(1, H, T, 128, device=DEV).to(torch.bfloat16) for _ in range(2)]
+    off = P.OffloadedLandmarkCache(1, H, T + 8, 1, 128, torch.bfloat16, DEV)
+    off.append(k[:, :, :8], v[:, :, :8])
+    cos, sin = P.rotary_tables_half(T + 9, 128, torch.bfloat16, DEV)
+    want = [t.cpu() for t in (k, v)]
+    for _ in range(2):                                # the first call loads the kernels
+        torch.cuda.synchronize()
+        off.v_host[:, :, 8:].zero_()
+        torch.cuda._sleep(20_000_000)                 # about 10 ms: the copies begin behind it, long after the call has returned
+        with pytest.raises(AssertionError):
+            off.attend(k, k, v, 1, cos, sin)
+    assert off.n_blocks == 8
+    torch.cuda.current_stream().synchronize()
+    last = off.v_host[0, H - 1, -1].clone()       # the last row to arrive, read before anything that takes time
+    assert torch.equal(last, want[1][0, H - 1, -1])
+    assert torch.equal(off.k_host[:, :, 8:], want[0]) and torch.equal(off.v_host[:, :, 8:], want[1])
