@@ -150,8 +150,11 @@ _SYMMETRIC = {}       # (id(cos), id(sin)) -> (weakref to cos, weakref to sin, v
 def _halves_equal(cos, sin, check=True):
     """Whether cos[p, d] == cos[p, d + D/2] and the same for sin (tables built as cat(freqs, freqs), as LLaMA's rotary
     embedding does).  One device comparison per pair of table tensors, remembered while those tensor objects live and
-    are not written to; check=False only looks the verdict up (None if unknown)."""
+    are not written to; check=False only looks the verdict up (None if unknown).  Tables made in inference mode do not count their
+    writes, so nothing can be remembered about them: they go to the kernels' general form."""
     import weakref
+    if cos.is_inference() or sin.is_inference():
+        return None
     key = (id(cos), id(sin))
     hit = _SYMMETRIC.get(key)
     if hit is not None and hit[0]() is cos and hit[1]() is sin and hit[2] == (cos._version, sin._version):

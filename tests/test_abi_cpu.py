@@ -126,3 +126,13 @@ def test_rotary_tables_match_oracle():
     from landmark_attention_b200.mem_cache import _rotate_interleaved
     ref = O.rotary_interleaved(x, pos.view(1, 1, 5).expand(2, 3, 5).to(torch.float32))
     assert torch.allclose(_rotate_interleaved(x, cos, sin, pos), ref, atol=1e-6)
+
+
+def test_verdicts_about_rotary_tables():
+    from landmark_attention_b200.retrieval import _halves_equal
+    cos, sin = P.rotary_tables_half(8, 16, torch.float32, "cpu")
+    assert _halves_equal(cos, sin, check=False) is None and _halves_equal(cos, sin) and _halves_equal(cos, sin, check=False)
+    cos[3, 2] += 1                                           # a write makes the verdict void
+    assert _halves_equal(cos, sin, check=False) is None and not _halves_equal(cos, sin)
+    with torch.inference_mode():                             # tensors without a version counter
+        assert _halves_equal(*P.rotary_tables_half(8, 16, torch.float32, "cpu")) is None
