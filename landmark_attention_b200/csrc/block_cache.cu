@@ -23,31 +23,6 @@ constexpr int kPad = 160;                 // 16-bit elements of a shared row: th
 constexpr int kSelMaxN = 128;
 constexpr int kGatherMaxBlk = 128;
 
-template <typename T> struct P2;          // two 16-bit values in one register, rounded like the tensor formulation
-template <> struct P2<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-};
-template <> struct P2<__half> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-};
 // one 16-byte vector of the low half (features d0..d0+7) and its partner of the high half, rotated at table row `pos`
 template <typename T>
 __device__ __forceinline__ void rotate_pair(uint4& lo, uint4& hi, const T* cos_t, const T* sin_t, int64_t po, int rotary) {
@@ -67,8 +42,8 @@ __device__ __forceinline__ void rotate_pair(uint4& lo, uint4& hi, const T* cos_t
       pl = __byte_perm(l[u], l[u], 0x1032) ^ 0x00008000u;
       ph = __byte_perm(h[u], h[u], 0x1032) ^ 0x00008000u;
     }
-    const uint32_t a = P2<T>::add(P2<T>::mul(l[u], c0[u]), P2<T>::mul(pl, s0[u]));
-    h[u] = P2<T>::add(P2<T>::mul(h[u], c1[u]), P2<T>::mul(ph, s1[u]));
+    const uint32_t a = Pair16<T>::add(Pair16<T>::mul(l[u], c0[u]), Pair16<T>::mul(pl, s0[u]));
+    h[u] = Pair16<T>::add(Pair16<T>::mul(h[u], c1[u]), Pair16<T>::mul(ph, s1[u]));
     l[u] = a;
   }
 }

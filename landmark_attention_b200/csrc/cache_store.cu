@@ -11,36 +11,11 @@
 // the append of the un-rotated keys / values to a preallocated cache (:424-425) -- one launch instead of the
 // index / multiply / concatenate / copy kernels of the tensor-library formulation.
 #include "common.cuh"
+#include "mma16.cuh"
 #include "sm100_ptx.cuh"
 
 namespace lmk {
 namespace {
-
-template <typename T> struct Pair16;      // arithmetic on two 16-bit values held in one 32-bit register
-template <> struct Pair16<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-};
-template <> struct Pair16<__half> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-};
 
 // x * cos + rotate_half(x) * sin on one 16-byte vector of the low half (lo) and its partner of the high half (hi),
 // with the three roundings of the tensor formulation (two products, one sum).
@@ -152,7 +127,6 @@ __global__ void __launch_bounds__(128) cache_store_kernel(const uint4* __restric
     if (lm_dst != nullptr && r == blk - 1) lm_dst[b * lm_b + h * lm_h + (int64_t)slot * lm_block + c] = kv;
   }
 }
-
 
 // Rotary position embedding of a [B,H,T,D] tensor pair (queries and keys of one layer) in one launch, both rotary
 // flavours, forward or inverse (the inverse rotation is the gradient of the forward one).  16-bit types use packed

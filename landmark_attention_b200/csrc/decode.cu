@@ -19,6 +19,7 @@
 #include <cooperative_groups.h>
 #include <type_traits>
 #include "common.cuh"
+#include "mma16.cuh"
 #include "sm100_ptx.cuh"
 
 namespace lmk {
@@ -47,36 +48,6 @@ struct DecParams {
   float scale;
 };
 
-template <typename T> struct Px2;         // two 16-bit values in one register, rounded like the tensor formulation
-template <> struct Px2<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ float2 f(uint32_t w) {
-    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-  }
-};
-template <> struct Px2<__half> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ float2 f(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
-};
-
 struct V4 { uint32_t w[4]; };
 __device__ __forceinline__ V4 ldv(const void* p) {
   const uint4 v = *reinterpret_cast<const uint4*>(p);
@@ -90,8 +61,8 @@ __device__ __forceinline__ void rotate(V4& lo, V4& hi, const V4& cl, const V4& c
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const uint32_t l = lo.w[u], h = hi.w[u];
-    lo.w[u] = Px2<T>::add(Px2<T>::mul(l, cl.w[u]), Px2<T>::mul(h ^ 0x80008000u, sl.w[u]));
-    hi.w[u] = Px2<T>::add(Px2<T>::mul(h, ch.w[u]), Px2<T>::mul(l, sh.w[u]));
+    lo.w[u] = Pair16<T>::add(Pair16<T>::mul(l, cl.w[u]), Pair16<T>::mul(h ^ 0x80008000u, sl.w[u]));
+    hi.w[u] = Pair16<T>::add(Pair16<T>::mul(h, ch.w[u]), Pair16<T>::mul(l, sh.w[u]));
   }
 }
 template <typename T>
@@ -99,7 +70,7 @@ __device__ __forceinline__ float dot_pair(const float (&q)[16], const V4& lo, co
   float a = 0.f, b = 0.f;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const float2 x = Px2<T>::f(lo.w[u]), y = Px2<T>::f(hi.w[u]);
+    const float2 x = Pair16<T>::f32(lo.w[u]), y = Pair16<T>::f32(hi.w[u]);
     a = fmaf(q[2 * u], x.x, a);
     b = fmaf(q[2 * u + 1], x.y, b);
     a = fmaf(q[8 + 2 * u], y.x, a);
@@ -199,7 +170,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDecWarps * 32) dec
     rotate<T>(ql, qh, ldv(cos_t + po), ldv(cos_t + po + kDecHalf), ldv(sin_t + po), ldv(sin_t + po + kDecHalf));
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const float2 x = Px2<T>::f(ql.w[u]), y = Px2<T>::f(qh.w[u]);
+      const float2 x = Pair16<T>::f32(ql.w[u]), y = Pair16<T>::f32(qh.w[u]);
       q[2 * u] = x.x;
       q[2 * u + 1] = x.y;
       q[8 + 2 * u] = y.x;
@@ -369,7 +340,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDecWarps * 32) dec
       const float pr = __shfl_sync(0xffffffffu, lg[s >> 1], 8 * (2 * (s & 1) + (lane >> 4)));
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const float2 x = Px2<T>::f(vv[s].w[u]);
+        const float2 x = Pair16<T>::f32(vv[s].w[u]);
         o[2 * u] = fmaf(pr, x.x, o[2 * u]);
         o[2 * u + 1] = fmaf(pr, x.y, o[2 * u + 1]);
       }

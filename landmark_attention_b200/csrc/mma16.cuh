@@ -1,4 +1,5 @@
-// mma.sync m16n8k16 on 16-bit types, for contractions too small or too irregular for tcgen05 tiles.
+// 16-bit types two to a register: arithmetic with the roundings of the tensor formulation, and mma.sync m16n8k16 for contractions too
+// small or too irregular for tcgen05 tiles.
 #pragma once
 #include <type_traits>
 #include "common.cuh"
@@ -8,6 +9,38 @@ namespace {
 
 template <typename T>
 __device__ __forceinline__ float rnd(float x) { return to_f32(from_f32<T>(x)); }
+
+// Two 16-bit values in one 32-bit register; every product and every sum is rounded to the type.
+template <typename T> struct Pair16;
+template <> struct Pair16<__nv_bfloat16> {
+  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  }
+  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  }
+  static __device__ __forceinline__ float2 f32(uint32_t w) {
+    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  }
+};
+template <> struct Pair16<__half> {
+  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  }
+  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  }
+  static __device__ __forceinline__ float2 f32(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+};
+template <> struct Pair16<float> {};      // named by kernels whose 16-bit branch is not compiled for fp32
 
 // D += A B, m16n8k16.  A thread (g = lane / 4, t = lane % 4) holds the 16-byte vectors [32 c + 8 t, +8) of rows g and g + 8 of A
 // and of row g of B^T; registers (0, 1) and (2, 3) of a vector serve as two k-steps.  A dot product does not depend on the

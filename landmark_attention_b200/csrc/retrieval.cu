@@ -5,6 +5,7 @@
 // "slot" positions: the newest top_k blocks occupy slots 1..top_k, every older block shares slot 0.
 #include <type_traits>
 #include "common.cuh"
+#include "mma16.cuh"
 #include "sm100_ptx.cuh"
 #include "scores_sm100.h"
 
@@ -499,40 +500,7 @@ __device__ __forceinline__ void load_vec_f32(const T* p, float (&o)[VEC]) {
 constexpr int kSelMinBlocks = 8;
 constexpr int kSelUnroll = 1;
 constexpr int kPvUnroll = 4;
-template <typename T> struct Packed;      // arithmetic on two 16-bit values held in one 32-bit register
-template <> struct Packed<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ void to_f32(uint32_t w, float& lo, float& hi) {
-    lo = __uint_as_float(w << 16);
-    hi = __uint_as_float(w & 0xffff0000u);
-  }
-};
-template <> struct Packed<__half> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ void to_f32(uint32_t w, float& lo, float& hi) {
-    asm("{\n\t.reg .f16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.f32.f16 %0, l;\n\tcvt.f32.f16 %1, h;\n\t}"
-        : "=f"(lo), "=f"(hi) : "r"(w));
-  }
-};
-template <> struct Packed<float> {};
+
 __device__ __forceinline__ void ld16(const void* p, uint32_t (&w)[4]) {
   const uint4 v = *reinterpret_cast<const uint4*>(p);
   w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
@@ -570,19 +538,17 @@ __device__ __forceinline__ float rotated_row_dot(const T* krow, const T* cr, con
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          xl[u] = Packed<T>::add(Packed<T>::mul(xl[u], cl[u]), Packed<T>::mul(pl[u], sl[u]));
-          xh[u] = Packed<T>::add(Packed<T>::mul(xh[u], ch[u]), Packed<T>::mul(ph[u], sh[u]));
+          xl[u] = Pair16<T>::add(Pair16<T>::mul(xl[u], cl[u]), Pair16<T>::mul(pl[u], sl[u]));
+          xh[u] = Pair16<T>::add(Pair16<T>::mul(xh[u], ch[u]), Pair16<T>::mul(ph[u], sh[u]));
         }
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        float f0, f1, g0, g1;
-        Packed<T>::to_f32(xl[u], f0, f1);
-        Packed<T>::to_f32(xh[u], g0, g1);
-        acc0 = fmaf(q0[2 * u], f0, acc0);
-        acc1 = fmaf(q0[2 * u + 1], f1, acc1);
-        acc0 = fmaf(q1[2 * u], g0, acc0);
-        acc1 = fmaf(q1[2 * u + 1], g1, acc1);
+        const float2 f = Pair16<T>::f32(xl[u]), g = Pair16<T>::f32(xh[u]);
+        acc0 = fmaf(q0[2 * u], f.x, acc0);
+        acc1 = fmaf(q0[2 * u + 1], f.y, acc1);
+        acc0 = fmaf(q1[2 * u], g.x, acc0);
+        acc1 = fmaf(q1[2 * u + 1], g.y, acc1);
       }
     } else {
       float xl[VEC], xh[VEC];
@@ -823,8 +789,8 @@ __global__ void __launch_bounds__(128, 8) selected_attend_kernel(const T* __rest
                   pl = __byte_perm(x[0][u], x[0][u], 0x1032) ^ 0x00008000u;
                   ph = __byte_perm(x[1][u], x[1][u], 0x1032) ^ 0x00008000u;
                 }
-                const uint32_t lo = Packed<T>::add(Packed<T>::mul(x[0][u], cl[u]), Packed<T>::mul(pl, sl[u]));
-                const uint32_t hi = Packed<T>::add(Packed<T>::mul(x[1][u], ch[u]), Packed<T>::mul(ph, sh[u]));
+                const uint32_t lo = Pair16<T>::add(Pair16<T>::mul(x[0][u], cl[u]), Pair16<T>::mul(pl, sl[u]));
+                const uint32_t hi = Pair16<T>::add(Pair16<T>::mul(x[1][u], ch[u]), Pair16<T>::mul(ph, sh[u]));
                 x[0][u] = lo;
                 x[1][u] = hi;
               }
@@ -836,19 +802,7 @@ __global__ void __launch_bounds__(128, 8) selected_attend_kernel(const T* __rest
             if (g8 == 0) ld16(qrow + 32 * cc + hh * HALF + 8 * t4, qf);
 #pragma unroll
             for (int h2 = 0; h2 < 2; ++h2) {
-              if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                             "{%0,%1,%2,%3};"
-                             : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
-                             : "r"(xa[hh][2 * h2]), "r"(xb[hh][2 * h2]), "r"(xa[hh][2 * h2 + 1]), "r"(xb[hh][2 * h2 + 1]),
-                               "r"(qf[2 * h2]), "r"(qf[2 * h2 + 1]));
-              } else {
-                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                             "{%0,%1,%2,%3};"
-                             : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
-                             : "r"(xa[hh][2 * h2]), "r"(xb[hh][2 * h2]), "r"(xa[hh][2 * h2 + 1]), "r"(xb[hh][2 * h2 + 1]),
-                               "r"(qf[2 * h2]), "r"(qf[2 * h2 + 1]));
-              }
+              mma16<T>(acc, xa[hh][2 * h2], xb[hh][2 * h2], xa[hh][2 * h2 + 1], xb[hh][2 * h2 + 1], qf[2 * h2], qf[2 * h2 + 1]);
             }
           }
         }

@@ -7,6 +7,7 @@
 //      roundings to the input dtype and writes fp32 scores.
 // Reference: llama/llama_mem.py:357-367, lm_benchmark/models/caches/mem_cache.py:51-61.
 #include "common.cuh"
+#include "mma16.cuh"
 #include "sm100_ptx.cuh"
 #include "scores_sm100.h"
 #include "attn_params.h"
@@ -23,32 +24,6 @@ __host__ __device__ __forceinline__ int logical_age2(int phys, int ring_start, i
 }
 
 constexpr int kRotPerCta = 16;
-
-template <typename T> struct Pk16;      // two 16-bit values in one register, rounded like the tensor formulation
-template <> struct Pk16<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-};
-template <> struct Pk16<__half> {
-  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-  static __device__ __forceinline__ uint32_t add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-  }
-};
 
 // Sixteen landmark rows per CTA, eight threads per row: each thread takes one 16-byte vector of the low half of the
 // row and its partner of the high half, so every load of the CTA is in flight at once.
@@ -90,8 +65,8 @@ __global__ void __launch_bounds__(128) rotate_landmarks_kernel(const T* __restri
         pl = __byte_perm(l[u], l[u], 0x1032) ^ 0x00008000u;      // pairs (x0, x1) -> (-x1, x0)
         ph = __byte_perm(hh[u], hh[u], 0x1032) ^ 0x00008000u;
       }
-      ol[u] = Pk16<T>::add(Pk16<T>::mul(l[u], c0[u]), Pk16<T>::mul(pl, s0[u]));
-      oh[u] = Pk16<T>::add(Pk16<T>::mul(hh[u], c1[u]), Pk16<T>::mul(ph, s1[u]));
+      ol[u] = Pair16<T>::add(Pair16<T>::mul(l[u], c0[u]), Pair16<T>::mul(pl, s0[u]));
+      oh[u] = Pair16<T>::add(Pair16<T>::mul(hh[u], c1[u]), Pair16<T>::mul(ph, s1[u]));
     }
     lo = make_uint4(ol[0], ol[1], ol[2], ol[3]);
     hi = make_uint4(oh[0], oh[1], oh[2], oh[3]);
