@@ -181,7 +181,10 @@ class MemLMCacheStorage(nn.Module):
             self.last_incomplete_ismem[:B, :inc].copy_(is_mem[:, full:])
         self.last_incomplete_len = inc
         if full:
-            L.host().check_regular(is_mem[:, :full], blk)      # every block ends in its only landmark, or AssertionError
+            flags = is_mem[:, :full]
+            if flags.dtype != torch.bool:
+                flags = flags.ne(0)                             # any value but zero marks a landmark
+            L.host().check_regular(flags, blk)                  # every block ends in its only landmark, or AssertionError
         added = full // blk
         dropped = max(0, added - cap)           # more blocks than the ring holds: only the newest `cap` are kept
         self.cache_iter = (self.cache_iter + dropped) % cap

@@ -74,3 +74,18 @@ def test_chunks_below_a_block_are_stored_as_the_whole_is(chunks, dtype, layout):
                  (many.last_incomplete_k[:, :, :tail], k[:, :, n - tail:]), (many.last_incomplete_v[:, :, :tail], v[:, :, n - tail:]),
                  (many.last_incomplete_ismem[:, :tail], im[:, n - tail:])):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,value", [(torch.uint8, 1), (torch.uint8, 255), (torch.int64, 7), (torch.float32, 0.5)])
+def test_any_value_but_zero_marks_a_landmark(dtype, value):
+    blk, n = 8, 19
+    cfg = types.SimpleNamespace(batch_size=2, mem_cache_size=4, mem_cache_freq=blk - 1, n_head=2, n_embd=256, cache_topk=2,
+                                cache_selection_method="per_token_and_head")
+    k = torch.randn(2, 2, n, 128, device=DEV)
+    im = (torch.arange(n, device=DEV) % blk == blk - 1).view(1, n).expand(2, n).to(dtype) * value
+    st = P.MemLMCacheStorage(cfg, None, dtype=torch.float32, device=DEV)
+    st.store_in_cache(k, {"v": k, "is_mem": im})
+    assert (st.cache_size, st.last_incomplete_len) == (2, 3) and torch.equal(st.cache_lm_k[:, :, 0], k[:, :, blk - 1])
+    im[1, 3] = value
+    with pytest.raises(AssertionError):
+        P.MemLMCacheStorage(cfg, None, dtype=torch.float32, device=DEV).store_in_cache(k, {"v": k, "is_mem": im})
