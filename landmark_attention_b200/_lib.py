@@ -26,7 +26,6 @@ class CacheDesc(Structure):
 
 
 I64x3 = c_int64 * 3
-I64x4 = c_int64 * 4
 
 PROTOTYPES = {
     "lmk_version": (c_int, []),
@@ -202,12 +201,6 @@ def stream_ptr(device):
 def strides3(t: torch.Tensor):
     assert t.dim() == 4 and t.stride(3) == 1
     return I64x3(t.stride(0), t.stride(1), t.stride(2))
-
-
-def strides4_broadcast(t: torch.Tensor, shape):
-    """Element strides of `t` expanded to 4-D `shape` (0 where broadcast)."""
-    t = t.expand(shape)
-    return t, I64x4(*t.stride())
 
 
 def check(rc: int, what: str):

@@ -4,6 +4,7 @@
 #include "common.cuh"
 #include "attn_params.h"
 
+#include <atomic>
 #include <mutex>
 
 // Scratch for lmk_attn_bwd_static: one float per (batch, head, query row).  Lives in every GPU that loads the library
@@ -24,6 +25,20 @@ int fail(int code, const char* fmt, ...) {
   vsnprintf(error_buffer(), 512, fmt, ap);
   va_end(ap);
   return code;
+}
+
+int sm_count(int* n) {
+  constexpr int kMax = 64;
+  static std::atomic<int> known[kMax];
+  int dev = 0;
+  LMK_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kMax) return fail(LMK_ERR_UNSUPPORTED, "device index %d out of range", dev);
+  *n = known[dev].load(std::memory_order_relaxed);
+  if (*n == 0) {
+    LMK_CUDA(cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev));
+    known[dev].store(*n, std::memory_order_relaxed);
+  }
+  return LMK_OK;
 }
 
 namespace {

@@ -585,13 +585,6 @@ bool f32_operands_ok(const AttnParams& p) {
   return p.block == kBK && p.D <= 128 && p.D % 8 == 0 && vec_ok(p.q, p.qs) && vec_ok(p.k, p.ks) && vec_ok(p.v, p.vs);
 }
 
-int sm_count(int* n) {
-  int dev = 0;
-  LMK_CUDA(cudaGetDevice(&dev));
-  LMK_CUDA(cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev));
-  return LMK_OK;
-}
-
 template <int kD>
 int fwd_launch(const AttnParams& p, cudaStream_t st) {
   int n_sm, rc = sm_count(&n_sm);

@@ -31,6 +31,7 @@
 //   sm100_mask_bwd_dkv_kernel, CTA per (64-key tile, batch*head) streaming the query tiles that see it: rebuilds P and dS
 //     from A, R, nD, delta and accumulates dV^T += dO^T P, dK^T += Q^T dS (transposed accumulators, M = 128).
 // The same identities as the regular-pattern kernels in attn_sm100.cu apply (see there for the derivation).
+#include <algorithm>
 #include <mutex>
 #include "common.cuh"
 #include "attn_params.h"
@@ -1213,7 +1214,9 @@ int attn_mask_sm100_fwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
   const int only_marked = attn_sm100_flags(p.Lk, G) && p.scale > 0.f;
   if (only_marked && (rc = attn_sm100_flags_fwd(p, is_mem, is_mem_stride, G, R, dtype, st)) != LMK_OK) return rc;
   const int tiles = p.B * p.H * (p.Lq / kQT);
-  const int grid = only_marked && tiles > 148 ? 148 : tiles;
+  int n_sm = 0;
+  if ((rc = sm_count(&n_sm)) != LMK_OK) return rc;
+  const int grid = only_marked ? std::min(tiles, n_sm) : tiles;
   const size_t smem = mf_smem_bytes(G, p.Lk / kKT);
   if (dtype == LMK_BF16)
     LMK_CUDA(launch_overlapped(sm100_mask_fwd_kernel<true>, dim3(grid), dim3(kMfThreads), smem, st, tq, tk, tv, is_mem, is_mem_stride,
@@ -1254,8 +1257,10 @@ int attn_mask_sm100_bwd(const AttnParams& p, const uint8_t* is_mem, int64_t is_m
     int* records = reinterpret_cast<int*>(nD + (size_t)p.B * p.H * G * p.Lq);
     if ((rc = attn_sm100_flags_bwd(p, is_mem, is_mem_stride, G, R, records, dtype, st)) != LMK_OK) return rc;
     plan = records;
-    grid_q = grid_q < 148 ? grid_q : 148;
-    grid_k = grid_k < 148 ? grid_k : 148;
+    int n_sm = 0;
+    if ((rc = sm_count(&n_sm)) != LMK_OK) return rc;
+    grid_q = std::min(grid_q, n_sm);
+    grid_k = std::min(grid_k, n_sm);
   }
 #define LMK_MASK_BWD(BF)                                                                                                \
   do {                                                                                                                  \

@@ -15,6 +15,9 @@ namespace lmk {
 char* error_buffer();
 int fail(int code, const char* fmt, ...);
 
+// Multiprocessors of the current device (asked for once per device); a status code.
+int sm_count(int* n);
+
 #define LMK_CHECK_ARG(cond, ...)                                   \
   do {                                                             \
     if (!(cond)) return lmk::fail(LMK_ERR_INVALID, __VA_ARGS__);   \

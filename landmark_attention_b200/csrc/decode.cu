@@ -450,7 +450,10 @@ extern "C" int lmk_decode_attend(const void* q, const void* k_new, const void* v
   p.cos_t = cos_table; p.sin_t = sin_table; p.n_pos = n_pos; p.out = out; p.H = H; p.T = T; p.scale = sm_scale;
   const int BH = B * H;
   // 8 CTAs a (token, head) while that still leaves SMs free, 4 otherwise: more CTAs only shorten the scoring phase
-  const bool wide = BH * T * 8 <= 148;
+  int n_sm = 0;
+  const int rc = sm_count(&n_sm);
+  if (rc != LMK_OK) return rc;
+  const bool wide = BH * T * 8 <= n_sm;
   if (dtype == LMK_BF16)
     return wide ? dec_launch<__nv_bfloat16, 8>(p, BH, (cudaStream_t)stream) : dec_launch<__nv_bfloat16, 4>(p, BH, (cudaStream_t)stream);
   return wide ? dec_launch<__half, 8>(p, BH, (cudaStream_t)stream) : dec_launch<__half, 4>(p, BH, (cudaStream_t)stream);

@@ -1610,7 +1610,10 @@ int launch(const GsParams& p, int dtype, cudaStream_t st) {
   // warps (causal rows differ in length), eight at most.
   int per_group = 1, per_warp = 0;
   if (lanes) {
-    const int64_t resident = 148 * kGsWarps * 8;
+    int n_sm = 0;
+    const int rc = sm_count(&n_sm);
+    if (rc != LMK_OK) return rc;
+    const int64_t resident = (int64_t)n_sm * kGsWarps * 8;
     per_group = (int)std::min<int64_t>(std::max<int64_t>(rows / (3 * resident), 1), std::min(p.H, 8));
     const int groups = (p.H + per_group - 1) / per_group;
     per_group = (p.H + groups - 1) / groups;
