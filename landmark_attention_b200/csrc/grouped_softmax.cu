@@ -1064,13 +1064,16 @@ __device__ __forceinline__ void causal_masks(const Bits<K>& f, const Bits<K>& be
 // Passes 1 and 2 of a row: maxima of the groups and of the bucket, then exponentials (they replace the scores in shared
 // memory), sums and landmark weights.  binv: 1 / the bucket's sum; for the lane's groups a and b: i = 1 / the group's sum, w = the
 // landmark's share of the bucket; elm: exponential of the lane's own landmark.
-// kTwo: some lanes hold two landmarks; the keys between them (gm) are a group of their own, closed by the second one (lm2_slot).
+// What lies between a lane's landmarks (gm): nothing (kInner = kNone: one landmark a lane at most), a group of its own that the second
+// one (lm2_slot) closes (kOne), or groups that the caller has worked out (kDone: their places are left alone).
+enum { kNone, kOne, kDone };
 struct LaneWeights { float binv, ia, ib, wa, wb, elm, im, wm, elm2; };
-template <typename T, int K, bool kTwo>
+template <typename T, int K, int kInner>
 __device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4, int lm_slot, const Bits<K>& ga, const Bits<K>& gb,
                                                     const Bits<K>& bk, const LaneGroups& lg, int ca, int G, bool guards,
                                                     const Bits<K>& gm = Bits<K>(), int lm2_slot = 0, int nlm = 1) {
-  const int cb = kTwo ? ca + max(nlm, 1) : ca + 1;
+  constexpr bool kTwo = kInner == kOne;
+  const int cb = kInner != kNone ? ca + max(nlm, 1) : ca + 1;
   float vm = -INFINITY;
   // pass 1: group and bucket maxima
   float va = -INFINITY, vb = -INFINITY, bmax = -INFINITY;
@@ -1113,6 +1116,7 @@ __device__ __forceinline__ LaneWeights lane_weights(LaneRow& xr, int c0, int n4,
     for (int v = 0; v < 4; ++v) {
       const bool ib = (fb >> v) & 1u, ik = (fk >> v) & 1u;
       const bool im = kTwo && ((gm.piece(q) >> v) & 1u);
+      if (kInner == kDone && ((gm.piece(q) >> v) & 1u)) continue;
       x[v] = exp_diff(x[v], ik ? bmax : ib ? mb : im ? mm : ma);       // keys outside the row hold -inf
       if (im) vm += x[v];
       if ((fa >> v) & 1u) va += x[v];
@@ -1260,7 +1264,7 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
     }
     if (lane == 0 && n_groups >= G && p.status != nullptr) atomicCAS(p.status, 0, kErrSoftmaxGroups);
 
-    const LaneWeights lw = lane_weights<T, K, kTwo>(xr, c0, n4, lm_slot, ga, gb, bk, lg, ca, G, guards, gm, lm2_slot, nlm);
+    const LaneWeights lw = lane_weights<T, K, kTwo ? kOne : kNone>(xr, c0, n4, lm_slot, ga, gb, bk, lg, ca, G, guards, gm, lm2_slot, nlm);
     const float binv = lw.binv, ia = lw.ia, ib = lw.ib, wa = lw.wa, elm = lw.elm;
     float va, vb, closed;
     const float sa = ia * wa, sb = ib * lw.wb, sm = lw.im * lw.wm;
@@ -1385,51 +1389,66 @@ __host__ __device__ constexpr size_t cr_smem(int T, int P) {
   return sizeof(float) * kCrRows * 144 * (size_t)cr_pieces(P + T) + 2 * (size_t)kCrRows * cr_prob_pitch(T) + 2 * 64 * kCrVPitch;
 }
 
-// A row in which two landmarks share a lane (cached rows): group after group, the whole warp on each.  Probabilities replace the scores.
+// A row in which landmarks share a lane (cached rows).  The groups between a lane's landmarks lie in the lane: it works them out first,
+// one after the other, as far as exponential over sum; the rest of the row goes the way of the other rows, and the last pass, back to
+// front, gives the inner groups their landmarks' weights.  Probabilities replace the scores.
+// Every key is looked at a fixed number of times, however many landmarks there are.  The call (us; with the scores and the softmax as
+// tensor operations / a walk of the whole row for every group / this): B16 H8 T255 P204, a landmark every 8 keys 468 / 2150 / 388, every
+// 2 552 / 6954 / 404; B4 H8 T512 P512, every 16 505 / 4797 / 563, every 2 581 / 29 170 / 591.
 template <int K>
-__device__ __noinline__ void crowded_smem_row(LaneRow xr, int c0, int n4, Bits<K> mem, Bits<K> last, Bits<K> bk, int G) {
-  const int lane = threadIdx.x & 31;
+__device__ __noinline__ void crowded_smem_row(LaneRow xr, int c0, int n4, Bits<K> mem, Bits<K> last, Bits<K> bk, unsigned owners, int G) {
   const int nlm = mem.count();
-  int inc = nlm;
+  int ca = nlm;                                         // landmarks in front of the lane
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += u;
+    const int u = __shfl_up_sync(0xffffffffu, ca, o);
+    if (xr.lane >= o) ca += u;
   }
-  const int before = inc - nlm, n_groups = __shfl_sync(0xffffffffu, inc, 31);
-  // f(score slot, landmarks in front of the key, landmark, last section, bucket) for every key of the lane
-  auto each = [&](auto f) {
-    int c = before;
-#pragma unroll 1
-    for (int v = 0; v < 4 * n4; ++v) {
-      const uint32_t m = mem.piece(v >> 2) >> (v & 3), l = last.piece(v >> 2) >> (v & 3), b = bk.piece(v >> 2) >> (v & 3);
-      f(xr.slot(c0 + (v >> 2)) * 4 + (v & 3), c, m & 1u, l & 1u, b & 1u);
-      c += m & 1u;
+  ca -= nlm;
+  const int t = mem.first(), t2 = nlm ? mem.top() : K;
+  const Bits<K> upto = Bits<K>::low(t), upto2 = Bits<K>::low(t2);
+  const Bits<K> ga = Bits<K>::zip([&](int w) { return ~bk.w[w] & upto.w[w]; });
+  const Bits<K> gb = Bits<K>::zip([&](int w) { return ~bk.w[w] & ~upto2.w[w]; });
+  const Bits<K> gm = Bits<K>::zip([&](int w) { return ~bk.w[w] & ~upto.w[w] & upto2.w[w]; });
+  auto at = [&](int v) { return xr.slot(c0 + (v >> 2)) * 4 + (v & 3); };
+  auto bit = [](const Bits<K>& m, int v) { return (m.piece(v >> 2) >> (v & 3)) & 1u; };
+  if (nlm > 1) {
+    for (int s = t, c = ca + 1; s < t2; ++c) {          // the group behind the landmark at s
+      float mx = -INFINITY, den = 0.f;
+      int e = s + 1;
+      for (; !bit(mem, e); ++e)
+        if (bit(gm, e)) mx = fmaxf(mx, xr.buf[at(e)]);
+      if (isinf(mx)) mx = 0.f;
+      for (int v = s + 1; v < e; ++v)
+        if (bit(gm, v)) {
+          const float x = exp_diff(xr.buf[at(v)], mx);
+          xr.buf[at(v)] = x;
+          den += x;
+        }
+      const float inv = c >= G || den < 0.5f ? 0.f : 1.f / den;
+      for (int v = s + 1; v < e; ++v)
+        if (bit(gm, v)) xr.buf[at(v)] *= inv;
+      s = e;
     }
-  };
-  float mx = -INFINITY, sum = 0.f;
-  each([&](int e, int, uint32_t, uint32_t, uint32_t b) { if (b) mx = fmaxf(mx, xr.buf[e]); });
-  mx = warp_max(mx);
-  if (isinf(mx)) mx = 0.f;
-  each([&](int e, int, uint32_t, uint32_t, uint32_t b) { if (b) sum += exp_diff(xr.buf[e], mx); });
-  sum = warp_sum(sum);
-  const float binv = sum < 0.5f ? 0.f : 1.f / sum;
-  for (int g = 0; g <= n_groups; ++g) {
-    float gm = -INFINITY, lm = 0.f, den = 0.f;
-    each([&](int e, int c, uint32_t m, uint32_t, uint32_t b) {
-      if (c != g) return;
-      if (!b) gm = fmaxf(gm, xr.buf[e]);
-      if (m) lm = exp_diff(xr.buf[e], mx);
-    });
-    gm = warp_max(gm);
-    lm = g < G ? warp_sum(lm) * binv : warp_sum(lm) * 0.f;
-    if (isinf(gm)) gm = 0.f;
-    each([&](int e, int c, uint32_t, uint32_t, uint32_t b) { if (c == g && !b) den += exp_diff(xr.buf[e], gm); });
-    den = warp_sum(den);
-    const float w = den < 0.5f ? 0.f : lm / den;
-    each([&](int e, int c, uint32_t, uint32_t, uint32_t b) { if (c == g && !b) xr.buf[e] = exp_diff(xr.buf[e], gm) * w; });
   }
-  each([&](int e, int, uint32_t, uint32_t l, uint32_t b) { if (b) xr.buf[e] = l ? exp_diff(xr.buf[e], mx) * binv : 0.f; });
+  const LaneGroups lg(xr.lane, owners);
+  const int lm_slot = xr.slot(min(c0 + (t >> 2), 32 * n4 - 1)) * 4 + (t & 3);
+  const LaneWeights lw = lane_weights<float, K, kDone>(xr, c0, n4, lm_slot, ga, gb, bk, lg, ca, G, true, gm, 0, nlm);
+  const float sa = lw.ia * lw.wa, sb = lw.ib * lw.wb;
+  float w = 0.f;                                        // of the landmark passed last
+  int c = ca + nlm;
+#pragma unroll 1
+  for (int q = n4 - 1; q >= 0; --q) {
+    const uint32_t fa = ga.piece(q), fb = gb.piece(q), fm = gm.piece(q), fl = last.piece(q), lm = mem.piece(q);
+    float x[4];
+    xr.get<float>(xr.slot(c0 + q), x);
+#pragma unroll
+    for (int v = 3; v >= 0; --v) {
+      if ((lm >> v) & 1u) w = --c < G ? x[v] * lw.binv : 0.f;
+      x[v] *= (fl >> v) & 1u ? lw.binv : (fb >> v) & 1u ? sb : (fm >> v) & 1u ? w : (fa >> v) & 1u ? sa : 0.f;
+    }
+    xr.put(xr.slot(c0 + q), x);
+  }
 }
 
 template <typename T, int K>
@@ -1508,7 +1527,7 @@ __global__ void __launch_bounds__(kCrThreads, K == 32 ? 4 : 2) cached_rows_kerne
     const int n_groups = __reduce_add_sync(0xffffffffu, nlm);
     if (lane == 0 && n_groups >= p.G && p.status != nullptr) atomicCAS(p.status, 0, kErrSoftmaxGroups);
     if (__any_sync(0xffffffffu, nlm > 1)) {
-      crowded_smem_row<K>(xr, c0, n4, mem, last, bk, p.G);
+      crowded_smem_row<K>(xr, c0, n4, mem, last, bk, owners, p.G);
     } else {
       const LaneGroups lg(lane, owners);
       const int t = mem.first();
@@ -1517,7 +1536,7 @@ __global__ void __launch_bounds__(kCrThreads, K == 32 ? 4 : 2) cached_rows_kerne
       const Mask gb = Mask::zip([&](int w) { return ~bk.w[w] & ~upto.w[w]; });
       const int lm_slot = xr.slot(min(c0 + (t >> 2), 32 * n4 - 1)) * 4 + (t & 3);
       const LaneWeights lw =
-          lane_weights<float, K, false>(xr, c0, n4, lm_slot, ga, gb, bk, lg, __popc(owners & ((1u << lane) - 1u)), p.G, true);
+          lane_weights<float, K, kNone>(xr, c0, n4, lm_slot, ga, gb, bk, lg, __popc(owners & ((1u << lane) - 1u)), p.G, true);
       const float sa = lw.ia * lw.wa, sb = lw.ib * lw.wb;
 #pragma unroll 1
       for (int c = 0; c < n4; ++c) {
