@@ -809,10 +809,12 @@ Tensor chunk_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
 // n blocks, on the device (lm undefined: landmarks are read from kc; append: k, v stored behind the n blocks) or in pinned host memory
 // (lm: their landmark keys; append: the chunk's whole blocks stored, on a second stream, because the writes over the host link
 // do not depend on the attention and run against the direction of its reads).  Undefined where the kernels do not take the call or a
-// gradient is asked for: the tensor formulation of the same call is differentiable.
+// gradient is asked for: the tensor formulation of the same call is differentiable.  It also takes blocks above 64: their attention runs
+// on the two-pass tensor-core kernels there (H8, 100 tokens, blocks of 128, top 4: 355 us; 550 on the general kernels, which
+// attn_fwd takes and which end at blocks of 128).
 Tensor per_head_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& kc, const Tensor& vc, const Tensor& lm, int64_t n,
                        bool append, int64_t block, int64_t top_k, const Tensor& cos, const Tensor& sin) {
-  if (needs_grad({q_, k_, v_, cos, sin})) return Tensor();
+  if (block > 64 || needs_grad({q_, k_, v_, cos, sin})) return Tensor();
   const bool host = lm.defined();
   Chunk c;
   if (block < 1 || n < 1 || n > 49152 || top_k < 1 || top_k > 32 || kc.is_cuda() == host || vc.is_cuda() == host ||

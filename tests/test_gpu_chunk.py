@@ -61,6 +61,23 @@ def test_per_head_selection_on_device_and_host_caches(B, H, T, blk, N, top_k, dt
     assert torch.equal(off.lm_keys[:, :, :off.n_blocks], past[0][:, :, blk - 1::blk])
 
 
+@pytest.mark.parametrize("T,blk,N,top_k", [(128, 128, 9, 2), (256, 256, 5, 1), (512, 256, 6, 3)])
+def test_per_head_selection_of_large_blocks(T, blk, N, top_k):
+    pk, pv, q, k, v, (cos, sin) = problem(1, 2, T, blk, N, torch.bfloat16, T)
+    exp, past, _ = P.llama_retrieval_attention(q, k, v, pk, pv, blk - 1, top_k, cos=cos, sin=sin, aggregate="max_over_tokens",
+                                               return_debug=True)
+    cache = P.LandmarkKVCache(1, 2, N * blk + T, 128, torch.bfloat16, DEV)
+    cache.append(pk, pv)
+    off = P.OffloadedLandmarkCache(1, 2, N + T // blk, blk, 128, torch.bfloat16, DEV)
+    off.append(pk, pv)
+    got, views = P.llama_retrieval_attention(q, k, v, mem_freq=blk - 1, cache_top_k=top_k, cos=cos, sin=sin, cache=cache,
+                                             aggregate="max_over_tokens")
+    assert close(got, exp) and torch.equal(views[0], past[0]) and torch.equal(views[1], past[1])
+    assert close(off.attend(q, k, v, top_k, cos, sin), exp) and off.length == N * blk + T
+    torch.cuda.synchronize()
+    assert torch.equal(off.k_host.to(DEV), past[0]) and torch.equal(off.v_host.to(DEV), past[1])
+
+
 def test_ragged_chunk_against_the_host_cache_waits_in_the_tail():
     pk, pv, q, k, v, (cos, sin) = problem(1, 2, 100, 64, 10, torch.bfloat16, 1)
     off = P.OffloadedLandmarkCache(1, 2, 12, 64, 128, torch.bfloat16, DEV)
