@@ -343,11 +343,13 @@ __global__ void __launch_bounds__(kDkvWarps * 32) general_bwd_dkv_kernel(AttnPar
   extern __shared__ __align__(16) float smem[];
   const int D = p.D, DP = D + 1, blk = p.block;
   const int blkpad = (blk + 31) & ~31;
-  float* Ks = smem;                         // [blk][D+1]
-  float* Vs = Ks + blk * DP;                // [blk][D+1]
-  float* Qs = Vs + blk * DP;                // [32][D]
+  // The query and dO rows are read as 16-byte vectors and come first: behind the keys' 2 blk (D + 1) floats they would start off
+  // a 16-byte boundary where blk is odd.
+  float* Qs = smem;                         // [32][D]
   float* dOs = Qs + kDkvRows * D;           // [32][D]
-  float* Pb = dOs + kDkvRows * D;           // [32][blkpad]
+  float* Ks = dOs + kDkvRows * D;           // [blk][D+1]
+  float* Vs = Ks + blk * DP;                // [blk][D+1]
+  float* Pb = Vs + blk * DP;                // [32][blkpad]
   float* dSb = Pb + kDkvRows * blkpad;      // [32][blkpad]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

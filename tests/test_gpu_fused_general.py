@@ -142,3 +142,17 @@ def test_reference_assertions_are_kept():
     out = P.fused_landmark_attention(qr, qr, qr, None, block_size=64, path=P.PATH_GENERAL)   # ragged forward is fine
     with pytest.raises(AssertionError):
         out.sum().backward()                                                                 # backward is not
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)])
+@pytest.mark.parametrize("blk,n,hist,D", [(3, 5, 0, 8), (5, 7, 2, 40), (17, 11, 2, 128), (51, 3, 1, 64), (127, 2, 0, 128)])
+def test_odd_blocks_backward(blk, n, hist, D, dtype, tol):
+    # the keys of an odd block leave the arrays behind them off the vectors' boundaries
+    g = torch.Generator().manual_seed(blk)
+    B, H, Lq, Lk = 2, 3, n * blk, (n + hist) * blk
+    q, k, v, do = [(torch.randn(B, H, L, D, generator=g) * 0.5).to(dtype) for L in (Lq, Lk, Lk, Lq)]
+    exp = O.landmark_attention_grads(q.float(), k.float(), v.float(), do.float(), blk)
+    qc, kc, vc = [t.to(DEV).requires_grad_(True) for t in (q, k, v)]
+    out = P.fused_landmark_attention(qc, kc, vc, None, block_size=blk, path=P.PATH_GENERAL)
+    for got, want in zip((out, *torch.autograd.grad(out, [qc, kc, vc], do.to(DEV))), exp):
+        assert (got.detach().float().cpu() - want).abs().max().item() < tol
