@@ -778,6 +778,8 @@ Tensor chunk_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   if (n > 49152 || kc.size(2) < len + (append ? q_.size(2) : 0) || !kc.is_cuda() || !vc.is_cuda() || !chunk_of(&c, q_, k_, v_, kc, vc, cos, sin))
     return Tensor();
   c10::cuda::OptionalCUDAGuard guard(q_.device());
+  // the values go to the attention as they are, and TMA addresses neither broadcast heads nor overlapping rows
+  if (c.v.stride(0) <= 0 || c.v.stride(1) <= 0 || c.v.stride(2) < c.D) c.v = c.v.clone(at::MemoryFormat::Contiguous);
   const lmk_cache_desc d = rows_desc(kc, n, block, top_k);
   Tensor qr = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q), kr = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q);
   check(lib.lmk_chunk_rotate(c.q.data_ptr(), c.k.data_ptr(), c.v.data_ptr(), S3(c.q).v, S3(c.k).v, S3(c.v).v, cos.data_ptr(),

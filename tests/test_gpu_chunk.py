@@ -37,6 +37,24 @@ def test_chunk_matches_the_gathered_route(B, H, T, blk, N, top_k, dtype):
     assert L.device_status() == 0
 
 
+@pytest.mark.parametrize("which", ["q", "k", "v", "qkv"])
+@pytest.mark.parametrize("form", ["heads", "batch", "rows", "offset", "features"])
+def test_chunk_of_any_strides(form, which):
+    B, H, T, blk, N, dtype = 2, 3, 40, 32, 6, torch.bfloat16
+    pk, pv, q, k, v, (cos, sin) = problem(B, H, T, blk, N, dtype, T)
+    odd = {"heads": lambda t: t[:, :1].expand(B, H, T, 128), "batch": lambda t: t[:1].expand(B, H, T, 128),
+           "rows": lambda t: t[:, :, :1].expand(B, H, T, 128),
+           "offset": lambda t: torch.cat((t.new_zeros(3), t.reshape(-1)))[3:].view(B, H, T, 128),
+           "features": lambda t: torch.stack((t, t), -1).flatten(-2)[..., ::2]}[form]
+    q, k, v = [odd(t) if name in which else t for name, t in (("q", q), ("k", k), ("v", v))]
+    exp, _ = P.llama_retrieval_attention(*[t.contiguous() for t in (q, k, v)], pk, pv, blk - 1, 3, cos=cos, sin=sin)
+    cache = P.LandmarkKVCache(B, H, N * blk + T, 128, dtype, DEV)
+    cache.append(pk, pv)
+    for args in (dict(cache=cache), dict(past_k=pk, past_v=pv)):
+        got, (gk, gv) = P.llama_retrieval_attention(q, k, v, mem_freq=blk - 1, cache_top_k=3, cos=cos, sin=sin, **args)
+        assert torch.equal(got, exp) and torch.equal(gk[:, :, N * blk:], k) and torch.equal(gv[:, :, N * blk:], v)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,H,T,blk,N,top_k", [(1, 3, 256, 64, 140, 4), (2, 2, 96, 32, 20, 1), (1, 4, 128, 32, 129, 6), (1, 2, 64, 64, 3, 3)])
 def test_per_head_selection_on_device_and_host_caches(B, H, T, blk, N, top_k, dtype):
