@@ -36,3 +36,26 @@ def test_ragged_lengths_and_small_heads(B, H, Lq, hist, D, dtype):
         assert (got - e).abs().max().item() < 2e-2 * max(1.0, e.abs().max().item()), name
         assert ((got - e).norm() / e.norm().clamp_min(1e-6)).item() < 1e-2 or e.norm() < 1e-3, name
     assert L.device_status() == 0
+
+
+@pytest.mark.parametrize("form", ["heads", "batch", "rows", "offset", "features"])
+@pytest.mark.parametrize("Lq,hist,D,blk", [(77, 64, 128, 64), (100, 0, 64, 32), (256, 0, 128, 64), (45, 0, 40, 2)])
+def test_operands_that_tma_cannot_address(Lq, hist, D, blk, form):
+    # they are copied: the same result as dense operands give, also where the sequence ends inside a block, and gradients of the views
+    g = torch.Generator(device="cuda").manual_seed(Lq)
+    B, H, Lk = 2, 3, Lq + hist
+    def make(L):
+        base = torch.randn(B, H, L, D, device="cuda", generator=g).to(torch.bfloat16)
+        return {"heads": lambda: base[:, :1].expand(B, H, L, D), "batch": lambda: base[:1].expand(B, H, L, D),
+                "rows": lambda: base[:, :, :1].expand(B, H, L, D),
+                "offset": lambda: torch.cat((base.new_zeros(3), base.reshape(-1)))[3:].view(B, H, L, D),
+                "features": lambda: torch.stack((base, base), -1).flatten(-2)[..., ::2]}[form]()
+    q, k, v = make(Lq), make(Lk), make(Lk)
+    do = torch.randn(B, H, Lq, D, device="cuda", generator=g).to(torch.bfloat16)
+    runs = []
+    for dense in (False, True):
+        a = [t.contiguous().requires_grad_(True) if dense else t.requires_grad_(True) for t in (q.detach(), k.detach(), v.detach())]
+        o = P.fused_landmark_attention(*a, None, block_size=blk)
+        runs.append((o, *torch.autograd.grad(o, a, do)))
+    for got, exp in zip(*runs):
+        assert got.shape == exp.shape and torch.equal(got, exp)
