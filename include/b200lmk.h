@@ -99,8 +99,8 @@ size_t lmk_attn_bwd_workspace(int B, int H, int Lq, int Lk, int D, int block, in
  * Replaces FusedLandmarkAttention.backward + _bwd_preprocess + _bwd_kernel
  *   (llama/ltriton/flash_landmark_attention.py:125-305, 356-389).
  *   o, dO, dQ [B,H,Lq,D] dense; dK, dV [B,H,Lk,D] dense; L, M from the forward call.
- *   Lq and Lk must be multiples of block (:359-360).  workspace: >= lmk_attn_bwd_workspace(...) bytes,
- *   256-byte aligned, contents irrelevant on entry.
+ *   fp32, and LMK_PATH_GENERAL: Lq and Lk must be multiples of block (:359-360); 16-bit types with LMK_PATH_AUTO take any
+ *   length.  workspace: >= lmk_attn_bwd_workspace(...) bytes, 256-byte aligned, contents irrelevant on entry.
  */
 int lmk_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dO,
                  const float* L, const float* M, void* dQ, void* dK, void* dV,

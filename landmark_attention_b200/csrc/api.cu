@@ -201,7 +201,9 @@ extern "C" int lmk_attn_bwd_strided(const void* q, const void* k, const void* v,
   for (int i = 0; i < 3; ++i) p.dos[i] = do_strides[i];
   int which = pick_path(path, p, dtype, true);
   if (which < 0) return which;
-  LMK_CHECK_ARG(which != LMK_PATH_GENERAL || (Lq % block == 0 && Lk % block == 0),
+  // The reference's rule.  It is kept for fp32 and where the general kernels are asked for by name; 16-bit calls of any length run on
+  // the tensor-core kernels, and a call that they leave (a scale that is not positive) has the same lengths.
+  LMK_CHECK_ARG(which != LMK_PATH_GENERAL || (Lq % block == 0 && Lk % block == 0) || (path == LMK_PATH_AUTO && dtype != LMK_F32),
                 "Backward supported only for full blocks (Lq=%d Lk=%d block=%d)", Lq, Lk, block);
   const size_t need = lmk_attn_bwd_workspace(B, H, Lq, Lk, D, block, dtype, which == kPathSmallBlocks ? LMK_PATH_TCGEN05 : which);
   if (need > 0 && (workspace == nullptr || workspace_bytes < need))

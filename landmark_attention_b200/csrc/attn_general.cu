@@ -1,7 +1,8 @@
 // General-path fused landmark attention: CUDA-core kernels with fp32 accumulation.
 //
-// These kernels cover every dtype (fp32 / fp16 / bf16), any head dim <= 128 that is a multiple of 32, any
-// landmark block size in [2, 128], a key prefix (Lk > Lq) and, in the forward pass, a ragged last block.
+// These kernels cover every dtype (fp32 / fp16 / bf16), any head dim <= 128 that is a multiple of 8, any
+// landmark block size in [2, 128], a key prefix (Lk > Lq) and a ragged last block (only rows of that block see its keys, and they
+// see them up to their own position: what lies behind the sequence is read as zeros and hidden).
 // They are the path for shapes that neither the tcgen05 kernels nor the tiled fp32 kernels (attn_f32.cu: blocks of 64) take.
 //
 // Math (same quantities as the reference Triton kernels, llama/ltriton/flash_landmark_attention.py):
@@ -245,11 +246,11 @@ __global__ void __launch_bounds__(kFwdWarps * 32) general_bwd_dq_kernel(AttnPara
   float* prows = Pb + warp * kRowsPerWarp * blkpad;
 
   for (int n = 0; n <= own_last; ++n) {
-    const int key0 = n * blk;
+    const int key0 = n * blk, key_end = min(key0 + blk, p.Lk);
     for (int c0 = 0; c0 < blk; c0 += kChunk) {
       __syncthreads();
-      load_rows_f32(Ks, DP, kp, p.ks[2], key0 + c0, kChunk, key0 + blk, D, tid, blockDim.x);
-      load_rows_f32(Vs, DP, vp, p.vs[2], key0 + c0, kChunk, key0 + blk, D, tid, blockDim.x);
+      load_rows_f32(Ks, DP, kp, p.ks[2], key0 + c0, kChunk, key_end, D, tid, blockDim.x);
+      load_rows_f32(Vs, DP, vp, p.vs[2], key0 + c0, kChunk, key_end, D, tid, blockDim.x);
       __syncthreads();
       float s[kRowsPerWarp], dp[kRowsPerWarp];
       dot_rows<kRowsPerWarp>(Ks + lane * DP, qrows, D, s);
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(kFwdWarps * 32) general_bwd_dq_kernel(AttnPara
     __syncwarp();
     for (int c0 = 0; c0 < blk; c0 += kChunk) {
       __syncthreads();
-      load_rows_f32(Ks, DP, kp, p.ks[2], key0 + c0, kChunk, key0 + blk, D, tid, blockDim.x);
+      load_rows_f32(Ks, DP, kp, p.ks[2], key0 + c0, kChunk, key_end, D, tid, blockDim.x);
       __syncthreads();
       const int jn = min(kChunk, blk - c0);
       for (int j = 0; j < jn; ++j) {
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(kDkvWarps * 32) general_bwd_dkv_kernel(AttnPar
 #pragma unroll
   for (int i = 0; i < kMaxKeysPerWarp; ++i) {
     int j = warp * kpw + i;
-    if (i < kpw && j < blk) {
+    if (i < kpw && j < blk && key0 + j < p.Lk) {
 #pragma unroll
       for (int e = 0; e < 4; ++e)
         if (lane + 32 * e < D) {
@@ -519,7 +520,7 @@ int launch_bwd(const AttnParams& p, cudaStream_t st) {
   size_t smem2 = sizeof(float) * ((size_t)2 * p.block * (p.D + 1) + (size_t)2 * kDkvRows * p.D +
                                   (size_t)2 * kDkvRows * blkpad);
   LMK_CUDA(cudaFuncSetAttribute(general_bwd_dkv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
-  dim3 grid2(p.Lk / p.block, p.B * p.H);
+  dim3 grid2((p.Lk + p.block - 1) / p.block, p.B * p.H);
   general_bwd_dkv_kernel<T><<<grid2, kDkvWarps * 32, smem2, st>>>(p);
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;

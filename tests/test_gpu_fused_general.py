@@ -156,3 +156,27 @@ def test_odd_blocks_backward(blk, n, hist, D, dtype, tol):
     out = P.fused_landmark_attention(qc, kc, vc, None, block_size=blk, path=P.PATH_GENERAL)
     for got, want in zip((out, *torch.autograd.grad(out, [qc, kc, vc], do.to(DEV))), exp):
         assert (got.detach().float().cpu() - want).abs().max().item() < tol
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Lq,hist,D,blk", [(140, 0, 72, 16), (274, 64, 16, 64), (24, 192, 64, 64), (1, 5, 128, 5), (33, 34, 40, 17), (200, 0, 128, 128)])
+def test_ragged_backward_with_a_negative_scale(Lq, hist, D, blk, dtype):
+    g = torch.Generator().manual_seed(Lq + D)
+    B, H, Lk, scale = 2, 2, Lq + hist, -0.2
+    q, k, v, do = [(torch.randn(B, H, L, D, generator=g) * 0.5).to(dtype) for L in (Lq, Lk, Lk, Lq)]
+    pad = -Lk % blk                                        # the oracle wants whole blocks: zero rows behind the real ones
+    fp = [torch.nn.functional.pad(t.float(), (0, 0, 0, pad)) for t in (q, k, v, do)]
+    exp = [t[:, :, :r] for t, r in zip(O.landmark_attention_grads(*fp, blk, sm_scale=scale), (Lq, Lq, Lk, Lk))]
+    # NaNs behind the sequence: nothing there may be read
+    tail = lambda t: torch.cat((t, torch.full((B, H, 130, D), float("nan")).to(dtype)), 2).to(DEV)[:, :, :t.shape[2]]
+    qc, kc, vc = [tail(t).requires_grad_(True) for t in (q, k, v)]
+    out = P.fused_landmark_attention(qc, kc, vc, None, sm_scale=scale, block_size=blk)
+    for got, want in zip((out, *torch.autograd.grad(out, [qc, kc, vc], do.to(DEV))), exp):
+        got = got.detach().float().cpu()
+        assert (got - want).abs().max().item() < 2e-2
+        assert rel_l2(got, want) < 1e-2 or want.norm() < 1e-3
+    with pytest.raises(AssertionError):                    # fp32 keeps the reference's rule
+        a = q.float().to(DEV).requires_grad_(True)
+        o = P.fused_landmark_attention(a, k.float().to(DEV), v.float().to(DEV), None, sm_scale=scale, block_size=blk)
+        assert pad
+        torch.autograd.grad(o, a, do.float().to(DEV))
