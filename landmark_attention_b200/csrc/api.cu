@@ -72,9 +72,9 @@ void fill(AttnParams& p, const void* q, const void* k, const void* v, int B, int
 
 constexpr int kPathSmallBlocks = 3;
 
-// 1 = general, 2 = tcgen05, 3 = tcgen05 with blocks below 64, <0 = error.  LMK_PATH_AUTO takes the tcgen05 kernels when the problem (16-bit type, block 64) AND
-// the operands (alignment, strides) qualify, and the general kernels otherwise; an explicit LMK_PATH_TCGEN05 request asks
-// for whole tiles of head dim 128 and is an error where that cannot be met.
+// 1 = general, 2 = tcgen05, 3 = tcgen05 with blocks below 64, <0 = error.  LMK_PATH_AUTO takes the tcgen05 kernels when the
+// problem (16-bit type, block of up to 64) AND the operands (alignment, strides) qualify, and the general kernels otherwise; an
+// explicit LMK_PATH_TCGEN05 request asks for whole tiles of head dim 128 and is an error where that cannot be met.
 int pick_path(int path, const AttnParams& p, int dtype, bool backward) {
   // the tcgen05 kernels take maxima on raw dot products, which needs a positive softmax scale
   const bool fast = attn_sm100_takes(p.B, p.H, p.Lq, p.Lk, p.D, p.block, dtype) && p.scale > 0.f && attn_sm100_operands_ok(p, backward);

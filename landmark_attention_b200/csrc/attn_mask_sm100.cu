@@ -158,11 +158,10 @@ __host__ __device__ constexpr size_t mf_smem_bytes(int G, int n_kt) {
 }
 
 template <bool kBf16>
-__device__ __forceinline__ void mask_fwd_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k,
-                      const CUtensorMap& tm_v, const uint8_t* __restrict__ is_mem, int64_t is_mem_stride,
-                      void* __restrict__ o_ptr, float* __restrict__ R_ptr, float* __restrict__ A_ptr, int H, int Lq,
-                      int Lk, int G, float scale_log2, int* status,
-    int t, int bh, uint32_t tmem) {
+__device__ __forceinline__ void mask_fwd_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
+                                              const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, void* __restrict__ o_ptr,
+                                              float* __restrict__ R_ptr, float* __restrict__ A_ptr, int H, int Lq, int Lk, int G,
+                                              float scale_log2, int* status, int t, int bh, uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -491,14 +490,15 @@ __device__ __forceinline__ float dot8(const uint4& a, const uint4& b, float acc)
 }
 
 template <bool kBf16>
-__device__ __forceinline__ void mask_bwd_dq_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k,
-                         const CUtensorMap& tm_v, const CUtensorMap& tm_do,
-                         const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const void* __restrict__ o_ptr,
-                         const void* __restrict__ do_ptr, int64_t do_b, int64_t do_h, int64_t do_row, const float* __restrict__ R_ptr,
-                         const float* __restrict__ A_ptr, float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
-                         void* __restrict__ dq_ptr, int H, int Lq, int Lk, int G, float scale, float scale_log2,
-                         const int* __restrict__ plan, int plan_stride, int* status,
-    int t, int bh, uint32_t tmem) {
+__device__ __forceinline__ void mask_bwd_dq_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
+                                                 const CUtensorMap& tm_do, const uint8_t* __restrict__ is_mem,
+                                                 int64_t is_mem_stride, const void* __restrict__ o_ptr,
+                                                 const void* __restrict__ do_ptr, int64_t do_b, int64_t do_h, int64_t do_row,
+                                                 const float* __restrict__ R_ptr, const float* __restrict__ A_ptr,
+                                                 float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
+                                                 void* __restrict__ dq_ptr, int H, int Lq, int Lk, int G, float scale,
+                                                 float scale_log2, const int* __restrict__ plan, int plan_stride, int* status,
+                                                 int t, int bh, uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -623,7 +623,8 @@ __device__ __forceinline__ void mask_bwd_dq_tile(const CUtensorMap& tm_q, const 
     float delta = 0.f;
     {
       const uint4* orow = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(o_ptr) + grow * kD);
-      const uint4* grw = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(do_ptr) + b * do_b + h * do_h + (int64_t)(t * kQT + row) * do_row);
+      const uint4* grw = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(do_ptr) + b * do_b + h * do_h +
+                                                        (int64_t)(t * kQT + row) * do_row);
 #pragma unroll 4
       for (int c = 0; c < kD / 8; ++c) delta = dot8<kBf16>(orow[c], grw[c], delta);
     }
@@ -789,7 +790,8 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       tmem = tmem_slot;
       held = true;
     }
-    mask_bwd_dq_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, o_ptr, do_ptr, do_b, do_h, do_row, R_ptr, A_ptr, delta_ptr, nD_ptr, dq_ptr, H, Lq, Lk, G, scale, scale_log2, plan, plan_stride, status, t, bh, tmem);
+    mask_bwd_dq_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, o_ptr, do_ptr, do_b, do_h, do_row, R_ptr, A_ptr, delta_ptr,
+                            nD_ptr, dq_ptr, H, Lq, Lk, G, scale, scale_log2, plan, plan_stride, status, t, bh, tmem);
   }
   if (held && warp == 5) {
     tc_fence_after();
@@ -820,13 +822,13 @@ struct MkSmem {
 constexpr size_t kMkSmemBytes = 1024 + 32768 + kMkStages * 65536 + 32768 + sizeof(MkSmem);
 
 template <bool kBf16>
-__device__ __forceinline__ void mask_bwd_dkv_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k,
-                          const CUtensorMap& tm_v, const CUtensorMap& tm_do,
-                          const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const float* __restrict__ R_ptr,
-                          const float* __restrict__ A_ptr, const float* __restrict__ delta_ptr,
-                          const float* __restrict__ nD_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                          int H, int Lq, int Lk, int G, float scale, float scale_log2, int* status,
-    int kt, int bh, uint32_t tmem) {
+__device__ __forceinline__ void mask_bwd_dkv_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
+                                                  const CUtensorMap& tm_do, const uint8_t* __restrict__ is_mem,
+                                                  int64_t is_mem_stride, const float* __restrict__ R_ptr,
+                                                  const float* __restrict__ A_ptr, const float* __restrict__ delta_ptr,
+                                                  const float* __restrict__ nD_ptr, void* __restrict__ dk_ptr,
+                                                  void* __restrict__ dv_ptr, int H, int Lq, int Lk, int G, float scale,
+                                                  float scale_log2, int* status, int kt, int bh, uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -1126,7 +1128,8 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                           const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const float* __restrict__ R_ptr,
                           const float* __restrict__ A_ptr, const float* __restrict__ delta_ptr,
                           const float* __restrict__ nD_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                          int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2, const int* __restrict__ plan, int plan_stride, int* status) {
+                          int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2,
+                          const int* __restrict__ plan, int plan_stride, int* status) {
   __shared__ uint32_t tmem_slot;
   const int n_tiles = Lk / kKT;
   const uint32_t warp = threadIdx.x >> 5;
@@ -1152,7 +1155,8 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       tmem = tmem_slot;
       held = true;
     }
-    mask_bwd_dkv_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, R_ptr, A_ptr, delta_ptr, nD_ptr, dk_ptr, dv_ptr, H, Lq, Lk, G, scale, scale_log2, status, kt, bh, tmem);
+    mask_bwd_dkv_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, R_ptr, A_ptr, delta_ptr, nD_ptr, dk_ptr, dv_ptr, H, Lq, Lk,
+                             G, scale, scale_log2, status, kt, bh, tmem);
   }
   if (held && warp == 5) {
     tc_fence_after();

@@ -3,7 +3,8 @@
 // Shape contract: bf16 / fp16, head dim up to 128 (a multiple of 8), landmark block 64, any Lq, Lk - Lq a multiple of 64.
 // Rows past the end of a sequence and features past the head dim are zeros that TMA fills in: no padded copies exist
 // (the copies took 86 of 146 us at Lq = 1999, H = 32, D = 128 and 104 of 237 us at D = 64), and what is computed for them
-// is dropped at the stores.  Head dims up to 64 run instances with half the products.
+// is dropped at the stores.  Head dims up to 64 have forward and dQ instances with half the products; the dK/dV kernel loads and
+// multiplies 128 features whatever the head dim is (56 of 117 us at B4 H16 L1024 D64, half of its products on zeros).
 //
 // Forward, one or two tiles of 128 query rows per CTA; rows 0-63 of a tile belong to landmark block `own0`, rows 64-127 to
 // `own0 + 1`.
@@ -129,6 +130,10 @@ __device__ __forceinline__ float row_sum(const float (&v)[64]) {
 // kernels of attn_mask_sm100.cu: the forward kernel marks them in R, the backward ones find them in the plan.
 constexpr int kIrrMaxTiles = 65;                    // 64 landmarks and the open group
 constexpr int kIrrMaxKeys = 64 * kIrrMaxTiles;
+// The single pass works on 64 columns a group, however short the group is.  Measured (us, forward + backward, single-pass / two-pass
+// kernels): B16 H8 T512, groups of 10 keys 525 / 625, 16 365 / 593, 51 183 / 361; B2 H8 T512, of 10 182 / 209, 51 98 / 122;
+// B16 H8 T256, of 8 258 / 228, 10 219 / 225, 16 159 / 216.  The line (16 keys a group, counted 256 keys longer than the row is) falls
+// at 8 keys for 256 and at 11 for 512: groups of 8 to 11 keys of longer rows would gain from a lower one.
 constexpr int kIrrMinMeanGroup = 16;
 
 struct IrrArgs {

@@ -394,7 +394,8 @@ extern "C" int lmk_block_select(const void* q, const void* landmark_keys, const 
   LMK_CHECK_ARG(q && landmark_keys && desc && (probs || idx), "block_select: null pointer");
   if (!lmk_block_select_supported(D, desc->n_blocks, desc->top_k, dtype) || !vec_aligned(desc))
     return fail(LMK_ERR_UNSUPPORTED, "block_select: 16-bit type, D=128, at most %d blocks, top_k <= 8", kSelMaxN);
-  LMK_CHECK_ARG(rotary >= LMK_ROTARY_NONE && rotary <= LMK_ROTARY_INTERLEAVED && (rotary == LMK_ROTARY_NONE || (cos_table && sin_table && n_pos >= 1)),
+  LMK_CHECK_ARG(rotary >= LMK_ROTARY_NONE && rotary <= LMK_ROTARY_INTERLEAVED &&
+                (rotary == LMK_ROTARY_NONE || (cos_table && sin_table && n_pos >= 1)),
                 "block_select: rotary tables missing");
   LMK_CHECK_ARG(B >= 1 && H >= 1 && T >= 1 && (int64_t)B * H <= 65535, "block_select: bad sizes");
   LMK_CHECK_ARG(idx == nullptr || desc->top_k >= 1, "block_select: indices asked for with top_k = 0");
@@ -433,7 +434,8 @@ extern "C" int lmk_prefix_gather(const void* q, const void* k_cache, const void*
   if (!lmk_prefix_gather_supported(D, kdesc->block, kdesc->top_k, T, tail_len, dtype) || !vec_aligned(kdesc) || !vec_aligned(vdesc))
     return fail(LMK_ERR_UNSUPPORTED, "prefix_gather: 16-bit type, D=128, block and tail <= %d, T <= 8192", kGatherMaxBlk);
   LMK_CHECK_ARG(kdesc->n_blocks >= 1 && kdesc->top_k <= kdesc->n_blocks && kdesc->block == vdesc->block, "prefix_gather: bad descriptor");
-  LMK_CHECK_ARG(rotary >= LMK_ROTARY_NONE && rotary <= LMK_ROTARY_INTERLEAVED && (rotary == LMK_ROTARY_NONE || (cos_table && sin_table && n_pos >= 1)),
+  LMK_CHECK_ARG(rotary >= LMK_ROTARY_NONE && rotary <= LMK_ROTARY_INTERLEAVED &&
+                (rotary == LMK_ROTARY_NONE || (cos_table && sin_table && n_pos >= 1)),
                 "prefix_gather: rotary tables missing");
   LMK_CHECK_ARG(B >= 1 && H >= 1 && (int64_t)B * H <= 65535, "prefix_gather: bad sizes");
   uintptr_t align = (uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos_table | (uintptr_t)sin_table | (uintptr_t)v_out;

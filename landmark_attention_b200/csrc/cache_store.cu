@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(128) cache_store_kernel(const uint4* __restric
 // flavours, forward or inverse (the inverse rotation is the gradient of the forward one).  16-bit types use packed
 // arithmetic with the three roundings of the tensor formulation x * cos + rotate(x) * sin.
 // Bound by HBM (four tensors read or written once): a thread takes the same vector of two heads of both tensors, four loads in
-// flight, and the tables' values once (B16 H8 T512 D128, the whole layer: one head 199.4 us, two 198.1, four 206.6; loads issued one
-// after the other 210).
+// flight, and the tables' values once.  The forward launch on [B, T, 3, H, D] projections, one / two / four heads a thread (us):
+// B16 H8 T512 10.87 / 10.02 / 14.1, T1024 28.4 / 27.1 / 33.8, T255 6.16 / 5.87 / 7.8, B2 H12 T256 2.45 / 2.66 / 3.7.
 constexpr int kRotHeads = 2;
 struct RotParams {
   const void* in[2];
@@ -255,13 +255,11 @@ extern "C" int lmk_cache_store(const void* k_src, const void* v_src, const int64
   return LMK_OK;
 }
 
-static int chunk_prepare(const void* q, const void* k, const void* v, const int64_t q_strides[3],
-                                 const int64_t k_strides[3], const int64_t v_strides[3], const void* cos_table,
-                                 const void* sin_table, int n_pos, int64_t pos0, const uint8_t* chunk_flags, int block,
-                                 void* q_rot, void* q_pad, void* k_pad, void* v_pad, int64_t pad_head,
-                         uint8_t* flags_pad, void* cache_k,
-                                 void* cache_v, const int64_t cache_strides[3], int64_t cache_pos, int B, int H, int T,
-                                 int t_pad, int D, int dtype, void* stream) {
+static int chunk_prepare(const void* q, const void* k, const void* v, const int64_t q_strides[3], const int64_t k_strides[3],
+                         const int64_t v_strides[3], const void* cos_table, const void* sin_table, int n_pos, int64_t pos0,
+                         const uint8_t* chunk_flags, int block, void* q_rot, void* q_pad, void* k_pad, void* v_pad,
+                         int64_t pad_head, uint8_t* flags_pad, void* cache_k, void* cache_v, const int64_t cache_strides[3],
+                         int64_t cache_pos, int B, int H, int T, int t_pad, int D, int dtype, void* stream) {
   using namespace lmk;
   LMK_CHECK_ARG(q && k && v && q_strides && k_strides && v_strides && cos_table && sin_table && q_rot && k_pad,
                 "chunk_prepare: null pointer");
@@ -311,8 +309,8 @@ extern "C" int lmk_chunk_prepare(const void* q, const void* k, const void* v, co
                                  int t_pad, int D, int dtype, void* stream) {
   using namespace lmk;
   LMK_CHECK_ARG(q_pad && v_pad && flags_pad, "chunk_prepare: null pointer");
-  return chunk_prepare(q, k, v, q_strides, k_strides, v_strides, cos_table, sin_table, n_pos, pos0, chunk_flags, block, q_rot, q_pad, k_pad, v_pad,
-                       (int64_t)t_pad * D, flags_pad, cache_k, cache_v, cache_strides, cache_pos, B, H, T, t_pad, D, dtype, stream);
+  return chunk_prepare(q, k, v, q_strides, k_strides, v_strides, cos_table, sin_table, n_pos, pos0, chunk_flags, block, q_rot, q_pad,
+                       k_pad, v_pad, (int64_t)t_pad * D, flags_pad, cache_k, cache_v, cache_strides, cache_pos, B, H, T, t_pad, D, dtype, stream);
 }
 
 extern "C" int lmk_chunk_rotate(const void* q, const void* k, const void* v, const int64_t q_strides[3], const int64_t k_strides[3],

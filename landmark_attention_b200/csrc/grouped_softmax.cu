@@ -850,7 +850,10 @@ __global__ void __launch_bounds__(kGsWarps * 32) grouped_softmax_rows_kernel(GsP
 // Keys are counted from the 4-element boundary at or in front of the row's place in the dense results (`lead` keys earlier),
 // so rows of any length are copied, read and written four elements at a time except for the row's two ends.
 // B16 H8 512 x 512 fp32, landmarks every 51 keys: forward 138 -> 98 us, backward 216 -> 130 us.  Two landmarks in a lane have code of
-// their own (rows of 1064 keys, groups of 32, B2 H32, forward and backward: 994 -> 668 us; by the chunked form 1054).
+// their own (rows of 1064 keys, groups of 32, B2 H32, forward and backward: 994 -> 668 us; by the chunked form 1054).  The chunked form costs
+// more from here than as a kernel of its own: rows in which a lane holds three landmarks and more take 1.1 to 1.4 times as long as when
+// all rows were done that way (forward and backward, us: B2 H8 1024 x 1024 with groups of 8 170 -> 222, B1 H4 2048 x 2048 with groups
+// of 16 221 -> 252, of 8 254 -> 301); whether a row is one of them is only known from its flags.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kLaneMaxPieces = 16;             // n4 of the longest row
 

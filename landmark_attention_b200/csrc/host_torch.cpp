@@ -519,8 +519,11 @@ Tensor vector_rows(const Tensor& t) {
   return ok ? t : t.clone(at::MemoryFormat::Contiguous);
 }
 
-// Behind a cache of whole blocks the generation kernel takes up to this many tokens: more are cheaper as a chunk, whose scores
-// and local attention run on the tensor cores.
+// Behind a cache of whole blocks the generation kernel takes up to this many tokens; more go the chunk's way, whose scores and local
+// attention run on the tensor cores.  Measured on the device (us, generation kernel / chunk kernels, blocks of 64, top 4): 8 heads,
+// 64 blocks, 8 tokens 18.6 / 32.6, 16 35.0 / 33.4, 32 67 / 35; 1024 blocks, 16 39.9 / 35.7; 32 heads, 64 blocks, 4 tokens
+// 35.1 / 33.1, 16 129 / 37; 1024 blocks, 4 39.9 / 58.8, 8 77 / 60, 16 158 / 68.  The line is right for 8 heads; with 32 it lies at
+// 4 to 8 tokens, and between there and 16 the chunk would be up to 3.4 times as fast.
 constexpr int64_t kDecodeMaxWholeBlockTokens = 16;
 
 // One layer of token generation behind `len` cached tokens (lmk_decode_attend): tokens that stay inside the unfinished
@@ -546,7 +549,8 @@ Tensor decode_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, const
     return t.is_contiguous() && t.dim() == 2 && t.size(1) == D && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
   };
   if (!cache_ok(kc) || !cache_ok(vc) || k_.sizes() != q_.sizes() || v_.sizes() != q_.sizes() || !table_ok(cos) ||
-      !table_ok(sin) || B * H > 65535 || T + tail > block || (!tail && T > kDecodeMaxWholeBlockTokens) || kc.size(2) < len + (append ? T : 0) || vc.size(2) < len + (append ? T : 0) ||
+      !table_ok(sin) || B * H > 65535 || T + tail > block || (!tail && T > kDecodeMaxWholeBlockTokens) ||
+      kc.size(2) < len + (append ? T : 0) || vc.size(2) < len + (append ? T : 0) ||
       !lib.lmk_decode_supported(D, block, top_k, len, T, dtype_code(q_)))
     return Tensor();
   c10::cuda::OptionalCUDAGuard guard(q_.device());
@@ -648,7 +652,8 @@ std::tuple<Tensor, Tensor> cache_retrieve(const Tensor& q_, const Tensor& kc, co
 bool prefix_pv(const Tensor& probs, const Tensor& v, const Tensor& y) {
   const auto st = v.scalar_type();
   const auto B = y.size(0), H = y.size(1), T = y.size(2), D = y.size(3), P = v.size(3);
-  if (needs_grad({probs, v}) || !v.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || y.scalar_type() != st || D != 128 || P > 8192 || B * H > 65535 ||
+  if (needs_grad({probs, v}) || !v.is_cuda() || (st != at::kHalf && st != at::kBFloat16) || y.scalar_type() != st || D != 128 ||
+      P > 8192 || B * H > 65535 ||
       P == 0 || !probs.is_contiguous() || !y.is_contiguous() || v.stride(4) != 1 || v.stride(3) != D || v.stride(0) % 8 ||
       v.stride(1) % 8 || v.stride(2) % 8 || (reinterpret_cast<uintptr_t>(v.data_ptr()) & 15))
     return false;
@@ -834,7 +839,8 @@ Tensor per_head_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, con
   if (block < 1 || n < 1 || n > 49152 || top_k < 1 || top_k > 32 || kc.is_cuda() == host || vc.is_cuda() == host ||
       kc.size(2) < n * block + (append ? q_.size(2) : 0) || !chunk_of(&c, q_, k_, v_, kc, vc, cos, sin))
     return Tensor();
-  if (host && (!kc.is_pinned() || !vc.is_pinned() || kc.stride(2) != c.D || lm.scalar_type() != q_.scalar_type() || !rows_ok(lm) || lm.size(2) < n || (append && c.T % block != 0)))
+  if (host && (!kc.is_pinned() || !vc.is_pinned() || kc.stride(2) != c.D || lm.scalar_type() != q_.scalar_type() || !rows_ok(lm) ||
+               lm.size(2) < n || (append && c.T % block != 0)))
     return Tensor();
   c10::cuda::OptionalCUDAGuard guard(q_.device());
   const lmk_cache_desc d = rows_desc(kc, n, block, top_k);
@@ -867,7 +873,8 @@ Tensor per_head_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, con
   }
   const bool device_append = append && !host;
   const int64_t P = top_k * block, W = P + c.T;
-  Tensor qr = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q), keys = empty_like_dtype({c.B, c.H, W, c.D}, c.q), vals = empty_like_dtype({c.B, c.H, W, c.D}, c.q);
+  Tensor qr = empty_like_dtype({c.B, c.H, c.T, c.D}, c.q);
+  Tensor keys = empty_like_dtype({c.B, c.H, W, c.D}, c.q), vals = empty_like_dtype({c.B, c.H, W, c.D}, c.q);
   auto behind = [&](const Tensor& t) { return static_cast<uint16_t*>(t.data_ptr()) + P * c.D; };
   check(lib.lmk_chunk_rotate(c.q.data_ptr(), c.k.data_ptr(), c.v.data_ptr(), S3(c.q).v, S3(c.k).v, S3(c.v).v, cos.data_ptr(),
                              sin.data_ptr(), cos.size(0), n * block, qr.data_ptr(), behind(keys), behind(vals), W * c.D,
@@ -875,7 +882,8 @@ Tensor per_head_attend(const Tensor& q_, const Tensor& k_, const Tensor& v_, con
                              device_append ? S3(kc).v : nullptr, n * block, c.B, c.H, c.T, c.D, c.code, c.stream), "lmk_chunk_rotate");
   const Tensor probs = landmark_scores(c, qr, host ? lm : kc, ld, cos, sin, true);
   Tensor idx = at::empty({c.B, c.H, 1, top_k}, c.q.options().requires_grad(false).dtype(at::kInt));
-  check(lib.lmk_topk_sorted(probs.data_ptr<float>(), idx.data_ptr<int>(), c.B * c.H, 1, c.T * n, 0, c.T, n, n, top_k, 0, c.stream), "lmk_topk_sorted");
+  check(lib.lmk_topk_sorted(probs.data_ptr<float>(), idx.data_ptr<int>(), c.B * c.H, 1, c.T * n, 0, c.T, n, n, top_k, 0, c.stream),
+        "lmk_topk_sorted");
   check(lib.lmk_gather_kv_to(kc.data_ptr(), vc.data_ptr(), &d, &d, idx.data_ptr<int>(), cos.data_ptr(), sin.data_ptr(), cos.size(0), LMK_ROTARY_HALF,
                              keys.data_ptr(), vals.data_ptr(), W * c.D, c.B, c.H, 1, c.D, c.code, c.stream), "lmk_gather_kv");
   Tensor stats;

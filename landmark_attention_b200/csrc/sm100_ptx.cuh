@@ -239,9 +239,9 @@ __device__ __forceinline__ float ex2(float x) {
 
 // exp2 of two values on the FMA and integer pipes instead of the special-function unit: round to the nearest integer
 // n with the 1.5 * 2^23 trick, evaluate a cubic for 2^(x - n) on [-0.5, 0.5] (relative error 7.5e-5, well below one
-// bf16 / fp16 rounding step of the 16-bit weights it feeds) and add n to the exponent field.  The forward softmax
-// threads are bound by the special-function unit (16 results per clock per SM), so a share of their exponentials
-// goes this way.  Inputs are clamped to >= -126 (results below 2^-126 are not needed).
+// bf16 / fp16 rounding step of the 16-bit weights it feeds) and add n to the exponent field.  The forward's softmax threads
+// take a small share of their exponentials this way (kFwdPolyEvery: the special-function unit is not what they wait for).  Inputs are
+// clamped to >= -126 (results below 2^-126 are not needed).
 __device__ __forceinline__ uint64_t ex2_poly2(uint64_t x) {
   float a, b;
   upk2(x, a, b);

@@ -1,5 +1,5 @@
 """Token generation in one launch (lmk_decode_attend) against the gathered route of the same call: edges of the 16-row items
-and of the 32-row score slices, a query that is a landmark, whole-block caches, one to sixteen tokens, both cluster sizes."""
+and of the 16 landmarks that a warp scores at a time, a query that is a landmark, whole-block caches, one to sixteen tokens, both cluster sizes."""
 import pytest
 import torch
 

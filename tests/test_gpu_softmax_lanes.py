@@ -1,6 +1,6 @@
-"""Grouped softmax rows whose landmarks lie further apart than one lane's keys: registers hold the row, one segmented
-scan reduces all groups.  Edges: row lengths around the pieces of 4, 128 and 512 keys, landmarks on the first and last
-key of a lane, rows with no landmark, rows that fall back because two landmarks share a lane, unaligned rows."""
+"""Grouped softmax rows with at most two landmarks in one lane's keys: shared memory holds the row, one segmented scan a pass
+reduces all groups.  Edges: row lengths around the pieces of 4, 128 and 512 keys, landmarks on the first and last key of a
+lane, rows with no landmark, two landmarks in a lane, rows that fall back because three share one, unaligned rows."""
 import pytest
 import torch
 
