@@ -288,7 +288,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   auto v_slot = [&](int s) { return base + kTiles * 32768u + (uint32_t)s * 32768u + 16384u; };
   Fwd2Smem<kStages>* sm = reinterpret_cast<Fwd2Smem<kStages>*>(smem_raw + (base - raw) + (kTiles + kStages) * 32768u);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int t_a = ((int)gridDim.y - 1 - (int)blockIdx.y) * kTiles;      // heaviest tiles first, across all heads
   const bool has_b = kTiles == 2 && (t_a + 1) * kQTile < Lq;            // the second tile has at least one row
   const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
@@ -309,8 +309,8 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   auto end_of = [&](int n) { return irr.flags != nullptr ? (n < 0 ? -1 : tab->ends[n]) : (n + 1) * irr.block - 1; };
   const int own0_a = prefix_blocks + 2 * t_a;           // tile A: blocks own0_a, own0_a+1; tile B: +2, +3
   // newest tile that any row of tile A / of the CTA sees
-  const int last_a = kIrr ? group_of(min(pos_a + kQTile, Lk) - 1) : own0_a + 1;
-  const int n_last = kIrr ? group_of(min(pos_a + (has_b ? 2 : 1) * kQTile, Lk) - 1)
+  const int last_a = kIrr ? warp_uniform(group_of(min(pos_a + kQTile, Lk) - 1)) : own0_a + 1;
+  const int n_last = kIrr ? warp_uniform(group_of(min(pos_a + (has_b ? 2 : 1) * kQTile, Lk) - 1))
                           : min(own0_a + (has_b ? 3 : 1), (Lk - 1) / kBlk);
   const int n_lm_tiles = (n_last + 63) / 64;            // landmarks 0 .. n_last-1
   const int total = n_lm_tiles + n_last + 1;
@@ -337,7 +337,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = sm->tmem_base;
+  const uint32_t tmem = (uint32_t)warp_uniform((int)sm->tmem_base);
   auto tmem_s = [&](int w, int sb) { return tmem + (uint32_t)(w * 128 + sb * 64); };
   auto tmem_o = [&](int w) { return tmem + kTiles * 128u + (uint32_t)w * 128u; };
   if constexpr (!kIrr) grid_dep_wait();      // only the set-up may overlap the kernel in front (see the launch; kIrr: above)
@@ -378,9 +378,9 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     __syncwarp();
   } else if (warp == kSw + 1) {
     // ------------------------------------------------------------------ MMA issuer 1: S = Q K^T
-    // Two issuer threads keep the scalar bookkeeping between tcgen05.mma instructions short, and the S MMAs of the
-    // next key block never queue behind a wait for the softmax of the current one.
-    if (lane == 0) {
+    // A second issuing warp takes the P V products: the S products of the next key block never queue behind a wait for the
+    // softmax of the current one.
+    {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
       constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 64, 0, 0);
       mbar_wait(smem_u32(&sm->q_full), 0, &g_lmk_status, kErrFwd2Mma);
@@ -399,11 +399,13 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           if (k >= 2) mbar_wait(smem_u32(&sm->s_free[w][sb]), ((k >> 1) & 1) ^ 1, &g_lmk_status, kErrFwd2Mma);
           tc_fence_after();
           const uint64_t dq = desc_advance(dq0, (uint32_t)w * 32768u);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kD / 16; ++kk)
-            mma_f16_ss(tmem_s(w, sb), desc_advance(dq, kmajor_step(kk, kTileBytes)),
-                       desc_advance(dk, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
-          mma_commit(smem_u32(&sm->s_full[w][sb]));
+            for (int kk = 0; kk < kD / 16; ++kk)
+              mma_f16_ss(tmem_s(w, sb), desc_advance(dq, kmajor_step(kk, kTileBytes)),
+                         desc_advance(dk, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
+            mma_commit(smem_u32(&sm->s_full[w][sb]));
+          }
         }
         if (++s == kStages) { s = 0; ph ^= 1; }
       }
@@ -411,7 +413,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     __syncwarp();
   } else if (warp == kSw + 2) {
     // ------------------------------------------------------------------ MMA issuer 2: O += P V
-    if (lane == 0) {
+    {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
       constexpr uint32_t idesc_o = instr_desc_f16(fmt, 128, kD, 0, 1);
       const uint64_t dv0 = smem_desc_sw128(v_slot(0), kHalfTile, 1024);
@@ -430,19 +432,21 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             // A = P straight from TMEM: the softmax threads wrote it over the first 32 columns of the S buffer it was
             // computed from (8 columns = 16 keys per K-step)
             const uint32_t tp = tmem_s(w, k & 1);
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kBlk / 16; ++kk)
-              mma_f16_ts(tmem_o(w), tp + kk * 8, desc_advance(dv, kk * 2048), idesc_o,
-                         (o_started[w] || kk > 0) ? 1u : 0u);
+              for (int kk = 0; kk < kBlk / 16; ++kk)
+                mma_f16_ts(tmem_o(w), tp + kk * 8, desc_advance(dv, kk * 2048), idesc_o,
+                           (o_started[w] || kk > 0) ? 1u : 0u);
+            }
             o_started[w] = true;
           }
-          mma_commit(smem_u32(&sm->s_free[w][k & 1]));      // the S / P buffer may take the next S product
+          if (elect_one()) mma_commit(smem_u32(&sm->s_free[w][k & 1]));      // the S / P buffer may take the next S product
         }
         // the stage is free once both P V products are done; each of them waited for its S product to be read
-        mma_commit(smem_u32(&sm->empty[s]));
+        if (elect_one()) mma_commit(smem_u32(&sm->empty[s]));
         if (++s == kStages) s = 0;
       }
-      mma_commit(smem_u32(&sm->o_full));
+      if (elect_one()) mma_commit(smem_u32(&sm->o_full));
     }
     __syncwarp();
   } else {
@@ -879,7 +883,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const uint32_t ds_tile = p_tile + 16384u;
   DkvSmem* sm = reinterpret_cast<DkvSmem*>(smem_raw + (base - raw) + 65536u + kDkvStages * 65536u + 32768u);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int prefix_blocks = (Lk - Lq) / kBlk;
   const int n_tiles = (Lq + kQTile - 1) / kQTile;
   const int n_blocks = (Lk + kBlk - 1) / kBlk;
@@ -933,7 +937,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = sm->tmem_base;
+  const uint32_t tmem = (uint32_t)warp_uniform((int)sm->tmem_base);
   auto tmem_s = [&](int g) { return tmem + (uint32_t)g * 64u; };
   auto tmem_dp = [&](int g) { return tmem + 128u + (uint32_t)g * 64u; };
   auto tmem_dv = [&](int g) { return tmem + 256u + (uint32_t)g * 128u; };
@@ -980,15 +984,15 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // S = Q K^T and dP = dO V^T for both blocks of the pair at once (N = 128: full-rate MMAs), one query tile at a
     // time.  S has its own full / free barriers: the warpgroups hold S in registers early in an item, so the next S
     // product runs while they are still busy with dP.
-    if (lane == 0) {
+    {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
       constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 128, 0, 0);
       const uint64_t dk0 = smem_desc_sw128(k_pair, 16, 1024), dv0 = smem_desc_sw128(v_pair, 16, 1024);
       const uint64_t dq0 = smem_desc_sw128(q_slot(0), 16, 1024), ddo0 = smem_desc_sw128(do_slot(0), 16, 1024);
       int it = 0, u = 0;
       for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-        if (skipped(w)) continue;
-        const int n_items = n_tiles - unit_tq0(w);
+        if (warp_uniform(skipped(w))) continue;
+        const int n_items = n_tiles - warp_uniform(unit_tq0(w));
         mbar_wait(smem_u32(&sm->kv_full), u & 1, &g_lmk_status, kErrDkvMma);
         for (int i = 0; i < n_items; ++i, ++it) {
           const int s = it % kDkvStages;
@@ -996,20 +1000,24 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const uint64_t dq = desc_advance(dq0, (uint32_t)s * 65536u), ddo = desc_advance(ddo0, (uint32_t)s * 65536u);
           if (it >= 1) mbar_wait(smem_u32(&sm->s_free), (it & 1) ^ 1, &g_lmk_status, kErrDkvMma);
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kD / 16; ++kk)
-            mma_f16_ss(tmem_s(0), desc_advance(dq, kmajor_step(kk, kTileBytes)),
-                       desc_advance(dk0, kmajor_step(kk, kTileBytes)), idesc_s, kk > 0);
-          mma_commit(smem_u32(&sm->s_full));
+            for (int kk = 0; kk < kD / 16; ++kk)
+              mma_f16_ss(tmem_s(0), desc_advance(dq, kmajor_step(kk, kTileBytes)),
+                         desc_advance(dk0, kmajor_step(kk, kTileBytes)), idesc_s, kk > 0);
+            mma_commit(smem_u32(&sm->s_full));
+          }
           if (it >= 1) mbar_wait(smem_u32(&sm->dp_free), (it & 1) ^ 1, &g_lmk_status, kErrDkvMma);
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kD / 16; ++kk)
-            mma_f16_ss(tmem_dp(0), desc_advance(ddo, kmajor_step(kk, kTileBytes)),
-                       desc_advance(dv0, kmajor_step(kk, kTileBytes)), idesc_s, kk > 0);
-          mma_commit(smem_u32(&sm->dp_full));
+            for (int kk = 0; kk < kD / 16; ++kk)
+              mma_f16_ss(tmem_dp(0), desc_advance(ddo, kmajor_step(kk, kTileBytes)),
+                         desc_advance(dv0, kmajor_step(kk, kTileBytes)), idesc_s, kk > 0);
+            mma_commit(smem_u32(&sm->dp_full));
+          }
         }
-        mma_commit(smem_u32(&sm->kv_empty));      // K / V tiles may be replaced once these products are done
+        if (elect_one()) mma_commit(smem_u32(&sm->kv_empty));      // K / V tiles may be replaced once these products are done
         ++u;
       }
     }
@@ -1018,7 +1026,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // dV_g^T += dO^T P and dK_g^T += Q^T dS.  A = dO^T / Q^T: MN-major view of the row-major [128 q x 128 d] tile (second
     // 64-feature half 16 KB further); B = P / dS: MN-major view of the [128 q x 64 k] tile; a K-step is 16 query rows
     // = 2048 bytes.
-    if (lane == 0) {
+    {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
       constexpr uint32_t idesc_t = instr_desc_f16(fmt, 128, 64, 1, 1);
       const uint64_t dq0t = smem_desc_sw128(q_slot(0), kTileBytes, 1024);
@@ -1026,8 +1034,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const uint64_t dpt = smem_desc_sw128(p_tile, 16, 1024), ddst = smem_desc_sw128(ds_tile, 16, 1024);
       int it = 0, u = 0;
       for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-        if (skipped(w)) continue;
-        const int n_items = n_tiles - unit_tq0(w);
+        if (warp_uniform(skipped(w))) continue;
+        const int n_items = n_tiles - warp_uniform(unit_tq0(w));
         for (int i = 0; i < n_items; ++i, ++it) {
           const int s = it % kDkvStages;
           const uint64_t ddot = desc_advance(ddo0t, (uint32_t)s * 65536u), dqt = desc_advance(dq0t, (uint32_t)s * 65536u);
@@ -1037,23 +1045,29 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             mbar_wait(smem_u32(&sm->p_ready), g, &g_lmk_status, kErrDkvMma);
             if (i == 0) mbar_wait(smem_u32(&sm->acc_empty[g]), (u & 1) ^ 1, &g_lmk_status, kErrDkvMma);
             tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kQTile / 16; ++kk)
-              mma_f16_ss(tmem_dv(g), desc_advance(ddot, kk * 2048), desc_advance(dpt, kk * 2048), idesc_t,
-                         (i > 0 || kk > 0) ? 1u : 0u);
-            mma_commit(smem_u32(&sm->p_free[g]));
+              for (int kk = 0; kk < kQTile / 16; ++kk)
+                mma_f16_ss(tmem_dv(g), desc_advance(ddot, kk * 2048), desc_advance(dpt, kk * 2048), idesc_t,
+                           (i > 0 || kk > 0) ? 1u : 0u);
+              mma_commit(smem_u32(&sm->p_free[g]));
+            }
             mbar_wait(smem_u32(&sm->ds_ready), g, &g_lmk_status, kErrDkvMma);
             tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kQTile / 16; ++kk)
-              mma_f16_ss(tmem_dk(g), desc_advance(dqt, kk * 2048), desc_advance(ddst, kk * 2048), idesc_t,
-                         (i > 0 || kk > 0) ? 1u : 0u);
-            mma_commit(smem_u32(&sm->ds_free[g]));
+              for (int kk = 0; kk < kQTile / 16; ++kk)
+                mma_f16_ss(tmem_dk(g), desc_advance(dqt, kk * 2048), desc_advance(ddst, kk * 2048), idesc_t,
+                           (i > 0 || kk > 0) ? 1u : 0u);
+              mma_commit(smem_u32(&sm->ds_free[g]));
+            }
           }
-          mma_commit(smem_u32(&sm->empty[s]));
+          if (elect_one()) mma_commit(smem_u32(&sm->empty[s]));
         }
-        mma_commit(smem_u32(&sm->acc_full[0]));
-        mma_commit(smem_u32(&sm->acc_full[1]));
+        if (elect_one()) {
+          mma_commit(smem_u32(&sm->acc_full[0]));
+          mma_commit(smem_u32(&sm->acc_full[1]));
+        }
         ++u;
       }
     }
@@ -1174,10 +1188,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
 // ---------------------------------------------------------------------------------------------- backward: dQ
 constexpr int kDqStages = 4;
-// The dQ kernel has a fourth single-thread role: S = Q K^T and dP = dO V^T are issued by two different threads.  With
-// the A operand in TMEM an N = 64 product needs only 32 clk of the tensor pipe, but one thread cannot issue such
-// instructions faster than one per ~45 clk; two issuers together reach the pipe's rate (measured with an issue-rate
-// microbenchmark: 44.7 clk per instruction from one thread, 32 clk per instruction from two).
+// The dQ kernel has a fourth role: S = Q K^T and dP = dO V^T are issued by two different warps, so that neither waits behind the
+// other one's buffer.
 constexpr int kDqThreads = kBwdThreads + 32;
 
 struct DqSmem {
@@ -1188,8 +1200,10 @@ struct DqSmem {
   uint64_t full[kDqStages];
   uint64_t empty[kDqStages];
   uint64_t ds_ready[kDqStages];
-  uint64_t sdp_full[kSdpBufs];
-  uint64_t sdp_free[kSdpBufs];
+  uint64_t s_full[kSdpBufs];       // S and dP are handed over separately: the next S product of a buffer runs while its
+  uint64_t s_free[kSdpBufs];       // warpgroup is still busy with dP
+  uint64_t dp_full[kSdpBufs];
+  uint64_t dp_free[kSdpBufs];
   uint64_t acc_full[2];     // per draining warpgroup (the one that took the unit's last item)
   uint64_t acc_empty;
   uint32_t tmem_base;
@@ -1216,7 +1230,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const uint32_t o_tile = base + 65536u + kDqStages * 32768u;      // forward output tile, only for delta
   DqSmem* sm = reinterpret_cast<DqSmem*>(smem_raw + (base - raw) + 65536u + kDqStages * 32768u + 32768u);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int n_tiles = (Lq + kQTile - 1) / kQTile;
   const int n_blocks = (Lk + kBlk - 1) / kBlk;
   const int prefix_blocks = (Lk - Lq) / kBlk;
@@ -1250,8 +1264,10 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       mbar_init(smem_u32(&sm->ds_ready[s]), 128);
     }
     for (int s = 0; s < kSdpBufs; ++s) {
-      mbar_init(smem_u32(&sm->sdp_full[s]), 2);     // S product done + dP product done
-      mbar_init(smem_u32(&sm->sdp_free[s]), 128);
+      mbar_init(smem_u32(&sm->s_full[s]), 1);
+      mbar_init(smem_u32(&sm->s_free[s]), 128);
+      mbar_init(smem_u32(&sm->dp_full[s]), 1);
+      mbar_init(smem_u32(&sm->dp_free[s]), 128);
     }
     mbar_init(smem_u32(&sm->acc_full[0]), 1);
     mbar_init(smem_u32(&sm->acc_full[1]), 1);
@@ -1262,7 +1278,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = sm->tmem_base;
+  const uint32_t tmem = (uint32_t)warp_uniform((int)sm->tmem_base);
   // TMEM: S buffers [0,128), dP buffers [128,256), dQ [256,384), Q rows [384,448), dO rows [448,512).  Q and dO are the
   // A operands of S = Q K^T and dP = dO V^T for every key block of the unit: held in TMEM they are not re-read from
   // shared memory 2 x 32 KB per block (half of the kernel's shared-memory operand traffic), and their shared-memory
@@ -1313,8 +1329,8 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     __syncwarp();
   } else if (warp == kBwdGroups * 4 + 1 || warp == kBwdGroups * 4 + 3) {
     // warp +1 issues S = Q K^T, warp +3 issues dP = dO V^T; both walk through the same items and wait for the same
-    // barriers (each is a waiter of its own on full / sdp_free / ops_ready and sees every phase)
-    if (lane == 0) {
+    // barriers (each is a waiter of its own on full / ops_ready and sees every phase)
+    {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
       constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 64, 0, 0);
       const bool is_s = warp == kBwdGroups * 4 + 1;
@@ -1322,49 +1338,53 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const uint32_t t_out = is_s ? tmem_s : tmem_dp, t_a = is_s ? tmem_q : tmem_do;
       int it = 0, u = 0;
       for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-        if (skipped(w)) continue;
-        const int total = unit_items(w);
+        if (warp_uniform(skipped(w))) continue;
+        const int total = warp_uniform(unit_items(w));
         mbar_wait(smem_u32(&sm->ops_ready), u & 1, &g_lmk_status, kErrDqMma);
         for (int i = 0; i < total; ++i, ++it) {
           const int s = it % kDqStages, sb = it % kSdpBufs;
           mbar_wait(smem_u32(&sm->full[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
           if (it >= kSdpBufs)
-            mbar_wait(smem_u32(&sm->sdp_free[sb]), ((it / kSdpBufs) & 1) ^ 1, &g_lmk_status, kErrDqMma);
+            mbar_wait(smem_u32(is_s ? &sm->s_free[sb] : &sm->dp_free[sb]), ((it / kSdpBufs) & 1) ^ 1, &g_lmk_status, kErrDqMma);
           tc_fence_after();
           const uint64_t db = desc_advance(db0, (uint32_t)s * 32768u);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kD / 16; ++kk)      // A from TMEM: 8 columns = 16 features per K-step
-            mma_f16_ts(t_out + sb * 64, t_a + kk * 8, desc_advance(db, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
-          mma_commit(smem_u32(&sm->sdp_full[sb]));
+            for (int kk = 0; kk < kD / 16; ++kk)      // A from TMEM: 8 columns = 16 features per K-step
+              mma_f16_ts(t_out + sb * 64, t_a + kk * 8, desc_advance(db, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
+            mma_commit(smem_u32(is_s ? &sm->s_full[sb] : &sm->dp_full[sb]));
+          }
         }
-        mma_commit(smem_u32(&sm->ops_free));        // the next unit's Q / dO rows may be written
+        if (elect_one()) mma_commit(smem_u32(&sm->ops_free));        // the next unit's Q / dO rows may be written
         ++u;
       }
     }
     __syncwarp();
   } else if (warp == kBwdGroups * 4 + 2) {
-    if (lane == 0) {
+    {
       constexpr uint32_t fmt = kBf16 ? 1u : 0u;
       constexpr uint32_t idesc_q = instr_desc_f16(fmt, 128, kD, 0, 1);   // dQ += dS K  (K is MN-major)
       const uint64_t dv0 = smem_desc_sw128(v_slot(0), 16, 1024);
       const uint64_t dk0t = smem_desc_sw128(k_slot(0), kHalfTile, 1024);
       int it = 0, u = 0;
       for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-        if (skipped(w)) continue;
-        const int total = unit_items(w);
+        if (warp_uniform(skipped(w))) continue;
+        const int total = warp_uniform(unit_items(w));
         for (int i = 0; i < total; ++i, ++it) {
           const int s = it % kDqStages;
           mbar_wait(smem_u32(&sm->ds_ready[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
           if (i == 0) mbar_wait(smem_u32(&sm->acc_empty), (u & 1) ^ 1, &g_lmk_status, kErrDqMma);
           tc_fence_after();
           const uint64_t dds = desc_advance(dv0, (uint32_t)s * 32768u), dkt = desc_advance(dk0t, (uint32_t)s * 32768u);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kBlk / 16; ++kk)
-            mma_f16_ss(tmem_dq, desc_advance(dds, kk * 32), desc_advance(dkt, kk * 2048), idesc_q,
-                       (i > 0 || kk > 0) ? 1u : 0u);
-          mma_commit(smem_u32(&sm->empty[s]));
+            for (int kk = 0; kk < kBlk / 16; ++kk)
+              mma_f16_ss(tmem_dq, desc_advance(dds, kk * 32), desc_advance(dkt, kk * 2048), idesc_q,
+                         (i > 0 || kk > 0) ? 1u : 0u);
+            mma_commit(smem_u32(&sm->empty[s]));
+          }
         }
-        mma_commit(smem_u32(&sm->acc_full[(it - 1) & 1]));     // drained by the warpgroup that took the last item
+        if (elect_one()) mma_commit(smem_u32(&sm->acc_full[(it - 1) & 1]));     // drained by the warpgroup that took the last item
         ++u;
       }
     }
@@ -1494,15 +1514,23 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int it = it0 + i;
         const int s = it % kDqStages, sb = it % kSdpBufs;
         const int n = n_last - i;
-        mbar_wait(smem_u32(&sm->sdp_full[sb]), (it / kSdpBufs) & 1, &g_lmk_status, kErrDqSoftmax);
+        mbar_wait(smem_u32(&sm->s_full[sb]), (it / kSdpBufs) & 1, &g_lmk_status, kErrDqSoftmax);
         tc_fence_after();
         const int kind = n > own ? 0 : (n == own ? 1 : 2);
         const int c_now = c0;
         if (kIrr) c0 = first_col(n - kBwdGroups);
         // dS replaces the V tile of this stage, which dP = dO V^T has finished reading
         bwd_item<kBf16, false, kIrr>(c_now, tmem_s + sb * 64 + lane_base, tmem_dp + sb * 64 + lane_base,
-                               smem_u32(&sm->sdp_free[sb]), kind, vis, scale_log2, scale, M2L, delta, 0u,
-                               v_slot(s), row, []() {});
+                               smem_u32(&sm->dp_free[sb]), kind, vis, scale_log2, scale, M2L, delta, 0u,
+                               v_slot(s), row, []() {},
+                               [&]() {
+                                 tc_fence_before();
+                                 mbar_arrive(smem_u32(&sm->s_free[sb]));
+                               },
+                               [&]() {
+                                 mbar_wait(smem_u32(&sm->dp_full[sb]), (it / kSdpBufs) & 1, &g_lmk_status, kErrDqSoftmax);
+                                 tc_fence_after();
+                               });
         fence_proxy_async_smem();
         mbar_arrive(smem_u32(&sm->ds_ready[s]));
       }

@@ -107,6 +107,22 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// True in one lane of a converged warp, always the same one.  A warp that issues MMAs runs its loops with all lanes and lets this
+// lane issue: descriptors, TMEM addresses and loop state are then warp-uniform and stay in uniform registers, where an `if (lane
+// == 0)` around the loops moves each of them there for every instruction.  Eight products of the dQ kernel take 162 clk to
+// issue instead of 608 (clock stamps, L = 8192).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(elected));
+  return elected != 0;
+}
+// a value that all lanes hold, as one that the compiler knows to be warp-uniform
+__device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 // D[tmem] (+)= A[smem desc] * B[smem desc]; 16-bit inputs, fp32 accumulate
 __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                            uint32_t accumulate) {
@@ -180,9 +196,9 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lbo_
   return d;
 }
 
-// The MMA issuer is ONE thread: every ALU instruction it executes between two tcgen05.mma costs a full dependent-issue
-// latency.  Descriptors are therefore built once per tile and advanced by adding a constant to the 14-bit address
-// field (shared-memory addresses are below 256 KB, so the add never carries out of the field).
+// ONE thread issues the MMAs, and what it executes between two tcgen05.mma is not hidden by anything.  Descriptors are
+// therefore built once per tile and advanced by adding a constant to the 14-bit address field (shared-memory addresses
+// are below 256 KB, so the add never carries out of the field).
 __device__ __forceinline__ uint64_t desc_advance(uint64_t desc, uint32_t byte_offset) {
   return desc + (uint64_t)(byte_offset >> 4);
 }
