@@ -3,8 +3,7 @@
 // Shape contract: bf16 / fp16, head dim up to 128 (a multiple of 8), landmark block 64, any Lq, Lk - Lq a multiple of 64.
 // Rows past the end of a sequence and features past the head dim are zeros that TMA fills in: no padded copies exist
 // (the copies took 86 of 146 us at Lq = 1999, H = 32, D = 128 and 104 of 237 us at D = 64), and what is computed for them
-// is dropped at the stores.  Head dims up to 64 have forward and dQ instances with half the products; the dK/dV kernel loads and
-// multiplies 128 features whatever the head dim is (56 of 117 us at B4 H16 L1024 D64, half of its products on zeros).
+// is dropped at the stores.  Head dims up to 64 have instances with half the products.
 //
 // Forward, one or two tiles of 128 query rows per CTA; rows 0-63 of a tile belong to landmark block `own0`, rows 64-127 to
 // `own0 + 1`.
@@ -26,9 +25,8 @@
 //      dQ += dS K with K as an MN-major operand.  Two softmax warpgroups take alternate blocks.
 //   b. dK/dV (sm100_bwd_dkv_kernel): persistent; a unit is a pair of adjacent key blocks of one head, held in shared
 //      memory while the query tiles that see them stream through.  Per tile: S, dP of both blocks into TMEM (N = 128);
-//      the softmax threads rebuild P and dS (bf16, [128 q x 64 k] swizzled tiles); dV^T += dO^T P and dK^T += Q^T dS accumulate
-//      TRANSPOSED ([128 features x 64 keys], M = 128) so that every MMA keeps the full 128-lane shape; dO, Q, P and dS
-//      are consumed as MN-major operands from their row-major tiles.
+//      the softmax threads rebuild P and dS (16 bits, [128 q x 64 k] swizzled tiles); dV += P^T dO and dK += dS^T Q with the
+//      pair's 128 keys as M; P, dS, dO and Q are consumed as MN-major operands from their row-major tiles.
 //   Per tile pair: earlier block  dS_j = g s_j (dP_j - nD) scale,  dS_landmark = g (nD - delta) scale,  P_j = g s_j,
 //   with s = softmax inside the block, g = exp(l_n - M) / L, nD = sum_j s_j dP_j;  own block: p = exp(S - M) / L,
 //   dS = p (dP - delta) scale.                                                                      (:152-305)
@@ -620,25 +618,12 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 // ---------------------------------------------------------------------------------------------- backward
 // One (query row, key block) pair of the backward pass, in packed fp32 pairs and within 168 registers per thread (so
-// that two softmax warpgroups fit next to the three single-thread roles).
+// that two softmax warpgroups fit next to the issuing warps).
 //   kind 0: block after the row's own block -> zeros;  kind 1: own block (causal, landmark hidden);
 //   kind 2: earlier block (grouped).
-// Writes the P row (kNeedP) into p_dst and the dS row into ds_dst ([128 x 64] 128B-swizzled tiles), arrives on
-// `free_bar` once the TMEM buffer has been read for the last time, and calls wait_dst() before the first store.
 // one in this many pairs of exponentials uses ex2_poly2 (measured: 3 % faster than "never" at L = 8192, equal at 2048)
 constexpr int kBwdPolyEvery = 4;
 
-struct NoHook {
-  __device__ __forceinline__ void operator()() const {}
-};
-
-// packed (bf16 or f16) pair -> packed fp32 pair
-template <bool kBf16>
-__device__ __forceinline__ uint64_t unpack2(uint32_t w) {
-  if (kBf16) return pk2u(w << 16, w & 0xffff0000u);
-  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
-  return pk2(f.x, f.y);
-}
 template <bool kBf16>
 __device__ __forceinline__ uint32_t pack2p(uint64_t v) {
   float lo, hi;
@@ -649,17 +634,16 @@ __device__ __forceinline__ uint32_t pack2p(uint64_t v) {
 // With kIrr the rows of a warp can be of different kinds (groups end anywhere).  The TMEM accesses have to be executed by all lanes
 // of a warp together, so nothing branches on `kind` there: mixed warps take one masked pass with per-row limits and shifts.
 // M2L = (row max + log(row sum)) * log2(e): exp2(s * c - M2L) is the outer-softmax probability.
-// S and dP are each read from TMEM once and held as packed pairs; dP's buffer is released (free_bar) as soon as it is
-// in registers, before the reductions, so the next dP product can start early.
-template <bool kBf16, bool kNeedP, bool kIrr, typename WaitFn, typename AfterSFn = NoHook, typename BeforeDpFn = NoHook,
-          typename BetweenFn = NoHook>
-__device__ __forceinline__ void bwd_item(int c0, uint32_t ts, uint32_t tdp, uint32_t free_bar, int kind, int vis, float c,
-                                         float scale, float M2L, float delta, uint32_t p_dst, uint32_t ds_dst, int row,
-                                         WaitFn wait_dst, AfterSFn after_s = AfterSFn(),
-                                         BeforeDpFn before_dp = BeforeDpFn(),
-                                         BetweenFn between_stores = BetweenFn()) {
-  uint64_t sp[32];      // the row as packed pairs: S, then P
-  uint64_t dp[32];      // dP, then dS
+//
+// bwd_weights: reads S from TMEM once and leaves the row's weights in sp (packed pairs) up to the row factor w: P = w * sp.
+struct RowFactors {
+  float rden = 0.f;       // grouped rows: 1 / sum of the in-block exponentials
+  float g = 0.f;          // grouped rows: the landmark's outer-softmax probability
+  float w = 1.f;          // g * rden, or 1 where sp holds probabilities
+};
+template <bool kIrr, typename AfterFn>
+__device__ __forceinline__ RowFactors bwd_weights(uint64_t (&sp)[32], int c0, uint32_t ts, int kind, int vis, float c, float M2L,
+                                                  AfterFn after_s) {
   float nmx = 0.f, lm2 = 0.f;
   if (kIrr) __syncwarp();
   {
@@ -697,8 +681,8 @@ __device__ __forceinline__ void bwd_item(int c0, uint32_t ts, uint32_t tdp, uint
       sp[16 + j] = pk2u(rb[2 * j], rb[2 * j + 1]);
     }
   }
-  after_s();      // S is in registers: a caller with separate S / dP buffers releases the S buffer here
-  float sub = delta, lm_ds = 0.f, pscale = 1.f;
+  after_s();      // S is in registers: its buffer may take the next product
+  RowFactors f;
   const uint64_t c2 = pk2(c, c);
   uint64_t s0 = 0ull, s1 = 0ull, s2 = 0ull, s3 = 0ull;
   // all rows of the warp are of kind 2 and the group has keys (votes: the branches below are taken by whole warps)
@@ -750,7 +734,22 @@ __device__ __forceinline__ void bwd_item(int c0, uint32_t ts, uint32_t tdp, uint
       s3 = add2(s3, sp[j + 3]);
     }
   }
-  before_dp();    // a caller with separate S / dP buffers waits for dP only now, after the exponentials
+  if (kIrr || kind == 2) {
+    float dl, dh;
+    upk2(add2(add2(s0, s1), add2(s2, s3)), dl, dh);
+    const bool grouped = !kIrr || kind == 2;       // the rest is selects
+    f.rden = kIrr && (c0 == 63 || !grouped) ? 0.f : __fdividef(1.f, dl + dh);
+    f.g = ex2(lm2 - M2L);
+    f.w = grouped ? f.g * f.rden : 1.f;
+  }
+  return f;
+}
+
+// bwd_dscores: reads dP from TMEM once, arrives on free_bar, and leaves the row of dS, packed to 16 bits, in wd.
+template <bool kBf16, bool kIrr>
+__device__ __forceinline__ void bwd_dscores(uint32_t (&wd)[32], const uint64_t (&sp)[32], const RowFactors& f, uint32_t tdp,
+                                            uint32_t free_bar, int kind, float scale, float delta) {
+  uint64_t dp[32];
   if (kIrr) __syncwarp();
   if (!kIrr && kind == 0) {
 #pragma unroll
@@ -768,6 +767,7 @@ __device__ __forceinline__ void bwd_item(int c0, uint32_t ts, uint32_t tdp, uint
   }
   tc_fence_before();
   mbar_arrive(free_bar);
+  float sub = delta, lm_ds = 0.f;
   if (kIrr || kind == 2) {
     uint64_t n0 = 0ull, n1 = 0ull, n2a = 0ull, n3 = 0ull;
 #pragma unroll
@@ -777,30 +777,17 @@ __device__ __forceinline__ void bwd_item(int c0, uint32_t ts, uint32_t tdp, uint
       n2a = fma2(sp[j + 2], dp[j + 2], n2a);
       n3 = fma2(sp[j + 3], dp[j + 3], n3);
     }
-    float dl, dh, ql, qh;
-    upk2(add2(add2(s0, s1), add2(s2, s3)), dl, dh);
+    float ql, qh;
     upk2(add2(add2(n0, n1), add2(n2a, n3)), ql, qh);
-    const bool grouped = !kIrr || kind == 2;       // the rest is selects
-    const float rden = kIrr && (c0 == 63 || !grouped) ? 0.f : __fdividef(1.f, dl + dh);
-    const float nd = (ql + qh) * rden;
-    const float g = ex2(lm2 - M2L);
-    const float w = grouped ? g * rden : 1.f;
-    if (kNeedP) {
-      const uint64_t w2 = pk2(w, w);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) sp[j] = mul2(sp[j], w2);
-    } else {
-      pscale = w;       // P itself is not stored: its row factor is folded into the dS coefficients below
-    }
-    sub = grouped ? nd : delta;
-    lm_ds = g * (nd - delta) * scale;
+    const float nd = (ql + qh) * f.rden;
+    sub = !kIrr || kind == 2 ? nd : delta;
+    lm_ds = f.g * (nd - delta) * scale;
   }
-  // dS = P * (dP - sub) * scale = P * fma(dP, scale, -sub * scale)
-  const float sc = scale * pscale;
+  // dS = P * (dP - sub) * scale = sp * fma(dP, w * scale, -sub * w * scale)
+  const float sc = scale * f.w;
   const uint64_t sc2 = pk2(sc, sc);
   const float nss = -sub * sc;
   const uint64_t nss2 = pk2(nss, nss);
-  uint32_t wd[32];
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
     float d0, d1;
@@ -808,60 +795,83 @@ __device__ __forceinline__ void bwd_item(int c0, uint32_t ts, uint32_t tdp, uint
     if (j == 31 && kind == 2) d1 = lm_ds;
     wd[j] = pack2<kBf16>(d0, d1);
   }
-  if (kNeedP) {
-    uint32_t wp[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) wp[j] = pack2p<kBf16>(sp[j]);
-    wait_dst();
-    store_row_sw128(p_dst, row, wp);
-    between_stores();   // the P tile and the dS tile are handed over separately
-    store_row_sw128(ds_dst, row, wd);
-  } else {
-    wait_dst();
-    store_row_sw128(ds_dst, row, wd);
-  }
 }
 
 enum { kErrDkvProducer = 201, kErrDkvMma = 202, kErrDkvSoftmax = 203, kErrDkvEpilogue = 204,
        kErrDqProducer = 301, kErrDqMma = 302, kErrDqSoftmax = 303, kErrDqEpilogue = 304 };
 
 // ---------------------------------------------------------------------------------------------- backward: dK, dV
-// Thread roles (both backward kernels): warps 0-3 and 4-7 are two softmax warpgroups that take alternate items
-// (the backward pass carries no state from one item to the next), warp 8 issues TMA loads, warp 9 issues the
-// S / dP MMAs and owns the TMEM allocation, warp 10 issues the accumulating MMAs.  Two issuer threads keep the
+// Thread roles (both backward kernels): warps 0-3 and 4-7 are two softmax warpgroups, warp 8 issues TMA loads, warp 9 issues
+// the S / dP MMAs and owns the TMEM allocation, warp 10 issues the accumulating MMAs.  Two issuing warps keep the
 // products of the next item from queueing behind a wait for the current one.  (Registers are granted to 4 warps at
 // a time, so 9 to 12 warps all leave 168 registers per thread.)
-constexpr int kBwdGroups = 2;                       // softmax warpgroups (items are dealt round-robin)
+constexpr int kBwdGroups = 2;                       // softmax warpgroups
 constexpr int kBwdThreads = (kBwdGroups * 4 + 3) * 32;
 constexpr int kSdpBufs = 2;                         // S / dP buffers in TMEM of the dQ kernel: 2 x (64 + 64) columns
-constexpr int kDkvStages = 2;
+template <int kD> constexpr int kDkvStages = kD == 128 ? 2 : 4;
 
-struct DkvSmem {
-  uint64_t kv_full;
-  uint64_t kv_empty;
-  uint64_t full[kDkvStages];
-  uint64_t empty[kDkvStages];
-  uint64_t s_full;          // S of both blocks (one N = 128 product)
-  uint64_t s_free;          // both warpgroups hold S in registers
-  uint64_t dp_full;
-  uint64_t dp_free;         // both warpgroups have read dP for the last time
-  uint64_t p_ready;         // the P tile / the dS tile are handed over separately, so that one warpgroup's stores
-  uint64_t ds_ready;        // overlap the other one's accumulating MMAs
-  uint64_t p_free[2];       // [g]: the dV MMAs of warpgroup g's latest item have read the P tile
-  uint64_t ds_free[2];      // [g]: likewise the dK MMAs and the dS tile
-  uint64_t acc_full[2];
-  uint64_t acc_empty[2];
+template <int kStages> struct DkvSmem {
+  uint64_t k_full, k_empty, v_full, v_empty;
+  uint64_t q_full[kStages], q_empty[kStages];       // Q: until dK has read it
+  uint64_t do_full[kStages], do_empty[kStages];     // dO: until dP and dV have read it
+  uint64_t s_full, s_free;                          // S of both blocks (one N = 128 product); both warpgroups hold it in registers
+  uint64_t dp_full, dp_free;
+  uint64_t p_ready, p_free;                         // the P rows are in the weight tiles / dV has read them
+  uint64_t ds_ready, ds_free;                       // likewise the dS rows that replace them, and dK
+  uint64_t acc_full[2], acc_empty[2];               // [0] dV, [1] dK
   uint32_t tmem_base;
 };
 
+// Stores 32 accumulator columns of one TMEM lane per thread as 16-bit values.  Four neighbouring lanes exchange 16-byte
+// chunks first, so that a warp's store covers 64 contiguous bytes of eight rows and not 16 bytes of thirty-two.
+// row_off[j]: element offset of row j of the lane's four rows, or -1 for a row that is not stored.
+template <bool kBf16>
+__device__ __forceinline__ void store_acc_cols(void* out, const int64_t (&row_off)[4], const uint32_t (&r)[32], int col0, int D,
+                                               int lane) {
+  uint4 v[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    v[e].x = pack2<kBf16>(__uint_as_float(r[8 * e + 0]), __uint_as_float(r[8 * e + 1]));
+    v[e].y = pack2<kBf16>(__uint_as_float(r[8 * e + 2]), __uint_as_float(r[8 * e + 3]));
+    v[e].z = pack2<kBf16>(__uint_as_float(r[8 * e + 4]), __uint_as_float(r[8 * e + 5]));
+    v[e].w = pack2<kBf16>(__uint_as_float(r[8 * e + 6]), __uint_as_float(r[8 * e + 7]));
+  }
+  // transpose of the 4 x 4 matrix (lane of the four, chunk): swap the off-diagonal chunks of 2 x 2 blocks, then the blocks
+  auto swap = [&](uint4& a, uint4& b, int step) {      // lower lane: b <-> partner's a
+    const bool up = (lane & step) != 0;
+    uint4 x = up ? a : b;
+    x.x = __shfl_xor_sync(0xffffffffu, x.x, step);
+    x.y = __shfl_xor_sync(0xffffffffu, x.y, step);
+    x.z = __shfl_xor_sync(0xffffffffu, x.z, step);
+    x.w = __shfl_xor_sync(0xffffffffu, x.w, step);
+    a = up ? x : a;
+    b = up ? b : x;
+  };
+  swap(v[0], v[1], 1);
+  swap(v[2], v[3], 1);
+  swap(v[0], v[2], 2);
+  swap(v[1], v[3], 2);
+  const int col = col0 + 8 * (lane & 3);
+  if (col < D) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (row_off[j] >= 0) *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(out) + row_off[j] + col) = v[j];
+  }
+}
+
 // Persistent; a work unit is a PAIR of adjacent 64-key blocks (a = 2c, b = 2c+1) of one (batch, head).  Both blocks
-// stay in shared memory while the unit streams the query tiles that see them, so each 64 KB Q/dO tile is fetched from
-// L2 once per 128 keys, and S / dP of the two blocks are single N = 128 products.  Warpgroup 0 rebuilds P and dS for
-// block a, warpgroup 1 for block b; they share a single P/dS tile pair (a writer waits until the accumulating MMAs of
-// the item written before have read it), which settles them half an item apart.
+// stay in shared memory while the unit streams the query tiles that see them, so each Q/dO tile is fetched from
+// L2 once per 128 keys.  All four products of an item are single ones over both blocks: S = Q K^T and dP = dO V^T with N = 128,
+// dV += P^T dO and dK += dS^T Q with M = 128 keys and N = kD.  Warpgroup 0 rebuilds P and dS for block a, warpgroup 1 for block b.
+// P is handed over as soon as S allows it, before dP is looked at; dS takes its place once dV has read it, and the next P takes
+// dS's place once dK has read that: each of these waits has half an item of other work in front of it.
+// Q and dO have barriers of their own, so dO's place is reloaded from the end of dV on and Q's from the end of dK on.
+// The former arrangement (one P and one dS tile that the warpgroups took in turns, dV and dK as four products of N = 64, 448 KB of
+// shared-memory traffic an item instead of 384, Q and dO handed over together, 128 features multiplied whatever kD is) against
+// this one, forward + backward: B4 H16 L1024 D64 102.6 / 95.4 us, B1 H32 L2048 D128 201.7 / 197.7.
 // CTA c takes units w = round * grid + c with the direction alternating per round (snake), heaviest pairs first.
 // Loads, S/dP products and the softmax of the next unit start while the accumulators of the current one are drained.
-template <bool kBf16, bool kWhole, bool kIrr>      // kWhole: whole tiles and D = 128
+template <bool kBf16, int kD, bool kWhole, bool kIrr>      // kWhole: whole tiles and D = kD
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -869,19 +879,18 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const float* __restrict__ delta_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
                      int H, int BH, int Lq, int Lk, int D_any, float scale, float scale_log2, int max_tiles,
                      IrrArgs irr) {
-  constexpr int kD = 128;
   const int D = kWhole ? kD : D_any;
+  constexpr int kStages = kDkvStages<kD>;
+  constexpr uint32_t kOperand = (kD / 64) * kTileBytes;     // [128 rows x kD] as 64-feature sub-tiles of 16 KB
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  // K of the pair as one [128 keys x 128 d] K-major operand: 64-feature sub-tile c at c * 16 KB, block g's 64 rows at
-  // g * 8 KB inside it; V likewise, 32 KB further
-  const uint32_t k_pair = base, v_pair = base + 32768u;
-  auto q_slot = [&](int s) { return base + 65536u + (uint32_t)s * 65536u; };
-  auto do_slot = [&](int s) { return base + 65536u + (uint32_t)s * 65536u + 32768u; };
-  const uint32_t p_tile = base + 65536u + kDkvStages * 65536u;
-  const uint32_t ds_tile = p_tile + 16384u;
-  DkvSmem* sm = reinterpret_cast<DkvSmem*>(smem_raw + (base - raw) + 65536u + kDkvStages * 65536u + 32768u);
+  // K of the pair as one [128 keys x kD] K-major operand, block g's 64 rows at g * 8 KB inside each sub-tile; V likewise
+  const uint32_t k_pair = base, v_pair = base + kOperand;
+  auto q_slot = [&](int s) { return base + 2 * kOperand + (uint32_t)s * 2 * kOperand; };
+  auto do_slot = [&](int s) { return base + 3 * kOperand + (uint32_t)s * 2 * kOperand; };
+  const uint32_t w_tile = base + (2 + 2 * kStages) * kOperand;         // P, then dS: [128 q x 64 keys] of block a, then of b
+  DkvSmem<kStages>* sm = reinterpret_cast<DkvSmem<kStages>*>(smem_raw + (base - raw) + (2 + 2 * kStages) * kOperand + 2 * kTileBytes);
 
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int prefix_blocks = (Lk - Lq) / kBlk;
@@ -911,25 +920,27 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   };
 
   if (tid == 0) {
-    mbar_init(smem_u32(&sm->kv_full), 1);
-    mbar_init(smem_u32(&sm->kv_empty), 1);
-    for (int s = 0; s < kDkvStages; ++s) {
-      mbar_init(smem_u32(&sm->full[s]), 1);
-      mbar_init(smem_u32(&sm->empty[s]), 1);
+    mbar_init(smem_u32(&sm->k_full), 1);
+    mbar_init(smem_u32(&sm->k_empty), 1);
+    mbar_init(smem_u32(&sm->v_full), 1);
+    mbar_init(smem_u32(&sm->v_empty), 1);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(smem_u32(&sm->q_full[s]), 1);
+      mbar_init(smem_u32(&sm->q_empty[s]), 1);
+      mbar_init(smem_u32(&sm->do_full[s]), 1);
+      mbar_init(smem_u32(&sm->do_empty[s]), 2);       // dP and dV, issued by different warps
     }
     mbar_init(smem_u32(&sm->s_full), 1);
     mbar_init(smem_u32(&sm->s_free), 256);
     mbar_init(smem_u32(&sm->dp_full), 1);
     mbar_init(smem_u32(&sm->dp_free), 256);
+    mbar_init(smem_u32(&sm->p_ready), 256);
+    mbar_init(smem_u32(&sm->p_free), 1);
+    mbar_init(smem_u32(&sm->ds_ready), 256);
+    mbar_init(smem_u32(&sm->ds_free), 1);
     for (int g = 0; g < 2; ++g) {
       mbar_init(smem_u32(&sm->acc_full[g]), 1);
       mbar_init(smem_u32(&sm->acc_empty[g]), 128);
-    }
-    mbar_init(smem_u32(&sm->p_ready), 128);
-    mbar_init(smem_u32(&sm->ds_ready), 128);
-    for (int g = 0; g < 2; ++g) {
-      mbar_init(smem_u32(&sm->p_free[g]), 1);
-      mbar_init(smem_u32(&sm->ds_free[g]), 1);
     }
     mbar_init_fence();
   }
@@ -938,10 +949,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = (uint32_t)warp_uniform((int)sm->tmem_base);
-  auto tmem_s = [&](int g) { return tmem + (uint32_t)g * 64u; };
-  auto tmem_dp = [&](int g) { return tmem + 128u + (uint32_t)g * 64u; };
-  auto tmem_dv = [&](int g) { return tmem + 256u + (uint32_t)g * 128u; };
-  auto tmem_dk = [&](int g) { return tmem + 320u + (uint32_t)g * 128u; };
+  const uint32_t tmem_s = tmem, tmem_dp = tmem + 128u, tmem_dv = tmem + 256u, tmem_dk = tmem + 256u + kD;
 
   if (warp == kBwdGroups * 4) {
     if (lane == 0) {
@@ -954,129 +962,125 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (skipped(w)) continue;
         const int pair = w / BH, bh = w - pair * BH, b = bh / H, h = bh - b * H;
         const int tq0 = unit_tq0(w), n_items = n_tiles - tq0;
-        const uint32_t kvb = smem_u32(&sm->kv_full);
-        mbar_wait(smem_u32(&sm->kv_empty), (u & 1) ^ 1, &g_lmk_status, kErrDkvProducer);
-        mbar_arrive_expect_tx(kvb, 4 * kTileBytes);
+        int key_row[2];
         for (int g = 0; g < 2; ++g) {       // a block past the end of the sequence reads as zeros
           const int n = 2 * pair + g;
-          const int r0 = kIrr ? (n < tiles_of(b) ? end_of(b, n) - 63 : Lk) : n * kBlk;
-          tma_load_4d(k_pair + g * kHalfTile, &tm_k, kvb, 0, r0, h, b);
-          tma_load_4d(k_pair + kTileBytes + g * kHalfTile, &tm_k, kvb, 64, r0, h, b);
-          tma_load_4d(v_pair + g * kHalfTile, &tm_v, kvb, 0, r0, h, b);
-          tma_load_4d(v_pair + kTileBytes + g * kHalfTile, &tm_v, kvb, 64, r0, h, b);
+          key_row[g] = kIrr ? (n < tiles_of(b) ? end_of(b, n) - 63 : Lk) : n * kBlk;
         }
+        auto load_pair = [&](uint32_t dst, const CUtensorMap* tm, uint64_t* full, uint64_t* empty) {
+          const uint32_t fb = smem_u32(full);
+          mbar_wait(smem_u32(empty), (u & 1) ^ 1, &g_lmk_status, kErrDkvProducer);
+          mbar_arrive_expect_tx(fb, kOperand);
+          for (int g = 0; g < 2; ++g)
+            for (int c = 0; c < kD / 64; ++c)
+              tma_load_4d(dst + c * kTileBytes + g * kHalfTile, tm, fb, 64 * c, key_row[g], h, b);
+        };
+        auto load_rows = [&](uint32_t dst, const CUtensorMap* tm, uint64_t* full, uint64_t* empty, int tile) {
+          const uint32_t fb = smem_u32(full);
+          mbar_wait(smem_u32(empty), ((it / kStages) & 1) ^ 1, &g_lmk_status, kErrDkvProducer);
+          mbar_arrive_expect_tx(fb, kOperand);
+          for (int c = 0; c < kD / 64; ++c) tma_load_4d(dst + c * kTileBytes, tm, fb, 64 * c, tile * kQTile, h, b);
+        };
+        load_pair(k_pair, &tm_k, &sm->k_full, &sm->k_empty);
         for (int i = 0; i < n_items; ++i, ++it) {
-          const int s = it % kDkvStages;
-          mbar_wait(smem_u32(&sm->empty[s]), ((it / kDkvStages) & 1) ^ 1, &g_lmk_status, kErrDkvProducer);
-          const uint32_t fb = smem_u32(&sm->full[s]);
-          const int r0 = (tq0 + i) * kQTile;
-          mbar_arrive_expect_tx(fb, 4 * kTileBytes);
-          tma_load_4d(q_slot(s), &tm_q, fb, 0, r0, h, b);
-          tma_load_4d(q_slot(s) + kTileBytes, &tm_q, fb, 64, r0, h, b);
-          tma_load_4d(do_slot(s), &tm_do, fb, 0, r0, h, b);
-          tma_load_4d(do_slot(s) + kTileBytes, &tm_do, fb, 64, r0, h, b);
+          const int s = it % kStages;
+          load_rows(q_slot(s), &tm_q, &sm->q_full[s], &sm->q_empty[s], tq0 + i);
+          if (i == 0) load_pair(v_pair, &tm_v, &sm->v_full, &sm->v_empty);
+          load_rows(do_slot(s), &tm_do, &sm->do_full[s], &sm->do_empty[s], tq0 + i);
         }
         ++u;
       }
     }
     __syncwarp();
   } else if (warp == kBwdGroups * 4 + 1) {
-    // S = Q K^T and dP = dO V^T for both blocks of the pair at once (N = 128: full-rate MMAs), one query tile at a
-    // time.  S has its own full / free barriers: the warpgroups hold S in registers early in an item, so the next S
-    // product runs while they are still busy with dP.
-    {
-      constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 128, 0, 0);
-      const uint64_t dk0 = smem_desc_sw128(k_pair, 16, 1024), dv0 = smem_desc_sw128(v_pair, 16, 1024);
-      const uint64_t dq0 = smem_desc_sw128(q_slot(0), 16, 1024), ddo0 = smem_desc_sw128(do_slot(0), 16, 1024);
-      int it = 0, u = 0;
-      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-        if (warp_uniform(skipped(w))) continue;
-        const int n_items = n_tiles - warp_uniform(unit_tq0(w));
-        mbar_wait(smem_u32(&sm->kv_full), u & 1, &g_lmk_status, kErrDkvMma);
-        for (int i = 0; i < n_items; ++i, ++it) {
-          const int s = it % kDkvStages;
-          mbar_wait(smem_u32(&sm->full[s]), (it / kDkvStages) & 1, &g_lmk_status, kErrDkvMma);
-          const uint64_t dq = desc_advance(dq0, (uint32_t)s * 65536u), ddo = desc_advance(ddo0, (uint32_t)s * 65536u);
-          if (it >= 1) mbar_wait(smem_u32(&sm->s_free), (it & 1) ^ 1, &g_lmk_status, kErrDkvMma);
-          tc_fence_after();
-          if (elect_one()) {
-#pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk)
-              mma_f16_ss(tmem_s(0), desc_advance(dq, kmajor_step(kk, kTileBytes)),
-                         desc_advance(dk0, kmajor_step(kk, kTileBytes)), idesc_s, kk > 0);
-            mma_commit(smem_u32(&sm->s_full));
-          }
-          if (it >= 1) mbar_wait(smem_u32(&sm->dp_free), (it & 1) ^ 1, &g_lmk_status, kErrDkvMma);
-          tc_fence_after();
-          if (elect_one()) {
-#pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk)
-              mma_f16_ss(tmem_dp(0), desc_advance(ddo, kmajor_step(kk, kTileBytes)),
-                         desc_advance(dv0, kmajor_step(kk, kTileBytes)), idesc_s, kk > 0);
-            mma_commit(smem_u32(&sm->dp_full));
-          }
-        }
-        if (elect_one()) mma_commit(smem_u32(&sm->kv_empty));      // K / V tiles may be replaced once these products are done
-        ++u;
-      }
-    }
-    __syncwarp();
-  } else if (warp == kBwdGroups * 4 + 2) {
-    // dV_g^T += dO^T P and dK_g^T += Q^T dS.  A = dO^T / Q^T: MN-major view of the row-major [128 q x 128 d] tile (second
-    // 64-feature half 16 KB further); B = P / dS: MN-major view of the [128 q x 64 k] tile; a K-step is 16 query rows
-    // = 2048 bytes.
-    {
-      constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_t = instr_desc_f16(fmt, 128, 64, 1, 1);
-      const uint64_t dq0t = smem_desc_sw128(q_slot(0), kTileBytes, 1024);
-      const uint64_t ddo0t = smem_desc_sw128(do_slot(0), kTileBytes, 1024);
-      const uint64_t dpt = smem_desc_sw128(p_tile, 16, 1024), ddst = smem_desc_sw128(ds_tile, 16, 1024);
-      int it = 0, u = 0;
-      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-        if (warp_uniform(skipped(w))) continue;
-        const int n_items = n_tiles - warp_uniform(unit_tq0(w));
-        for (int i = 0; i < n_items; ++i, ++it) {
-          const int s = it % kDkvStages;
-          const uint64_t ddot = desc_advance(ddo0t, (uint32_t)s * 65536u), dqt = desc_advance(dq0t, (uint32_t)s * 65536u);
-#pragma unroll
-          for (int g = 0; g < 2; ++g) {
-            // item j = 2 * it + g of the single P/dS tile pair
-            mbar_wait(smem_u32(&sm->p_ready), g, &g_lmk_status, kErrDkvMma);
-            if (i == 0) mbar_wait(smem_u32(&sm->acc_empty[g]), (u & 1) ^ 1, &g_lmk_status, kErrDkvMma);
-            tc_fence_after();
-            if (elect_one()) {
-#pragma unroll
-              for (int kk = 0; kk < kQTile / 16; ++kk)
-                mma_f16_ss(tmem_dv(g), desc_advance(ddot, kk * 2048), desc_advance(dpt, kk * 2048), idesc_t,
-                           (i > 0 || kk > 0) ? 1u : 0u);
-              mma_commit(smem_u32(&sm->p_free[g]));
-            }
-            mbar_wait(smem_u32(&sm->ds_ready), g, &g_lmk_status, kErrDkvMma);
-            tc_fence_after();
-            if (elect_one()) {
-#pragma unroll
-              for (int kk = 0; kk < kQTile / 16; ++kk)
-                mma_f16_ss(tmem_dk(g), desc_advance(dqt, kk * 2048), desc_advance(ddst, kk * 2048), idesc_t,
-                           (i > 0 || kk > 0) ? 1u : 0u);
-              mma_commit(smem_u32(&sm->ds_free[g]));
-            }
-          }
-          if (elect_one()) mma_commit(smem_u32(&sm->empty[s]));
-        }
+    // S = Q K^T and dP = dO V^T of both blocks of the pair at once, one query tile at a time.  The warpgroups hold S in
+    // registers early in an item, so the next S product runs while they are still busy with dP.
+    constexpr uint32_t fmt = kBf16 ? 1u : 0u;
+    constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 128, 0, 0);
+    const uint64_t dk0 = smem_desc_sw128(k_pair, 16, 1024), dv0 = smem_desc_sw128(v_pair, 16, 1024);
+    const uint64_t dq0 = smem_desc_sw128(q_slot(0), 16, 1024), ddo0 = smem_desc_sw128(do_slot(0), 16, 1024);
+    int it = 0, u = 0;
+    for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+      if (warp_uniform(skipped(w))) continue;
+      const int n_items = n_tiles - warp_uniform(unit_tq0(w));
+      mbar_wait(smem_u32(&sm->k_full), u & 1, &g_lmk_status, kErrDkvMma);
+      for (int i = 0; i < n_items; ++i, ++it) {
+        const int s = it % kStages;
+        const uint64_t dq = desc_advance(dq0, (uint32_t)s * 2 * kOperand), ddo = desc_advance(ddo0, (uint32_t)s * 2 * kOperand);
+        mbar_wait(smem_u32(&sm->q_full[s]), (it / kStages) & 1, &g_lmk_status, kErrDkvMma);
+        if (it >= 1) mbar_wait(smem_u32(&sm->s_free), (it & 1) ^ 1, &g_lmk_status, kErrDkvMma);
+        tc_fence_after();
         if (elect_one()) {
-          mma_commit(smem_u32(&sm->acc_full[0]));
-          mma_commit(smem_u32(&sm->acc_full[1]));
+#pragma unroll
+          for (int kk = 0; kk < kD / 16; ++kk)
+            mma_f16_ss(tmem_s, desc_advance(dq, kmajor_step(kk, kTileBytes)), desc_advance(dk0, kmajor_step(kk, kTileBytes)),
+                       idesc_s, kk > 0);
+          mma_commit(smem_u32(&sm->s_full));
+          if (i == n_items - 1) mma_commit(smem_u32(&sm->k_empty));
         }
-        ++u;
+        if (i == 0) mbar_wait(smem_u32(&sm->v_full), u & 1, &g_lmk_status, kErrDkvMma);
+        mbar_wait(smem_u32(&sm->do_full[s]), (it / kStages) & 1, &g_lmk_status, kErrDkvMma);
+        if (it >= 1) mbar_wait(smem_u32(&sm->dp_free), (it & 1) ^ 1, &g_lmk_status, kErrDkvMma);
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < kD / 16; ++kk)
+            mma_f16_ss(tmem_dp, desc_advance(ddo, kmajor_step(kk, kTileBytes)), desc_advance(dv0, kmajor_step(kk, kTileBytes)),
+                       idesc_s, kk > 0);
+          mma_commit(smem_u32(&sm->dp_full));
+          mma_commit(smem_u32(&sm->do_empty[s]));
+          if (i == n_items - 1) mma_commit(smem_u32(&sm->v_empty));
+        }
       }
+      ++u;
     }
-    __syncwarp();
+  } else if (warp == kBwdGroups * 4 + 2) {
+    // dV += P^T dO and dK += dS^T Q.  A = P^T / dS^T: MN-major view of the two [128 q x 64 keys] tiles; B = dO / Q: MN-major view of
+    // the row-major [128 q x kD] tile; a K-step is 16 query rows = 2048 bytes.  dV waits for dO itself: P may be there first.
+    constexpr uint32_t fmt = kBf16 ? 1u : 0u;
+    constexpr uint32_t idesc_t = instr_desc_f16(fmt, 128, kD, 1, 1);
+    const uint64_t dq0t = smem_desc_sw128(q_slot(0), kTileBytes, 1024);
+    const uint64_t ddo0t = smem_desc_sw128(do_slot(0), kTileBytes, 1024);
+    const uint64_t dwt = smem_desc_sw128(w_tile, kTileBytes, 1024);
+    int it = 0, u = 0;
+    for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+      if (warp_uniform(skipped(w))) continue;
+      const int n_items = n_tiles - warp_uniform(unit_tq0(w));
+      for (int i = 0; i < n_items; ++i, ++it) {
+        const int s = it % kStages;
+        const uint64_t ddot = desc_advance(ddo0t, (uint32_t)s * 2 * kOperand), dqt = desc_advance(dq0t, (uint32_t)s * 2 * kOperand);
+        mbar_wait(smem_u32(&sm->do_full[s]), (it / kStages) & 1, &g_lmk_status, kErrDkvMma);
+        mbar_wait(smem_u32(&sm->p_ready), it & 1, &g_lmk_status, kErrDkvMma);
+        if (i == 0) mbar_wait(smem_u32(&sm->acc_empty[0]), (u & 1) ^ 1, &g_lmk_status, kErrDkvMma);
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < kQTile / 16; ++kk)
+            mma_f16_ss(tmem_dv, desc_advance(dwt, kk * 2048), desc_advance(ddot, kk * 2048), idesc_t, (i > 0 || kk > 0) ? 1u : 0u);
+          mma_commit(smem_u32(&sm->p_free));
+          mma_commit(smem_u32(&sm->do_empty[s]));
+          if (i == n_items - 1) mma_commit(smem_u32(&sm->acc_full[0]));
+        }
+        mbar_wait(smem_u32(&sm->ds_ready), it & 1, &g_lmk_status, kErrDkvMma);
+        if (i == 0) mbar_wait(smem_u32(&sm->acc_empty[1]), (u & 1) ^ 1, &g_lmk_status, kErrDkvMma);
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < kQTile / 16; ++kk)
+            mma_f16_ss(tmem_dk, desc_advance(dwt, kk * 2048), desc_advance(dqt, kk * 2048), idesc_t, (i > 0 || kk > 0) ? 1u : 0u);
+          mma_commit(smem_u32(&sm->ds_free));
+          mma_commit(smem_u32(&sm->q_empty[s]));
+          if (i == n_items - 1) mma_commit(smem_u32(&sm->acc_full[1]));
+        }
+      }
+      ++u;
+    }
   } else {
-    const int g = warp >> 2;                       // warpgroup g owns block g of every pair
+    const int g = warp >> 2;                       // warpgroup g owns block g of every pair, and drains dV (0) or dK (1) of both
     const int row = tid & 127;
     const int half = row >> 6;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t my_tile = w_tile + (uint32_t)g * kTileBytes;
     int it = 0, u = 0;
     for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
       if (skipped(w)) continue;
@@ -1107,73 +1111,68 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           nDelta = delta_ptr[grow];
           nOwn = own_of((tq + 1) * kQTile + row);
         }
+        const int kind = n > own ? 0 : (n == own ? 1 : 2);
         mbar_wait(smem_u32(&sm->s_full), it & 1, &g_lmk_status, kErrDkvSoftmax);
         tc_fence_after();
-        const int kind = n > own ? 0 : (n == own ? 1 : 2);
-        bwd_item<kBf16, true, kIrr>(c0, tmem_s(g) + lane_base, tmem_dp(g) + lane_base, smem_u32(&sm->dp_free), kind, vis,
-                              scale_log2, scale, M2L, delta, p_tile, ds_tile, row, [&]() {
-                                // The single P/dS tile pair is written in the order a, b, a, b, ...: before writing,
-                                // the accumulating MMAs of the OTHER warpgroup's latest item must have read it.  Each
-                                // warpgroup is the only waiter on the other one's barriers and sees every phase.
-                                const int prev = 2 * it + g - 1;          // item written just before this one
-                                if (prev >= 0)
-                                  mbar_wait(smem_u32(&sm->p_free[1 - g]), (prev >> 1) & 1, &g_lmk_status,
-                                            kErrDkvSoftmax);
-                              },
-                              [&]() {
-                                tc_fence_before();
-                                mbar_arrive(smem_u32(&sm->s_free));
-                              },
-                              [&]() {
-                                mbar_wait(smem_u32(&sm->dp_full), it & 1, &g_lmk_status, kErrDkvSoftmax);
-                                tc_fence_after();
-                              },
-                              [&]() {
-                                fence_proxy_async_smem();
-                                mbar_arrive(smem_u32(&sm->p_ready));
-                                const int prev = 2 * it + g - 1;
-                                if (prev >= 0)
-                                  mbar_wait(smem_u32(&sm->ds_free[1 - g]), (prev >> 1) & 1, &g_lmk_status,
-                                            kErrDkvSoftmax);
-                              });
+        uint64_t sp[32];
+        const RowFactors f = bwd_weights<kIrr>(sp, c0, tmem_s + (uint32_t)g * 64u + lane_base, kind, vis, scale_log2, M2L, [&]() {
+          tc_fence_before();
+          mbar_arrive(smem_u32(&sm->s_free));
+        });
+        uint32_t wd[32];
+        {
+          const uint64_t w2 = pk2(f.w, f.w);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) wd[j] = pack2p<kBf16>(mul2(sp[j], w2));
+        }
+        if (it >= 1) mbar_wait(smem_u32(&sm->ds_free), (it & 1) ^ 1, &g_lmk_status, kErrDkvSoftmax);
+        store_row_sw128(my_tile, row, wd);
+        fence_proxy_async_smem();
+        mbar_arrive(smem_u32(&sm->p_ready));
+        mbar_wait(smem_u32(&sm->dp_full), it & 1, &g_lmk_status, kErrDkvSoftmax);
+        tc_fence_after();
+        bwd_dscores<kBf16, kIrr>(wd, sp, f, tmem_dp + (uint32_t)g * 64u + lane_base, smem_u32(&sm->dp_free), kind, scale, delta);
+        mbar_wait(smem_u32(&sm->p_free), it & 1, &g_lmk_status, kErrDkvSoftmax);
+        store_row_sw128(my_tile, row, wd);
         fence_proxy_async_smem();
         mbar_arrive(smem_u32(&sm->ds_ready));
       }
-      // epilogue: each warpgroup drains its own block; thread = feature d, TMEM column = key j -> dV[key][d], dK[key][d]
+      // epilogue: TMEM lane = key of the pair
+      int64_t off = -1;
+      {
+        const int n_r = 2 * pair + half;
+        int key = n_r * kBlk + (row & 63);
+        bool stored = key < Lk;
+        if (kIrr) {
+          stored = n_r < tiles_of(b);
+          if (stored) {
+            const int end_r = end_of(b, n_r);
+            key = end_r - 63 + (row & 63);
+            stored = key > end_of(b, n_r - 1) && key < Lk;       // the tile's own keys
+          }
+        }
+        if (stored) off = ((int64_t)bh * Lk + key) * D;
+      }
+      int64_t row_off[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) row_off[j] = __shfl_sync(0xffffffffu, off, (lane & ~3) + j);
       mbar_wait(smem_u32(&sm->acc_full[g]), u & 1, &g_lmk_status, kErrDkvEpilogue);
       tc_fence_after();
       if (kIrr) __syncwarp();
-      uint32_t rv[2][32], rk[2][32];
-      tmem_ld_32x32b_x32(tmem_dv(g) + lane_base, rv[0]);
-      tmem_ld_32x32b_x32(tmem_dv(g) + 32 + lane_base, rv[1]);
-      tmem_ld_32x32b_x32(tmem_dk(g) + lane_base, rk[0]);
-      tmem_ld_32x32b_x32(tmem_dk(g) + 32 + lane_base, rk[1]);
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(smem_u32(&sm->acc_empty[g]));     // the next unit may start accumulating into this block's columns
-      if (tile_exists) {
-        const int key0 = kIrr ? end - 63 : n * kBlk;        // key of column 0; columns c0 ... keys-1 are this tile's own
-        const int keys = min(kBlk, Lk - key0);
-        // A lane holds one feature of all keys.  Neighbouring lanes swap halves, so that a lane stores two features of every
-        // second key in one word (half as many stores as 16-bit ones, and the same 64 bytes a row and warp).
-        const bool odd = lane & 1;
-        const int f = row & ~1;
-        uint32_t* dvp = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dv_ptr) + ((int64_t)bh * Lk + key0 + (odd ? 1 : 0)) * D + f);
-        uint32_t* dkp = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(dk_ptr) + ((int64_t)bh * Lk + key0 + (odd ? 1 : 0)) * D + f);
-        const bool stores = kWhole || f < D;
+      const uint32_t t_acc = (g == 0 ? tmem_dv : tmem_dk) + lane_base;
+      void* const out = g == 0 ? dv_ptr : dk_ptr;
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const uint32_t v = pack2<kBf16>(__uint_as_float(rv[c][j]), __uint_as_float(rv[c][j + 1]));
-            const uint32_t k = pack2<kBf16>(__uint_as_float(rk[c][j]), __uint_as_float(rk[c][j + 1]));
-            const uint32_t vo = __shfl_xor_sync(0xffffffffu, v, 1), ko = __shfl_xor_sync(0xffffffffu, k, 1);
-            const int col = c * 32 + j + (odd ? 1 : 0);
-            if (stores && (kWhole || (col < keys && (!kIrr || col >= c0)))) {
-              dvp[(c * 32 + j) * (D / 2)] = odd ? __byte_perm(vo, v, 0x7632) : __byte_perm(v, vo, 0x5410);
-              dkp[(c * 32 + j) * (D / 2)] = odd ? __byte_perm(ko, k, 0x7632) : __byte_perm(k, ko, 0x5410);
-            }
-          }
+      for (int c = 0; c < kD / 64; ++c) {
+        uint32_t ra[32], rb[32];
+        tmem_ld_32x32b_x32(t_acc + c * 64, ra);
+        tmem_ld_32x32b_x32(t_acc + c * 64 + 32, rb);
+        tmem_ld_wait();
+        if (c == kD / 64 - 1) {
+          tc_fence_before();
+          mbar_arrive(smem_u32(&sm->acc_empty[g]));     // the next unit may start accumulating
+        }
+        store_acc_cols<kBf16>(out, row_off, ra, c * 64, D, lane);
+        store_acc_cols<kBf16>(out, row_off, rb, c * 64 + 32, D, lane);
       }
       ++u;
     }
@@ -1519,18 +1518,16 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int kind = n > own ? 0 : (n == own ? 1 : 2);
         const int c_now = c0;
         if (kIrr) c0 = first_col(n - kBwdGroups);
-        // dS replaces the V tile of this stage, which dP = dO V^T has finished reading
-        bwd_item<kBf16, false, kIrr>(c_now, tmem_s + sb * 64 + lane_base, tmem_dp + sb * 64 + lane_base,
-                               smem_u32(&sm->dp_free[sb]), kind, vis, scale_log2, scale, M2L, delta, 0u,
-                               v_slot(s), row, []() {},
-                               [&]() {
-                                 tc_fence_before();
-                                 mbar_arrive(smem_u32(&sm->s_free[sb]));
-                               },
-                               [&]() {
-                                 mbar_wait(smem_u32(&sm->dp_full[sb]), (it / kSdpBufs) & 1, &g_lmk_status, kErrDqSoftmax);
-                                 tc_fence_after();
-                               });
+        uint64_t sp[32];
+        const RowFactors f = bwd_weights<kIrr>(sp, c_now, tmem_s + sb * 64 + lane_base, kind, vis, scale_log2, M2L, [&]() {
+          tc_fence_before();
+          mbar_arrive(smem_u32(&sm->s_free[sb]));
+        });
+        mbar_wait(smem_u32(&sm->dp_full[sb]), (it / kSdpBufs) & 1, &g_lmk_status, kErrDqSoftmax);
+        tc_fence_after();
+        uint32_t wd[32];
+        bwd_dscores<kBf16, kIrr>(wd, sp, f, tmem_dp + sb * 64 + lane_base, smem_u32(&sm->dp_free[sb]), kind, scale, delta);
+        store_row_sw128(v_slot(s), row, wd);      // dS replaces the V tile of this stage, which dP has finished reading
         fence_proxy_async_smem();
         mbar_arrive(smem_u32(&sm->ds_ready[s]));
       }
@@ -1673,7 +1670,9 @@ template <int kTiles> constexpr size_t fwd_smem(bool irr) {
   return 1024 + (kTiles + kFwdStages<kTiles>) * 32768 + sizeof(Fwd2Smem<kFwdStages<kTiles>>) + (irr ? sizeof(IrrSmem) : 0);
 }
 static_assert(fwd_smem<2>(true) <= 232448 && fwd_smem<1>(true) <= 232448 / 2 - 1024, "shared memory of one SM");
-constexpr size_t kSmemDkv = 1024 + 65536 + kDkvStages * 65536 + 32768 + sizeof(DkvSmem);
+template <int kD> constexpr size_t kSmemDkv =
+    1024 + (2 + 2 * kDkvStages<kD>) * (kD / 64) * kTileBytes + 2 * kTileBytes + sizeof(DkvSmem<kDkvStages<kD>>);
+static_assert(kSmemDkv<128> <= 232448 && kSmemDkv<64> <= 232448, "shared memory of one SM");
 constexpr size_t kSmemDq = 1024 + 65536 + kDqStages * 32768 + 32768 + sizeof(DqSmem);
 
 int device_facts(const DeviceFacts** out) {
@@ -1694,15 +1693,12 @@ int device_facts(const DeviceFacts** out) {
     LMK_CUDA(cudaFuncSetAttribute(sm100_fwd2_kernel<BF, DIM, true, 2>, attr, (int)fwd_smem<2>(true)));       \
     LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, true, false>, attr, (int)kSmemDq));           \
     LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, false, false>, attr, (int)kSmemDq));          \
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, false, true>, attr, (int)kSmemDq));
-#define LMK_ATTRS_DKV(BF)                                                                                    \
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, true, false>, attr, (int)kSmemDkv));              \
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, false, false>, attr, (int)kSmemDkv));             \
-    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, false, true>, attr, (int)kSmemDkv));
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dq_kernel<BF, DIM, false, true>, attr, (int)kSmemDq));           \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, DIM, true, false>, attr, (int)kSmemDkv<DIM>));    \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, DIM, false, false>, attr, (int)kSmemDkv<DIM>));   \
+    LMK_CUDA(cudaFuncSetAttribute(sm100_bwd_dkv_kernel<BF, DIM, false, true>, attr, (int)kSmemDkv<DIM>));
     LMK_ATTRS(true, 128) LMK_ATTRS(true, 64) LMK_ATTRS(false, 128) LMK_ATTRS(false, 64)
-    LMK_ATTRS_DKV(true) LMK_ATTRS_DKV(false)
 #undef LMK_ATTRS
-#undef LMK_ATTRS_DKV
     f.ready = true;
   }
   *out = &f;
@@ -1861,7 +1857,7 @@ static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   if ((rc = make_map_4d(&tdo, p.dO, dtype, p.B, p.H, p.Lq, p.D, p.dos, kQTile)) != LMK_OK) return rc;
   float* delta = reinterpret_cast<float*>(p.workspace);
   const float scale_log2 = p.scale * kLog2e;
-  const size_t smem_dkv = kSmemDkv, smem_dq = kSmemDq;
+  const size_t smem_dkv = p.D <= 64 ? kSmemDkv<64> : kSmemDkv<128>, smem_dq = kSmemDq;
   CUtensorMap to;
   if ((rc = make_map_4d(&to, p.o, dtype, p.B, p.H, p.Lq, p.D, dense, kQTile)) != LMK_OK) return rc;
   const DeviceFacts* facts = nullptr;
@@ -1897,25 +1893,23 @@ static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   const float* Mc = p.M;
   const float* deltac = delta;
   const int BH = p.B * p.H;
-#define LMK_BWD_LAUNCH(BF, DIM, DQ_WHOLE, DKV_WHOLE, IRR)                                                                  \
+#define LMK_BWD_LAUNCH(BF, DIM, WHOLE, IRR)                                                                                \
   do {                                                                                                                     \
-    LMK_CUDA(cudaLaunchKernelEx(&cfg_dq, sm100_bwd_dq_kernel<BF, DIM, DQ_WHOLE, IRR>, tq, tk, tv, tdo, to, Lc, Mc, delta,  \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg_dq, sm100_bwd_dq_kernel<BF, DIM, WHOLE, IRR>, tq, tk, tv, tdo, to, Lc, Mc, delta,     \
                                 p.dq, p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2, args));                               \
-    LMK_CUDA(cudaLaunchKernelEx(&cfg_dkv, sm100_bwd_dkv_kernel<BF, DKV_WHOLE, IRR>, tq, tk, tv, tdo, Lc, Mc, deltac, p.dk, \
-                                p.dv, p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2, max_tiles, args));                    \
+    LMK_CUDA(cudaLaunchKernelEx(&cfg_dkv, sm100_bwd_dkv_kernel<BF, DIM, WHOLE, IRR>, tq, tk, tv, tdo, Lc, Mc, deltac,      \
+                                p.dk, p.dv, p.H, BH, p.Lq, p.Lk, p.D, p.scale, scale_log2, max_tiles, args));              \
+  } while (0)
+#define LMK_BWD_DIM(BF, DIM)                                                   \
+  do {                                                                         \
+    if (irr != nullptr) LMK_BWD_LAUNCH(BF, DIM, false, true);                  \
+    else if (whole && p.D == DIM) LMK_BWD_LAUNCH(BF, DIM, true, false);        \
+    else LMK_BWD_LAUNCH(BF, DIM, false, false);                                \
   } while (0)
 #define LMK_BWD_DTYPE(BF)                                                      \
   do {                                                                         \
-    if (irr != nullptr) {                                                      \
-      if (p.D <= 64) LMK_BWD_LAUNCH(BF, 64, false, false, true);               \
-      else LMK_BWD_LAUNCH(BF, 128, false, false, true);                        \
-    } else if (p.D <= 64) {                                                    \
-      if (whole && p.D == 64) LMK_BWD_LAUNCH(BF, 64, true, false, false);      \
-      else LMK_BWD_LAUNCH(BF, 64, false, false, false);                        \
-    } else {                                                                   \
-      if (whole && p.D == 128) LMK_BWD_LAUNCH(BF, 128, true, true, false);     \
-      else LMK_BWD_LAUNCH(BF, 128, false, false, false);                       \
-    }                                                                          \
+    if (p.D <= 64) LMK_BWD_DIM(BF, 64);                                        \
+    else LMK_BWD_DIM(BF, 128);                                                 \
   } while (0)
   const IrrArgs args = irr != nullptr ? *irr : IrrArgs{};
   // instances without bounds where every tile is whole (the checks and run-time strides cost 8 us of 147 at L = 2048)
@@ -1923,6 +1917,7 @@ static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   if (dtype == LMK_BF16) LMK_BWD_DTYPE(true);
   else LMK_BWD_DTYPE(false);
 #undef LMK_BWD_DTYPE
+#undef LMK_BWD_DIM
 #undef LMK_BWD_LAUNCH
   LMK_CUDA(cudaGetLastError());
   return LMK_OK;
