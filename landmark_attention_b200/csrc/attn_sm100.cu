@@ -1096,7 +1096,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // (rows past the end of the sequence have zero Q and dO tiles: whatever finite weights they get contribute nothing)
       const int64_t grow0 = (int64_t)bh * Lq + (kWhole ? tq0 * kQTile + row : min(tq0 * kQTile + row, Lq - 1));
       if (u == 0) grid_dep_wait();     // delta comes from the dQ kernel, which may still be running (see the launch)
-      float nM = stat_m(grow0), nL = stat_l(grow0), nDelta = delta_ptr[grow0];
+      float nM = stat_m(grow0), nL = stat_l(grow0), nDelta = ld_behind_wait(delta_ptr + grow0);
       int nOwn = own_of(tq0 * kQTile + row);
       for (int i = 0; i < n_items; ++i, ++it) {
         const int tq = tq0 + i;
@@ -1108,7 +1108,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const int64_t grow = (int64_t)bh * Lq + (kWhole ? (tq + 1) * kQTile + row : min((tq + 1) * kQTile + row, Lq - 1));
           nM = stat_m(grow);
           nL = stat_l(grow);
-          nDelta = delta_ptr[grow];
+          nDelta = ld_behind_wait(delta_ptr + grow);
           nOwn = own_of((tq + 1) * kQTile + row);
         }
         const int kind = n > own ? 0 : (n == own ? 1 : 2);
