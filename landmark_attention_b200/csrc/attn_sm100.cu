@@ -255,9 +255,9 @@ template <int kTiles> constexpr int kFwdStages = kTiles == 2 ? 5 : 2;
 template <int kTiles> constexpr int kFwdThreads = (4 * kTiles + 3) * 32;
 enum { kErrFwd2Producer = 111, kErrFwd2Mma = 112, kErrFwd2Softmax = 113, kErrFwd2Epilogue = 114 };
 
-// one in this many pairs of exponentials uses ex2_poly2 (measured at L = 8192: 2 -> 544 us, 4 -> 523, 8 -> 515, 64 -> 508;
-// no difference at L = 2048: the special-function pipe is not what the forward kernel waits for)
-constexpr int kFwdPolyEvery = 64;
+// one in this many pairs of exponentials uses ex2_poly2 (forward at B1 H32 L2048: 64 -> 44.7 us, 16 -> 43.7, 8 -> 42.6, 4 -> 43.1
+// device time; heads of 64 features show no difference)
+constexpr int kFwdPolyEvery = 8;
 
 template <int kStages> struct Fwd2Smem {
   uint64_t q_full;
