@@ -235,14 +235,19 @@ __global__ void __launch_bounds__(256) irr_plan_kernel(const uint8_t* __restrict
   for (int k = threadIdx.x; k < Lk; k += blockDim.x) own[k] = (uint8_t)irr_group(t, k);
 }
 
-// hides the columns of the group before: uniform tests, selects only in the chunks that need them
-__device__ __forceinline__ void irr_hide(float (&sv)[64], int c0) {
+// Hides the columns of the group before (c0 of them, the same for the whole warp), eight at a time up to the last one: eight tests of
+// their own, one a chunk, took 400 - 600 clk an item whatever c0 was (clock stamps, groups of 51), nested ones end with the chunk
+// that needs them.
+template <int kChunk = 0, typename GetFn>
+__device__ __forceinline__ void irr_hide(GetFn col, int c0) {
+  if constexpr (kChunk < 8) {
+    if (c0 > 8 * kChunk) {
 #pragma unroll
-  for (int ch = 0; ch < 8; ++ch)
-    if (c0 > 8 * ch) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) sv[8 * ch + e] = 8 * ch + e < c0 ? -INFINITY : sv[8 * ch + e];
+      for (int e = 0; e < 8; ++e)
+        if (8 * kChunk + e < c0) col(8 * kChunk + e) = -INFINITY;
+      irr_hide<kChunk + 1>(col, c0);
     }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------- forward, two tiles
@@ -455,6 +460,14 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int pos = min(pos_a + w * kQTile + row, Lk - 1);
     const int own = kIrr ? group_of(pos) : own0_a + 2 * w + half;
     const int vis = min(kIrr ? 63 - (end_of(own) - pos) : row & 63, kBlk - 2);
+    // kIrr: newest and oldest own tile of the warp's rows; ends of the next tile that this warp takes and of the one before it
+    const int own_max = kIrr ? __reduce_max_sync(0xffffffffu, own) : own, own_min = kIrr ? __reduce_min_sync(0xffffffffu, own) : own;
+    int e_hi = 0, e_lo = 0;
+    if constexpr (kIrr) {
+      const int first = kTiles == 2 && w == 0 ? last_a : n_last;
+      e_hi = end_of(first);
+      e_lo = end_of(first - 1);
+    }
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     float m2 = -INFINITY, l = 0.f;
     int k = 0;
@@ -500,10 +513,12 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // (votes), because the TMEM accesses behind it have to be executed by all lanes together.
         bool later = n > own, mixed = false;
         if constexpr (kIrr) {
-          const int c0 = 64 - (end_of(n) - end_of(n - 1));
-          irr_hide(sv, c0);
-          later = __all_sync(0xffffffffu, n > own);
-          mixed = !later && (c0 == 63 || !__all_sync(0xffffffffu, n < own));      // (c0 == 63: a landmark without keys)
+          const int c0 = warp_uniform(64 - (e_hi - e_lo));
+          e_hi = e_lo;
+          if (n > 0) e_lo = end_of(n - 2);
+          later = n > own_max;
+          if (!later) irr_hide([&](int j) -> float& { return sv[j]; }, c0);
+          mixed = !later && (c0 == 63 || n >= own_min);      // (c0 == 63: a landmark without keys)
         }
         if (later) {
 #pragma unroll
@@ -511,13 +526,16 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         } else if (kIrr && mixed) {
           const bool earlier = n < own;
           const int last = earlier ? kBlk - 2 : (n == own ? vis : -1);
-          const float mx = row_max_upto(sv, last) * scale_log2;
+          const float lm = sv[63];
+#pragma unroll
+          for (int j = 0; j < 64; ++j) sv[j] = j <= last ? sv[j] : -INFINITY;
+          const float mx = row_max<63>(sv) * scale_log2;
           if (n == own) m2 = fmaxf(m2, mx);
-          const float el = earlier ? ex2(fmaf(sv[63], scale_log2, -m2)) : 0.f;
+          const float el = earlier ? ex2(fmaf(lm, scale_log2, -m2)) : 0.f;
           float shift = earlier ? mx : m2;
           shift = shift == -INFINITY ? 0.f : shift;                               // nothing visible
 #pragma unroll
-          for (int j = 0; j < 64; ++j) sv[j] = (j <= last) ? ex2(fmaf(sv[j], scale_log2, -shift)) : 0.f;
+          for (int j = 0; j < 64; ++j) sv[j] = ex2(fmaf(sv[j], scale_log2, -shift));      // (hidden ones: 0)
           const float sum = row_sum<64>(sv);
           const float wg = earlier ? (sum > 0.f ? __fdividef(el, sum) : 0.f) : 1.f;
           l += earlier ? el : sum;
@@ -651,19 +669,8 @@ __device__ __forceinline__ RowFactors bwd_weights(uint64_t (&sp)[32], int c0, ui
     tmem_ld_32x32b_x32(ts, ra);
     tmem_ld_32x32b_x32(ts + 32, rb);
     tmem_ld_wait();
-    if constexpr (kIrr) {             // the first c0 columns belong to the group before (uniform tests, see irr_hide)
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        if (c0 > 8 * ch) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) ra[8 * ch + e] = 8 * ch + e < c0 ? 0xff800000u : ra[8 * ch + e];
-        }
-        if (c0 > 32 + 8 * ch) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) rb[8 * ch + e] = 32 + 8 * ch + e < c0 ? 0xff800000u : rb[8 * ch + e];
-        }
-      }
-    }
+    if constexpr (kIrr)               // the first c0 columns belong to the group before
+      irr_hide([&](int j) -> float& { return reinterpret_cast<float&>(j < 32 ? ra[j] : rb[j - 32]); }, c0);
     if (kIrr || kind == 2) {
       float sv[64];
 #pragma unroll
@@ -1082,35 +1089,56 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t my_tile = w_tile + (uint32_t)g * kTileBytes;
     int it = 0, u = 0;
-    for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-      if (skipped(w)) continue;
-      const int pair = w / BH, bh = w - pair * BH, b = bh / H;
-      const int n = 2 * pair + g;
-      const int tq0 = unit_tq0(w), n_items = n_tiles - tq0;
-      const bool tile_exists = n < tiles_of(b);
-      const int end = kIrr && tile_exists ? end_of(b, n) : 0, c0 = kIrr && tile_exists ? 64 - (end - end_of(b, n - 1)) : 0;
-      auto stat_m = [&](int64_t i) { return kIrr && irr.R != nullptr ? irr.R[i] : M_ptr[i]; };
-      auto stat_l = [&](int64_t i) { return kIrr && irr.R != nullptr ? 1.f : L_ptr[i]; };
-      auto own_of = [&](int r) { return kIrr ? group_of(b, min(Lk - Lq + r, Lk - 1)) : 0; };
-      // the row statistics of the next item are fetched one item ahead, so their latency is never exposed
-      // (rows past the end of the sequence have zero Q and dO tiles: whatever finite weights they get contribute nothing)
-      const int64_t grow0 = (int64_t)bh * Lq + (kWhole ? tq0 * kQTile + row : min(tq0 * kQTile + row, Lq - 1));
-      if (u == 0) grid_dep_wait();     // delta comes from the dQ kernel, which may still be running (see the launch)
-      float nM = stat_m(grow0), nL = stat_l(grow0), nDelta = ld_behind_wait(delta_ptr + grow0);
-      int nOwn = own_of(tq0 * kQTile + row);
+    auto stat_m = [&](int64_t i) { return kIrr && irr.R != nullptr ? irr.R[i] : M_ptr[i]; };
+    auto stat_l = [&](int64_t i) { return kIrr && irr.R != nullptr ? 1.f : L_ptr[i]; };
+    // What a unit needs from global memory, asked for while the unit before it drains: the tile table first (all entries at
+    // once), then the row statistics of the first item.  Read one after the other at the start of a unit they took 1500 - 2000 clk of it.
+    // (rows past the end of the sequence have zero Q and dO tiles: whatever finite weights they get contribute nothing)
+    int bh = -1, b = 0, pair = 0, tq0 = 0, tiles = n_blocks, e_m = 0, e_0 = 0, e_1 = 0;      // bh < 0: no unit left
+    float nM = 0.f, nL = 1.f, nDelta = 0.f;
+    int nOwn = 0;
+    auto own_of = [&](int r) { return kIrr ? group_of(b, min(Lk - Lq + r, Lk - 1)) : 0; };
+    auto fetch_rows = [&](int tq) {
+      const int64_t grow = (int64_t)bh * Lq + (kWhole ? tq * kQTile + row : min(tq * kQTile + row, Lq - 1));
+      nM = stat_m(grow);
+      nL = stat_l(grow);
+      nDelta = ld_behind_wait(delta_ptr + grow);
+      nOwn = own_of(tq * kQTile + row);
+    };
+    int r = 0;
+    auto fetch_unit = [&]() {                       // kIrr
+      for (;; ++r) {
+        const int w = unit_of(r);
+        if (w >= n_units) {
+          bh = -1;
+          return;
+        }
+        pair = w / BH;
+        bh = w - pair * BH;
+        b = bh / H;
+        const bool fallback = irr.flags != nullptr && irr_plan_fallback(irr.plan, b);
+        tiles = tiles_of(b);
+        e_m = end_of(b, 2 * pair - 1);              // (entries behind the last tile: inside the table, not used)
+        e_0 = end_of(b, 2 * pair);
+        e_1 = end_of(b, 2 * pair + 1);
+        if (fallback || 2 * pair >= tiles) continue;
+        tq0 = max(e_m + 1 - (Lk - Lq), 0) / kQTile;
+        fetch_rows(tq0);
+        ++r;
+        return;
+      }
+    };
+    auto run_unit = [&]() {
+      const int n = 2 * pair + g, n_items = n_tiles - tq0;
+      const int end = g == 0 ? e_0 : e_1;
+      const int c0 = kIrr && n < tiles ? warp_uniform(64 - (end - (g == 0 ? e_m : e_0))) : 0;
       for (int i = 0; i < n_items; ++i, ++it) {
         const int tq = tq0 + i;
         const int own = kIrr ? nOwn : prefix_blocks + 2 * tq + half;
         const int vis = min(kIrr ? 63 - (end - (Lk - Lq + tq * kQTile + row)) : row & 63, kBlk - 2);      // used where n == own
         const bool row_valid = kWhole || tq * kQTile + row < Lq;
         const float M2L = !row_valid ? 0.f : (kIrr && irr.R != nullptr ? nM : fmaf(nM, kLog2e, __log2f(nL))), delta = row_valid ? nDelta : 0.f;
-        if (i + 1 < n_items) {
-          const int64_t grow = (int64_t)bh * Lq + (kWhole ? (tq + 1) * kQTile + row : min((tq + 1) * kQTile + row, Lq - 1));
-          nM = stat_m(grow);
-          nL = stat_l(grow);
-          nDelta = ld_behind_wait(delta_ptr + grow);
-          nOwn = own_of((tq + 1) * kQTile + row);
-        }
+        if (i + 1 < n_items) fetch_rows(tq + 1);      // one item ahead, so that their latency is never exposed
         const int kind = n > own ? 0 : (n == own ? 1 : 2);
         mbar_wait(smem_u32(&sm->s_full), it & 1, &g_lmk_status, kErrDkvSoftmax);
         tc_fence_after();
@@ -1144,18 +1172,15 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         int key = n_r * kBlk + (row & 63);
         bool stored = key < Lk;
         if (kIrr) {
-          stored = n_r < tiles_of(b);
-          if (stored) {
-            const int end_r = end_of(b, n_r);
-            key = end_r - 63 + (row & 63);
-            stored = key > end_of(b, n_r - 1) && key < Lk;       // the tile's own keys
-          }
+          key = (half == 0 ? e_0 : e_1) - 63 + (row & 63);
+          stored = n_r < tiles && key > (half == 0 ? e_m : e_0) && key < Lk;       // the tile's own keys
         }
         if (stored) off = ((int64_t)bh * Lk + key) * D;
       }
       int64_t row_off[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) row_off[j] = __shfl_sync(0xffffffffu, off, (lane & ~3) + j);
+      if constexpr (kIrr) fetch_unit();
       mbar_wait(smem_u32(&sm->acc_full[g]), u & 1, &g_lmk_status, kErrDkvEpilogue);
       tc_fence_after();
       if (kIrr) __syncwarp();
@@ -1175,6 +1200,20 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         store_acc_cols<kBf16>(out, row_off, rb, c * 64 + 32, D, lane);
       }
       ++u;
+    };
+    if constexpr (kIrr) {
+      grid_dep_wait();     // delta comes from the dQ kernel, which may still be running (see the launch)
+      fetch_unit();
+      while (bh >= 0) run_unit();
+    } else {               // nothing but the statistics to ask for: holding them over the epilogue's stores costs more than it hides
+      for (int k = 0, w = unit_of(0); w < n_units; w = unit_of(++k)) {
+        pair = w / BH;
+        bh = w - pair * BH;
+        tq0 = unit_tq0(w);
+        if (u == 0) grid_dep_wait();
+        fetch_rows(tq0);
+        run_unit();
+      }
     }
     tc_fence_before();
   }
@@ -1438,7 +1477,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
       const int t = unit_tile(w), bh = w % BH, b = bh / H;
-      const int total = unit_items(w), n_last = total - 1;
+      int total = kIrr ? 0 : unit_items(w);
       const int64_t grow = (int64_t)bh * Lq + t * kQTile + row;
       const bool row_valid = kWhole || t * kQTile + row < Lq;
       const float M2L = kIrr && irr.R != nullptr ? nM : fmaf(nM, kLog2e, __log2f(nL));
@@ -1450,13 +1489,18 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           nL = kIrr && irr.R != nullptr ? 1.f : L_ptr[gn];
         }
       }
-      if (skipped(w)) continue;                     // after the prefetch, which belongs to the next unit
+      // tile table: everything that depends on the unit alone first, then what hangs on it (kIrr: loads from global memory)
       const int pos = min(Lk - Lq + t * kQTile + row, Lk - 1);
+      const bool skip = skipped(w);
+      if constexpr (kIrr) total = warp_uniform(unit_items(w));
+      const int n_last = total - 1;
       const int own = kIrr ? group_of(b, pos) : prefix_blocks + 2 * t + half;
-      const int vis = min(kIrr ? 63 - (end_of(b, own) - pos) : row & 63, kBlk - 2);
+      if (skip) continue;                           // after the prefetch, which belongs to the next unit
+      const int end_own = kIrr ? end_of(b, own) : 0;
       // kIrr: first visible column of this warpgroup's items, read one item ahead (hidden columns of tile n)
-      auto first_col = [&](int n) { return n < 0 ? 0 : 64 - (end_of(b, n) - (n > 0 ? end_of(b, n - 1) : -1)); };
+      auto first_col = [&](int n) { return n < 0 ? 0 : warp_uniform(64 - (end_of(b, n) - (n > 0 ? end_of(b, n - 1) : -1))); };
       int c0 = kIrr ? first_col(n_last - ((it0 + g) & 1)) : 0;
+      const int vis = min(kIrr ? 63 - (end_own - pos) : row & 63, kBlk - 2);
       // delta = rowsum(O * dO), straight from the swizzled tiles (one row per thread, 16-byte chunks); warpgroup 0
       // also publishes it for the dK/dV kernel, which runs after this one
       mbar_wait(smem_u32(&sm->qdo_full), u & 1, &g_lmk_status, kErrDqSoftmax);
