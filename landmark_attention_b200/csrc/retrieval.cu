@@ -687,6 +687,14 @@ __global__ void __launch_bounds__(128) selected_pv_kernel(const T* __restrict__ 
   }
 }
 
+// packed pair of a 16-bit type -> packed fp32 pair
+template <typename T>
+__device__ __forceinline__ uint64_t pair_f32(uint32_t w) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) return ptx::pk2u(w << 16, w & 0xffff0000u);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  return ptx::pk2(f.x, f.y);
+}
+
 // Attention over the selected blocks, fused with the merge into the attention over the local keys: nothing between
 // the block reads and the final output goes through global memory (no logits, no probabilities).  One CTA per
 // (token, batch*head); warp i takes selected block i (then i + 4, ...):
@@ -840,17 +848,38 @@ __global__ void __launch_bounds__(128, 8) selected_attend_kernel(const T* __rest
     __syncwarp();
     // o_i = sum_r p_r V[r]: LPR lanes cover one value row, VGROUPS rows per step
     const int vcol = lane % LPR, rg = lane / LPR;
-    float acc[VEC];
-#pragma unroll
-    for (int u = 0; u < VEC; ++u) acc[u] = 0.f;
     const T* vsrc = vbase + (int64_t)sel * vd.stride_block + vcol * VEC;
-    if (rg < VGROUPS) {
-#pragma unroll 4
-      for (int r = rg; r < blk; r += VGROUPS) {
-        const Vec v = *reinterpret_cast<const Vec*>(vsrc + (int64_t)r * vd.stride_row);
-        const float p = lrow[r];
+    float acc[VEC];
+    if constexpr (sizeof(T) == 2) {
+      // two features an instruction: the same sums with half the multiply-adds (T258, H32, top 4 of 1024 blocks of 32: the kernel
+      // 95.2 -> 93.8 us)
+      uint64_t acc2[VEC / 2];
 #pragma unroll
-        for (int u = 0; u < VEC; ++u) acc[u] = fmaf(p, to_f32(v.v[u]), acc[u]);
+      for (int u = 0; u < VEC / 2; ++u) acc2[u] = 0ull;
+      if (rg < VGROUPS) {
+#pragma unroll 4
+        for (int r = rg; r < blk; r += VGROUPS) {
+          uint32_t w[4];
+          ld16(vsrc + (int64_t)r * vd.stride_row, w);
+          const float p = lrow[r];
+          const uint64_t p2 = ptx::pk2(p, p);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) acc2[u] = ptx::fma2(p2, pair_f32<T>(w[u]), acc2[u]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < VEC / 2; ++u) ptx::upk2(acc2[u], acc[2 * u], acc[2 * u + 1]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < VEC; ++u) acc[u] = 0.f;
+      if (rg < VGROUPS) {
+#pragma unroll 4
+        for (int r = rg; r < blk; r += VGROUPS) {
+          const Vec v = *reinterpret_cast<const Vec*>(vsrc + (int64_t)r * vd.stride_row);
+          const float p = lrow[r];
+#pragma unroll
+          for (int u = 0; u < VEC; ++u) acc[u] = fmaf(p, to_f32(v.v[u]), acc[u]);
+        }
       }
     }
 #pragma unroll
