@@ -1919,20 +1919,16 @@ static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   // right after its set-up (only the set-up overlaps).  The dK/dV kernel reads q, k, v, dO, L, M, which were complete
   // before the dQ kernel started, and `delta`, which the dQ kernel writes: its loads and S / dP products start on
   // every SM the dQ kernel has left, and only its softmax threads wait (griddepcontrol.wait) before they read delta.
-  // Not for other landmark patterns outside of graphs: the dK/dV kernel's units start late there (plan, gathered landmarks), and
-  // its CTAs that wait on SMs which the dQ kernel has left cost more than they hide (B16 H8 T512, groups of 51: the layer
-  // 212 -> 215 us; blocks of 64 at B1 H32 L2048 206 -> 203, B4 H16 L1024 D64 120 -> 118.5).
+  // (Blocks of 64 at B1 H32 L2048 206 -> 203 us, B4 H16 L1024 D64 120 -> 118.5; the layer with groups of 51 at B16 H8 T512
+  // 166.7 -> 161.2.)
   cudaLaunchAttribute pdl[1];
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  LMK_CUDA(cudaStreamIsCapturing(st, &capturing));
-  const unsigned n_attrs = irr == nullptr || capturing == cudaStreamCaptureStatusActive ? 1u : 0u;
   cudaLaunchConfig_t cfg_dq = {}, cfg_dkv = {};
   cfg_dq.gridDim = grid_dq;  cfg_dq.blockDim = dim3(kDqThreads);  cfg_dq.dynamicSmemBytes = smem_dq;  cfg_dq.stream = st;
-  cfg_dq.attrs = pdl;  cfg_dq.numAttrs = n_attrs;
+  cfg_dq.attrs = pdl;  cfg_dq.numAttrs = 1;
   cfg_dkv.gridDim = grid_dkv;  cfg_dkv.blockDim = dim3(kBwdThreads);  cfg_dkv.dynamicSmemBytes = smem_dkv;
-  cfg_dkv.stream = st;  cfg_dkv.attrs = pdl;  cfg_dkv.numAttrs = n_attrs;
+  cfg_dkv.stream = st;  cfg_dkv.attrs = pdl;  cfg_dkv.numAttrs = 1;
   const float* Lc = p.L;
   const float* Mc = p.M;
   const float* deltac = delta;
