@@ -1057,8 +1057,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int s = it % kStages;
         const uint64_t ddot = desc_advance(ddo0t, (uint32_t)s * 2 * kOperand), dqt = desc_advance(dq0t, (uint32_t)s * 2 * kOperand);
         mbar_wait(smem_u32(&sm->do_full[s]), (it / kStages) & 1, &g_lmk_status, kErrDkvMma);
-        mbar_wait(smem_u32(&sm->p_ready), it & 1, &g_lmk_status, kErrDkvMma);
         if (i == 0) mbar_wait(smem_u32(&sm->acc_empty[0]), (u & 1) ^ 1, &g_lmk_status, kErrDkvMma);
+        mbar_wait(smem_u32(&sm->p_ready), it & 1, &g_lmk_status, kErrDkvMma);
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -1068,8 +1068,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           mma_commit(smem_u32(&sm->do_empty[s]));
           if (i == n_items - 1) mma_commit(smem_u32(&sm->acc_full[0]));
         }
-        mbar_wait(smem_u32(&sm->ds_ready), it & 1, &g_lmk_status, kErrDkvMma);
         if (i == 0) mbar_wait(smem_u32(&sm->acc_empty[1]), (u & 1) ^ 1, &g_lmk_status, kErrDkvMma);
+        mbar_wait(smem_u32(&sm->ds_ready), it & 1, &g_lmk_status, kErrDkvMma);
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -1378,12 +1378,13 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
         if (warp_uniform(skipped(w))) continue;
         const int total = warp_uniform(unit_items(w));
-        mbar_wait(smem_u32(&sm->ops_ready), u & 1, &g_lmk_status, kErrDqMma);
         for (int i = 0; i < total; ++i, ++it) {
           const int s = it % kDqStages, sb = it % kSdpBufs;
           mbar_wait(smem_u32(&sm->full[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
           if (it >= kSdpBufs)
             mbar_wait(smem_u32(is_s ? &sm->s_free[sb] : &sm->dp_free[sb]), ((it / kSdpBufs) & 1) ^ 1, &g_lmk_status, kErrDqMma);
+          // the unit's rows come last: waited for in front of the other two they cost the unit another 1000 clk
+          if (i == 0) mbar_wait(smem_u32(&sm->ops_ready), u & 1, &g_lmk_status, kErrDqMma);
           tc_fence_after();
           const uint64_t db = desc_advance(db0, (uint32_t)s * 32768u);
           if (elect_one()) {
@@ -1410,8 +1411,8 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int total = warp_uniform(unit_items(w));
         for (int i = 0; i < total; ++i, ++it) {
           const int s = it % kDqStages;
-          mbar_wait(smem_u32(&sm->ds_ready[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
           if (i == 0) mbar_wait(smem_u32(&sm->acc_empty), (u & 1) ^ 1, &g_lmk_status, kErrDqMma);
+          mbar_wait(smem_u32(&sm->ds_ready[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
           tc_fence_after();
           const uint64_t dds = desc_advance(dv0, (uint32_t)s * 32768u), dkt = desc_advance(dk0t, (uint32_t)s * 32768u);
           if (elect_one()) {
