@@ -1370,7 +1370,7 @@ __global__ void __launch_bounds__(kGsWarps * 32, K == 32 ? 8 : 6)
 // probabilities; scores and local output as mma.sync tiles, rounded where the tensor formulation rounds (the product, the
 // scaling, the probabilities, the output).  Written out: the prefix' probabilities (fp32) and the local output.
 // Bound by latency: 5 MB of operands and 80 MB of prefix logits and probabilities at B16 H8 T255 P204; library products, scaling,
-// concatenation, softmax and casts as kernels of their own took 167 us, this one takes 116 us (32 rows a CTA, half as many warps an SM: 130).
+// concatenation, softmax and casts as kernels of their own took 167 us, this one takes 98 us (32 rows a CTA, half as many warps an SM: 130).
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kCrRows = 16, kCrTiles = kCrRows / 16, kCrThreads = 256, kCrVPitch = 136;
 constexpr size_t kCrMaxSmem = 224 * 1024;
@@ -1388,9 +1388,13 @@ struct CrParams {
 };
 __host__ __device__ constexpr int cr_pieces(int W) { return (W + 10 + 127) / 128; }      // lead, and scores are computed for eight keys at a time
 __host__ __device__ constexpr int cr_prob_pitch(int T) { return ((T + 15) & ~15) + 8; }
-__host__ __device__ constexpr size_t cr_smem(int T, int P) {
-  return sizeof(float) * kCrRows * 144 * (size_t)cr_pieces(P + T) + 2 * (size_t)kCrRows * cr_prob_pitch(T) + 2 * 64 * kCrVPitch;
+// The rows of scores; once their probabilities are written the value tiles take their place, which leaves room for a fourth CTA on
+// an SM (62.7 -> 45.3 KB at B16 H8 T255 P204: the kernel 111 -> 98.4 us).
+__host__ __device__ constexpr size_t cr_rows_bytes(int W) {
+  const size_t rows = sizeof(float) * kCrRows * 144 * (size_t)cr_pieces(W), values = 2 * 64 * kCrVPitch;
+  return rows > values ? rows : values;
 }
+__host__ __device__ constexpr size_t cr_smem(int T, int P) { return cr_rows_bytes(P + T) + 2 * (size_t)kCrRows * cr_prob_pitch(T); }
 
 // A row in which landmarks share a lane (cached rows).  The groups between a lane's landmarks lie in the lane: it works them out first,
 // one after the other, as far as exponential over sum; the rest of the row goes the way of the other rows, and the last pass, back to
@@ -1464,8 +1468,8 @@ __global__ void __launch_bounds__(kCrThreads, K == 32 ? 4 : 2) cached_rows_kerne
   const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kCrRows;             // longest rows first
   const int W = p.P + p.T, n4max = cr_pieces(W), row_floats = 144 * n4max, pitch = cr_prob_pitch(p.T);
   const int lead = (4 - (p.P & 3)) & 3;                                       // the chunk's first key starts a piece
-  T* pb = reinterpret_cast<T*>(gs_smem + kCrRows * row_floats);               // [16][pitch] local probabilities
-  T* vt = pb + kCrRows * pitch;                                               // [64][kCrVPitch] values
+  T* pb = reinterpret_cast<T*>(gs_smem + cr_rows_bytes(W) / sizeof(float));   // [16][pitch] local probabilities
+  T* vt = reinterpret_cast<T*>(gs_smem);                                      // [64][kCrVPitch] values, when the scores are done with
   const T* q = reinterpret_cast<const T*>(p.q) + b * p.qs[0] + h * p.qs[1];
   const T* k = reinterpret_cast<const T*>(p.k) + b * p.ks[0] + h * p.ks[1];
   const T* v = reinterpret_cast<const T*>(p.v) + b * p.vs[0] + h * p.vs[1];
@@ -1568,7 +1572,7 @@ __global__ void __launch_bounds__(kCrThreads, K == 32 ? 4 : 2) cached_rows_kerne
   // ---- local output: warp w has features 16 w .. 16 w + 15 of all rows
   float acc[kCrTiles][2][4] = {};
   for (int j0 = 0; j0 < n_keys; j0 += 64) {
-    __syncthreads();                                    // probabilities written; the tile before has been read
+    __syncthreads();                                    // probabilities written, scores done with; the tile before has been read
     for (int e = tid; e < 64 * 16; e += kCrThreads) {
       const int r = e >> 4, c = (e & 15) * 8;
       uint4 x = make_uint4(0u, 0u, 0u, 0u);
@@ -1808,7 +1812,7 @@ extern "C" int lmk_grouped_softmax_causal_bwd_typed(const void* x, const int64_t
 
 extern "C" int lmk_cached_rows_supported(int D, int T, int P, int dtype) {
   return (dtype == LMK_BF16 || dtype == LMK_F16) && D == 128 && T >= 1 && P >= 1 && P + T <= 2000 &&
-         lmk::cr_smem(T, P) <= lmk::kCrMaxSmem ? 1 : 0;
+         lmk::cr_smem(T, P) + 2 * 64 * lmk::kCrVPitch <= lmk::kCrMaxSmem ? 1 : 0;      // as when the values had room of their own
 }
 
 extern "C" int lmk_cached_rows(const void* q, const void* k, const void* v, const int64_t q_strides[3], const int64_t k_strides[3],
