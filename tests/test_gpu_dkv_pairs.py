@@ -1,0 +1,44 @@
+"""dK / dV units of two key blocks, for head dims of one and two 64-feature sub-tiles: sequences whose last pair has one block,
+units of a single query tile, key histories, and CTAs that walk through one or many units (the same bits whatever their number)."""
+import pytest
+import torch
+
+import landmark_attention_b200 as P
+from landmark_attention_b200 import _lib as L
+from oracle import landmark_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("B,H,Lq,hist,D,dtype", [
+    (1, 3, 320, 0, 64, torch.bfloat16), (2, 2, 192, 64, 64, torch.float16), (1, 5, 128, 192, 64, torch.bfloat16),
+    (1, 3, 320, 0, 128, torch.float16), (2, 3, 64, 64, 128, torch.bfloat16), (1, 4, 384, 320, 128, torch.bfloat16),
+    (1, 4, 449, 64, 48, torch.bfloat16), (1, 2, 449, 0, 112, torch.float16)])
+def test_units_of_key_block_pairs(B, H, Lq, hist, D, dtype):
+    g = torch.Generator().manual_seed(Lq + hist + D)
+    Lk = Lq + hist
+    q, k, v = [(torch.randn(B, H, n, D, generator=g) * 0.5).to(dtype) for n in (Lq, Lk, Lk)]
+    do = torch.randn(B, H, Lq, D, generator=g).to(dtype)
+
+    def run(cap):
+        L.lib().lmk_debug_set_max_ctas(cap)
+        try:
+            qc, kc, vc = [t.to(DEV).requires_grad_(True) for t in (q, k, v)]
+            out = P.fused_landmark_attention(qc, kc, vc, None, block_size=64)
+            return torch.autograd.grad(out, [qc, kc, vc], do.to(DEV))
+        finally:
+            L.lib().lmk_debug_set_max_ctas(0)
+
+    ref = run(0)
+    for cap in (1, 2, 5):
+        assert all(torch.equal(a, b) for a, b in zip(run(cap), ref)), cap
+    pad = -Lq % 64                                         # the oracle wants whole blocks: zero rows behind the real ones
+    fp = [torch.nn.functional.pad(t.float(), (0, 0, 0, pad)) for t in (q, k, v, do)]
+    exp = O.landmark_attention_grads(*fp, 64, sm_scale=D ** -0.5)[1:]
+    for name, got, e, n in zip(("dq", "dk", "dv"), ref, exp, (Lq, Lk, Lk)):
+        got, e = got.float().cpu(), e[:, :, :n]
+        # P and dS are rounded to 16 bits in front of the products and the results behind them: the bound of the other kernel tests
+        assert (got - e).abs().max().item() < 2e-2 * max(1.0, e.abs().max().item()), name
+        assert ((got - e).norm() / e.norm()).item() < 1e-2, name
+    assert L.device_status() == 0
