@@ -260,8 +260,8 @@ template <int kTiles> constexpr int kFwdStages = kTiles == 2 ? 5 : 2;
 template <int kTiles> constexpr int kFwdThreads = (4 * kTiles + 3) * 32;
 enum { kErrFwd2Producer = 111, kErrFwd2Mma = 112, kErrFwd2Softmax = 113, kErrFwd2Epilogue = 114 };
 
-// one in this many pairs of exponentials uses ex2_poly2 (forward at B1 H32 L2048: 64 -> 44.7 us, 16 -> 43.7, 8 -> 42.6, 4 -> 43.1
-// device time; heads of 64 features show no difference)
+// one in this many pairs of exponentials uses ex2_poly2, of degree 4 (calls at B1 H32 L2048: 32 -> 42.2 us, 16 -> 41.3, 8 -> 39.9;
+// a cubic 39.8.  Further from the truth by less than a cubic in one pair of 64: 2.7e-6 / 8 against 7.5e-5 / 64 on average)
 constexpr int kFwdPolyEvery = 8;
 
 template <int kStages> struct Fwd2Smem {
@@ -557,7 +557,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           for (int j = 0; j < 32; ++j) {
             const uint64_t x = fma2(pk2(sv[2 * j], sv[2 * j + 1]), c2, n2);
             if (j % kFwdPolyEvery == 1) {
-              sp[j] = ex2_poly2(x);       // a share of the exponentials runs on the FMA pipe
+              sp[j] = ex2_poly2<4>(x);       // a share of the exponentials runs on the FMA pipe
             } else {
               float a, b;
               upk2(x, a, b);
@@ -725,7 +725,7 @@ __device__ __forceinline__ RowFactors bwd_weights(uint64_t (&sp)[32], int c0, ui
     for (int j = 0; j < 32; ++j) {
       const uint64_t x = fma2(sp[j], c2, n2);
       if (j % kBwdPolyEvery == 1) {
-        sp[j] = ex2_poly2(x);         // a share of the exponentials runs on the FMA pipe
+        sp[j] = ex2_poly2<3>(x);         // a share of the exponentials runs on the FMA pipe
       } else {
         float a, b;
         upk2(x, a, b);
