@@ -1791,12 +1791,16 @@ int tensor_map_4d(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int 
 bool tensor_map_operand_ok(const void* p, const int64_t st[3]) { return tma_ok(p, st); }
 
 // Two query tiles a CTA share one K/V stream; one tile a CTA puts two CTAs on an SM, whose starts and ends overlap and which the
-// hardware deals out in smaller pieces.  Measured (us, one / two): 32 heads of L = 512 14.4 / 16.5, 1024 24.7 / 25.0, 1536 35.0 /
-// 33.1, 2048 50.0 / 47.5, 4096 164 / 148; 8 heads of 2048 (less than two CTAs an SM) 36.9 / 39.0; 51-key groups, 128 heads of
-// 512 37.0 / 41.1, 32-key blocks at 2000 105 / 109.  A single tile of a long history wants the deeper pipeline of the second form.
-static int fwd_tiles_per_cta(int n_tiles, int BH, int n_sm, bool irr) {
+// hardware deals out in smaller pieces.  Measured (us a call, one / two): D128, 32 heads of L = 512 11.5 / 13.5, 768 15.3 / 17.1,
+// 896 19.2 / 17.3, 1024 22.2 / 20.7, 2048 43.0 / 39.9, 8192 545 / 469; 256 heads of 512 45.9 / 49.7; small grids, 8 heads of 1024 18.0 /
+// 18.8, 3072 44.1 / 45.1, 4096 61.7 / 59.7.  Heads of 64 features have half the products for the stream to feed: 64 heads of 1024
+// 22.2 / 25.7, of 2048 66 / 73, 32 heads of 4096 112 / 118, 8192 423 / 409.  Groups as key tiles: 51 keys, 128 heads of 512 29.6 / 31.7,
+// 32 heads of 1024 28.2 / 31.4, 32-key blocks at 1280 51.1 / 54.1, 1700 69.0 / 67.3.  A single tile of a long history wants the deeper
+// pipeline of the second form.
+static int fwd_tiles_per_cta(int n_tiles, int BH, int n_sm, bool irr, int D) {
   if (n_tiles == 1) return 2;
-  return n_tiles <= (irr ? 16 : 8) || (int64_t)n_tiles * BH <= 2 * n_sm ? 1 : 2;
+  const int most = irr ? 12 : D <= 64 ? 32 : 6;
+  return n_tiles <= most || (int64_t)n_tiles * BH <= n_sm + n_sm / 2 ? 1 : 2;
 }
 
 static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaStream_t st) {
@@ -1817,7 +1821,7 @@ static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   const DeviceFacts* facts = nullptr;
   if ((rc = device_facts(&facts)) != LMK_OK) return rc;
   const int n_tiles = (p.Lq + kQTile - 1) / kQTile;
-  const int per_cta = fwd_tiles_per_cta(n_tiles, p.B * p.H, facts->n_sm, other);
+  const int per_cta = fwd_tiles_per_cta(n_tiles, p.B * p.H, facts->n_sm, other, p.D);
   const dim3 grid(p.B * p.H, (n_tiles + per_cta - 1) / per_cta);
   // With the programmatic-stream-serialization attribute the set-up (barriers, TMEM, tensor maps) may run while the kernel in
   // front drains: it is a quarter of a short prompt's time (L = 77: 8.2 -> 5.9 us a call).
