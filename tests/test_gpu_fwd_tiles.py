@@ -1,0 +1,28 @@
+"""Forward on both sides of the lines between one and two query tiles a CTA: by sequence length for blocks of 64, for heads of 64
+features and for groups as key tiles, and by the size of the grid."""
+import pytest
+import torch
+
+import landmark_attention_b200 as P
+from landmark_attention_b200 import _lib as L
+from oracle import landmark_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,Lq,D,block", [
+    (40, 768, 128, 64), (40, 896, 128, 64), (1, 896, 128, 64), (40, 833, 128, 64),      # six and seven tiles, few and many heads
+    (8, 4096, 64, 64), (8, 4224, 64, 64),                                               # 32 and 33 tiles
+    (20, 1536, 128, 32), (20, 1664, 128, 32)])                                          # twelve and thirteen tiles
+def test_both_sides_of_the_tile_lines(H, Lq, D, block):
+    g = torch.Generator().manual_seed(Lq + H)
+    q, k, v = [(torch.randn(1, H, Lq, D, generator=g) * 0.5).to(torch.bfloat16) for _ in range(3)]
+    out = P.fused_landmark_attention(q.cuda(), k.cuda(), v.cuda(), None, block_size=block)
+    pad = -Lq % block                                      # the oracle wants whole blocks: zero rows behind the real ones
+    f = [torch.nn.functional.pad(t[:, -1:].float(), (0, 0, 0, pad)) for t in (q, k, v)]
+    exp = O.landmark_attention_grads(*f, torch.zeros_like(f[0]), block, sm_scale=D ** -0.5)[0][:, :, :Lq]
+    got = out[:, -1:].float().cpu()
+    # weights rounded to 16 bits in front of the product, the result behind it: the bound of the other kernel tests
+    assert (got - exp).abs().max().item() < 2e-2
+    assert ((got - exp).norm() / exp.norm()).item() < 1e-2
+    assert L.device_status() == 0
