@@ -883,9 +883,8 @@ template <bool kBf16, int kD, bool kWhole, bool kIrr>      // kWhole: whole tile
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                     const float* __restrict__ L_ptr, const float* __restrict__ M_ptr,
-                     const float* __restrict__ delta_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                     int H, int BH, int Lq, int Lk, int D_any, float scale, float scale_log2, int max_tiles,
+                     const float* L_ptr, const float* M_ptr, const float* delta_ptr, void* __restrict__ dk_ptr,
+                     void* __restrict__ dv_ptr, int H, int BH, int Lq, int Lk, int D_any, float scale, float scale_log2, int max_tiles,
                      IrrArgs irr) {
   const int D = kWhole ? kD : D_any;
   constexpr int kStages = kDkvStages<kD>;
@@ -1090,8 +1089,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t my_tile = w_tile + (uint32_t)g * kTileBytes;
     int it = 0, u = 0;
-    auto stat_m = [&](int64_t i) { return kIrr && irr.R != nullptr ? irr.R[i] : M_ptr[i]; };
-    auto stat_l = [&](int64_t i) { return kIrr && irr.R != nullptr ? 1.f : L_ptr[i]; };
+    auto stat_m = [&](int64_t i) { return ld_behind_wait((kIrr && irr.R != nullptr ? irr.R : M_ptr) + i); };
+    auto stat_l = [&](int64_t i) { return kIrr && irr.R != nullptr ? 1.f : ld_behind_wait(L_ptr + i); };
     // What a unit needs from global memory, asked for while the unit before it drains: the tile table first (all entries at
     // once), then the row statistics of the first item.  Read one after the other at the start of a unit they took 1500 - 2000 clk of it.
     // (rows past the end of the sequence have zero Q and dO tiles: whatever finite weights they get contribute nothing)
@@ -1256,9 +1255,9 @@ template <bool kBf16, int kD, bool kWhole, bool kIrr>
 __global__ void __launch_bounds__(kDqThreads, 1)
 sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                    const __grid_constant__ CUtensorMap tm_o, const float* __restrict__ L_ptr,
-                    const float* __restrict__ M_ptr, float* __restrict__ delta_ptr, void* __restrict__ dq_ptr, int H,
-                    int BH, int Lq, int Lk, int D_any, float scale, float scale_log2, IrrArgs irr) {
+                    const __grid_constant__ CUtensorMap tm_o, const float* L_ptr, const float* M_ptr,
+                    float* __restrict__ delta_ptr, void* __restrict__ dq_ptr, int H, int BH, int Lq, int Lk, int D_any,
+                    float scale, float scale_log2, IrrArgs irr) {
   const int D = kWhole ? kD : D_any;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -1467,30 +1466,24 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       drain_row = -1;
     };
-    // the row statistics of the next unit are fetched while the current one runs, so their latency is never exposed
+    // The row statistics of the next unit are fetched while the current one runs, so their latency is never exposed.  The forward
+    // kernel in front writes them and may be running when this kernel starts.
     float nM = 0.f, nL = 1.f;
-    {
-      const int w0 = unit_of(0);
-      if (w0 < n_units) {
-        const int64_t g0 = (int64_t)(w0 % BH) * Lq + (kWhole ? unit_tile(w0) * kQTile + row : min(unit_tile(w0) * kQTile + row, Lq - 1));
-        nM = kIrr && irr.R != nullptr ? irr.R[g0] : M_ptr[g0];
-        nL = kIrr && irr.R != nullptr ? 1.f : L_ptr[g0];
-      }
-    }
+    auto fetch_rows = [&](int w) {
+      if (w >= n_units) return;
+      const int r = unit_tile(w) * kQTile + row;
+      const int64_t at = (int64_t)(w % BH) * Lq + (kWhole ? r : min(r, Lq - 1));
+      nM = ld_behind_wait((kIrr && irr.R != nullptr ? irr.R : M_ptr) + at);
+      nL = kIrr && irr.R != nullptr ? 1.f : ld_behind_wait(L_ptr + at);
+    };
+    fetch_rows(unit_of(0));
     for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
       const int t = unit_tile(w), bh = w % BH, b = bh / H;
       int total = kIrr ? 0 : unit_items(w);
       const int64_t grow = (int64_t)bh * Lq + t * kQTile + row;
       const bool row_valid = kWhole || t * kQTile + row < Lq;
       const float M2L = kIrr && irr.R != nullptr ? nM : fmaf(nM, kLog2e, __log2f(nL));
-      {
-        const int wn = unit_of(r + 1);
-        if (wn < n_units) {
-          const int64_t gn = (int64_t)(wn % BH) * Lq + (kWhole ? unit_tile(wn) * kQTile + row : min(unit_tile(wn) * kQTile + row, Lq - 1));
-          nM = kIrr && irr.R != nullptr ? irr.R[gn] : M_ptr[gn];
-          nL = kIrr && irr.R != nullptr ? 1.f : L_ptr[gn];
-        }
-      }
+      fetch_rows(unit_of(r + 1));
       // tile table: everything that depends on the unit alone first, then what hangs on it (kIrr: loads from global memory)
       const int pos = min(Lk - Lq + t * kQTile + row, Lk - 1);
       const bool skip = skipped(w);
