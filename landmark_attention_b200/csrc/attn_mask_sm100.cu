@@ -84,8 +84,7 @@ __device__ __forceinline__ void store_row16_sw128(uint32_t tile_base, int row, i
 // ---------------------------------------------------------------------------------------------- landmark bookkeeping
 // kmask[t] bit j = key 64 t + j of batch row b is a landmark; gbase[t] = landmarks before tile t.  Built by the
 // four softmax warps from the byte flags; n_kt tiles (the ones at or below the CTA's diagonal).
-__device__ __forceinline__ void build_masks(const uint8_t* __restrict__ is_mem_row, int n_kt, uint64_t* kmask,
-                                            int* gbase, int tid) {
+__device__ __forceinline__ void build_masks(const uint8_t* is_mem_row, int n_kt, uint64_t* kmask, int* gbase, int tid) {
   const int warp = tid >> 5, lane = tid & 31;
   for (int t = warp; t < n_kt; t += 4) {
     const unsigned lo = __ballot_sync(0xffffffffu, is_mem_row[t * kKT + lane] != 0);
@@ -159,9 +158,9 @@ __host__ __device__ constexpr size_t mf_smem_bytes(int G, int n_kt) {
 
 template <bool kBf16>
 __device__ __forceinline__ void mask_fwd_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
-                                              const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, void* __restrict__ o_ptr,
-                                              float* __restrict__ R_ptr, float* __restrict__ A_ptr, int H, int Lq, int Lk, int G,
-                                              float scale_log2, int* status, int t, int bh, uint32_t tmem) {
+                                              const uint8_t* is_mem, int64_t is_mem_stride, void* o_ptr, float* R_ptr, float* A_ptr,
+                                              int H, int Lq, int Lk, int G, float scale_log2, int* status, int t, int bh,
+                                              uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -411,9 +410,9 @@ __device__ __forceinline__ void mask_fwd_tile(const CUtensorMap& tm_q, const CUt
 template <bool kBf16>
 __global__ void __launch_bounds__(kMfThreads, 2)
 sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                      const __grid_constant__ CUtensorMap tm_v, const uint8_t* __restrict__ is_mem, int64_t is_mem_stride,
-                      void* __restrict__ o_ptr, float* __restrict__ R_ptr, float* __restrict__ A_ptr, int H, int BH, int Lq,
-                      int Lk, int G, float scale_log2, int only_marked, int* status) {
+                      const __grid_constant__ CUtensorMap tm_v, const uint8_t* is_mem, int64_t is_mem_stride, void* o_ptr,
+                      float* R_ptr, float* A_ptr, int H, int BH, int Lq, int Lk, int G, float scale_log2, int only_marked,
+                      int* status) {
   __shared__ uint32_t tmem_slot;
   const int n_tiles = Lq / kQT;
   const uint32_t warp = threadIdx.x >> 5;
@@ -491,14 +490,11 @@ __device__ __forceinline__ float dot8(const uint4& a, const uint4& b, float acc)
 
 template <bool kBf16>
 __device__ __forceinline__ void mask_bwd_dq_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
-                                                 const CUtensorMap& tm_do, const uint8_t* __restrict__ is_mem,
-                                                 int64_t is_mem_stride, const void* __restrict__ o_ptr,
-                                                 const void* __restrict__ do_ptr, int64_t do_b, int64_t do_h, int64_t do_row,
-                                                 const float* __restrict__ R_ptr, const float* __restrict__ A_ptr,
-                                                 float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
-                                                 void* __restrict__ dq_ptr, int H, int Lq, int Lk, int G, float scale,
-                                                 float scale_log2, const int* __restrict__ plan, int plan_stride, int* status,
-                                                 int t, int bh, uint32_t tmem) {
+                                                 const CUtensorMap& tm_do, const uint8_t* is_mem, int64_t is_mem_stride,
+                                                 const void* o_ptr, const void* do_ptr, int64_t do_b, int64_t do_h, int64_t do_row,
+                                                 const float* R_ptr, const float* A_ptr, float* delta_ptr, float* nD_ptr,
+                                                 void* dq_ptr, int H, int Lq, int Lk, int G, float scale, float scale_log2,
+                                                 const int* plan, int plan_stride, int* status, int t, int bh, uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -760,11 +756,10 @@ template <bool kBf16>
 __global__ void __launch_bounds__(kMqThreads, 1)
 sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                         const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const void* __restrict__ o_ptr,
-                         const void* __restrict__ do_ptr, int64_t do_b, int64_t do_h, int64_t do_row, const float* __restrict__ R_ptr,
-                         const float* __restrict__ A_ptr, float* __restrict__ delta_ptr, float* __restrict__ nD_ptr,
-                         void* __restrict__ dq_ptr, int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2,
-                         const int* __restrict__ plan, int plan_stride, int* status) {
+                         const uint8_t* is_mem, int64_t is_mem_stride, const void* o_ptr, const void* do_ptr, int64_t do_b,
+                         int64_t do_h, int64_t do_row, const float* R_ptr, const float* A_ptr, float* delta_ptr, float* nD_ptr,
+                         void* dq_ptr, int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2, const int* plan,
+                         int plan_stride, int* status) {
   __shared__ uint32_t tmem_slot;
   const int n_tiles = Lq / kQT;
   const uint32_t warp = threadIdx.x >> 5;
@@ -823,12 +818,10 @@ constexpr size_t kMkSmemBytes = 1024 + 32768 + kMkStages * 65536 + 32768 + sizeo
 
 template <bool kBf16>
 __device__ __forceinline__ void mask_bwd_dkv_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
-                                                  const CUtensorMap& tm_do, const uint8_t* __restrict__ is_mem,
-                                                  int64_t is_mem_stride, const float* __restrict__ R_ptr,
-                                                  const float* __restrict__ A_ptr, const float* __restrict__ delta_ptr,
-                                                  const float* __restrict__ nD_ptr, void* __restrict__ dk_ptr,
-                                                  void* __restrict__ dv_ptr, int H, int Lq, int Lk, int G, float scale,
-                                                  float scale_log2, int* status, int kt, int bh, uint32_t tmem) {
+                                                  const CUtensorMap& tm_do, const uint8_t* is_mem, int64_t is_mem_stride,
+                                                  const float* R_ptr, const float* A_ptr, const float* delta_ptr,
+                                                  const float* nD_ptr, void* dk_ptr, void* dv_ptr, int H, int Lq, int Lk, int G,
+                                                  float scale, float scale_log2, int* status, int kt, int bh, uint32_t tmem) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -1125,11 +1118,9 @@ template <bool kBf16>
 __global__ void __launch_bounds__(kMkThreads, 1)
 sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                          const uint8_t* __restrict__ is_mem, int64_t is_mem_stride, const float* __restrict__ R_ptr,
-                          const float* __restrict__ A_ptr, const float* __restrict__ delta_ptr,
-                          const float* __restrict__ nD_ptr, void* __restrict__ dk_ptr, void* __restrict__ dv_ptr,
-                          int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2,
-                          const int* __restrict__ plan, int plan_stride, int* status) {
+                          const uint8_t* is_mem, int64_t is_mem_stride, const float* R_ptr, const float* A_ptr,
+                          const float* delta_ptr, const float* nD_ptr, void* dk_ptr, void* dv_ptr, int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2,
+                          const int* plan, int plan_stride, int* status) {
   __shared__ uint32_t tmem_slot;
   const int n_tiles = Lk / kKT;
   const uint32_t warp = threadIdx.x >> 5;

@@ -154,7 +154,7 @@ __device__ __forceinline__ int irr_group(const IrrSmem& t, int pos) {          /
   return t.gbase[pos >> 6] + __popcll(t.kmask[pos >> 6] & ((1ull << (pos & 63)) - 1ull));
 }
 // All threads of the CTA; contains __syncthreads().
-__device__ __forceinline__ void irr_build(IrrSmem& t, const uint8_t* __restrict__ flags, int Lk, int G) {
+__device__ __forceinline__ void irr_build(IrrSmem& t, const uint8_t* flags, int Lk, int G) {
   const int words = (Lk + 63) / 64, warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int w = warp; w < words; w += warps) {
     const int k0 = w * 64 + lane;
@@ -213,12 +213,16 @@ __device__ __forceinline__ void irr_build(IrrSmem& t, const uint8_t* __restrict_
 // ends, then one byte per key with its group.
 constexpr int kIrrPlanHead = 2 + kIrrMaxTiles + 1;
 constexpr int kIrrPlanInts = kIrrPlanHead + (kIrrMaxKeys + 3) / 4;
-__device__ __forceinline__ bool irr_plan_fallback(const int* plan, int b) { return __ldg(plan + (int64_t)b * kIrrPlanInts + 1) != 0; }
-__device__ __forceinline__ int irr_plan_end(const int* plan, int b, int n) { return __ldg(plan + (int64_t)b * kIrrPlanInts + 2 + n); }
-__device__ __forceinline__ int irr_plan_group(const int* plan, int b, int pos) {
-  return __ldg(reinterpret_cast<const uint8_t*>(plan + (int64_t)b * kIrrPlanInts + kIrrPlanHead) + pos);
+__device__ __forceinline__ bool irr_plan_fallback(const int* plan, int b) {
+  return ld_behind_wait(plan + (int64_t)b * kIrrPlanInts + 1) != 0;
 }
-__global__ void __launch_bounds__(256) irr_plan_kernel(const uint8_t* __restrict__ flags, int64_t stride, int Lk, int G, int* plan) {
+__device__ __forceinline__ int irr_plan_end(const int* plan, int b, int n) {
+  return ld_behind_wait(plan + (int64_t)b * kIrrPlanInts + 2 + n);
+}
+__device__ __forceinline__ int irr_plan_group(const int* plan, int b, int pos) {
+  return ld_behind_wait(reinterpret_cast<const uint8_t*>(plan + (int64_t)b * kIrrPlanInts + kIrrPlanHead) + pos);
+}
+__global__ void __launch_bounds__(256) irr_plan_kernel(const uint8_t* flags, int64_t stride, int Lk, int G, int* plan) {
   grid_dep_wait();
   grid_dep_launch();
   __shared__ IrrSmem t;
@@ -279,9 +283,8 @@ template <bool kBf16, int kD, bool kIrr, int kTiles>
 __global__ void __launch_bounds__(kFwdThreads<kTiles>, 3 - kTiles)
 sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_klm,
-                  void* __restrict__ o_ptr, float* __restrict__ L_ptr, float* __restrict__ M_ptr, int H, int Lq, int Lk,
-                  int D, int lm_box, float scale_log2, const void* __restrict__ k_ptr, int64_t ks_b, int64_t ks_h,
-                  int64_t ks_row, IrrArgs irr) {
+                  void* o_ptr, float* L_ptr, float* M_ptr, int H, int Lq, int Lk, int D, int lm_box, float scale_log2,
+                  const void* k_ptr, int64_t ks_b, int64_t ks_h, int64_t ks_row, IrrArgs irr) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -883,9 +886,8 @@ template <bool kBf16, int kD, bool kWhole, bool kIrr>      // kWhole: whole tile
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                     const float* L_ptr, const float* M_ptr, const float* delta_ptr, void* __restrict__ dk_ptr,
-                     void* __restrict__ dv_ptr, int H, int BH, int Lq, int Lk, int D_any, float scale, float scale_log2, int max_tiles,
-                     IrrArgs irr) {
+                     const float* L_ptr, const float* M_ptr, const float* delta_ptr, void* dk_ptr, void* dv_ptr, int H, int BH,
+                     int Lq, int Lk, int D_any, float scale, float scale_log2, int max_tiles, IrrArgs irr) {
   const int D = kWhole ? kD : D_any;
   constexpr int kStages = kDkvStages<kD>;
   constexpr uint32_t kOperand = (kD / 64) * kTileBytes;     // [128 rows x kD] as 64-feature sub-tiles of 16 KB
@@ -1255,9 +1257,8 @@ template <bool kBf16, int kD, bool kWhole, bool kIrr>
 __global__ void __launch_bounds__(kDqThreads, 1)
 sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                    const __grid_constant__ CUtensorMap tm_o, const float* L_ptr, const float* M_ptr,
-                    float* __restrict__ delta_ptr, void* __restrict__ dq_ptr, int H, int BH, int Lq, int Lk, int D_any,
-                    float scale, float scale_log2, IrrArgs irr) {
+                    const __grid_constant__ CUtensorMap tm_o, const float* L_ptr, const float* M_ptr, float* delta_ptr,
+                    void* dq_ptr, int H, int BH, int Lq, int Lk, int D_any, float scale, float scale_log2, IrrArgs irr) {
   const int D = kWhole ? kD : D_any;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -1915,9 +1916,10 @@ static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   const int dq_units = ((p.Lq + kQTile - 1) / kQTile) * p.B * p.H;
   dim3 grid_dkv(dkv_units < n_sm ? dkv_units : n_sm), grid_dq(dq_units < n_sm ? dq_units : n_sm);
   // Both launches can carry the programmatic-stream-serialization attribute.  The dQ kernel waits for the kernel before it
-  // right after its set-up (only the set-up overlaps).  The dK/dV kernel reads q, k, v, dO, L, M, which were complete
-  // before the dQ kernel started, and `delta`, which the dQ kernel writes: its loads and S / dP products start on
-  // every SM the dQ kernel has left, and only its softmax threads wait (griddepcontrol.wait) before they read delta.
+  // right after its set-up (only the set-up overlaps).  The dK/dV kernel reads q, k, v, dO, L, M and the tile table, which
+  // were complete before any CTA of the dQ kernel was behind its wait and could let this one start, and `delta`, which the
+  // dQ kernel writes: its loads and S / dP products start on every SM the dQ kernel has left, and only its softmax threads
+  // wait (griddepcontrol.wait) before they read delta.
   // (Blocks of 64 at B1 H32 L2048 206 -> 203 us, B4 H16 L1024 D64 120 -> 118.5; the layer with groups of 51 at B16 H8 T512
   // 166.7 -> 161.2.)
   cudaLaunchAttribute pdl[1];

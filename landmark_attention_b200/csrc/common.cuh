@@ -55,8 +55,8 @@ static inline int dtype_size(int dtype) { return dtype == LMK_F32 ? 4 : 2; }
 
 // Launch with the programmatic-stream-serialization attribute: the kernel's CTAs may start, and its launch be processed, while the
 // kernel in front of it in the stream drains.  Such a kernel executes griddepcontrol.wait (ptx::grid_dep_wait) before it
-// touches global memory, and takes what it reads through plain pointers: const __restrict__ and __ldg promise memory that nothing
-// writes while the kernel runs, and allow the compiler to read it in front of the wait.
+// touches global memory, has no __restrict__ pointer among its parameters and uses no __ldg: both promise memory that no other
+// kernel writes meanwhile, and allow the compiler to read it in front of the wait.
 template <typename... P, typename... A>
 cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute attr[1];

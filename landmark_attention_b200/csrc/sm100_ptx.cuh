@@ -68,12 +68,22 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // stream is still running; grid_dep_wait() blocks until that kernel has completed and its writes are visible (a no-op
 // without the attribute).  grid_dep_launch() lets the NEXT kernel of the stream start its CTAs as soon as SMs free up.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// A load that stays behind grid_dep_wait(), for memory that the kernel in front writes.  One through a const __restrict__ pointer, or
-// __ldg, counts as a load of memory that nothing writes while the kernel runs, which the compiler may move in front of the wait;
-// the waiting kernels therefore take their inputs through plain pointers (see launch_overlapped).
+// A load that stays behind grid_dep_wait(), for memory that the kernel in front writes.  Loads through __restrict__ pointers and __ldg
+// may be moved in front of the wait by the compiler: the first promise memory that nothing but the pointer's own stores
+// touches while the kernel runs, the second memory that nothing writes.
 __device__ __forceinline__ float ld_behind_wait(const float* p) {
   float v;
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_behind_wait(const int* p) {
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_behind_wait(const uint8_t* p) {
+  int v;
+  asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -1,13 +1,13 @@
 """Kernels that may start while the kernel in front of them is running (they execute griddepcontrol.wait) read what it writes.  A
-const __restrict__ parameter promises memory that nothing writes meanwhile, and allows the compiler to load from it before the wait:
-none of these kernels takes an input that way.  Read off the sources, since a stale read shows itself only now and then."""
+__restrict__ parameter promises memory that nobody else touches meanwhile, and allows the compiler to load from it before the wait, and
+so does __ldg: none of these kernels uses them.  Read off the sources, since a stale read shows itself only now and then."""
 import os
 import re
 
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "landmark_attention_b200", "csrc")
-PROMISE = re.compile(r"const\s+[\w:<>\s]*\*\s*(?:const\s+)?__restrict__")
+PROMISE = re.compile(r"__restrict__|__ldg|ld\.global\.nc")
 
 
 def closing(text, at, pair):
@@ -21,28 +21,44 @@ def closing(text, at, pair):
 
 
 def functions(text):
-    """name -> (parameters, body) of the kernels of a source."""
+    """(kernels, device functions) of a source: name -> (parameters, body)."""
     text = re.sub(r"//[^\n]*", "", text)
-    found = {}
-    for m in re.finditer(r"__global__", text):
+    kernels, device = {}, {}
+    for m in re.finditer(r"__global__|__device__", text):
         at, params, name = m.end(), None, None
-        while text[at] not in "{;":
+        while text[at] not in "{;=":
             if text[at] == "(":
                 name = re.search(r"(\w+)\s*$", text[m.end():at]).group(1)
                 end = closing(text, at, "()")
                 params, at = text[at:end], end
             else:
                 at += 1
-        if text[at] == "{":
-            found[name] = (params, text[at:closing(text, at, "{}")])
-    return found
+        if text[at] == "{" and name:
+            kept = kernels if m.group() == "__global__" else device
+            kept.setdefault(name, []).append((params, text[at:closing(text, at, "{}")]))
+    return kernels, device
 
 
-@pytest.mark.parametrize("source,kernels", [("attn_sm100.cu", ("sm100_bwd_dq_kernel", "sm100_bwd_dkv_kernel"))])
-def test_waiting_kernels_promise_nothing_about_their_inputs(source, kernels):
+def reached(body, device):
+    """The device functions of the same source that a body calls, directly or not."""
+    names, queue = set(), [body]
+    while queue:
+        for name in set(re.findall(r"\w+", queue.pop())) & device.keys() - names:
+            names.add(name)
+            queue += [b for _, b in device[name]]
+    return names
+
+
+@pytest.mark.parametrize("source", ["attn_sm100.cu", "attn_mask_sm100.cu"])
+def test_waiting_kernels_promise_nothing_about_their_inputs(source):
     with open(os.path.join(CSRC, source)) as f:
-        found = functions(f.read())
-    for name in kernels:
-        params, body = found[name]
-        assert "grid_dep_wait()" in body, name
-        assert not PROMISE.search(params), name
+        kernels, device = functions(f.read())
+    waiting = 0
+    for kernel, forms in kernels.items():
+        for params, body in forms:
+            if "grid_dep_wait()" not in body:
+                continue
+            waiting += 1
+            for name, (p, b) in [(kernel, (params, body)), *[(n, f) for n in reached(body, device) for f in device[n]]]:
+                assert not PROMISE.search(p + b), f"{kernel}: {name}"
+    assert waiting

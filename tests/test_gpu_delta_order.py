@@ -1,5 +1,6 @@
 """A backward kernel may start while the kernel in front of it is still running: dQ reads the row statistics and the output that the
-forward writes, dK/dV reads delta = rowsum(O * dO) that dQ writes.  All of that is scratch memory or fresh memory of the allocator,
+forward writes, or the table of landmark groups that a kernel of its own works out, dK/dV reads delta = rowsum(O * dO) that dQ
+writes.  All of that is scratch memory or fresh memory of the allocator,
 which may hold anything, or the right values of a call before.  So: calls whose memory holds NaNs, many times, against the oracle and
 bit by bit against one another."""
 import pytest
@@ -64,4 +65,29 @@ def test_first_backward_into_poisoned_scratch(B, H, L, D):
     for b, h in ((0, 0), (B - 1, H - 1)):
         one = [t[b:b + 1, h:h + 1].detach().float().cpu() for t in (q, k, v, do)]
         for (name, t), e in zip(got.items(), O.landmark_attention_grads(*one, 64, sm_scale=D ** -0.5)):
+            close(t[b:b + 1, h:h + 1], e, f"{name}, batch {b}, head {h}")
+
+
+def test_groups_into_poisoned_scratch():
+    B, H, T, D, G = 16, 8, 512, 128, 16
+    g = torch.Generator().manual_seed(5)
+    q, k, v = [(torch.randn(B, H, T, D, generator=g) * 0.5).bfloat16() for _ in range(3)]
+    do = torch.randn(B, H, T, D, generator=g).bfloat16()
+    im = (torch.arange(T).view(1, T) + torch.randint(0, 51, (B, 1), generator=g)) % 51 == 50
+    im[5] = False                                          # no landmark: a row for the two-pass kernels
+    qc, kc, vc = [t.cuda().requires_grad_(True) for t in (q, k, v)]
+    doc, imc = do.cuda(), im.cuda()
+
+    def call():
+        out = P.landmark_attention_masked(qc, kc, vc, imc, max_groups=G)
+        return (out, *torch.autograd.grad(out, [qc, kc, vc], doc))
+
+    rows, data = 4 * B * H * T, 2 * B * H * T * D
+    ws = int(L.lib().lmk_attn_mask_bwd_workspace(B, H, T, G))               # delta, sums of the groups, tile table
+    got = check_calls(call, [rows, G * rows, ws, data, data, data, data])    # R, A, o, dq, dk, dv
+    for b, h in ((0, 0), (5, 3), (B - 1, H - 1)):
+        f = [t[b:b + 1, h:h + 1].float().requires_grad_(True) for t in (q, k, v)]
+        out = O.lm_attention(*f, im[b:b + 1])
+        exp = (out.detach(), *torch.autograd.grad(out, f, do[b:b + 1, h:h + 1].float()))
+        for (name, t), e in zip(got.items(), exp):
             close(t[b:b + 1, h:h + 1], e, f"{name}, batch {b}, head {h}")
