@@ -1534,7 +1534,11 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             delta = fmaf(fo.y, fg.y, delta);
           }
         }
-      mbar_arrive(smem_u32(&sm->delta_read));       // the shared-memory tiles may take the next unit's rows
+      // The shared-memory tiles may take the next unit's rows.  TMA writes them through another proxy than these loads went through,
+      // and an arrival alone does not hold it back until they are done: of 15 000 calls at B4 H16 L1024 D64 twenty had rows of dQ
+      // from tiles half overwritten, always of a unit with no more items than stages, behind which the producer is already waiting.
+      fence_proxy_async_smem();
+      mbar_arrive(smem_u32(&sm->delta_read));
       // row -> TMEM lane, 32-bit word j (two features) -> column j: the layout of a K-major A operand
       mbar_wait(smem_u32(&sm->ops_free), (u & 1) ^ 1, &g_lmk_status, kErrDqSoftmax);
       tc_fence_after();

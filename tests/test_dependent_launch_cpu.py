@@ -1,6 +1,7 @@
 """Kernels that may start while the kernel in front of them is running (they execute griddepcontrol.wait) read what it writes.  A
 __restrict__ parameter promises memory that nobody else touches meanwhile, and allows the compiler to load from it before the wait, and
-so does __ldg: none of these kernels uses them.  Read off the sources, since a stale read shows itself only now and then."""
+so does __ldg: none of these kernels uses them.  And a thread that has read a tile from shared memory lets TMA overwrite it only
+behind a fence between the two proxies.  Read off the sources, since either fault shows itself only now and then."""
 import os
 import re
 
@@ -62,3 +63,11 @@ def test_waiting_kernels_promise_nothing_about_their_inputs(source):
             for name, (p, b) in [(kernel, (params, body)), *[(n, f) for n in reached(body, device) for f in device[n]]]:
                 assert not PROMISE.search(p + b), f"{kernel}: {name}"
     assert waiting
+
+
+def test_tiles_read_by_threads_are_released_behind_a_proxy_fence():
+    with open(os.path.join(CSRC, "attn_sm100.cu")) as f:
+        (_, body), = functions(f.read())[0]["sm100_bwd_dq_kernel"]
+    release = body.index("mbar_arrive(smem_u32(&sm->delta_read))")
+    assert body.rindex("fence_proxy_async_smem()", 0, release) > body.rindex("ld.shared", 0, release)
+    assert body.count("ld.shared") == body[:release].count("ld.shared")

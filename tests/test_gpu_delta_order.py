@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import landmark_attention_b200 as P
-from landmark_attention_b200 import _lib as L
+from landmark_attention_b200 import _lib as lib
 from oracle import landmark_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -39,7 +39,7 @@ def check_calls(call, sizes, names=("o", "dq", "dk", "dv")):
             first = got
         for name, a, b in zip(names, first, got):
             assert torch.equal(a, b), f"call {i}: " + first_difference(name, a, b)
-    assert L.device_status() == 0
+    assert lib.device_status() == 0
     return dict(zip(names, first))
 
 
@@ -68,6 +68,27 @@ def test_first_backward_into_poisoned_scratch(B, H, L, D):
             close(t[b:b + 1, h:h + 1], e, f"{name}, batch {b}, head {h}")
 
 
+@pytest.mark.parametrize("B,H,L,D", [(64, 16, 256, 64), (16, 32, 256, 128), (8, 64, 384, 64), (32, 16, 449, 96), (64, 32, 64, 64)])
+def test_units_with_few_key_blocks(B, H, L, D):
+    # dQ units whose key blocks all fit the stages: the next unit's tiles are loaded as soon as the rows in shared memory are read
+    g = torch.Generator(device="cuda").manual_seed(L + D)
+    q, k, v = [(torch.randn(B, H, L, D, generator=g, device="cuda") * 0.5).bfloat16().requires_grad_(True) for _ in range(3)]
+    do = torch.randn(B, H, L, D, generator=g, device="cuda").bfloat16()
+    first = None
+    for i in range(300):
+        out = P.fused_landmark_attention(q, k, v, None, block_size=64)
+        got = (out.detach(), *torch.autograd.grad(out, [q, k, v], do))
+        first = first or got
+        for name, a, b in zip(("o", "dq", "dk", "dv"), first, got):
+            assert torch.equal(a, b), f"call {i}: " + first_difference(name, a, b)
+    pad = -L % 64                                          # the oracle wants whole blocks: zero rows behind the real ones
+    for b, h in ((0, 0), (B - 1, H - 1)):
+        one = [torch.nn.functional.pad(t[b:b + 1, h:h + 1].detach().float().cpu(), (0, 0, 0, pad)) for t in (q, k, v, do)]
+        for name, t, e in zip(("o", "dq", "dk", "dv"), first, O.landmark_attention_grads(*one, 64, sm_scale=D ** -0.5)):
+            close(t[b:b + 1, h:h + 1], e[:, :, :L], f"{name}, batch {b}, head {h}")
+    assert lib.device_status() == 0
+
+
 def test_groups_into_poisoned_scratch():
     B, H, T, D, G = 16, 8, 512, 128, 16
     g = torch.Generator().manual_seed(5)
@@ -83,7 +104,7 @@ def test_groups_into_poisoned_scratch():
         return (out, *torch.autograd.grad(out, [qc, kc, vc], doc))
 
     rows, data = 4 * B * H * T, 2 * B * H * T * D
-    ws = int(L.lib().lmk_attn_mask_bwd_workspace(B, H, T, G))               # delta, sums of the groups, tile table
+    ws = int(lib.lib().lmk_attn_mask_bwd_workspace(B, H, T, G))               # delta, sums of the groups, tile table
     got = check_calls(call, [rows, G * rows, ws, data, data, data, data])    # R, A, o, dq, dk, dv
     for b, h in ((0, 0), (5, 3), (B - 1, H - 1)):
         f = [t[b:b + 1, h:h + 1].float().requires_grad_(True) for t in (q, k, v)]
