@@ -159,8 +159,7 @@ constexpr int kTopkMaxK = 32;
 
 // k rounds of warp arg-max over vals[0..n) in shared memory (ties: lower index), then the picks are written in
 // ascending order of logical age.  Called by one full warp.
-__device__ __forceinline__ void select_topk_sorted(float* vals, int n, int k, int ring_start, bool vec4,
-                                                   int32_t* __restrict__ out_row) {
+__device__ __forceinline__ void select_topk_sorted(float* vals, int n, int k, int ring_start, bool vec4, int32_t* out_row) {
   const int lane = threadIdx.x & 31;
   int mine = -1;   // lane i keeps the i-th pick
   for (int it = 0; it < k; ++it) {
@@ -251,10 +250,9 @@ __global__ void __launch_bounds__(128) topk_sorted_kernel(const float* __restric
 // run over the candidates only.  Rows with too many candidates (long runs of equal scores) take the general selection.
 constexpr int kTopkRegCand = 64;
 
-__global__ void __launch_bounds__(128, 8) topk_sorted_rows_kernel(const float* __restrict__ scores,
-                                                               int32_t* __restrict__ idx, int64_t rows,
-                                                               int64_t inner_count, int64_t outer_stride,
-                                                               int64_t inner_stride, int n, int k, int ring_start) {
+__global__ void __launch_bounds__(128, 8) topk_sorted_rows_kernel(const float* scores, int32_t* idx, int64_t rows,
+                                                                  int64_t inner_count, int64_t outer_stride,
+                                                                  int64_t inner_stride, int n, int k, int ring_start) {
   extern __shared__ __align__(16) float tk_smem[];          // per warp: n floats (general selection) + candidates
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t row = (int64_t)blockIdx.x * 4 + warp;
@@ -705,13 +703,11 @@ __device__ __forceinline__ uint64_t pair_f32(uint32_t w) {
 // This is the grouped softmax of llama/llama_mem.py:222-243 over [selected blocks | local keys] written out for the
 // prefix pattern of :415 (every selected block is a closed group whose last row is its landmark).
 template <typename T, int LPR>
-__global__ void __launch_bounds__(128, 8) selected_attend_kernel(const T* __restrict__ q, const T* __restrict__ kc,
-                                                              lmk_cache_desc kd, const T* __restrict__ vc,
-                                                              lmk_cache_desc vd, const int32_t* __restrict__ idx,
-                                                              const T* __restrict__ cos_t, const T* __restrict__ sin_t,
-                                                              int n_pos, int rotary, const T* __restrict__ o_local,
-                                                              const float* __restrict__ R_local, int64_t local_rows,
-                                                              T* __restrict__ out, int H, int Tq, float scale) {
+__global__ void __launch_bounds__(128, 8) selected_attend_kernel(const T* q, const T* kc, lmk_cache_desc kd, const T* vc,
+                                                                 lmk_cache_desc vd, const int32_t* idx, const T* cos_t,
+                                                                 const T* sin_t, int n_pos, int rotary, const T* o_local,
+                                                                 const float* R_local, int64_t local_rows, T* out, int H,
+                                                                 int Tq, float scale) {
   constexpr int VEC = 16 / sizeof(T);
   constexpr int D = LPR * VEC, HALF = D / 2, LP = LPR / 2, RPS = 32 / LP;
   constexpr int VGROUPS = 32 / LPR > 0 ? 32 / LPR : 1;      // value rows a warp reads per step

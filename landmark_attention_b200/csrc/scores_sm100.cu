@@ -28,9 +28,8 @@ constexpr int kRotPerCta = 16;
 // Sixteen landmark rows per CTA, eight threads per row: each thread takes one 16-byte vector of the low half of the
 // row and its partner of the high half, so every load of the CTA is in flight at once.
 template <typename T>
-__global__ void __launch_bounds__(128) rotate_landmarks_kernel(const T* __restrict__ kc, lmk_cache_desc desc,
-                                                               const T* __restrict__ cos_t, const T* __restrict__ sin_t,
-                                                               int n_pos, int rotary, T* __restrict__ out, int H) {
+__global__ void __launch_bounds__(128) rotate_landmarks_kernel(const T* kc, lmk_cache_desc desc, const T* cos_t, const T* sin_t,
+                                                               int n_pos, int rotary, T* out, int H) {
   constexpr int D = 128, HALF = 64;
   const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
   const int N = desc.n_blocks, blk = desc.block;
@@ -84,9 +83,8 @@ struct ScoreSmem {
 
 template <typename T>
 __global__ void __launch_bounds__(128) scores_gemm_kernel(const __grid_constant__ CUtensorMap tm_q,
-                                                          const __grid_constant__ CUtensorMap tm_k,
-                                                          float* __restrict__ scores, int Tq, int N, float scale,
-                                                          int* __restrict__ status) {
+                                                          const __grid_constant__ CUtensorMap tm_k, float* scores, int Tq,
+                                                          int N, float scale, int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;

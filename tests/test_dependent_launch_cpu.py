@@ -22,14 +22,14 @@ def closing(text, at, pair):
 
 
 def functions(text):
-    """(kernels, device functions) of a source: name -> (parameters, body)."""
+    """(kernels, device functions) of a source: name -> [(parameters, body)]."""
     text = re.sub(r"//[^\n]*", "", text)
     kernels, device = {}, {}
     for m in re.finditer(r"__global__|__device__", text):
         at, params, name = m.end(), None, None
         while text[at] not in "{;=":
             if text[at] == "(":
-                name = re.search(r"(\w+)\s*$", text[m.end():at]).group(1)
+                name = re.search(r"(\w*)\s*$", text[m.end():at]).group(1)       # "": an operator
                 end = closing(text, at, "()")
                 params, at = text[at:end], end
             else:
@@ -50,10 +50,18 @@ def reached(body, device):
     return names
 
 
-@pytest.mark.parametrize("source", ["attn_sm100.cu", "attn_mask_sm100.cu"])
-def test_waiting_kernels_promise_nothing_about_their_inputs(source):
+def read(source):
     with open(os.path.join(CSRC, source)) as f:
-        kernels, device = functions(f.read())
+        return f.read()
+
+
+SHARED = "".join(read(f) for f in sorted(os.listdir(CSRC)) if f.endswith((".cuh", ".h")))
+WAITING = [f for f in sorted(os.listdir(CSRC)) if f.endswith(".cu") and "grid_dep_wait()" in read(f)]
+
+
+@pytest.mark.parametrize("source", WAITING)
+def test_waiting_kernels_promise_nothing_about_their_inputs(source):
+    kernels, device = functions(SHARED + read(source))
     waiting = 0
     for kernel, forms in kernels.items():
         for params, body in forms:
@@ -65,9 +73,13 @@ def test_waiting_kernels_promise_nothing_about_their_inputs(source):
     assert waiting
 
 
+def test_every_source_that_launches_before_the_end_is_looked_at():
+    launching = [f for f in os.listdir(CSRC) if f.endswith(".cu") and re.search(r"launch_overlapped|ProgrammaticStream", read(f))]
+    assert set(launching) <= set(WAITING)
+
+
 def test_tiles_read_by_threads_are_released_behind_a_proxy_fence():
-    with open(os.path.join(CSRC, "attn_sm100.cu")) as f:
-        (_, body), = functions(f.read())[0]["sm100_bwd_dq_kernel"]
+    (_, body), = functions(read("attn_sm100.cu"))[0]["sm100_bwd_dq_kernel"]
     release = body.index("mbar_arrive(smem_u32(&sm->delta_read))")
     assert body.rindex("fence_proxy_async_smem()", 0, release) > body.rindex("ld.shared", 0, release)
     assert body.count("ld.shared") == body[:release].count("ld.shared")
