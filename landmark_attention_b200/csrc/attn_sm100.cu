@@ -76,19 +76,20 @@ __device__ __forceinline__ void store_row_sw128(uint32_t tile_base, int row, con
 
 // Row reductions with four independent chains: one softmax thread has little other work in flight, so a single
 // 63-deep dependent chain of max / add would expose the ALU latency on every step.
+// row_max: NaN where a value is NaN.
 template <int N>
 __device__ __forceinline__ float row_max(const float (&v)[64]) {
-  float a = -INFINITY, b = -INFINITY, c = -INFINITY, d = -INFINITY;
+  float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-  for (int j = 0; j + 3 < N; j += 4) {
-    a = fmaxf(a, v[j]);
-    b = fmaxf(b, v[j + 1]);
-    c = fmaxf(c, v[j + 2]);
-    d = fmaxf(d, v[j + 3]);
-  }
-#pragma unroll
-  for (int j = N & ~3; j < N; ++j) a = fmaxf(a, v[j]);
-  return fmaxf(fmaxf(a, b), fmaxf(c, d));
+  for (int j = 0; j + 1 < N; j += 2) m[j / 2 % 4] = max3_nan(m[j / 2 % 4], v[j], v[j + 1]);
+  return max3_nan(max3_nan(m[0], m[1], N % 2 ? v[N - 1] : -INFINITY), m[2], m[3]);
+}
+// Shift of the exponentials of an earlier block, -(row maximum) * c.  Some of them are polynomials, which make finite numbers of
+// NaN and infinities (ex2_poly2): where the maximum is one of these the shift is NaN, and with it the exponentials between
+// the polynomials, their sum, and everything that is divided by it.
+__device__ __forceinline__ float block_shift(const float (&v)[64], float c) {
+  const float mx = row_max<63>(v);
+  return fmaf(mx, 0.f, -mx * c);
 }
 __device__ __forceinline__ float row_max_upto(const float (&v)[64], int last) {
   float a = -INFINITY, b = -INFINITY, c = -INFINITY, d = -INFINITY;
@@ -552,7 +553,7 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
           for (int j = 0; j < 32; ++j) wgt[j] = pack2<kBf16>(sv[2 * j], sv[2 * j + 1]);
         } else {
-          const float nmx = -row_max<63>(sv) * scale_log2;
+          const float nmx = block_shift(sv, scale_log2);
           const float el = ex2(fmaf(sv[63], scale_log2, -m2));
           const uint64_t c2 = pk2(scale_log2, scale_log2), n2 = pk2(nmx, nmx);
           uint64_t sp[32];
@@ -682,7 +683,7 @@ __device__ __forceinline__ RowFactors bwd_weights(uint64_t (&sp)[32], int c0, ui
         sv[j] = __uint_as_float(ra[j]);
         sv[32 + j] = __uint_as_float(rb[j]);
       }
-      nmx = -row_max<63>(sv) * c;
+      nmx = block_shift(sv, c);
       lm2 = sv[63] * c;
       if (kIrr && c0 == 63) nmx = 0.f;      // no key but the landmark
     }

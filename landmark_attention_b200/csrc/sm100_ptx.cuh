@@ -265,6 +265,13 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   return d;
 }
 
+// the largest of three, NaN where one is NaN
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -274,8 +281,9 @@ __device__ __forceinline__ float ex2(float x) {
 // exp2 of two values on the FMA and integer pipes instead of the special-function unit: round to the nearest integer
 // n with the 1.5 * 2^23 trick, evaluate a minimax polynomial (smallest relative error, exchange algorithm) for 2^(x - n) on
 // [-0.5, 0.5] and add n to the exponent field.  Relative error 2.7e-6 for degree 4 and 7.5e-5 for a cubic, both below half a bf16 / fp16
-// rounding step of the weights they feed.  The softmax threads take a share of
-// their exponentials this way (kFwdPolyEvery, kBwdPolyEvery).  Inputs are clamped to >= -126 (results below 2^-126 are not needed).
+// rounding step of the weights they feed.  The softmax threads take a share of their exponentials this way (kFwdPolyEvery,
+// kBwdPolyEvery).  Inputs are clamped to >= -126 (results below 2^-126 are not needed).  NaN and infinities come out as finite
+// numbers: the exponentials beside these have to carry them (block_shift).
 template <int kDegree>
 __device__ __forceinline__ uint64_t ex2_poly2(uint64_t x) {
   float a, b;
