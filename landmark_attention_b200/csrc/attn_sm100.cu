@@ -836,7 +836,8 @@ template <int kStages> struct DkvSmem {
 
 // Stores 32 accumulator columns of one TMEM lane per thread as 16-bit values.  Four neighbouring lanes exchange 16-byte
 // chunks first, so that a warp's store covers 64 contiguous bytes of eight rows and not 16 bytes of thirty-two.
-// row_off[j]: element offset of row j of the lane's four rows, or -1 for a row that is not stored.
+// row_off[j]: element offset of row j of the lane's four rows, or -1 for a row that is not stored.  An output of the C interface
+// may start at any word: one off a 16-byte boundary is stored word by word.
 template <bool kBf16>
 __device__ __forceinline__ void store_acc_cols(void* out, const int64_t (&row_off)[4], const uint32_t (&r)[32], int col0, int D,
                                                int lane) {
@@ -864,10 +865,20 @@ __device__ __forceinline__ void store_acc_cols(void* out, const int64_t (&row_of
   swap(v[0], v[2], 2);
   swap(v[1], v[3], 2);
   const int col = col0 + 8 * (lane & 3);
-  if (col < D) {
+  if (col >= D) return;
+  const bool wide = ((uintptr_t)out & 15) == 0;       // rows and columns are multiples of 16 bytes
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (row_off[j] >= 0) *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(out) + row_off[j] + col) = v[j];
+  for (int j = 0; j < 4; ++j) {
+    if (row_off[j] < 0) continue;
+    uint32_t* to = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(out) + row_off[j] + col);
+    if (wide) {
+      *reinterpret_cast<uint4*>(to) = v[j];
+    } else {
+      to[0] = v[j].x;
+      to[1] = v[j].y;
+      to[2] = v[j].z;
+      to[3] = v[j].w;
+    }
   }
 }
 

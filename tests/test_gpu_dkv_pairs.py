@@ -42,3 +42,32 @@ def test_units_of_key_block_pairs(B, H, Lq, hist, D, dtype):
         assert (got - e).abs().max().item() < 2e-2 * max(1.0, e.abs().max().item()), name
         assert ((got - e).norm() / e.norm()).item() < 1e-2, name
     assert L.device_status() == 0
+
+
+@pytest.mark.parametrize("L_,D", [(320, 64), (449, 96), (256, 128)])
+def test_outputs_off_a_16_byte_boundary(L_, D):
+    # the C interface takes dK and dV at any word (2, 4 and 6 elements behind a boundary), and writes nothing beside them
+    g = torch.Generator().manual_seed(D)
+    B, H, dtype, lib = 2, 3, torch.bfloat16, L.lib()
+    q, k, v, do = [(torch.randn(B, H, L_, D, generator=g) * 0.5).to(dtype).to(DEV) for _ in range(4)]
+    n, code, scale, s3, st = q.numel(), L.dtype_code(q), D ** -0.5, L.strides3(q), L.stream_ptr(q.device)
+    o, dq = torch.empty_like(q), torch.empty_like(q)
+    l, m = [torch.empty(B * H, L_, device=DEV) for _ in range(2)]
+    ws = torch.empty(int(lib.lmk_attn_bwd_workspace(B, H, L_, L_, D, 64, code, P.PATH_AUTO)), dtype=torch.uint8, device=DEV)
+    L.check(lib.lmk_attn_fwd(L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(o), L.ptr(l), L.ptr(m), B, H, L_, L_, D, s3, s3, s3, 64, scale,
+                             code, P.PATH_AUTO, st), "lmk_attn_fwd")
+
+    def backward(off):
+        bufs = [torch.full((n + 16,), 7.0, dtype=dtype, device=DEV) for _ in range(2)]
+        dk, dv = [b[off:off + n] for b in bufs]
+        L.check(lib.lmk_attn_bwd(L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(o), L.ptr(do), L.ptr(l), L.ptr(m), L.ptr(dq), L.ptr(dk),
+                                 L.ptr(dv), L.ptr(ws), ws.numel(), B, H, L_, L_, D, s3, s3, s3, 64, scale, code, P.PATH_AUTO, st),
+                "lmk_attn_bwd")
+        for b in bufs:
+            assert (b[:off] == 7).all() and (b[off + n:] == 7).all()
+        return dk, dv
+
+    ref = backward(0)
+    for off in (2, 4, 6):
+        assert all(torch.equal(a, b) for a, b in zip(backward(off), ref)), off
+    assert L.device_status() == 0
