@@ -71,3 +71,34 @@ def test_outputs_off_a_16_byte_boundary(L_, D):
     for off in (2, 4, 6):
         assert all(torch.equal(a, b) for a, b in zip(backward(off), ref)), off
     assert L.device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,T,block,D", [(2, 3, 512, 51, 128), (1, 2, 256, 26, 128), (2, 2, 449, 32, 64), (1, 3, 320, 16, 96)])
+def test_units_of_groups(B, H, T, block, D):
+    # groups as key tiles: landmarks at each row's own positions (handed over as flags), or a regular pattern of smaller blocks
+    g = torch.Generator().manual_seed(T + block)
+    q, k, v, do = [(torch.randn(B, H, T, D, generator=g) * 0.5).to(torch.bfloat16) for _ in range(4)]
+    flags = T % 128 == 0
+    first = torch.randint(0, block, (B, 1), generator=g) if flags else block - 1
+    im = ((torch.arange(T).view(1, T) - first) % block == 0).expand(B, T)
+
+    def run(cap):
+        L.lib().lmk_debug_set_max_ctas(cap)
+        try:
+            t = [x.to(DEV).requires_grad_(True) for x in (q, k, v)]
+            out = (P.landmark_attention_masked(*t, im.to(DEV), max_groups=16) if flags
+                   else P.fused_landmark_attention(*t, None, block_size=block))
+            return (out.detach(), *torch.autograd.grad(out, t, do.to(DEV)))
+        finally:
+            L.lib().lmk_debug_set_max_ctas(0)
+
+    ref = run(0)
+    for cap in (1, 2, 5):
+        assert all(torch.equal(a, b) for a, b in zip(run(cap), ref)), cap
+    f = [x.float().requires_grad_(True) for x in (q, k, v)]
+    out = O.lm_attention(*f, im)
+    for name, got, e in zip(("o", "dq", "dk", "dv"), ref, (out.detach(), *torch.autograd.grad(out, f, do.float()))):
+        got = got.float().cpu()
+        assert (got - e).abs().max().item() < 2e-2 * max(1.0, e.abs().max().item()), name
+        assert ((got - e).norm() / e.norm()).item() < 1e-2, name
+    assert L.device_status() == 0

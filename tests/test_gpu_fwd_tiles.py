@@ -19,10 +19,12 @@ def test_both_sides_of_the_tile_lines(H, Lq, D, block):
     q, k, v = [(torch.randn(1, H, Lq, D, generator=g) * 0.5).to(torch.bfloat16) for _ in range(3)]
     out = P.fused_landmark_attention(q.cuda(), k.cuda(), v.cuda(), None, block_size=block)
     pad = -Lq % block                                      # the oracle wants whole blocks: zero rows behind the real ones
-    f = [torch.nn.functional.pad(t[:, -1:].float(), (0, 0, 0, pad)) for t in (q, k, v)]
-    exp = O.landmark_attention_grads(*f, torch.zeros_like(f[0]), block, sm_scale=D ** -0.5)[0][:, :, :Lq]
-    got = out[:, -1:].float().cpu()
-    # weights rounded to 16 bits in front of the product, the result behind it: the bound of the other kernel tests
-    assert (got - exp).abs().max().item() < 2e-2
-    assert ((got - exp).norm() / exp.norm()).item() < 1e-2
+    f = [torch.nn.functional.pad(t.float(), (0, 0, 0, pad)) for t in (q, k, v)]
+    for h in {0, H // 2, H - 1}:                           # (a head at a time: the oracle holds its scores)
+        one = [t[:, h:h + 1] for t in f]
+        exp = O.landmark_attention_grads(*one, torch.zeros_like(one[0]), block, sm_scale=D ** -0.5)[0][:, :, :Lq]
+        got = out[:, h:h + 1].float().cpu()
+        # weights rounded to 16 bits in front of the product, the result behind it: the bound of the other kernel tests
+        assert (got - exp).abs().max().item() < 2e-2, h
+        assert ((got - exp).norm() / exp.norm()).item() < 1e-2, h
     assert L.device_status() == 0
