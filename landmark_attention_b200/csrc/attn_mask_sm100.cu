@@ -440,7 +440,8 @@ sm100_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tmem = tmem_slot;
       held = true;
     }
-    mask_fwd_tile<kBf16>(tm_q, tm_k, tm_v, is_mem, is_mem_stride, o_ptr, R_ptr, A_ptr, H, Lq, Lk, G, scale_log2, status, t, bh, tmem);
+    mask_fwd_tile<kBf16>(tm_q, tm_k, tm_v, is_mem, is_mem_stride, o_ptr, R_ptr, A_ptr, H, Lq, Lk, G, scale_log2, status, t, bh,
+                         tmem);
   }
   if (held && warp == 5) {
     tc_fence_after();
@@ -785,8 +786,8 @@ sm100_mask_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       tmem = tmem_slot;
       held = true;
     }
-    mask_bwd_dq_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, o_ptr, do_ptr, do_b, do_h, do_row, R_ptr, A_ptr, delta_ptr,
-                            nD_ptr, dq_ptr, H, Lq, Lk, G, scale, scale_log2, plan, plan_stride, status, t, bh, tmem);
+    mask_bwd_dq_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, o_ptr, do_ptr, do_b, do_h, do_row, R_ptr, A_ptr,
+                            delta_ptr, nD_ptr, dq_ptr, H, Lq, Lk, G, scale, scale_log2, plan, plan_stride, status, t, bh, tmem);
   }
   if (held && warp == 5) {
     tc_fence_after();
@@ -1119,8 +1120,8 @@ __global__ void __launch_bounds__(kMkThreads, 1)
 sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                           const uint8_t* is_mem, int64_t is_mem_stride, const float* R_ptr, const float* A_ptr,
-                          const float* delta_ptr, const float* nD_ptr, void* dk_ptr, void* dv_ptr, int H, int BH, int Lq, int Lk, int G, float scale, float scale_log2,
-                          const int* plan, int plan_stride, int* status) {
+                          const float* delta_ptr, const float* nD_ptr, void* dk_ptr, void* dv_ptr, int H, int BH, int Lq, int Lk,
+                          int G, float scale, float scale_log2, const int* plan, int plan_stride, int* status) {
   __shared__ uint32_t tmem_slot;
   const int n_tiles = Lk / kKT;
   const uint32_t warp = threadIdx.x >> 5;
@@ -1146,8 +1147,8 @@ sm100_mask_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       tmem = tmem_slot;
       held = true;
     }
-    mask_bwd_dkv_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, R_ptr, A_ptr, delta_ptr, nD_ptr, dk_ptr, dv_ptr, H, Lq, Lk,
-                             G, scale, scale_log2, status, kt, bh, tmem);
+    mask_bwd_dkv_tile<kBf16>(tm_q, tm_k, tm_v, tm_do, is_mem, is_mem_stride, R_ptr, A_ptr, delta_ptr, nD_ptr, dk_ptr, dv_ptr, H,
+                             Lq, Lk, G, scale, scale_log2, status, kt, bh, tmem);
   }
   if (held && warp == 5) {
     tc_fence_after();

@@ -129,10 +129,10 @@ __device__ __forceinline__ float row_sum(const float (&v)[64]) {
 // kernels of attn_mask_sm100.cu: the forward kernel marks them in R, the backward ones find them in the plan.
 constexpr int kIrrMaxTiles = 65;                    // 64 landmarks and the open group
 constexpr int kIrrMaxKeys = 64 * kIrrMaxTiles;
-// The single pass works on 64 columns a group, however short the group is.  Measured (us, forward + backward, single-pass / two-pass
-// kernels): B16 H8 T512, groups of 10 keys 525 / 625, 16 365 / 593, 51 183 / 361; B2 H8 T512, of 10 182 / 209, 51 98 / 122;
-// B16 H8 T256, of 8 258 / 228, 10 219 / 225, 16 159 / 216.  The line (16 keys a group, counted 256 keys longer than the row is) falls
-// at 8 keys for 256 and at 11 for 512: groups of 8 to 11 keys of longer rows would gain from a lower one.
+// The single pass works on 64 columns a group, however short the group is.  Measured (us, forward + backward, single-pass /
+// two-pass kernels): B16 H8 T512, groups of 10 keys 525 / 625, 16 365 / 593, 51 183 / 361; B2 H8 T512, of 10 182 / 209,
+// 51 98 / 122; B16 H8 T256, of 8 258 / 228, 10 219 / 225, 16 159 / 216.  The line (16 keys a group, counted 256 keys longer than
+// the row is) falls at 8 keys for 256 and at 11 for 512: groups of 8 to 11 keys of longer rows would gain from a lower one.
 constexpr int kIrrMinMeanGroup = 16;
 
 struct IrrArgs {
@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(256) irr_plan_kernel(const uint8_t* flags, int
   for (int k = threadIdx.x; k < Lk; k += blockDim.x) own[k] = (uint8_t)irr_group(t, k);
 }
 
-// Hides the columns of the group before (c0 of them, the same for the whole warp), eight at a time up to the last one: eight tests of
-// their own, one a chunk, took 400 - 600 clk an item whatever c0 was (clock stamps, groups of 51), nested ones end with the chunk
-// that needs them.
+// Hides the columns of the group before (c0 of them, the same for the whole warp), eight at a time up to the last one: eight
+// tests of their own, one a chunk, took 400 - 600 clk an item whatever c0 was (clock stamps, groups of 51), nested ones end with
+// the chunk that needs them.
 template <int kChunk = 0, typename GetFn>
 __device__ __forceinline__ void irr_hide(GetFn col, int c0) {
   if constexpr (kChunk < 8) {
@@ -260,7 +260,8 @@ __device__ __forceinline__ void irr_hide(GetFn col, int c0) {
 // (rows 256u .. 256u+127), warpgroup 1 owns tile B (the next 128 rows).  Both tiles consume the same K/V stream, so
 // every K/V block is fetched from L2 once per 256 query rows, and the two softmax pipelines overlap with each
 // other and with the MMAs.  Tile A skips the two newest key blocks (they lie after its own blocks).
-// With one tile a CTA uses half of the registers, TMEM and shared memory, so that two CTAs share an SM and each other's start and end.
+// With one tile a CTA uses half of the registers, TMEM and shared memory, so that two CTAs share an SM and each other's start
+// and end.
 template <int kTiles> constexpr int kFwdStages = kTiles == 2 ? 5 : 2;
 template <int kTiles> constexpr int kFwdThreads = (4 * kTiles + 3) * 32;
 enum { kErrFwd2Producer = 111, kErrFwd2Mma = 112, kErrFwd2Softmax = 113, kErrFwd2Epilogue = 114 };
@@ -387,74 +388,70 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     // ------------------------------------------------------------------ MMA issuer 1: S = Q K^T
     // A second issuing warp takes the P V products: the S products of the next key block never queue behind a wait for the
     // softmax of the current one.
-    {
-      constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 64, 0, 0);
-      mbar_wait(smem_u32(&sm->q_full), 0, &g_lmk_status, kErrFwd2Mma);
-      const uint64_t dq0 = smem_desc_sw128(q_tile(0), 16, 1024);
-      const uint64_t dk0 = smem_desc_sw128(k_slot(0), 16, 1024);
-      int ks[2] = {0, 0};
-      int s = 0;
-      uint32_t ph = 0;
-      for (int j = 0; j < total; ++j) {
-        mbar_wait(smem_u32(&sm->full[s]), ph, &g_lmk_status, kErrFwd2Mma);
-        const uint64_t dk = desc_advance(dk0, (uint32_t)s * 32768u);
+    constexpr uint32_t fmt = kBf16 ? 1u : 0u;
+    constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 64, 0, 0);
+    mbar_wait(smem_u32(&sm->q_full), 0, &g_lmk_status, kErrFwd2Mma);
+    const uint64_t dq0 = smem_desc_sw128(q_tile(0), 16, 1024);
+    const uint64_t dk0 = smem_desc_sw128(k_slot(0), 16, 1024);
+    int ks[2] = {0, 0};
+    int s = 0;
+    uint32_t ph = 0;
+    for (int j = 0; j < total; ++j) {
+      mbar_wait(smem_u32(&sm->full[s]), ph, &g_lmk_status, kErrFwd2Mma);
+      const uint64_t dk = desc_advance(dk0, (uint32_t)s * 32768u);
 #pragma unroll
-        for (int w = 0; w < kTiles; ++w) {
-          if (!active(w, j)) continue;
-          const int k = ks[w]++, sb = k & 1;
-          if (k >= 2) mbar_wait(smem_u32(&sm->s_free[w][sb]), ((k >> 1) & 1) ^ 1, &g_lmk_status, kErrFwd2Mma);
-          tc_fence_after();
-          const uint64_t dq = desc_advance(dq0, (uint32_t)w * 32768u);
-          if (elect_one()) {
+      for (int w = 0; w < kTiles; ++w) {
+        if (!active(w, j)) continue;
+        const int k = ks[w]++, sb = k & 1;
+        if (k >= 2) mbar_wait(smem_u32(&sm->s_free[w][sb]), ((k >> 1) & 1) ^ 1, &g_lmk_status, kErrFwd2Mma);
+        tc_fence_after();
+        const uint64_t dq = desc_advance(dq0, (uint32_t)w * 32768u);
+        if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk)
-              mma_f16_ss(tmem_s(w, sb), desc_advance(dq, kmajor_step(kk, kTileBytes)),
-                         desc_advance(dk, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
-            mma_commit(smem_u32(&sm->s_full[w][sb]));
-          }
+          for (int kk = 0; kk < kD / 16; ++kk)
+            mma_f16_ss(tmem_s(w, sb), desc_advance(dq, kmajor_step(kk, kTileBytes)),
+                       desc_advance(dk, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
+          mma_commit(smem_u32(&sm->s_full[w][sb]));
         }
-        if (++s == kStages) { s = 0; ph ^= 1; }
       }
+      if (++s == kStages) { s = 0; ph ^= 1; }
     }
     __syncwarp();
   } else if (warp == kSw + 2) {
     // ------------------------------------------------------------------ MMA issuer 2: O += P V
-    {
-      constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_o = instr_desc_f16(fmt, 128, kD, 0, 1);
-      const uint64_t dv0 = smem_desc_sw128(v_slot(0), kHalfTile, 1024);
-      int kp[2] = {0, 0};
-      bool o_started[2] = {false, false};
-      int s = 0;
-      for (int i = 0; i < total; ++i) {
-        const uint64_t dv = desc_advance(dv0, (uint32_t)s * 32768u);
+    constexpr uint32_t fmt = kBf16 ? 1u : 0u;
+    constexpr uint32_t idesc_o = instr_desc_f16(fmt, 128, kD, 0, 1);
+    const uint64_t dv0 = smem_desc_sw128(v_slot(0), kHalfTile, 1024);
+    int kp[2] = {0, 0};
+    bool o_started[2] = {false, false};
+    int s = 0;
+    for (int i = 0; i < total; ++i) {
+      const uint64_t dv = desc_advance(dv0, (uint32_t)s * 32768u);
 #pragma unroll
-        for (int w = 0; w < kTiles; ++w) {
-          if (!active(w, i)) continue;
-          const int k = kp[w]++;
-          mbar_wait(smem_u32(&sm->p_ready[w][k & 1]), (k >> 1) & 1, &g_lmk_status, kErrFwd2Mma);
-          tc_fence_after();
-          if (i >= n_lm_tiles) {
-            // A = P straight from TMEM: the softmax threads wrote it over the first 32 columns of the S buffer it was
-            // computed from (8 columns = 16 keys per K-step)
-            const uint32_t tp = tmem_s(w, k & 1);
-            if (elect_one()) {
+      for (int w = 0; w < kTiles; ++w) {
+        if (!active(w, i)) continue;
+        const int k = kp[w]++;
+        mbar_wait(smem_u32(&sm->p_ready[w][k & 1]), (k >> 1) & 1, &g_lmk_status, kErrFwd2Mma);
+        tc_fence_after();
+        if (i >= n_lm_tiles) {
+          // A = P straight from TMEM: the softmax threads wrote it over the first 32 columns of the S buffer it was
+          // computed from (8 columns = 16 keys per K-step)
+          const uint32_t tp = tmem_s(w, k & 1);
+          if (elect_one()) {
 #pragma unroll
-              for (int kk = 0; kk < kBlk / 16; ++kk)
-                mma_f16_ts(tmem_o(w), tp + kk * 8, desc_advance(dv, kk * 2048), idesc_o,
-                           (o_started[w] || kk > 0) ? 1u : 0u);
-            }
-            o_started[w] = true;
+            for (int kk = 0; kk < kBlk / 16; ++kk)
+              mma_f16_ts(tmem_o(w), tp + kk * 8, desc_advance(dv, kk * 2048), idesc_o,
+                         (o_started[w] || kk > 0) ? 1u : 0u);
           }
-          if (elect_one()) mma_commit(smem_u32(&sm->s_free[w][k & 1]));      // the S / P buffer may take the next S product
+          o_started[w] = true;
         }
-        // the stage is free once both P V products are done; each of them waited for its S product to be read
-        if (elect_one()) mma_commit(smem_u32(&sm->empty[s]));
-        if (++s == kStages) s = 0;
+        if (elect_one()) mma_commit(smem_u32(&sm->s_free[w][k & 1]));      // the S / P buffer may take the next S product
       }
-      if (elect_one()) mma_commit(smem_u32(&sm->o_full));
+      // the stage is free once both P V products are done; each of them waited for its S product to be read
+      if (elect_one()) mma_commit(smem_u32(&sm->empty[s]));
+      if (++s == kStages) s = 0;
     }
+    if (elect_one()) mma_commit(smem_u32(&sm->o_full));
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ softmax warpgroups
@@ -465,7 +462,8 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int own = kIrr ? group_of(pos) : own0_a + 2 * w + half;
     const int vis = min(kIrr ? 63 - (end_of(own) - pos) : row & 63, kBlk - 2);
     // kIrr: newest and oldest own tile of the warp's rows; ends of the next tile that this warp takes and of the one before it
-    const int own_max = kIrr ? __reduce_max_sync(0xffffffffu, own) : own, own_min = kIrr ? __reduce_min_sync(0xffffffffu, own) : own;
+    const int own_max = kIrr ? __reduce_max_sync(0xffffffffu, own) : own;
+    const int own_min = kIrr ? __reduce_min_sync(0xffffffffu, own) : own;
     int e_hi = 0, e_lo = 0;
     if constexpr (kIrr) {
       const int first = kTiles == 2 && w == 0 ? last_a : n_last;
@@ -481,7 +479,8 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         const int n = e / (kD / 8), c = e - n * (kD / 8);
         uint4 x = make_uint4(0u, 0u, 0u, 0u);
         if (c * 8 < D) x = *reinterpret_cast<const uint4*>(kb + (int64_t)end_of(n) * ks_row + c * 8);
-        const uint32_t addr = k_slot(0) + (uint32_t)(c >> 3) * kHalfTile + (uint32_t)n * 128u + (uint32_t)(((c & 7) ^ (n & 7)) << 4);
+        const uint32_t addr = k_slot(0) + (uint32_t)(c >> 3) * kHalfTile + (uint32_t)n * 128u +
+                              (uint32_t)(((c & 7) ^ (n & 7)) << 4);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
       }
       fence_proxy_async_smem();
@@ -643,8 +642,8 @@ sm100_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 // that two softmax warpgroups fit next to the issuing warps).
 //   kind 0: block after the row's own block -> zeros;  kind 1: own block (causal, landmark hidden);
 //   kind 2: earlier block (grouped).
-// one in this many pairs of exponentials uses ex2_poly2, a cubic (forward + backward, us: B4 H16 L1024 D64 2 -> 91.4, 3 -> 90.4, 4 ->
-// 90.3, 64 -> 91.3; B1 H32 L8192 D128 2 -> 2590, 3 -> 2577, 4 -> 2566)
+// one in this many pairs of exponentials uses ex2_poly2, a cubic (forward + backward, us: B4 H16 L1024 D64 2 -> 91.4, 3 -> 90.4,
+// 4 -> 90.3, 64 -> 91.3; B1 H32 L8192 D128 2 -> 2590, 3 -> 2577, 4 -> 2566)
 constexpr int kBwdPolyEvery = 4;
 
 template <bool kBf16>
@@ -911,7 +910,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   auto q_slot = [&](int s) { return base + 2 * kOperand + (uint32_t)s * 2 * kOperand; };
   auto do_slot = [&](int s) { return base + 3 * kOperand + (uint32_t)s * 2 * kOperand; };
   const uint32_t w_tile = base + (2 + 2 * kStages) * kOperand;         // P, then dS: [128 q x 64 keys] of block a, then of b
-  DkvSmem<kStages>* sm = reinterpret_cast<DkvSmem<kStages>*>(smem_raw + (base - raw) + (2 + 2 * kStages) * kOperand + 2 * kTileBytes);
+  DkvSmem<kStages>* sm =
+      reinterpret_cast<DkvSmem<kStages>*>(smem_raw + (base - raw) + (2 + 2 * kStages) * kOperand + 2 * kTileBytes);
 
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int prefix_blocks = (Lk - Lq) / kBlk;
@@ -1056,8 +1056,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       ++u;
     }
   } else if (warp == kBwdGroups * 4 + 2) {
-    // dV += P^T dO and dK += dS^T Q.  A = P^T / dS^T: MN-major view of the two [128 q x 64 keys] tiles; B = dO / Q: MN-major view of
-    // the row-major [128 q x kD] tile; a K-step is 16 query rows = 2048 bytes.  dV waits for dO itself: P may be there first.
+    // dV += P^T dO and dK += dS^T Q.  A = P^T / dS^T: MN-major view of the two [128 q x 64 keys] tiles; B = dO / Q: MN-major view
+    // of the row-major [128 q x kD] tile; a K-step is 16 query rows = 2048 bytes.  dV waits for dO itself: P may be there first.
     constexpr uint32_t fmt = kBf16 ? 1u : 0u;
     constexpr uint32_t idesc_t = instr_desc_f16(fmt, 128, kD, 1, 1);
     const uint64_t dq0t = smem_desc_sw128(q_slot(0), kTileBytes, 1024);
@@ -1106,7 +1106,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     auto stat_m = [&](int64_t i) { return ld_behind_wait((kIrr && irr.R != nullptr ? irr.R : M_ptr) + i); };
     auto stat_l = [&](int64_t i) { return kIrr && irr.R != nullptr ? 1.f : ld_behind_wait(L_ptr + i); };
     // What a unit needs from global memory, asked for while the unit before it drains: the tile table first (all entries at
-    // once), then the row statistics of the first item.  Read one after the other at the start of a unit they took 1500 - 2000 clk of it.
+    // once), then the row statistics of the first item.  Read one after the other at the start of a unit they took
+    // 1500 - 2000 clk of it.
     // (rows past the end of the sequence have zero Q and dO tiles: whatever finite weights they get contribute nothing)
     int bh = -1, b = 0, pair = 0, tq0 = 0, tiles = n_blocks, e_m = 0, e_0 = 0, e_1 = 0;      // bh < 0: no unit left
     float nM = 0.f, nL = 1.f, nDelta = 0.f;
@@ -1151,7 +1152,8 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int own = kIrr ? nOwn : prefix_blocks + 2 * tq + half;
         const int vis = min(kIrr ? 63 - (end - (Lk - Lq + tq * kQTile + row)) : row & 63, kBlk - 2);      // used where n == own
         const bool row_valid = kWhole || tq * kQTile + row < Lq;
-        const float M2L = !row_valid ? 0.f : (kIrr && irr.R != nullptr ? nM : fmaf(nM, kLog2e, __log2f(nL))), delta = row_valid ? nDelta : 0.f;
+        const float M2L = !row_valid ? 0.f : (kIrr && irr.R != nullptr ? nM : fmaf(nM, kLog2e, __log2f(nL)));
+        const float delta = row_valid ? nDelta : 0.f;
         if (i + 1 < n_items) fetch_rows(tq + 1);      // one item ahead, so that their latency is never exposed
         const int kind = n > own ? 0 : (n == own ? 1 : 2);
         mbar_wait(smem_u32(&sm->s_full), it & 1, &g_lmk_status, kErrDkvSoftmax);
@@ -1219,7 +1221,7 @@ sm100_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       grid_dep_wait();     // delta comes from the dQ kernel, which may still be running (see the launch)
       fetch_unit();
       while (bh >= 0) run_unit();
-    } else {               // nothing but the statistics to ask for: holding them over the epilogue's stores costs more than it hides
+    } else {      // nothing but the statistics to ask for: holding them over the epilogue's stores costs more than it hides
       for (int k = 0, w = unit_of(0); w < n_units; w = unit_of(++k)) {
         pair = w / BH;
         bh = w - pair * BH;
@@ -1381,64 +1383,60 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   } else if (warp == kBwdGroups * 4 + 1 || warp == kBwdGroups * 4 + 3) {
     // warp +1 issues S = Q K^T, warp +3 issues dP = dO V^T; both walk through the same items and wait for the same
     // barriers (each is a waiter of its own on full / ops_ready and sees every phase)
-    {
-      constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 64, 0, 0);
-      const bool is_s = warp == kBwdGroups * 4 + 1;
-      const uint64_t db0 = smem_desc_sw128(is_s ? k_slot(0) : v_slot(0), 16, 1024);
-      const uint32_t t_out = is_s ? tmem_s : tmem_dp, t_a = is_s ? tmem_q : tmem_do;
-      int it = 0, u = 0;
-      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-        if (warp_uniform(skipped(w))) continue;
-        const int total = warp_uniform(unit_items(w));
-        for (int i = 0; i < total; ++i, ++it) {
-          const int s = it % kDqStages, sb = it % kSdpBufs;
-          mbar_wait(smem_u32(&sm->full[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
-          if (it >= kSdpBufs)
-            mbar_wait(smem_u32(is_s ? &sm->s_free[sb] : &sm->dp_free[sb]), ((it / kSdpBufs) & 1) ^ 1, &g_lmk_status, kErrDqMma);
-          // the unit's rows come last: waited for in front of the other two they cost the unit another 1000 clk
-          if (i == 0) mbar_wait(smem_u32(&sm->ops_ready), u & 1, &g_lmk_status, kErrDqMma);
-          tc_fence_after();
-          const uint64_t db = desc_advance(db0, (uint32_t)s * 32768u);
-          if (elect_one()) {
+    constexpr uint32_t fmt = kBf16 ? 1u : 0u;
+    constexpr uint32_t idesc_s = instr_desc_f16(fmt, 128, 64, 0, 0);
+    const bool is_s = warp == kBwdGroups * 4 + 1;
+    const uint64_t db0 = smem_desc_sw128(is_s ? k_slot(0) : v_slot(0), 16, 1024);
+    const uint32_t t_out = is_s ? tmem_s : tmem_dp, t_a = is_s ? tmem_q : tmem_do;
+    int it = 0, u = 0;
+    for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+      if (warp_uniform(skipped(w))) continue;
+      const int total = warp_uniform(unit_items(w));
+      for (int i = 0; i < total; ++i, ++it) {
+        const int s = it % kDqStages, sb = it % kSdpBufs;
+        mbar_wait(smem_u32(&sm->full[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
+        if (it >= kSdpBufs)
+          mbar_wait(smem_u32(is_s ? &sm->s_free[sb] : &sm->dp_free[sb]), ((it / kSdpBufs) & 1) ^ 1, &g_lmk_status, kErrDqMma);
+        // the unit's rows come last: waited for in front of the other two they cost the unit another 1000 clk
+        if (i == 0) mbar_wait(smem_u32(&sm->ops_ready), u & 1, &g_lmk_status, kErrDqMma);
+        tc_fence_after();
+        const uint64_t db = desc_advance(db0, (uint32_t)s * 32768u);
+        if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk)      // A from TMEM: 8 columns = 16 features per K-step
-              mma_f16_ts(t_out + sb * 64, t_a + kk * 8, desc_advance(db, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
-            mma_commit(smem_u32(is_s ? &sm->s_full[sb] : &sm->dp_full[sb]));
-          }
+          for (int kk = 0; kk < kD / 16; ++kk)      // A from TMEM: 8 columns = 16 features per K-step
+            mma_f16_ts(t_out + sb * 64, t_a + kk * 8, desc_advance(db, kmajor_step(kk, kHalfTile)), idesc_s, kk > 0);
+          mma_commit(smem_u32(is_s ? &sm->s_full[sb] : &sm->dp_full[sb]));
         }
-        if (elect_one()) mma_commit(smem_u32(&sm->ops_free));        // the next unit's Q / dO rows may be written
-        ++u;
       }
+      if (elect_one()) mma_commit(smem_u32(&sm->ops_free));        // the next unit's Q / dO rows may be written
+      ++u;
     }
     __syncwarp();
   } else if (warp == kBwdGroups * 4 + 2) {
-    {
-      constexpr uint32_t fmt = kBf16 ? 1u : 0u;
-      constexpr uint32_t idesc_q = instr_desc_f16(fmt, 128, kD, 0, 1);   // dQ += dS K  (K is MN-major)
-      const uint64_t dv0 = smem_desc_sw128(v_slot(0), 16, 1024);
-      const uint64_t dk0t = smem_desc_sw128(k_slot(0), kHalfTile, 1024);
-      int it = 0, u = 0;
-      for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
-        if (warp_uniform(skipped(w))) continue;
-        const int total = warp_uniform(unit_items(w));
-        for (int i = 0; i < total; ++i, ++it) {
-          const int s = it % kDqStages;
-          if (i == 0) mbar_wait(smem_u32(&sm->acc_empty), (u & 1) ^ 1, &g_lmk_status, kErrDqMma);
-          mbar_wait(smem_u32(&sm->ds_ready[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
-          tc_fence_after();
-          const uint64_t dds = desc_advance(dv0, (uint32_t)s * 32768u), dkt = desc_advance(dk0t, (uint32_t)s * 32768u);
-          if (elect_one()) {
+    constexpr uint32_t fmt = kBf16 ? 1u : 0u;
+    constexpr uint32_t idesc_q = instr_desc_f16(fmt, 128, kD, 0, 1);   // dQ += dS K  (K is MN-major)
+    const uint64_t dv0 = smem_desc_sw128(v_slot(0), 16, 1024);
+    const uint64_t dk0t = smem_desc_sw128(k_slot(0), kHalfTile, 1024);
+    int it = 0, u = 0;
+    for (int r = 0, w = unit_of(0); w < n_units; w = unit_of(++r)) {
+      if (warp_uniform(skipped(w))) continue;
+      const int total = warp_uniform(unit_items(w));
+      for (int i = 0; i < total; ++i, ++it) {
+        const int s = it % kDqStages;
+        if (i == 0) mbar_wait(smem_u32(&sm->acc_empty), (u & 1) ^ 1, &g_lmk_status, kErrDqMma);
+        mbar_wait(smem_u32(&sm->ds_ready[s]), (it / kDqStages) & 1, &g_lmk_status, kErrDqMma);
+        tc_fence_after();
+        const uint64_t dds = desc_advance(dv0, (uint32_t)s * 32768u), dkt = desc_advance(dk0t, (uint32_t)s * 32768u);
+        if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kBlk / 16; ++kk)
-              mma_f16_ss(tmem_dq, desc_advance(dds, kk * 32), desc_advance(dkt, kk * 2048), idesc_q,
-                         (i > 0 || kk > 0) ? 1u : 0u);
-            mma_commit(smem_u32(&sm->empty[s]));
-          }
+          for (int kk = 0; kk < kBlk / 16; ++kk)
+            mma_f16_ss(tmem_dq, desc_advance(dds, kk * 32), desc_advance(dkt, kk * 2048), idesc_q,
+                       (i > 0 || kk > 0) ? 1u : 0u);
+          mma_commit(smem_u32(&sm->empty[s]));
         }
-        if (elect_one()) mma_commit(smem_u32(&sm->acc_full[(it - 1) & 1]));     // drained by the warpgroup that took the last item
-        ++u;
       }
+      if (elect_one()) mma_commit(smem_u32(&sm->acc_full[(it - 1) & 1]));     // drained by the warpgroup that took the last item
+      ++u;
     }
     __syncwarp();
   } else {
@@ -1546,9 +1544,10 @@ sm100_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             delta = fmaf(fo.y, fg.y, delta);
           }
         }
-      // The shared-memory tiles may take the next unit's rows.  TMA writes them through another proxy than these loads went through,
-      // and an arrival alone does not hold it back until they are done: of 15 000 calls at B4 H16 L1024 D64 twenty had rows of dQ
-      // from tiles half overwritten, always of a unit with no more items than stages, behind which the producer is already waiting.
+      // The shared-memory tiles may take the next unit's rows.  TMA writes them through another proxy than these loads went
+      // through, and an arrival alone does not hold it back until they are done: of 15 000 calls at B4 H16 L1024 D64 twenty had
+      // rows of dQ from tiles half overwritten, always of a unit with no more items than stages, behind which the producer is
+      // already waiting.
       fence_proxy_async_smem();
       mbar_arrive(smem_u32(&sm->delta_read));
       // row -> TMEM lane, 32-bit word j (two features) -> column j: the layout of a K-major A operand
@@ -1927,7 +1926,8 @@ static int launch_bwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaSt
   if (cap >= 1 && cap < n_sm) n_sm = cap;
   // key tiles of a batch row: whole blocks, or at most that many groups
   const int max_tiles = irr == nullptr ? (p.Lk + kBlk - 1) / kBlk
-                        : (irr->flags != nullptr ? (irr->G < kIrrMaxTiles - 1 ? irr->G : kIrrMaxTiles - 1) + 1 : (p.Lk - 1) / irr->block + 1);
+                        : irr->flags != nullptr ? (irr->G < kIrrMaxTiles - 1 ? irr->G : kIrrMaxTiles - 1) + 1
+                                                : (p.Lk - 1) / irr->block + 1;
   const int dkv_units = ((max_tiles + 1) / 2) * p.B * p.H;
   const int dq_units = ((p.Lq + kQTile - 1) / kQTile) * p.B * p.H;
   dim3 grid_dkv(dkv_units < n_sm ? dkv_units : n_sm), grid_dq(dq_units < n_sm ? dq_units : n_sm);
