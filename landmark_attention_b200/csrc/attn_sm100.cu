@@ -1801,16 +1801,22 @@ int tensor_map_4d(CUtensorMap* m, const void* ptr, int dtype, int B, int H, int 
 bool tensor_map_operand_ok(const void* p, const int64_t st[3]) { return tma_ok(p, st); }
 
 // Two query tiles a CTA share one K/V stream; one tile a CTA puts two CTAs on an SM, whose starts and ends overlap and which the
-// hardware deals out in smaller pieces.  Measured (us a call, one / two): D128, 32 heads of L = 512 11.5 / 13.5, 768 15.3 / 17.1,
-// 896 19.2 / 17.3, 1024 22.2 / 20.7, 2048 43.0 / 39.9, 8192 545 / 469; 256 heads of 512 45.9 / 49.7; small grids, 8 heads of 1024 18.0 /
-// 18.8, 3072 44.1 / 45.1, 4096 61.7 / 59.7.  Heads of 64 features have half the products for the stream to feed: 64 heads of 1024
-// 22.2 / 25.7, of 2048 66 / 73, 32 heads of 4096 112 / 118, 8192 423 / 409.  Groups as key tiles: 51 keys, 128 heads of 512 29.6 / 31.7,
-// 32 heads of 1024 28.2 / 31.4, 32-key blocks at 1280 51.1 / 54.1, 1700 69.0 / 67.3.  A single tile of a long history wants the deeper
-// pipeline of the second form.
+// hardware deals out in smaller pieces.  Measured (us, one / two):
+//   D128, 32 heads of L = 512 11.5 / 13.5, 768 15.3 / 17.1, 896 19.2 / 17.3, 1024 22.2 / 20.7, 2048 43.0 / 39.9, 8192 545 / 469;
+//   256 heads of 512 45.9 / 49.7.  Grids below 1.5 tiles an SM: 8 heads of 1024 18.0 / 18.8, 3072 44.1 / 45.1; at 1.73 (8 heads of
+//   4096, 16 of 2048) both take the same.
+//   Heads of 64 features have half the products for the stream to feed: 64 heads of 1024 22.2 / 25.7, of 2048 66 / 73, 32 heads of
+//   4096 112 / 118, 8192 423 / 409; below two tiles an SM 8 heads of 4224 54 / 67, 4 of 8192 98 / 120.  Above 32 tiles one stays
+//   ahead up to about five an SM (8 heads of 6144 80 / 94, 16 of 6144 127 / 133), where the line does not lie yet.
+//   Groups as key tiles, D128: 51 keys, 128 heads of 512 29.6 / 31.7, 32 heads of 1024 28.2 / 31.4, of 1664 51 / 55, 1920 65 / 67;
+//   32-key blocks, 32 heads of 1280 51.1 / 54.1, 1700 70 / 68 (an even number of tiles), 1920 81 / 86, 2000 90 / 86, 16 heads of
+//   2000 (below two tiles an SM) 74 / 80.  D64: 32-key blocks, 64 heads of 1920 131 / 148, 2000 148 / 153.
+// A single tile of a long history wants the deeper pipeline of the second form.
 static int fwd_tiles_per_cta(int n_tiles, int BH, int n_sm, bool irr, int D) {
   if (n_tiles == 1) return 2;
-  const int most = irr ? 12 : D <= 64 ? 32 : 6;
-  return n_tiles <= most || (int64_t)n_tiles * BH <= n_sm + n_sm / 2 ? 1 : 2;
+  const int most = irr ? (D <= 64 ? 16 : 15) : (D <= 64 ? 32 : 6);
+  const int64_t few = irr || D <= 64 ? 2 * n_sm : n_sm + n_sm / 2;
+  return n_tiles <= most || (int64_t)n_tiles * BH <= few ? 1 : 2;
 }
 
 static int launch_fwd(const AttnParams& p, int dtype, const IrrArgs* irr, cudaStream_t st) {

@@ -13,7 +13,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("H,Lq,D,block", [
     (40, 768, 128, 64), (40, 896, 128, 64), (1, 896, 128, 64), (40, 833, 128, 64),      # six and seven tiles, few and many heads
     (8, 4096, 64, 64), (8, 4224, 64, 64),                                               # 32 and 33 tiles
-    (20, 1536, 128, 32), (20, 1664, 128, 32)])                                          # twelve and thirteen tiles
+    (20, 1536, 128, 32), (20, 1664, 128, 32),                                           # twelve and thirteen tiles
+    (9, 4096, 64, 64), (9, 4224, 64, 64),                                               # 32 and 33 tiles, two an SM and more
+    (20, 1920, 128, 32), (20, 2000, 128, 32), (18, 2048, 128, 32),                      # 15 and 16 tiles, few and many heads
+    (20, 2048, 64, 32), (20, 2080, 64, 32), (17, 2080, 64, 32)])                        # 16 and 17 tiles
 def test_both_sides_of_the_tile_lines(H, Lq, D, block):
     g = torch.Generator().manual_seed(Lq + H)
     q, k, v = [(torch.randn(1, H, Lq, D, generator=g) * 0.5).to(torch.bfloat16) for _ in range(3)]
